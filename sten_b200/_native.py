@@ -1,9 +1,11 @@
-"""ctypes binding of ``libnmg_b200.so`` (the C ABI declared in ``include/nmg_b200.h``).
+"""Loader of the two native parts: ``libnmg_b200.so`` (the C ABI declared in ``include/nmg_b200.h``, bound with ctypes) and
+``_nmg_host.so`` (the CPython extension every per-call path of the package goes through).
 
 The library is the only implementation of the arithmetic: if it cannot be loaded, or a tensor is not on a
 CUDA device, the operations raise -- there is no CPU or eager-PyTorch fallback.
 """
 import ctypes
+import importlib
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -85,3 +87,21 @@ def lib():
 def check(status):
     if status != 0:
         raise NmgError(status, lib().nmg_last_error().decode(errors="replace"))
+
+
+_host = None
+
+
+def host():
+    """The host extension (checks, allocation and the library call of every tensor-level entry point), loaded once."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            import torch  # noqa: F401  (its libraries must be in the process before the extension that links to them)
+            mod = importlib.import_module("sten_b200._nmg_host")
+        except ImportError as e:
+            raise ImportError(f"sten_b200/_nmg_host.so cannot be loaded ({e}): build it with `python -m sten_b200.build`") from e
+        mod.set_error_class(NmgError)
+        _host = mod
+    return _host

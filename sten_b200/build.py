@@ -1,4 +1,5 @@
-"""Ahead-of-time build of ``libnmg_b200.so`` (the C-ABI CUDA library) for sm_100a.
+"""Ahead-of-time build of ``libnmg_b200.so`` (the C-ABI CUDA library) for sm_100a and of ``_nmg_host.so`` (the CPython
+extension that checks tensors, allocates and calls the library).
 
     python -m sten_b200.build [--force] [--verbose]
 
@@ -14,10 +15,13 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libnmg_b200.so")
+HOST_SRC = os.path.join(CSRC, "host", "nmg_host.cpp")
+HOST_LIB = os.path.join(HERE, "_nmg_host.so")
 OBJ_DIR = os.path.join(HERE, "csrc", "build")
 
 NVCC_FLAGS = [
@@ -50,7 +54,40 @@ def _stamp():
     return h.hexdigest()
 
 
+def build_host(force=False, verbose=False):
+    """The host extension: one C++ file against the Python and torch headers, linked to the library next to it."""
+    import torch
+    from torch.utils import cpp_extension
+    h = hashlib.sha256(torch.__version__.encode() + sys.version.encode())
+    for p in (HOST_SRC, os.path.join(os.path.dirname(HERE), "include", "nmg_b200.h")):
+        with open(p, "rb") as fh:
+            h.update(fh.read())
+    stamp, stamp_file = h.hexdigest(), os.path.join(OBJ_DIR, "stamp_host")
+    if not force and os.path.isfile(HOST_LIB) and os.path.isfile(stamp_file) and open(stamp_file).read() == stamp:
+        return HOST_LIB
+    tmp = HOST_LIB + f".{os.getpid()}.tmp"
+    include = [sysconfig.get_paths()["include"], *cpp_extension.include_paths("cuda")]
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{p}" for p in include], HOST_SRC, "-o", tmp, *[f"-L{p}" for p in cpp_extension.library_paths("cuda")], f"-L{HERE}",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10_cuda", "-lc10", "-l:libnmg_b200.so", "-Wl,-rpath,$ORIGIN"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, HOST_LIB)
+    with open(stamp_file, "w") as f:
+        f.write(stamp)
+    return HOST_LIB
+
+
 def build(force=False, verbose=False):
+    lib = build_lib(force, verbose)
+    build_host(force, verbose)
+    return lib
+
+
+def build_lib(force=False, verbose=False):
     stamp_file = os.path.join(OBJ_DIR, "stamp")
     stamp = _stamp()
     if not force and os.path.isfile(LIB) and os.path.isfile(stamp_file) and open(stamp_file).read() == stamp:
@@ -71,7 +108,7 @@ def build(force=False, verbose=False):
     with concurrent.futures.ThreadPoolExecutor(max_workers=min(8, os.cpu_count() or 1)) as ex:
         objs = list(ex.map(compile_one, sources()))
     tmp = LIB + f".{os.getpid()}.tmp"
-    cmd = [nvcc, "-shared", "-o", tmp, *objs, "-gencode", "arch=compute_100a,code=sm_100a"]
+    cmd = [nvcc, "-shared", "-Xlinker", "-soname=libnmg_b200.so", "-o", tmp, *objs, "-gencode", "arch=compute_100a,code=sm_100a"]
     if verbose:
         print(" ".join(cmd), flush=True)
     r = subprocess.run(cmd, capture_output=True, text=True)

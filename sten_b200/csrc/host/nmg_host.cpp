@@ -1,0 +1,541 @@
+// Host path between Python and the C ABI: tensor checks, output and workspace allocation, and the calls themselves.
+//
+// A sparse linear of a few tokens runs for a few microseconds on the GPU, so what a call costs is the interpreter: with the
+// checks, the allocations and a 22-argument foreign-function call written in Python, one F.linear took 40 us of host time
+// (17 us of it here).  These are the same steps against the CPython and ATen interfaces (no argument parsing library:
+// positional arguments only, METH_FASTCALL).  All arithmetic stays in libnmg_b200.so.
+#include <Python.h>
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <string>
+#include <vector>
+
+#include "../../../include/nmg_b200.h"
+
+namespace {
+
+PyObject *g_error_class = nullptr;  // sten_b200._native.NmgError(status, message)
+PyObject *g_s_val, *g_s_idx, *g_s_packed, *g_s_packed_sp24;
+
+struct PyRaised {};  // a Python exception is set
+
+[[noreturn]] void py_raise(PyObject *type, const std::string &msg) {
+    PyErr_SetString(type, msg.c_str());
+    throw PyRaised();
+}
+
+void check(int status) {
+    if (status == NMG_OK) return;
+    PyObject *args = Py_BuildValue("(is)", status, nmg_last_error());
+    if (args) {
+        PyErr_SetObject(g_error_class ? g_error_class : PyExc_RuntimeError, args);
+        Py_DECREF(args);
+    }
+    throw PyRaised();
+}
+
+int dtype_code(const at::Tensor &t) {
+    switch (t.scalar_type()) {
+        case at::kFloat: return NMG_F32;
+        case at::kHalf: return NMG_F16;
+        case at::kBFloat16: return NMG_BF16;
+        default: break;
+    }
+    py_raise(PyExc_TypeError, std::string("grouped n:m kernels support float32, float16 and bfloat16, got ") + c10::toString(t.scalar_type()));
+}
+
+const at::Tensor &tensor_arg(PyObject *o) {
+    if (!THPVariable_Check(o)) py_raise(PyExc_TypeError, "expected a torch.Tensor");
+    return THPVariable_Unpack(o);
+}
+at::Tensor optional_tensor(PyObject *o) { return o == Py_None ? at::Tensor() : tensor_arg(o); }
+
+int64_t int_arg(PyObject *o) {
+    const long long v = PyLong_AsLongLong(o);
+    if (v == -1 && PyErr_Occurred()) throw PyRaised();
+    return v;
+}
+
+void require_cuda(const at::Tensor &t, c10::Device &dev, bool &have) {
+    if (!t.defined()) return;
+    if (!t.is_cuda())
+        py_raise(PyExc_RuntimeError, "grouped n:m kernels run on CUDA devices only (there is no CPU fallback); move the tensor with .cuda()");
+    if (!have) {
+        dev = t.device();
+        have = true;
+    } else if (t.device() != dev) {
+        py_raise(PyExc_RuntimeError, "operands live on different devices: " + dev.str() + " and " + t.device().str());
+    }
+}
+c10::Device device_of(std::initializer_list<const at::Tensor *> ts) {
+    c10::Device dev(c10::kCPU);
+    bool have = false;
+    for (const at::Tensor *t : ts) require_cuda(*t, dev, have);
+    return dev;
+}
+
+std::string shape_str(c10::IntArrayRef s) {
+    std::string r = "(";
+    for (size_t i = 0; i < s.size(); i++) r += (i ? ", " : "") + std::to_string(s[i]);
+    return r + (s.size() == 1 ? ",)" : ")");
+}
+
+// contiguous() with the call skipped where it would return the tensor itself
+at::Tensor packed_rows(const at::Tensor &t) { return t.is_contiguous() ? t : t.contiguous(); }
+
+// Rows of a 2-D operand with unit stride along them; the copy is made only where the strides do not allow it.
+struct Rows {
+    at::Tensor t;
+    int64_t rows, cols, ld;
+};
+Rows row_major_2d(const at::Tensor &t) {
+    if (t.dim() != 2) py_raise(PyExc_ValueError, "expected a 2-D tensor");
+    Rows r{t, t.size(0), t.size(1), 0};
+    if (t.stride(1) != 1 || t.stride(0) < r.cols) r.t = t.contiguous();
+    r.ld = r.t.is_contiguous() ? r.cols : r.t.stride(0);
+    return r;
+}
+// The same for an operand whose leading dims all count as rows.
+Rows rows_of(const at::Tensor &t, int64_t cols) {
+    if (t.dim() == 2) {
+        Rows r = row_major_2d(t);
+        if (r.cols != cols) py_raise(PyExc_ValueError, "activation shape " + shape_str(t.sizes()) + " does not match K=" + std::to_string(cols));
+        return r;
+    }
+    if (t.dim() < 1 || t.size(-1) != cols) py_raise(PyExc_ValueError, "activation shape " + shape_str(t.sizes()) + " does not match K=" + std::to_string(cols));
+    if (!t.is_contiguous()) return row_major_2d(t.reshape({cols ? t.numel() / cols : 0, cols}));
+    return Rows{t, cols ? t.numel() / cols : 0, cols, cols};
+}
+
+struct Geo {
+    int64_t M, K;
+    int n, m, g;
+};
+
+void *stream_of(c10::Device dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
+
+struct Epi {
+    int act = NMG_EPI_NONE;
+    at::Tensor residual;  // rows of the output's shape, contiguous along the last dim
+    int64_t ld = 0;
+};
+
+// out[rows_out][ld_out] = activation(product + bias) + residual; every operand has been checked against the others.
+void call_spmm(const Geo &geo, int code, c10::Device dev, const at::Tensor &val, const at::Tensor &idx, const at::Tensor &packed, const Rows &act,
+               int64_t tokens, const at::Tensor &bias, const Epi &epi, const at::Tensor &out, int64_t ld_out, int layout, int algo) {
+    const at::Tensor v = packed_rows(val), i = packed_rows(idx), b = bias.defined() ? packed_rows(bias) : bias;
+    const size_t nbytes = nmg_spmm_workspace_bytes(geo.M, geo.K, tokens, geo.n, geo.m, geo.g, code, layout, algo, packed.defined() ? 1 : 0);
+    at::Tensor ws;
+    if (nbytes) ws = at::empty({(int64_t)nbytes}, val.options().dtype(at::kByte));
+    void *st = stream_of(dev);
+    void *wsp = nbytes ? ws.mutable_data_ptr() : nullptr;
+    const void *pk = packed.defined() ? packed.const_data_ptr() : nullptr;
+    const void *bp = b.defined() ? b.const_data_ptr() : nullptr;
+    const int16_t *ip = static_cast<const int16_t *>(i.const_data_ptr());
+    int rc;
+    PyThreadState *save = PyEval_SaveThread();
+    if (epi.act != NMG_EPI_NONE || epi.residual.defined())
+        rc = nmg_spmm_fused(v.const_data_ptr(), ip, pk, geo.M, geo.K, geo.n, geo.m, geo.g, code, act.t.const_data_ptr(), act.ld, tokens, bp, epi.act,
+                            epi.residual.defined() ? epi.residual.const_data_ptr() : nullptr, epi.ld, out.mutable_data_ptr(), ld_out, layout, algo, wsp,
+                            nbytes, st);
+    else
+        rc = nmg_spmm(v.const_data_ptr(), ip, pk, geo.M, geo.K, geo.n, geo.m, geo.g, code, act.t.const_data_ptr(), act.ld, tokens, bp,
+                      out.mutable_data_ptr(), ld_out, layout, algo, wsp, nbytes, st);
+    PyEval_RestoreThread(save);
+    check(rc);
+}
+
+void call_spmm_t(const Geo &geo, int code, c10::Device dev, const at::Tensor &val, const at::Tensor &idx, const at::Tensor &packed, const at::Tensor &sp24,
+                 const Rows &dy, const at::Tensor &dx, int algo) {
+    const at::Tensor v = packed_rows(val), i = packed_rows(idx);
+    void *st = stream_of(dev);
+    at::Tensor ws;
+    size_t nbytes = 0;
+    if (!sp24.defined()) {
+        nbytes = nmg_spmm_t_workspace_bytes(geo.M, geo.K, dy.rows, geo.n, geo.m, geo.g, code, algo, packed.defined() ? 1 : 0);
+        if (nbytes) ws = at::empty({(int64_t)nbytes}, val.options().dtype(at::kByte));
+    }
+    int rc;
+    PyThreadState *save = PyEval_SaveThread();
+    if (sp24.defined())
+        rc = nmg_spmm_t_sp24(sp24.const_data_ptr(), geo.M, geo.K, geo.n, geo.m, geo.g, code, dy.t.const_data_ptr(), dy.ld, dy.rows, dx.mutable_data_ptr(),
+                             geo.K, st);
+    else
+        rc = nmg_spmm_t(v.const_data_ptr(), static_cast<const int16_t *>(i.const_data_ptr()), packed.defined() ? packed.const_data_ptr() : nullptr, geo.M,
+                        geo.K, geo.n, geo.m, geo.g, code, dy.t.const_data_ptr(), dy.ld, dy.rows, dx.mutable_data_ptr(), geo.K, algo,
+                        nbytes ? ws.mutable_data_ptr() : nullptr, nbytes, st);
+    PyEval_RestoreThread(save);
+    check(rc);
+}
+
+bool sp24_rows_ok(const Rows &dy) { return reinterpret_cast<uintptr_t>(dy.t.const_data_ptr()) % 16 == 0 && dy.ld % 8 == 0; }
+
+// ------------------------------------------------------------------------------------------------ module functions
+#define NMG_PY_BEGIN(nargs_wanted)                                                           \
+    HANDLE_TH_ERRORS                                                                         \
+    if (nargs != (nargs_wanted)) {                                                           \
+        PyErr_Format(PyExc_TypeError, "expected %d arguments, got %zd", (nargs_wanted), nargs); \
+        return nullptr;                                                                      \
+    }                                                                                        \
+    try {
+#define NMG_PY_END                    \
+    } catch (const PyRaised &) { return nullptr; } \
+    END_HANDLE_TH_ERRORS
+
+Geo geo_args(PyObject *const *a) { return Geo{int_arg(a[0]), int_arg(a[1]), (int)int_arg(a[2]), (int)int_arg(a[3]), (int)int_arg(a[4])}; }
+
+// spmm(val, idx, M, K, n, m, g, act, bias, layout, algo, out, packed, activation, residual) -> out
+PyObject *py_spmm(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(15)
+    const at::Tensor &val = tensor_arg(a[0]), &idx = tensor_arg(a[1]), &act0 = tensor_arg(a[7]);
+    const Geo geo = geo_args(a + 2);
+    const at::Tensor bias = optional_tensor(a[8]), out0 = optional_tensor(a[11]), packed = optional_tensor(a[12]), residual = optional_tensor(a[14]);
+    const int layout = (int)int_arg(a[9]), algo = (int)int_arg(a[10]);
+    const c10::Device dev = device_of({&val, &idx, &act0, &bias, &residual});
+    const int code = dtype_code(val);
+    if (act0.scalar_type() != val.scalar_type() || (bias.defined() && bias.scalar_type() != val.scalar_type()))
+        py_raise(PyExc_TypeError, std::string("activation / bias dtype must match the weight dtype ") + c10::toString(val.scalar_type()));
+    const c10::cuda::CUDAGuard guard(dev);
+    const Rows act = row_major_2d(act0);
+    const bool token_major = layout != NMG_ACT_K_MAJOR, out_tm = layout == NMG_ACT_TOKEN_MAJOR;
+    const int64_t tokens = token_major ? act.rows : act.cols;
+    if ((token_major ? act.cols : act.rows) != geo.K)
+        py_raise(PyExc_ValueError, "activation shape " + shape_str(act0.sizes()) + " does not match K=" + std::to_string(geo.K));
+    const int64_t out_rows = out_tm ? tokens : geo.M, out_cols = out_tm ? geo.M : tokens;
+    at::Tensor out = out0;
+    if (!out.defined()) {
+        out = at::empty({out_rows, out_cols}, val.options());
+    } else {
+        // the kernel writes out_rows rows of out_cols elements, ld_out apart: anything else would land outside `out`
+        if (out.scalar_type() != val.scalar_type() || out.device() != dev)
+            py_raise(PyExc_ValueError, std::string("out must be a ") + c10::toString(val.scalar_type()) + " tensor on " + dev.str());
+        if (out.dim() != 2 || out.size(0) != out_rows || out.size(1) != out_cols)
+            py_raise(PyExc_ValueError, "out must have shape (" + std::to_string(out_rows) + ", " + std::to_string(out_cols) + ") for this layout, got " + shape_str(out.sizes()));
+        if (out_cols > 1 && out.stride(1) != 1) py_raise(PyExc_ValueError, "out must have unit stride along its rows (a transposed view cannot be written in place)");
+        if (out_rows > 1 && out.stride(0) < out_cols) py_raise(PyExc_ValueError, "out rows overlap: the row stride is smaller than the row length");
+    }
+    Epi epi;
+    epi.act = (int)int_arg(a[13]);
+    if (residual.defined()) {
+        if (residual.scalar_type() != val.scalar_type() || residual.dim() != 2 || residual.size(0) != out_rows || residual.size(1) != out_cols ||
+            (out_cols > 1 && residual.stride(1) != 1))
+            py_raise(PyExc_ValueError, "residual must match the output's dtype and shape (" + std::to_string(out_rows) + ", " + std::to_string(out_cols) + "), with contiguous rows");
+        epi.residual = residual;
+        epi.ld = out_rows > 1 ? residual.stride(0) : out_cols;
+    }
+    if (tokens > 0) call_spmm(geo, code, dev, val, idx, packed, act, tokens, bias, epi, out, out_rows > 1 ? out.stride(0) : out_cols, layout, algo);
+    if (a[11] != Py_None) return Py_NewRef(a[11]);
+    return THPVariable_Wrap(out);
+    NMG_PY_END
+}
+
+// spmm_t(val, idx, M, K, n, m, g, dy, algo, packed, sp24, sp24_min_tokens) -> dx
+PyObject *py_spmm_t(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(12)
+    const at::Tensor &val = tensor_arg(a[0]), &idx = tensor_arg(a[1]), &dy0 = tensor_arg(a[7]);
+    const Geo geo = geo_args(a + 2);
+    const int algo = (int)int_arg(a[8]);
+    const at::Tensor packed = optional_tensor(a[9]), sp24 = optional_tensor(a[10]);
+    const c10::Device dev = device_of({&val, &idx, &dy0});
+    const int code = dtype_code(val);
+    if (dy0.scalar_type() != val.scalar_type())
+        py_raise(PyExc_TypeError, std::string("gradient dtype must match the weight dtype ") + c10::toString(val.scalar_type()));
+    const c10::cuda::CUDAGuard guard(dev);
+    const Rows dy = row_major_2d(dy0);
+    if (dy.cols != geo.M) py_raise(PyExc_ValueError, "gradient shape " + shape_str(dy0.sizes()) + " does not match M=" + std::to_string(geo.M));
+    const at::Tensor dx = at::empty({dy.rows, geo.K}, val.options());
+    const bool kept = sp24.defined() && dy.rows >= int_arg(a[11]) && (algo == NMG_ALGO_AUTO || algo == NMG_ALGO_TENSOR) && sp24_rows_ok(dy);
+    if (dy.rows > 0) call_spmm_t(geo, code, dev, val, idx, packed, kept ? sp24 : at::Tensor(), dy, dx, algo);
+    return THPVariable_Wrap(dx);
+    NMG_PY_END
+}
+
+// [B, M, K] operand of the conversions: unit stride along K, packed strides where a size-1 dim carries arbitrary ones.
+struct Dense3 {
+    at::Tensor t;
+    int64_t B, M, K, ld, bs;
+};
+Dense3 dense3_arg(const at::Tensor &t) {
+    if (t.dim() != 3) py_raise(PyExc_ValueError, "expected a 3-D tensor");
+    Dense3 d{t, t.size(0), t.size(1), t.size(2), 0, 0};
+    if (t.stride(2) != 1 || t.stride(1) < d.K || (d.B > 1 && t.stride(0) < d.M * t.stride(1))) d.t = t.contiguous();
+    const bool c = d.t.is_contiguous();
+    d.ld = c ? d.K : d.t.stride(1);
+    d.bs = c ? d.M * d.K : d.t.stride(0);
+    return d;
+}
+struct Tiles { int64_t C, cc, count; };
+Tiles tiles_of(int64_t B, int64_t M, int64_t K, int n, int m, int g) {
+    const int64_t C = nmg_num_patterns(n, m), cc = C * g;
+    if (C < 1 || cc < 1) py_raise(PyExc_ValueError, "need 0 <= n <= m and a positive group size");
+    return Tiles{C, cc, B * ((M + m - 1) / m) * ((K + cc - 1) / cc)};
+}
+
+// sparsify(dense3, n, m, g) -> (val, idx)
+PyObject *py_sparsify(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(4)
+    const at::Tensor &w = tensor_arg(a[0]);
+    const c10::Device dev = device_of({&w});
+    const int code = dtype_code(w), n = (int)int_arg(a[1]), m = (int)int_arg(a[2]), g = (int)int_arg(a[3]);
+    const c10::cuda::CUDAGuard guard(dev);
+    const Dense3 d = dense3_arg(w);
+    const Tiles t = tiles_of(d.B, d.M, d.K, n, m, g);
+    const at::Tensor val = at::empty({t.count, t.C, g, n}, w.options()), idx = at::empty({t.count, t.C, g, 1}, w.options().dtype(at::kShort));
+    void *st = stream_of(dev);
+    PyThreadState *save = PyEval_SaveThread();
+    const int rc = nmg_sparsify(d.t.const_data_ptr(), d.B, d.M, d.K, d.ld, d.bs, n, m, g, code, val.mutable_data_ptr(),
+                                static_cast<int16_t *>(idx.mutable_data_ptr()), st);
+    PyEval_RestoreThread(save);
+    check(rc);
+    PyObject *v = THPVariable_Wrap(val), *i = THPVariable_Wrap(idx);
+    PyObject *r = PyTuple_New(2);
+    PyTuple_SET_ITEM(r, 0, v);
+    PyTuple_SET_ITEM(r, 1, i);
+    return r;
+    NMG_PY_END
+}
+
+// gather(dense3, idx, n, m, g) -> val
+PyObject *py_gather(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(5)
+    const at::Tensor &w = tensor_arg(a[0]), &idx0 = tensor_arg(a[1]);
+    const c10::Device dev = device_of({&w, &idx0});
+    const int code = dtype_code(w), n = (int)int_arg(a[2]), m = (int)int_arg(a[3]), g = (int)int_arg(a[4]);
+    const c10::cuda::CUDAGuard guard(dev);
+    const Dense3 d = dense3_arg(w);
+    const Tiles t = tiles_of(d.B, d.M, d.K, n, m, g);
+    const at::Tensor idx = packed_rows(idx0);
+    if (idx.numel() != t.count * t.cc) py_raise(PyExc_ValueError, "idx does not belong to a layout of this shape");
+    const at::Tensor val = at::empty({t.count, t.C, g, n}, w.options());
+    void *st = stream_of(dev);
+    PyThreadState *save = PyEval_SaveThread();
+    const int rc = nmg_gather(d.t.const_data_ptr(), static_cast<const int16_t *>(idx.const_data_ptr()), d.B, d.M, d.K, d.ld, d.bs, n, m, g, code,
+                              val.mutable_data_ptr(), st);
+    PyEval_RestoreThread(save);
+    check(rc);
+    return THPVariable_Wrap(val);
+    NMG_PY_END
+}
+
+// densify(val, idx, B, M, K, n, m, g) -> dense3
+PyObject *py_densify(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(8)
+    const at::Tensor &val0 = tensor_arg(a[0]), &idx0 = tensor_arg(a[1]);
+    const c10::Device dev = device_of({&val0, &idx0});
+    const int code = dtype_code(val0);
+    const int64_t B = int_arg(a[2]);
+    const Geo geo = geo_args(a + 3);
+    const c10::cuda::CUDAGuard guard(dev);
+    const at::Tensor val = packed_rows(val0), idx = packed_rows(idx0);
+    const at::Tensor out = at::empty({B, geo.M, geo.K}, val.options());
+    void *st = stream_of(dev);
+    PyThreadState *save = PyEval_SaveThread();
+    const int rc = nmg_densify(val.const_data_ptr(), static_cast<const int16_t *>(idx.const_data_ptr()), B, geo.M, geo.K, geo.n, geo.m, geo.g, code,
+                               out.mutable_data_ptr(), geo.K, geo.M * geo.K, st);
+    PyEval_RestoreThread(save);
+    check(rc);
+    return THPVariable_Wrap(out);
+    NMG_PY_END
+}
+
+PyObject *py_set_error_class(PyObject *, PyObject *cls) {
+    Py_XSETREF(g_error_class, Py_NewRef(cls));
+    Py_RETURN_NONE;
+}
+
+// ------------------------------------------------------------------------------------------------ Handle
+// What the host keeps of one 2-D weight between calls: its geometry and, for the kernels that read them, the derived copies
+// together with the identity and version of the (val, idx) they were derived from.  The copies themselves belong to the
+// GroupedNMTensor (packed(), packed_sp24()), which is asked again as soon as either tensor has been replaced or written.
+struct Derived {
+    const void *val = nullptr, *idx = nullptr;
+    uint32_t val_version = 0, idx_version = 0;
+    bool valid = false;
+    at::Tensor copy;  // undefined: there is none for this weight
+};
+struct Handle {
+    PyObject_HEAD
+    Geo geo;
+    Derived *packed, *sp24;
+};
+
+at::Tensor attr_tensor(PyObject *o, PyObject *name) {
+    PyObject *v = PyObject_GetAttr(o, name);
+    if (!v) throw PyRaised();
+    if (!THPVariable_Check(v)) {
+        Py_DECREF(v);
+        py_raise(PyExc_TypeError, "val and idx must be tensors");
+    }
+    at::Tensor t = THPVariable_Unpack(v);
+    Py_DECREF(v);
+    return t;
+}
+
+const at::Tensor &derived(Derived &d, PyObject *gnm, PyObject *method, const at::Tensor &val, const at::Tensor &idx) {
+    const uint32_t vv = val.unsafeGetTensorImpl()->version_counter().enabled() ? val._version() : 0;
+    const uint32_t iv = idx.unsafeGetTensorImpl()->version_counter().enabled() ? idx._version() : 0;
+    const void *vp = val.const_data_ptr(), *ip = idx.const_data_ptr();
+    if (!d.valid || d.val != vp || d.idx != ip || d.val_version != vv || d.idx_version != iv) {
+        PyObject *r = PyObject_CallMethodNoArgs(gnm, method);
+        if (!r) throw PyRaised();
+        d.copy = r == Py_None || !THPVariable_Check(r) ? at::Tensor() : THPVariable_Unpack(r);
+        Py_DECREF(r);
+        d.val = vp; d.idx = ip; d.val_version = vv; d.idx_version = iv;
+        d.valid = true;
+    }
+    return d.copy;
+}
+
+PyObject *handle_new(PyTypeObject *type, PyObject *args, PyObject *) {
+    long long M, K;
+    int n, m, g;
+    if (!PyArg_ParseTuple(args, "LLiii", &M, &K, &n, &m, &g)) return nullptr;
+    Handle *h = reinterpret_cast<Handle *>(type->tp_alloc(type, 0));
+    if (!h) return nullptr;
+    h->geo = Geo{M, K, n, m, g};
+    h->packed = new Derived();
+    h->sp24 = new Derived();
+    return reinterpret_cast<PyObject *>(h);
+}
+void handle_dealloc(PyObject *self) {
+    Handle *h = reinterpret_cast<Handle *>(self);
+    delete h->packed;
+    delete h->sp24;
+    Py_TYPE(self)->tp_free(self);
+}
+
+// linear(gnm, x, bias, activation, residual): x [..., K] -> [..., M] = activation(x W^T + bias) + residual
+PyObject *handle_linear(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(5)
+    Handle *h = reinterpret_cast<Handle *>(self);
+    const Geo &geo = h->geo;
+    const at::Tensor val = attr_tensor(a[0], g_s_val), idx = attr_tensor(a[0], g_s_idx);
+    const at::Tensor &x = tensor_arg(a[1]);
+    const at::Tensor bias = optional_tensor(a[2]), residual = optional_tensor(a[4]);
+    const c10::Device dev = device_of({&val, &idx, &x, &bias, &residual});
+    const int code = dtype_code(val);
+    if (x.scalar_type() != val.scalar_type() || (bias.defined() && bias.scalar_type() != val.scalar_type()))
+        py_raise(PyExc_TypeError, std::string("activation / bias dtype must match the weight dtype ") + c10::toString(val.scalar_type()));
+    const c10::cuda::CUDAGuard guard(dev);
+    const Rows act = rows_of(x, geo.K);
+    c10::DimVector sizes(x.sizes().begin(), x.sizes().end());
+    sizes.back() = geo.M;
+    const at::Tensor out = at::empty(sizes, val.options());
+    Epi epi;
+    epi.act = (int)int_arg(a[3]);
+    if (residual.defined()) {
+        if (residual.scalar_type() != val.scalar_type() || residual.numel() != act.rows * geo.M || residual.dim() < 1 || residual.size(-1) != geo.M)
+            py_raise(PyExc_ValueError, "residual must match the output's dtype and shape, with contiguous rows");
+        const Rows r = rows_of(residual, geo.M);
+        epi.residual = r.t;
+        epi.ld = act.rows > 1 ? r.ld : geo.M;
+    }
+    if (act.rows > 0) {
+        const bool wants = nmg_spmm_uses_packed(geo.M, geo.K, act.rows, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 0) != 0;
+        call_spmm(geo, code, dev, val, idx, wants ? derived(*h->packed, a[0], g_s_packed, val, idx) : at::Tensor(), act, act.rows, bias, epi, out, geo.M,
+                  NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO);
+    }
+    return THPVariable_Wrap(out);
+    NMG_PY_END
+}
+
+// mm(gnm, b): b [K, tokens] -> [M, tokens] = W b
+PyObject *handle_mm(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(2)
+    Handle *h = reinterpret_cast<Handle *>(self);
+    const Geo &geo = h->geo;
+    const at::Tensor val = attr_tensor(a[0], g_s_val), idx = attr_tensor(a[0], g_s_idx);
+    const at::Tensor &b = tensor_arg(a[1]);
+    const c10::Device dev = device_of({&val, &idx, &b});
+    const int code = dtype_code(val);
+    if (b.scalar_type() != val.scalar_type())
+        py_raise(PyExc_TypeError, std::string("activation / bias dtype must match the weight dtype ") + c10::toString(val.scalar_type()));
+    const c10::cuda::CUDAGuard guard(dev);
+    const Rows act = row_major_2d(b);
+    if (act.rows != geo.K) py_raise(PyExc_ValueError, "activation shape " + shape_str(b.sizes()) + " does not match K=" + std::to_string(geo.K));
+    const at::Tensor out = at::empty({geo.M, act.cols}, val.options());
+    if (act.cols > 0) {
+        const bool wants = nmg_spmm_uses_packed(geo.M, geo.K, act.cols, geo.n, geo.m, geo.g, code, NMG_ACT_K_MAJOR, NMG_ALGO_AUTO, 0) != 0;
+        call_spmm(geo, code, dev, val, idx, wants ? derived(*h->packed, a[0], g_s_packed, val, idx) : at::Tensor(), act, act.cols, at::Tensor(), Epi(), out,
+                  act.cols, NMG_ACT_K_MAJOR, NMG_ALGO_AUTO);
+    }
+    return THPVariable_Wrap(out);
+    NMG_PY_END
+}
+
+// linear_t(gnm, dy, sp24_min_tokens): dy [..., M] -> [..., K] = dy W
+PyObject *handle_linear_t(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(3)
+    Handle *h = reinterpret_cast<Handle *>(self);
+    const Geo &geo = h->geo;
+    const at::Tensor val = attr_tensor(a[0], g_s_val), idx = attr_tensor(a[0], g_s_idx);
+    const at::Tensor &dy0 = tensor_arg(a[1]);
+    const c10::Device dev = device_of({&val, &idx, &dy0});
+    const int code = dtype_code(val);
+    if (dy0.scalar_type() != val.scalar_type())
+        py_raise(PyExc_TypeError, std::string("gradient dtype must match the weight dtype ") + c10::toString(val.scalar_type()));
+    const c10::cuda::CUDAGuard guard(dev);
+    const Rows dy = rows_of(dy0, geo.M);
+    c10::DimVector sizes(dy0.sizes().begin(), dy0.sizes().end());
+    sizes.back() = geo.K;
+    const at::Tensor dx = at::empty(sizes, val.options());
+    if (dy.rows > 0) {
+        at::Tensor sp24, packed;
+        // the compressed transposed copy serves the large batches of a 16-bit weight inside the 2:4 structure
+        if (dy.rows >= int_arg(a[2])) sp24 = derived(*h->sp24, a[0], g_s_packed_sp24, val, idx);
+        if (!sp24.defined() && nmg_spmm_uses_packed(geo.M, geo.K, dy.rows, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 1))
+            packed = derived(*h->packed, a[0], g_s_packed, val, idx);
+        call_spmm_t(geo, code, dev, val, idx, packed, sp24.defined() && sp24_rows_ok(dy) ? sp24 : at::Tensor(), dy, dx, NMG_ALGO_AUTO);
+    }
+    return THPVariable_Wrap(dx);
+    NMG_PY_END
+}
+
+#define NMG_METHOD(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
+PyMethodDef handle_methods[] = {
+    NMG_METHOD("linear", handle_linear),
+    NMG_METHOD("mm", handle_mm),
+    NMG_METHOD("linear_t", handle_linear_t),
+    {nullptr, nullptr, 0, nullptr},
+};
+PyTypeObject handle_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
+PyMethodDef module_methods[] = {
+    NMG_METHOD("spmm", py_spmm),
+    NMG_METHOD("spmm_t", py_spmm_t),
+    NMG_METHOD("sparsify", py_sparsify),
+    NMG_METHOD("gather", py_gather),
+    NMG_METHOD("densify", py_densify),
+    {"set_error_class", py_set_error_class, METH_O, nullptr},
+    {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "_nmg_host", "Host path of the grouped n:m kernels.", -1, module_methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__nmg_host(void) {
+    handle_type.tp_name = "sten_b200._nmg_host.Handle";
+    handle_type.tp_basicsize = sizeof(Handle);
+    handle_type.tp_flags = Py_TPFLAGS_DEFAULT;
+    handle_type.tp_doc = "Geometry and derived copies of one 2-D grouped n:m weight.";
+    handle_type.tp_new = handle_new;
+    handle_type.tp_dealloc = handle_dealloc;
+    handle_type.tp_methods = handle_methods;
+    if (PyType_Ready(&handle_type) < 0) return nullptr;
+    g_s_val = PyUnicode_InternFromString("val");
+    g_s_idx = PyUnicode_InternFromString("idx");
+    g_s_packed = PyUnicode_InternFromString("packed");
+    g_s_packed_sp24 = PyUnicode_InternFromString("packed_sp24");
+    PyObject *mod = PyModule_Create(&module_def);
+    if (!mod) return nullptr;
+    if (PyModule_AddObjectRef(mod, "Handle", reinterpret_cast<PyObject *>(&handle_type)) < 0) {
+        Py_DECREF(mod);
+        return nullptr;
+    }
+    return mod;
+}

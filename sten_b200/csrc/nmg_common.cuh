@@ -8,6 +8,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/nmg_b200.h"
 
 namespace nmg {
@@ -90,6 +92,24 @@ ProfileEvents take_profile_events();
 bool tc_expand_plain_supported(const Geo &geo, int dtype, const void *dense, int64_t ld);
 int tc_expand_plain(const Geo &geo, int dtype, const void *val, const int16_t *idx, void *dense, int64_t ld, cudaStream_t st);
 int get_status_word(int **dev_ptr);
+int device_sms(int *sms_out);  // SM count of the current device, queried once per device
+constexpr int kMaxDevices = 64;
+// Raise a kernel's dynamic shared-memory limit on the current device; the runtime call (about 0.5 us) is made only when a
+// launch needs more than any launch of that kernel on that device before it.
+template <auto Kernel> inline int allow_smem(size_t bytes) {
+    static std::atomic<int> have[kMaxDevices];
+    int dev = 0;
+    NMG_CUDA(cudaGetDevice(&dev));
+    if (dev >= kMaxDevices || have[dev].load(std::memory_order_relaxed) < (int)bytes) {
+        NMG_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        if (dev < kMaxDevices) have[dev].store((int)bytes, std::memory_order_relaxed);
+    }
+    return NMG_OK;
+}
+#define NMG_ALLOW_SMEM(bytes, ...)                                              \
+    do {                                                                        \
+        if (const int rc__ = ::nmg::allow_smem<__VA_ARGS__>(bytes)) return rc__; \
+    } while (0)
 int get_wave_counter(unsigned **dev_ptr);  // one of a few rotating 4-byte counters of the current device (spare bytes of the status block)
 // Status word of nmg_spmm_noalloc on device `dev` (start of the built-in scratch array), or NULL before its first call there.
 int *noalloc_status_word(int dev);

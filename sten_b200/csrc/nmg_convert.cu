@@ -642,9 +642,8 @@ __global__ void __launch_bounds__(256) gather_layout_kernel(GatherParams prm) {
 }
 
 static int sm_count() {
-    int dev = 0, sms = 148;
-    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms > 0 ? sms : 148;
+    int sms = 148;
+    return device_sms(&sms) == NMG_OK ? sms : 148;
 }
 
 static int check_dtype(int dtype) {
@@ -704,7 +703,7 @@ extern "C" int nmg_sparsify(const void *dense, int64_t batch, int64_t M, int64_t
 #define NMG_SPARSIFY_CASE(N_, M_)                                                                                     \
     if (!launched && n == N_ && m == M_) {                                                                            \
         NMG_DISPATCH_DTYPE(dtype, T, {                                                                                \
-            NMG_CUDA(cudaFuncSetAttribute(sparsify_nm_kernel<N_, M_, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+            NMG_ALLOW_SMEM(smem, sparsify_nm_kernel<N_, M_, T>); \
             sparsify_nm_kernel<N_, M_, T><<<(unsigned)ctas, warps * 32, smem, st>>>(p);                               \
         });                                                                                                           \
         launched = true;                                                                                              \
@@ -717,7 +716,7 @@ extern "C" int nmg_sparsify(const void *dense, int64_t batch, int64_t M, int64_t
 #undef NMG_SPARSIFY_CASE
     if (!launched) {
         NMG_DISPATCH_DTYPE(dtype, T, {
-            NMG_CUDA(cudaFuncSetAttribute(sparsify_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            NMG_ALLOW_SMEM(smem, sparsify_kernel<T>);
             sparsify_kernel<T><<<(unsigned)ctas, warps * 32, smem, st>>>(p);
         });
     }
@@ -763,7 +762,7 @@ extern "C" int nmg_densify(const void *val, const int16_t *idx, int64_t batch, i
     const int64_t max_ctas = (int64_t)sm_count() * 32;
     if (ctas > max_ctas) ctas = max_ctas;
     NMG_DISPATCH_DTYPE(dtype, T, {
-        NMG_CUDA(cudaFuncSetAttribute(densify_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        NMG_ALLOW_SMEM(smem, densify_kernel<T>);
         densify_kernel<T><<<(unsigned)ctas, 128, smem, st>>>(p);
     });
     NMG_CUDA(cudaGetLastError());

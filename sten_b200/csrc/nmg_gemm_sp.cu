@@ -380,11 +380,10 @@ static SpLayout sp_layout(const Geo &geo) {
 }
 
 template <typename T, int N_> static int sp_expand_launch(const SpExpandParams &p, size_t smem, int64_t items, cudaStream_t st) {
-    int dev = 0, sms = 148;
-    NMG_CUDA(cudaGetDevice(&dev));
-    NMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms = 148, rc_sms;
+    if ((rc_sms = device_sms(&sms))) return rc_sms;
     const int64_t cap = (int64_t)sms * 16;
-    NMG_CUDA(cudaFuncSetAttribute(expand_sp_kernel<T, N_>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NMG_ALLOW_SMEM(smem, expand_sp_kernel<T, N_>);
     expand_sp_kernel<T, N_><<<(unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st>>>(p);
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;
@@ -392,12 +391,11 @@ template <typename T, int N_> static int sp_expand_launch(const SpExpandParams &
 
 template <typename T> static int sp_gemm_launch(const SpGemmParams &p, const SpGemmMaps &maps, cudaStream_t st) {
     const size_t smem = (size_t)SP_STAGES * SP_STAGE + SP_STAGING_BYTES + 256 + 1024;
-    int dev = 0, sms = 148;
-    NMG_CUDA(cudaGetDevice(&dev));
-    NMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms = 148, rc_sms;
+    if ((rc_sms = device_sms(&sms))) return rc_sms;
     const int64_t tiles = (int64_t)p.tiles_f * p.tiles_t;
     if (tiles > 0x3fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many output tiles for one launch");
-    NMG_CUDA(cudaFuncSetAttribute(gemm_sp_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NMG_ALLOW_SMEM(smem, gemm_sp_kernel<T>);
     cudaLaunchConfig_t cfg = {};
     const int64_t pairs = sms / 2;
     cfg.gridDim = dim3((unsigned)(2 * (tiles < pairs ? tiles : pairs)));  // persistent CTA pairs
@@ -481,9 +479,8 @@ int tc_sp_matmul_t(const Geo &geo, int dtype, const void *sp_copy, const void *d
     gp.band = TC_BAND_PAIR;
     {
         // many waves over a long reduction: keep the producers in step; the counter is zeroed in stream order
-        int dev = 0, sms = 148;
-        NMG_CUDA(cudaGetDevice(&dev));
-        NMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        int sms = 148, rc_sms;
+        if ((rc_sms = device_sms(&sms))) return rc_sms;
         if ((int64_t)gp.tiles_f * gp.tiles_t >= 3 * (int64_t)(sms / 2) && geo.M >= 4096) {
             if ((rc = get_wave_counter(&gp.wave_ctr))) return rc;
             NMG_CUDA(cudaMemsetAsync(gp.wave_ctr, 0, sizeof(unsigned), st));

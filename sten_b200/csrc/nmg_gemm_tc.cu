@@ -700,11 +700,10 @@ size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed) {
 }
 
 template <typename T, bool TR, int N_, bool PLAIN> static int expand_launch_n(const ExpandParams &p, size_t smem, int64_t items, cudaStream_t st) {
-    int dev = 0, sms = 148;
-    NMG_CUDA(cudaGetDevice(&dev));
-    NMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms = 148, rc_sms;
+    if ((rc_sms = device_sms(&sms))) return rc_sms;
     const int64_t cap = (int64_t)sms * 16;
-    NMG_CUDA(cudaFuncSetAttribute(expand_dense_kernel<T, TR, N_, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NMG_ALLOW_SMEM(smem, expand_dense_kernel<T, TR, N_, PLAIN>);
     expand_dense_kernel<T, TR, N_, PLAIN><<<(unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st>>>(p);
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;
@@ -719,12 +718,11 @@ template <typename T, bool TR, bool PLAIN = false> static int expand_launch(cons
 
 template <typename T, bool PAIR, bool TMA_OUT> static int gemm_launch_as(const GemmParams &p, const GemmMaps &maps, cudaStream_t st) {
     const size_t smem = (size_t)GEMM_RING_BYTES + GEMM_STAGING_BYTES + 256 + 1024;
-    int dev = 0, sms = 148;
-    NMG_CUDA(cudaGetDevice(&dev));
-    NMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    int sms = 148, rc_sms;
+    if ((rc_sms = device_sms(&sms))) return rc_sms;
     const int64_t tiles = (int64_t)p.tiles_f * p.tiles_t;
     if (tiles > 0x3fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many output tiles for one launch");
-    NMG_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<T, PAIR, TMA_OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NMG_ALLOW_SMEM(smem, gemm_tc_kernel<T, PAIR, TMA_OUT>);
     cudaLaunchConfig_t cfg = {};
     const int64_t units = PAIR ? sms / 2 : sms;  // persistent CTAs, or CTA pairs
     cfg.gridDim = dim3((unsigned)((tiles < units ? tiles : units) * (PAIR ? 2 : 1)));
@@ -855,9 +853,8 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, bool pair, const char *d
     gp.band = pair ? TC_BAND_PAIR : TC_BAND;
     {
         // many waves over a long reduction: keep the producers in step (see the kernel); the counter is zeroed in stream order
-        int dev = 0, sms = 148;
-        NMG_CUDA(cudaGetDevice(&dev));
-        NMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        int sms = 148, rc_sms;
+        if ((rc_sms = device_sms(&sms))) return rc_sms;
         const int64_t units = pair ? sms / 2 : sms;
         if ((int64_t)gp.tiles_f * gp.tiles_t >= 3 * units && red >= 4096) {
             if ((rc = get_wave_counter(&gp.wave_ctr))) return rc;

@@ -30,7 +30,6 @@ namespace nmg {
 // with cudaGetSymbolAddress, once per device, below.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[NMG_NOALLOC_SCRATCH_BYTES];
 
-constexpr int kMaxDevices = 64;
 static std::mutex g_noalloc_mu;
 static unsigned char *g_noalloc_ptr[kMaxDevices] = {};
 

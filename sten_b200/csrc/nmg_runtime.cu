@@ -54,10 +54,16 @@ static std::map<int, int *> g_status;
 int get_pattern_table(int n, int m, PatternTable *out) {
     int dev = 0;
     NMG_CUDA(cudaGetDevice(&dev));
+    static thread_local struct { int dev = -1, n = -1, m = -1; PatternTable tab; } last;  // the table this thread used last
+    if (last.dev == dev && last.n == n && last.m == m) { *out = last.tab; return NMG_OK; }
     std::lock_guard<std::mutex> lk(g_mu);
     auto key = std::make_tuple(dev, n, m);
     auto it = g_tables.find(key);
-    if (it != g_tables.end()) { *out = it->second; return NMG_OK; }
+    if (it != g_tables.end()) {
+        *out = last.tab = it->second;
+        last.dev = dev; last.n = n; last.m = m;
+        return NMG_OK;
+    }
     int C = (int)comb(n, m);
     int nn = n > 0 ? n : 1;
     std::vector<int8_t> host((size_t)C * nn + (size_t)C * m, (int8_t)-1);
@@ -75,8 +81,11 @@ int get_pattern_table(int n, int m, PatternTable *out) {
 }
 
 int get_status_word(int **dev_ptr) {
+    // every launch asks for it: after the first call on a device the answer is one load
+    static std::atomic<int *> ready[kMaxDevices];
     int dev = 0;
     NMG_CUDA(cudaGetDevice(&dev));
+    if (dev < kMaxDevices && (*dev_ptr = ready[dev].load(std::memory_order_acquire))) return NMG_OK;
     std::lock_guard<std::mutex> lk(g_mu);
     auto it = g_status.find(dev);
     if (it == g_status.end()) {
@@ -86,6 +95,20 @@ int get_status_word(int **dev_ptr) {
         it = g_status.emplace(dev, p).first;
     }
     *dev_ptr = it->second;
+    if (dev < kMaxDevices) ready[dev].store(it->second, std::memory_order_release);
+    return NMG_OK;
+}
+
+int device_sms(int *sms_out) {
+    static std::atomic<int> known[kMaxDevices];
+    int dev = 0;
+    NMG_CUDA(cudaGetDevice(&dev));
+    int sms = dev < kMaxDevices ? known[dev].load(std::memory_order_relaxed) : 0;
+    if (sms == 0) {
+        NMG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        if (dev < kMaxDevices) known[dev].store(sms, std::memory_order_relaxed);
+    }
+    *sms_out = sms;
     return NMG_OK;
 }
 
@@ -139,9 +162,17 @@ int encode_tmap_2d(CUtensorMap *map, int dtype, const void *base, uint64_t cols,
     cuuint64_t strides[1] = {ld_elems * es};
     cuuint32_t box[2] = {box_cols, box_rows};
     cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, dt, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    swizzle_128b ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
-                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    auto encode = [&] {
+        return fn(map, dt, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  swizzle_128b ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+        // a thread that has made no runtime call yet (an autograd worker in its first backward): bind the primary context
+        NMG_CUDA(cudaFree(nullptr));
+        r = encode();
+    }
     if (r != CUDA_SUCCESS) NMG_FAIL(NMG_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
     return NMG_OK;
 }

@@ -159,10 +159,10 @@ int launch_fwd(const FwdParams &p, const CUtensorMap &tm, int rbc, size_t smem, 
     dim3 grid((unsigned)((tokens + 32 * TT - 1) / (32 * TT)), (unsigned)((p.nb + rbc - 1) / rbc));
     if (grid.y > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "weight has too many row-blocks for one launch");
     if (token_major) {
-        NMG_CUDA(cudaFuncSetAttribute(spmm_fwd_simt_kernel<N_, M_, TT, T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        NMG_ALLOW_SMEM(smem, spmm_fwd_simt_kernel<N_, M_, TT, T, true>);
         spmm_fwd_simt_kernel<N_, M_, TT, T, true><<<grid, kWarps * 32, smem, st>>>(p, tm);
     } else {
-        NMG_CUDA(cudaFuncSetAttribute(spmm_fwd_simt_kernel<N_, M_, TT, T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        NMG_ALLOW_SMEM(smem, spmm_fwd_simt_kernel<N_, M_, TT, T, false>);
         spmm_fwd_simt_kernel<N_, M_, TT, T, false><<<grid, kWarps * 32, smem, st>>>(p, tm);
     }
     NMG_CUDA(cudaGetLastError());

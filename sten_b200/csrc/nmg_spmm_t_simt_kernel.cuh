@@ -139,7 +139,7 @@ int launch_bwd(const BwdParams &p, const CUtensorMap &tm, int64_t tokens, cudaSt
     const size_t smem = bwd_smem_plan(M_, N_, p.rb_stage, sizeof(T)).total;
     dim3 grid((unsigned)((tokens + kBwdTok - 1) / kBwdTok), (unsigned)((p.K + kColsCta - 1) / kColsCta));
     if (grid.y > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "weight has too many columns for one launch");
-    NMG_CUDA(cudaFuncSetAttribute(spmm_bwd_simt_kernel<N_, M_, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NMG_ALLOW_SMEM(smem, spmm_bwd_simt_kernel<N_, M_, T>);
     spmm_bwd_simt_kernel<N_, M_, T><<<grid, kBwdWarps * 32, smem, st>>>(p, tm);
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;

@@ -587,7 +587,7 @@ static int tc_launch_one(const TcParams &p, const CUtensorMap *tm, cudaStream_t 
     const int64_t ctas = (int64_t)p.tiles_f * p.tiles_t * p.ksplit;
     if (ctas > 0x7fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many output tiles for one launch");
     dim3 grid((unsigned)ctas);
-    NMG_CUDA(cudaFuncSetAttribute(spmm_tc_kernel<N_, M_, T, TR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NMG_ALLOW_SMEM(smem, spmm_tc_kernel<N_, M_, T, TR>);
     spmm_tc_kernel<N_, M_, T, TR><<<grid, TC_THREADS, smem, st>>>(p, tm[0], tm[1], tm[2]);
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;

@@ -329,6 +329,20 @@ def implements(*torch_functions):
     return decorator
 
 
+_ZERO_DUMMIES = {}
+
+
+def _zero_dummy(dtype, device):
+    """One-element zero for a gradient's wrapper.  All of them share one storage per (dtype, device): autograd only ever adds
+    such zeros to each other, and a gradient that is wrapped on every step should not cost an allocation and a fill.  ``.data``
+    gives each its own version counter, so that accumulating into one does not look like a write to another."""
+    key = (dtype, device)
+    zero = _ZERO_DUMMIES.get(key)
+    if zero is None:
+        zero = _ZERO_DUMMIES[key] = torch.zeros([1], dtype=dtype, device=device)
+    return zero.data
+
+
 class SparseTensorWrapper(torch.Tensor):
     """A tensor whose payload is ``self.wrapped_tensor`` (any object with ``to_dense()``).
 
@@ -340,15 +354,16 @@ class SparseTensorWrapper(torch.Tensor):
     def wrapped_from_dense(wrapped, dense, grad_fmt=None):
         return SparseTensorWrapper([wrapped], dense.requires_grad, grad_fmt if grad_fmt is not None else _DEFAULT_GRAD_FMT())
 
-    def __new__(cls, wrapped_tensor_container, requires_grad, grad_fmt, *, dummy_shape=None):
+    def __new__(cls, wrapped_tensor_container, requires_grad, grad_fmt, *, dummy_shape=None, shared_dummy=False):
         payload = wrapped_tensor_container[0]
         assert not isinstance(payload, SparseTensorWrapper)
         meta = payload if hasattr(payload, "dtype") and hasattr(payload, "device") else payload.to_dense()
-        dummy = torch.zeros([1], dtype=meta.dtype, device=meta.device)
+        dummy = _zero_dummy(meta.dtype, meta.device) if shared_dummy else torch.zeros([1], dtype=meta.dtype, device=meta.device)
         self = torch.Tensor._make_subclass(cls, dummy, requires_grad)
         self._wrapped_tensor_container = wrapped_tensor_container
         self.grad_fmt = grad_fmt
-        self.update_grad_fix_hook()
+        if requires_grad:
+            self.grad_fix_hook_handle = self.register_hook(self.grad_fix_hook)
         return self
 
     # autograd hands back gradients as plain views of the subclass; keep the wrapper in .grad
@@ -406,6 +421,10 @@ class SparseTensorWrapper(torch.Tensor):
 
     @classmethod
     def __torch_function__(cls, func, types, args=(), kwargs=None):
+        if not kwargs:
+            out = _repeat_call(func, args)
+            if out is not NotImplemented:
+                return out
         kwargs = kwargs or {}
         handler = HANDLED_FUNCTIONS.get(func)
         if handler is not None:
@@ -429,8 +448,26 @@ class SparseParameterWrapper(SparseTensorWrapper, torch.nn.parameter.Parameter):
 
     @classmethod
     def __torch_function__(cls, func, types, args=(), kwargs=None):
+        if not kwargs:
+            out = _repeat_call(func, args)
+            if out is not NotImplemented:
+                return out
         base = tuple(SparseTensorWrapper if t is SparseParameterWrapper else t for t in types)
         return SparseTensorWrapper.__torch_function__(func, base, args, kwargs or {})
+
+
+def _repeat_call(func, args):
+    """The result of a call whose operator has been resolved on one of its sparse operands before, else NotImplemented (then
+    the general route below decides).  Only operators that went through the fall-back are kept there, so an overridden torch
+    function never lands here."""
+    for a in args:
+        if isinstance(a, SparseTensorWrapper):
+            ops = a.__dict__.get("sparsified_ops")
+            if ops is not None:
+                op = ops.get(func)
+                if op is not None:
+                    return op.sparse_op.repeat(args)
+    return NotImplemented
 
 
 def sparse_tensor_builder(wrapper_type, wrapped_tensor_container, requires_grad, grad_fmt):
@@ -784,6 +821,8 @@ def _run_forward(ctx, st, flat_inputs):
         _resolve_forward(st, flat_inputs)
     sp1, fmt1, sp2, fmt2 = st["out_fmt4"]
     tmp = st["op_impl_fwd"](ctx, flat_inputs, sp1)
+    if not first and type(tmp) is torch.Tensor and len(st["fwd_sp_impls"]) == 1:  # one dense output: nothing to flatten
+        return st["fwd_sp_impls"][0](st["fwd_out_fmt_sp_fmt"][1][0], tmp)
     out_stubs, flat_out = flatten_list_of_tensors_in_args(tmp)
     if first:
         _check_formats(f"{st['orig_op']} (fwd)", flat_out, fmt1)
@@ -842,7 +881,7 @@ class SparseOperatorDispatcher(torch.autograd.Function):
                 continue
             g = impl(s, g)
             if isinstance(g, SparseTensorWrapper):  # gradient wrapper must look like the input's dummy
-                g = SparseTensorWrapper(g._wrapped_tensor_container, g.requires_grad, g.grad_fmt, dummy_shape=shape)
+                g = SparseTensorWrapper(g._wrapped_tensor_container, torch.is_grad_enabled() and g.requires_grad, g.grad_fmt, dummy_shape=shape, shared_dummy=True)
             grads.append(g)
         return (None, *grads)
 
@@ -855,22 +894,27 @@ class SparseOp:
     def clear_disp_state(self):
         self.disp_state = {"orig_op": self.orig_op, "out_fmt": self.out_fmt, "grad_out_fmt": self.grad_out_fmt}
 
-    def _run_fast(self, args):
-        """Repeat of a call this op has already resolved: positional tensors only, same formats, nothing needs a
-        gradient, a registered (not fallback) implementation and one dense output.  Skips flattening and signature
-        binding, which dominate the host time of a sparse ``F.linear`` in inference."""
+    def repeat(self, args):
+        """Repeat of a call this op has already resolved: positional tensors only, same types and formats, a registered (not
+        fallback) implementation and one dense output; NotImplemented otherwise.  Skips flattening and signature binding,
+        which dominate the host time of a sparse ``F.linear``."""
         st = self.disp_state
         fast = st.get("fast")
         if fast is None or len(args) != len(fast):
-            return None
-        for a, fmt in zip(args, fast):
-            if not isinstance(a, torch.Tensor) or get_format(a) != fmt:
-                return None
-        if torch.is_grad_enabled() and any(a.requires_grad for a in args):
-            return None
+            return NotImplemented
+        for a, (cls, fmt) in zip(args, fast):
+            if type(a) is not cls or (fmt is not None and a._wrapped_tensor_container[0].__class__ is not fmt):
+                return NotImplemented
+        if CUDA_PROFILING[0]:
+            return NotImplemented
+        if torch.is_grad_enabled():
+            with torch._C.DisableTorchFunctionSubclass():
+                need_grad = any(a.requires_grad for a in args)
+            if need_grad:
+                return SparseOperatorDispatcher.apply(st, *args)
         tmp = st["op_impl_fwd"](_NoGradCtx(st), args, st["out_fmt4"][0])
         if type(tmp) is not torch.Tensor:
-            return None if tmp is None else self._finish_slow_output(tmp)
+            return self._finish_slow_output(tmp)
         return st["fwd_sp_impls"][0](st["fwd_out_fmt_sp_fmt"][1][0], tmp)
 
     def _finish_slow_output(self, tmp):
@@ -882,10 +926,6 @@ class SparseOp:
         return unflatten_list_of_tensors_in_args(out_stubs, outs)
 
     def run(self, *args, **kwargs):
-        if not kwargs and "fast" in self.disp_state:
-            out = self._run_fast(args)
-            if out is not None:
-                return out
         call_stubs, flat_call = flatten_list_of_tensors_in_args((tuple(args), dict(kwargs)))
         bound, _ = bind_func_signature(self.orig_op, args, kwargs)
         flat, order = flat_call, list(range(len(flat_call)))
@@ -909,9 +949,10 @@ class SparseOp:
             outputs = SparseOperatorDispatcher.apply(st, *flat)
         else:
             outputs = _run_forward(_NoGradCtx(st), st, tuple(flat))
-        if (not need_grad and not kwargs and type(outputs) is torch.Tensor and not st.get("fwd_impl_fallback")
+        if (not kwargs and type(outputs) is torch.Tensor and not st.get("fwd_impl_fallback")
                 and len(flat) == len(args) and all(a is b for a, b in zip(flat, args)) and len(st.get("fwd_sp_impls", ())) == 1):
-            st["fast"] = tuple(get_format(t) for t in flat)  # next identical call takes _run_fast
+            # the next call with operands of these types and formats takes repeat()
+            st["fast"] = tuple((type(t), t.wrapped_tensor.__class__ if isinstance(t, SparseTensorWrapper) else None) for t in flat)
         out_tuple = outputs if isinstance(outputs, (tuple, list)) else (outputs,)
         grad_fmts = _exact_formats(st["grad_out_fmt"], out_tuple)
         for o, gf in zip(out_tuple, grad_fmts):

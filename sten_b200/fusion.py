@@ -15,7 +15,6 @@ import types
 
 import torch
 
-from . import _native as nat
 from . import ops
 from .dispatch import SparseTensorWrapper
 from .grouped_nm_tensor import GroupedNMTensor
@@ -32,20 +31,18 @@ def _nmg_weight(linear):
 
 def sparse_linear_fused(x, gnm, bias=None, activation=None, residual=None):
     """``activation(x W^T + bias) + residual`` for a grouped n:m weight in one library call (no autograd)."""
-    s = gnm.nm_strides
-    M, K = (int(v) for v in s["dense_shape"])
-    n, m, g = s["n"], s["m"], s["group_size"]
-    x2d = x.reshape(-1, K)
-    tokens = x2d.shape[0]
-    res2d = residual.reshape(-1, M) if residual is not None else None
-    from .nmg_impls import _wants_expanded
-    if x2d.stride(-1) != 1:
-        x2d = x2d.contiguous()
-    if _wants_expanded(gnm, x2d, tokens):
-        return ops.spmm_expanded(gnm.expanded(), M, K, x2d, bias=bias, activation=activation, residual=res2d).reshape(*x.shape[:-1], M)
-    packed = gnm.packed() if tokens and ops.uses_packed(M, K, tokens, n, m, g, gnm.val.dtype, nat.NMG_ACT_TOKEN_MAJOR) else None
-    y = ops.spmm(gnm.val, gnm.idx, M, K, n, m, g, x2d, bias=bias, packed=packed, activation=activation, residual=res2d)
-    return y.reshape(*x.shape[:-1], M)
+    if activation not in ops._ACTIVATIONS:
+        raise ValueError("activation must be None or 'gelu'")
+    if gnm.nm_strides.get("kernel") == "sm100-expanded":
+        from .nmg_impls import _wants_expanded
+        M, K = (int(v) for v in gnm.nm_strides["dense_shape"])
+        x2d = x.reshape(-1, K)
+        if x2d.stride(-1) != 1:
+            x2d = x2d.contiguous()
+        if _wants_expanded(gnm, x2d, x2d.shape[0]):
+            res2d = residual.reshape(-1, M) if residual is not None else None
+            return ops.spmm_expanded(gnm.expanded(), M, K, x2d, bias=bias, activation=activation, residual=res2d).reshape(*x.shape[:-1], M)
+    return gnm.native().linear(gnm, x, bias, ops._ACTIVATIONS[activation], residual)
 
 
 def _is_exact_gelu(fn):

@@ -10,6 +10,7 @@ import math
 
 import torch
 
+from . import _native as nat
 from . import ops
 from .layout import compute_nm_strides, make_n_m  # noqa: F401  (re-exported like the reference module does)
 
@@ -118,6 +119,18 @@ class GroupedNMTensor:
     @property
     def shape(self):
         return torch.Size(self.nm_strides["dense_shape"])
+
+    def native(self):
+        """Host-side handle of a 2-D weight with n:m blocks along dim 0 and groups along dim 1 (its geometry and the derived
+        copies its kernels read), or None for any other layout.  Built on first use; never pickled or copied."""
+        h = self.__dict__.get("_native")
+        if h is None:
+            s = self.nm_strides
+            if len(s["dense_shape"]) != 2 or s["sparse_dim"] != 0 or s["group_dim"] != 1:
+                return None
+            M, K = s["dense_shape"]
+            h = self.__dict__["_native"] = nat.host().Handle(int(M), int(K), s["n"], s["m"], s["group_size"])
+        return h
 
     def packed(self):
         """Column-ordered device copy used by the tensor-core and transposed kernels (``nmg_pack``).

@@ -58,56 +58,50 @@ def dense_to_same_grouped_nm(sparsifier, tensor, grad_fmt=None):
     return sten.SparseTensorWrapper.wrapped_from_dense(gnm, tensor, grad_fmt if grad_fmt is not None else ref.grad_fmt)
 
 
-def _weight_geometry(weight):
-    gnm = weight.wrapped_tensor
-    s = gnm.nm_strides
-    if len(s["dense_shape"]) != 2 or s["sparse_dim"] != 0 or s["group_dim"] != 1:
-        raise sten.DispatchError("grouped n:m matmul needs a 2-D weight with n:m blocks along dim 0 and groups along dim 1")
-    M, K = s["dense_shape"]
-    return gnm, int(M), int(K), s["n"], s["m"], s["group_size"]
-
-
-def _packed_or_none(gnm, geometry, tokens, layout=nat.NMG_ACT_TOKEN_MAJOR, transposed=False):
-    """The cached column-ordered copy when the kernel that will run reads it, else None (nothing is built)."""
-    M, K, n, m, g = geometry
-    if not gnm.val.is_cuda or not ops.uses_packed(M, K, tokens, n, m, g, gnm.val.dtype, layout, transposed=transposed):
-        return None
-    return gnm.packed()
-
-
-def _sp24_or_none(gnm, tokens):
-    """The cached compressed transposed copy when the backward product of this many tokens runs on the structured-sparse
-    tensor cores (16-bit weight inside the 2:4 structure), else None (nothing is built)."""
-    return gnm.packed_sp24() if tokens >= ops.SP24_MIN_TOKENS else None
-
-
-def _wants_expanded(gnm, x2d, tokens, layout=nat.NMG_ACT_TOKEN_MAJOR):
+def _wants_expanded(gnm, x2d, tokens):
     """The opt-in of ``set_spmm_opt(kernel="sm100-expanded")`` applies: 16-bit weight, token-major activation whose rows TMA
     can read, and a batch large enough for the two-pass regime (fewer tokens stay on the compressed-weight kernel)."""
-    return (gnm.nm_strides.get("kernel") == "sm100-expanded" and layout == nat.NMG_ACT_TOKEN_MAJOR and tokens >= ops.SP24_MIN_TOKENS
+    return (gnm.nm_strides.get("kernel") == "sm100-expanded" and tokens >= ops.SP24_MIN_TOKENS
             and gnm.val.dtype != torch.float32 and x2d.stride(-1) == 1 and x2d.data_ptr() % 16 == 0 and x2d.stride(0) % 8 == 0
             and gnm.expanded() is not None)
 
 
+def _native_weight(weight):
+    """(GroupedNMTensor, its host-side handle) of a weight the matmul kernels can serve."""
+    gnm = weight.wrapped_tensor
+    h = gnm.native()
+    if h is None:
+        raise sten.DispatchError("grouped n:m matmul needs a 2-D weight with n:m blocks along dim 0 and groups along dim 1")
+    return gnm, h
+
+
 def sparse_dense_mul_dispatch(weight, dense2d, bias, layout):
     """One C-ABI call; replaces the compile-or-load + ctypes call of the reference (sten_impls.py:44-140)."""
-    gnm, M, K, n, m, g = _weight_geometry(weight)
-    tokens = dense2d.shape[1] if layout == nat.NMG_ACT_K_MAJOR else dense2d.shape[0]
-    if _wants_expanded(gnm, dense2d, tokens, layout):
+    gnm, h = _native_weight(weight)
+    if layout == nat.NMG_ACT_K_MAJOR and bias is None:
+        return h.mm(gnm, dense2d)
+    if layout != nat.NMG_ACT_TOKEN_MAJOR:
+        s = gnm.nm_strides
+        M, K = s["dense_shape"]
+        return ops.spmm(gnm.val, gnm.idx, M, K, s["n"], s["m"], s["group_size"], dense2d, bias=bias, layout=layout)
+    if gnm.nm_strides.get("kernel") == "sm100-expanded" and _wants_expanded(gnm, dense2d, dense2d.shape[0]):
+        M, K = gnm.nm_strides["dense_shape"]
         return ops.spmm_expanded(gnm.expanded(), M, K, dense2d, bias=bias)
-    packed = _packed_or_none(gnm, (M, K, n, m, g), tokens, layout) if tokens else None
-    return ops.spmm(gnm.val, gnm.idx, M, K, n, m, g, dense2d, bias=bias, layout=layout, packed=packed)
+    return h.linear(gnm, dense2d, bias, nat.NMG_EPI_NONE, None)
 
 
 def _linear_fwd(ctx, inputs, output_sparsifiers):
     if len(inputs) == 3:
         x, weight, bias = inputs
+        ctx.save_for_backward(x, weight, bias)
     else:
         (x, weight), bias = inputs, None
-    ctx.save_for_backward(x, weight, bias) if bias is not None else ctx.save_for_backward(x, weight)
-    x2d = x.reshape(-1, x.shape[-1])
-    y = sparse_dense_mul_dispatch(weight, x2d, bias, nat.NMG_ACT_TOKEN_MAJOR)
-    return y.reshape(*x.shape[:-1], y.shape[-1])
+        ctx.save_for_backward(x, weight)
+    gnm, h = _native_weight(weight)
+    if gnm.nm_strides.get("kernel") == "sm100-expanded":
+        y = sparse_dense_mul_dispatch(weight, x.reshape(-1, x.shape[-1]), bias, nat.NMG_ACT_TOKEN_MAJOR)
+        return y.reshape(*x.shape[:-1], y.shape[-1])
+    return h.linear(gnm, x, bias, nat.NMG_EPI_NONE, None)
 
 
 _LIN_OUT = [(sten.KeepAll, torch.Tensor)]
@@ -122,16 +116,15 @@ def _linear_bwd(ctx, grad_outputs, input_sparsifiers):
     has_bias = len(saved) == 3
     [dy] = grad_outputs
     needs = tuple(ctx.needs_input_grad[1:]) + (False,) * 3
-    gnm, M, K, n, m, g = _weight_geometry(weight)
-    dy2d = dy.reshape(-1, M)
+    gnm, h = _native_weight(weight)
     dx = dw = db = None
     if needs[0]:
-        sp24 = _sp24_or_none(gnm, dy2d.shape[0])
-        dx = ops.spmm_t(gnm.val, gnm.idx, M, K, n, m, g, dy2d, sp24=sp24,
-                        packed=None if sp24 is not None else _packed_or_none(gnm, (M, K, n, m, g), dy2d.shape[0], transposed=True)).reshape(x.shape)
+        dx = h.linear_t(gnm, dy, ops.SP24_MIN_TOKENS)
+    if needs[1] or needs[2]:
+        dy2d = dy.reshape(-1, dy.shape[-1])
     if needs[1]:
         # dense weight gradient (training of nmg weights is outside the inference hot path): plain GEMM
-        dw = dy2d.t().mm(x.reshape(-1, K))
+        dw = dy2d.t().mm(x.reshape(-1, x.shape[-1]))
     if has_bias and needs[2]:
         db = dy2d.sum(dim=0)
     return (dx, dw, db) if has_bias else (dx, dw)
@@ -145,7 +138,7 @@ def _linear_bwd_weight_layout(ctx, grad_outputs, input_sparsifiers):
     if grads[1] is not None:
         weight = ctx.saved_tensors[1]
         masked = weight.wrapped_tensor.clone_layout(grads[1])
-        grads[1] = sten.SparseTensorWrapper.wrapped_from_dense(masked, grads[1], None)
+        grads[1] = sten.SparseTensorWrapper([masked], False, sten._DEFAULT_GRAD_FMT(), shared_dummy=True)
     return tuple(grads)
 
 
@@ -164,23 +157,21 @@ def _mm_fwd(ctx, inputs, output_sparsifiers):
     ctx.save_for_backward(weight, b)
     if b.dim() != 2:
         raise sten.DispatchError("grouped n:m matmul expects a 2-D right operand")
-    return sparse_dense_mul_dispatch(weight, b, None, nat.NMG_ACT_K_MAJOR)
+    gnm, h = _native_weight(weight)
+    return h.mm(gnm, b)
 
 
 def _mm_bwd(ctx, grad_outputs, input_sparsifiers):
     weight, b = ctx.saved_tensors
     [dc] = grad_outputs  # [M, N]
     needs = tuple(ctx.needs_input_grad[1:]) + (False,) * 2
-    gnm, M, K, n, m, g = _weight_geometry(weight)
+    gnm, h = _native_weight(weight)
     dw = db = None
     if needs[0]:
         dw = dc.mm(b.t())
     if needs[1]:
         # dB = W^T dC : the transposed kernel computes (dC^T W)[N, K]; hand back its transpose
-        dct = dc.t().contiguous()
-        sp24 = _sp24_or_none(gnm, dct.shape[0])
-        db = ops.spmm_t(gnm.val, gnm.idx, M, K, n, m, g, dct, sp24=sp24,
-                        packed=None if sp24 is not None else _packed_or_none(gnm, (M, K, n, m, g), dct.shape[0], transposed=True)).t()
+        db = h.linear_t(gnm, dc.t().contiguous(), ops.SP24_MIN_TOKENS).t()
     return dw, db
 
 

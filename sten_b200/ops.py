@@ -78,53 +78,17 @@ def geometry(M, K, n, m, g):
 
 def sparsify(dense3, n, m, g):
     """dense3: [B, M, K] view with unit stride along K.  Returns (val [T, C, g, n], idx [T, C, g, 1])."""
-    assert dense3.dim() == 3
-    dev = _require_cuda(dense3)
-    code = _dtype_code(dense3)
-    B, M, K = dense3.shape
-    if dense3.stride(2) != 1 or dense3.stride(1) < K or (B > 1 and dense3.stride(0) < M * dense3.stride(1)):
-        dense3 = dense3.contiguous()
-    # size-1 dims may carry arbitrary strides even in a contiguous tensor: state the packed strides then
-    ld, bs = (K, M * K) if dense3.is_contiguous() else (dense3.stride(1), dense3.stride(0))
-    C, cc, nb, nc = geometry(M, K, n, m, g)
-    T = B * nc * nb
-    val = torch.empty((T, C, g, n), dtype=dense3.dtype, device=dev)
-    idx = torch.empty((T, C, g, 1), dtype=torch.int16, device=dev)
-    with torch.cuda.device(dev):
-        nat.check(nat.lib().nmg_sparsify(dense3.data_ptr(), B, M, K, ld, bs, n, m, g, code,
-                                         val.data_ptr(), idx.data_ptr(), _stream(dev)))
-    return val, idx
+    return nat.host().sparsify(dense3, n, m, g)
 
 
 def gather_layout(dense3, idx, n, m, g):
     """Values of dense3 [B, M, K] at the positions the layout ``idx`` keeps: val [T, C, g, n] of dense3's dtype."""
-    assert dense3.dim() == 3
-    dev = _require_cuda(dense3, idx)
-    code = _dtype_code(dense3)
-    B, M, K = dense3.shape
-    if dense3.stride(2) != 1 or dense3.stride(1) < K or (B > 1 and dense3.stride(0) < M * dense3.stride(1)):
-        dense3 = dense3.contiguous()
-    ld, bs = (K, M * K) if dense3.is_contiguous() else (dense3.stride(1), dense3.stride(0))
-    C, cc, nb, nc = geometry(M, K, n, m, g)
-    idx = idx.contiguous()
-    if idx.numel() != B * nc * nb * cc:
-        raise ValueError("idx does not belong to a layout of this shape")
-    val = torch.empty((B * nc * nb, C, g, n), dtype=dense3.dtype, device=dev)
-    with torch.cuda.device(dev):
-        nat.check(nat.lib().nmg_gather(dense3.data_ptr(), idx.data_ptr(), B, M, K, ld, bs, n, m, g, code, val.data_ptr(), _stream(dev)))
-    return val
+    return nat.host().gather(dense3, idx, n, m, g)
 
 
 def densify(val, idx, B, M, K, n, m, g):
     """Returns the dense [B, M, K] tensor of a (val, idx) pair."""
-    dev = _require_cuda(val, idx)
-    code = _dtype_code(val)
-    val, idx = val.contiguous(), idx.contiguous()
-    out = torch.empty((B, M, K), dtype=val.dtype, device=dev)
-    with torch.cuda.device(dev):
-        nat.check(nat.lib().nmg_densify(val.data_ptr(), idx.data_ptr(), B, M, K, n, m, g, code, out.data_ptr(), K,
-                                        M * K, _stream(dev)))
-    return out
+    return nat.host().densify(val, idx, B, M, K, n, m, g)
 
 
 def perfect_nm_select(dense, n, m, sparse_dim):
@@ -191,9 +155,7 @@ def uses_packed(M, K, tokens, n, m, g, dtype, layout=nat.NMG_ACT_TOKEN_MAJOR, al
     return bool(nat.lib().nmg_spmm_uses_packed(M, K, tokens, n, m, g, code, layout, algo, 1 if transposed else 0))
 
 
-@functools.lru_cache(maxsize=4096)
-def _spmm_workspace_bytes(M, K, tokens, n, m, g, code, layout, algo, have_packed):
-    return nat.lib().nmg_spmm_workspace_bytes(M, K, tokens, n, m, g, code, layout, algo, have_packed)
+_ACTIVATIONS = {None: nat.NMG_EPI_NONE, "gelu": nat.NMG_EPI_GELU}
 
 
 def spmm(val, idx, M, K, n, m, g, act, bias=None, layout=nat.NMG_ACT_TOKEN_MAJOR, algo=nat.NMG_ALGO_AUTO, out=None,
@@ -202,58 +164,10 @@ def spmm(val, idx, M, K, n, m, g, act, bias=None, layout=nat.NMG_ACT_TOKEN_MAJOR
        layout K_MAJOR:              act [K, tokens] -> out [M, tokens] = W @ act   (+ bias per row)
        layout TOKEN_MAJOR_OUT_ROWS: act [tokens, K] -> out [M, tokens] = W @ act^T (+ bias per row)
     ``activation="gelu"`` and ``residual`` (a tensor of the output's shape) make it out = activation(product + bias) + residual
-    in the same call (fused into the matmul's epilogue on the two-pass tensor-core path)."""
-    dev = _require_cuda(val, idx, act, bias)
-    code = _dtype_code(val)
-    if act.dtype != val.dtype or (bias is not None and bias.dtype != val.dtype):
-        raise TypeError(f"activation / bias dtype must match the weight dtype {val.dtype}")
-    act, ld_act = _row_major_2d(act)
-    token_major = layout != nat.NMG_ACT_K_MAJOR
-    tokens = act.shape[0] if token_major else act.shape[1]
-    if (act.shape[1] if token_major else act.shape[0]) != K:
-        raise ValueError(f"activation shape {tuple(act.shape)} does not match K={K}")
-    out_shape = (tokens, M) if layout == nat.NMG_ACT_TOKEN_MAJOR else (M, tokens)
-    if out is None:
-        out = torch.empty(out_shape, dtype=val.dtype, device=dev)
-    else:
-        # the kernel writes out_shape[0] rows of out_shape[1] elements, ld_out apart: anything else would land outside `out`
-        if out.dtype != val.dtype or out.device != dev:
-            raise ValueError(f"out must be a {val.dtype} tensor on {dev}, got {out.dtype} on {out.device}")
-        if tuple(out.shape) != out_shape:
-            raise ValueError(f"out must have shape {out_shape} for this layout, got {tuple(out.shape)}")
-        if out_shape[1] > 1 and out.stride(1) != 1:
-            raise ValueError("out must have unit stride along its rows (a transposed view cannot be written in place)")
-        if out_shape[0] > 1 and out.stride(0) < out_shape[1]:
-            raise ValueError(f"out rows overlap: stride {out.stride(0)} is smaller than the row length {out_shape[1]}")
-    ld_out = out.stride(0) if out_shape[0] > 1 else out_shape[1]
-    if tokens == 0:
-        return out
-    val, idx = val.contiguous(), idx.contiguous()
-    if bias is not None:
-        bias = bias.contiguous()
-    L = nat.lib()
-    if activation not in (None, "gelu"):
+    in the same call (fused into the matmul's epilogue on the tensor-core path)."""
+    if activation not in _ACTIVATIONS:
         raise ValueError("activation must be None or 'gelu'")
-    fused = activation is not None or residual is not None
-    if residual is not None:
-        _require_cuda(residual)
-        if residual.dtype != val.dtype or tuple(residual.shape) != out_shape or (out_shape[1] > 1 and residual.stride(1) != 1):
-            raise ValueError(f"residual must be a {val.dtype} tensor of shape {out_shape} with contiguous rows")
-    with _on_device(dev):
-        ws, nbytes = _workspace(_spmm_workspace_bytes(M, K, tokens, n, m, g, code, layout, algo, 1 if packed is not None else 0), dev)
-        if fused:
-            nat.check(L.nmg_spmm_fused(val.data_ptr(), idx.data_ptr(), packed.data_ptr() if packed is not None else None, M, K, n,
-                                       m, g, code, act.data_ptr(), ld_act, tokens, bias.data_ptr() if bias is not None else None,
-                                       nat.NMG_EPI_GELU if activation == "gelu" else nat.NMG_EPI_NONE,
-                                       residual.data_ptr() if residual is not None else None,
-                                       (residual.stride(0) if out_shape[0] > 1 else out_shape[1]) if residual is not None else 0,
-                                       out.data_ptr(), ld_out, layout, algo, ws.data_ptr() if ws is not None else None, nbytes, _stream(dev)))
-        else:
-            nat.check(L.nmg_spmm(val.data_ptr(), idx.data_ptr(), packed.data_ptr() if packed is not None else None, M, K, n,
-                                 m, g, code, act.data_ptr(), ld_act, tokens,
-                                 bias.data_ptr() if bias is not None else None, out.data_ptr(), ld_out, layout, algo,
-                                 ws.data_ptr() if ws is not None else None, nbytes, _stream(dev)))
-    return out
+    return nat.host().spmm(val, idx, M, K, n, m, g, act, bias, layout, algo, out, packed, _ACTIVATIONS[activation], residual)
 
 
 def expand(val, idx, M, K, n, m, g):
@@ -345,32 +259,7 @@ def pack_sp24(val, idx, M, K, n, m, g):
 def spmm_t(val, idx, M, K, n, m, g, dy, algo=nat.NMG_ALGO_AUTO, packed=None, sp24=None):
     """dy [tokens, M] -> dx [tokens, K] = dy @ W.  ``sp24``: result of pack_sp24 for the same weight; used (and the per-call
     compression skipped) when the call would take the structured-sparse path anyway."""
-    dev = _require_cuda(val, idx, dy)
-    code = _dtype_code(val)
-    if dy.dtype != val.dtype:
-        raise TypeError(f"gradient dtype must match the weight dtype {val.dtype}")
-    dy, ld_dy = _row_major_2d(dy)
-    tokens = dy.shape[0]
-    if dy.shape[1] != M:
-        raise ValueError(f"gradient shape {tuple(dy.shape)} does not match M={M}")
-    dx = torch.empty((tokens, K), dtype=val.dtype, device=dev)
-    if tokens == 0:
-        return dx
-    val, idx = val.contiguous(), idx.contiguous()
-    L = nat.lib()
-    if (sp24 is not None and tokens >= SP24_MIN_TOKENS and algo in (nat.NMG_ALGO_AUTO, nat.NMG_ALGO_TENSOR)
-            and dy.data_ptr() % 16 == 0 and ld_dy % 8 == 0):
-        with _on_device(dev):
-            nat.check(L.nmg_spmm_t_sp24(sp24.data_ptr(), M, K, n, m, g, code, dy.data_ptr(), ld_dy, tokens, dx.data_ptr(), K, _stream(dev)))
-        return dx
-    with _on_device(dev):
-        ws, nbytes = _workspace(L.nmg_spmm_t_workspace_bytes(M, K, tokens, n, m, g, code, algo,
-                                                             1 if packed is not None else 0), dev)
-        nat.check(L.nmg_spmm_t(val.data_ptr(), idx.data_ptr(), packed.data_ptr() if packed is not None else None, M, K,
-                               n, m, g, code, dy.data_ptr(), ld_dy, tokens,
-                               dx.data_ptr(), K, algo, ws.data_ptr() if ws is not None else None, nbytes,
-                               _stream(dev)))
-    return dx
+    return nat.host().spmm_t(val, idx, M, K, n, m, g, dy, algo, packed, sp24, SP24_MIN_TOKENS)
 
 
 def copy_2d_async(dst, src, stream=None):

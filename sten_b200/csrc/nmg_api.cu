@@ -39,27 +39,27 @@ extern "C" int nmg_pack(const void *val, const int16_t *idx, int64_t M, int64_t 
     const size_t need = natural_bytes(geo, dtype, &pat_bytes) + 256;
     if (packed_bytes < need) NMG_FAIL(NMG_ERR_WORKSPACE, "packed buffer of %zu bytes required, got %zu", need, packed_bytes);
     char *base = align256(packed);
-    return launch_build_natural(geo, dtype, val, idx, reinterpret_cast<uint16_t *>(base), base + pat_bytes, (cudaStream_t)stream);
+    return launch_build_natural(geo, dtype, val, idx, base, base + pat_bytes, (cudaStream_t)stream);
 }
 
 // Resolve the column-ordered copy: the caller's, or one built at the front of the workspace.  Advances *ws.
 static int resolve_packed(const Geo &geo, int dtype, const void *val, const int16_t *idx, const void *packed, char **ws,
-                          size_t *ws_left, const uint16_t **pat, const void **nval, cudaStream_t st) {
+                          size_t *ws_left, const void **pat, const void **nval, cudaStream_t st) {
     size_t pat_bytes = 0;
     const size_t nat = natural_bytes(geo, dtype, &pat_bytes);
     if (packed) {
         char *base = align256(const_cast<void *>(packed));
-        *pat = reinterpret_cast<const uint16_t *>(base);
+        *pat = base;
         *nval = base + pat_bytes;
         return NMG_OK;
     }
     if (!*ws || *ws_left < nat + 256) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace too small for the column-ordered weight copy (%zu bytes)", nat + 256);
     char *base = align256(*ws);
-    *pat = reinterpret_cast<const uint16_t *>(base);
+    *pat = base;
     *nval = base + pat_bytes;
     *ws_left -= (size_t)(base + nat - *ws);
     *ws = base + nat;
-    return launch_build_natural(geo, dtype, val, idx, reinterpret_cast<uint16_t *>(base), base + pat_bytes, st);
+    return launch_build_natural(geo, dtype, val, idx, base, base + pat_bytes, st);
 }
 
 // K-major activations (B[K][tokens], the torch.mm orientation) reach the tensor cores through one same-dtype transpose
@@ -77,8 +77,7 @@ extern "C" size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens,
     if (algo == NMG_ALGO_TENSOR_DENSE) algo = NMG_ALGO_TENSOR;
     if (algo != NMG_ALGO_SIMT && (tc_supported(geo, dtype) || tc_dense_supported(geo, dtype)))
         tensor = (tc_use_dense(geo, dtype, tokens) ? tc_dense_workspace_bytes(geo, dtype, false)
-                                                   : (have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512) +
-                                                         tc_ksplit_workspace_bytes(geo, dtype, false, tokens)) +
+                                                   : (have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512)) +
                  tc_split_workspace_bytes(geo, dtype, false, tokens) + (layout == NMG_ACT_K_MAJOR ? kmajor_transpose_bytes(geo, dtype, tokens) : 0);
     if (algo == NMG_ALGO_TENSOR) return tensor;
     return simt > tensor ? simt : tensor;  // AUTO may take either path depending on operand alignment
@@ -128,7 +127,7 @@ static int spmm_impl(const void *val, const int16_t *idx, const void *packed, in
     if (algo == NMG_ALGO_TENSOR || (algo == NMG_ALGO_AUTO && can_tensor && M >= 64)) {
         char *ws = static_cast<char *>(workspace);
         size_t left = workspace_bytes;
-        const uint16_t *pat = nullptr;
+        const void *pat = nullptr;
         const void *nval = nullptr;
         const bool dense = force_dense || tc_use_dense(geo, dtype, tokens);
         if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st))) return rc;
@@ -207,8 +206,7 @@ extern "C" size_t nmg_spmm_t_workspace_bytes(int64_t M, int64_t K, int64_t token
     const size_t simt = algo != NMG_ALGO_TENSOR ? pack + simt_bwd_workspace_bytes(geo, tokens, dtype) + 256 : 0;
     size_t tensor = 0;
     if (algo != NMG_ALGO_SIMT && (tc_supported(geo, dtype) || tc_dense_supported(geo, dtype)))
-        tensor = (tc_use_dense(geo, dtype, tokens) ? tc_dense_workspace_bytes(geo, dtype, true)
-                                                   : pack + tc_ksplit_workspace_bytes(geo, dtype, true, tokens)) +
+        tensor = (tc_use_dense(geo, dtype, tokens) ? tc_dense_workspace_bytes(geo, dtype, true) : pack) +
                  tc_split_workspace_bytes(geo, dtype, true, tokens);
     if (use_sp(geo, dtype, tokens, algo) && tc_sp_copy_bytes(geo) + 256 > tensor) tensor = tc_sp_copy_bytes(geo) + 256;
     return simt > tensor ? simt : tensor;
@@ -232,7 +230,7 @@ extern "C" int nmg_spmm_t(const void *val, const int16_t *idx, const void *packe
         NMG_FAIL(NMG_ERR_UNSUPPORTED, "tensor-core path needs gradient rows that are 16-byte aligned (16-bit dtypes) and a chunk that fits shared memory");
     char *ws = static_cast<char *>(workspace);
     size_t left = workspace_bytes;
-    const uint16_t *pat = nullptr;
+    const void *pat = nullptr;
     const void *nval = nullptr;
     const bool tensor = algo == NMG_ALGO_TENSOR || algo == NMG_ALGO_TENSOR_DENSE || (algo == NMG_ALGO_AUTO && can_tensor && K >= 64);
     // The rows of W are the reduction axis here, so the n:m structure is one the tensor cores can skip: structured-sparse

@@ -202,6 +202,11 @@ __device__ __forceinline__ void tma_load_2d(void *smem_dst, const CUtensorMap *m
         ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
         : "memory");
 }
+// `bytes` consecutive bytes, a multiple of 16 with both addresses 16-byte aligned.
+__device__ __forceinline__ void bulk_load(void *smem_dst, const void *gsrc, int bytes, uint64_t *bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(bytes), "r"(smem_u32(bar)) : "memory");
+}
 // Tiled store shared -> global of one box (bulk async-group completion).  Rows and columns of the box that fall outside
 // the tensor are not written.  x * element size must be a multiple of 16 bytes and neither coordinate may be negative.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, const void *smem_src, int x, int y) {
@@ -235,5 +240,6 @@ __device__ __forceinline__ const char *stage_bytes_async(char *dst16, const void
 // Host: encode a 2-D tiled tensor map (row-major [rows][ld] array, box = box_rows x box_cols) without linking libcuda.
 int encode_tmap_2d(CUtensorMap *map, int dtype, const void *base, uint64_t cols, uint64_t rows, uint64_t ld_elems,
                    uint32_t box_cols, uint32_t box_rows, int swizzle_128b);
+int encode_tmap_2d_bytes(CUtensorMap *map, const void *base, uint64_t cols, uint64_t rows, uint64_t ld, uint32_t box_cols, uint32_t box_rows);  // no swizzle
 
 }  // namespace nmg

@@ -195,20 +195,6 @@ struct GemmMaps {
     CUtensorMap out;   // out_tma: the output, box 128 bytes x 32 rows, 128-byte swizzle
 };
 
-// Exact (erf) GELU with a short erf: erf(x) = 1 - (a1 t + ... + a5 t^5) exp(-x^2), t = 1 / (1 + p x) for x >= 0 (Abramowitz &
-// Stegun 7.1.26, absolute error 1.5e-7, i.e. below fp32 rounding of the result for |v| of order one).  With x = |v| / sqrt(2)
-// and v * sign(v) = |v|, gelu(v) = v (1 + erf(v / sqrt 2)) / 2 collapses to max(v, 0) - |v| q(t) 2^(-v^2 log2(e) / 2) where q
-// carries the halved coefficients: fourteen instructions, two of them on the special-function unit (flush-to-zero forms, which
-// need no range fix-up), against the library erf's thirty.  The drain warps apply it to 128 x 256 values per tile.
-__device__ __forceinline__ float gelu_erf(float v) {
-    const float av = fabsf(v);
-    float t, e;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.23164189f, av, 1.f)));   // p / sqrt(2)
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((v * -0.72134752f) * v));          // log2(e) / 2
-    const float q = fmaf(fmaf(fmaf(fmaf(0.5307027145f, t, -0.7265760135f), t, 0.7107068705f), t, -0.142248368f), t, 0.127414796f) * t;
-    return fmaf(-(av * q), e, fmaxf(v, 0.f));
-}
-
 // PAIR = false: one CTA per 128-feature x 256-token tile.
 // PAIR = true (16-bit operands): two CTAs of a cluster share a 256-feature x 256-token tile.  Each loads the weight rows
 // of its own 128 features and only half of the activation tile (128 tokens); the MMA (cta_group::2, M = 256, issued by the

@@ -148,16 +148,12 @@ static EncodeTiledFn get_encode_fn() {
     return fn;
 }
 
-int encode_tmap_2d(CUtensorMap *map, int dtype, const void *base, uint64_t cols, uint64_t rows, uint64_t ld_elems,
+static int encode_tmap(CUtensorMap *map, CUtensorMapDataType dt, size_t es, const void *base, uint64_t cols, uint64_t rows, uint64_t ld_elems,
                    uint32_t box_cols, uint32_t box_rows, int swizzle_128b) {
     EncodeTiledFn fn = get_encode_fn();
     if (!fn) NMG_FAIL(NMG_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-    size_t es = dtype_size(dtype);
     if (((uintptr_t)base & 15) || ((ld_elems * es) & 15))
         NMG_FAIL(NMG_ERR_INVALID, "TMA operand needs a 16-byte aligned base and row pitch");
-    CUtensorMapDataType dt = dtype == NMG_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
-                             : dtype == NMG_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
-                                                : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     cuuint64_t dims[2] = {cols, rows};
     cuuint64_t strides[1] = {ld_elems * es};
     cuuint32_t box[2] = {box_cols, box_rows};
@@ -175,6 +171,18 @@ int encode_tmap_2d(CUtensorMap *map, int dtype, const void *base, uint64_t cols,
     }
     if (r != CUDA_SUCCESS) NMG_FAIL(NMG_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
     return NMG_OK;
+}
+
+int encode_tmap_2d(CUtensorMap *map, int dtype, const void *base, uint64_t cols, uint64_t rows, uint64_t ld_elems,
+                   uint32_t box_cols, uint32_t box_rows, int swizzle_128b) {
+    const CUtensorMapDataType dt = dtype == NMG_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                   : dtype == NMG_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                                      : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    return encode_tmap(map, dt, dtype_size(dtype), base, cols, rows, ld_elems, box_cols, box_rows, swizzle_128b);
+}
+
+int encode_tmap_2d_bytes(CUtensorMap *map, const void *base, uint64_t cols, uint64_t rows, uint64_t ld, uint32_t box_cols, uint32_t box_rows) {
+    return encode_tmap(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, base, cols, rows, ld, box_cols, box_rows, 0);
 }
 
 }  // namespace nmg

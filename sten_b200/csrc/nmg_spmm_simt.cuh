@@ -16,13 +16,13 @@ int launch_widen_to_f32(const void *src, int dtype, int64_t rows, int64_t cols, 
                         int64_t ld_dst, cudaStream_t st);
 
 // Column-order ("natural") copy of a weight: for every row-block mb and column k of the padded width Kp,
-// pat[mb][k] = pattern of that column, nval[mb][k][s] = its n kept values.
-struct NaturalLayout { size_t pat_bytes, val_bytes, plane_bytes, total; };
+// pat[mb][k] = pattern of that column (id * m in one byte for the specialised patterns, else a 16-bit id), nval[mb][k][s] = its n kept values.
+struct NaturalLayout { size_t pat_bytes, val_bytes, mask_bytes, total; };
 NaturalLayout natural_layout(const Geo &geo, int dtype);
 int64_t natural_width(const Geo &geo);
+int64_t natural_mask_rows(const Geo &geo);  // rows of the row masks: M rounded up to the tensor-core tile
 size_t natural_bytes(const Geo &geo, int dtype, size_t *pat_bytes_out);
-int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16_t *idx, uint16_t *pat, void *nval,
-                         cudaStream_t st);
+int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16_t *idx, void *pat, void *nval, cudaStream_t st);
 
 // SIMT kernels (fp32 accumulate).  xt is the activation as [K][ld_xt] fp32 (tokens contiguous).
 size_t simt_fwd_workspace_bytes(const Geo &geo, int64_t tokens, int dtype, int layout);
@@ -31,7 +31,7 @@ int simt_fwd(const Geo &geo, int dtype, const void *val, const int16_t *idx, con
              cudaStream_t st);
 // pat / nval: the column-ordered copy; the workspace only holds the fp32 transpose of dY
 size_t simt_bwd_workspace_bytes(const Geo &geo, int64_t tokens, int dtype);
-int simt_bwd(const Geo &geo, int dtype, const uint16_t *pat, const void *nval, const void *dy, int64_t ld_dy,
+int simt_bwd(const Geo &geo, int dtype, const void *pat, const void *nval, const void *dy, int64_t ld_dy,
              int64_t tokens, void *dx, int64_t ld_dx, void *ws, size_t ws_bytes, cudaStream_t st);
 
 // Tensor-core kernels.  act: [tokens][ld_act] with the reduction axis contiguous.  fp32 operands are multiplied as
@@ -56,12 +56,9 @@ bool tc_dense_supported(const Geo &geo, int dtype);  // two-pass variant
 bool tc_use_dense(const Geo &geo, int dtype, int64_t tokens);
 size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens);
 size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed);
-// fused kernel with few output tiles: the reduction axis is cut over tc_ksplit CTAs per tile, fp32 partial tiles in `ws`
-int tc_ksplit(const Geo &geo, int dtype, bool transposed, int64_t tokens);
-size_t tc_ksplit_workspace_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens);
 // outs / n_outs: the result goes to every listed buffer (same shape and pitch); more than one needs `dense`.  mc_out, when
 // not NULL, is an NVSwitch multicast address that maps onto all of them: full 16-byte chunks are then stored once.
-int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void *val, const int16_t *idx, const uint16_t *pat,
+int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void *val, const int16_t *idx, const void *pat,
               const void *nval, const void *act, int64_t ld_act, int64_t tokens, const void *bias, void *const *outs, int n_outs,
               void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi = Epilogue());
 int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const CUtensorMap *act_maps,
@@ -124,7 +121,7 @@ int simt_fwd_launch(int dtype, int tt, const FwdParams &p, const CUtensorMap &tm
 
 // ---- specialised transposed kernel: parameters, shared-memory plan, per-(n, m) launchers
 struct BwdParams {
-    const uint16_t *pat;  // [nb][Kp]
+    const uint8_t *pat;   // [nb][Kp] pattern id * m
     const void *nval;     // [nb][Kp][n]
     void *dx;
     int64_t M, K, Kp, ntok, ld_dx, nb;
@@ -142,7 +139,7 @@ struct BwdSmemPlan { size_t y_bytes, p_bytes, v_bytes, stage_bytes, total; };
 __host__ __device__ inline BwdSmemPlan bwd_smem_plan(int m, int n, int rb_stage, size_t es) {
     BwdSmemPlan p;
     p.y_bytes = (size_t)rb_stage * m * kBwdTok * 4;
-    p.p_bytes = ((size_t)rb_stage * kColsCta * 2 + 127) & ~(size_t)127;
+    p.p_bytes = ((size_t)rb_stage * kColsCta + 127) & ~(size_t)127;
     p.v_bytes = ((size_t)rb_stage * kColsCta * n * es + 127) & ~(size_t)127;
     p.stage_bytes = p.y_bytes + p.p_bytes + p.v_bytes;
     p.total = 2 * p.stage_bytes + 256;

@@ -8,61 +8,94 @@
 // warp pulls the m x TT slice of dY^T from shared memory into registers once and re-uses it for all KW
 // columns; the pattern of each column selects, through a warp-uniform switch over the compile-time pattern
 // table, which n of those registers are multiplied.  Accumulators stay in registers over all row-blocks.
+#include <type_traits>
+
 #include "nmg_spmm_simt.cuh"
 
 namespace nmg {
 
 // ------------------------------------------------------------------------------------------ column-ordered copy
 struct NaturalParams {
-    const void *val; const int16_t *idx; uint16_t *pat; void *nval;
-    __nv_bfloat16 *plane[3];  // fp32 weights only, else NULL
+    const void *val; const int16_t *idx; void *pat; void *nval;
     int64_t nb, nc, Kp;
-    int n, g, cc;
+    int n, m, g, cc;
+    int wide;    // 16-bit pattern ids
+    int planar;  // n = 2: neighbouring columns' first values, then their second values
 };
-template <typename T>
+// One thread per stored column slot.  SMALL: fewer than 2^31 slots, 32-bit index arithmetic.
+template <typename T, bool SMALL>
 __global__ void build_natural_kernel(const NaturalParams prm) {
-    const int64_t total = prm.nb * prm.nc * prm.cc;  // one thread per stored column slot
+    using I = typename std::conditional<SMALL, uint32_t, uint64_t>::type;
+    const I total = (I)(prm.nb * prm.nc * prm.cc), nb = (I)prm.nb;
     const T *val = static_cast<const T *>(prm.val);
     T *nval = static_cast<T *>(prm.nval);
-    for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t tile = e / prm.cc;
-        const int slot = (int)(e - tile * prm.cc);
-        const int64_t mb = tile % prm.nb, kc = tile / prm.nb;
+    for (I e = (I)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (I)gridDim.x * blockDim.x) {
+        const I tile = e / (uint32_t)prm.cc, kc = tile / nb;
+        const int slot = (int)(e - tile * (uint32_t)prm.cc);
+        const int64_t mb = (int64_t)(tile - kc * nb);
         const int c = prm.idx[e];
         if (c < 0 || c >= prm.cc) continue;  // malformed index: leave the column empty
-        const int64_t k = kc * prm.cc + c;
-        prm.pat[mb * prm.Kp + k] = (uint16_t)(slot / prm.g);
-        for (int s = 0; s < prm.n; s++) {
-            const T v = val[e * prm.n + s];
-            const int64_t o = (mb * prm.Kp + k) * prm.n + s;
-            nval[o] = v;
-            if (prm.plane[0]) {  // exact three-way split of an fp32 value into bf16 pieces
-                const float f = DT<T>::to_f32(v);
-                const __nv_bfloat16 hi = __float2bfloat16_rn(f);
-                const float r1 = f - __bfloat162float(hi);
-                const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
-                const __nv_bfloat16 lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
-                prm.plane[0][o] = hi; prm.plane[1][o] = mid; prm.plane[2][o] = lo;
+        const int64_t o = mb * prm.Kp + (int64_t)kc * prm.cc + c;
+        if (prm.wide) static_cast<uint16_t *>(prm.pat)[o] = (uint16_t)(slot / prm.g);
+        else static_cast<uint8_t *>(prm.pat)[o] = (uint8_t)(slot / prm.g * prm.m);
+        for (int s = 0; s < prm.n; s++) nval[prm.planar ? (o & ~(int64_t)1) * 2 + s * 2 + (o & 1) : o * prm.n + s] = val[(int64_t)e * prm.n + s];
+    }
+}
+
+// Row masks of the forward tensor-core kernel, [k-block of 64 columns][row][8 n bytes]: per slot two words of "the row holds
+// the column's value of this slot"; bit 8 j + q of a word is column 4 q + j of its 32.
+__global__ void __launch_bounds__(256) build_masks_kernel(const uint8_t *__restrict__ pat, const int8_t *__restrict__ slot_of_row, uint32_t *__restrict__ masks, int64_t M,
+                                                          int64_t Kp, int64_t rows, int n, int m) {
+    const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, kb = blockIdx.y;
+    if (row >= rows) return;
+    uint32_t mask[2][2] = {{0, 0}, {0, 0}};
+    if (row < M) {
+        const int64_t mb = row / m;
+        const int r = (int)(row - mb * m);
+        const uint4 *src = reinterpret_cast<const uint4 *>(pat + mb * Kp + kb * 64);
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint4 v = __ldg(src + i);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int c = 0; c < 16; c++) {
+                const int col = i * 16 + c, bit = 8 * (col & 3) + ((col & 31) >> 2);
+                // the byte is pattern * m: where the pattern's row table starts
+                const int s = slot_of_row[((w[c >> 2] >> (8 * (c & 3))) & 0xffu) + r];
+                if (s == 0) mask[0][col >> 5] |= 1u << bit;
+                if (s == 1) mask[1][col >> 5] |= 1u << bit;
             }
         }
     }
+    uint32_t *dst = masks + (kb * rows + row) * 2 * n;
+    dst[0] = mask[0][0];
+    dst[1] = mask[0][1];
+    if (n == 2) { dst[2] = mask[1][0]; dst[3] = mask[1][1]; }
+}
+
+static bool bwd_specialised(int n, int m) {
+    return (n == 1 && m == 4) || (n == 2 && m == 4) || (n == 1 && m == 8) || (n == 2 && m == 8) || (n == 1 && m == 16) ||
+           (n == 3 && m == 6);
 }
 
 // Width of the column-ordered copy: the padded weight width rounded up to the 128-column CTA tile, so every
 // row segment a CTA stages is full-size and 16-byte aligned.
 int64_t natural_width(const Geo &geo) { return round_up(geo.nc * geo.cc, 128); }
 
-// Sections of the copy: pattern ids, values in the weight's dtype, and -- for fp32 weights -- three bf16 planes
-// holding the exact split v = hi + mid + lo that the tensor-core kernel multiplies term by term.
+// Sections of the copy: one pattern entry per column, the values in the weight's dtype and, where the tensor-core kernel
+// serves the pattern, the row masks.  The patterns with specialised
+// kernels (at most 28) store one byte, pattern id times m: the offset of the pattern's row selectors in the expansion table of
+// the tensor-core kernel; with n = 2 their values are stored pair-wise planar.  All others store 16-bit ids.
 NaturalLayout natural_layout(const Geo &geo, int dtype) {
     const size_t entries = (size_t)geo.nb * (size_t)natural_width(geo);
     NaturalLayout l;
-    l.pat_bytes = (entries * 2 + 255) & ~(size_t)255;
+    l.pat_bytes = (entries * (bwd_specialised(geo.n, geo.m) ? 1 : 2) + 255) & ~(size_t)255;
     l.val_bytes = (entries * geo.n * dtype_size(dtype) + 255) & ~(size_t)255;
-    l.plane_bytes = dtype == NMG_F32 ? ((entries * geo.n * 2 + 255) & ~(size_t)255) : 0;
-    l.total = l.pat_bytes + l.val_bytes + 3 * l.plane_bytes;
+    l.mask_bytes = tc_supported(geo, dtype) ? (size_t)(natural_width(geo) / 64) * (size_t)natural_mask_rows(geo) * 8 * geo.n : 0;
+    l.total = l.pat_bytes + l.val_bytes + l.mask_bytes;
     return l;
 }
+int64_t natural_mask_rows(const Geo &geo) { return round_up(geo.M, 128); }
 
 size_t natural_bytes(const Geo &geo, int dtype, size_t *pat_bytes_out) {
     const NaturalLayout l = natural_layout(geo, dtype);
@@ -70,23 +103,30 @@ size_t natural_bytes(const Geo &geo, int dtype, size_t *pat_bytes_out) {
     return l.total;
 }
 
-int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16_t *idx, uint16_t *pat, void *nval,
-                         cudaStream_t st) {
-    const NaturalLayout lay = natural_layout(geo, dtype);
-    NaturalParams p{val, idx, pat, nval, {nullptr, nullptr, nullptr}, geo.nb, geo.nc, natural_width(geo), geo.n, geo.g, geo.cc};
-    if (lay.plane_bytes)
-        for (int c = 0; c < 3; c++)
-            p.plane[c] = reinterpret_cast<__nv_bfloat16 *>(static_cast<char *>(nval) + lay.val_bytes + c * lay.plane_bytes);
+int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16_t *idx, void *pat, void *nval, cudaStream_t st) {
+    NaturalParams p{val, idx, pat, nval, geo.nb, geo.nc, natural_width(geo), geo.n, geo.m, geo.g, geo.cc, bwd_specialised(geo.n, geo.m) ? 0 : 1,
+                    bwd_specialised(geo.n, geo.m) && geo.n == 2 ? 1 : 0};
     const int64_t total = geo.nb * geo.nc * geo.cc;
     int64_t blocks = (total + 255) / 256;
     if (blocks > 148 * 64) blocks = 148 * 64;
-    // every (mb, k) of the padded width is written exactly once because idx is a permutation per tile;
-    // clear first so that a malformed idx leaves zeros, not stale workspace contents
-    size_t pat_bytes = 0;
-    const size_t all = natural_bytes(geo, dtype, &pat_bytes);
-    NMG_CUDA(cudaMemsetAsync(pat, 0, pat_bytes, st));
-    NMG_CUDA(cudaMemsetAsync(nval, 0, all - pat_bytes, st));
-    NMG_DISPATCH_DTYPE(dtype, T, (build_natural_kernel<T><<<(unsigned)blocks, 256, 0, st>>>(p)));
+    // every (mb, k) of the chunks is written exactly once because idx is a permutation per tile; clear first so that the
+    // columns between the last chunk and the padded width, and what a malformed idx leaves out, are zeros
+    const NaturalLayout lay = natural_layout(geo, dtype);
+    NMG_CUDA(cudaMemsetAsync(pat, 0, lay.pat_bytes + lay.val_bytes, st));  // the values follow the patterns
+    if (total < 0x40000000ll) {
+        NMG_DISPATCH_DTYPE(dtype, T, (build_natural_kernel<T, true><<<(unsigned)blocks, 256, 0, st>>>(p)));
+    } else {
+        NMG_DISPATCH_DTYPE(dtype, T, (build_natural_kernel<T, false><<<(unsigned)blocks, 256, 0, st>>>(p)));
+    }
+    if (lay.mask_bytes) {
+        PatternTable tab;
+        int rc = get_pattern_table(geo.n, geo.m, &tab);
+        if (rc) return rc;
+        const int64_t rows = natural_mask_rows(geo), kbs = natural_width(geo) / 64;
+        if (kbs > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "weight has too many columns for the column-ordered copy");
+        build_masks_kernel<<<dim3((unsigned)((rows + 255) / 256), (unsigned)kbs), 256, 0, st>>>(
+            static_cast<const uint8_t *>(pat), tab.slot_of_row, reinterpret_cast<uint32_t *>(static_cast<char *>(nval) + lay.val_bytes), geo.M, natural_width(geo), rows, geo.n, geo.m);
+    }
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;
 }
@@ -116,11 +156,6 @@ __global__ void spmm_bwd_generic_kernel(const GenBwdParams prm) {
 }
 
 // ------------------------------------------------------------------------------------------ host side
-static bool bwd_specialised(int n, int m) {
-    return (n == 1 && m == 4) || (n == 2 && m == 4) || (n == 1 && m == 8) || (n == 2 && m == 8) || (n == 1 && m == 16) ||
-           (n == 3 && m == 6);
-}
-
 static int bwd_rb_stage(int m) {  // rows per stage <= 64 keeps one TMA box (256-row limit) and ~32 KB of dY^T
     int rs = 64 / m;
     return rs > 0 ? rs : 1;
@@ -131,7 +166,7 @@ size_t simt_bwd_workspace_bytes(const Geo &geo, int64_t tokens, int dtype) {
     return bwd_specialised(geo.n, geo.m) ? (size_t)geo.M * (size_t)round_up(tokens, 128) * 4 + 256 : 0;
 }
 
-int simt_bwd(const Geo &geo, int dtype, const uint16_t *pat, const void *nval, const void *dy, int64_t ld_dy,
+int simt_bwd(const Geo &geo, int dtype, const void *pat, const void *nval, const void *dy, int64_t ld_dy,
              int64_t tokens, void *dx, int64_t ld_dx, void *ws, size_t ws_bytes, cudaStream_t st) {
     const size_t need = simt_bwd_workspace_bytes(geo, tokens, dtype);
     if (need && (!ws || ws_bytes < need)) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required, got %zu", need, ws_bytes);
@@ -143,7 +178,7 @@ int simt_bwd(const Geo &geo, int dtype, const uint16_t *pat, const void *nval, c
         PatternTable tab;
         if ((rc = get_pattern_table(geo.n, geo.m, &tab))) return rc;
         if (tokens > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "generic transposed kernel handles at most 65535 tokens per call");
-        GenBwdParams p{pat, nval, dy, dx, tab.order, geo.M, geo.K, Kp, tokens, ld_dy, ld_dx, geo.nb, geo.n, geo.m};
+        GenBwdParams p{static_cast<const uint16_t *>(pat), nval, dy, dx, tab.order, geo.M, geo.K, Kp, tokens, ld_dy, ld_dx, geo.nb, geo.n, geo.m};
         dim3 grid((unsigned)((geo.K + 127) / 128), (unsigned)tokens);
         const ProfileEvents pe = take_profile_events();
         if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));
@@ -162,7 +197,7 @@ int simt_bwd(const Geo &geo, int dtype, const uint16_t *pat, const void *nval, c
         return rc;
     int *status = nullptr;
     if ((rc = get_status_word(&status))) return rc;
-    BwdParams p{pat, nval, dx, geo.M, geo.K, Kp, tokens, ld_dx, geo.nb, rs, status};
+    BwdParams p{static_cast<const uint8_t *>(pat), nval, dx, geo.M, geo.K, Kp, tokens, ld_dx, geo.nb, rs, status};
     const ProfileEvents pe = take_profile_events();
     if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));
 #define NMG_BWD_LAUNCH(N_, M_)                                                \

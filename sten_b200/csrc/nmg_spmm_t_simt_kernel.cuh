@@ -56,7 +56,7 @@ spmm_bwd_simt_kernel(const BwdParams prm, const __grid_constant__ CUtensorMap tm
         // pattern / value slabs: per row-block one 128-column run, 16-byte aligned because the copy is 128 wide
         char *ps = base + plan.y_bytes;
         char *vs = base + plan.y_bytes + plan.p_bytes;
-        constexpr int PB = kColsCta * 2 / 16, VB = kColsCta * N_ * (int)sizeof(T) / 16;  // 16-byte blocks per row-block
+        constexpr int PB = kColsCta / 16, VB = kColsCta * N_ * (int)sizeof(T) / 16;  // 16-byte blocks per row-block
         for (int e = tid; e < nrb * PB; e += kBwdWarps * 32) {
             const int rb = e / PB, b = e - rb * PB;
             cp_async_16(ps + (size_t)e * 16, reinterpret_cast<const char *>(prm.pat + (mb_first + rb) * prm.Kp + k0) + b * 16);
@@ -89,7 +89,7 @@ spmm_bwd_simt_kernel(const BwdParams prm, const __grid_constant__ CUtensorMap tm
 
         const char *base = smem + plan.stage_bytes * st;
         const float *Ys = reinterpret_cast<const float *>(base);
-        const uint16_t *ps = reinterpret_cast<const uint16_t *>(base + plan.y_bytes);
+        const uint8_t *ps = reinterpret_cast<const uint8_t *>(base + plan.y_bytes);
         const T *vs = reinterpret_cast<const T *>(base + plan.y_bytes + plan.p_bytes);
         const int64_t mb_first = step * RS;
         const int nrb = (int)((prm.nb - mb_first) < RS ? (prm.nb - mb_first) : RS);
@@ -100,14 +100,14 @@ spmm_bwd_simt_kernel(const BwdParams prm, const __grid_constant__ CUtensorMap tm
                 const float4 v = *reinterpret_cast<const float4 *>(Ys + (size_t)(rb * M_ + r) * kBwdTok + lane * kBwdTT);
                 dy[r][0] = v.x; dy[r][1] = v.y; dy[r][2] = v.z; dy[r][3] = v.w;
             }
-            const uint16_t *pw = ps + rb * kColsCta + warp * kKW;
+            const uint8_t *pw = ps + rb * kColsCta + warp * kKW;
             const T *vw = vs + (size_t)(rb * kColsCta + warp * kKW) * N_;
 #pragma unroll
             for (int kk = 0; kk < kKW; kk++) {
-                const int p = pw[kk];
+                const int p = pw[kk] / M_;
                 float w[N_];
 #pragma unroll
-                for (int s = 0; s < N_; s++) w[s] = DT<T>::to_f32(vw[kk * N_ + s]);
+                for (int s = 0; s < N_; s++) w[s] = DT<T>::to_f32(vw[N_ == 2 ? (kk & ~1) * 2 + s * 2 + (kk & 1) : kk * N_ + s]);
                 switch (p) {
                     NMG_BWD_CASE(0) NMG_BWD_CASE(1) NMG_BWD_CASE(2) NMG_BWD_CASE(3) NMG_BWD_CASE(4) NMG_BWD_CASE(5)
                     NMG_BWD_CASE(6) NMG_BWD_CASE(7) NMG_BWD_CASE(8) NMG_BWD_CASE(9) NMG_BWD_CASE(10) NMG_BWD_CASE(11)

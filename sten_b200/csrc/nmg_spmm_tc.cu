@@ -9,13 +9,20 @@
 // against activation tiles that arrive by TMA.  The same kernel computes the transposed product dX = dY W: only
 // the expansion routine differs (the tile is W^T, the reduction runs over weight rows).
 //
-// CTA = 14 warps: warp 0 issues TMA loads of the activation tile (256 tokens x 64 reduction elements), warp 1
-// allocates TMEM and issues the MMAs (128 x 256 x 16, fp32 accumulate in TMEM), warps 2..13 form three groups
+// CTA = 14 warps: warp 0 issues TMA loads of the activation tile (up to 256 tokens x 64 reduction elements), warp 1
+// allocates TMEM and issues the MMAs (128 x tokens x 16, fp32 accumulate in TMEM), warps 2..13 form three groups
 // that expand the weight tile (128 output features x 64 reduction elements) of every third k-block each; every
-// group fetches its next tile's compressed data into registers before it scatters the current one.  Group 0 also runs the epilogue
-// (tcgen05.ld -> bias -> convert -> store).  All waits are bounded; a wait that runs out sets the status word
-// and the CTA drains to the common exit where TMEM is released.
-#include <cstdlib>
+// group fetches its next tile's compressed data into registers before it scatters the current one.  fp32 weights: a
+// k-block's three bf16 planes are expanded once and multiplied six times (the split products), instead of once per product.
+// All twelve then run the epilogue (tcgen05.ld -> bias -> activation -> residual -> store).
+//
+// What bounds it with few tokens is latency, not bandwidth: at 4096 x 4096 and 16 tokens the 25 MB of compressed weight are
+// 4 us of HBM time.  So the reduction axis is cut over a cluster of CTAs that fills the chip, and the partial tiles meet in
+// distributed shared memory -- a second kernel that reads partial tiles from memory cost 4 .. 9 us for 7 .. 14 us of matmul
+// (4096 x 1024, 384 tokens: 14.0 + 9.4 us) -- the tile is as wide as the batch needs, and the first tile's loads leave
+// before the set-up barrier.  All waits are bounded; a wait that runs out sets the status word and the CTA drains to the
+// common exit where TMEM is released.
+#include <type_traits>
 
 #include "nmg_spmm_simt.cuh"
 #include "nmg_tc_common.cuh"
@@ -23,453 +30,612 @@
 namespace nmg {
 
 
+constexpr int FX_A_COLS = TC_BK / 2;  // TMEM columns of one A plane: 64 reduction elements, two per 32-bit column
+
 struct TcParams {
-    const uint16_t *pat;  // [nb][Kpn]
-    const void *nval[3];  // [nb][Kpn][n] 16-bit values; fp32 weights: the hi / mid / lo bf16 planes
     const void *bias;     // [out_feats] or NULL
+    const void *residual; // added after the activation, same orientation as the output, or NULL
+    int64_t ld_res;
+    int act;              // NMG_EPI_NONE / NMG_EPI_GELU applied to (product + bias)
     void *out;
+    const char *masks;    // forward: row masks [k-block][mask_rows][8 n bytes]
+    int64_t mask_rows;
     int64_t out_feats;    // M (forward) or K (transposed)
     int64_t red;          // reduction length: K (forward) or M (transposed)
-    int64_t ntok, ld_out, Kpn, nb;
+    int64_t ntok, ld_out;
     int out_token_major;  // 1: out[token][feature], 0: out[feature][token]
+    int out_vec;          // token-major 16-bit: rows are 4-byte aligned and hold an even count; feature-major: rows are 16-byte aligned
     int tiles_f, tiles_t; // output tiles along features / tokens
-    int ksplit;           // > 1: the reduction axis is cut into ksplit ranges, one CTA each; fp32 partial tiles go to `partial`
-    float *partial;       // [ksplit][tiles_f * 128][ld_partial] fp32, feature-major
-    int64_t ld_partial;
+    int bn;               // tokens per tile: a multiple of 32, at most 256 (96 for fp32)
+    int stages, slots;    // ring depths, from fx_plan
+    int ksplit;           // CTAs per tile = cluster size: each takes one range of the reduction axis
+    int exch_off;         // exchange area of the partial tiles: offset in shared memory; 0 = on top of the rings
+    int misc_off;         // selector table and barriers
+    uint32_t tmem_cols;
     int *status;
+};
+struct FxMaps {
+    CUtensorMap x[3];  // activation planes, box 64 x bn, 128-byte swizzle
+    CUtensorMap val;   // values [nb][Kpn * n]: box 128 bytes x 128/m row-blocks, 128-byte swizzle (forward), or 128 columns x 64/m (transposed)
+    CUtensorMap pat;   // transposed: pattern bytes [nb][Kpn], box 128 columns x 64/m row-blocks
 };
 
 // ---- weight-tile expansion ------------------------------------------------------------------------------
-// A column of a row-block is n values plus a pattern id; its dense form (m halfs, n of them non-zero) is a byte
-// permutation of the packed values and zero.  The per-pattern permutation selectors are tabulated once per CTA
-// in shared memory: sel[p][q] is the PRMT selector that turns (v0 | v1 << 16, 0) into (row 2q | row 2q+1 << 16).
-// Expansion is then M_/2 PRMTs per column, the tile is written with full-width, conflict-free stores, and no
-// separate clearing pass exists.
+// The A operand lives in TMEM (lane = tile row, 32-bit column = two neighbouring reduction elements), so a tile is expanded
+// in registers and never passes through shared memory: with the tile in swizzled shared memory its stores, the tensor core's
+// reads of it and the table look-ups took 576 of the SM's 128-byte shared-memory cycles per 64 reduction elements of a 2:4
+// weight.  One thread owns one tile row.
 //
-// Swizzled K-major tile: element (row, e) lives at row*128 + (((e >> 3) ^ (row & 7)) << 4) + (e & 7)*2.
-template <int M_> struct SelWords {  // the M_/2 16-bit selectors of one pattern, as 32-bit words
-    static constexpr int W = M_ / 4;
-    uint32_t w[W];
-};
-template <int M_> __device__ __forceinline__ SelWords<M_> load_sel(const uint16_t *sel, uint32_t p) {
-    SelWords<M_> r;
-    if constexpr (M_ == 4) r.w[0] = *reinterpret_cast<const uint32_t *>(sel + p * 2);
-    else if constexpr (M_ == 8) { const uint2 v = *reinterpret_cast<const uint2 *>(sel + p * 4); r.w[0] = v.x; r.w[1] = v.y; }
-    else { const uint4 v = *reinterpret_cast<const uint4 *>(sel + p * 8); r.w[0] = v.x; r.w[1] = v.y; r.w[2] = v.z; r.w[3] = v.w; }
+// Forward: the row is a weight row.  Its row masks say for every column whether the row holds the column's first (second)
+// kept value; the values are shared by the m rows of the block and arrive as broadcast reads.  An output word (two columns) is
+// the OR over the slots of (pair of values AND mask), and PRMT's sign mode spreads two mask bits over the halves of a word:
+// two (n = 1) or four (n = 2) instructions per word on the half-rate integer pipe, which is what bounds the expansion, and
+// the shift that brings a mask bit to the top of its byte runs on the multiply-add pipe.  Bit 8 j + q of a 32-column mask
+// word is column 4 q + j.
+__device__ __forceinline__ void split3_bits(float f, uint32_t (&x)[3]) {  // exact three-way bf16 split, as 16-bit patterns
+    const __nv_bfloat16 hi = __float2bfloat16_rn(f);
+    const float r1 = f - __bfloat162float(hi);
+    const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
+    x[0] = __bfloat16_as_ushort(hi);
+    x[1] = __bfloat16_as_ushort(mid);
+    x[2] = __bfloat16_as_ushort(__float2bfloat16_rn(r1 - __bfloat162float(mid)));
+}
+// two fp32 values -> one word of each bf16 plane
+__device__ __forceinline__ void split3_pair(float lo, float hi, uint32_t &w0, uint32_t &w1, uint32_t &w2) {
+    uint32_t a[3], b[3];
+    split3_bits(lo, a);
+    split3_bits(hi, b);
+    w0 = a[0] | (b[0] << 16); w1 = a[1] | (b[1] << 16); w2 = a[2] | (b[2] << 16);
+}
+
+// prmt with selector nibbles 8 + i: byte i's sign bit in all eight bits (__byte_perm knows no such selectors)
+__device__ __forceinline__ uint32_t spread_signs(uint32_t w, uint32_t sel) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, 0, %2;" : "=r"(r) : "r"(w), "r"(sel));
     return r;
 }
-// rows (2q, 2q+1) of the column whose packed values are vv
-template <int M_> __device__ __forceinline__ uint32_t expand_pair(const SelWords<M_> &s, uint32_t vv, int q) {
-    return __byte_perm(vv, 0u, (q & 1) ? (s.w[q >> 1] >> 16) : (s.w[q >> 1] & 0xffffu));
+// mask of columns 4 q + 2 i, 4 q + 2 i + 1 of a 32-column mask word: all ones in the half of every column whose bit is set
+__device__ __forceinline__ uint32_t pair_mask(uint32_t word, int q, int i) { return spread_signs(word << (7 - q), i ? 0xbbaau : 0x9988u); }
+
+// Offsets of the eight 16-byte pieces of this row-block's 128 bytes in a box of values (128-byte swizzle: piece ^ row-block)
+template <int M_> __device__ __forceinline__ void piece_offsets(int row, uint32_t (&off)[8]) {
+    const uint32_t rb = (uint32_t)(row / M_);
+#pragma unroll
+    for (int i = 0; i < 8; i++) off[i] = rb * 128u + (((uint32_t)i ^ rb) & 7u) * 16u;
 }
 
-// Forward: tile rows are weight rows feat0 .. feat0+127, tile columns are weight columns kb*64 .. +63.
-// A thread owns one 8-column chunk (16 bytes of every tile row) of one row-block: lane = (row-block & 3) * 8 + chunk,
-// warp w of the group takes row-blocks 4w .. 4w+3 (+16 per extra pass).  It loads the chunk's 8 pattern ids and
-// 8*n values with 16-byte loads, expands them with PRMTs and writes every row of the row-block with one 16-byte
-// store; the 8 lanes that share a row cover its 128 bytes, so stores are conflict-free.
-template <int N_, int M_> struct FwdRegs {
-    static constexpr int RB = TC_BM / M_;               // row-blocks per tile
-    static constexpr int PASSES = (RB + 15) / 16;       // 16 row-blocks per pass of the group's 4 warps
-    uint4 pat[PASSES];                                   // 8 pattern ids (16 bits each); .x = 0xffffffff marks "no row-block"
-    uint4 val[PASSES][N_];                               // 8 * n halfs
-};
-
-template <int N_, int M_>
-__device__ __forceinline__ void fetch_forward(FwdRegs<N_, M_> &t, const TcParams &prm, const void *plane, int64_t feat0, int64_t kb,
-                                              int gwarp, int lane) {
-    constexpr int RB = FwdRegs<N_, M_>::RB;
-    const uint16_t *nval = static_cast<const uint16_t *>(plane);
-    const int c8 = lane & 7;
-#pragma unroll
-    for (int i = 0; i < FwdRegs<N_, M_>::PASSES; i++) {
-        const int rbl = i * 16 + gwarp * 4 + (lane >> 3);
-        const int64_t mb = feat0 / M_ + rbl;
-        if (rbl < RB && mb < prm.nb) {
-            const int64_t e0 = mb * prm.Kpn + kb * TC_BK + c8 * 8;
-            t.pat[i] = __ldg(reinterpret_cast<const uint4 *>(prm.pat + e0));
-#pragma unroll
-            for (int q = 0; q < N_; q++) t.val[i][q] = __ldg(reinterpret_cast<const uint4 *>(nval + e0 * N_) + q);
-        } else {
-            t.pat[i] = make_uint4(0xffffffffu, 0, 0, 0);
-#pragma unroll
-            for (int q = 0; q < N_; q++) t.val[i][q] = make_uint4(0, 0, 0, 0);
-        }
+template <int N_, int M_, typename T, int PLANES>
+__device__ __forceinline__ void expand_forward(const char *vals, const char *masks, uint32_t a_tmem, int row, const uint32_t (&off)[8]) {
+    constexpr int BOX = (TC_BM / M_) * 128;
+    uint32_t mask[N_][2];  // 32 columns per word
+    if constexpr (N_ == 2) {
+        const uint4 k = *reinterpret_cast<const uint4 *>(masks + row * 16);
+        mask[0][0] = k.x; mask[0][1] = k.y; mask[N_ - 1][0] = k.z; mask[N_ - 1][1] = k.w;
+    } else {
+        const uint2 k = *reinterpret_cast<const uint2 *>(masks + row * 8);
+        mask[0][0] = k.x; mask[0][1] = k.y;
     }
-}
-
-template <int N_, int M_>
-__device__ __forceinline__ void write_forward(const FwdRegs<N_, M_> &t, char *a_tile, const uint16_t *sel, int gwarp, int lane) {
-    constexpr int C = (int)comb(N_, M_);
-    constexpr int RB = FwdRegs<N_, M_>::RB;
-    const int c8 = lane & 7;
+    auto piece = [&](int box, int i) { return *reinterpret_cast<const uint4 *>(vals + box * BOX + off[i]); };
 #pragma unroll
-    for (int i = 0; i < FwdRegs<N_, M_>::PASSES; i++) {
-        const int rbl = i * 16 + gwarp * 4 + (lane >> 3);
-        if (rbl >= RB) continue;
-        const int row0 = rbl * M_;
-        const bool live = t.pat[i].x != 0xffffffffu;
-        const uint32_t pw[4] = {t.pat[i].x, t.pat[i].y, t.pat[i].z, t.pat[i].w};
-        uint32_t pid[8];  // clamped pattern ids of the 8 columns
-        uint32_t v[8];    // packed values (slot 0 | slot 1 << 16) of the 8 columns
+    for (int h = 0; h < 2; h++) {
+        uint32_t w[PLANES][16];
+        if constexpr (PLANES == 1 && N_ == 1) {  // eight columns per piece
 #pragma unroll
-        for (int c = 0; c < 8; c++) pid[c] = min(live ? ((pw[c >> 1] >> ((c & 1) * 16)) & 0xffffu) : 0u, (uint32_t)(C - 1));
-        if (N_ == 2) {
-            const uint32_t a[8] = {t.val[i][0].x, t.val[i][0].y, t.val[i][0].z, t.val[i][0].w,
-                                   t.val[i][N_ - 1].x, t.val[i][N_ - 1].y, t.val[i][N_ - 1].z, t.val[i][N_ - 1].w};
+            for (int i = 0; i < 4; i++) {
+                const uint4 v = piece(0, h * 4 + i);
+                w[0][4 * i] = v.x & pair_mask(mask[0][h], 2 * i, 0);
+                w[0][4 * i + 1] = v.y & pair_mask(mask[0][h], 2 * i, 1);
+                w[0][4 * i + 2] = v.z & pair_mask(mask[0][h], 2 * i + 1, 0);
+                w[0][4 * i + 3] = v.w & pair_mask(mask[0][h], 2 * i + 1, 1);
+            }
+        } else if constexpr (PLANES == 1) {  // four columns: first values, second values of a pair, twice
 #pragma unroll
-            for (int c = 0; c < 8; c++) v[c] = a[c];
+            for (int q = 0; q < 8; q++) {
+                const uint4 v = piece(h, q);
+                w[0][2 * q] = (v.x & pair_mask(mask[0][h], q, 0)) | (v.y & pair_mask(mask[N_ - 1][h], q, 0));
+                w[0][2 * q + 1] = (v.z & pair_mask(mask[0][h], q, 1)) | (v.w & pair_mask(mask[N_ - 1][h], q, 1));
+            }
         } else {
-            const uint32_t a[4] = {t.val[i][0].x, t.val[i][0].y, t.val[i][0].z, t.val[i][0].w};
 #pragma unroll
-            for (int c = 0; c < 8; c++) v[c] = (a[c >> 1] >> ((c & 1) * 16)) & 0xffffu;
-        }
-        char *rowp = a_tile + row0 * 128;
-        const uint32_t cx = (uint32_t)((c8 ^ (row0 & 7)) << 4);  // chunk offset of row row0; row r adds (r - row0) under the xor
+            for (int p = 0; p < 16; p++) {  // pair by pair: n = 1 half a piece, n = 2 one piece (first values, second values)
+                uint32_t x[N_][3];
+                if constexpr (N_ == 1) {
+                    const float2 v = *reinterpret_cast<const float2 *>(vals + h * BOX + off[p >> 1] + (p & 1) * 8);
+                    split3_pair(v.x, v.y, x[0][0], x[0][1], x[0][2]);
+                } else {
+                    const uint4 v = piece(2 * h + (p >> 3), p & 7);
+                    split3_pair(__uint_as_float(v.x), __uint_as_float(v.y), x[0][0], x[0][1], x[0][2]);
+                    split3_pair(__uint_as_float(v.z), __uint_as_float(v.w), x[N_ - 1][0], x[N_ - 1][1], x[N_ - 1][2]);
+                }
+                const uint32_t m0 = pair_mask(mask[0][h], p >> 1, p & 1), m1 = N_ == 2 ? pair_mask(mask[N_ - 1][h], p >> 1, p & 1) : 0u;
 #pragma unroll
-        for (int w = 0; w < M_ / 4; w++) {  // one selector word (rows 4w .. 4w+3) at a time keeps the live registers few
-            uint32_t sw[8];
-#pragma unroll
-            for (int c = 0; c < 8; c++) sw[c] = *reinterpret_cast<const uint32_t *>(sel + pid[c] * (M_ / 2) + 2 * w);
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int q = 2 * w + h;
-                uint32_t e[8];  // rows (2q | 2q+1 << 16) of each column
-#pragma unroll
-                for (int c = 0; c < 8; c++) e[c] = live ? __byte_perm(v[c], 0u, h ? (sw[c] >> 16) : sw[c]) : 0u;
-                const uint4 lo = make_uint4(__byte_perm(e[0], e[1], 0x5410), __byte_perm(e[2], e[3], 0x5410),
-                                            __byte_perm(e[4], e[5], 0x5410), __byte_perm(e[6], e[7], 0x5410));
-                const uint4 hi = make_uint4(__byte_perm(e[0], e[1], 0x7632), __byte_perm(e[2], e[3], 0x7632),
-                                            __byte_perm(e[4], e[5], 0x7632), __byte_perm(e[6], e[7], 0x7632));
-                // row0 is a multiple of 4, so (row0 + k) & 7 == (row0 & 7) ^ k for k < 4, and for M_ >= 8 row0 & 7 == 0
-                *reinterpret_cast<uint4 *>(rowp + (2 * q) * 128 + (cx ^ (uint32_t)(((2 * q) & 7) << 4))) = lo;
-                *reinterpret_cast<uint4 *>(rowp + (2 * q + 1) * 128 + (cx ^ (uint32_t)(((2 * q + 1) & 7) << 4))) = hi;
+                for (int pl = 0; pl < PLANES; pl++) w[pl][p] = N_ == 2 ? ((x[0][pl] & m0) | (x[N_ - 1][pl] & m1)) : (x[0][pl] & m0);
             }
         }
+#pragma unroll
+        for (int pl = 0; pl < PLANES; pl++) tmem_st16(a_tmem + (uint32_t)(pl * FX_A_COLS + h * 16), w[pl]);
     }
 }
 
-// Transposed: tile rows are weight columns feat0 .. feat0+127 (one per thread of the group), the tile's K axis is
-// weight rows kb*64 .. +63, i.e. 64/m row-blocks whose expanded columns lie side by side in the thread's row.
-template <int N_, int M_> struct TrRegs {
-    static constexpr int E = TC_BK / M_;  // row-blocks per k-block
-    uint32_t pat[E];                       // 0xffffffff = row-block past the end of the weight
-    uint32_t val[E];                       // n <= 2 halfs
-};
-
-template <int N_, int M_>
-__device__ __forceinline__ void fetch_transposed(TrRegs<N_, M_> &t, const TcParams &prm, const void *plane, int64_t feat0, int64_t kb,
-                                                 int row) {
-    constexpr int E = TrRegs<N_, M_>::E;
-    const int64_t kg = feat0 + row;
-    const uint16_t *nval = static_cast<const uint16_t *>(plane);
-#pragma unroll
-    for (int j = 0; j < E; j++) {
-        const int64_t mb = kb * E + j;
-        t.pat[j] = 0xffffffffu;
-        t.val[j] = 0;
-        if (mb < prm.nb) {
-            const int64_t e = mb * prm.Kpn + kg;
-            t.pat[j] = __ldg(prm.pat + e);
-            if (N_ == 2) t.val[j] = __ldg(reinterpret_cast<const uint32_t *>(nval + e * 2));
-            else t.val[j] = __ldg(nval + e);
-        }
-    }
+// Transposed: the row is a weight column, the reduction runs over 64 weight rows = 64/m row-blocks.  A column of a row-block
+// is n values plus a pattern; its m rows (n of them non-zero) are a byte permutation of the packed values and zero.  The
+// permutation selectors of rows (2q, 2q+1) of every pattern are tabulated in shared memory, m/4 words per pattern, and the
+// pattern byte of the column-ordered copy is the offset of its entry.
+constexpr int FX_TABLE_BYTES = 256;
+template <int W> struct Words { uint32_t w[W]; };
+template <int W> __device__ __forceinline__ Words<W> lds_words(const char *p) {
+    Words<W> r;
+    if constexpr (W == 1) r.w[0] = *reinterpret_cast<const uint32_t *>(p);
+    else if constexpr (W == 2) { const uint2 v = *reinterpret_cast<const uint2 *>(p); r.w[0] = v.x; r.w[1] = v.y; }
+    else { const uint4 v = *reinterpret_cast<const uint4 *>(p); r.w[0] = v.x; r.w[1] = v.y; r.w[2] = v.z; r.w[3] = v.w; }
+    return r;
 }
-
-template <int N_, int M_>
-__device__ __forceinline__ void write_transposed(const TrRegs<N_, M_> &t, char *a_tile, const uint16_t *sel, int row) {
-    constexpr int C = (int)comb(N_, M_);
-    constexpr int E = TrRegs<N_, M_>::E;
-    constexpr int WPE = M_ / 2;  // 32-bit words per expanded column
-    uint32_t w[TC_BK / 2];       // the thread's whole tile row
-#pragma unroll
-    for (int j = 0; j < E; j++) {
-        const bool live = t.pat[j] != 0xffffffffu;
-        const SelWords<M_> s = load_sel<M_>(sel, min(t.pat[j], (uint32_t)(C - 1)));
-#pragma unroll
-        for (int q = 0; q < WPE; q++) w[j * WPE + q] = live ? expand_pair<M_>(s, t.val[j], q) : 0u;
-    }
-    char *rowp = a_tile + row * 128;
-#pragma unroll
-    for (int c = 0; c < 8; c++)
-        *reinterpret_cast<uint4 *>(rowp + (((c ^ row) & 7) << 4)) = make_uint4(w[4 * c], w[4 * c + 1], w[4 * c + 2], w[4 * c + 3]);
-}
-
-
-// ---- the kernel -------------------------------------------------------------------------------------------
-template <int N_, int M_, typename T, bool TRANSPOSED>
-__global__ void __launch_bounds__(TC_THREADS, 1)
-spmm_tc_kernel(const TcParams prm, const __grid_constant__ CUtensorMap tmap0, const __grid_constant__ CUtensorMap tmap1,
-               const __grid_constant__ CUtensorMap tmap2) {
-    constexpr int TERMS = TcMode<T>::TERMS;
-    using E = typename TcMode<T>::elem;  // element type the tensor cores see
-    static_assert((3 * TC_STAGES + 2) * 8 <= 120, "barriers overlap the TMEM slot");
-    static_assert(TC_BM % (4 * M_) == 0 && TC_BK % M_ == 0 && M_ % 4 == 0 && N_ <= 2, "tile must hold whole row-blocks; pattern rows are packed in 32 bits");
+template <int N_, int M_> __device__ __forceinline__ void build_table(char *table, int tid, int nthreads) {
     constexpr Order<N_, M_> ORD{};
     constexpr int C = Order<N_, M_>::C;
+    for (int e = tid; e < C * (M_ / 4); e += nthreads) {  // word e: rows 4q .. 4q+3 of pattern p
+        const int p = e / (M_ / 4), q = e - p * (M_ / 4);
+        uint32_t word = 0;
+        for (int r = 0; r < 4; r++) {
+            uint32_t nib = 0x44;  // byte 4 of (values, 0): zero
+            for (int sl = 0; sl < N_; sl++)
+                if (ORD.v[p * Order<N_, M_>::LD + sl] == 4 * q + r) nib = sl == 0 ? 0x10 : 0x32;
+            word |= nib << (8 * r);
+        }
+        reinterpret_cast<uint32_t *>(table)[e] = word;
+    }
+}
 
-    constexpr bool SPLIT = TERMS > 1;
-    constexpr int GROUPS = TcMode<T>::GROUPS;
-    constexpr uint32_t TMEM_COLS = SPLIT ? 2 * TC_ACC_COLS : TC_ACC_COLS;
+template <int N_, int M_, typename T, int PLANES>
+__device__ __forceinline__ void expand_transposed(const char *vals, const char *pats, const char *table, uint32_t a_tmem, int row) {
+    constexpr int W = M_ / 4, J = 32 / M_;  // row-blocks per 32 reduction elements
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        uint32_t w[PLANES][16];
+#pragma unroll
+        for (int jj = 0; jj < J; jj++) {
+            const int j = h * J + jj;
+            const Words<W> sw = lds_words<W>(table + *reinterpret_cast<const uint8_t *>(pats + j * TC_BM + row));
+            uint32_t v[PLANES];
+            if constexpr (N_ == 1) {
+                const char *src = vals + (j * TC_BM + row) * (int)sizeof(T);
+                if constexpr (PLANES == 1) v[0] = *reinterpret_cast<const uint16_t *>(src);
+                else split3_pair(*reinterpret_cast<const float *>(src), 0.f, v[0], v[1], v[2]);
+            } else {  // two columns' first values, then their second values
+                const char *src = vals + (j * TC_BM + (row & ~1)) * 2 * (int)sizeof(T);
+                if constexpr (PLANES == 1) {
+                    const uint2 a = *reinterpret_cast<const uint2 *>(src);
+                    v[0] = __byte_perm(a.x, a.y, (row & 1) ? 0x7632 : 0x5410);
+                } else {
+                    const float *f = reinterpret_cast<const float *>(src) + (row & 1);
+                    split3_pair(f[0], f[2], v[0], v[1], v[2]);
+                }
+            }
+#pragma unroll
+            for (int pl = 0; pl < PLANES; pl++)
+#pragma unroll
+                for (int q = 0; q < M_ / 2; q++) w[pl][jj * (M_ / 2) + q] = __byte_perm(v[pl], 0u, (q & 1) ? (sw.w[q >> 1] >> 16) : sw.w[q >> 1]);
+        }
+#pragma unroll
+        for (int pl = 0; pl < PLANES; pl++) tmem_st16(a_tmem + (uint32_t)(pl * FX_A_COLS + h * 16), w[pl]);
+    }
+}
+
+// ---- the kernel -------------------------------------------------------------------------------------------
+// Shared memory of one CTA: a ring of activation stages, a ring of slots for compressed weight tiles, the exchange area of the
+// partial tiles (on top of the rings when it does not fit beside them), the selector table and the barriers.
+constexpr int FX_GROUPS = 3;                       // expansion groups of four warps: warps 0 .. 11
+constexpr int FX_WARP_X = 12, FX_WARP_MMA = 13, FX_WARP_W = 14;  // activation loads, MMA issue (and TMEM), weight loads
+constexpr int FX_THREADS = 32 * 15;
+constexpr int FX_MAX_STAGES = 8, FX_MAX_SLOTS = 12;
+constexpr int FX_SMEM_LIMIT = 224 * 1024;
+constexpr int FX_MISC_BYTES = 512 + FX_TABLE_BYTES;
+struct FxPlan { int stages, slots, exch_off; uint32_t tmem_cols; size_t total; };
+__host__ __device__ constexpr int fx_slot_bytes(int n, int m, int es, bool transposed) {  // values, then masks (forward) or pattern bytes
+    return 128 * TC_BK / m * n * es + (transposed ? 128 * TC_BK / m : 128 * 8 * n);
+}
+// columns per CTA of a cluster in the exchange, a multiple of four.  The area is [source][4 columns][128 features][4]: a warp's
+// push is 512 consecutive bytes (16-byte pieces scattered over feature rows moved 16 bytes per clock), and so is its read.
+__host__ __device__ inline int fx_cols_per_owner(int bn, int ks) { return ((bn + ks - 1) / ks + 3) & ~3; }
+static FxPlan fx_plan(int planes, int bn, int ks, int slot_bytes) {
+    FxPlan p;
+    const int x_bytes = planes * bn * TC_BK * 2;
+    const int acc = planes > 1 ? 2 * bn : bn;  // fp32: accumulator and running tile
+    const int exch = ks > 1 ? ks * 128 * fx_cols_per_owner(bn, ks) * 4 : 0;
+    const int budget = FX_SMEM_LIMIT - FX_MISC_BYTES - 1024;
+    // A slot always serves the same group and stages are at least as many as groups: no barrier is waited on two phases ahead.
+    const int min_rings = FX_GROUPS * x_bytes + FX_GROUPS * slot_bytes;
+    const int room = exch + min_rings <= budget ? budget - exch : budget;
+    p.slots = 2 * FX_GROUPS;
+    while (p.slots > FX_GROUPS && FX_GROUPS * x_bytes + p.slots * slot_bytes > room) p.slots -= FX_GROUPS;
+    p.stages = (room - p.slots * slot_bytes) / x_bytes;
+    const int tmem_stages = (512 - acc) / (planes * FX_A_COLS);
+    if (p.stages > tmem_stages) p.stages = tmem_stages;
+    if (p.stages > FX_MAX_STAGES) p.stages = FX_MAX_STAGES;
+    while (p.slots + FX_GROUPS <= FX_MAX_SLOTS && p.stages * x_bytes + (p.slots + FX_GROUPS) * slot_bytes <= room) p.slots += FX_GROUPS;
+    const int rings = p.stages * x_bytes + p.slots * slot_bytes;
+    p.exch_off = (ks > 1 && room < budget) ? (rings + 1023) & ~1023 : 0;
+    const int used = p.exch_off ? p.exch_off + exch : (rings > exch ? rings : exch);
+    p.total = (size_t)((used + 255) & ~255) + FX_MISC_BYTES + 1024;
+    p.tmem_cols = 32;
+    while ((int)p.tmem_cols < acc + p.stages * planes * FX_A_COLS) p.tmem_cols *= 2;
+    return p;
+}
+
+// 16 bytes into a CTA of the cluster, counted by the mbarrier at `bar` in that CTA
+__device__ __forceinline__ void dsmem_push_v4(uint32_t cluster_addr, uint32_t bar, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%2, %3, %4, %5}, [%1];"
+                 ::"r"(cluster_addr), "r"(bar), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+// Epilogue of COLS neighbouring tokens of one feature per lane (a warp: 32 neighbouring features): bias, activation, residual,
+// conversion, store.  nt of the tokens exist.  All lanes of the warp call this.
+template <typename T, int COLS>
+__device__ __forceinline__ void finish_store(const TcParams &prm, uint32_t (&r)[COLS], int64_t feat, bool feat_ok, int64_t tokc, int nt, float b) {
+    T *out = static_cast<T *>(prm.out);
+    const T *res = static_cast<const T *>(prm.residual);
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < COLS; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) + b);
+    if (prm.act == NMG_EPI_GELU) {
+#pragma unroll
+        for (int j = 0; j < COLS; j++) r[j] = __float_as_uint(gelu_erf(__uint_as_float(r[j])));
+    }
+    if (res && feat_ok) {
+        const int64_t step = prm.out_token_major ? prm.ld_res : 1;
+        const T *src = prm.out_token_major ? res + tokc * prm.ld_res + feat : res + feat * prm.ld_res + tokc;
+#pragma unroll
+        for (int j = 0; j < COLS; j++)
+            if (j < nt) r[j] = __float_as_uint(__uint_as_float(r[j]) + DT<T>::to_f32(src[j * step]));
+    }
+    if (!prm.out_token_major) {
+        if (!feat_ok) return;
+        T *dst = out + feat * prm.ld_out + tokc;
+        if (nt >= COLS && prm.out_vec) {  // whole 8- or 16-byte stores
+            if constexpr (sizeof(T) == 4) {
+#pragma unroll
+                for (int v = 0; v < COLS / 4; v++) reinterpret_cast<uint4 *>(dst)[v] = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+            } else {
+#pragma unroll
+                for (int v = 0; v < COLS / 4; v++)
+                    reinterpret_cast<uint2 *>(dst)[v] = make_uint2(pack2<T>(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1])),
+                                                                  pack2<T>(__uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3])));
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < COLS; j++)
+                if (j < nt) dst[j] = DT<T>::from_f32(__uint_as_float(r[j]));
+        }
+        return;
+    }
+    if (sizeof(T) == 2 && prm.out_vec) {
+        // neighbouring lanes exchange one value so that each stores two neighbouring features of one token
+        const int odd = lane & 1;
+        T *dst = out + (tokc + odd) * prm.ld_out + (feat - odd);
+        const bool pair_ok = feat - odd < prm.out_feats;
+#pragma unroll
+        for (int j = 0; j < COLS; j += 2, dst += 2 * prm.ld_out) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, odd ? r[j] : r[j + 1], 1);
+            const uint32_t w = odd ? pack2<T>(__uint_as_float(got), __uint_as_float(r[j + 1])) : pack2<T>(__uint_as_float(r[j]), __uint_as_float(got));
+            if (j + odd < nt && pair_ok) *reinterpret_cast<uint32_t *>(dst) = w;
+        }
+        return;
+    }
+    if (feat_ok) {
+        T *dst = out + tokc * prm.ld_out + feat;
+#pragma unroll
+        for (int j = 0; j < COLS; j++, dst += prm.ld_out)
+            if (j < nt) *dst = DT<T>::from_f32(__uint_as_float(r[j]));
+    }
+}
+
+// One CTA computes 128 features x bn tokens over its range of the reduction axis; the `ksplit` CTAs of a cluster share the
+// tile and add their partial tiles through distributed shared memory, in the order of the ranges.
+template <int N_, int M_, typename T, bool TRANSPOSED>
+__global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams prm, const __grid_constant__ FxMaps maps) {
+    constexpr bool SPLIT = TcMode<T>::TERMS > 1;
+    constexpr int PLANES = SPLIT ? 3 : 1;
+    using E = typename TcMode<T>::elem;  // element type the tensor cores see
+    static_assert(TC_BM % M_ == 0 && 32 % M_ == 0 && M_ % 4 == 0 && N_ <= 2, "tile must hold whole row-blocks; a column's values fit one word");
+    static_assert(Order<N_, M_>::C * M_ <= FX_TABLE_BYTES, "a pattern byte is an offset into the selector table");
+    constexpr int SLOT_BYTES = fx_slot_bytes(N_, M_, (int)sizeof(T), TRANSPOSED), VAL_BYTES = 128 * TC_BK / M_ * N_ * (int)sizeof(T);
+    static_assert(TRANSPOSED || (SLOT_BYTES % 1024 == 0 && VAL_BYTES % 1024 == 0), "swizzled boxes start on 1024-byte boundaries");
 
     extern __shared__ char smem_raw[];
     char *smem = reinterpret_cast<char *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    char *a_stages = smem;
-    char *b_stages = smem + TC_STAGES * TC_A_BYTES;
-    char *misc = smem + TC_STAGES * (TC_A_BYTES + TC_B_BYTES);  // 1024-byte aligned: barriers first
-    uint64_t *full_a = reinterpret_cast<uint64_t *>(misc);
-    uint64_t *full_b = full_a + TC_STAGES;
-    uint64_t *empty = full_b + TC_STAGES;
-    uint64_t *chunk_done = empty + TC_STAGES;  // MMA -> promotion / epilogue: the accumulator tile is complete
-    uint64_t *promoted = chunk_done + 1;       // promotion -> MMA: the accumulator tile may be overwritten
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(misc + 120);
-    uint16_t *sel = reinterpret_cast<uint16_t *>(misc + 128);  // [C][M_/2] PRMT selectors, 16-byte aligned
+    const int bn = prm.bn, stages = prm.stages, slots = prm.slots;
+    const int b_bytes = bn * TC_BK * 2;
+    const int x_bytes = PLANES * b_bytes;
+    char *slot0 = smem + stages * x_bytes;  // 1024-byte aligned
+    char *table = smem + prm.misc_off;
+    char *misc = table + FX_TABLE_BYTES;
+    uint64_t *full = reinterpret_cast<uint64_t *>(misc);  // activation loads and the expansion group's four warps -> MMA
+    uint64_t *empty = full + FX_MAX_STAGES;
+    uint64_t *full_w = empty + FX_MAX_STAGES;      // weight loads -> expansion group
+    uint64_t *empty_w = full_w + FX_MAX_SLOTS;     // expansion group -> weight loads
+    uint64_t *chunk_done = empty_w + FX_MAX_SLOTS; // MMA -> promotion: the accumulator holds a finished chunk (fp32)
+    uint64_t *promoted = chunk_done + 1;           // promotion -> MMA: the accumulator may be overwritten
+    uint64_t *all_done = promoted + 1;             // MMA -> everyone: the tile is complete
+    uint64_t *exchanged = all_done + 1;            // partial tiles of this CTA's columns have arrived
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(misc + 496);
+    static_assert((2 * FX_MAX_STAGES + 2 * FX_MAX_SLOTS + 4) * 8 <= 496, "barriers overlap the TMEM slot");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // Few output tiles (few tokens): the grid is ksplit x tiles and every CTA takes one range of the reduction axis, so
-    // that the compressed weight streams from HBM through all SMs; a second kernel adds the partial tiles.
-    const int ntiles = prm.tiles_f * prm.tiles_t;
-    const int split = (int)blockIdx.x / ntiles;
+    const int ks = prm.ksplit;
+    const int split = ks > 1 ? (int)cluster_ctarank() : 0;
     int tile_f, tile_t;
-    tile_of_cta((int)blockIdx.x - split * ntiles, prm.tiles_f, prm.tiles_t, tile_f, tile_t);
-    const int64_t tok0 = (int64_t)tile_t * TC_BN;
+    tile_of_cta((int)blockIdx.x / ks, prm.tiles_f, prm.tiles_t, tile_f, tile_t);
+    const int64_t tok0 = (int64_t)tile_t * bn;
     const int64_t feat0 = (int64_t)tile_f * TC_BM;
     // 32-bit loop arithmetic throughout: the single MMA-issuing thread must stay ahead of the tensor core, and a
     // 64-bit division per iteration on that thread is enough to make issue the bottleneck.
-    const int nkb_all = (int)((prm.red + TC_BK - 1) / TC_BK) * TERMS;  // iterations: k-blocks x split terms (term fastest)
-    const int kb_per = (nkb_all + prm.ksplit - 1) / prm.ksplit;
-    const int kb_base = split * kb_per;                                 // this CTA's first iteration (0 unless ksplit > 1)
+    const int nkb_all = (int)((prm.red + TC_BK - 1) / TC_BK);
+    const int kb_per = (nkb_all + ks - 1) / ks;
+    const int kb_base = split * kb_per;  // this CTA's first k-block
     const int nkb = (nkb_all < kb_base + kb_per ? nkb_all : kb_base + kb_per) - kb_base;  // >= 1 by the host's choice of ksplit
-    const int chunk_it = SPLIT ? TC_CHUNK_KB * TERMS : nkb;          // iterations per accumulation chunk
-    const int nchunks = (nkb + chunk_it - 1) / chunk_it;
+    const int chunk_kb = SPLIT ? TC_CHUNK_KB : nkb;  // k-blocks per accumulation chunk
+    const int nchunks = (nkb + chunk_kb - 1) / chunk_kb;
+    const uint32_t tmem_cols = prm.tmem_cols;
+    const int cols_live = (int)(prm.ntok - tok0 < bn ? prm.ntok - tok0 : bn);  // token columns of this tile that exist
+    const int cpo = fx_cols_per_owner(bn, ks);                                    // columns each CTA of the cluster finishes
+    const bool exch_apart = ks > 1 && prm.exch_off != 0;
 
-    if (tid == 0) {
-        for (int s = 0; s < TC_STAGES; s++) {
-            mbar_init(&full_a[s], 128);
-            mbar_init(&full_b[s], 1);
-            mbar_init(&empty[s], 1);
+    // ---- loads, by the two producer warps
+    auto load_x = [&](int kb, int s) {
+        mbar_expect_tx(&full[s], (uint32_t)x_bytes);
+#pragma unroll
+        for (int pl = 0; pl < PLANES; pl++)
+            tma_load_2d(smem + s * x_bytes + pl * b_bytes, &maps.x[pl], (kb_base + kb) * TC_BK, (int)tok0, &full[s]);
+    };
+    auto load_w = [&](int kb, int s) {
+        mbar_expect_tx(&full_w[s], (uint32_t)SLOT_BYTES);
+        char *w = slot0 + s * SLOT_BYTES;
+        if constexpr (TRANSPOSED) {
+            const int y = (kb_base + kb) * (TC_BK / M_);
+            tma_load_2d(w, &maps.val, (int)feat0 * N_, y, &full_w[s]);
+            tma_load_2d(w + VAL_BYTES, &maps.pat, (int)feat0, y, &full_w[s]);
+        } else {
+            constexpr int BOXES = TC_BK * N_ * (int)sizeof(T) / 128, BOX_ELEMS = 128 / (int)sizeof(T);
+#pragma unroll
+            for (int bx = 0; bx < BOXES; bx++)
+                tma_load_2d(w + bx * (TC_BM / M_) * 128, &maps.val, (kb_base + kb) * TC_BK * N_ + bx * BOX_ELEMS, (int)(feat0 / M_), &full_w[s]);
+            bulk_load(w + VAL_BYTES, prm.masks + ((int64_t)(kb_base + kb) * prm.mask_rows + feat0) * (8 * N_), 128 * 8 * N_, &full_w[s]);
         }
-        mbar_init(chunk_done, 1);
-        mbar_init(promoted, 128);
-        mbar_fence_init();
-    }
-    for (int e = tid; e < C * (M_ / 2); e += TC_THREADS) {
-        // selector for rows (2q, 2q+1) of pattern p: bytes of slot 0 are 0,1, of slot 1 are 2,3, byte 4 is zero
-        const int p = e / (M_ / 2), q = e - p * (M_ / 2);
-        uint32_t code = 0;
-        for (int h = 0; h < 2; h++) {
-            uint32_t nib = 0x44;
-            for (int sl = 0; sl < N_; sl++)
-                if (ORD.v[p * Order<N_, M_>::LD + sl] == 2 * q + h) nib = sl == 0 ? 0x10 : 0x32;
-            code |= nib << (8 * h);
+    };
+    const int lead_x = nkb < 2 ? nkb : 2, lead_w = nkb < FX_GROUPS ? nkb : FX_GROUPS;  // loads issued before the set-up barrier
+
+    // ---- set-up.  The producers initialise their own barriers and issue every group's first loads before the CTA-wide barrier,
+    // so that their latency runs beside the TMEM allocation.
+    if (warp == FX_WARP_W) {
+        if (lane == 0) {
+            for (int s = 0; s < slots; s++) {
+                mbar_init(&full_w[s], 1);
+                mbar_init(&empty_w[s], 4);
+            }
+            mbar_fence_init();
         }
-        sel[e] = (uint16_t)code;
+        __syncwarp();
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // from here on other kernels' results may be read
+        if (elect_one())
+            for (int kb = 0; kb < lead_w; kb++) load_w(kb, kb);
+        __syncwarp();
+    } else if (warp == FX_WARP_X) {
+        if (lane == 0) {
+            for (int s = 0; s < stages; s++) {
+                mbar_init(&full[s], 5);
+                mbar_init(&empty[s], 1);
+            }
+            mbar_init(chunk_done, 1);
+            mbar_init(promoted, 128);
+            mbar_init(all_done, 1);
+            mbar_init(exchanged, 1);
+            mbar_fence_init();
+            if (ks > 1) {  // bytes this CTA will receive: 16 per feature, source and four live columns
+                int mine = cols_live - split * cpo;
+                mine = mine < 0 ? 0 : (mine < cpo ? mine : cpo);
+                mbar_expect_tx(exchanged, (uint32_t)(ks * 128 * 16 * ((mine + 3) / 4)));
+            }
+        }
+        __syncwarp();
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (elect_one())
+            for (int kb = 0; kb < lead_x; kb++) load_x(kb, kb);
+        __syncwarp();
+    } else {
+        if (warp == FX_WARP_MMA) tmem_alloc(tmem_slot, tmem_cols);
+        if (TRANSPOSED && warp < FX_WARP_X) build_table<N_, M_>(table, tid, FX_WARP_X * 32);
+        asm volatile("griddepcontrol.wait;" ::: "memory");
     }
-    if (warp == 1) tmem_alloc(tmem_slot, TMEM_COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    const uint32_t a_base = tmem_base + (uint32_t)(SPLIT ? 2 * bn : bn);  // A stages follow the accumulator (and the running tile)
+    // A partial tile is pushed into the other CTAs' shared memory: they must have started (waited for before the push).
+    __syncwarp();
+    if (exch_apart) cluster_arrive();
 
-    // Promotion + epilogue, run by four warps that together cover the 128 TMEM lanes.  For every finished chunk the
-    // accumulator tile is added to the running tile (columns 256..511) with round-to-nearest adds; the last chunk is
-    // added, biased, converted and stored to global memory instead.  16-bit mode has a single chunk.
-    // Bias, convert and store one 32-column slice (32 tokens) of this thread's feature row.
-    auto store_slice = [&](const uint32_t (&r)[32], int sl, int64_t feat, float b) {
-        T *out = static_cast<T *>(prm.out);
-        const int64_t tokc = tok0 + sl * 32;
-        const bool vec = !prm.out_token_major && tokc + 32 <= prm.ntok && (prm.ld_out % (16 / (int)sizeof(T))) == 0 &&
-                         (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-        if (vec) {  // 32 consecutive tokens of this feature: 16-byte stores
-            uint4 *dst = reinterpret_cast<uint4 *>(out + feat * prm.ld_out + tokc);
-            if constexpr (sizeof(T) == 4) {
-#pragma unroll
-                for (int v = 0; v < 8; v++)
-                    dst[v] = make_uint4(__float_as_uint(__uint_as_float(r[4 * v]) + b), __float_as_uint(__uint_as_float(r[4 * v + 1]) + b),
-                                        __float_as_uint(__uint_as_float(r[4 * v + 2]) + b), __float_as_uint(__uint_as_float(r[4 * v + 3]) + b));
-            } else {
-#pragma unroll
-                for (int v = 0; v < 4; v++) {
-                    uint32_t w[4];
-#pragma unroll
-                    for (int h = 0; h < 4; h++) {
-                        const T lo = DT<T>::from_f32(__uint_as_float(r[8 * v + 2 * h]) + b);
-                        const T hi = DT<T>::from_f32(__uint_as_float(r[8 * v + 2 * h + 1]) + b);
-                        w[h] = (uint32_t)bits16<T>(lo) | ((uint32_t)bits16<T>(hi) << 16);
-                    }
-                    dst[v] = make_uint4(w[0], w[1], w[2], w[3]);
-                }
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 32; j++) {
-                const int64_t tok = tokc + j;
-                if (tok < prm.ntok) {
-                    const T o = DT<T>::from_f32(__uint_as_float(r[j]) + b);
-                    if (prm.out_token_major) out[tok * prm.ld_out + feat] = o;
-                    else out[feat * prm.ld_out + tok] = o;
-                }
-            }
-        }
-    };
-
-    // 16-bit mode: one accumulation chunk, so the four draining warps only run the epilogue.
-    auto epilogue_once = [&]() {
-        if (!mbar_wait_bounded(chunk_done, 0, prm.status, 15)) return;
-        tc_fence_after();
-        const int q = warp & 3;  // TMEM lane quarter this warp may read
-        const int64_t feat = feat0 + q * 32 + lane;
-        const bool feat_ok = feat < prm.out_feats;
-        const float b = (prm.bias && feat_ok) ? DT<T>::to_f32(static_cast<const T *>(prm.bias)[feat]) : 0.f;
-        for (int sl = 0; sl < TC_BN / 32; sl++) {
-            uint32_t r[32];
-            tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(sl * 32), r);
-            if (tok0 + sl * 32 >= prm.ntok) continue;  // warp-uniform
-            if (prm.ksplit > 1) {  // raw fp32 partial sums; rows exist for every feature of the tile, ld_partial covers the slice
-                uint4 *dst = reinterpret_cast<uint4 *>(prm.partial + ((int64_t)split * prm.tiles_f * TC_BM + feat) * prm.ld_partial + tok0 + sl * 32);
-#pragma unroll
-                for (int v = 0; v < 8; v++) dst[v] = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
-                continue;
-            }
-            if (feat_ok) store_slice(r, sl, feat, b);
-        }
-        tc_fence_before();
-    };
-
-    // fp32 mode: for every finished chunk the accumulator tile is added to the running tile (columns 256..511) with
-    // round-to-nearest adds; the last chunk is added and stored to global memory instead.
-    auto drain_chunk = [&](int c) -> bool {
-        const int q = warp & 3;
-        const int64_t feat = feat0 + q * 32 + lane;
-        const bool feat_ok = feat < prm.out_feats;
-        const float b = (prm.bias && feat_ok) ? DT<T>::to_f32(static_cast<const T *>(prm.bias)[feat]) : 0.f;
-        const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
+    // fp32 mode: a finished chunk of the accumulator is added to the running tile (columns bn .. 2 bn) with round-to-nearest
+    // adds, by the four warps of group 0
+    auto promote_chunk = [&](int c) -> bool {
+        const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
         if (!mbar_wait_bounded(chunk_done, (uint32_t)(c & 1), prm.status, 15)) return false;
         tc_fence_after();
-        const bool last = c == nchunks - 1;
-        for (int sl = 0; sl < TC_BN / 32; sl++) {
+        for (int sl = 0; sl < bn / 32; sl++) {
             uint32_t r[32];
             tmem_ld32(lane_base + (uint32_t)(sl * 32), r);
             if (c > 0) {
                 uint32_t run[32];
-                tmem_ld32(lane_base + (uint32_t)(TC_ACC_COLS + sl * 32), run);
+                tmem_ld32(lane_base + (uint32_t)(bn + sl * 32), run);
 #pragma unroll
                 for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(run[j]), __uint_as_float(r[j])));
             }
-            if (!last) {
-                tmem_st32(lane_base + (uint32_t)(TC_ACC_COLS + sl * 32), r);
-                continue;
-            }
-            if (tok0 + sl * 32 < prm.ntok && feat_ok) store_slice(r, sl, feat, b);
+            tmem_st32(lane_base + (uint32_t)(bn + sl * 32), r);
         }
         tc_fence_before();
-        if (!last) mbar_arrive(promoted);
+        mbar_arrive(promoted);
         return true;
     };
 
-    if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer (one lane)
-        if (lane == 0) {
-            for (int kb = 0; kb < nkb; kb++) {
-                const int s = kb % TC_STAGES;
-                const uint32_t ph = (uint32_t)((kb / TC_STAGES) & 1);
-                if (!mbar_wait_bounded(&empty[s], ph ^ 1, prm.status, 11)) break;
-                mbar_expect_tx(&full_b[s], TC_B_BYTES);
-                const int xc = TERMS == 1 ? 0 : kSplitX[kb % TERMS];
-                const CUtensorMap *tm = xc == 0 ? &tmap0 : (xc == 1 ? &tmap1 : &tmap2);
-                tma_load_2d(b_stages + s * TC_B_BYTES, tm, ((kb_base + kb) / TERMS) * TC_BK, (int)tok0, &full_b[s]);
+    bool ok = true;
+    if (warp == FX_WARP_X || warp == FX_WARP_W) {
+        // ------------------------------------------------------------------ activation and compressed weight loads
+        const bool is_x = warp == FX_WARP_X;
+        const int ring = is_x ? stages : slots;
+        uint64_t *freed = is_x ? empty : empty_w;
+        int s = is_x ? lead_x : lead_w;
+        uint32_t ph = 1;
+        if (s >= ring) { s -= ring; ph ^= 1; }
+        for (int kb = is_x ? lead_x : lead_w; kb < nkb; kb++) {
+            ok = mbar_wait_bounded(&freed[s], ph, prm.status, is_x ? 11 : 18);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            if (elect_one()) {
+                if (is_x) load_x(kb, s);
+                else load_w(kb, s);
             }
+            __syncwarp();
+            if (++s == ring) { s = 0; ph ^= 1; }
         }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer (one lane)
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc<E>();
-            bool ok = true;
-            int chunk = 0, in_chunk = 0;  // position inside the accumulation chunk, kept without divisions
-            for (int kb = 0; kb < nkb && ok; kb++) {
-                const int s = kb % TC_STAGES;
-                const uint32_t ph = (uint32_t)((kb / TC_STAGES) & 1);
-                const bool first = in_chunk == 0;
-                if (first && chunk > 0) ok = mbar_wait_bounded(promoted, (uint32_t)((chunk - 1) & 1), prm.status, 16);
-                ok = ok && mbar_wait_bounded(&full_a[s], ph, prm.status, 12) && mbar_wait_bounded(&full_b[s], ph, prm.status, 13);
-                if (!ok) break;
-                tc_fence_after();
-                const uint64_t adesc = make_sw128_desc(smem_u32(a_stages + s * TC_A_BYTES));
-                const uint64_t bdesc = make_sw128_desc(smem_u32(b_stages + s * TC_B_BYTES));
+    } else if (warp == FX_WARP_MMA) {
+        // ------------------------------------------------------------------ MMA issuer
+        const uint32_t idesc = make_idesc<E>(bn);
+        const uint32_t d_tmem = __shfl_sync(0xffffffffu, tmem_base, 0), at_base = __shfl_sync(0xffffffffu, a_base, 0);
+        const uint64_t bdesc0 = make_sw128_desc(smem_u32(smem));
+        int s = 0, chunk = 0, in_chunk = 0;
+        uint32_t ph = 0;
+        for (int kb = 0; kb < nkb; kb++) {
+            const bool first = in_chunk == 0;
+            if (first && chunk > 0) ok = mbar_wait_bounded(promoted, (uint32_t)((chunk - 1) & 1), prm.status, 16);
+            ok = ok && mbar_wait_bounded(&full[s], ph, prm.status, 12);
+            if (!__all_sync(0xffffffffu, ok)) break;
+            tc_fence_after();
+            const bool chunk_end = in_chunk + 1 == chunk_kb && kb + 1 < nkb;
+            if (elect_one()) {
+                const uint32_t at0 = at_base + (uint32_t)(s * PLANES * FX_A_COLS);
+                const uint64_t bs = bdesc0 + (uint64_t)(uint32_t)(s * (x_bytes >> 4));
 #pragma unroll
-                for (int k = 0; k < TC_BK / 16; k++)  // 16 elements = 32 bytes = 2 descriptor units per step
-                    tc_mma_f16(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
-                tc_commit(&empty[s]);  // arrives when the MMAs above have read the stage
-                if (++in_chunk == chunk_it || kb + 1 == nkb) {
-                    tc_commit(chunk_done);
-                    in_chunk = 0;
-                    chunk++;
+                for (int t = 0; t < TcMode<T>::TERMS; t++) {
+                    const uint32_t at = at0 + (uint32_t)((SPLIT ? split_w(t) : 0) * FX_A_COLS);
+                    const uint64_t bt = bs + (uint64_t)(uint32_t)((SPLIT ? split_x(t) : 0) * (b_bytes >> 4));
+#pragma unroll
+                    for (int k = 0; k < TC_BK / 16; k++)  // 16 elements = 8 TMEM columns of A, 32 bytes = 2 descriptor units of B
+                        tc_mma_f16_ta(d_tmem, at + 8 * k, bt + 2 * k, idesc, (first && t == 0 && k == 0) ? 0u : 1u);
                 }
+                tc_commit(&empty[s]);  // arrives when the MMAs above have read the stage
+                if (chunk_end) tc_commit(chunk_done);
             }
-            if (!ok) tc_commit(chunk_done);  // error path: let the drain warps fall through their bounded wait sooner
+            __syncwarp();
+            in_chunk++;
+            if (chunk_end) {
+                in_chunk = 0;
+                chunk++;
+            }
+            if (++s == stages) { s = 0; ph ^= 1; }
         }
+        if (elect_one()) tc_commit(all_done);  // also on the error path: the others fall through their bounded waits sooner
+        __syncwarp();
     } else {
         // ------------------------------------------------------------------ expansion groups
-        const int group = (warp - 2) >> 2;
-        const int gwarp = (warp - 2) & 3;
-        const int gtid = tid - 64 - group * 128;
-        // Two register buffers in ping-pong: the global loads of the group's next tile are in flight while the
-        // current one is written, and nothing is copied between the buffers.
+        const int group = warp >> 2, gtid = tid & 127;
         int drained = 0;  // group 0: accumulation chunks already promoted
-        auto run_group = [&](auto fetch, auto write, auto &buf_a, auto &buf_b) {
-            auto publish = [&](int kb, auto &buf) -> bool {
-                const int s = kb % TC_STAGES;
-                const uint32_t ph = (uint32_t)((kb / TC_STAGES) & 1);
-                if (SPLIT && group == 0) {
-                    // Before feeding a later chunk, promote the finished ones: the MMAs of a chunk depend only on
-                    // tiles that are already published, so this wait cannot deadlock, and the MMA issuer needs
-                    // the promotion before it may restart the accumulator.
-                    while (drained < kb / chunk_it) {
-                        if (!drain_chunk(drained)) return false;
-                        drained++;
-                    }
+        int s = group, w = group;
+        uint32_t ph = 0, phw = 0;
+        const uint32_t a_lane = a_base + ((uint32_t)((warp & 3) * 32) << 16);
+        uint32_t off[8];
+        if constexpr (!TRANSPOSED) piece_offsets<M_>(gtid, off);
+        for (int kb = group; kb < nkb; kb += FX_GROUPS) {
+            if (SPLIT && group == 0) {
+                // Before feeding a later chunk, promote the finished ones: the MMAs of a chunk depend only on tiles that are
+                // already published, so this wait cannot deadlock, and the MMA issuer needs the promotion before it may
+                // restart the accumulator.
+                while (ok && drained < kb / chunk_kb) {
+                    ok = promote_chunk(drained);
+                    drained++;
                 }
-                if (!mbar_wait_bounded(&empty[s], ph ^ 1, prm.status, 14)) return false;
-                write(buf, a_stages + s * TC_A_BYTES);
-                fence_proxy_async_smem();  // generic-proxy stores -> visible to the tensor core's async-proxy reads
-                mbar_arrive(&full_a[s]);
-                return true;
-            };
-            if (group < nkb) fetch(buf_a, group);
-            for (int kb = group; kb < nkb; kb += 2 * GROUPS) {
-                if (kb + GROUPS < nkb) fetch(buf_b, kb + GROUPS);
-                if (!publish(kb, buf_a)) break;
-                if (kb + GROUPS >= nkb) break;
-                if (kb + 2 * GROUPS < nkb) fetch(buf_a, kb + 2 * GROUPS);
-                if (!publish(kb + GROUPS, buf_b)) break;
             }
-        };
-        if (TRANSPOSED) {
-            TrRegs<N_, M_> ra, rb;
-            run_group([&](TrRegs<N_, M_> &t, int it) {
-                          fetch_transposed<N_, M_>(t, prm, prm.nval[TERMS == 1 ? 0 : kSplitW[it % TERMS]], feat0, (kb_base + it) / TERMS, gtid);
-                      },
-                      [&](const TrRegs<N_, M_> &t, char *tile) { write_transposed<N_, M_>(t, tile, sel, gtid); }, ra, rb);
-        } else {
-            FwdRegs<N_, M_> ra, rb;
-            run_group([&](FwdRegs<N_, M_> &t, int it) {
-                          fetch_forward<N_, M_>(t, prm, prm.nval[TERMS == 1 ? 0 : kSplitW[it % TERMS]], feat0, (kb_base + it) / TERMS, gwarp, lane);
-                      },
-                      [&](const FwdRegs<N_, M_> &t, char *tile) { write_forward<N_, M_>(t, tile, sel, gwarp, lane); }, ra, rb);
+            ok = ok && mbar_wait_bounded(&full_w[w], phw, prm.status, 19) && mbar_wait_bounded(&empty[s], ph ^ 1, prm.status, 14);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc_fence_after();  // the MMAs that read this stage are done
+            const char *vals = slot0 + w * SLOT_BYTES;
+            const uint32_t a_tmem = a_lane + (uint32_t)(s * PLANES * FX_A_COLS);
+            if constexpr (TRANSPOSED) expand_transposed<N_, M_, T, PLANES>(vals, vals + VAL_BYTES, table, a_tmem, gtid);
+            else expand_forward<N_, M_, T, PLANES>(vals, vals + VAL_BYTES, a_tmem, gtid, off);
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&empty_w[w]);  // the slot has been read
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full[s]);
+            if ((s += FX_GROUPS) >= stages) { s -= stages; ph ^= 1; }
+            if ((w += FX_GROUPS) >= slots) { w -= slots; phw ^= 1; }
         }
-        if (group == 0) {
-            if constexpr (SPLIT) {
-                while (drained < nchunks && drain_chunk(drained)) drained++;  // remaining promotions, then the result
+        if (SPLIT && group == 0)
+            while (ok && drained < nchunks - 1) {  // the chunks behind the last tile this group published
+                ok = promote_chunk(drained);
+                drained++;
+            }
+        ok = mbar_wait_bounded(all_done, 0, prm.status, 17) && ok;
+    }
+    __syncwarp();
+    tc_fence_before();
+    if (exch_apart) cluster_wait();          // the other CTAs have started
+    else if (ks > 1) cluster_sync_all();     // every CTA's MMAs are done: shared memory of all of them is free for the exchange
+    if (SPLIT && nchunks > 1) __syncthreads();  // group 0's promotions, before everybody's reads of the running tile
+    tc_fence_after();
+
+    // ---- epilogue: warps 0 .. 11, each a quarter of the TMEM lanes and every third slice of 32 token columns
+    const int fl = tid & 127;                     // this thread's feature row of the tile (warps 0 .. 11)
+    const int64_t feat = feat0 + fl;
+    const bool feat_ok = warp < FX_WARP_X && feat < prm.out_feats;
+    const float bias = (prm.bias && feat_ok) ? DT<T>::to_f32(static_cast<const T *>(prm.bias)[feat]) : 0.f;
+    if (warp < FX_WARP_X) {
+        const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
+        const uint32_t exch = smem_u32(smem + prm.exch_off) + (uint32_t)(split * cpo * 128 * 4 + fl * 16), bar = smem_u32(exchanged);
+        const uint32_t inv_cpo = 65536u / (uint32_t)cpo + 1u;
+        for (int sl = warp >> 2; sl * 32 < cols_live; sl += FX_GROUPS) {
+            uint32_t r[32];
+            __syncwarp();
+            tmem_ld32(lane_base + (uint32_t)(sl * 32), r);
+            if (SPLIT && nchunks > 1) {
+                uint32_t run[32];
+                tmem_ld32(lane_base + (uint32_t)(bn + sl * 32), run);
+#pragma unroll
+                for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(run[j]), __uint_as_float(r[j])));
+            }
+            if (ks > 1) {
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {  // cpo is a multiple of four: four columns have one owner
+                    const uint32_t col = (uint32_t)(sl * 32 + j), owner = (col * inv_cpo) >> 16;
+                    if ((int)col < cols_live)
+                        dsmem_push_v4(map_to_rank(exch + (col - owner * (uint32_t)cpo) * 512u, owner), map_to_rank(bar, owner), r[j], r[j + 1], r[j + 2], r[j + 3]);
+                }
             } else {
-                epilogue_once();
+                finish_store<T, 32>(prm, r, feat, feat_ok, tok0 + sl * 32, cols_live - sl * 32, bias);
+            }
+        }
+    }
+    if (ks > 1 && warp < FX_WARP_X) {
+        const int c0 = split * cpo;
+        const int ncols = cols_live - c0 < cpo ? cols_live - c0 : cpo;  // may be <= 0
+        ok = mbar_wait_cluster_bounded(exchanged, 0, prm.status, 20);
+        if (__all_sync(0xffffffffu, ok)) {
+            const char *src = smem + prm.exch_off + fl * 16;
+            for (int c = (warp >> 2) * 4; c < ncols; c += 4 * FX_GROUPS) {
+                float4 acc = *reinterpret_cast<const float4 *>(src + c * 512);
+                for (int s = 1; s < ks; s++) {  // in the order of the ranges
+                    const float4 v = *reinterpret_cast<const float4 *>(src + (s * cpo + c) * 512);
+                    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+                }
+                uint32_t r[4] = {__float_as_uint(acc.x), __float_as_uint(acc.y), __float_as_uint(acc.z), __float_as_uint(acc.w)};
+                finish_store<T, 4>(prm, r, feat, feat_ok, tok0 + c0 + c, ncols - c, bias);
             }
         }
     }
     __syncthreads();
-    if (warp == 1) {
+    if (warp == FX_WARP_MMA) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, TMEM_COLS);
+        tmem_dealloc(tmem_base, tmem_cols);
     }
 }
 
@@ -480,8 +646,44 @@ bool tc_supported(const Geo &geo, int dtype) {
            (geo.n == 1 && geo.m == 16);
 }
 
-static size_t tc_smem_bytes(int C) {
-    return (size_t)TC_STAGES * (TC_A_BYTES + TC_B_BYTES) + 128 + (size_t)C * 16 + 1024;
+// Tile width and cluster size: the pair with the smallest estimate of a CTA's time, from what the parts of the kernel measure
+// on a B200 (timestamps inside the kernel, 2:4 weights, ns):
+//   per k-block of 64: 300, the expansion and the issue of its MMAs (three planes in fp32: 900); above 192 tokens the MMAs
+//     themselves (2 clocks per token)
+//   per 32-column slice a warp finishes: 450
+//   exchange between ks CTAs: 900 for its barriers, 17 per column for the distributed-shared-memory traffic, 27 per column
+//     finished (bn / ks of them)
+// The token axis is cut into equal tiles, so that a batch just above a multiple does not pay for a nearly empty one.
+// A grid that does not fit the chip at once runs in waves; kFxClusters is what fits (cudaOccupancyMaxActiveClusters: the GPCs
+// are not all alike, 24 clusters of 6 do not fit although 144 < 148).
+constexpr int kFxClusters[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+struct FxChoice { int bn, tiles_f, tiles_t, ksplit; };
+static FxChoice fx_choose(int64_t feats, int64_t red, int64_t tokens, int dtype) {
+    const int max_bn = dtype == NMG_F32 ? 96 : 256;  // fp32: three stages of three A planes, the accumulator and the running tile share TMEM
+    const int64_t tiles_f = (feats + TC_BM - 1) / TC_BM, nkb = (red + TC_BK - 1) / TC_BK;
+    FxChoice best{};
+    int64_t best_ns = -1;
+    for (int64_t cap = 32; cap <= max_bn; cap += 32) {
+        const int64_t parts = (tokens + cap - 1) / cap;
+        const int bn = (int)round_up((tokens + parts - 1) / parts, 32);
+        if (bn != cap) continue;
+        const int64_t tiles_t = (tokens + bn - 1) / bn, tiles = tiles_f * tiles_t;
+        for (int want = 1; want <= 8; want++) {  // 8: the portable cluster size
+            if (want > 1 && want > nkb / 2) break;
+            const int64_t per = (nkb + want - 1) / want;
+            const int ks = (int)((nkb + per - 1) / per);  // every range non-empty
+            const int64_t waves = (tiles + kFxClusters[ks] - 1) / kFxClusters[ks];
+            int64_t ns = 3000 + per * (dtype == NMG_F32 ? 900 : bn > 192 ? 300 + (bn - 192) : 300);
+            if (ks > 1) ns += 900 + bn * 17 + bn * 27 / ks;
+            else ns += (bn / 32 + 2) / 3 * 450;
+            ns *= waves;
+            if (best_ns < 0 || ns < best_ns) {
+                best_ns = ns;
+                best = FxChoice{bn, (int)tiles_f, (int)tiles_t, ks};
+            }
+        }
+    }
+    return best;
 }
 
 // ---- fp32 activations: three bf16 planes [3][rows][ldp], written by one elementwise pass ---------------------------
@@ -519,62 +721,6 @@ __global__ void __launch_bounds__(128) split_f32_kernel(const float *__restrict_
     }
 }
 
-// ---- split-K of the fused kernel for few output tiles ----------------------------------------------------------------
-// Policy (pure arithmetic, so that workspace queries need no device): with fewer output tiles than half the SMs of a
-// B200 the reduction axis is cut so that about one CTA per SM runs, every range keeping at least four k-blocks.
-constexpr int TC_POLICY_SMS = 148;
-int tc_ksplit(const Geo &geo, int dtype, bool transposed, int64_t tokens) {
-    if (dtype == NMG_F32) return 1;  // fp32 mode accumulates in promoted chunks inside one CTA
-    const int64_t feats = transposed ? geo.K : geo.M, red = transposed ? geo.M : geo.K;
-    const int64_t tiles = ((feats + TC_BM - 1) / TC_BM) * ((tokens + TC_BN - 1) / TC_BN);
-    const int64_t nkb = (red + TC_BK - 1) / TC_BK;
-    if (tiles * 2 > TC_POLICY_SMS || nkb < 8) return 1;
-    int64_t want = TC_POLICY_SMS / tiles;
-    if (want > nkb / 4) want = nkb / 4;
-    if (want > 32) want = 32;
-    if (want < 2) return 1;
-    const int64_t per = (nkb + want - 1) / want;
-    return (int)((nkb + per - 1) / per);  // every range non-empty
-}
-size_t tc_ksplit_workspace_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens) {
-    const int ks = tc_ksplit(geo, dtype, transposed, tokens);
-    if (ks <= 1) return 0;
-    const int64_t feats = transposed ? geo.K : geo.M;
-    return (size_t)ks * (size_t)round_up(feats, TC_BM) * (size_t)round_up(tokens, TC_BN) * 4 + 512;
-}
-
-// out = sum over the ranges of partial[s] (+ bias), converted; 32 x 32 tiles through shared memory so that both the reads
-// (tokens contiguous) and token-major writes (features contiguous) are coalesced.  Ranges are added in a fixed order.
-template <typename T>
-__global__ void __launch_bounds__(256) splitk_reduce_kernel(const float *__restrict__ partial, int ksplit, int64_t plane, int64_t ldp,
-                                                            int64_t feats, int64_t ntok, const T *__restrict__ bias, T *__restrict__ out,
-                                                            int64_t ld_out, int token_major) {
-    __shared__ float tile[32][33];
-    const int64_t f0 = (int64_t)blockIdx.y * 32, t0 = (int64_t)blockIdx.x * 32;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (int r = ty; r < 32; r += 8) {
-        const int64_t f = f0 + r, t = t0 + tx;
-        float acc = 0.f;
-        if (f < feats && t < ntok) {
-            for (int s = 0; s < ksplit; s++) acc += partial[s * plane + f * ldp + t];
-            if (bias) acc += DT<T>::to_f32(bias[f]);
-        }
-        tile[r][tx] = acc;
-    }
-    __syncthreads();
-    if (token_major) {
-        for (int r = ty; r < 32; r += 8) {  // r = token, tx = feature
-            const int64_t t = t0 + r, f = f0 + tx;
-            if (f < feats && t < ntok) out[t * ld_out + f] = DT<T>::from_f32(tile[tx][r]);
-        }
-    } else {
-        for (int r = ty; r < 32; r += 8) {
-            const int64_t f = f0 + r, t = t0 + tx;
-            if (f < feats && t < ntok) out[f * ld_out + t] = DT<T>::from_f32(tile[r][tx]);
-        }
-    }
-}
-
 size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens) {
     if (dtype != NMG_F32) return 0;
     const int64_t red = transposed ? geo.M : geo.K;
@@ -582,22 +728,40 @@ size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, int6
 }
 
 template <int N_, int M_, typename T, bool TR>
-static int tc_launch_one(const TcParams &p, const CUtensorMap *tm, cudaStream_t st) {
-    const size_t smem = tc_smem_bytes((int)comb(N_, M_));
+static int tc_launch_one(const TcParams &p0, const FxMaps &maps, cudaStream_t st) {
+    const FxPlan plan = fx_plan(TcMode<T>::TERMS > 1 ? 3 : 1, p0.bn, p0.ksplit, fx_slot_bytes(N_, M_, (int)sizeof(T), TR));
+    TcParams p = p0;
+    p.stages = plan.stages;
+    p.slots = plan.slots;
+    p.exch_off = plan.exch_off;
+    p.tmem_cols = plan.tmem_cols;
+    p.misc_off = (int)(plan.total - 1024 - FX_MISC_BYTES);
     const int64_t ctas = (int64_t)p.tiles_f * p.tiles_t * p.ksplit;
     if (ctas > 0x7fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many output tiles for one launch");
-    dim3 grid((unsigned)ctas);
-    NMG_ALLOW_SMEM(smem, spmm_tc_kernel<N_, M_, T, TR>);
-    spmm_tc_kernel<N_, M_, T, TR><<<grid, TC_THREADS, smem, st>>>(p, tm[0], tm[1], tm[2]);
-    NMG_CUDA(cudaGetLastError());
+    NMG_ALLOW_SMEM(plan.total, spmm_tc_kernel<N_, M_, T, TR>);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)ctas);
+    cfg.blockDim = dim3(FX_THREADS);
+    cfg.dynamicSmemBytes = plan.total;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // the set-up overlaps the preceding kernel's end
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = (unsigned)p.ksplit;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = p.ksplit > 1 ? 2 : 1;
+    NMG_CUDA(cudaLaunchKernelEx(&cfg, spmm_tc_kernel<N_, M_, T, TR>, p, maps));
     return NMG_OK;
 }
 
 template <int N_, int M_>
-static int tc_launch_nm(int dtype, bool transposed, const TcParams &p, const CUtensorMap *tm, cudaStream_t st) {
-    if (dtype == NMG_F16) return transposed ? tc_launch_one<N_, M_, __half, true>(p, tm, st) : tc_launch_one<N_, M_, __half, false>(p, tm, st);
-    if (dtype == NMG_F32) return transposed ? tc_launch_one<N_, M_, float, true>(p, tm, st) : tc_launch_one<N_, M_, float, false>(p, tm, st);
-    return transposed ? tc_launch_one<N_, M_, __nv_bfloat16, true>(p, tm, st) : tc_launch_one<N_, M_, __nv_bfloat16, false>(p, tm, st);
+static int tc_launch_nm(int dtype, bool transposed, const TcParams &p, const FxMaps &maps, cudaStream_t st) {
+    if (dtype == NMG_F16) return transposed ? tc_launch_one<N_, M_, __half, true>(p, maps, st) : tc_launch_one<N_, M_, __half, false>(p, maps, st);
+    if (dtype == NMG_F32) return transposed ? tc_launch_one<N_, M_, float, true>(p, maps, st) : tc_launch_one<N_, M_, float, false>(p, maps, st);
+    return transposed ? tc_launch_one<N_, M_, __nv_bfloat16, true>(p, maps, st) : tc_launch_one<N_, M_, __nv_bfloat16, false>(p, maps, st);
 }
 
 // Policy of the two tensor-core variants.
@@ -612,17 +776,18 @@ bool tc_use_dense(const Geo &geo, int dtype, int64_t tokens) {
 }
 
 // act: [tokens][ld_act] with the reduction axis contiguous (X for the forward, dY for the transposed product).
-int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void *val, const int16_t *idx, const uint16_t *pat,
+int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void *val, const int16_t *idx, const void *pat,
               const void *nval, const void *act, int64_t ld_act, int64_t tokens, const void *bias, void *const *outs, int n_outs,
               void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi) {
     if (n_outs < 1 || (n_outs > 1 && !dense)) NMG_FAIL(NMG_ERR_UNSUPPORTED, "several output buffers need the two-pass tensor-core variant");
     void *out = outs[0];
     const int64_t red = transposed ? geo.M : geo.K;
     // the two-pass variant on CTA pairs loads the activation tile in two halves of 128 tokens
-    const uint32_t box_tok = (dense && tc_dense_uses_pair(geo, dtype, transposed)) ? 128 : TC_BN;
+    const int64_t feats = transposed ? geo.K : geo.M;
+    const FxChoice fx = fx_choose(feats, red, tokens, dtype);
+    const uint32_t box_tok = dense ? (tc_dense_uses_pair(geo, dtype, transposed) ? 128 : TC_BN) : (uint32_t)fx.bn;
     CUtensorMap tm[3];
     int rc;
-    const void *planes[3] = {nval, nval, nval};
     if (dtype == NMG_F32) {
         const size_t need = tc_split_workspace_bytes(geo, dtype, transposed, tokens);
         if (!ws || ws_bytes < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the split activation, got %zu", need, ws_bytes);
@@ -639,10 +804,6 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
         NMG_CUDA(cudaGetLastError());
         for (int c = 0; c < 3; c++)
             if ((rc = encode_tmap_2d(&tm[c], NMG_BF16, xs + c * plane_elems, (uint64_t)red, (uint64_t)tokens, (uint64_t)ldp, TC_BK, box_tok, 1))) return rc;
-        if (!dense) {
-            const NaturalLayout lay = natural_layout(geo, dtype);
-            for (int c = 0; c < 3; c++) planes[c] = static_cast<const char *>(nval) + lay.val_bytes + c * lay.plane_bytes;
-        }
         ws = static_cast<char *>(ws) + need;  // what follows the split activation is free for the expanded weight
         ws_bytes -= need;
     } else {
@@ -659,29 +820,35 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     }
     int *status = nullptr;
     if ((rc = get_status_word(&status))) return rc;
-    const int64_t feats = transposed ? geo.K : geo.M;
-    const int64_t ftile = TC_BM;
-    TcParams p{};
-    p.pat = pat;
-    for (int c = 0; c < 3; c++) p.nval[c] = planes[c];
-    p.bias = bias; p.out = out; p.out_feats = feats; p.red = red; p.ntok = tokens; p.ld_out = ld_out;
-    p.Kpn = natural_width(geo); p.nb = geo.nb; p.out_token_major = out_token_major;
-    p.tiles_f = (int)((feats + ftile - 1) / ftile);
-    p.tiles_t = (int)((tokens + TC_BN - 1) / TC_BN);
-    p.status = status;
-    p.ksplit = tc_ksplit(geo, dtype, transposed, tokens);
-    if (p.ksplit > 1) {
-        const size_t need = tc_ksplit_workspace_bytes(geo, dtype, transposed, tokens);
-        if (!ws || ws_bytes < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the partial tiles, got %zu", need, ws_bytes);
-        p.partial = reinterpret_cast<float *>(((uintptr_t)ws + 255) & ~(uintptr_t)255);
-        p.ld_partial = (int64_t)p.tiles_t * TC_BN;
+    const size_t es = dtype_size(dtype);
+    FxMaps maps;
+    for (int c = 0; c < 3; c++) maps.x[c] = tm[c];
+    const int64_t Kpn = natural_width(geo);
+    const char *masks = static_cast<const char *>(nval) + natural_layout(geo, dtype).val_bytes;
+    if (transposed) {
+        if ((rc = encode_tmap_2d_bytes(&maps.pat, pat, (uint64_t)Kpn, (uint64_t)geo.nb, (uint64_t)Kpn, TC_BM, (uint32_t)(TC_BK / geo.m)))) return rc;
+        if ((rc = encode_tmap_2d(&maps.val, dtype, nval, (uint64_t)(Kpn * geo.n), (uint64_t)geo.nb, (uint64_t)(Kpn * geo.n), (uint32_t)(TC_BM * geo.n), (uint32_t)(TC_BK / geo.m), 0)))
+            return rc;
+    } else {
+        if ((rc = encode_tmap_2d(&maps.val, dtype, nval, (uint64_t)(Kpn * geo.n), (uint64_t)geo.nb, (uint64_t)(Kpn * geo.n), (uint32_t)(128 / dtype_size(dtype)), (uint32_t)(TC_BM / geo.m), 1)))
+            return rc;
+        maps.pat = maps.val;  // never used; keeps the parameter defined
     }
+    TcParams p{};
+    p.bias = bias; p.out = out; p.out_feats = feats; p.red = red; p.ntok = tokens; p.ld_out = ld_out;
+    p.residual = epi.residual; p.ld_res = epi.ld_res; p.act = epi.act;
+    p.out_token_major = out_token_major;
+    p.out_vec = out_token_major ? (ld_out % 2 == 0 && feats % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0)
+                                : (ld_out * es % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0);
+    p.tiles_f = fx.tiles_f; p.tiles_t = fx.tiles_t; p.bn = fx.bn; p.ksplit = fx.ksplit;
+    p.masks = masks; p.mask_rows = natural_mask_rows(geo);
+    p.status = status;
     const ProfileEvents pe = take_profile_events();
     if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));
     rc = NMG_ERR_UNSUPPORTED;
 #define NMG_TC_CASE(N_, M_)                                                                         \
     if (geo.n == N_ && geo.m == M_)                                                                \
-        rc = tc_launch_nm<N_, M_>(dtype, transposed, p, tm, st);
+        rc = tc_launch_nm<N_, M_>(dtype, transposed, p, maps, st);
     NMG_TC_CASE(1, 4)
     NMG_TC_CASE(2, 4)
     NMG_TC_CASE(1, 8)
@@ -689,23 +856,6 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     NMG_TC_CASE(1, 16)
 #undef NMG_TC_CASE
     if (rc == NMG_ERR_UNSUPPORTED) set_error("no tensor-core kernel for %d:%d", geo.n, geo.m);
-    if (rc == NMG_OK && p.ksplit > 1) {
-        const int64_t plane = (int64_t)p.tiles_f * TC_BM * p.ld_partial;
-        dim3 grid((unsigned)((tokens + 31) / 32), (unsigned)((feats + 31) / 32));
-        if (grid.y > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many output features for the split-K reduction");
-        if (dtype == NMG_F16)
-            splitk_reduce_kernel<__half><<<grid, 256, 0, st>>>(p.partial, p.ksplit, plane, p.ld_partial, feats, tokens, static_cast<const __half *>(bias),
-                                                                static_cast<__half *>(out), ld_out, out_token_major);
-        else
-            splitk_reduce_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>(p.partial, p.ksplit, plane, p.ld_partial, feats, tokens,
-                                                                       static_cast<const __nv_bfloat16 *>(bias), static_cast<__nv_bfloat16 *>(out), ld_out,
-                                                                       out_token_major);
-        NMG_CUDA(cudaGetLastError());
-    }
-    if (rc == NMG_OK && epi.any()) {
-        const int64_t feats_out = transposed ? geo.K : geo.M;
-        rc = out_token_major ? launch_epilogue(dtype, out, tokens, feats_out, ld_out, epi, st) : launch_epilogue(dtype, out, feats_out, tokens, ld_out, epi, st);
-    }
     if (rc == NMG_OK && pe.stop) NMG_CUDA(cudaEventRecord(pe.stop, st));
     return rc;
 }

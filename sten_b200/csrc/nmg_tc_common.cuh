@@ -9,7 +9,6 @@ constexpr int TC_BM = 128;    // output features per CTA (MMA M)
 constexpr int TC_BN = 256;    // tokens per CTA (MMA N)
 constexpr int TC_BK = 64;     // reduction elements per stage: one 128-byte swizzle span of 16-bit data
 constexpr int TC_STAGES = 4;
-constexpr int TC_THREADS = 32 * 14;  // fused kernel: TMA warp, MMA warp, three expansion groups of 4 warps (group 0 also drains)
 constexpr int TC_CHUNK_KB = 8;       // fp32 mode: k-blocks (of 64) accumulated in the tensor core before promotion
 constexpr int TC_A_BYTES = TC_BM * TC_BK * 2;  // 16 KB
 constexpr int TC_B_BYTES = TC_BN * TC_BK * 2;  // 32 KB
@@ -31,6 +30,14 @@ __device__ __forceinline__ void tile_of_cta(int lin, int tiles_f, int tiles_t, i
 }
 
 
+// One lane of a converged warp.  The issuing warps run their loops with all lanes and issue under this predicate: their operands
+// then stay in uniform registers, which is where the tensor-core instructions want them.  Under `if (lane == 0)` every operand
+// is moved over per instruction, and a step of four MMAs took 460 ns whatever its width.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
+}
 __device__ __forceinline__ void tmem_alloc(uint32_t *smem_slot, uint32_t cols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_slot)), "r"(cols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -49,6 +56,15 @@ __device__ __forceinline__ void tc_mma_f16(uint32_t d_tmem, uint64_t adesc, uint
         "setp.ne.b32 p, %4, 0;\n\t"
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// the A operand in TMEM: lane = row, 32-bit column = two neighbouring reduction elements
+__device__ __forceinline__ void tc_mma_f16_ta(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -98,6 +114,14 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
         : "memory");
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {  // completion: tmem_wait_st
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+          "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 // One 16-byte store to a multicast address: NVSwitch writes it to the same offset on every GPU of the multicast group.
 __device__ __forceinline__ void multimem_st_v4(void *mc_addr, uint4 v) {
     asm volatile("multimem.st.weak.global.v4.f32 [%0], {%1, %2, %3, %4};"
@@ -119,6 +143,9 @@ __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// the two halves of the cluster barrier, for a rendezvous that is only waited for later
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 // shared::cluster address of `local` (a shared::cta address of this CTA) in the CTA with the given cluster rank
 __device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
     uint32_t r;
@@ -190,9 +217,9 @@ __device__ __forceinline__ uint64_t make_sw128_desc(uint32_t smem_addr) {
 }
 // Instruction descriptor (kind::f16): D = fp32 (bits 4-5 = 1), A / B format (7-9, 10-12: 0 = f16, 1 = bf16), both
 // K-major (15, 16 = 0), N >> 3 (17-22), M >> 4 (24-28).
-template <typename T> __device__ __forceinline__ uint32_t make_idesc() {
+template <typename T> __device__ __forceinline__ uint32_t make_idesc(int n_cols = TC_BN) {
     const uint32_t fmt = sizeof(T) == 2 && DT<T>::id == NMG_BF16 ? 1u : 0u;
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(TC_BN >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+    return (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(n_cols >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
 }
 
 // Two fp32 values -> two 16-bit values in one word (first in the low half) with one packed conversion.
@@ -213,6 +240,20 @@ template <> __device__ __forceinline__ uint16_t bits16<__nv_bfloat16>(__nv_bfloa
 template <> __device__ __forceinline__ uint16_t bits16<float>(float) { return 0; }  // never used: fp32 outputs are stored as words
 
 
+// Exact (erf) GELU with a short erf: erf(x) = 1 - (a1 t + ... + a5 t^5) exp(-x^2), t = 1 / (1 + p x) for x >= 0 (Abramowitz &
+// Stegun 7.1.26, absolute error 1.5e-7, i.e. below fp32 rounding of the result for |v| of order one).  With x = |v| / sqrt(2)
+// and v * sign(v) = |v|, gelu(v) = v (1 + erf(v / sqrt 2)) / 2 collapses to max(v, 0) - |v| q(t) 2^(-v^2 log2(e) / 2) where q
+// carries the halved coefficients: fourteen instructions, two of them on the special-function unit (flush-to-zero forms, which
+// need no range fix-up), against the library erf's thirty.  The drain warps apply it to 128 x 256 values per tile.
+__device__ __forceinline__ float gelu_erf(float v) {
+    const float av = fabsf(v);
+    float t, e;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.23164189f, av, 1.f)));   // p / sqrt(2)
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((v * -0.72134752f) * v));          // log2(e) / 2
+    const float q = fmaf(fmaf(fmaf(fmaf(0.5307027145f, t, -0.7265760135f), t, 0.7107068705f), t, -0.142248368f), t, 0.127414796f) * t;
+    return fmaf(-(av * q), e, fmaxf(v, 0.f));
+}
+
 // fp32 operands run on the bf16 tensor cores as exact three-way splits x = xh + xm + xl, w = wh + wm + wl.  The
 // product keeps the six terms whose weight is >= 2^-16 of the leading one (wh xh, wm xh, wh xm, wm xm, wl xh, wh xl);
 // the dropped terms are below 2^-24 relative, the size of an fp32 rounding error.  Each term is one more pass
@@ -223,9 +264,11 @@ template <> __device__ __forceinline__ uint16_t bits16<float>(float) { return 0;
 // second accumulator tile in TMEM: every TC_CHUNK_KB k-blocks the first expansion group adds the tensor core's
 // partial tile into it with round-to-nearest FADDs (tcgen05.ld / tcgen05.st), and the MMAs restart from zero.  The
 // error then no longer depends on K.
-template <typename T> struct TcMode { using elem = T; static constexpr int TERMS = 1; static constexpr int GROUPS = 3; };
-template <> struct TcMode<float> { using elem = __nv_bfloat16; static constexpr int TERMS = 6; static constexpr int GROUPS = 3; };
+template <typename T> struct TcMode { using elem = T; static constexpr int TERMS = 1; };
+template <> struct TcMode<float> { using elem = __nv_bfloat16; static constexpr int TERMS = 6; };
 static __device__ __constant__ int kSplitW[6] = {0, 1, 0, 1, 2, 0};
 static __device__ __constant__ int kSplitX[6] = {0, 0, 1, 1, 0, 2};
+__host__ __device__ constexpr int split_w(int t) { return t == 1 || t == 3 ? 1 : t == 4 ? 2 : 0; }  // the same for unrolled loops
+__host__ __device__ constexpr int split_x(int t) { return t == 2 || t == 3 ? 1 : t == 5 ? 2 : 0; }
 
 }  // namespace nmg

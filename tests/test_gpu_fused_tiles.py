@@ -1,0 +1,45 @@
+"""The fused tensor-core matmul where its tiling changes: tile widths in steps of 32 tokens, one and several ranges of the
+reduction axis (partial tiles exchanged between the CTAs of a cluster), ragged last tiles in every direction, one k-block per
+range, and the fp32 mode's accumulation chunks.  Reference: float64 matmul of the rounded operands."""
+import pytest
+import torch
+
+from gpu_util import cuda, seeded_normal
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    # n, m, g, M, K, tokens
+    (2, 4, 16, 128, 64, 1),       # one tile, one k-block
+    (2, 4, 16, 129, 72, 33),      # a second feature tile with one row, a ragged second k-block, 33 of 64 token columns
+    (1, 8, 16, 1000, 1032, 31),   # ranges of the reduction with a ragged last one
+    (1, 16, 4, 384, 4160, 97),    # eight ranges, an odd token count in the exchange
+    (2, 8, 16, 136, 4104, 257),   # two token tiles of 160, many k-blocks per CTA
+    (1, 4, 8, 4096, 520, 96),     # as many tiles as SMs: no exchange
+    (2, 4, 4, 260, 1000, 200),    # rows that are not 4-byte pairs apart in the output are covered by M = 129 and 1000
+]
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 1e-2), (torch.float16, 2e-3), (torch.float32, 1e-5)])
+@pytest.mark.parametrize("n,m,g,M,K,tokens", CASES)
+def test_fused_matmul_tiles(n, m, g, M, K, tokens, dtype, tol):
+    from sten_b200 import _native as nat, ops
+    dev = cuda()
+    w = (seeded_normal((M, K), 1) * K ** -0.5).to(dtype).to(dev)
+    val, idx = ops.sparsify(w.unsqueeze(0), n, m, g)
+    dense = ops.densify(val, idx, 1, M, K, n, m, g)[0].double()
+    x = seeded_normal((tokens, K), 2).to(dtype).to(dev)
+    bias, res = seeded_normal((M,), 3).to(dtype).to(dev), seeded_normal((tokens, M), 4).to(dtype).to(dev)
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm())  # noqa: E731
+    product = x.double() @ dense.t()
+    y = ops.spmm(val, idx, M, K, n, m, g, x, algo=nat.NMG_ALGO_TENSOR)
+    assert rel(y, product) <= tol
+    assert torch.equal(y, ops.spmm(val, idx, M, K, n, m, g, x, algo=nat.NMG_ALGO_TENSOR))  # ranges are added in a fixed order
+    fused = ops.spmm(val, idx, M, K, n, m, g, x, bias=bias, activation="gelu", residual=res, algo=nat.NMG_ALGO_TENSOR)
+    assert rel(fused, torch.nn.functional.gelu(product + bias.double()) + res.double()) <= tol
+    rows = ops.spmm(val, idx, M, K, n, m, g, x, bias=bias, layout=nat.NMG_ACT_TOKEN_MAJOR_OUT_ROWS, algo=nat.NMG_ALGO_TENSOR)
+    assert rel(rows, (product + bias.double()).t()) <= tol
+    if M % 8 == 0 or dtype == torch.float32:
+        dy = seeded_normal((tokens, M), 5).to(dtype).to(dev)
+        assert rel(ops.spmm_t(val, idx, M, K, n, m, g, dy, algo=nat.NMG_ALGO_TENSOR), dy.double() @ dense) <= tol
+    assert ops.read_status() == 0

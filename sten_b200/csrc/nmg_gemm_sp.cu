@@ -226,24 +226,25 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_sp_kernel(const SpGemmPara
     };
 
     if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer (one lane per CTA)
-        if (lane == 0) {
-            int it = 0;
-            bool ok = true;
-            asm volatile("griddepcontrol.wait;" ::: "memory");  // the expansion pass's output arrives through the loads below
-            unsigned arrivals = 0;
-            for (int ti = 0; ti < my_tiles && ok; ti++) {
-                int tile_f, tok0;
-                tile_origin(ti, tile_f, tok0);
-                const int half_f = tile_f * 2 + (int)rank;  // this CTA's 128-feature tile = its metadata atom row
-                if (prm.wave_ctr && ti > 0) {  // keep the CTAs that share operand panels through L2 in step (soft_rendezvous)
-                    const int left = ntiles - ti * npairs;
-                    arrivals += (unsigned)((left < npairs ? left : npairs) * 2);
-                    soft_rendezvous(prm.wave_ctr, arrivals, (uint64_t)nst * 80);
-                }
-                for (int j = 0; j < nst; j++, it++) {
-                    const int s = it % SP_STAGES;
-                    if (!(ok = mbar_wait_cluster_bounded(&empty[s], (uint32_t)(((it / SP_STAGES) & 1) ^ 1), prm.status, 31))) break;
+        // ------------------------------------------------------------------ TMA producer (converged warp, issues under elect_one)
+        int it = 0;
+        bool ok = true;
+        asm volatile("griddepcontrol.wait;" ::: "memory");  // the expansion pass's output arrives through the loads below
+        unsigned arrivals = 0;
+        for (int ti = 0; ti < my_tiles && ok; ti++) {
+            int tile_f, tok0;
+            tile_origin(ti, tile_f, tok0);
+            const int half_f = tile_f * 2 + (int)rank;  // this CTA's 128-feature tile = its metadata atom row
+            if (prm.wave_ctr && ti > 0) {  // keep the CTAs that share operand panels through L2 in step (soft_rendezvous)
+                const int left = ntiles - ti * npairs;
+                arrivals += (unsigned)((left < npairs ? left : npairs) * 2);
+                if (lane == 0) soft_rendezvous(prm.wave_ctr, arrivals, (uint64_t)nst * 80);
+                __syncwarp();
+            }
+            for (int j = 0; j < nst; j++, it++) {
+                const int s = it % SP_STAGES;
+                if (!(ok = __all_sync(0xffffffffu, mbar_wait_cluster_bounded(&empty[s], (uint32_t)(((it / SP_STAGES) & 1) ^ 1), prm.status, 31)))) break;
+                if (elect_one()) {
                     if (leader) mbar_expect_tx(&full[s], 2 * SP_STAGE);  // both CTAs report to this barrier
                     char *stage = smem + s * SP_STAGE;
                     const uint32_t bar = full_leader + s * 8;
@@ -252,34 +253,40 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_sp_kernel(const SpGemmPara
                     tma_load_2d_pair(stage + SP_OFF_B + SP_B_HALF, &maps.b, j * SP_ATOM + TC_BK, tok0 + (int)rank * 128, bar);
                     tma_load_2d_pair(stage + SP_OFF_E, &maps.e, 0, (int)(((int64_t)half_f * prm.n_rt + j) * 2), bar);
                 }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer (one lane of the leader)
-        if (leader && lane == 0) {
+        // ------------------------------------------------------------------ MMA issuer (of the leader; converged warp)
+        if (leader) {
             const uint32_t idesc = make_idesc_sp_pair<T>();
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0), stage0 = smem_u32(smem);
+            const uint64_t desc0 = make_sw128_desc(stage0);
             bool ok = true;
             int it = 0;
             for (int ti = 0; ti < my_tiles && ok; ti++) {
-                if (ti > 0) ok = mbar_wait_cluster_bounded(acc_free, (uint32_t)((ti - 1) & 1), prm.status, 36);
+                if (ti > 0) ok = __all_sync(0xffffffffu, mbar_wait_cluster_bounded(acc_free, (uint32_t)((ti - 1) & 1), prm.status, 36));
                 if (!ok) break;
                 tc_fence_after();
                 for (int j = 0; j < nst; j++, it++) {
                     const int s = it % SP_STAGES;
-                    if (!(ok = mbar_wait_cluster_bounded(&full[s], (uint32_t)((it / SP_STAGES) & 1), prm.status, 33))) break;
+                    if (!(ok = __all_sync(0xffffffffu, mbar_wait_cluster_bounded(&full[s], (uint32_t)((it / SP_STAGES) & 1), prm.status, 33)))) break;
                     tc_fence_after();
-                    const uint32_t stage = smem_u32(smem + s * SP_STAGE);
-                    const uint32_t e_set = tmem_base + SP_E_COL + 4u * (uint32_t)(it & 1);
-                    tc2_copy_meta(e_set, stage + SP_OFF_E);
-                    const uint64_t adesc = make_sw128_desc(stage);
-                    const uint64_t bdesc0 = make_sw128_desc(stage + SP_OFF_B), bdesc1 = make_sw128_desc(stage + SP_OFF_B + SP_B_HALF);
+                    if (elect_one()) {
+                        const uint32_t e_set = tmem_u + SP_E_COL + 4u * (uint32_t)(it & 1);
+                        tc2_copy_meta(e_set, stage0 + (uint32_t)(s * SP_STAGE + SP_OFF_E));
+                        const uint64_t adesc = desc0 + (uint64_t)(uint32_t)(s * (SP_STAGE / 16));
+                        const uint64_t bdesc0 = adesc + SP_OFF_B / 16, bdesc1 = bdesc0 + SP_B_HALF / 16;
 #pragma unroll
-                    for (int k = 0; k < 4; k++)  // 32 reduction elements per instruction: 16 stored values of A (2 descriptor units), 32 of dY (4 units)
-                        tc2_mma_sp_f16(tmem_base, adesc + 2 * k, (k < 2 ? bdesc0 : bdesc1) + 4 * (k & 1), e_set + (uint32_t)(k & 2),
-                                       idesc | (uint32_t)(k & 1), (j == 0 && k == 0) ? 0u : 1u);  // metadata columns are addressed in pairs
-                    tc2_commit_both(&empty[s]);
+                        for (int k = 0; k < 4; k++)  // 32 reduction elements per instruction: 16 stored values of A (2 descriptor units), 32 of dY (4 units)
+                            tc2_mma_sp_f16(tmem_u, adesc + 2 * k, (k < 2 ? bdesc0 : bdesc1) + 4 * (k & 1), e_set + (uint32_t)(k & 2),
+                                           idesc | (uint32_t)(k & 1), (j == 0 && k == 0) ? 0u : 1u);  // metadata columns are addressed in pairs
+                        tc2_commit_both(&empty[s]);
+                    }
+                    __syncwarp();
                 }
-                tc2_commit_both(acc_full);  // arrives in both CTAs when the tile's MMAs have written TMEM (also on the error path)
+                if (elect_one()) tc2_commit_both(acc_full);  // arrives in both CTAs when the tile's MMAs have written TMEM (also on the error path)
+                __syncwarp();
             }
         }
     } else {
@@ -344,6 +351,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_sp_kernel(const SpGemmPara
             }
         }
     }
+    __syncwarp();
     if (warp >= 2 && lane == 0) tma_store_wait_read();  // sources read before shared memory is given up; writes complete with the grid
     __syncthreads();
     cluster_sync_all();  // the peer no longer reads this CTA's shared memory or signals its barriers

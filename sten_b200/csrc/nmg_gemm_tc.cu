@@ -275,30 +275,32 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     };
 
     if (warp == 0) {
-        // ------------------------------------------------------------------ TMA producer (one lane per CTA)
-        if (lane == 0) {
-            int it = 0;
-            bool ok = true;
-            // Everything this kernel reads that an earlier kernel of the stream wrote (the expanded weight, the
-            // activations) arrives through the loads below: wait here for the preceding grid to complete and flush.
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            unsigned arrivals = 0;
-            for (int ti = 0; ti < my_tiles && ok; ti++) {
-                int feat0, tok0;
-                tile_origin(ti, feat0, tok0);
-                if (prm.wave_ctr && ti > 0) {
-                    // CTAs whose tiles share operand panels read them from HBM once only while they stream through the
-                    // reduction in step; left alone they drift apart over the waves (measured: 2.2 MB of DRAM reads per
-                    // 256 x 256 x 16384 tile in the first dozen waves, 3.9 MB averaged over 55).  So the producers meet,
-                    // softly, before each tile: everyone that has a tile ti counts in.
-                    const int left = ntiles - ti * nunits;
-                    arrivals += (unsigned)((left < nunits ? left : nunits) * (PAIR ? 2 : 1));
-                    soft_rendezvous(prm.wave_ctr, arrivals, (uint64_t)nkb * 40);
-                }
-                for (int kb = 0; kb < nkb; kb++, it++) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (uint32_t)((it / STAGES) & 1);
-                    if (!(ok = wait(&empty[s], ph ^ 1, 21))) break;
+        // ------------------------------------------------------------------ TMA producer
+        // The warp stays converged and issues under elect_one (see there).
+        int it = 0;
+        bool ok = true;
+        // Everything this kernel reads that an earlier kernel of the stream wrote (the expanded weight, the
+        // activations) arrives through the loads below: wait here for the preceding grid to complete and flush.
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        unsigned arrivals = 0;
+        for (int ti = 0; ti < my_tiles && ok; ti++) {
+            int feat0, tok0;
+            tile_origin(ti, feat0, tok0);
+            if (prm.wave_ctr && ti > 0) {
+                // CTAs whose tiles share operand panels read them from HBM once only while they stream through the
+                // reduction in step; left alone they drift apart over the waves (measured: 2.2 MB of DRAM reads per
+                // 256 x 256 x 16384 tile in the first dozen waves, 3.9 MB averaged over 55).  So the producers meet,
+                // softly, before each tile: everyone that has a tile ti counts in.
+                const int left = ntiles - ti * nunits;
+                arrivals += (unsigned)((left < nunits ? left : nunits) * (PAIR ? 2 : 1));
+                if (lane == 0) soft_rendezvous(prm.wave_ctr, arrivals, (uint64_t)nkb * 40);
+                __syncwarp();
+            }
+            for (int kb = 0; kb < nkb; kb++, it++) {
+                const int s = it % STAGES;
+                const uint32_t ph = (uint32_t)((it / STAGES) & 1);
+                if (!(ok = __all_sync(0xffffffffu, wait(&empty[s], ph ^ 1, 21)))) break;
+                if (elect_one()) {
                     const int term = kb % TERMS;
                     const int wc = TERMS == 1 ? 0 : kSplitW[term], xc = TERMS == 1 ? 0 : kSplitX[term];
                     char *stage = smem + s * STAGE_BYTES;
@@ -312,42 +314,50 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                         tma_load_2d(stage + TC_A_BYTES, &maps.b[xc], (kb / TERMS) * TC_BK, tok0, &full[s]);
                     }
                 }
+                __syncwarp();
             }
         }
     } else if (warp == 1) {
-        // ------------------------------------------------------------------ MMA issuer (one lane; of the leader for pairs)
-        if (lane == 0 && leader) {
+        // ------------------------------------------------------------------ MMA issuer (of the leader for pairs)
+        if (leader) {
             uint32_t idesc = make_idesc<E>();
             if constexpr (PAIR) idesc = (idesc & ~(0x1fu << 24)) | ((uint32_t)(256 >> 4) << 24);  // M = 256 across the pair
+            const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
+            const uint64_t desc0 = make_sw128_desc(smem_u32(smem));
             bool ok = true;
             int it = 0, unit = 0;
             for (int ti = 0; ti < my_tiles && ok; ti++) {
                 int kb = 0;
                 for (int c = 0; c < nchunks && ok; c++, unit++) {
                     const int b = unit % NBUF, use = unit / NBUF;
-                    if (use > 0) ok = wait(&acc_free[b], (uint32_t)((use - 1) & 1), 26);
+                    if (use > 0) ok = __all_sync(0xffffffffu, wait(&acc_free[b], (uint32_t)((use - 1) & 1), 26));
                     if (!ok) break;
                     tc_fence_after();
-                    const uint32_t d_tmem = tmem_base + (uint32_t)(b * TC_ACC_COLS);
+                    const uint32_t d_tmem = tmem_u + (uint32_t)(b * TC_ACC_COLS);
                     const int kend = (kb + chunk_it < nkb) ? kb + chunk_it : nkb;
                     for (bool first = true; kb < kend; kb++, it++, first = false) {
                         const int s = it % STAGES;
                         const uint32_t ph = (uint32_t)((it / STAGES) & 1);
-                        if (!(ok = wait(&full[s], ph, 22))) break;
+                        if (!(ok = __all_sync(0xffffffffu, wait(&full[s], ph, 22)))) break;
                         tc_fence_after();
-                        const uint64_t adesc = make_sw128_desc(smem_u32(smem + s * STAGE_BYTES));
-                        const uint64_t bdesc = make_sw128_desc(smem_u32(smem + s * STAGE_BYTES + TC_A_BYTES));
+                        if (elect_one()) {
+                            const uint64_t adesc = desc0 + (uint64_t)(uint32_t)(s * (STAGE_BYTES / 16)), bdesc = adesc + TC_A_BYTES / 16;
 #pragma unroll
-                        for (int k = 0; k < TC_BK / 16; k++) {  // 16 elements = 32 bytes = 2 descriptor units per step
-                            if constexpr (PAIR) tc2_mma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
-                            else tc_mma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
+                            for (int k = 0; k < TC_BK / 16; k++) {  // 16 elements = 32 bytes = 2 descriptor units per step
+                                if constexpr (PAIR) tc2_mma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
+                                else tc_mma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
+                            }
+                            if constexpr (PAIR) tc2_commit_both(&empty[s]);
+                            else tc_commit(&empty[s]);  // arrives when the MMAs above have read the stage
                         }
-                        if constexpr (PAIR) tc2_commit_both(&empty[s]);
-                        else tc_commit(&empty[s]);  // arrives when the MMAs above have read the stage
+                        __syncwarp();
                     }
                     // arrives when the unit's MMAs have written TMEM (also on the error path)
-                    if constexpr (PAIR) tc2_commit_both(&acc_full[b]);
-                    else tc_commit(&acc_full[b]);
+                    if (elect_one()) {
+                        if constexpr (PAIR) tc2_commit_both(&acc_full[b]);
+                        else tc_commit(&acc_full[b]);
+                    }
+                    __syncwarp();
                 }
             }
         }

@@ -460,7 +460,8 @@ PyObject *handle_mm(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     if (act.rows != geo.K) py_raise(PyExc_ValueError, "activation shape " + shape_str(b.sizes()) + " does not match K=" + std::to_string(geo.K));
     const at::Tensor out = at::empty({geo.M, act.cols}, val.options());
     if (act.cols > 0) {
-        const bool wants = nmg_spmm_uses_packed(geo.M, geo.K, act.cols, geo.n, geo.m, geo.g, code, NMG_ACT_K_MAJOR, NMG_ALGO_AUTO, 0) != 0;
+        // a handful of columns runs on the tensor cores when the packed copy is there already: keep one for the token-major call
+        const bool wants = nmg_spmm_uses_packed(geo.M, geo.K, act.cols, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 0) != 0;
         call_spmm(geo, code, dev, val, idx, wants ? derived(*h->packed, a[0], g_s_packed, val, idx) : at::Tensor(), act, act.cols, at::Tensor(), Epi(), out,
                   act.cols, NMG_ACT_K_MAJOR, NMG_ALGO_AUTO);
     }

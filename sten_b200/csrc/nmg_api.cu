@@ -14,13 +14,22 @@ static int check_common(int dtype, int64_t tokens, const void *a, const void *b,
 
 static char *align256(void *p) { return reinterpret_cast<char *>(((uintptr_t)p + 255) & ~(uintptr_t)255); }
 
-// The tensor-core kernel reads the activation through a TMA descriptor: 16-bit dtype, reduction axis contiguous,
-// 16-byte aligned base and row pitch.
-static bool tensor_ok(const Geo &geo, int dtype, const void *act, int64_t ld_act) {
-    if (!tc_supported(geo, dtype) && !tc_dense_supported(geo, dtype)) return false;
-    if (dtype == NMG_F32) return true;  // fp32 activations are re-laid out into aligned bf16 planes first
-    return (((uintptr_t)act) & 15) == 0 && (ld_act % 8) == 0;
+static bool any_tensor(const Geo &geo, int dtype) { return tc_supported(geo, dtype) || tc_dense_supported(geo, dtype); }
+
+// The tensor-core kernels read the activation through a TMA descriptor: 16-bit dtype, reduction axis contiguous, 16-byte
+// aligned base and row pitch.  fp32 activations are re-laid out into aligned bf16 planes first.
+static bool rows_aligned(int dtype, const void *act, int64_t ld_act) {
+    return dtype == NMG_F32 || ((((uintptr_t)act) & 15) == 0 && (ld_act % 8) == 0);
 }
+
+// 16-bit activations whose rows TMA cannot read (an odd reduction length, a sliced view) are copied into the workspace with
+// padded rows under NMG_ALGO_AUTO: the copy is a few percent of the matmul, the gather kernels that read such rows in place
+// are 7 .. 50 times slower (1023 x 777 f16, 333 tokens: 84 us against 2 + 9).
+static size_t pad_rows_bytes(int dtype, int64_t rows, int64_t cols) {
+    return dtype == NMG_F32 ? 0 : (size_t)rows * (size_t)round_up(cols, 8) * 2 + 512;
+}
+// Whether NMG_ALGO_AUTO runs a product with `feats` output features on the tensor cores (whatever the operands' alignment).
+static bool auto_tensor(const Geo &geo, int dtype, int64_t feats) { return feats >= 64 && any_tensor(geo, dtype); }
 
 extern "C" size_t nmg_packed_bytes(int64_t M, int64_t K, int n, int m, int g, int dtype) {
     Geo geo;
@@ -65,22 +74,28 @@ static int resolve_packed(const Geo &geo, int dtype, const void *val, const int1
 // K-major activations (B[K][tokens], the torch.mm orientation) reach the tensor cores through one same-dtype transpose
 // into the workspace: X[tokens][round_up(K, 8)], after which the call is the token-major one with row-major output.
 static size_t kmajor_transpose_bytes(const Geo &geo, int dtype, int64_t tokens) {
-    return (size_t)tokens * (size_t)round_up(geo.K, 8) * dtype_size(dtype) + 512;
+    return dtype == NMG_F32 ? 0 : (size_t)tokens * (size_t)round_up(geo.K, 8) * 2 + 512;  // fp32: transposed while it is split
 }
+// Fewer than 64 columns do not pay for re-ordering the weight on every call; with a packed copy in hand they take the tensor
+// cores like any other batch (192 x 3200 f16, 2 columns: 7 us against 229 us in the gather kernel).
+static bool kmajor_few(int layout, int64_t tokens, bool have_packed) { return layout == NMG_ACT_K_MAJOR && tokens < 64 && !have_packed; }
 
 extern "C" size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype,
                                            int layout, int algo, int have_packed) {
     Geo geo;
     if (make_geo(M, K, n, m, g, &geo) || tokens < 1 || n < 1) return 0;
-    size_t simt = simt_fwd_workspace_bytes(geo, tokens, dtype, layout);
-    size_t tensor = 0;
     if (algo == NMG_ALGO_TENSOR_DENSE) algo = NMG_ALGO_TENSOR;
-    if (algo != NMG_ALGO_SIMT && (tc_supported(geo, dtype) || tc_dense_supported(geo, dtype)))
+    size_t tensor = 0;
+    const bool tensor_runs = algo == NMG_ALGO_TENSOR ? any_tensor(geo, dtype) : algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, M);
+    if (tensor_runs)
         tensor = (tc_use_dense(geo, dtype, tokens) ? tc_dense_workspace_bytes(geo, dtype, false)
                                                    : (have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512)) +
-                 tc_split_workspace_bytes(geo, dtype, false, tokens) + (layout == NMG_ACT_K_MAJOR ? kmajor_transpose_bytes(geo, dtype, tokens) : 0);
-    if (algo == NMG_ALGO_TENSOR) return tensor;
-    return simt > tensor ? simt : tensor;  // AUTO may take either path depending on operand alignment
+                 tc_split_workspace_bytes(geo, dtype, false, tokens) +
+                 (layout == NMG_ACT_K_MAJOR ? kmajor_transpose_bytes(geo, dtype, tokens) : algo == NMG_ALGO_AUTO ? pad_rows_bytes(dtype, tokens, K) : 0);
+    // AUTO: the gather kernels serve what the tensor cores do not, and a handful of K-major columns without a packed copy
+    const bool simt_runs = algo == NMG_ALGO_SIMT || (algo == NMG_ALGO_AUTO && (!tensor_runs || kmajor_few(layout, tokens, have_packed != 0)));
+    const size_t simt = simt_runs ? simt_fwd_workspace_bytes(geo, tokens, dtype, layout) : 0;
+    return simt > tensor ? simt : tensor;
 }
 
 static int spmm_impl(const void *val, const int16_t *idx, const void *packed, int64_t M, int64_t K, int n, int m, int g, int dtype,
@@ -103,35 +118,31 @@ static int spmm_impl(const void *val, const int16_t *idx, const void *packed, in
         NMG_FAIL(NMG_ERR_INVALID, "unknown algo %d", algo);
     if (algo == NMG_ALGO_TENSOR_DENSE) algo = NMG_ALGO_TENSOR;  // the forward product has no structured-sparse variant
     cudaStream_t st = (cudaStream_t)stream;
-    // K-major activations take the tensor cores when the weight is large enough to pay for the transpose pre-pass
-    const bool kmajor_tensor = !tm && n_outs == 1 && (tc_supported(geo, dtype) || tc_dense_supported(geo, dtype)) &&
-                               (algo == NMG_ALGO_TENSOR || (algo == NMG_ALGO_AUTO && M >= 64 && tokens >= 64));
-    if (kmajor_tensor) {
-        const size_t need = kmajor_transpose_bytes(geo, dtype, tokens);
-        if (!workspace || workspace_bytes < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the transposed activation, got %zu", need, workspace_bytes);
-        char *xt = align256(workspace);
-        const int64_t ld_xt = round_up(K, 8);
-        if ((rc = launch_transpose(act, dtype, K, tokens, ld_act, xt, ld_xt, st))) return rc;
-        char *rest = xt + (size_t)tokens * ld_xt * dtype_size(dtype);
-        const size_t used = (size_t)(rest - static_cast<char *>(workspace));
-        return spmm_impl(val, idx, packed, M, K, n, m, g, dtype, xt, ld_xt, tokens, bias, outs, n_outs, ld_out, NMG_ACT_TOKEN_MAJOR_OUT_ROWS,
-                         NMG_ALGO_TENSOR, rest, workspace_bytes - used, stream, force_dense, mc_out, epi);
-    }
-    const bool can_tensor = tm && tensor_ok(geo, dtype, act, ld_act);
-    if (algo == NMG_ALGO_TENSOR && !can_tensor)
+    const bool tensor = algo == NMG_ALGO_TENSOR || (algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, M) && !kmajor_few(layout, tokens, packed != nullptr));
+    if (algo == NMG_ALGO_TENSOR && (!any_tensor(geo, dtype) || (tm && !rows_aligned(dtype, act, ld_act)) || (!tm && n_outs > 1)))
         NMG_FAIL(NMG_ERR_UNSUPPORTED, "tensor-core path needs activation rows that are 16-byte aligned (16-bit dtypes) and a chunk that fits shared memory");
-    // AUTO: tensor cores whenever the operands allow it and the weight has at least 64 rows, at every token count (measured
-    // at 16 tokens on a 4096^2 bf16 weight: 0.05 ms against 0.71 ms on the SIMT kernel, which is built for wide token
-    // tiles); unsupported layouts / alignments and tiny weights stay on the SIMT kernels.  fp32 on tensor cores means exact bf16 splitting with
-    // promoted accumulation (measured relative error 3.5e-6, independent of K); NMG_ALGO_SIMT keeps plain fp32 FMAs.
-    if (algo == NMG_ALGO_TENSOR || (algo == NMG_ALGO_AUTO && can_tensor && M >= 64)) {
+    // AUTO: tensor cores whenever the weight has at least 64 rows, at every token count.  fp32 on tensor cores means exact bf16
+    // splitting with promoted accumulation (measured relative error 3.5e-6, independent of K); NMG_ALGO_SIMT keeps plain fp32 FMAs.
+    if (tensor) {
         char *ws = static_cast<char *>(workspace);
         size_t left = workspace_bytes;
-        const void *pat = nullptr;
-        const void *nval = nullptr;
+        const int64_t ld_x = round_up(K, 8);
+        if (dtype != NMG_F32 && (!tm || !rows_aligned(dtype, act, ld_act))) {  // re-lay the activation out as [tokens][round_up(K, 8)]
+            const size_t need = (size_t)tokens * (size_t)ld_x * 2 + 512;
+            if (!ws || left < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the re-laid activation, got %zu", need, left);
+            char *xt = align256(ws);
+            if ((rc = tm ? launch_pad_rows(act, tokens, K, ld_act, xt, ld_x, st) : launch_transpose(act, dtype, K, tokens, ld_act, xt, ld_x, st))) return rc;
+            act = xt;
+            ld_act = ld_x;
+            char *rest = xt + (size_t)tokens * ld_x * 2;
+            left -= (size_t)(rest - ws);
+            ws = rest;
+        }
+        const void *pat = nullptr, *nval = nullptr;
         const bool dense = force_dense || tc_use_dense(geo, dtype, tokens);
         if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st))) return rc;
-        return tc_matmul(geo, dtype, false, dense, val, idx, pat, nval, act, ld_act, tokens, bias, outs, n_outs, mc_out, ld_out, out_tm ? 1 : 0, ws, left, st, epi);
+        return tc_matmul(geo, dtype, false, dense, val, idx, pat, nval, act, ld_act, dtype == NMG_F32 && !tm, tokens, bias, outs, n_outs, mc_out, ld_out, out_tm ? 1 : 0,
+                         ws, left, st, epi);
     }
     if (n_outs > 1) NMG_FAIL(NMG_ERR_UNSUPPORTED, "several output buffers need the tensor-core path (aligned token-major activations, >= 64 tokens and rows)");
     if ((rc = simt_fwd(geo, dtype, val, idx, act, ld_act, tokens, bias, out, ld_out, layout, workspace, workspace_bytes, st))) return rc;
@@ -185,7 +196,7 @@ extern "C" int nmg_spmm_uses_packed(int64_t M, int64_t K, int64_t tokens, int n,
                                     int algo, int transposed) {
     Geo geo;
     if (make_geo(M, K, n, m, g, &geo) || tokens < 1 || n < 1) return 0;
-    const bool any_tc = tc_supported(geo, dtype) || tc_dense_supported(geo, dtype);
+    const bool any_tc = any_tensor(geo, dtype);
     const bool wants = algo == NMG_ALGO_TENSOR || algo == NMG_ALGO_TENSOR_DENSE || (algo == NMG_ALGO_AUTO && (transposed ? K : M) >= 64);
     const bool tensor = any_tc && wants && (transposed || layout != NMG_ACT_K_MAJOR || tokens >= 64 || algo == NMG_ALGO_TENSOR);
     if (tensor) return tc_use_dense(geo, dtype, tokens) ? 0 : 1;
@@ -203,12 +214,14 @@ extern "C" size_t nmg_spmm_t_workspace_bytes(int64_t M, int64_t K, int64_t token
     Geo geo;
     if (make_geo(M, K, n, m, g, &geo) || tokens < 1 || n < 1) return 0;
     const size_t pack = have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512;
-    const size_t simt = algo != NMG_ALGO_TENSOR ? pack + simt_bwd_workspace_bytes(geo, tokens, dtype) + 256 : 0;
+    const bool tensor_only = algo == NMG_ALGO_TENSOR || algo == NMG_ALGO_TENSOR_DENSE || (algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, K));
+    const size_t simt = tensor_only ? 0 : pack + simt_bwd_workspace_bytes(geo, tokens, dtype) + 256;
     size_t tensor = 0;
-    if (algo != NMG_ALGO_SIMT && (tc_supported(geo, dtype) || tc_dense_supported(geo, dtype)))
+    if (algo != NMG_ALGO_SIMT && any_tensor(geo, dtype))
         tensor = (tc_use_dense(geo, dtype, tokens) ? tc_dense_workspace_bytes(geo, dtype, true) : pack) +
                  tc_split_workspace_bytes(geo, dtype, true, tokens);
-    if (use_sp(geo, dtype, tokens, algo) && tc_sp_copy_bytes(geo) + 256 > tensor) tensor = tc_sp_copy_bytes(geo) + 256;
+    if (use_sp(geo, dtype, tokens, algo) && tc_sp_copy_bytes(geo) + 512 > tensor) tensor = tc_sp_copy_bytes(geo) + 512;
+    if (algo == NMG_ALGO_AUTO && tensor_only) tensor += pad_rows_bytes(dtype, tokens, M);
     return simt > tensor ? simt : tensor;
 }
 
@@ -225,20 +238,32 @@ extern "C" int nmg_spmm_t(const void *val, const int16_t *idx, const void *packe
     if (algo != NMG_ALGO_AUTO && algo != NMG_ALGO_SIMT && algo != NMG_ALGO_TENSOR && algo != NMG_ALGO_TENSOR_DENSE)
         NMG_FAIL(NMG_ERR_INVALID, "unknown algo %d", algo);
     cudaStream_t st = (cudaStream_t)stream;
-    const bool can_tensor = tensor_ok(geo, dtype, dy, ld_dy);
+    const bool can_tensor = any_tensor(geo, dtype) && rows_aligned(dtype, dy, ld_dy);
     if ((algo == NMG_ALGO_TENSOR || algo == NMG_ALGO_TENSOR_DENSE) && !can_tensor)
         NMG_FAIL(NMG_ERR_UNSUPPORTED, "tensor-core path needs gradient rows that are 16-byte aligned (16-bit dtypes) and a chunk that fits shared memory");
     char *ws = static_cast<char *>(workspace);
     size_t left = workspace_bytes;
     const void *pat = nullptr;
     const void *nval = nullptr;
-    const bool tensor = algo == NMG_ALGO_TENSOR || algo == NMG_ALGO_TENSOR_DENSE || (algo == NMG_ALGO_AUTO && can_tensor && K >= 64);
+    const bool tensor = algo == NMG_ALGO_TENSOR || algo == NMG_ALGO_TENSOR_DENSE || (algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, K));
+    if (tensor && !rows_aligned(dtype, dy, ld_dy)) {  // AUTO only: see pad_rows_bytes
+        const size_t need = pad_rows_bytes(dtype, tokens, M);
+        if (!ws || left < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the re-laid gradient, got %zu", need, left);
+        char *yt = align256(ws);
+        const int64_t ld_y = round_up(M, 8);
+        if ((rc = launch_pad_rows(dy, tokens, M, ld_dy, yt, ld_y, st))) return rc;
+        dy = yt;
+        ld_dy = ld_y;
+        char *rest = yt + (size_t)tokens * ld_y * 2;
+        left -= (size_t)(rest - ws);
+        ws = rest;
+    }
     // The rows of W are the reduction axis here, so the n:m structure is one the tensor cores can skip: structured-sparse
     // MMA at twice the dense rate (16-bit weights, n <= 2, m a power of two >= 4).
     if (tensor && use_sp(geo, dtype, tokens, algo)) {
         const size_t need = tc_sp_copy_bytes(geo);
-        char *buf = align256(workspace);
-        if (!workspace || workspace_bytes < need + 256) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the compressed transposed weight, got %zu", need + 256, workspace_bytes);
+        char *buf = align256(ws);
+        if (!ws || left < need + 256) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the compressed transposed weight, got %zu", need + 256, left);
         const ProfileEvents pe = take_profile_events();
         if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));
         if ((rc = tc_sp_pack(geo, dtype, val, idx, buf, need, st))) return rc;
@@ -249,7 +274,7 @@ extern "C" int nmg_spmm_t(const void *val, const int16_t *idx, const void *packe
     const bool dense = tensor && tc_use_dense(geo, dtype, tokens);
     if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st))) return rc;
     void *dxs[1] = {dx};
-    if (tensor) return tc_matmul(geo, dtype, true, dense, val, idx, pat, nval, dy, ld_dy, tokens, nullptr, dxs, 1, nullptr, ld_dx, 1, ws, left, st);
+    if (tensor) return tc_matmul(geo, dtype, true, dense, val, idx, pat, nval, dy, ld_dy, false, tokens, nullptr, dxs, 1, nullptr, ld_dx, 1, ws, left, st);
     return simt_bwd(geo, dtype, pat, nval, dy, ld_dy, tokens, dx, ld_dx, ws, left, st);
 }
 

@@ -53,6 +53,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) transpose_kernel(const T *__restrict__ src, int64_t rows, int64_t cols, int64_t ld_src,
                                                         T *__restrict__ dst, int64_t ld_dst) {
     __shared__ T tile[64][66];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the matmul's set-up may overlap this pass
     const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
     const int64_t c0 = (int64_t)blockIdx.x * 64, r0 = (int64_t)blockIdx.y * 64;
     for (int i = ty; i < 64; i += 8) {
@@ -81,6 +82,33 @@ int launch_transpose(const void *src, int dtype, int64_t rows, int64_t cols, int
     if (gy > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "reduction axis too long for the transpose pre-pass");
     dim3 grid((unsigned)((cols + 63) / 64), (unsigned)gy);
     NMG_DISPATCH_DTYPE(dtype, T, (transpose_kernel<T><<<grid, block, 0, st>>>(static_cast<const T *>(src), rows, cols, ld_src, static_cast<T *>(dst), ld_dst)));
+    NMG_CUDA(cudaGetLastError());
+    return NMG_OK;
+}
+
+// Eight elements per thread: 2-byte loads (the rows have no alignment; a warp's eight loads share their lines in L1), one
+// 16-byte store.
+__global__ void __launch_bounds__(256) pad_rows_kernel(const uint16_t *__restrict__ src, int64_t rows, int64_t cols, int64_t ld_src, uint16_t *__restrict__ dst, int64_t ld_dst) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the matmul's set-up may overlap this pass
+    const int64_t per_row = ld_dst / 8;
+    for (int64_t r = (int64_t)blockIdx.y * blockDim.y + threadIdx.y; r < rows; r += (int64_t)gridDim.y * blockDim.y)
+        for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < per_row; v += (int64_t)gridDim.x * blockDim.x) {
+            const uint16_t *s = src + r * ld_src + v * 8;
+            const int left = (int)(cols - v * 8 < 8 ? cols - v * 8 : 8);
+            uint32_t e[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) e[i] = i < left ? (uint32_t)__ldg(s + i) : 0u;
+            *reinterpret_cast<uint4 *>(dst + r * ld_dst + v * 8) = make_uint4(e[0] | (e[1] << 16), e[2] | (e[3] << 16), e[4] | (e[5] << 16), e[6] | (e[7] << 16));
+        }
+}
+
+int launch_pad_rows(const void *src, int64_t rows, int64_t cols, int64_t ld_src, void *dst, int64_t ld_dst, cudaStream_t st) {
+    const int64_t per_row = ld_dst / 8;
+    dim3 block(32, 8);
+    while (block.x < 256 && (int64_t)block.x < per_row) { block.x *= 2; block.y /= 2; }
+    const int64_t bx = (per_row + block.x - 1) / block.x, by = (rows + block.y - 1) / block.y;
+    pad_rows_kernel<<<dim3((unsigned)(bx < 1024 ? bx : 1024), (unsigned)(by < 65535 ? by : 65535)), block, 0, st>>>(
+        static_cast<const uint16_t *>(src), rows, cols, ld_src, static_cast<uint16_t *>(dst), ld_dst);
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;
 }

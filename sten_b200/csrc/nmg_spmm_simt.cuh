@@ -11,6 +11,9 @@ int launch_transpose_to_f32(const void *src, int dtype, int64_t rows, int64_t co
                             int64_t ld_dst, cudaStream_t st);
 // Same-dtype transpose: src[rows][ld_src] -> dst[cols][ld_dst]; columns of dst beyond `rows` (up to ld_dst) are zeroed.
 int launch_transpose(const void *src, int dtype, int64_t rows, int64_t cols, int64_t ld_src, void *dst, int64_t ld_dst, cudaStream_t st);
+// 16-bit rows copied with a padded pitch: src[rows][ld_src] -> dst[rows][ld_dst], columns beyond `cols` zero; ld_dst a multiple
+// of 8, dst 16-byte aligned.
+int launch_pad_rows(const void *src, int64_t rows, int64_t cols, int64_t ld_src, void *dst, int64_t ld_dst, cudaStream_t st);
 // Copy + widen without transposing: src[rows][ld_src] (dtype) -> dst[rows][ld_dst] fp32.
 int launch_widen_to_f32(const void *src, int dtype, int64_t rows, int64_t cols, int64_t ld_src, float *dst,
                         int64_t ld_dst, cudaStream_t st);
@@ -58,8 +61,9 @@ size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, int6
 size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed);
 // outs / n_outs: the result goes to every listed buffer (same shape and pitch); more than one needs `dense`.  mc_out, when
 // not NULL, is an NVSwitch multicast address that maps onto all of them: full 16-byte chunks are then stored once.
+// act_k_major (fp32 only): act is [reduction][ld_act >= tokens]; it is transposed while it is split into planes.
 int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void *val, const int16_t *idx, const void *pat,
-              const void *nval, const void *act, int64_t ld_act, int64_t tokens, const void *bias, void *const *outs, int n_outs,
+              const void *nval, const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, const void *bias, void *const *outs, int n_outs,
               void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi = Epilogue());
 int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const CUtensorMap *act_maps,
                     int64_t tokens, const void *bias, void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major,

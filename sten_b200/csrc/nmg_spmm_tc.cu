@@ -689,6 +689,7 @@ static FxChoice fx_choose(int64_t feats, int64_t red, int64_t tokens, int dtype)
 // ---- fp32 activations: three bf16 planes [3][rows][ldp], written by one elementwise pass ---------------------------
 __global__ void __launch_bounds__(128) split_f32_kernel(const float *__restrict__ src, int64_t rows, int64_t cols, int64_t ld_src,
                                                         __nv_bfloat16 *__restrict__ dst, int64_t ldp, int64_t plane_elems) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the matmul's set-up may overlap this pass
     const int64_t r = blockIdx.y;
     const float *row = src + r * ld_src;
     const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
@@ -718,6 +719,34 @@ __global__ void __launch_bounds__(128) split_f32_kernel(const float *__restrict_
         const int64_t o = r * ldp + c;
 #pragma unroll
         for (int p = 0; p < 3; p++) *reinterpret_cast<uint4 *>(dst + p * plane_elems + o) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    }
+}
+
+// The same from a K-major activation src[red][ld_src >= tokens]: transposed through a 64 x 32 tile on the way, so that the
+// torch.mm orientation needs no pass of its own (1024 x 256: 3.4 us).
+__global__ void __launch_bounds__(256) split_f32_t_kernel(const float *__restrict__ src, int64_t red, int64_t tokens, int64_t ld_src,
+                                                          __nv_bfloat16 *__restrict__ dst, int64_t ldp, int64_t plane_elems) {
+    __shared__ float tile[64][33];  // [reduction][token]
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const int64_t k0 = (int64_t)blockIdx.x * 64;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int64_t t0 = (int64_t)blockIdx.y * 32; t0 < tokens; t0 += (int64_t)gridDim.y * 32) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 8; i++) {
+            const int64_t k = k0 + warp * 8 + i, t = t0 + lane;
+            tile[warp * 8 + i][lane] = (k < red && t < tokens) ? __ldg(src + k * ld_src + t) : 0.f;
+        }
+        __syncthreads();
+        const int tok = threadIdx.x >> 3, c = (threadIdx.x & 7) * 8;  // eight reduction elements of one token
+        if (t0 + tok < tokens && k0 + c < ldp) {
+            uint32_t w[3][4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) split3_pair(tile[c + 2 * i][tok], tile[c + 2 * i + 1][tok], w[0][i], w[1][i], w[2][i]);
+#pragma unroll
+            for (int p = 0; p < 3; p++)
+                *reinterpret_cast<uint4 *>(dst + p * plane_elems + (t0 + tok) * ldp + k0 + c) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+        }
     }
 }
 
@@ -777,7 +806,7 @@ bool tc_use_dense(const Geo &geo, int dtype, int64_t tokens) {
 
 // act: [tokens][ld_act] with the reduction axis contiguous (X for the forward, dY for the transposed product).
 int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void *val, const int16_t *idx, const void *pat,
-              const void *nval, const void *act, int64_t ld_act, int64_t tokens, const void *bias, void *const *outs, int n_outs,
+              const void *nval, const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, const void *bias, void *const *outs, int n_outs,
               void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi) {
     if (n_outs < 1 || (n_outs > 1 && !dense)) NMG_FAIL(NMG_ERR_UNSUPPORTED, "several output buffers need the two-pass tensor-core variant");
     void *out = outs[0];
@@ -795,6 +824,11 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
         const int64_t ldp = round_up(red, 8);
         const int64_t plane_elems = tokens * ldp;
         if (tokens > 65535 * 16) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
+        if (act_k_major) {
+            const int64_t gy = (tokens + 31) / 32;
+            split_f32_t_kernel<<<dim3((unsigned)((ldp + 63) / 64), (unsigned)(gy < 65535 ? gy : 65535)), 256, 0, st>>>(static_cast<const float *>(act), red, tokens, ld_act, xs, ldp,
+                                                                                                                       plane_elems);
+        } else
         for (int64_t r0 = 0; r0 < tokens; r0 += 65535) {  // grid.y limit
             const int64_t nr = tokens - r0 < 65535 ? tokens - r0 : 65535;
             const int64_t bx = (ldp / 8 + 127) / 128;

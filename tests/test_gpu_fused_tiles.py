@@ -43,3 +43,39 @@ def test_fused_matmul_tiles(n, m, g, M, K, tokens, dtype, tol):
         dy = seeded_normal((tokens, M), 5).to(dtype).to(dev)
         assert rel(ops.spmm_t(val, idx, M, K, n, m, g, dy, algo=nat.NMG_ALGO_TENSOR), dy.double() @ dense) <= tol
     assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 1e-2), (torch.float16, 2e-3)])
+@pytest.mark.parametrize("n,m,g,M,K,tokens", [(1, 8, 16, 1023, 777, 333), (2, 4, 16, 130, 250, 1), (2, 4, 4, 66, 1031, 1500)])
+def test_rows_tma_cannot_read_are_laid_out_again(n, m, g, M, K, tokens, dtype, tol):
+    """Odd reduction lengths, and aligned ones behind an odd offset, on both products; every token count's kernel."""
+    from sten_b200 import ops
+    dev = cuda()
+    w = (seeded_normal((M, K), 1) * K ** -0.5).to(dtype).to(dev)
+    val, idx = ops.sparsify(w.unsqueeze(0), n, m, g)
+    dense = ops.densify(val, idx, 1, M, K, n, m, g)[0].double()
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm())  # noqa: E731
+    for pad in (0, 3):
+        x = seeded_normal((tokens, K + pad), 2).to(dtype).to(dev)[:, pad:]
+        assert rel(ops.spmm(val, idx, M, K, n, m, g, x), x.double() @ dense.t()) <= tol
+        dy = seeded_normal((tokens, M + pad), 5).to(dtype).to(dev)[:, pad:]
+        assert rel(ops.spmm_t(val, idx, M, K, n, m, g, dy), dy.double() @ dense) <= tol
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 1e-2), (torch.float32, 1e-5)])
+@pytest.mark.parametrize("tokens", [1, 33, 63, 64, 200, 700])
+def test_k_major_columns(tokens, dtype, tol):
+    """torch.mm through the plugin: a handful of columns, and the fp32 mode's transposing split at ragged tile edges."""
+    import sten_b200 as sten
+    sten.set_dispatch_failure("raise")
+    dev, M, K = cuda(), 200, 333
+    lin = torch.nn.Linear(K, M, bias=False).to(dev).to(dtype)
+    sb = sten.SparsityBuilder()
+    sb.set_weight("weight", initial_sparsifier=sten.GroupedNMSparsifier(2, 4, 16), out_format=sten.GroupedNMTensor)
+    w = sb.get_sparse_model(lin).weight
+    b = seeded_normal((K, tokens), 7).to(dtype).to(dev)
+    with torch.no_grad():
+        c = torch.mm(w, b)
+    want = w.wrapped_tensor.to_dense().double() @ b.double()
+    assert float((c.double() - want).norm() / want.norm()) <= tol

@@ -121,8 +121,8 @@ int nmg_pack(const void *val, const int16_t *idx, int64_t M, int64_t K, int n, i
  * caller for the duration of the call (may be NULL when the query returns 0).
  * algo: NMG_ALGO_AUTO uses the tensor cores for weights of at least 64 rows, at every token count (16-bit rows that are not
  * 16-byte aligned, and K-major activations, are re-laid out into the workspace first); fewer than 64 K-major columns take
- * them when `packed` is given.  The SIMT kernels serve the rest.  Two tensor-core variants exist.  Below 1280 tokens (256 for
- * fp32), for m in {4, 8, 16} and n <= 2, one fused kernel expands tiles of the packed copy inside the matmul.  From
+ * them when `packed` is given.  The SIMT kernels serve the rest.  Two tensor-core variants exist.  Below 1536 tokens (1024
+ * for fp32), for m in {4, 8, 16} and n <= 2, one fused kernel expands tiles of the packed copy inside the matmul.  From
  * there on, and for every other (n, m), the weight is first expanded into a transient dense 16-bit matrix in the workspace
  * (M * round_up(K, 8) * 2 bytes; three such planes for fp32) and multiplied by a persistent TMA-fed kernel; that
  * variant reads val / idx and ignores `packed`.  fp32 operands go through the tensor cores as exact three-way bf16
@@ -174,7 +174,7 @@ int nmg_pack_sp24(const void *val, const int16_t *idx, int64_t M, int64_t K, int
 int nmg_spmm_t_sp24(const void *sp24, int64_t M, int64_t K, int n, int m, int g, int dtype, const void *dy, int64_t ld_dy,
                     int64_t tokens, void *dx, int64_t ld_dx, void *stream);
 
-/* Opt-in for compute-bound serving: keep the EXPANDED 16-bit weight across calls.  From 1280 tokens on nmg_spmm expands
+/* Opt-in for compute-bound serving: keep the EXPANDED 16-bit weight across calls.  From 1536 tokens on nmg_spmm expands
  * the weight into its workspace on every call (about M * K * 2.5 bytes of HBM traffic); a caller that prefers speed over
  * the format's memory saving expands once (nmg_expand: M * round_up(K, 8) * 2 bytes) and calls nmg_spmm_expanded, which
  * runs the tensor-core matmul and the fused epilogue of nmg_spmm_fused alone.  The counterpart of the kernel-choice knob

@@ -18,7 +18,7 @@ struct ExpandParams {
     int64_t ld, plane_elems;
     int64_t M, K, nb, nc;
     int n, m, g, C, cc;
-    int R;                  // row-blocks per work item
+    int R, Q;               // row-blocks and (rows kernel) column chunks per work item
     int pitch;              // elements per line of the shared-memory tile
 };
 

@@ -20,7 +20,7 @@ int launch_widen_to_f32(const void *src, int dtype, int64_t rows, int64_t cols, 
 
 // Column-order ("natural") copy of a weight: for every row-block mb and column k of the padded width Kp,
 // pat[mb][k] = pattern of that column (id * m in one byte for the specialised patterns, else a 16-bit id), nval[mb][k][s] = its n kept values.
-struct NaturalLayout { size_t pat_bytes, val_bytes, mask_bytes, total; };
+struct NaturalLayout { size_t pat_bytes, val_bytes, mask_bytes, plane_bytes, total; };
 NaturalLayout natural_layout(const Geo &geo, int dtype);
 int64_t natural_width(const Geo &geo);
 int64_t natural_mask_rows(const Geo &geo);  // rows of the row masks: M rounded up to the tensor-core tile
@@ -42,7 +42,7 @@ int simt_bwd(const Geo &geo, int dtype, const void *pat, const void *nval, const
 // entry point tc_matmul: the fused kernel (nmg_spmm_tc.cu) expands the column-ordered copy (pat / nval) tile by tile
 // inside the matmul; the two-pass variant (nmg_gemm_tc.cu, `dense` = true) first expands (val, idx) into a dense 16-bit
 // matrix in `ws` (tc_dense_workspace_bytes, after the split activation) and multiplies that.  tc_use_dense is the
-// policy: two passes from 1280 tokens on (256 for fp32), and for every (n, m) the fused kernel has no instantiation for.
+// policy: two passes for large batches, and for every (n, m) the fused kernel has no instantiation for.
 // What follows the product: out = activation(product + bias) + residual.  The two-pass tensor-core matmul applies it in its
 // epilogue; every other kernel is followed by one elementwise pass (launch_epilogue).
 struct Epilogue {
@@ -56,7 +56,7 @@ bool tc_dense_uses_pair(const Geo &geo, int dtype, bool transposed);
 
 bool tc_supported(const Geo &geo, int dtype);        // fused kernel
 bool tc_dense_supported(const Geo &geo, int dtype);  // two-pass variant
-bool tc_use_dense(const Geo &geo, int dtype, int64_t tokens);
+bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens);
 size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens);
 size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed);
 // outs / n_outs: the result goes to every listed buffer (same shape and pitch); more than one needs `dense`.  mc_out, when

@@ -17,6 +17,7 @@ namespace nmg {
 // ------------------------------------------------------------------------------------------ column-ordered copy
 struct NaturalParams {
     const void *val; const int16_t *idx; void *pat; void *nval;
+    __nv_bfloat16 *planes;  // fp32 weights the tensor-core kernel serves: three bf16 planes, else NULL
     int64_t nb, nc, Kp;
     int n, m, g, cc;
     int wide;    // 16-bit pattern ids
@@ -38,7 +39,21 @@ __global__ void build_natural_kernel(const NaturalParams prm) {
         const int64_t o = mb * prm.Kp + (int64_t)kc * prm.cc + c;
         if (prm.wide) static_cast<uint16_t *>(prm.pat)[o] = (uint16_t)(slot / prm.g);
         else static_cast<uint8_t *>(prm.pat)[o] = (uint8_t)(slot / prm.g * prm.m);
-        for (int s = 0; s < prm.n; s++) nval[prm.planar ? (o & ~(int64_t)1) * 2 + s * 2 + (o & 1) : o * prm.n + s] = val[(int64_t)e * prm.n + s];
+        for (int s = 0; s < prm.n; s++) {
+            const int64_t d = prm.planar ? (o & ~(int64_t)1) * 2 + s * 2 + (o & 1) : o * prm.n + s;
+            const T v = val[(int64_t)e * prm.n + s];
+            nval[d] = v;
+            if (sizeof(T) == 4 && prm.planes) {  // exact three-way split
+                const int64_t plane = prm.nb * prm.Kp * prm.n;
+                const float f = DT<T>::to_f32(v);
+                const __nv_bfloat16 hi = __float2bfloat16_rn(f);
+                const float r1 = f - __bfloat162float(hi);
+                const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
+                prm.planes[d] = hi;
+                prm.planes[plane + d] = mid;
+                prm.planes[2 * plane + d] = __float2bfloat16_rn(r1 - __bfloat162float(mid));
+            }
+        }
     }
 }
 
@@ -83,7 +98,8 @@ static bool bwd_specialised(int n, int m) {
 int64_t natural_width(const Geo &geo) { return round_up(geo.nc * geo.cc, 128); }
 
 // Sections of the copy: one pattern entry per column, the values in the weight's dtype and, where the tensor-core kernel
-// serves the pattern, the row masks.  The patterns with specialised
+// serves the pattern, the row masks and an fp32 weight's values split into three bf16 planes (split in the kernel, every one
+// of a block's m rows would repeat the conversions: 4096 x 4096 2:4, 256 tokens 132 us).  The patterns with specialised
 // kernels (at most 28) store one byte, pattern id times m: the offset of the pattern's row selectors in the expansion table of
 // the tensor-core kernel; with n = 2 their values are stored pair-wise planar.  All others store 16-bit ids.
 NaturalLayout natural_layout(const Geo &geo, int dtype) {
@@ -92,7 +108,8 @@ NaturalLayout natural_layout(const Geo &geo, int dtype) {
     l.pat_bytes = (entries * (bwd_specialised(geo.n, geo.m) ? 1 : 2) + 255) & ~(size_t)255;
     l.val_bytes = (entries * geo.n * dtype_size(dtype) + 255) & ~(size_t)255;
     l.mask_bytes = tc_supported(geo, dtype) ? (size_t)(natural_width(geo) / 64) * (size_t)natural_mask_rows(geo) * 8 * geo.n : 0;
-    l.total = l.pat_bytes + l.val_bytes + l.mask_bytes;
+    l.plane_bytes = (dtype == NMG_F32 && tc_supported(geo, dtype)) ? (3 * entries * geo.n * 2 + 255) & ~(size_t)255 : 0;
+    l.total = l.pat_bytes + l.val_bytes + l.mask_bytes + l.plane_bytes;
     return l;
 }
 int64_t natural_mask_rows(const Geo &geo) { return round_up(geo.M, 128); }
@@ -104,15 +121,19 @@ size_t natural_bytes(const Geo &geo, int dtype, size_t *pat_bytes_out) {
 }
 
 int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16_t *idx, void *pat, void *nval, cudaStream_t st) {
-    NaturalParams p{val, idx, pat, nval, geo.nb, geo.nc, natural_width(geo), geo.n, geo.m, geo.g, geo.cc, bwd_specialised(geo.n, geo.m) ? 0 : 1,
+    const NaturalLayout lay = natural_layout(geo, dtype);
+    NaturalParams p{val, idx, pat, nval, nullptr, geo.nb, geo.nc, natural_width(geo), geo.n, geo.m, geo.g, geo.cc, bwd_specialised(geo.n, geo.m) ? 0 : 1,
                     bwd_specialised(geo.n, geo.m) && geo.n == 2 ? 1 : 0};
     const int64_t total = geo.nb * geo.nc * geo.cc;
     int64_t blocks = (total + 255) / 256;
     if (blocks > 148 * 64) blocks = 148 * 64;
     // every (mb, k) of the chunks is written exactly once because idx is a permutation per tile; clear first so that the
     // columns between the last chunk and the padded width, and what a malformed idx leaves out, are zeros
-    const NaturalLayout lay = natural_layout(geo, dtype);
     NMG_CUDA(cudaMemsetAsync(pat, 0, lay.pat_bytes + lay.val_bytes, st));  // the values follow the patterns
+    if (lay.plane_bytes) {
+        p.planes = reinterpret_cast<__nv_bfloat16 *>(static_cast<char *>(nval) + lay.val_bytes + lay.mask_bytes);
+        NMG_CUDA(cudaMemsetAsync(p.planes, 0, lay.plane_bytes, st));
+    }
     if (total < 0x40000000ll) {
         NMG_DISPATCH_DTYPE(dtype, T, (build_natural_kernel<T, true><<<(unsigned)blocks, 256, 0, st>>>(p)));
     } else {

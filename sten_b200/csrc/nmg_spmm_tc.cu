@@ -39,15 +39,16 @@ struct TcParams {
     int act;              // NMG_EPI_NONE / NMG_EPI_GELU applied to (product + bias)
     void *out;
     const char *masks;    // forward: row masks [k-block][mask_rows][8 n bytes]
-    int64_t mask_rows;
+    int64_t mask_rows, nb;
     int64_t out_feats;    // M (forward) or K (transposed)
     int64_t red;          // reduction length: K (forward) or M (transposed)
     int64_t ntok, ld_out;
     int out_token_major;  // 1: out[token][feature], 0: out[feature][token]
     int out_vec;          // token-major 16-bit: rows are 4-byte aligned and hold an even count; feature-major: rows are 16-byte aligned
     int tiles_f, tiles_t; // output tiles along features / tokens
-    int bn;               // tokens per tile: a multiple of 32, at most 256 (96 for fp32)
+    int bn;               // tokens per tile: a multiple of 32, at most 256 (128 for fp32)
     int stages, slots;    // ring depths, from fx_plan
+    int groups;           // expansion groups at work: 3, or 2 with two stages
     int ksplit;           // CTAs per tile = cluster size: each takes one range of the reduction axis
     int exch_off;         // exchange area of the partial tiles: offset in shared memory; 0 = on top of the rings
     int misc_off;         // selector table and barriers
@@ -56,7 +57,7 @@ struct TcParams {
 };
 struct FxMaps {
     CUtensorMap x[3];  // activation planes, box 64 x bn, 128-byte swizzle
-    CUtensorMap val;   // values [nb][Kpn * n]: box 128 bytes x 128/m row-blocks, 128-byte swizzle (forward), or 128 columns x 64/m (transposed)
+    CUtensorMap val;   // forward: 16-bit values [planes * nb][Kpn * n], box 64 x 128/m row-blocks, 128-byte swizzle; transposed: [nb][Kpn * n], box 128 columns x 64/m
     CUtensorMap pat;   // transposed: pattern bytes [nb][Kpn], box 128 columns x 64/m row-blocks
 };
 
@@ -104,9 +105,10 @@ template <int M_> __device__ __forceinline__ void piece_offsets(int row, uint32_
     for (int i = 0; i < 8; i++) off[i] = rb * 128u + (((uint32_t)i ^ rb) & 7u) * 16u;
 }
 
-template <int N_, int M_, typename T, int PLANES>
+// vals: PLANES planes of 16-bit values
+template <int N_, int M_, int PLANES>
 __device__ __forceinline__ void expand_forward(const char *vals, const char *masks, uint32_t a_tmem, int row, const uint32_t (&off)[8]) {
-    constexpr int BOX = (TC_BM / M_) * 128;
+    constexpr int BOX = (TC_BM / M_) * 128, PLANE = BOX * N_;
     uint32_t mask[N_][2];  // 32 columns per word
     if constexpr (N_ == 2) {
         const uint4 k = *reinterpret_cast<const uint4 *>(masks + row * 16);
@@ -115,41 +117,35 @@ __device__ __forceinline__ void expand_forward(const char *vals, const char *mas
         const uint2 k = *reinterpret_cast<const uint2 *>(masks + row * 8);
         mask[0][0] = k.x; mask[0][1] = k.y;
     }
-    auto piece = [&](int box, int i) { return *reinterpret_cast<const uint4 *>(vals + box * BOX + off[i]); };
+    auto piece = [&](int pl, int box, int i) { return *reinterpret_cast<const uint4 *>(vals + pl * PLANE + box * BOX + off[i]); };
 #pragma unroll
     for (int h = 0; h < 2; h++) {
         uint32_t w[PLANES][16];
-        if constexpr (PLANES == 1 && N_ == 1) {  // eight columns per piece
+        if constexpr (N_ == 1) {  // eight columns per piece
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const uint4 v = piece(0, h * 4 + i);
-                w[0][4 * i] = v.x & pair_mask(mask[0][h], 2 * i, 0);
-                w[0][4 * i + 1] = v.y & pair_mask(mask[0][h], 2 * i, 1);
-                w[0][4 * i + 2] = v.z & pair_mask(mask[0][h], 2 * i + 1, 0);
-                w[0][4 * i + 3] = v.w & pair_mask(mask[0][h], 2 * i + 1, 1);
+                const uint32_t m0 = pair_mask(mask[0][h], 2 * i, 0), m1 = pair_mask(mask[0][h], 2 * i, 1);
+                const uint32_t m2 = pair_mask(mask[0][h], 2 * i + 1, 0), m3 = pair_mask(mask[0][h], 2 * i + 1, 1);
+#pragma unroll
+                for (int pl = 0; pl < PLANES; pl++) {
+                    const uint4 v = piece(pl, 0, h * 4 + i);
+                    w[pl][4 * i] = v.x & m0;
+                    w[pl][4 * i + 1] = v.y & m1;
+                    w[pl][4 * i + 2] = v.z & m2;
+                    w[pl][4 * i + 3] = v.w & m3;
+                }
             }
-        } else if constexpr (PLANES == 1) {  // four columns: first values, second values of a pair, twice
+        } else {  // four columns: first values, second values of a pair, twice
 #pragma unroll
             for (int q = 0; q < 8; q++) {
-                const uint4 v = piece(h, q);
-                w[0][2 * q] = (v.x & pair_mask(mask[0][h], q, 0)) | (v.y & pair_mask(mask[N_ - 1][h], q, 0));
-                w[0][2 * q + 1] = (v.z & pair_mask(mask[0][h], q, 1)) | (v.w & pair_mask(mask[N_ - 1][h], q, 1));
-            }
-        } else {
+                const uint32_t a0 = pair_mask(mask[0][h], q, 0), a1 = pair_mask(mask[N_ - 1][h], q, 0);
+                const uint32_t b0 = pair_mask(mask[0][h], q, 1), b1 = pair_mask(mask[N_ - 1][h], q, 1);
 #pragma unroll
-            for (int p = 0; p < 16; p++) {  // pair by pair: n = 1 half a piece, n = 2 one piece (first values, second values)
-                uint32_t x[N_][3];
-                if constexpr (N_ == 1) {
-                    const float2 v = *reinterpret_cast<const float2 *>(vals + h * BOX + off[p >> 1] + (p & 1) * 8);
-                    split3_pair(v.x, v.y, x[0][0], x[0][1], x[0][2]);
-                } else {
-                    const uint4 v = piece(2 * h + (p >> 3), p & 7);
-                    split3_pair(__uint_as_float(v.x), __uint_as_float(v.y), x[0][0], x[0][1], x[0][2]);
-                    split3_pair(__uint_as_float(v.z), __uint_as_float(v.w), x[N_ - 1][0], x[N_ - 1][1], x[N_ - 1][2]);
+                for (int pl = 0; pl < PLANES; pl++) {
+                    const uint4 v = piece(pl, h, q);
+                    w[pl][2 * q] = (v.x & a0) | (v.y & a1);
+                    w[pl][2 * q + 1] = (v.z & b0) | (v.w & b1);
                 }
-                const uint32_t m0 = pair_mask(mask[0][h], p >> 1, p & 1), m1 = N_ == 2 ? pair_mask(mask[N_ - 1][h], p >> 1, p & 1) : 0u;
-#pragma unroll
-                for (int pl = 0; pl < PLANES; pl++) w[pl][p] = N_ == 2 ? ((x[0][pl] & m0) | (x[N_ - 1][pl] & m1)) : (x[0][pl] & m0);
             }
         }
 #pragma unroll
@@ -230,9 +226,12 @@ constexpr int FX_THREADS = 32 * 15;
 constexpr int FX_MAX_STAGES = 8, FX_MAX_SLOTS = 12;
 constexpr int FX_SMEM_LIMIT = 224 * 1024;
 constexpr int FX_MISC_BYTES = 512 + FX_TABLE_BYTES;
-struct FxPlan { int stages, slots, exch_off; uint32_t tmem_cols; size_t total; };
+struct FxPlan { int stages, slots, groups, exch_off; uint32_t tmem_cols; size_t total; };
+__host__ __device__ constexpr int fx_val_bytes(int n, int m, int es, bool transposed) {  // forward fp32: three 16-bit planes
+    return 128 * TC_BK / m * n * (es == 4 && !transposed ? 6 : es);
+}
 __host__ __device__ constexpr int fx_slot_bytes(int n, int m, int es, bool transposed) {  // values, then masks (forward) or pattern bytes
-    return 128 * TC_BK / m * n * es + (transposed ? 128 * TC_BK / m : 128 * 8 * n);
+    return fx_val_bytes(n, m, es, transposed) + (transposed ? 128 * TC_BK / m : 128 * 8 * n);
 }
 // columns per CTA of a cluster in the exchange, a multiple of four.  The area is [source][4 columns][128 features][4]: a warp's
 // push is 512 consecutive bytes (16-byte pieces scattered over feature rows moved 16 bytes per clock), and so is its read.
@@ -243,16 +242,18 @@ static FxPlan fx_plan(int planes, int bn, int ks, int slot_bytes) {
     const int acc = planes > 1 ? 2 * bn : bn;  // fp32: accumulator and running tile
     const int exch = ks > 1 ? ks * 128 * fx_cols_per_owner(bn, ks) * 4 : 0;
     const int budget = FX_SMEM_LIMIT - FX_MISC_BYTES - 1024;
-    // A slot always serves the same group and stages are at least as many as groups: no barrier is waited on two phases ahead.
-    const int min_rings = FX_GROUPS * x_bytes + FX_GROUPS * slot_bytes;
-    const int room = exch + min_rings <= budget ? budget - exch : budget;
-    p.slots = 2 * FX_GROUPS;
-    while (p.slots > FX_GROUPS && FX_GROUPS * x_bytes + p.slots * slot_bytes > room) p.slots -= FX_GROUPS;
-    p.stages = (room - p.slots * slot_bytes) / x_bytes;
+    // A slot always serves the same group (slots are a multiple of the groups) and there are at least as many stages as groups:
+    // no barrier is waited on two phases ahead, which a parity wait could not tell apart.
     const int tmem_stages = (512 - acc) / (planes * FX_A_COLS);
+    p.groups = tmem_stages < FX_GROUPS ? tmem_stages : FX_GROUPS;
+    const int min_rings = p.groups * (x_bytes + slot_bytes);
+    const int room = exch + min_rings <= budget ? budget - exch : budget;
+    p.slots = 2 * p.groups;
+    while (p.slots > p.groups && p.groups * x_bytes + p.slots * slot_bytes > room) p.slots -= p.groups;
+    p.stages = (room - p.slots * slot_bytes) / x_bytes;
     if (p.stages > tmem_stages) p.stages = tmem_stages;
     if (p.stages > FX_MAX_STAGES) p.stages = FX_MAX_STAGES;
-    while (p.slots + FX_GROUPS <= FX_MAX_SLOTS && p.stages * x_bytes + (p.slots + FX_GROUPS) * slot_bytes <= room) p.slots += FX_GROUPS;
+    while (p.slots + p.groups <= FX_MAX_SLOTS && p.stages * x_bytes + (p.slots + p.groups) * slot_bytes <= room) p.slots += p.groups;
     const int rings = p.stages * x_bytes + p.slots * slot_bytes;
     p.exch_off = (ks > 1 && room < budget) ? (rings + 1023) & ~1023 : 0;
     const int used = p.exch_off ? p.exch_off + exch : (rings > exch ? rings : exch);
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
     using E = typename TcMode<T>::elem;  // element type the tensor cores see
     static_assert(TC_BM % M_ == 0 && 32 % M_ == 0 && M_ % 4 == 0 && N_ <= 2, "tile must hold whole row-blocks; a column's values fit one word");
     static_assert(Order<N_, M_>::C * M_ <= FX_TABLE_BYTES, "a pattern byte is an offset into the selector table");
-    constexpr int SLOT_BYTES = fx_slot_bytes(N_, M_, (int)sizeof(T), TRANSPOSED), VAL_BYTES = 128 * TC_BK / M_ * N_ * (int)sizeof(T);
+    constexpr int SLOT_BYTES = fx_slot_bytes(N_, M_, (int)sizeof(T), TRANSPOSED), VAL_BYTES = fx_val_bytes(N_, M_, (int)sizeof(T), TRANSPOSED);
     static_assert(TRANSPOSED || (SLOT_BYTES % 1024 == 0 && VAL_BYTES % 1024 == 0), "swizzled boxes start on 1024-byte boundaries");
 
     extern __shared__ char smem_raw[];
@@ -395,14 +396,14 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
             tma_load_2d(w, &maps.val, (int)feat0 * N_, y, &full_w[s]);
             tma_load_2d(w + VAL_BYTES, &maps.pat, (int)feat0, y, &full_w[s]);
         } else {
-            constexpr int BOXES = TC_BK * N_ * (int)sizeof(T) / 128, BOX_ELEMS = 128 / (int)sizeof(T);
 #pragma unroll
-            for (int bx = 0; bx < BOXES; bx++)
-                tma_load_2d(w + bx * (TC_BM / M_) * 128, &maps.val, (kb_base + kb) * TC_BK * N_ + bx * BOX_ELEMS, (int)(feat0 / M_), &full_w[s]);
+            for (int bx = 0; bx < PLANES * N_; bx++)  // 64 values per box; the planes lie below one another
+                tma_load_2d(w + bx * (TC_BM / M_) * 128, &maps.val, ((kb_base + kb) * N_ + bx % N_) * TC_BK, bx / N_ * (int)prm.nb + (int)(feat0 / M_), &full_w[s]);
             bulk_load(w + VAL_BYTES, prm.masks + ((int64_t)(kb_base + kb) * prm.mask_rows + feat0) * (8 * N_), 128 * 8 * N_, &full_w[s]);
         }
     };
-    const int lead_x = nkb < 2 ? nkb : 2, lead_w = nkb < FX_GROUPS ? nkb : FX_GROUPS;  // loads issued before the set-up barrier
+    const int groups = prm.groups;
+    const int lead_x = nkb < 2 ? nkb : 2, lead_w = nkb < groups ? nkb : groups;  // loads issued before the set-up barrier
 
     // ---- set-up.  The producers initialise their own barriers and issue every group's first loads before the CTA-wide barrier,
     // so that their latency runs beside the TMEM allocation.
@@ -426,7 +427,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
                 mbar_init(&empty[s], 1);
             }
             mbar_init(chunk_done, 1);
-            mbar_init(promoted, 128);
+            mbar_init(promoted, 4 * FX_GROUPS);
             mbar_init(all_done, 1);
             mbar_init(exchanged, 1);
             mbar_fence_init();
@@ -456,12 +457,12 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
     if (exch_apart) cluster_arrive();
 
     // fp32 mode: a finished chunk of the accumulator is added to the running tile (columns bn .. 2 bn) with round-to-nearest
-    // adds, by the four warps of group 0
+    // adds.  The MMAs wait for it, so all twelve warps take part: each its quarter of the lanes of every third slice.
     auto promote_chunk = [&](int c) -> bool {
         const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
-        if (!mbar_wait_bounded(chunk_done, (uint32_t)(c & 1), prm.status, 15)) return false;
+        if (!__all_sync(0xffffffffu, mbar_wait_bounded(chunk_done, (uint32_t)(c & 1), prm.status, 15))) return false;
         tc_fence_after();
-        for (int sl = 0; sl < bn / 32; sl++) {
+        for (int sl = warp >> 2; sl < bn / 32; sl += FX_GROUPS) {
             uint32_t r[32];
             tmem_ld32(lane_base + (uint32_t)(sl * 32), r);
             if (c > 0) {
@@ -473,7 +474,8 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
             tmem_st32(lane_base + (uint32_t)(bn + sl * 32), r);
         }
         tc_fence_before();
-        mbar_arrive(promoted);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(promoted);
         return true;
     };
 
@@ -537,14 +539,14 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
     } else {
         // ------------------------------------------------------------------ expansion groups
         const int group = warp >> 2, gtid = tid & 127;
-        int drained = 0;  // group 0: accumulation chunks already promoted
+        int drained = 0;  // fp32: accumulation chunks already promoted
         int s = group, w = group;
         uint32_t ph = 0, phw = 0;
         const uint32_t a_lane = a_base + ((uint32_t)((warp & 3) * 32) << 16);
         uint32_t off[8];
         if constexpr (!TRANSPOSED) piece_offsets<M_>(gtid, off);
-        for (int kb = group; kb < nkb; kb += FX_GROUPS) {
-            if (SPLIT && group == 0) {
+        for (int kb = group; group < groups && kb < nkb; kb += groups) {
+            if constexpr (SPLIT) {
                 // Before feeding a later chunk, promote the finished ones: the MMAs of a chunk depend only on tiles that are
                 // already published, so this wait cannot deadlock, and the MMA issuer needs the promotion before it may
                 // restart the accumulator.
@@ -560,18 +562,18 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
             const char *vals = slot0 + w * SLOT_BYTES;
             const uint32_t a_tmem = a_lane + (uint32_t)(s * PLANES * FX_A_COLS);
             if constexpr (TRANSPOSED) expand_transposed<N_, M_, T, PLANES>(vals, vals + VAL_BYTES, table, a_tmem, gtid);
-            else expand_forward<N_, M_, T, PLANES>(vals, vals + VAL_BYTES, a_tmem, gtid, off);
+            else expand_forward<N_, M_, PLANES>(vals, vals + VAL_BYTES, a_tmem, gtid, off);
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_w[w]);  // the slot has been read
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[s]);
-            if ((s += FX_GROUPS) >= stages) { s -= stages; ph ^= 1; }
-            if ((w += FX_GROUPS) >= slots) { w -= slots; phw ^= 1; }
+            if ((s += groups) >= stages) { s -= stages; ph ^= 1; }
+            if ((w += groups) >= slots) { w -= slots; phw ^= 1; }
         }
-        if (SPLIT && group == 0)
-            while (ok && drained < nchunks - 1) {  // the chunks behind the last tile this group published
+        if constexpr (SPLIT)
+            while (ok && drained < nchunks - 1) {  // the chunks behind the last tile this group published (all of them for an idle group)
                 ok = promote_chunk(drained);
                 drained++;
             }
@@ -659,7 +661,7 @@ bool tc_supported(const Geo &geo, int dtype) {
 constexpr int kFxClusters[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
 struct FxChoice { int bn, tiles_f, tiles_t, ksplit; };
 static FxChoice fx_choose(int64_t feats, int64_t red, int64_t tokens, int dtype) {
-    const int max_bn = dtype == NMG_F32 ? 96 : 256;  // fp32: three stages of three A planes, the accumulator and the running tile share TMEM
+    const int max_bn = dtype == NMG_F32 ? 128 : 256;  // fp32: the accumulator, the running tile and two stages of three A planes share TMEM
     const int64_t tiles_f = (feats + TC_BM - 1) / TC_BM, nkb = (red + TC_BK - 1) / TC_BK;
     FxChoice best{};
     int64_t best_ns = -1;
@@ -762,6 +764,7 @@ static int tc_launch_one(const TcParams &p0, const FxMaps &maps, cudaStream_t st
     TcParams p = p0;
     p.stages = plan.stages;
     p.slots = plan.slots;
+    p.groups = plan.groups;
     p.exch_off = plan.exch_off;
     p.tmem_cols = plan.tmem_cols;
     p.misc_off = (int)(plan.total - 1024 - FX_MISC_BYTES);
@@ -793,15 +796,15 @@ static int tc_launch_nm(int dtype, bool transposed, const TcParams &p, const FxM
     return transposed ? tc_launch_one<N_, M_, __nv_bfloat16, true>(p, maps, st) : tc_launch_one<N_, M_, __nv_bfloat16, false>(p, maps, st);
 }
 
-// Policy of the two tensor-core variants.
-bool tc_use_dense(const Geo &geo, int dtype, int64_t tokens) {
+// Policy of the two tensor-core variants.  Measured (us, fused / two passes; 2:4): bf16 4096 x 4096 29 / 44 at 1024 tokens,
+// 53 / 62 at 1280, 56 / 64 at 2048, 85 / 86 at 3072; 4096 x 1024 12 / 18 at 1024, 21 / 22 at 1536, 33 / 28 at 3072.  fp32
+// 4096 x 1024 27 / 50 at 512 tokens, 51 / 52 at 1024, 97 / 91 at 2048; 4096 x 4096 168 / 187 at 1024, 336 / 338 at 2048.
+// The transposed product of a 16-bit weight has the structured-sparse kernel in place of the second variant (from 1280 tokens).
+bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens) {
     const bool fused = tc_supported(geo, dtype), dense = tc_dense_supported(geo, dtype);
     if (!dense) return false;
     if (!fused) return true;
-    // Measured crossover (4096^2 and 16384^2 bf16 weights): a tie around 1024 tokens (0.055 / 0.053 ms and 0.567 / 0.598 ms,
-    // fused / two-pass), two passes clearly ahead at 1536 (0.099 / 0.072 ms and 0.836 / 0.799 ms); fp32 (six split products,
-    // so six in-kernel expansions per tile) prefers two passes from 256 tokens.
-    return tokens >= (dtype == NMG_F32 ? 256 : 1280);
+    return tokens >= (dtype == NMG_F32 ? 1024 : transposed ? 1280 : 1536);
 }
 
 // act: [tokens][ld_act] with the reduction axis contiguous (X for the forward, dY for the transposed product).
@@ -858,13 +861,16 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     FxMaps maps;
     for (int c = 0; c < 3; c++) maps.x[c] = tm[c];
     const int64_t Kpn = natural_width(geo);
-    const char *masks = static_cast<const char *>(nval) + natural_layout(geo, dtype).val_bytes;
+    const NaturalLayout lay = natural_layout(geo, dtype);
+    const char *masks = static_cast<const char *>(nval) + lay.val_bytes;
+    const uint64_t row_elems = (uint64_t)(Kpn * geo.n);
     if (transposed) {
         if ((rc = encode_tmap_2d_bytes(&maps.pat, pat, (uint64_t)Kpn, (uint64_t)geo.nb, (uint64_t)Kpn, TC_BM, (uint32_t)(TC_BK / geo.m)))) return rc;
-        if ((rc = encode_tmap_2d(&maps.val, dtype, nval, (uint64_t)(Kpn * geo.n), (uint64_t)geo.nb, (uint64_t)(Kpn * geo.n), (uint32_t)(TC_BM * geo.n), (uint32_t)(TC_BK / geo.m), 0)))
-            return rc;
+        if ((rc = encode_tmap_2d(&maps.val, dtype, nval, row_elems, (uint64_t)geo.nb, row_elems, (uint32_t)(TC_BM * geo.n), (uint32_t)(TC_BK / geo.m), 0))) return rc;
     } else {
-        if ((rc = encode_tmap_2d(&maps.val, dtype, nval, (uint64_t)(Kpn * geo.n), (uint64_t)geo.nb, (uint64_t)(Kpn * geo.n), (uint32_t)(128 / dtype_size(dtype)), (uint32_t)(TC_BM / geo.m), 1)))
+        const bool split = dtype == NMG_F32;
+        if ((rc = encode_tmap_2d(&maps.val, split ? NMG_BF16 : dtype, split ? masks + lay.mask_bytes : nval, row_elems, (uint64_t)(geo.nb * (split ? 3 : 1)), row_elems, TC_BK,
+                                 (uint32_t)(TC_BM / geo.m), 1)))
             return rc;
         maps.pat = maps.val;  // never used; keeps the parameter defined
     }
@@ -875,7 +881,7 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     p.out_vec = out_token_major ? (ld_out % 2 == 0 && feats % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0)
                                 : (ld_out * es % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0);
     p.tiles_f = fx.tiles_f; p.tiles_t = fx.tiles_t; p.bn = fx.bn; p.ksplit = fx.ksplit;
-    p.masks = masks; p.mask_rows = natural_mask_rows(geo);
+    p.masks = masks; p.mask_rows = natural_mask_rows(geo); p.nb = geo.nb;
     p.status = status;
     const ProfileEvents pe = take_profile_events();
     if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));

@@ -89,7 +89,7 @@ ProfileEvents take_profile_events();
 
 // One int per device that kernels set to a non-zero code when a bounded wait runs out.
 // the weight-expansion pass of the matmul path used as the densifier (nmg_gemm_tc.cu)
-bool tc_expand_plain_supported(const Geo &geo, int dtype, const void *dense, int64_t ld);
+bool tc_expand_plain_supported(const Geo &geo, int dtype, const void *val, const int16_t *idx, const void *dense, int64_t ld);
 int tc_expand_plain(const Geo &geo, int dtype, const void *val, const int16_t *idx, void *dense, int64_t ld, cudaStream_t st);
 int get_status_word(int **dev_ptr);
 int device_sms(int *sms_out);  // SM count of the current device, queried once per device

@@ -19,6 +19,7 @@ struct ExpandParams {
     int64_t M, K, nb, nc;
     int n, m, g, C, cc;
     int R, Q;               // row-blocks and (rows kernel) column chunks per work item
+    int vec;                // the destination's rows take 16-byte stores
     int pitch;              // elements per line of the shared-memory tile
 };
 

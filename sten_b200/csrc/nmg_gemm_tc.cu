@@ -206,6 +206,17 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
         const int span = (int)(item / groups), grp = (int)(item - (int64_t)span * groups);
         const int64_t r0 = (int64_t)grp * rows, c0 = (int64_t)span * cols;
         const int row_lim = (int)(prm.M - r0 < rows ? prm.M - r0 : rows), col_lim = (int)(prm.K - c0 < cols ? prm.K - c0 : cols);
+        if (PLAIN && !prm.vec) {  // rows of the destination are not 16-byte aligned: neighbouring threads store neighbouring elements
+            const int dle = EXPAND_THREADS / cols, dee = EXPAND_THREADS - dle * cols;
+            for (int v = tid, l = tid / cols, e = tid - l * cols; v < rows * cols; v += EXPAND_THREADS) {
+                if (l < row_lim && e < col_lim) static_cast<T *>(prm.dst)[(r0 + l) * prm.ld + c0 + e] = tile[v];
+                tile[v] = DT<T>::from_f32(0.f);
+                l += dle;
+                if ((e += dee) >= cols) { e -= cols; l++; }
+            }
+            __syncthreads();
+            continue;
+        }
         // A vector that starts inside the weight may run past K only into the row's padding (ld = round_up(K, 8)).
         for (int v = tid, l = l0, e = e0; v < total; v += EXPAND_THREADS) {
             T *line = tile + v * V;
@@ -860,7 +871,7 @@ bool tc_dense_uses_pair(const Geo &geo, int dtype, bool transposed) {
 
 // (val, idx) -> the weight with its zeros restored, rows `ld` elements apart at `dst` (16-byte aligned, ld a multiple of 8).
 // plain = false: the matmul's operand, 16-bit or three bf16 planes for fp32 (plane_rows rows each); plain = true: the
-// weight in its own dtype (the densifier), where full 8-element stores must not run past the row: K a multiple of 8.
+// weight in its own dtype (the densifier), where full stores must not run past the row: K a multiple of 8, or the rows kernel.
 static int expand_to(const Geo &geo, int dtype, bool transposed, bool plain, const void *val, const int16_t *idx, void *dst, int64_t ld,
                      cudaStream_t st) {
     const int64_t rows = transposed ? geo.K : geo.M;
@@ -871,13 +882,14 @@ static int expand_to(const Geo &geo, int dtype, bool transposed, bool plain, con
     ExpandParams ep{};
     ep.val = val; ep.idx = idx; ep.order = tab.order; ep.dst = dst;
     ep.ld = ld; ep.plane_elems = rows * ld;
+    ep.vec = geo.K % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
     ep.M = geo.M; ep.K = geo.K; ep.nb = geo.nb; ep.nc = geo.nc;
     ep.n = geo.n; ep.m = geo.m; ep.g = geo.g; ep.C = geo.C; ep.cc = geo.cc;
     size_t rsmem = 0;
     const bool aligned = ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0;
     if (!transposed && aligned && expand_rows_plan(geo, es, &ep.R, &ep.Q, &rsmem)) {
-        if (dtype == NMG_F16) return expand_rows_launch<__half, false>(ep, rsmem, st);
-        if (dtype == NMG_BF16) return expand_rows_launch<__nv_bfloat16, false>(ep, rsmem, st);
+        if (dtype == NMG_F16) return plain ? expand_rows_launch<__half, true>(ep, rsmem, st) : expand_rows_launch<__half, false>(ep, rsmem, st);
+        if (dtype == NMG_BF16) return plain ? expand_rows_launch<__nv_bfloat16, true>(ep, rsmem, st) : expand_rows_launch<__nv_bfloat16, false>(ep, rsmem, st);
         return plain ? expand_rows_launch<float, true>(ep, rsmem, st) : expand_rows_launch<float, false>(ep, rsmem, st);
     }
     ep.R = expand_rows_per_item(geo, es, transposed);
@@ -895,9 +907,13 @@ int tc_dense_expand(const Geo &geo, int dtype, bool transposed, const void *val,
     return expand_to(geo, dtype, transposed, false, val, idx, dense, dense_ld(transposed ? geo.M : geo.K), st);
 }
 
-// The densifier through the expansion pass: whole tiles are scattered into shared memory and leave as 16-byte stores.
-bool tc_expand_plain_supported(const Geo &geo, int dtype, const void *dense, int64_t ld) {
+// The densifier through the expansion pass: whole tiles are scattered into shared memory and leave as 16-byte stores, or, from
+// the rows kernel and whatever the destination's alignment, element by element.
+bool tc_expand_plain_supported(const Geo &geo, int dtype, const void *val, const int16_t *idx, const void *dense, int64_t ld) {
     const size_t es = dtype == NMG_F32 ? 4 : 2;
+    int R, Q;
+    size_t smem;
+    if (geo.C <= 65535 && ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0 && expand_rows_plan(geo, es, &R, &Q, &smem)) return true;
     if (geo.cc > 32767 || geo.C > 65535 || geo.K % 8 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(dense) & 15) != 0) return false;
     return expand_smem_bytes(geo, es, false, expand_rows_per_item(geo, es, false)) <= 200 * 1024;
 }

@@ -43,6 +43,11 @@ __device__ __forceinline__ void tile_coords(int64_t tile, int64_t nb, int64_t nc
     }
 }
 
+static int sm_count() {
+    int sms = 148;
+    return device_sms(&sms) == NMG_OK ? sms : 148;
+}
+
 struct SparsifyParams {
     const void *dense;
     void *val;
@@ -503,6 +508,346 @@ __global__ void __launch_bounds__(256, 4) sparsify_nm_kernel(SparsifyParams prm)
     }
 }
 
+// ---- several tiles per warp: few patterns ----------------------------------------------------------------------------
+// L lanes per tile, 32 / L tiles per warp.  The selection is bound by instructions and by the latency of its dependent steps;
+// with a warp per tile most lanes idle after the first round, where a few displaced columns are left (counted on random
+// weights, 2:4, g = 16: 12 more proposals per 96-column tile).
+//   round 0   every column's best pattern from registers, four columns per lane and step; the proposals are grouped by
+//             pattern, and a proposal's place in its pattern's sorted list is its rank among them.
+//   rounds    every lane lets one of its displaced columns propose to the best pattern that would keep it (a pattern's
+//             threshold is the score of its weakest kept entry); the lanes that own the patterns insert what they were
+//             sent, at the same time, and hand the entry that falls out back to its column's lane.
+//   zeros     scores of zero are placed by the closed form of sparsify_zero_phase.
+// Entries are 64-bit keys, score above column + 1: one comparison is the format's order.  The tile is staged in shared memory
+// (16-byte asynchronous copies where the alignment allows).  A tile's slab is 32 bytes more than a multiple of 128, so that
+// the tiles of a warp use different banks.
+// 4096 x 4096, before (a warp per tile) and now: 2:4 fp32 187 -> 127 us, bf16 184 -> 111, 1:4 fp32 173 -> 98, 1:8 fp32 93 -> 80
+// (there all 32 lanes), 1:8 g = 4 fp16 195 -> 72.  Of the instructions ranking takes 40 %, the later rounds 25 %.  Tried and
+// slower: sorting a pattern per lane by a network (139), the tile left in global memory for more resident warps (129).
+struct SparsifyLanes { int xs, x, in, list, prop, thr, sent, cnt, off, fmask, zmask, words, total; };
+__host__ __device__ inline SparsifyLanes sparsify_lanes(int m, int cc, int C, int lanes, int es) {
+    SparsifyLanes l;
+    const int quads = (cc + 3) / 4;
+    int o = 0;
+    l.words = ((quads + lanes - 1) / lanes * 4 + 31) / 32;  // one bit per column of a lane
+    l.xs = quads * 4;                                       // row stride of the staged tile
+    l.x = o;      o += m * l.xs * es;                       // [m][xs] the tile
+    l.in = o = (o + 15) & ~15; o += (cc + 2 * C) * 8;       // round 0: proposals grouped by pattern, every group padded to 2
+    l.list = o = (o + 15) & ~15; o += l.xs * 8;             // [C][g] kept entries, descending (round 0: by column)
+    l.prop = o;   o += lanes * 8;                           // later rounds: the proposal of every lane
+    l.thr = o = (o + 15) & ~15; o += C * 4;                 // smallest score that a pattern may still keep
+    l.sent = o;   o += C * 4;                               // lanes that propose to the pattern
+    l.cnt = o;    o += C * 4;
+    l.off = o;    o += C * 4;
+    l.fmask = o;  o += lanes * l.words * 4;                 // displaced columns of every lane
+    l.zmask = o;  o += lanes * l.words * 4;                 // columns with no open pattern above zero
+    l.total = ((o + 127) & ~127) + 32;
+    return l;
+}
+
+template <typename T> __device__ __forceinline__ void load_quad(const T *p, float *a) {  // magnitudes of four staged neighbours
+    if constexpr (sizeof(T) == 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(p);
+        a[0] = fabsf(v.x); a[1] = fabsf(v.y); a[2] = fabsf(v.z); a[3] = fabsf(v.w);
+    } else {
+        __align__(8) T v[4];
+        *reinterpret_cast<uint2 *>(v) = *reinterpret_cast<const uint2 *>(p);
+#pragma unroll
+        for (int u = 0; u < 4; u++) a[u] = fabsf(DT<T>::to_f32(v[u]));
+    }
+}
+
+template <int N_, int M_, int L, typename T>
+__global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm) {
+    extern __shared__ __align__(16) char smem[];
+    constexpr Order<N_, M_> ORD{};
+    constexpr int C = Order<N_, M_>::C, TILES = 32 / L;
+    static_assert(C <= 31, "pattern 31 marks a column without a proposal");
+    constexpr int V = 16 / (int)sizeof(T);
+    constexpr uint32_t FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    const int sub = lane / L, sl = lane % L;  // tile of the warp, lane of the tile
+    const int g = prm.g, cc = prm.cc;
+    int8_t *ord = reinterpret_cast<int8_t *>(smem);  // run-time copy of the table for the output stage
+    constexpr int ORD_BYTES = (C * N_ + 15) & ~15;
+    for (int i = threadIdx.x; i < C * N_; i += blockDim.x) ord[i] = (int8_t)ORD.v[(i / N_) * Order<N_, M_>::LD + (i % N_)];
+    __syncthreads();
+
+    const SparsifyLanes lay = sparsify_lanes(M_, cc, C, L, (int)sizeof(T));
+    char *slab = smem + ORD_BYTES + (warp * TILES + sub) * lay.total;
+    T *x = reinterpret_cast<T *>(slab + lay.x);
+    uint64_t *in = reinterpret_cast<uint64_t *>(slab + lay.in), *list = reinterpret_cast<uint64_t *>(slab + lay.list);
+    uint64_t *prop = reinterpret_cast<uint64_t *>(slab + lay.prop);
+    uint32_t *thr = reinterpret_cast<uint32_t *>(slab + lay.thr), *sent = reinterpret_cast<uint32_t *>(slab + lay.sent);
+    int *cnt = reinterpret_cast<int *>(slab + lay.cnt), *off = reinterpret_cast<int *>(slab + lay.off);
+    uint32_t *fmask = reinterpret_cast<uint32_t *>(slab + lay.fmask), *zmask = reinterpret_cast<uint32_t *>(slab + lay.zmask);
+    const int words = lay.words, xs = lay.xs, quads = xs >> 2;
+    uint32_t *my_f = fmask + sl * words, *my_z = zmask + sl * words;
+    const bool g_pow2 = (g & (g - 1)) == 0;
+    const int g_shift = 31 - __clz(g);
+    const T *dense = static_cast<const T *>(prm.dense);
+    T *val = static_cast<T *>(prm.val);
+    // column c belongs to lane (c / 4) % L, as bit (c / 4) / L * 4 + c % 4
+    auto give_back = [&](int c) {
+        const int q = c >> 2, bit = (q / L) * 4 + (c & 3);
+        atomicOr(&fmask[(q % L) * words + (bit >> 5)], 1u << (bit & 31));
+    };
+    auto col_of = [](uint64_t key) { return (int)(uint32_t)key - 1; };
+
+    const int64_t stride = (int64_t)gridDim.x * nwarps * TILES;
+    for (int64_t tile0 = ((int64_t)blockIdx.x * nwarps + warp) * TILES; tile0 < prm.tiles; tile0 += stride) {
+        const int64_t tile = tile0 + sub;
+        const bool live = tile < prm.tiles;
+        int64_t mb, kc, b;
+        tile_coords(live ? tile : tile0, prm.nb, prm.nc, prm.tiles, mb, kc, b);
+        const int64_t row0 = mb * M_, col0 = kc * cc;
+        const T *src = dense + b * prm.batch_stride + row0 * prm.ld + col0;  // element (r, c) of the tile at src[r * ld + c]
+        const int rows_ok = (int)(prm.M - row0 < M_ ? prm.M - row0 : M_);    // rows beyond M and columns beyond K read as zero
+        const int cols_ok = (int)(prm.K - col0 < cc ? prm.K - col0 : cc);
+        auto global_at = [&](int r, int c) -> T { return (r < rows_ok && c < cols_ok) ? __ldg(src + r * prm.ld + c) : DT<T>::from_f32(0.f); };
+        // ---- the tile
+        if (rows_ok == M_ && cols_ok == cc && (cc % V) == 0 && (prm.ld % V) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+#pragma unroll
+            for (int r = 0; r < M_; r++)
+                for (int v = sl * V; v < cc; v += L * V) cp_async_16(x + r * xs + v, src + r * prm.ld + v);
+            cp_async_commit();
+        } else {
+            for (int r = 0; r < M_; r++)
+                for (int c = sl; c < xs; c += L) x[r * xs + c] = global_at(r, c);
+        }
+        for (int p = sl; p < C; p += L) cnt[p] = 0;
+        for (int w = 0; w < words; w++) my_f[w] = my_z[w] = 0;
+        cp_async_wait<0>();
+        __syncwarp();
+
+        // ---- round 0: proposals.  By column: score, number within the pattern (in no order), pattern (31: none)
+        for (int q = sl, bit = 0; q < quads; q += L, bit += 4) {
+            float a[M_][4];
+#pragma unroll
+            for (int r = 0; r < M_; r++) load_quad(x + r * xs + q * 4, a[r]);
+            uint32_t best_s[4] = {0, 0, 0, 0};
+            int best_p[4] = {0, 0, 0, 0};
+            // the sum starts from the first value (0 + x = x exactly for x >= 0); a zero maximum means that every score is zero
+#pragma unroll
+            for (int p = 0; p < C; p++)
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    float sc = a[ORD.row(p, 0)][u];
+#pragma unroll
+                    for (int i = 1; i < N_; i++) sc = __fadd_rn(sc, a[ORD.row(p, i)][u]);
+                    const uint32_t sb = __float_as_uint(sc);
+                    if (sb >= best_s[u]) { best_s[u] = sb; best_p[u] = p; }
+                }
+            uint32_t zero = 0, w[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                w[u] = 31;
+                if (best_s[u] != 0) w[u] = (uint32_t)best_p[u] | ((uint32_t)atomicAdd(&cnt[best_p[u]], 1) << 5);
+                else if (q * 4 + u < cc) zero |= 1u << u;
+            }
+            if (zero) my_z[bit >> 5] |= zero << (bit & 31);
+            uint4 *by_col = reinterpret_cast<uint4 *>(list + q * 4);
+            by_col[0] = make_uint4(w[0], best_s[0], w[1], best_s[1]);
+            by_col[1] = make_uint4(w[2], best_s[2], w[3], best_s[3]);
+        }
+        __syncwarp();
+        for (int p = sl; p < C; p += L) {
+            int o = 0;
+            for (int r = 0; r < p; r++) o += (cnt[r] + 1) & ~1;
+            off[p] = o;
+            if (cnt[p] & 1) in[o + cnt[p]] = 0;
+        }
+        __syncwarp();
+        for (int c = sl; c < cc; c += L) {
+            const uint64_t e = list[c];
+            const int p = (int)(e & 31);
+            if (p < 31) in[off[p] + ((uint32_t)e >> 5)] = (e & 0xffffffff00000000ull) | (uint32_t)((c + 1) | (p << 16));
+        }
+        __syncwarp();
+        const int slots = off[C - 1] + cnt[C - 1];
+        for (int e = sl; e < slots; e += L) {
+            const uint64_t key = in[e];
+            if (key == 0) continue;  // padding
+            const int p = (int)((uint32_t)key >> 16);
+            const ulonglong2 *from = reinterpret_cast<const ulonglong2 *>(in + off[p]);
+            const int pairs = (cnt[p] + 1) >> 1;
+            int rank = 0;
+#pragma unroll 2
+            for (int j = 0; j < pairs; j++) {
+                const ulonglong2 v = from[j];
+                rank += v.x > key ? 1 : 0;
+                rank += v.y > key ? 1 : 0;
+            }
+            const int c1 = (int)(key & 0xffff);
+            if (rank < g) list[p * g + rank] = (key & 0xffffffff00000000ull) | (uint32_t)c1;
+            else give_back(c1 - 1);
+        }
+        __syncwarp();
+        for (int p = sl; p < C; p += L) {
+            const int n = min(cnt[p], g);
+            cnt[p] = n;
+            thr[p] = n == g ? (uint32_t)(list[p * g + g - 1] >> 32) : 1u;
+            sent[p] = 0;
+        }
+        __syncwarp();
+
+        // ---- later rounds.  Every round with a proposal makes at least one (column, pattern) proposal that was never made
+        // before, so cc * C rounds cannot be exceeded.
+        for (int round = 0; round < cc * C; round++) {
+            uint32_t bits = 0;
+            int w = 0;
+            for (; w < words; w++)
+                if ((bits = my_f[w]) != 0) break;
+            if (!__any_sync(FULL, bits != 0)) break;
+            if (bits) {
+                const int bit = (w << 5) + __ffs(bits) - 1, c = ((bit >> 2) * L + sl) * 4 + (bit & 3);
+                my_f[w] = bits & (bits - 1);
+                float a[M_];
+#pragma unroll
+                for (int r = 0; r < M_; r++) a[r] = fabsf(DT<T>::to_f32(x[r * xs + c]));
+                uint32_t best_s = 0;
+                int best_p = -1;
+#pragma unroll
+                for (int p = 0; p < C; p++) {
+                    float sc = a[ORD.row(p, 0)];
+#pragma unroll
+                    for (int i = 1; i < N_; i++) sc = __fadd_rn(sc, a[ORD.row(p, i)]);
+                    const uint32_t sb = __float_as_uint(sc), t = thr[p];
+                    bool open = sb >= best_s && sb >= t;
+                    if (open && sb == t && cnt[p] == g) open = c > col_of(list[p * g + g - 1]);  // equal score: the larger column wins
+                    if (open) { best_s = sb; best_p = p; }
+                }
+                if (best_p >= 0) {
+                    prop[sl] = ((uint64_t)best_s << 32) | (uint32_t)(c + 1);
+                    atomicOr(&sent[best_p], 1u << sl);
+                } else {
+                    my_z[w] |= bits & -bits;  // nothing above zero is open: placed by the zero phase
+                }
+            }
+            __syncwarp();
+            for (int p = sl; p < C; p += L) {
+                uint32_t from = sent[p];
+                if (from == 0) continue;
+                sent[p] = 0;
+                uint64_t *lp = list + p * g;
+                int n = cnt[p];
+                for (; from; from &= from - 1) {
+                    const uint64_t key = prop[__ffs(from) - 1];
+                    int j = n;
+                    if (n == g) {
+                        const uint64_t last = lp[--j];
+                        give_back(col_of(key < last ? key : last));  // the weakest falls out, a kept entry or the proposal
+                        if (key < last) continue;
+                    } else {
+                        n++;
+                    }
+                    for (; j > 0; j--) {
+                        const uint64_t prev = lp[j - 1];
+                        if (prev > key) break;
+                        lp[j] = prev;
+                    }
+                    lp[j] = key;
+                }
+                cnt[p] = n;
+                if (n == g) thr[p] = (uint32_t)(lp[g - 1] >> 32);
+            }
+            __syncwarp();
+        }
+
+        // ---- zero phase (padded columns, pruned weights): see sparsify_zero_phase
+        uint32_t zeros = 0;
+        for (int w = 0; w < words; w++) zeros |= my_z[w];
+        if (__any_sync(FULL, zeros != 0)) {
+            for (int p = sl; p < C; p += L) {
+                int o = 0;
+                for (int q = p + 1; q < C; q++) o += g - cnt[q];
+                off[p] = o;  // free places in larger patterns
+            }
+            __syncwarp();
+            constexpr uint32_t TILE_LANES = L == 32 ? FULL : (1u << (L & 31)) - 1u;
+            int above = 0;  // free columns with larger indices
+            for (int k = (quads - 1) / L; k >= 0; k--) {
+                const uint32_t nib = (my_z[k >> 3] >> ((k & 7) * 4)) & 15u;
+                int later = 0, all = 0;  // free columns of larger lanes, of all lanes
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const uint32_t mask = (__ballot_sync(FULL, (nib >> u) & 1u) >> (sub * L)) & TILE_LANES;
+                    all += __popc(mask);
+                    later += __popc(sl == 31 ? 0u : mask >> (sl + 1));
+                }
+                for (int u = 3; u >= 0; u--) {
+                    if (((nib >> u) & 1u) == 0) continue;
+                    const int i = above + later++;
+                    int p = C - 1;
+                    while (p > 0 && off[p] + (g - cnt[p]) <= i) p--;  // largest pattern whose range of places contains i
+                    list[p * g + cnt[p] + (i - off[p])] = (uint32_t)((k * L + sl) * 4 + u + 1);
+                }
+                above += all;
+            }
+        }
+        __syncwarp();
+
+        // ---- output
+        if (live) {
+            uint16_t *idx_out = reinterpret_cast<uint16_t *>(prm.idx) + tile * cc;
+            T *val_out = val + tile * (int64_t)cc * N_;
+            if ((cc & 3) == 0 && (reinterpret_cast<uintptr_t>(idx_out) & 7) == 0) {
+                for (int s0 = sl * 4; s0 < cc; s0 += L * 4) {
+                    const ulonglong2 e0 = *reinterpret_cast<const ulonglong2 *>(list + s0), e1 = *reinterpret_cast<const ulonglong2 *>(list + s0 + 2);
+                    const uint32_t lo = (uint32_t)(col_of(e0.x) | (col_of(e0.y) << 16)), hi = (uint32_t)(col_of(e1.x) | (col_of(e1.y) << 16));
+                    *reinterpret_cast<uint2 *>(idx_out + s0) = make_uint2(lo, hi);
+                }
+            } else {
+                for (int s0 = sl; s0 < cc; s0 += L) idx_out[s0] = (uint16_t)col_of(list[s0]);
+            }
+            const int nvals = cc * N_;
+            if ((nvals % V) == 0 && (reinterpret_cast<uintptr_t>(val_out) & 15) == 0) {
+                for (int v = sl * V; v < nvals; v += L * V) {
+                    __align__(16) T out[V];
+#pragma unroll
+                    for (int u = 0; u < V; u++) {
+                        const int e = v + u, s0 = e / N_, t = e % N_;
+                        const int p = g_pow2 ? (s0 >> g_shift) : s0 / g;
+                        out[u] = x[(int)ord[p * N_ + t] * xs + col_of(list[s0])];
+                    }
+                    *reinterpret_cast<uint4 *>(val_out + v) = *reinterpret_cast<const uint4 *>(out);
+                }
+            } else {
+                for (int e = sl; e < nvals; e += L) {
+                    const int s0 = e / N_, t = e % N_;
+                    val_out[e] = x[(int)ord[(s0 / g) * N_ + t] * xs + col_of(list[s0])];
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// Launch with L lanes per tile; *served = false when fewer than `min_warps` warps would be resident per SM.
+template <int N_, int M_, int L> static int sparsify_lanes_launch(int dtype, const SparsifyParams &p, int min_warps, bool *served, cudaStream_t st) {
+    const int es = (int)dtype_size(dtype);
+    constexpr int C = Order<N_, M_>::C, ORD_BYTES = (C * N_ + 15) & ~15, TILES = 32 / L;
+    const size_t per_warp = (size_t)TILES * sparsify_lanes(M_, p.cc, C, L, es).total;
+    int warps = 0, resident = 0;  // whatever keeps the most warps resident; on a tie the smaller CTA
+    for (int w = 1; w <= 4; w++) {
+        const size_t cta = ORD_BYTES + w * per_warp;
+        if (cta > 226 * 1024) break;
+        int per_sm = (int)((size_t)227 * 1024 / (cta + 1024));
+        if (per_sm > 24) per_sm = 24;
+        if (per_sm * w > resident) { resident = per_sm * w; warps = w; }
+    }
+    *served = resident >= min_warps;
+    if (!*served) return NMG_OK;
+    const size_t smem = ORD_BYTES + warps * per_warp;
+    const int64_t ctas = (p.tiles + warps * TILES - 1) / (warps * TILES), cap = (int64_t)sm_count() * 64;
+    NMG_DISPATCH_DTYPE(dtype, T, {
+        NMG_ALLOW_SMEM(smem, sparsify_lanes_kernel<N_, M_, L, T>);
+        sparsify_lanes_kernel<N_, M_, L, T><<<(unsigned)(ctas < cap ? ctas : cap), warps * 32, smem, st>>>(p);
+    });
+    NMG_CUDA(cudaGetLastError());
+    return NMG_OK;
+}
+
 // =====================================================================================================
 // Densifier: one CTA per tile.  The tile's idx is inverted in shared memory (column -> slot), val is staged,
 // and the m x cc block is written row by row with coalesced stores; zeros are produced by the same stores, so
@@ -641,11 +986,6 @@ __global__ void __launch_bounds__(256) gather_layout_kernel(GatherParams prm) {
     }
 }
 
-static int sm_count() {
-    int sms = 148;
-    return device_sms(&sms) == NMG_OK ? sms : 148;
-}
-
 static int check_dtype(int dtype) {
     if (dtype != NMG_F32 && dtype != NMG_F16 && dtype != NMG_BF16)
         NMG_FAIL(NMG_ERR_INVALID, "dtype must be NMG_F32, NMG_F16 or NMG_BF16, got %d", dtype);
@@ -675,6 +1015,20 @@ extern "C" int nmg_sparsify(const void *dense, int64_t batch, int64_t M, int64_t
     p.M = M; p.K = K; p.ld = ld_dense; p.batch_stride = batch_stride;
     p.nb = geo.nb; p.nc = geo.nc; p.tiles = batch * geo.nb * geo.nc;
     p.n = n; p.m = m; p.g = g; p.C = geo.C; p.cc = geo.cc;
+    cudaStream_t st = (cudaStream_t)stream;
+    // Few patterns: several tiles per warp.  Eight lanes per tile when that leaves at least twelve resident warps to hide the
+    // latency of the shared memory, else a warp per tile down to four; larger tiles, and 16 or 28 patterns (whose later rounds
+    // keep 32 lanes busy: 1:16 68 us against 74 to 102, 2:8 152 against 158), go to the kernel that does not stage the tile.
+#define NMG_SPARSIFY_CASE(N_, M_)                                                                     \
+    if (n == N_ && m == M_) {                                                                         \
+        bool served = false;                                                                          \
+        if ((rc = sparsify_lanes_launch<N_, M_, 8>(dtype, p, 12, &served, st)) || served) return rc;  \
+        if ((rc = sparsify_lanes_launch<N_, M_, 32>(dtype, p, 4, &served, st)) || served) return rc;  \
+    }
+    NMG_SPARSIFY_CASE(1, 4)
+    NMG_SPARSIFY_CASE(2, 4)
+    NMG_SPARSIFY_CASE(1, 8)
+#undef NMG_SPARSIFY_CASE
     const bool specialised = (n == 1 && (m == 4 || m == 8 || m == 16)) || (n == 2 && (m == 4 || m == 8));
     const size_t slab = specialised ? sparsify_lean(geo.cc, geo.C).total : sparsify_slab(m, geo.cc, geo.C, dtype_size(dtype)).total;
     const size_t ord_bytes = ((size_t)geo.C * n + 15) & ~(size_t)15;
@@ -698,7 +1052,6 @@ extern "C" int nmg_sparsify(const void *dense, int64_t batch, int64_t M, int64_t
     int64_t ctas = (p.tiles + warps - 1) / warps;
     const int64_t max_ctas = (int64_t)sm_count() * 16;
     if (ctas > max_ctas) ctas = max_ctas;
-    cudaStream_t st = (cudaStream_t)stream;
     bool launched = false;
 #define NMG_SPARSIFY_CASE(N_, M_)                                                                                     \
     if (!launched && n == N_ && m == M_) {                                                                            \

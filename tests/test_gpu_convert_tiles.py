@@ -1,0 +1,31 @@
+"""Edges of the conversion kernels' tiles: partly filled warps, remainder tiles, unaligned rows, ties and zeros."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import cuda, np_of, seeded_normal
+from oracle import nmg_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,m,g", [(1, 4, 1), (1, 4, 16), (2, 4, 3), (2, 4, 16), (2, 4, 300), (1, 8, 16), (2, 8, 2), (2, 8, 16),
+                                   (1, 16, 16), (2, 8, 100), (1, 4, 2000)])
+def test_sparsify_and_densify_at_tile_edges(n, m, g, dtype):
+    """One tile, tiles that do not fill a warp, cut tiles in both directions, rows without 16-byte alignment; few distinct
+    values (ties) with many zeros, and random weights."""
+    from sten_b200 import ops
+    cc = g * len(orc.nm_order(n, m)) if hasattr(orc, "nm_order") else g * {(1, 4): 4, (2, 4): 6, (1, 8): 8, (2, 8): 28, (1, 16): 16}[n, m]
+    for M, K, off in [(m, cc, 0), (3 * m + 1, cc, 1), (2 * m, 2 * cc + cc // 2 + 1, 0)]:
+        for ties in (False, True):
+            w = seeded_normal((M, K + off), M + K)
+            if ties:
+                w = w.round()
+            w = w.to(dtype)[:, off:]
+            val_o, idx_o = orc.sparsify(w.float().numpy(), n, m, g)
+            val, idx = ops.sparsify(w.to(cuda())[None], n, m, g)
+            assert np.array_equal(np_of(idx), idx_o) and np.array_equal(np_of(val.float()), val_o)
+            d = torch.full((M, K + off), 7.0, dtype=dtype, device=cuda())
+            ops.densify_into(val, idx, d[None, :, off:], n, m, g) if hasattr(ops, "densify_into") else None
+            assert np.array_equal(np_of(ops.densify(val, idx, 1, M, K, n, m, g).float())[0], orc.densify(val_o, idx_o, (M, K), n, m, g))

@@ -342,18 +342,13 @@ extern "C" int nmg_spmm_expanded(const void *expanded, int64_t M, int64_t K, int
     if (ld_act < K || ld_out < (out_tm ? M : tokens) || (residual && ld_res < (out_tm ? M : tokens))) NMG_FAIL(NMG_ERR_INVALID, "leading dimension smaller than the row");
     if ((reinterpret_cast<uintptr_t>(expanded) & 255) || (reinterpret_cast<uintptr_t>(act) & 15) || (ld_act % 8))
         NMG_FAIL(NMG_ERR_UNSUPPORTED, "the expanded copy must be 256-byte aligned and the activation rows 16-byte aligned");
-    const bool pair = M > 128;
-    CUtensorMap tm[3];
-    if ((rc = encode_tmap_2d(&tm[0], dtype, act, (uint64_t)K, (uint64_t)tokens, (uint64_t)ld_act, 64, pair ? 128 : 256, 1))) return rc;
-    tm[1] = tm[0];
-    tm[2] = tm[0];
     Epilogue epi;
     epi.act = activation; epi.residual = residual; epi.ld_res = ld_res;
     void *outs[1] = {out};
     cudaStream_t st = (cudaStream_t)stream;
     const ProfileEvents pe = take_profile_events();
     if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));
-    rc = tc_dense_gemm(M, K, dtype, pair, static_cast<const char *>(expanded), tm, tokens, bias, outs, 1, nullptr, ld_out, out_tm ? 1 : 0, st, epi);
+    rc = tc_dense_gemm(M, K, dtype, static_cast<const char *>(expanded), DenseAct{act, ld_act, 0}, tokens, bias, outs, 1, nullptr, ld_out, out_tm ? 1 : 0, st, epi);
     if (rc == NMG_OK && pe.stop) NMG_CUDA(cudaEventRecord(pe.stop, st));
     return rc;
 }

@@ -12,8 +12,8 @@
 //   gemm_tc_kernel        persistent, one CTA per SM.  Warp 0 issues the TMA loads of both operands, warp 1 the
 //                         MMAs (128 x 256 x 16, fp32 accumulators in TMEM), warps 2..9 drain accumulators.  16-bit
 //                         mode double-buffers the accumulator (2 x 256 TMEM columns) so that the drain of one tile
-//                         overlaps the MMAs of the next; fp32 mode uses the second half for the running sum into which
-//                         the tensor core's partial tile is promoted every TC_CHUNK_KB k-blocks.
+//                         overlaps the MMAs of the next; in fp32 mode a buffer is a chunk of TC_CHUNK_KB k-blocks, and
+//                         the drain warps keep the running sum of the chunks in registers.
 //
 // All device-side waits are bounded: a wait that runs out sets the status word and the role leaves its loop; the
 // CTA then meets at the common exit where TMEM is released.
@@ -292,6 +292,7 @@ struct GemmParams {
     int out_staged;    // feature-major output whose rows are 16-byte aligned: go through the staging tile
     int out_tm_vec;    // token-major output (and residual) whose rows are 16-byte aligned: transposed in the staging tile, 16-byte stores
     int tiles_f, tiles_t;  // tiles_f counts tiles of 128 features (one CTA per tile) or 256 (CTA pairs)
+    int bn;                // width of a tile: TC_BN, or what gemm_split_cols chose (fp32)
     int band;              // width of the tile order's bands, in feature tiles
     unsigned *wave_ctr;    // zeroed counter for the producers' soft rendezvous before every tile, or NULL
     int *status;
@@ -300,17 +301,20 @@ constexpr int GEMM_STAGING_BYTES = GEMM_DRAIN_WARPS * 4096;  // per drain warp: 
 
 struct GemmMaps {
     CUtensorMap a[3];  // weight planes, box 64 x 128, 128-byte swizzle
-    CUtensorMap b[3];  // activation planes, box 64 x 256 (64 x 128 for CTA pairs)
+    CUtensorMap b[3];  // activation planes, box 64 x bn (64 x bn / 2 for CTA pairs)
     CUtensorMap out;   // out_tma: the output, box 128 bytes x 32 rows, 128-byte swizzle
 };
 
 // PAIR = false: one CTA per 128-feature x 256-token tile.
-// PAIR = true (16-bit operands): two CTAs of a cluster share a 256-feature x 256-token tile.  Each loads the weight rows
+// PAIR = true: two CTAs of a cluster share a 256-feature x 256-token tile.  Each loads the weight rows
 // of its own 128 features and only half of the activation tile (128 tokens); the MMA (cta_group::2, M = 256, issued by the
 // even CTA) reads both halves from both shared memories.  An SM then takes in 32 KB per 64 reduction elements instead of
 // 48 KB, which is what keeps the tensor core fed from L2.  full[s] lives in the even ("leader") CTA and receives the TMA
 // bytes of both; empty[s] and acc_full[b] exist in both CTAs and are signalled by multicast commits; acc_free[b] lives in
 // the leader and collects the drain warps of both CTAs.  No load is multicast.
+// fp32 (always pairs): a stage is one k-block of all six planes, 96 KB, and its six products run from it.  With a stage per
+// product (48 KB per 512 clocks and SM, over what L2 delivers) and the running sum in the second TMEM buffer the MMAs waited
+// for loads and for every promotion: 4096 tokens, 3072 <- 768 took 104 us, now 86, at the rate of a long cuBLAS product but for the last wave.
 // TMA_OUT = true: the one-destination staged output, leaving as tiled bulk stores; only that output path is compiled,
 // which keeps the drain warps' code and register needs small.  TMA_OUT = false: every other output form.
 template <typename T, bool PAIR, bool TMA_OUT>
@@ -318,12 +322,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     constexpr int TERMS = TcMode<T>::TERMS;
     using E = typename TcMode<T>::elem;
     constexpr bool SPLIT = TERMS > 1;
-    static_assert(!(PAIR && SPLIT), "CTA pairs serve the 16-bit mode");
-    constexpr int NBUF = SPLIT ? 1 : 2;  // accumulator tiles in flight between the MMA issuer and the drain warps
-    constexpr uint32_t TMEM_COLS = 2 * TC_ACC_COLS;
-    constexpr int B_BYTES = PAIR ? TC_B_BYTES / 2 : TC_B_BYTES;
-    constexpr int STAGE_BYTES = TC_A_BYTES + B_BYTES;
-    constexpr int STAGES = GEMM_RING_BYTES / STAGE_BYTES;  // 4, or 6 for pairs
+    static_assert(PAIR || !SPLIT, "fp32 runs on CTA pairs");
+    constexpr int NBUF = 2;  // accumulator tiles in flight between the MMA issuer and the drain warps
+    constexpr uint32_t TMEM_COLS = NBUF * TC_ACC_COLS;
+    constexpr int PLANES = SPLIT ? 3 : 1;
+    constexpr int B_BYTES = PAIR ? TC_B_BYTES / 2 : TC_B_BYTES;  // room of one plane; the widest tile fills it
+    constexpr int OFF_B = PLANES * TC_A_BYTES, STAGE_BYTES = OFF_B + PLANES * B_BYTES;
+    constexpr int STAGES = GEMM_RING_BYTES / STAGE_BYTES;  // 4, 6 for pairs, 2 for fp32
+    const int bn = SPLIT ? prm.bn : TC_BN;
     constexpr int TILE_FEATS = PAIR ? 2 * TC_BM : TC_BM;
 
     extern __shared__ char smem_raw[];
@@ -345,8 +351,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     // A "unit" is what the MMA issuer hands to the drain warps: a whole tile (16-bit) or a chunk of k-blocks (fp32).
     const int ntiles = prm.tiles_f * prm.tiles_t;
     const int my_tiles = (unit_id < ntiles) ? (ntiles - unit_id + nunits - 1) / nunits : 0;
-    const int nkb = (int)((prm.red + TC_BK - 1) / TC_BK) * TERMS;  // iterations per tile: k-blocks x split terms (term fastest)
-    const int chunk_it = SPLIT ? TC_CHUNK_KB * TERMS : nkb;
+    const int nkb = (int)((prm.red + TC_BK - 1) / TC_BK);  // iterations per tile
+    const int chunk_it = SPLIT ? TC_CHUNK_KB : nkb;
     const int nchunks = (nkb + chunk_it - 1) / chunk_it;
 
     if (tid == 0) {
@@ -380,7 +386,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         int tile_f, tile_t;
         tile_of_cta(unit_id + ti * nunits, prm.tiles_f, prm.tiles_t, tile_f, tile_t, prm.band);
         feat0 = tile_f * TILE_FEATS + (int)rank * TC_BM;
-        tok0 = tile_t * TC_BN;
+        tok0 = tile_t * bn;
     };
 
     if (warp == 0) {
@@ -410,17 +416,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 const uint32_t ph = (uint32_t)((it / STAGES) & 1);
                 if (!(ok = __all_sync(0xffffffffu, wait(&empty[s], ph ^ 1, 21)))) break;
                 if (elect_one()) {
-                    const int term = kb % TERMS;
-                    const int wc = TERMS == 1 ? 0 : kSplitW[term], xc = TERMS == 1 ? 0 : kSplitX[term];
                     char *stage = smem + s * STAGE_BYTES;
                     if constexpr (PAIR) {
-                        if (leader) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);  // both CTAs report to this barrier
-                        tma_load_2d_pair(stage, &maps.a[wc], (kb / TERMS) * TC_BK, feat0, full_leader + s * 8);
-                        tma_load_2d_pair(stage + TC_A_BYTES, &maps.b[xc], (kb / TERMS) * TC_BK, tok0 + (int)rank * 128, full_leader + s * 8);
+                        const int half = bn / 2;
+                        if (leader) mbar_expect_tx(&full[s], (uint32_t)(2 * PLANES * (TC_A_BYTES + half * TC_BK * 2)));  // both CTAs report to this barrier
+#pragma unroll
+                        for (int c = 0; c < PLANES; c++) {
+                            tma_load_2d_pair(stage + c * TC_A_BYTES, &maps.a[c], kb * TC_BK, feat0, full_leader + s * 8);
+                            tma_load_2d_pair(stage + OFF_B + c * B_BYTES, &maps.b[c], kb * TC_BK, tok0 + (int)rank * half, full_leader + s * 8);
+                        }
                     } else {
                         mbar_expect_tx(&full[s], STAGE_BYTES);
-                        tma_load_2d(stage, &maps.a[wc], (kb / TERMS) * TC_BK, feat0, &full[s]);
-                        tma_load_2d(stage + TC_A_BYTES, &maps.b[xc], (kb / TERMS) * TC_BK, tok0, &full[s]);
+                        tma_load_2d(stage, &maps.a[0], kb * TC_BK, feat0, &full[s]);
+                        tma_load_2d(stage + TC_A_BYTES, &maps.b[0], kb * TC_BK, tok0, &full[s]);
                     }
                 }
                 __syncwarp();
@@ -429,7 +437,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (of the leader for pairs)
         if (leader) {
-            uint32_t idesc = make_idesc<E>();
+            uint32_t idesc = make_idesc<E>(bn);
             if constexpr (PAIR) idesc = (idesc & ~(0x1fu << 24)) | ((uint32_t)(256 >> 4) << 24);  // M = 256 across the pair
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint64_t desc0 = make_sw128_desc(smem_u32(smem));
@@ -450,11 +458,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                         if (!(ok = __all_sync(0xffffffffu, wait(&full[s], ph, 22)))) break;
                         tc_fence_after();
                         if (elect_one()) {
-                            const uint64_t adesc = desc0 + (uint64_t)(uint32_t)(s * (STAGE_BYTES / 16)), bdesc = adesc + TC_A_BYTES / 16;
+                            const uint64_t stage_a = desc0 + (uint64_t)(uint32_t)(s * (STAGE_BYTES / 16)), stage_b = stage_a + OFF_B / 16;
 #pragma unroll
-                            for (int k = 0; k < TC_BK / 16; k++) {  // 16 elements = 32 bytes = 2 descriptor units per step
-                                if constexpr (PAIR) tc2_mma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
-                                else tc_mma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
+                            for (int t = 0; t < TERMS; t++) {
+                                // bias_cols: the operands' roles are exchanged, the order of the products is not (equal results either way)
+                                const int ap = !SPLIT ? 0 : prm.bias_cols ? split_x(t) : split_w(t), bp = !SPLIT ? 0 : prm.bias_cols ? split_w(t) : split_x(t);
+                                const uint64_t adesc = stage_a + (uint32_t)(ap * (TC_A_BYTES / 16)), bdesc = stage_b + (uint32_t)(bp * (B_BYTES / 16));
+#pragma unroll
+                                for (int k = 0; k < TC_BK / 16; k++) {  // 16 elements = 32 bytes = 2 descriptor units per step
+                                    if constexpr (PAIR) tc2_mma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (first && t == 0 && k == 0) ? 0u : 1u);
+                                    else tc_mma_f16(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (first && k == 0) ? 0u : 1u);
+                                }
                             }
                             if constexpr (PAIR) tc2_commit_both(&empty[s]);
                             else tc_commit(&empty[s]);  // arrives when the MMAs above have read the stage
@@ -482,8 +496,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         constexpr bool RES_AHEAD = TMA_OUT && sizeof(T) == 2;  // residual fetched one slice ahead (fp32 rows would take 2 x 32 registers)
         constexpr int RQ = RES_AHEAD ? 4 : 1;                  // 16-byte pieces of one slice row of the residual
         const int q = warp & 3;  // TMEM lane quarter this warp may access
-        constexpr int SLICES = (TC_BN / 32) / (GEMM_DRAIN_WARPS / 4);  // 32-column slices per warp
-        const int sl0 = ((warp - 2) >> 2) * SLICES;                    // this warp's first slice
+        constexpr int SLICES = (TC_BN / 32) / (GEMM_DRAIN_WARPS / 4);  // 32-column slices per warp, at most
+        const int per_warp = (bn / 32 + 1) / 2, sl0 = ((warp - 2) >> 2) * per_warp;  // this warp's first slice
+        const int nsl = min(per_warp, bn / 32 - sl0);                                // and how many it has
         const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
         char *stage_w = staging + (warp - 2) * 4096;
         const T *res = static_cast<const T *>(prm.residual);
@@ -493,6 +508,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         asm volatile("griddepcontrol.wait;" ::: "memory");
         int unit = 0;
         bool ok = true;
+        float run[SPLIT ? SLICES : 1][32];  // fp32: sum of the tile's finished chunks
         for (int ti = 0; ti < my_tiles && ok; ti++) {
             int feat0, tok0;
             tile_origin(ti, feat0, tok0);
@@ -535,17 +551,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 // handle(sl, r, qr): slice sl of the unit is in registers r (this lane's feature row, 32 tokens); qr holds the
                 // same 32 elements of the residual when res_fetch found them loadable in 16-byte pieces
                 auto handle = [&](int sl, uint32_t (&r)[32], const uint4 (&qr)[RQ]) {
-                    if (SPLIT && c > 0) {
-                        uint32_t run[32];
-                        tmem_ld32(lane_base + (uint32_t)(TC_ACC_COLS + sl * 32), run);
-#pragma unroll
-                        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(run[j]), __uint_as_float(r[j])));
-                    }
-                    if (!last) {
-                        tmem_st32(lane_base + (uint32_t)(TC_ACC_COLS + sl * 32), r);
-                        return;
-                    }
-                    if (sl == sl0 + SLICES - 1) release();
+                    if (sl == sl0 + nsl - 1) release();
                     const int64_t tokc = (int64_t)tok0 + sl * 32;
                     // activation(product + bias), kept as fp32 bits in r.  The activation sits in one warp-uniform branch
                     // around its own unrolled loop: the 32 evaluations are independent and interleave, where a test per
@@ -758,22 +764,42 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 uint32_t ra[32], rb[32];
                 uint4 qa[RQ], qb[RQ];
                 const uint32_t acc_addr = lane_base + (uint32_t)(b * TC_ACC_COLS);
+                if constexpr (SPLIT) {
+                    if (nchunks > 1) {
+                        // promotion: the chunk joins the running sum; with the last one the total goes back to TMEM for the epilogue
+#pragma unroll
+                        for (int i = 0; i < SLICES; i++) {
+                            if (i >= nsl) break;
+                            tmem_ld32(acc_addr + (uint32_t)((sl0 + i) * 32), ra);
+#pragma unroll
+                            for (int j = 0; j < 32; j++) {
+                                run[i][j] = c > 0 ? __fadd_rn(run[i][j], __uint_as_float(ra[j])) : __uint_as_float(ra[j]);
+                                ra[j] = __float_as_uint(run[i][j]);
+                            }
+                            if (last) tmem_st32(acc_addr + (uint32_t)((sl0 + i) * 32), ra);
+                        }
+                        if (!last) { release(); continue; }
+                    }
+                }
+                const int sl_end = sl0 + nsl;
                 tmem_ld32_issue(acc_addr + (uint32_t)(sl0 * 32), ra);
-                if (last) res_fetch(sl0, qa);
+                res_fetch(sl0, qa);
 #pragma unroll 1
-                for (int sl = sl0; sl < sl0 + SLICES; sl += 2) {
+                for (int sl = sl0; sl < sl_end; sl += 2) {
                     tmem_ld_fence(ra);
-                    tmem_ld32_issue(acc_addr + (uint32_t)((sl + 1) * 32), rb);
-                    if (last) res_fetch(sl + 1, qb);
+                    if (sl + 1 < sl_end) {
+                        tmem_ld32_issue(acc_addr + (uint32_t)((sl + 1) * 32), rb);
+                        res_fetch(sl + 1, qb);
+                    }
                     handle(sl, ra, qa);
+                    if (sl + 1 >= sl_end) break;
                     tmem_ld_fence(rb);
-                    if (sl + 2 < sl0 + SLICES) {
+                    if (sl + 2 < sl_end) {
                         tmem_ld32_issue(acc_addr + (uint32_t)((sl + 2) * 32), ra);
-                        if (last) res_fetch(sl + 2, qa);
+                        res_fetch(sl + 2, qa);
                     }
                     handle(sl + 1, rb, qb);
                 }
-                if (!last) release();  // promotion finished: hand the accumulator back
             }
         }
         // the bulk stores must have read their shared-memory source before the CTA's shared memory is given up; their
@@ -864,11 +890,19 @@ template <typename T, bool PAIR> static int gemm_launch(const GemmParams &p, con
     return p.out_tma ? gemm_launch_as<T, PAIR, true>(p, maps, st) : gemm_launch_as<T, PAIR, false>(p, maps, st);
 }
 
-// CTA pairs serve 16-bit operands when the output has at least two 128-feature tiles (a pair covers 256 features).
-bool tc_dense_uses_pair(const Geo &geo, int dtype, bool transposed) {
-    return dtype != NMG_F32 && (transposed ? geo.K : geo.M) > TC_BM;
+// Tile width of the fp32 product: the one whose waves cost least.  A tile of bn columns takes about as long as bn + 40 columns
+// at full rate (narrow tiles read more shared memory per product; measured 3072 <- 768, 4096 tokens: 28.6 us per wave at 256, 15.8
+// at 128, 10.8 at 64).  768 <- 3072 is 48 tiles of 256 columns on 74 pairs and 107.9 us, or 66 of 192 and 89.5; 1024 <- 4096 at
+// 1536 tokens takes 131 us at 256 and 76 at 96.
+static int gemm_split_cols(int64_t tiles_f, int64_t cols, int64_t units) {
+    int best = TC_BN;
+    int64_t best_cost = INT64_MAX;
+    for (int bn = TC_BN; bn >= 64; bn -= 32) {
+        const int64_t tiles = tiles_f * ((cols + bn - 1) / bn), cost = (tiles + units - 1) / units * (bn + 40);
+        if (cost < best_cost) { best = bn; best_cost = cost; }
+    }
+    return best;
 }
-
 // (val, idx) -> the weight with its zeros restored, rows `ld` elements apart at `dst` (16-byte aligned, ld a multiple of 8).
 // plain = false: the matmul's operand, 16-bit or three bf16 planes for fp32 (plane_rows rows each); plain = true: the
 // weight in its own dtype (the densifier), where full stores must not run past the row: K a multiple of 8, or the rows kernel.
@@ -921,11 +955,10 @@ int tc_expand_plain(const Geo &geo, int dtype, const void *val, const int16_t *i
     return expand_to(geo, dtype, false, true, val, idx, dense, ld, st);
 }
 
-// out = dense[rows][round_up(red, 8)] (16-bit, or three bf16 planes for fp32) x activations.  act_maps: tensor maps of the
-// activation planes (128-byte swizzle; box 64 x 128 when `pair`, else 64 x 256), one for 16-bit data, three for the fp32 split.
-int tc_dense_gemm(int64_t rows, int64_t red, int dtype, bool pair, const char *dense, const CUtensorMap *act_maps, int64_t tokens,
-                  const void *bias, void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major, cudaStream_t st,
-                  const Epilogue &epi) {
+// out = dense[rows][round_up(red, 8)] (16-bit, or three bf16 planes for fp32) x activations (16-bit, or the planes of the split).
+// CTA pairs (256 rows per tile) unless a 16-bit output has one tile of 128 features only.
+int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const DenseAct &act, int64_t tokens, const void *bias,
+                  void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major, cudaStream_t st, const Epilogue &epi) {
     if (n_outs < 1 || n_outs > GEMM_MAX_OUTS) NMG_FAIL(NMG_ERR_INVALID, "between 1 and %d output buffers, got %d", GEMM_MAX_OUTS, n_outs);
     const int64_t ld = dense_ld(red);
     const int planes = dtype == NMG_F32 ? 3 : 1;
@@ -933,18 +966,24 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, bool pair, const char *d
     GemmMaps maps;
     const int edt = dtype == NMG_F32 ? NMG_BF16 : dtype;
     const size_t osz = dtype == NMG_F32 ? 4 : 2;
-    // Token-major output of a CTA-pair product: exchange the operands' roles.  Both boxes are 64 x 128 in pair mode, so the
-    // activations can be the row operand (tokens on the accumulator's lanes) and the weight the column operand; the
-    // output is then "feature-major" in the kernel's terms -- accumulator rows are output rows -- and leaves through the
+    const bool pair = dtype == NMG_F32 || rows > TC_BM;
+    // Token-major output of a CTA-pair product: exchange the operands' roles.  The activations become the row operand (tokens
+    // on the accumulator's lanes) and the weight the column operand; the output is then "feature-major" in the kernel's terms -- accumulator rows are output rows -- and leaves through the
     // staged 16-byte path with no transposition, the bias running along the columns.
     const bool swap = pair && out_token_major && n_outs == 1 && !mc_out && tokens > TC_BM && (ld_out * osz) % 16 == 0 &&
                       (reinterpret_cast<uintptr_t>(outs[0]) & 15) == 0;
+    int sms = 148;
+    if ((rc = device_sms(&sms))) return rc;
+    const int64_t units = pair ? sms / 2 : sms, row_ext = swap ? tokens : rows, col_ext = swap ? rows : tokens;
+    const int tile_feats = pair ? 2 * TC_BM : TC_BM;
+    const int64_t tiles_f = (row_ext + tile_feats - 1) / tile_feats;
+    const int bn = dtype == NMG_F32 ? gemm_split_cols(tiles_f, col_ext, units) : TC_BN;
     for (int c = 0; c < 3; c++) {
         const int pc = c < planes ? c : 0;
-        CUtensorMap wmap;
-        if ((rc = encode_tmap_2d(&wmap, edt, dense + (size_t)pc * rows * ld * 2, (uint64_t)red, (uint64_t)rows, (uint64_t)ld, TC_BK, TC_BM, 1))) return rc;
-        maps.a[c] = swap ? act_maps[c] : wmap;
-        maps.b[c] = swap ? wmap : act_maps[c];
+        const char *w = dense + (size_t)pc * rows * ld * 2, *x = static_cast<const char *>(act.base) + (size_t)pc * act.plane_elems * 2;
+        const uint32_t col_box = (uint32_t)(pair ? bn / 2 : bn);
+        if ((rc = encode_tmap_2d(swap ? &maps.b[c] : &maps.a[c], edt, w, (uint64_t)red, (uint64_t)rows, (uint64_t)ld, TC_BK, swap ? col_box : TC_BM, 1))) return rc;
+        if ((rc = encode_tmap_2d(swap ? &maps.a[c] : &maps.b[c], edt, x, (uint64_t)red, (uint64_t)tokens, (uint64_t)act.ld, TC_BK, swap ? TC_BM : col_box, 1))) return rc;
     }
     if (swap) {  // from here on "rows" are the accumulator's rows (tokens) and "tokens" its columns (output features)
         const int64_t t = rows;
@@ -978,30 +1017,25 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, bool pair, const char *d
         maps.out = maps.a[0];  // never used; keeps the parameter defined
     }
     gp.mc_out = (vec && mc_out && (reinterpret_cast<uintptr_t>(mc_out) & 15) == 0) ? mc_out : nullptr;
-    const int tile_feats = pair ? 2 * TC_BM : TC_BM;
-    gp.tiles_f = (int)((rows + tile_feats - 1) / tile_feats);
-    gp.tiles_t = (int)((tokens + TC_BN - 1) / TC_BN);
+    gp.tiles_f = (int)tiles_f;
+    gp.tiles_t = (int)((tokens + bn - 1) / bn);
+    gp.bn = bn;
     gp.band = pair ? TC_BAND_PAIR : TC_BAND;
-    {
-        // many waves over a long reduction: keep the producers in step (see the kernel); the counter is zeroed in stream order
-        int sms = 148, rc_sms;
-        if ((rc_sms = device_sms(&sms))) return rc_sms;
-        const int64_t units = pair ? sms / 2 : sms;
-        if ((int64_t)gp.tiles_f * gp.tiles_t >= 3 * units && red >= 4096) {
-            if ((rc = get_wave_counter(&gp.wave_ctr))) return rc;
-            NMG_CUDA(cudaMemsetAsync(gp.wave_ctr, 0, sizeof(unsigned), st));
-        }
+    // many waves over a long reduction: keep the producers in step (see the kernel); the counter is zeroed in stream order
+    if ((int64_t)gp.tiles_f * gp.tiles_t >= 3 * units && red >= 4096) {
+        if ((rc = get_wave_counter(&gp.wave_ctr))) return rc;
+        NMG_CUDA(cudaMemsetAsync(gp.wave_ctr, 0, sizeof(unsigned), st));
     }
     gp.status = status;
     gp.act = epi.act; gp.residual = epi.residual; gp.ld_res = epi.ld_res;
     gp.res_vec = (epi.residual && (epi.ld_res * osz) % 16 == 0 && (reinterpret_cast<uintptr_t>(epi.residual) & 15) == 0) ? 1 : 0;
-    if (dtype == NMG_F32) return gemm_launch<float, false>(gp, maps, st);
+    if (dtype == NMG_F32) return gemm_launch<float, true>(gp, maps, st);
     if (dtype == NMG_F16) return pair ? gemm_launch<__half, true>(gp, maps, st) : gemm_launch<__half, false>(gp, maps, st);
     return pair ? gemm_launch<__nv_bfloat16, true>(gp, maps, st) : gemm_launch<__nv_bfloat16, false>(gp, maps, st);
 }
 
 // Two passes: expansion into `ws`, then the matmul on the expanded weight.
-int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const CUtensorMap *act_maps,
+int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const DenseAct &act,
                     int64_t tokens, const void *bias, void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major,
                     void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi) {
     const int64_t rows = transposed ? geo.K : geo.M, red = transposed ? geo.M : geo.K;
@@ -1010,8 +1044,7 @@ int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val,
     char *dense = reinterpret_cast<char *>(((uintptr_t)ws + 255) & ~(uintptr_t)255);
     int rc;
     if ((rc = tc_dense_expand(geo, dtype, transposed, val, idx, dense, st))) return rc;
-    return tc_dense_gemm(rows, red, dtype, tc_dense_uses_pair(geo, dtype, transposed), dense, act_maps, tokens, bias, outs, n_outs, mc_out,
-                         ld_out, out_token_major, st, epi);
+    return tc_dense_gemm(rows, red, dtype, dense, act, tokens, bias, outs, n_outs, mc_out, ld_out, out_token_major, st, epi);
 }
 
 }  // namespace nmg

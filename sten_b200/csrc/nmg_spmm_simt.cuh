@@ -52,7 +52,8 @@ struct Epilogue {
     bool any() const { return act != NMG_EPI_NONE || residual != nullptr; }
 };
 int launch_epilogue(int dtype, void *out, int64_t rows, int64_t cols, int64_t ld_out, const Epilogue &epi, cudaStream_t st);
-bool tc_dense_uses_pair(const Geo &geo, int dtype, bool transposed);
+// Activations of the two-pass variant: [tokens][ld], reduction contiguous, 16-byte aligned rows; three bf16 planes for fp32.
+struct DenseAct { const void *base; int64_t ld, plane_elems; };
 
 bool tc_supported(const Geo &geo, int dtype);        // fused kernel
 bool tc_dense_supported(const Geo &geo, int dtype);  // two-pass variant
@@ -65,7 +66,7 @@ size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed);
 int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void *val, const int16_t *idx, const void *pat,
               const void *nval, const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, const void *bias, void *const *outs, int n_outs,
               void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi = Epilogue());
-int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const CUtensorMap *act_maps,
+int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const DenseAct &act,
                     int64_t tokens, const void *bias, void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major,
                     void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi);
 
@@ -81,9 +82,8 @@ int tc_sp_matmul_t(const Geo &geo, int dtype, const void *sp_copy, const void *d
 // The two halves of the two-pass variant on their own: a caller may keep the expanded weight across calls (opt-in: it
 // trades the format's memory saving for skipping the expansion pass of every call).
 int tc_dense_expand(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, char *dense, cudaStream_t st);
-int tc_dense_gemm(int64_t rows, int64_t red, int dtype, bool pair, const char *dense, const CUtensorMap *act_maps, int64_t tokens,
-                  const void *bias, void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major, cudaStream_t st,
-                  const Epilogue &epi);
+int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const DenseAct &act, int64_t tokens, const void *bias,
+                  void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major, cudaStream_t st, const Epilogue &epi);
 
 // ---- specialised forward kernel: parameters, shared-memory plan, per-(n, m) launchers
 struct FwdParams {

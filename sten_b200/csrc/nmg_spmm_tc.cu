@@ -814,11 +814,9 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     if (n_outs < 1 || (n_outs > 1 && !dense)) NMG_FAIL(NMG_ERR_UNSUPPORTED, "several output buffers need the two-pass tensor-core variant");
     void *out = outs[0];
     const int64_t red = transposed ? geo.M : geo.K;
-    // the two-pass variant on CTA pairs loads the activation tile in two halves of 128 tokens
     const int64_t feats = transposed ? geo.K : geo.M;
     const FxChoice fx = fx_choose(feats, red, tokens, dtype);
-    const uint32_t box_tok = dense ? (tc_dense_uses_pair(geo, dtype, transposed) ? 128 : TC_BN) : (uint32_t)fx.bn;
-    CUtensorMap tm[3];
+    DenseAct planes{act, ld_act, 0};
     int rc;
     if (dtype == NMG_F32) {
         const size_t need = tc_split_workspace_bytes(geo, dtype, transposed, tokens);
@@ -839,19 +837,14 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
             split_f32_kernel<<<grid, 128, 0, st>>>(static_cast<const float *>(act) + r0 * ld_act, nr, red, ld_act, xs + r0 * ldp, ldp, plane_elems);
         }
         NMG_CUDA(cudaGetLastError());
-        for (int c = 0; c < 3; c++)
-            if ((rc = encode_tmap_2d(&tm[c], NMG_BF16, xs + c * plane_elems, (uint64_t)red, (uint64_t)tokens, (uint64_t)ldp, TC_BK, box_tok, 1))) return rc;
+        planes = DenseAct{xs, ldp, plane_elems};
         ws = static_cast<char *>(ws) + need;  // what follows the split activation is free for the expanded weight
         ws_bytes -= need;
-    } else {
-        if ((rc = encode_tmap_2d(&tm[0], dtype, act, (uint64_t)red, (uint64_t)tokens, (uint64_t)ld_act, TC_BK, box_tok, 1))) return rc;
-        tm[1] = tm[0];
-        tm[2] = tm[0];
     }
     if (dense) {
         const ProfileEvents pe = take_profile_events();
         if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));
-        rc = tc_dense_matmul(geo, dtype, transposed, val, idx, tm, tokens, bias, outs, n_outs, mc_out, ld_out, out_token_major, ws, ws_bytes, st, epi);
+        rc = tc_dense_matmul(geo, dtype, transposed, val, idx, planes, tokens, bias, outs, n_outs, mc_out, ld_out, out_token_major, ws, ws_bytes, st, epi);
         if (rc == NMG_OK && pe.stop) NMG_CUDA(cudaEventRecord(pe.stop, st));
         return rc;
     }
@@ -859,7 +852,12 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     if ((rc = get_status_word(&status))) return rc;
     const size_t es = dtype_size(dtype);
     FxMaps maps;
-    for (int c = 0; c < 3; c++) maps.x[c] = tm[c];
+    for (int c = 0; c < 3; c++) {
+        if (c > 0 && dtype != NMG_F32) { maps.x[c] = maps.x[0]; continue; }
+        if ((rc = encode_tmap_2d(&maps.x[c], dtype == NMG_F32 ? NMG_BF16 : dtype, static_cast<const char *>(planes.base) + (size_t)c * planes.plane_elems * 2, (uint64_t)red,
+                                 (uint64_t)tokens, (uint64_t)planes.ld, TC_BK, (uint32_t)fx.bn, 1)))
+            return rc;
+    }
     const int64_t Kpn = natural_width(geo);
     const NaturalLayout lay = natural_layout(geo, dtype);
     const char *masks = static_cast<const char *>(nval) + lay.val_bytes;

@@ -266,9 +266,7 @@ __device__ __forceinline__ float gelu_erf(float v) {
 // error then no longer depends on K.
 template <typename T> struct TcMode { using elem = T; static constexpr int TERMS = 1; };
 template <> struct TcMode<float> { using elem = __nv_bfloat16; static constexpr int TERMS = 6; };
-static __device__ __constant__ int kSplitW[6] = {0, 1, 0, 1, 2, 0};
-static __device__ __constant__ int kSplitX[6] = {0, 0, 1, 1, 0, 2};
-__host__ __device__ constexpr int split_w(int t) { return t == 1 || t == 3 ? 1 : t == 4 ? 2 : 0; }  // the same for unrolled loops
+__host__ __device__ constexpr int split_w(int t) { return t == 1 || t == 3 ? 1 : t == 4 ? 2 : 0; }  // planes of product t
 __host__ __device__ constexpr int split_x(int t) { return t == 2 || t == 3 ? 1 : t == 5 ? 2 : 0; }
 
 }  // namespace nmg

@@ -103,5 +103,7 @@ def host():
         except ImportError as e:
             raise ImportError(f"sten_b200/_nmg_host.so cannot be loaded ({e}): build it with `python -m sten_b200.build`") from e
         mod.set_error_class(NmgError)
+        from . import dispatch
+        dispatch.use_native_repeat(mod)
         _host = mod
     return _host

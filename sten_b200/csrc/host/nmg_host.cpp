@@ -7,6 +7,7 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <c10/core/GradMode.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -20,7 +21,7 @@
 namespace {
 
 PyObject *g_error_class = nullptr;  // sten_b200._native.NmgError(status, message)
-PyObject *g_s_val, *g_s_idx, *g_s_packed, *g_s_packed_sp24;
+PyObject *g_s_val, *g_s_idx, *g_s_packed, *g_s_packed_sp24, *g_zero;
 
 struct PyRaised {};  // a Python exception is set
 
@@ -358,6 +359,7 @@ struct Derived {
     bool valid = false;
     at::Tensor copy;  // undefined: there is none for this weight
 };
+extern PyTypeObject handle_type;
 struct Handle {
     PyObject_HEAD
     Geo geo;
@@ -497,6 +499,108 @@ PyObject *handle_linear_t(PyObject *self, PyObject *const *a, Py_ssize_t nargs) 
     NMG_PY_END
 }
 
+// ------------------------------------------------------------------------------------------------ repeated calls
+// What a torch function does when one of its operands has resolved it before (dispatch.SparseOp.repeat), without the
+// interpreter for the implementations that end in one call of a Handle: an F.linear of one token took 9.0 us of host time, 3.3
+// of them between the torch function and the handle, and takes 6.9.
+PyObject *g_wrapper_type = nullptr, *g_profiling = nullptr;  // SparseTensorWrapper, [bool]
+PyObject *g_s_sparsified_ops, *g_s_sparse_op, *g_s_disp_state, *g_s_fast, *g_s_native, *g_s_repeat, *g_s_container, *g_s_native_handle, *g_s_nm_strides,
+    *g_s_kernel, *g_s_expanded;
+
+struct Ref {  // owned reference
+    PyObject *p;
+    explicit Ref(PyObject *o) : p(o) {}
+    Ref(const Ref &) = delete;
+    ~Ref() { Py_XDECREF(p); }
+};
+
+// set_dispatch(wrapper_type, profiling_switch)
+PyObject *py_set_dispatch(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    if (nargs != 2 || !PyType_Check(a[0]) || !PyList_Check(a[1])) {
+        PyErr_SetString(PyExc_TypeError, "set_dispatch(wrapper_type, profiling_switch)");
+        return nullptr;
+    }
+    g_wrapper_type = Py_NewRef(a[0]);
+    g_profiling = Py_NewRef(a[1]);
+    Py_RETURN_NONE;
+}
+
+// First item of a wrapper's container (borrowed), or NULL.
+PyObject *payload_of(PyObject *wrapper) {
+    Ref c(PyObject_GetAttr(wrapper, g_s_container));
+    if (!c.p || !PyList_Check(c.p) || PyList_GET_SIZE(c.p) < 1) {
+        PyErr_Clear();
+        return nullptr;
+    }
+    return PyList_GET_ITEM(c.p, 0);  // the wrapper keeps the list
+}
+
+// The call on the weight's handle: kind "linear" (x, weight[, bias]) or "mm" (weight, b); NotImplemented when the general route has to decide.
+PyObject *native_call(PyObject *kind, PyObject *args) {
+    const bool mm = PyUnicode_CompareWithASCIIString(kind, "mm") == 0;
+    PyObject *gnm = payload_of(PyTuple_GET_ITEM(args, mm ? 0 : 1));
+    if (!gnm) Py_RETURN_NOTIMPLEMENTED;
+    Ref keep(Py_NewRef(gnm));
+    Ref strides(PyObject_GetAttr(gnm, g_s_nm_strides)), handle(PyObject_GetAttr(gnm, g_s_native_handle));
+    if (!strides.p || !handle.p || !PyDict_Check(strides.p) || Py_TYPE(handle.p) != &handle_type) {
+        PyErr_Clear();
+        Py_RETURN_NOTIMPLEMENTED;
+    }
+    if (mm) {
+        PyObject *b = PyTuple_GET_ITEM(args, 1);
+        if (THPVariable_Unpack(b).dim() != 2) Py_RETURN_NOTIMPLEMENTED;
+        PyObject *call[2] = {gnm, b};
+        return handle_mm(handle.p, call, 2);
+    }
+    PyObject *kernel = PyDict_GetItemWithError(strides.p, g_s_kernel);
+    if (kernel && PyUnicode_Check(kernel) && PyUnicode_Compare(kernel, g_s_expanded) == 0) Py_RETURN_NOTIMPLEMENTED;
+    PyObject *call[5] = {gnm, PyTuple_GET_ITEM(args, 0), PyTuple_GET_SIZE(args) > 2 ? PyTuple_GET_ITEM(args, 2) : Py_None, g_zero, Py_None};
+    return handle_linear(handle.p, call, 5);
+}
+
+// repeat_call(func, args) -> result or NotImplemented
+PyObject *py_repeat_call(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    if (nargs != 2 || !PyTuple_Check(a[1])) Py_RETURN_NOTIMPLEMENTED;
+    PyObject *func = a[0], *args = a[1];
+    const Py_ssize_t n = PyTuple_GET_SIZE(args);
+    for (Py_ssize_t i = 0; i < n; i++) {
+        PyObject *t = PyTuple_GET_ITEM(args, i);
+        if (!PyType_IsSubtype(Py_TYPE(t), reinterpret_cast<PyTypeObject *>(g_wrapper_type))) continue;
+        Ref dict(PyObject_GenericGetDict(t, nullptr));
+        PyObject *ops = dict.p ? PyDict_GetItemWithError(dict.p, g_s_sparsified_ops) : nullptr;
+        PyObject *op = ops && PyDict_Check(ops) ? PyDict_GetItemWithError(ops, func) : nullptr;
+        if (!op) {
+            PyErr_Clear();
+            continue;
+        }
+        Ref sparse_op(PyObject_GetAttr(op, g_s_sparse_op));
+        if (!sparse_op.p) return nullptr;
+        Ref state(PyObject_GetAttr(sparse_op.p, g_s_disp_state));
+        if (!state.p) return nullptr;
+        PyObject *fast = PyDict_GetItemWithError(state.p, g_s_fast), *native = PyDict_GetItemWithError(state.p, g_s_native);
+        if (!fast) Py_RETURN_NOTIMPLEMENTED;
+        bool direct = native && PyUnicode_Check(native) && PyTuple_GET_SIZE(fast) == n && PyList_GET_ITEM(g_profiling, 0) == Py_False;
+        for (Py_ssize_t j = 0; j < n && direct; j++) {  // same types and formats, nothing that needs a gradient
+            PyObject *x = PyTuple_GET_ITEM(args, j), *want = PyTuple_GET_ITEM(fast, j), *fmt = PyTuple_GET_ITEM(want, 1);
+            direct = reinterpret_cast<PyObject *>(Py_TYPE(x)) == PyTuple_GET_ITEM(want, 0) && THPVariable_Check(x);
+            if (direct && fmt != Py_None) {
+                PyObject *payload = payload_of(x);
+                direct = payload && reinterpret_cast<PyObject *>(Py_TYPE(payload)) == fmt;
+            }
+            if (direct && c10::GradMode::is_enabled()) direct = !THPVariable_Unpack(x).requires_grad();
+        }
+        if (direct) {
+            PyObject *r = native_call(native, args);
+            if (r != Py_NotImplemented) return r;
+            Py_DECREF(r);
+        }
+        return PyObject_CallMethodOneArg(sparse_op.p, g_s_repeat, args);
+    }
+    Py_RETURN_NOTIMPLEMENTED;
+    END_HANDLE_TH_ERRORS
+}
+
 #define NMG_METHOD(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
 PyMethodDef handle_methods[] = {
     NMG_METHOD("linear", handle_linear),
@@ -512,6 +616,8 @@ PyMethodDef module_methods[] = {
     NMG_METHOD("sparsify", py_sparsify),
     NMG_METHOD("gather", py_gather),
     NMG_METHOD("densify", py_densify),
+    NMG_METHOD("set_dispatch", py_set_dispatch),
+    NMG_METHOD("repeat_call", py_repeat_call),
     {"set_error_class", py_set_error_class, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr},
 };
@@ -532,6 +638,18 @@ PyMODINIT_FUNC PyInit__nmg_host(void) {
     g_s_idx = PyUnicode_InternFromString("idx");
     g_s_packed = PyUnicode_InternFromString("packed");
     g_s_packed_sp24 = PyUnicode_InternFromString("packed_sp24");
+    g_s_sparsified_ops = PyUnicode_InternFromString("sparsified_ops");
+    g_s_sparse_op = PyUnicode_InternFromString("sparse_op");
+    g_s_disp_state = PyUnicode_InternFromString("disp_state");
+    g_s_fast = PyUnicode_InternFromString("fast");
+    g_s_native = PyUnicode_InternFromString("native");
+    g_s_repeat = PyUnicode_InternFromString("repeat");
+    g_s_container = PyUnicode_InternFromString("_wrapped_tensor_container");
+    g_s_native_handle = PyUnicode_InternFromString("_native");
+    g_s_nm_strides = PyUnicode_InternFromString("nm_strides");
+    g_s_kernel = PyUnicode_InternFromString("kernel");
+    g_s_expanded = PyUnicode_InternFromString("sm100-expanded");
+    g_zero = PyLong_FromLong(0);  // NMG_EPI_NONE
     PyObject *mod = PyModule_Create(&module_def);
     if (!mod) return nullptr;
     if (PyModule_AddObjectRef(mod, "Handle", reinterpret_cast<PyObject *>(&handle_type)) < 0) {

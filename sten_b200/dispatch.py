@@ -470,6 +470,14 @@ def _repeat_call(func, args):
     return NotImplemented
 
 
+def use_native_repeat(host):
+    """The host extension's ``repeat_call``, which does the same and ends the calls it knows (``native`` in the dispatch state)
+    without returning to the interpreter."""
+    global _repeat_call
+    host.set_dispatch(SparseTensorWrapper, CUDA_PROFILING)
+    _repeat_call = host.repeat_call
+
+
 def sparse_tensor_builder(wrapper_type, wrapped_tensor_container, requires_grad, grad_fmt):
     """Unpickling / copying constructor; its module path and argument order are part of the pickle format."""
     assert issubclass(wrapper_type, SparseTensorWrapper)
@@ -953,6 +961,8 @@ class SparseOp:
                 and len(flat) == len(args) and all(a is b for a, b in zip(flat, args)) and len(st.get("fwd_sp_impls", ())) == 1):
             # the next call with operands of these types and formats takes repeat()
             st["fast"] = tuple((type(t), t.wrapped_tensor.__class__ if isinstance(t, SparseTensorWrapper) else None) for t in flat)
+            if self.out_fmt is None and st["fwd_out_fmt_sp_fmt"][2][0] is torch.Tensor:  # dense output, handed back as it is
+                st["native"] = getattr(st["op_impl_fwd"], "native_call", None)
         out_tuple = outputs if isinstance(outputs, (tuple, list)) else (outputs,)
         grad_fmts = _exact_formats(st["grad_out_fmt"], out_tuple)
         for o, gf in zip(out_tuple, grad_fmts):

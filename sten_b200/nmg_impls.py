@@ -104,6 +104,7 @@ def _linear_fwd(ctx, inputs, output_sparsifiers):
     return h.linear(gnm, x, bias, nat.NMG_EPI_NONE, None)
 
 
+_linear_fwd.native_call = "linear"  # a repeated call without gradients is one call of the handle (see dispatch.use_native_repeat)
 _LIN_OUT = [(sten.KeepAll, torch.Tensor)]
 sparse_torch_nn_functional_linear = sten.register_fwd_op_impl(
     operator=torch.nn.functional.linear, inp=(torch.Tensor, GroupedNMTensor, torch.Tensor), out=_LIN_OUT)(_linear_fwd)
@@ -159,6 +160,9 @@ def _mm_fwd(ctx, inputs, output_sparsifiers):
         raise sten.DispatchError("grouped n:m matmul expects a 2-D right operand")
     gnm, h = _native_weight(weight)
     return h.mm(gnm, b)
+
+
+_mm_fwd.native_call = "mm"
 
 
 def _mm_bwd(ctx, grad_outputs, input_sparsifiers):

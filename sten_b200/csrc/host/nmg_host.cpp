@@ -7,7 +7,9 @@
 #include <Python.h>
 
 #include <ATen/ATen.h>
+#include <ATen/EmptyTensor.h>
 #include <c10/core/GradMode.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Exceptions.h>
@@ -113,6 +115,11 @@ Rows rows_of(const at::Tensor &t, int64_t cols) {
     return Rows{t, cols ? t.numel() / cols : 0, cols, cols};
 }
 
+// Uninitialised tensor on the current device, straight from the caching allocator (torch's operator dispatch is half a microsecond)
+at::Tensor new_empty(c10::IntArrayRef sizes, at::ScalarType type) {
+    return at::detail::empty_generic(sizes, c10::cuda::CUDACachingAllocator::get(), c10::DispatchKeySet(c10::DispatchKey::CUDA), type, std::nullopt);
+}
+
 struct Geo {
     int64_t M, K;
     int n, m, g;
@@ -132,7 +139,7 @@ void call_spmm(const Geo &geo, int code, c10::Device dev, const at::Tensor &val,
     const at::Tensor v = packed_rows(val), i = packed_rows(idx), b = bias.defined() ? packed_rows(bias) : bias;
     const size_t nbytes = nmg_spmm_workspace_bytes(geo.M, geo.K, tokens, geo.n, geo.m, geo.g, code, layout, algo, packed.defined() ? 1 : 0);
     at::Tensor ws;
-    if (nbytes) ws = at::empty({(int64_t)nbytes}, val.options().dtype(at::kByte));
+    if (nbytes) ws = new_empty({(int64_t)nbytes}, at::kByte);
     void *st = stream_of(dev);
     void *wsp = nbytes ? ws.mutable_data_ptr() : nullptr;
     const void *pk = packed.defined() ? packed.const_data_ptr() : nullptr;
@@ -159,7 +166,7 @@ void call_spmm_t(const Geo &geo, int code, c10::Device dev, const at::Tensor &va
     size_t nbytes = 0;
     if (!sp24.defined()) {
         nbytes = nmg_spmm_t_workspace_bytes(geo.M, geo.K, dy.rows, geo.n, geo.m, geo.g, code, algo, packed.defined() ? 1 : 0);
-        if (nbytes) ws = at::empty({(int64_t)nbytes}, val.options().dtype(at::kByte));
+        if (nbytes) ws = new_empty({(int64_t)nbytes}, at::kByte);
     }
     int rc;
     PyThreadState *save = PyEval_SaveThread();
@@ -210,7 +217,7 @@ PyObject *py_spmm(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     const int64_t out_rows = out_tm ? tokens : geo.M, out_cols = out_tm ? geo.M : tokens;
     at::Tensor out = out0;
     if (!out.defined()) {
-        out = at::empty({out_rows, out_cols}, val.options());
+        out = new_empty({out_rows, out_cols}, val.scalar_type());
     } else {
         // the kernel writes out_rows rows of out_cols elements, ld_out apart: anything else would land outside `out`
         if (out.scalar_type() != val.scalar_type() || out.device() != dev)
@@ -249,7 +256,7 @@ PyObject *py_spmm_t(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     const c10::cuda::CUDAGuard guard(dev);
     const Rows dy = row_major_2d(dy0);
     if (dy.cols != geo.M) py_raise(PyExc_ValueError, "gradient shape " + shape_str(dy0.sizes()) + " does not match M=" + std::to_string(geo.M));
-    const at::Tensor dx = at::empty({dy.rows, geo.K}, val.options());
+    const at::Tensor dx = new_empty({dy.rows, geo.K}, val.scalar_type());
     const bool kept = sp24.defined() && dy.rows >= int_arg(a[11]) && (algo == NMG_ALGO_AUTO || algo == NMG_ALGO_TENSOR) && sp24_rows_ok(dy);
     if (dy.rows > 0) call_spmm_t(geo, code, dev, val, idx, packed, kept ? sp24 : at::Tensor(), dy, dx, algo);
     return THPVariable_Wrap(dx);
@@ -286,7 +293,7 @@ PyObject *py_sparsify(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     const c10::cuda::CUDAGuard guard(dev);
     const Dense3 d = dense3_arg(w);
     const Tiles t = tiles_of(d.B, d.M, d.K, n, m, g);
-    const at::Tensor val = at::empty({t.count, t.C, g, n}, w.options()), idx = at::empty({t.count, t.C, g, 1}, w.options().dtype(at::kShort));
+    const at::Tensor val = new_empty({t.count, t.C, g, n}, w.scalar_type()), idx = new_empty({t.count, t.C, g, 1}, at::kShort);
     void *st = stream_of(dev);
     PyThreadState *save = PyEval_SaveThread();
     const int rc = nmg_sparsify(d.t.const_data_ptr(), d.B, d.M, d.K, d.ld, d.bs, n, m, g, code, val.mutable_data_ptr(),
@@ -312,7 +319,7 @@ PyObject *py_gather(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     const Tiles t = tiles_of(d.B, d.M, d.K, n, m, g);
     const at::Tensor idx = packed_rows(idx0);
     if (idx.numel() != t.count * t.cc) py_raise(PyExc_ValueError, "idx does not belong to a layout of this shape");
-    const at::Tensor val = at::empty({t.count, t.C, g, n}, w.options());
+    const at::Tensor val = new_empty({t.count, t.C, g, n}, w.scalar_type());
     void *st = stream_of(dev);
     PyThreadState *save = PyEval_SaveThread();
     const int rc = nmg_gather(d.t.const_data_ptr(), static_cast<const int16_t *>(idx.const_data_ptr()), d.B, d.M, d.K, d.ld, d.bs, n, m, g, code,
@@ -333,7 +340,7 @@ PyObject *py_densify(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     const Geo geo = geo_args(a + 3);
     const c10::cuda::CUDAGuard guard(dev);
     const at::Tensor val = packed_rows(val0), idx = packed_rows(idx0);
-    const at::Tensor out = at::empty({B, geo.M, geo.K}, val.options());
+    const at::Tensor out = new_empty({B, geo.M, geo.K}, val.scalar_type());
     void *st = stream_of(dev);
     PyThreadState *save = PyEval_SaveThread();
     const int rc = nmg_densify(val.const_data_ptr(), static_cast<const int16_t *>(idx.const_data_ptr()), B, geo.M, geo.K, geo.n, geo.m, geo.g, code,
@@ -427,7 +434,7 @@ PyObject *handle_linear(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     const Rows act = rows_of(x, geo.K);
     c10::DimVector sizes(x.sizes().begin(), x.sizes().end());
     sizes.back() = geo.M;
-    const at::Tensor out = at::empty(sizes, val.options());
+    const at::Tensor out = new_empty(sizes, val.scalar_type());
     Epi epi;
     epi.act = (int)int_arg(a[3]);
     if (residual.defined()) {
@@ -460,7 +467,7 @@ PyObject *handle_mm(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     const c10::cuda::CUDAGuard guard(dev);
     const Rows act = row_major_2d(b);
     if (act.rows != geo.K) py_raise(PyExc_ValueError, "activation shape " + shape_str(b.sizes()) + " does not match K=" + std::to_string(geo.K));
-    const at::Tensor out = at::empty({geo.M, act.cols}, val.options());
+    const at::Tensor out = new_empty({geo.M, act.cols}, val.scalar_type());
     if (act.cols > 0) {
         // a handful of columns runs on the tensor cores when the packed copy is there already: keep one for the token-major call
         const bool wants = nmg_spmm_uses_packed(geo.M, geo.K, act.cols, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 0) != 0;
@@ -486,7 +493,7 @@ PyObject *handle_linear_t(PyObject *self, PyObject *const *a, Py_ssize_t nargs) 
     const Rows dy = rows_of(dy0, geo.M);
     c10::DimVector sizes(dy0.sizes().begin(), dy0.sizes().end());
     sizes.back() = geo.K;
-    const at::Tensor dx = at::empty(sizes, val.options());
+    const at::Tensor dx = new_empty(sizes, val.scalar_type());
     if (dy.rows > 0) {
         at::Tensor sp24, packed;
         // the compressed transposed copy serves the large batches of a 16-bit weight inside the 2:4 structure

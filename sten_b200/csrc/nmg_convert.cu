@@ -664,23 +664,29 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
             if (p < 31) in[off[p] + ((uint32_t)e >> 5)] = (e & 0xffffffff00000000ull) | (uint32_t)((c + 1) | (p << 16));
         }
         __syncwarp();
+        // a lane ranks two neighbours at a time: groups are padded to two, so they share a pattern
         const int slots = off[C - 1] + cnt[C - 1];
-        for (int e = sl; e < slots; e += L) {
-            const uint64_t key = in[e];
-            if (key == 0) continue;  // padding
-            const int p = (int)((uint32_t)key >> 16);
+        for (int e = 2 * sl; e < slots; e += 2 * L) {
+            const ulonglong2 key = *reinterpret_cast<const ulonglong2 *>(in + e);
+            const int p = (int)((uint32_t)key.x >> 16);
             const ulonglong2 *from = reinterpret_cast<const ulonglong2 *>(in + off[p]);
             const int pairs = (cnt[p] + 1) >> 1;
-            int rank = 0;
+            int rank0 = 0, rank1 = 0;
 #pragma unroll 2
             for (int j = 0; j < pairs; j++) {
                 const ulonglong2 v = from[j];
-                rank += v.x > key ? 1 : 0;
-                rank += v.y > key ? 1 : 0;
+                rank0 += v.x > key.x ? 1 : 0;
+                rank1 += v.x > key.y ? 1 : 0;
+                rank0 += v.y > key.x ? 1 : 0;
+                rank1 += v.y > key.y ? 1 : 0;
             }
-            const int c1 = (int)(key & 0xffff);
-            if (rank < g) list[p * g + rank] = (key & 0xffffffff00000000ull) | (uint32_t)c1;
-            else give_back(c1 - 1);
+            auto place = [&](uint64_t k, int rank) {
+                const int c1 = (int)(k & 0xffff);
+                if (rank < g) list[p * g + rank] = (k & 0xffffffff00000000ull) | (uint32_t)c1;
+                else give_back(c1 - 1);
+            };
+            place(key.x, rank0);
+            if (key.y != 0) place(key.y, rank1);  // zero: padding
         }
         __syncwarp();
         for (int p = sl; p < C; p += L) {
@@ -707,15 +713,28 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
                 for (int r = 0; r < M_; r++) a[r] = fabsf(DT<T>::to_f32(x[r * xs + c]));
                 uint32_t best_s = 0;
                 int best_p = -1;
+                bool tie = false;
 #pragma unroll
                 for (int p = 0; p < C; p++) {
                     float sc = a[ORD.row(p, 0)];
 #pragma unroll
                     for (int i = 1; i < N_; i++) sc = __fadd_rn(sc, a[ORD.row(p, i)]);
                     const uint32_t sb = __float_as_uint(sc), t = thr[p];
-                    bool open = sb >= best_s && sb >= t;
-                    if (open && sb == t && cnt[p] == g) open = c > col_of(list[p * g + g - 1]);  // equal score: the larger column wins
-                    if (open) { best_s = sb; best_p = p; }
+                    tie |= sb == t;
+                    if (sb >= best_s && sb >= t) { best_s = sb; best_p = p; }
+                }
+                if (tie) {  // a score like some pattern's weakest: if it is full, only the larger column gets in
+                    best_s = 0;
+                    best_p = -1;
+                    for (int p = 0; p < C; p++) {
+                        float sc = fabsf(DT<T>::to_f32(x[(int)ord[p * N_] * xs + c]));
+#pragma unroll
+                        for (int i = 1; i < N_; i++) sc = __fadd_rn(sc, fabsf(DT<T>::to_f32(x[(int)ord[p * N_ + i] * xs + c])));
+                        const uint32_t sb = __float_as_uint(sc), t = thr[p];
+                        if (sb < best_s || sb < t || (sb == t && cnt[p] == g && c < col_of(list[p * g + g - 1]))) continue;
+                        best_s = sb;
+                        best_p = p;
+                    }
                 }
                 if (best_p >= 0) {
                     prop[sl] = ((uint64_t)best_s << 32) | (uint32_t)(c + 1);

@@ -514,9 +514,9 @@ __global__ void __launch_bounds__(256, 4) sparsify_nm_kernel(SparsifyParams prm)
 // weights, 2:4, g = 16: 12 more proposals per 96-column tile).
 //   round 0   every column's best pattern from registers, four columns per lane and step; the proposals are grouped by
 //             pattern, and a proposal's place in its pattern's sorted list is its rank among them.
-//   rounds    every lane lets one of its displaced columns propose to the best pattern that would keep it (a pattern's
-//             threshold is the score of its weakest kept entry); the lanes that own the patterns insert what they were
-//             sent, at the same time, and hand the entry that falls out back to its column's lane.
+//   rounds    the first L columns of the tile's queue of displaced columns propose, each to the best pattern that would keep
+//             it (a pattern's threshold is the score of its weakest kept entry); the lanes that own the patterns insert what
+//             they were sent, at the same time, and queue the entry that falls out.
 //   zeros     scores of zero are placed by the closed form of sparsify_zero_phase.
 // Entries are 64-bit keys, score above column + 1: one comparison is the format's order.  The tile is staged in shared memory
 // (16-byte asynchronous copies where the alignment allows).  A tile's slab is 32 bytes more than a multiple of 128, so that
@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(256, 4) sparsify_nm_kernel(SparsifyParams prm)
 // 4096 x 4096, before (a warp per tile) and now: 2:4 fp32 187 -> 127 us, bf16 184 -> 111, 1:4 fp32 173 -> 98, 1:8 fp32 93 -> 80
 // (there all 32 lanes), 1:8 g = 4 fp16 195 -> 72.  Of the instructions ranking takes 40 %, the later rounds 25 %.  Tried and
 // slower: sorting a pattern per lane by a network (139), the tile left in global memory for more resident warps (129).
-struct SparsifyLanes { int xs, x, in, list, prop, thr, sent, cnt, off, fmask, zmask, words, total; };
+struct SparsifyLanes { int xs, x, in, list, prop, thr, sent, cnt, off, queue, qmask, zmask, words, total; };
 __host__ __device__ inline SparsifyLanes sparsify_lanes(int m, int cc, int C, int lanes, int es) {
     SparsifyLanes l;
     const int quads = (cc + 3) / 4;
@@ -539,8 +539,11 @@ __host__ __device__ inline SparsifyLanes sparsify_lanes(int m, int cc, int C, in
     l.sent = o;   o += C * 4;                               // lanes that propose to the pattern
     l.cnt = o;    o += C * 4;
     l.off = o;    o += C * 4;
-    l.fmask = o;  o += lanes * l.words * 4;                 // displaced columns of every lane
     l.zmask = o;  o += lanes * l.words * 4;                 // columns with no open pattern above zero
+    l.qmask = 1;
+    while (l.qmask < cc) l.qmask <<= 1;
+    l.queue = o;  o += l.qmask * 2 + 4;                     // ring of displaced columns, its write position
+    l.qmask--;
     l.total = ((o + 127) & ~127) + 32;
     return l;
 }
@@ -580,18 +583,15 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
     uint64_t *prop = reinterpret_cast<uint64_t *>(slab + lay.prop);
     uint32_t *thr = reinterpret_cast<uint32_t *>(slab + lay.thr), *sent = reinterpret_cast<uint32_t *>(slab + lay.sent);
     int *cnt = reinterpret_cast<int *>(slab + lay.cnt), *off = reinterpret_cast<int *>(slab + lay.off);
-    uint32_t *fmask = reinterpret_cast<uint32_t *>(slab + lay.fmask), *zmask = reinterpret_cast<uint32_t *>(slab + lay.zmask);
-    const int words = lay.words, xs = lay.xs, quads = xs >> 2;
-    uint32_t *my_f = fmask + sl * words, *my_z = zmask + sl * words;
+    uint16_t *queue = reinterpret_cast<uint16_t *>(slab + lay.queue);
+    const int words = lay.words, xs = lay.xs, quads = xs >> 2, qmask = lay.qmask;
+    uint32_t *tail = reinterpret_cast<uint32_t *>(queue + qmask + 1);
+    uint32_t *zmask = reinterpret_cast<uint32_t *>(slab + lay.zmask), *my_z = zmask + sl * words;
     const bool g_pow2 = (g & (g - 1)) == 0;
     const int g_shift = 31 - __clz(g);
     const T *dense = static_cast<const T *>(prm.dense);
     T *val = static_cast<T *>(prm.val);
-    // column c belongs to lane (c / 4) % L, as bit (c / 4) / L * 4 + c % 4
-    auto give_back = [&](int c) {
-        const int q = c >> 2, bit = (q / L) * 4 + (c & 3);
-        atomicOr(&fmask[(q % L) * words + (bit >> 5)], 1u << (bit & 31));
-    };
+    auto displace = [&](int c) { queue[atomicAdd(tail, 1u) & qmask] = (uint16_t)c; };  // a column is in the queue at most once
     auto col_of = [](uint64_t key) { return (int)(uint32_t)key - 1; };
 
     const int64_t stride = (int64_t)gridDim.x * nwarps * TILES;
@@ -616,7 +616,8 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
                 for (int c = sl; c < xs; c += L) x[r * xs + c] = global_at(r, c);
         }
         for (int p = sl; p < C; p += L) cnt[p] = 0;
-        for (int w = 0; w < words; w++) my_f[w] = my_z[w] = 0;
+        for (int w = 0; w < words; w++) my_z[w] = 0;
+        if (sl == 0) *tail = 0;
         cp_async_wait<0>();
         __syncwarp();
 
@@ -683,7 +684,7 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
             auto place = [&](uint64_t k, int rank) {
                 const int c1 = (int)(k & 0xffff);
                 if (rank < g) list[p * g + rank] = (k & 0xffffffff00000000ull) | (uint32_t)c1;
-                else give_back(c1 - 1);
+                else displace(c1 - 1);
             };
             place(key.x, rank0);
             if (key.y != 0) place(key.y, rank1);  // zero: padding
@@ -699,15 +700,13 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
 
         // ---- later rounds.  Every round with a proposal makes at least one (column, pattern) proposal that was never made
         // before, so cc * C rounds cannot be exceeded.
+        uint32_t head = 0;
         for (int round = 0; round < cc * C; round++) {
-            uint32_t bits = 0;
-            int w = 0;
-            for (; w < words; w++)
-                if ((bits = my_f[w]) != 0) break;
-            if (!__any_sync(FULL, bits != 0)) break;
-            if (bits) {
-                const int bit = (w << 5) + __ffs(bits) - 1, c = ((bit >> 2) * L + sl) * 4 + (bit & 3);
-                my_f[w] = bits & (bits - 1);
+            const int queued = (int)(*tail - head);
+            const bool active = sl < queued;
+            if (!__any_sync(FULL, active)) break;
+            if (active) {
+                const int c = queue[(head + sl) & qmask];
                 float a[M_];
 #pragma unroll
                 for (int r = 0; r < M_; r++) a[r] = fabsf(DT<T>::to_f32(x[r * xs + c]));
@@ -740,9 +739,12 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
                     prop[sl] = ((uint64_t)best_s << 32) | (uint32_t)(c + 1);
                     atomicOr(&sent[best_p], 1u << sl);
                 } else {
-                    my_z[w] |= bits & -bits;  // nothing above zero is open: placed by the zero phase
+                    // nothing above zero is open: placed by the zero phase.  Column c is bit (c / 4) / L * 4 + c % 4 of lane (c / 4) % L
+                    const int q = c >> 2, bit = (q / L) * 4 + (c & 3);
+                    atomicOr(&zmask[(q % L) * words + (bit >> 5)], 1u << (bit & 31));
                 }
             }
+            head += (uint32_t)min(queued, L);
             __syncwarp();
             for (int p = sl; p < C; p += L) {
                 uint32_t from = sent[p];
@@ -755,7 +757,7 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
                     int j = n;
                     if (n == g) {
                         const uint64_t last = lp[--j];
-                        give_back(col_of(key < last ? key : last));  // the weakest falls out, a kept entry or the proposal
+                        displace(col_of(key < last ? key : last));  // the weakest falls out, a kept entry or the proposal
                         if (key < last) continue;
                     } else {
                         n++;

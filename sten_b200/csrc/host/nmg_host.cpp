@@ -308,14 +308,8 @@ PyObject *py_sparsify(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     NMG_PY_END
 }
 
-// gather(dense3, idx, n, m, g) -> val
-PyObject *py_gather(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
-    NMG_PY_BEGIN(5)
-    const at::Tensor &w = tensor_arg(a[0]), &idx0 = tensor_arg(a[1]);
-    const c10::Device dev = device_of({&w, &idx0});
-    const int code = dtype_code(w), n = (int)int_arg(a[2]), m = (int)int_arg(a[3]), g = (int)int_arg(a[4]);
-    const c10::cuda::CUDAGuard guard(dev);
-    const Dense3 d = dense3_arg(w);
+PyObject *gather_values(const Dense3 &d, const at::Tensor &idx0, int n, int m, int g, int code, c10::Device dev) {
+    const at::Tensor &w = d.t;
     const Tiles t = tiles_of(d.B, d.M, d.K, n, m, g);
     const at::Tensor idx = packed_rows(idx0);
     if (idx.numel() != t.count * t.cc) py_raise(PyExc_ValueError, "idx does not belong to a layout of this shape");
@@ -327,6 +321,16 @@ PyObject *py_gather(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     PyEval_RestoreThread(save);
     check(rc);
     return THPVariable_Wrap(val);
+}
+
+// gather(dense3, idx, n, m, g) -> val
+PyObject *py_gather(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(5)
+    const at::Tensor &w = tensor_arg(a[0]), &idx = tensor_arg(a[1]);
+    const c10::Device dev = device_of({&w, &idx});
+    const int code = dtype_code(w), n = (int)int_arg(a[2]), m = (int)int_arg(a[3]), g = (int)int_arg(a[4]);
+    const c10::cuda::CUDAGuard guard(dev);
+    return gather_values(dense3_arg(w), idx, n, m, g, code, dev);
     NMG_PY_END
 }
 
@@ -609,7 +613,23 @@ PyObject *py_repeat_call(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
 }
 
 #define NMG_METHOD(name, fn) {name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL, nullptr}
+// gather(gnm, dense2d) -> the dense tensor's values at the weight's kept positions
+PyObject *handle_gather(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(2)
+    const Geo &geo = reinterpret_cast<Handle *>(self)->geo;
+    const at::Tensor idx = attr_tensor(a[0], g_s_idx);
+    const at::Tensor &w = tensor_arg(a[1]);
+    const c10::Device dev = device_of({&w, &idx});
+    const int code = dtype_code(w);
+    const c10::cuda::CUDAGuard guard(dev);
+    const Rows r = row_major_2d(w);
+    if (r.rows != geo.M || r.cols != geo.K) py_raise(PyExc_ValueError, "expected a tensor of the weight's shape, got " + shape_str(w.sizes()));
+    return gather_values(Dense3{r.t, 1, geo.M, geo.K, r.ld, geo.M * r.ld}, idx, geo.n, geo.m, geo.g, code, dev);
+    NMG_PY_END
+}
+
 PyMethodDef handle_methods[] = {
+    NMG_METHOD("gather", handle_gather),
     NMG_METHOD("linear", handle_linear),
     NMG_METHOD("mm", handle_mm),
     NMG_METHOD("linear_t", handle_linear_t),

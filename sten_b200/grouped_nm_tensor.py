@@ -100,6 +100,9 @@ class GroupedNMTensor:
         s = self.nm_strides
         if tuple(dense_tensor.shape) != tuple(s["dense_shape"]):
             raise ValueError(f"expected a tensor of shape {tuple(s['dense_shape'])}, got {tuple(dense_tensor.shape)}")
+        h = self.native()
+        if h is not None:
+            return GroupedNMTensor(h.gather(self, dense_tensor), self.idx, s)
         view3, _ = _kernel_view(dense_tensor.detach(), s["sparse_dim"], s["group_dim"])
         val = ops.gather_layout(view3, self.idx, s["n"], s["m"], s["group_size"])
         return GroupedNMTensor(val, self.idx, s)

@@ -122,10 +122,10 @@ def _linear_bwd(ctx, grad_outputs, input_sparsifiers):
     if needs[0]:
         dx = h.linear_t(gnm, dy, ops.SP24_MIN_TOKENS)
     if needs[1] or needs[2]:
-        dy2d = dy.reshape(-1, dy.shape[-1])
+        dy2d = dy if dy.dim() == 2 else dy.reshape(-1, dy.shape[-1])
     if needs[1]:
         # dense weight gradient (training of nmg weights is outside the inference hot path): plain GEMM
-        dw = dy2d.t().mm(x.reshape(-1, x.shape[-1]))
+        dw = dy2d.t().mm(x if x.dim() == 2 else x.reshape(-1, x.shape[-1]))
     if has_bias and needs[2]:
         db = dy2d.sum(dim=0)
     return (dx, dw, db) if has_bias else (dx, dw)

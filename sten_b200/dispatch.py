@@ -964,7 +964,6 @@ class SparseOp:
             st["call_signature"] = signature
         st["call_stubs"] = call_stubs
         st["call_order"] = order
-        st["bound_args"] = bound
 
         need_grad = torch.is_grad_enabled() and any(t.requires_grad for t in flat)
         if need_grad:

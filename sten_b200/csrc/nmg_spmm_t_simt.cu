@@ -57,10 +57,93 @@ __global__ void build_natural_kernel(const NaturalParams prm) {
     }
 }
 
+// The same for n <= 2, byte patterns and chunks of whole 16-byte pieces.  HBM-bound work that one scattered store per slot and
+// a memset before it did slowly (with the row masks, 4096 x 4096: 74 us bf16 2:4, 128 fp32; now 56 and 75): an item is R row-blocks x Q chunks, about 512
+// columns, one piece of eight slots per thread; slots are scattered in shared memory and leave as whole rows, zeros included.
+constexpr int NATURAL_THREADS = 256;
+struct NaturalRows { int R, Q, groups, spans; };
+template <typename T, int N_>
+__global__ void __launch_bounds__(NATURAL_THREADS) build_natural_rows_kernel(const NaturalParams prm, const NaturalRows it) {
+    extern __shared__ __align__(16) char smem[];
+    constexpr int V = 16 / (int)sizeof(T), VL = N_ * 8 / V;  // values per 16 bytes, 16-byte loads of values per piece
+    const int R = it.R, Q = it.Q, cc = prm.cc, cols = Q * cc, tid = (int)threadIdx.x;
+    T *vals = reinterpret_cast<T *>(smem);                               // [R][cols * N_]
+    uint8_t *pats = reinterpret_cast<uint8_t *>(vals + R * cols * N_);  // [R][cols]
+    for (int i = tid; i < R * cols * N_ / V; i += NATURAL_THREADS) reinterpret_cast<uint4 *>(vals)[i] = make_uint4(0, 0, 0, 0);
+    for (int i = tid; i < R * cols / 8; i += NATURAL_THREADS) reinterpret_cast<uint2 *>(pats)[i] = make_uint2(0, 0);
+    const int per_chunk = R * cc / 8, q = tid / per_chunk, e8 = (tid - q * per_chunk) * 8, j = e8 / cc, slot0 = e8 - j * cc;
+    const bool has = tid < Q * per_chunk;
+    const T *val = static_cast<const T *>(prm.val);
+    T *nval = static_cast<T *>(prm.nval);
+    const int64_t plane = prm.nb * prm.Kp * N_;
+    for (int64_t item = blockIdx.x; item < (int64_t)it.groups * it.spans; item += gridDim.x) {
+        const int span = (int)(item / it.groups), grp = (int)(item - (int64_t)span * it.groups);
+        __syncthreads();  // the buffers are zeros
+        const int64_t mb0 = (int64_t)grp * R;
+        if (has && span * Q + q < prm.nc && mb0 + j < prm.nb) {
+            const int64_t e = ((int64_t)(span * Q + q) * prm.nb + mb0 + j) * cc + slot0;
+            const uint4 iv = __ldg(reinterpret_cast<const uint4 *>(prm.idx + e));
+            uint4 vv[VL];
+#pragma unroll
+            for (int i = 0; i < VL; i++) vv[i] = __ldg(reinterpret_cast<const uint4 *>(val + e * N_) + i);
+            const int16_t *ci = reinterpret_cast<const int16_t *>(&iv);
+            const T *v = reinterpret_cast<const T *>(vv);
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int c = ci[k];
+                if ((unsigned)c >= (unsigned)cc) continue;  // malformed index: leave the column empty
+                const int o = j * cols + q * cc + c;
+                pats[o] = (uint8_t)((slot0 + k) / prm.g * prm.m);
+                if (N_ == 1) {
+                    vals[o] = v[k];
+                } else {  // pairs of columns, planar
+                    T *d = vals + (o & ~1) * 2 + (o & 1);
+                    d[0] = v[k * N_];
+                    d[2] = v[k * N_ + (N_ - 1)];
+                }
+            }
+        }
+        __syncthreads();
+        const int64_t c0 = (int64_t)span * cols;
+        const int rows = (int)(prm.nb - mb0 < R ? prm.nb - mb0 : R), lim = (int)(prm.Kp - c0 < cols ? prm.Kp - c0 : cols);
+        for (int i = tid; i < R * cols / 8; i += NATURAL_THREADS) {
+            const int l = i / (cols / 8), c = (i - l * (cols / 8)) * 8;
+            if (l < rows && c < lim) {
+                const int64_t o = (mb0 + l) * prm.Kp + c0 + c;
+                *reinterpret_cast<uint2 *>(static_cast<uint8_t *>(prm.pat) + o) = *reinterpret_cast<const uint2 *>(pats + i * 8);
+#pragma unroll
+                for (int u = 0; u < VL; u++) reinterpret_cast<uint4 *>(nval + o * N_)[u] = reinterpret_cast<const uint4 *>(vals + i * 8 * N_)[u];
+                if (sizeof(T) == 4 && prm.planes) {  // exact three-way split
+#pragma unroll
+                    for (int u = 0; u < N_; u++) {
+                        __align__(16) __nv_bfloat16 w[3][8];
+#pragma unroll
+                        for (int k = 0; k < 8; k++) {
+                            const float f = DT<T>::to_f32(vals[(i * N_ + u) * 8 + k]);
+                            w[0][k] = __float2bfloat16_rn(f);
+                            const float r1 = f - __bfloat162float(w[0][k]);
+                            w[1][k] = __float2bfloat16_rn(r1);
+                            w[2][k] = __float2bfloat16_rn(r1 - __bfloat162float(w[1][k]));
+                        }
+#pragma unroll
+                        for (int t = 0; t < 3; t++) *reinterpret_cast<uint4 *>(prm.planes + t * plane + o * N_ + u * 8) = *reinterpret_cast<const uint4 *>(w[t]);
+                    }
+                }
+            }
+            *reinterpret_cast<uint2 *>(pats + i * 8) = make_uint2(0, 0);
+#pragma unroll
+            for (int u = 0; u < VL; u++) reinterpret_cast<uint4 *>(vals + i * 8 * N_)[u] = make_uint4(0, 0, 0, 0);
+        }
+    }
+}
+
 // Row masks of the forward tensor-core kernel, [k-block of 64 columns][row][8 n bytes]: per slot two words of "the row holds
 // the column's value of this slot"; bit 8 j + q of a word is column 4 q + j of its 32.
 __global__ void __launch_bounds__(256) build_masks_kernel(const uint8_t *__restrict__ pat, const int8_t *__restrict__ slot_of_row, uint32_t *__restrict__ masks, int64_t M,
-                                                          int64_t Kp, int64_t rows, int n, int m) {
+                                                          int64_t Kp, int64_t rows, int n, int m, int patterns) {
+    __shared__ int8_t table[31 * 16];  // row -> slot of every pattern; at most 28 patterns of up to 16 rows
+    for (int i = threadIdx.x; i < patterns * m; i += blockDim.x) table[i] = slot_of_row[i];
+    __syncthreads();
     const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, kb = blockIdx.y;
     if (row >= rows) return;
     uint32_t mask[2][2] = {{0, 0}, {0, 0}};
@@ -76,7 +159,7 @@ __global__ void __launch_bounds__(256) build_masks_kernel(const uint8_t *__restr
             for (int c = 0; c < 16; c++) {
                 const int col = i * 16 + c, bit = 8 * (col & 3) + ((col & 31) >> 2);
                 // the byte is pattern * m: where the pattern's row table starts
-                const int s = slot_of_row[((w[c >> 2] >> (8 * (c & 3))) & 0xffu) + r];
+                const int s = table[((w[c >> 2] >> (8 * (c & 3))) & 0xffu) + r];
                 if (s == 0) mask[0][col >> 5] |= 1u << bit;
                 if (s == 1) mask[1][col >> 5] |= 1u << bit;
             }
@@ -127,17 +210,33 @@ int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16
     const int64_t total = geo.nb * geo.nc * geo.cc;
     int64_t blocks = (total + 255) / 256;
     if (blocks > 148 * 64) blocks = 148 * 64;
+    const bool rows_kernel = bwd_specialised(geo.n, geo.m) && geo.n <= 2 && geo.cc % 8 == 0 && geo.cc <= 8 * NATURAL_THREADS &&
+                             ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0;
+    if (lay.plane_bytes) p.planes = reinterpret_cast<__nv_bfloat16 *>(static_cast<char *>(nval) + lay.val_bytes + lay.mask_bytes);
+    if (rows_kernel) {
+        NaturalRows it;
+        it.Q = 512 / geo.cc < 1 ? 1 : 512 / geo.cc;
+        it.R = NATURAL_THREADS * 8 / (it.Q * geo.cc);  // one piece per thread
+        it.groups = (int)((geo.nb + it.R - 1) / it.R);
+        it.spans = (int)((p.Kp + it.Q * geo.cc - 1) / (it.Q * geo.cc));  // up to the padded width: the padding becomes zeros too
+        int sms = 148, rc;
+        if ((rc = device_sms(&sms))) return rc;
+        const int64_t items = (int64_t)it.groups * it.spans, cap = (int64_t)sms * 8;
+        const size_t smem = (size_t)it.R * it.Q * geo.cc * (geo.n * dtype_size(dtype) + 1);
+        NMG_DISPATCH_DTYPE(dtype, T, {
+            if (geo.n == 1) build_natural_rows_kernel<T, 1><<<(unsigned)(items < cap ? items : cap), NATURAL_THREADS, smem, st>>>(p, it);
+            else build_natural_rows_kernel<T, 2><<<(unsigned)(items < cap ? items : cap), NATURAL_THREADS, smem, st>>>(p, it);
+        });
+    } else {
     // every (mb, k) of the chunks is written exactly once because idx is a permutation per tile; clear first so that the
     // columns between the last chunk and the padded width, and what a malformed idx leaves out, are zeros
     NMG_CUDA(cudaMemsetAsync(pat, 0, lay.pat_bytes + lay.val_bytes, st));  // the values follow the patterns
-    if (lay.plane_bytes) {
-        p.planes = reinterpret_cast<__nv_bfloat16 *>(static_cast<char *>(nval) + lay.val_bytes + lay.mask_bytes);
-        NMG_CUDA(cudaMemsetAsync(p.planes, 0, lay.plane_bytes, st));
-    }
+    if (lay.plane_bytes) NMG_CUDA(cudaMemsetAsync(p.planes, 0, lay.plane_bytes, st));
     if (total < 0x40000000ll) {
         NMG_DISPATCH_DTYPE(dtype, T, (build_natural_kernel<T, true><<<(unsigned)blocks, 256, 0, st>>>(p)));
     } else {
         NMG_DISPATCH_DTYPE(dtype, T, (build_natural_kernel<T, false><<<(unsigned)blocks, 256, 0, st>>>(p)));
+    }
     }
     if (lay.mask_bytes) {
         PatternTable tab;
@@ -146,7 +245,7 @@ int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16
         const int64_t rows = natural_mask_rows(geo), kbs = natural_width(geo) / 64;
         if (kbs > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "weight has too many columns for the column-ordered copy");
         build_masks_kernel<<<dim3((unsigned)((rows + 255) / 256), (unsigned)kbs), 256, 0, st>>>(
-            static_cast<const uint8_t *>(pat), tab.slot_of_row, reinterpret_cast<uint32_t *>(static_cast<char *>(nval) + lay.val_bytes), geo.M, natural_width(geo), rows, geo.n, geo.m);
+            static_cast<const uint8_t *>(pat), tab.slot_of_row, reinterpret_cast<uint32_t *>(static_cast<char *>(nval) + lay.val_bytes), geo.M, natural_width(geo), rows, geo.n, geo.m, geo.C);
     }
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;

@@ -1144,6 +1144,73 @@ extern "C" int nmg_densify(const void *val, const int16_t *idx, int64_t batch, i
     return NMG_OK;
 }
 
+// The same for n <= 2 and chunks of whole 16-byte pieces.  Element by element from global memory 4096 x 4096 bf16 2:4 took 29 us, now 18
+// (59 MB: 9 us at the copy rate).  An item is R row-blocks x Q chunks, about 512 columns; its rows come in whole lines, and a
+// thread gathers one piece of eight slots from shared memory and stores it in 16-byte pieces.  VEC: 16-byte aligned rows.
+constexpr int GATHER_THREADS = 256;
+struct GatherRows { int R, Q, groups, spans; };
+template <typename T, int N_, bool VEC>
+__global__ void __launch_bounds__(GATHER_THREADS) gather_rows_kernel(const GatherParams prm, const GatherRows it) {
+    extern __shared__ __align__(16) char smem[];
+    constexpr int V = 16 / (int)sizeof(T);
+    const int m = prm.m, cc = prm.cc, R = it.R, Q = it.Q, cols = Q * cc, rows = R * m, tid = (int)threadIdx.x;
+    T *tile = reinterpret_cast<T *>(smem);                                 // [rows][cols]
+    int8_t *ord = reinterpret_cast<int8_t *>(tile + (size_t)rows * cols);  // [C][N_]
+    for (int i = tid; i < prm.C * N_; i += GATHER_THREADS) ord[i] = prm.order[i];
+    const int per_chunk = R * cc / 8, q = tid / per_chunk, e8 = (tid - q * per_chunk) * 8, j = e8 / cc, slot0 = e8 - j * cc;
+    const bool has = tid < Q * per_chunk;
+    const T *dense = static_cast<const T *>(prm.dense);
+    T *val = static_cast<T *>(prm.val);
+    const int64_t per_batch = (int64_t)it.groups * it.spans, items = prm.tiles / (prm.nb * prm.nc) * per_batch;
+    for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
+        const int64_t b = item / per_batch;
+        const int in_batch = (int)(item - b * per_batch), span = in_batch / it.groups, grp = in_batch - span * it.groups;
+        const int64_t mb0 = (int64_t)grp * R, r0 = mb0 * m, c0 = (int64_t)span * cols;
+        const bool mine = has && span * Q + q < prm.nc && mb0 + j < prm.nb;
+        const int64_t slot = ((b * prm.nc + span * Q + q) * prm.nb + mb0 + j) * cc + slot0;
+        uint4 iv = make_uint4(0, 0, 0, 0);
+        if (mine) iv = __ldg(reinterpret_cast<const uint4 *>(prm.idx + slot));
+        const T *src = dense + b * prm.batch_stride + r0 * prm.ld + c0;
+        const int row_lim = (int)(prm.M - r0 < rows ? prm.M - r0 : rows), col_lim = (int)(prm.K - c0 < cols ? prm.K - c0 : cols);
+        __syncthreads();  // the previous item has been gathered
+        if constexpr (VEC) {
+            const int vpl = cols / V;
+            for (int i = tid; i < rows * vpl; i += GATHER_THREADS) {
+                const int l = i / vpl, c = (i - l * vpl) * V;
+                if (l < row_lim && c + V <= col_lim) {
+                    cp_async_16(tile + i * V, src + l * prm.ld + c);
+                } else {  // the weight's edge
+#pragma unroll
+                    for (int u = 0; u < V; u++) tile[i * V + u] = (l < row_lim && c + u < col_lim) ? __ldg(src + l * prm.ld + c + u) : DT<T>::from_f32(0.f);
+                }
+            }
+            cp_async_commit();
+            cp_async_wait<0>();
+        } else {
+            for (int i = tid; i < rows * cols; i += GATHER_THREADS) {
+                const int l = i / cols, c = i - l * cols;
+                tile[i] = (l < row_lim && c < col_lim) ? __ldg(src + l * prm.ld + c) : DT<T>::from_f32(0.f);
+            }
+        }
+        __syncthreads();
+        if (mine) {
+            const int16_t *ci = reinterpret_cast<const int16_t *>(&iv);
+            __align__(16) T out[8 * N_];
+            const T *base = tile + j * m * cols + q * cc;
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const int c = ci[k];
+                const int8_t *o = ord + (slot0 + k) / prm.g * N_;
+#pragma unroll
+                for (int t = 0; t < N_; t++) out[k * N_ + t] = (unsigned)c < (unsigned)cc ? base[(int)o[t] * cols + c] : DT<T>::from_f32(0.f);  // a malformed index reads as zero
+            }
+            uint4 *dst = reinterpret_cast<uint4 *>(val + slot * N_);
+#pragma unroll
+            for (int i = 0; i < 8 * N_ / V; i++) dst[i] = reinterpret_cast<const uint4 *>(out)[i];
+        }
+    }
+}
+
 extern "C" int nmg_gather(const void *dense, const int16_t *idx, int64_t batch, int64_t M, int64_t K, int64_t ld_dense,
                           int64_t batch_stride, int n, int m, int g, int dtype, void *val, void *stream) {
     Geo geo;
@@ -1161,10 +1228,37 @@ extern "C" int nmg_gather(const void *dense, const int16_t *idx, int64_t batch, 
     p.M = M; p.K = K; p.ld = ld_dense; p.batch_stride = batch_stride;
     p.nb = geo.nb; p.nc = geo.nc; p.tiles = batch * geo.nb * geo.nc;
     p.n = n; p.m = m; p.g = g; p.C = geo.C; p.cc = geo.cc;
+    cudaStream_t st = (cudaStream_t)stream;
+    const size_t es = dtype_size(dtype);
+    GatherRows it;
+    it.Q = 512 / geo.cc < 1 ? 1 : 512 / geo.cc;
+    if (it.Q > geo.nc) it.Q = (int)geo.nc;
+    it.R = GATHER_THREADS * 8 / (it.Q * geo.cc);
+    const int fit = (int)(32 * 1024 / ((size_t)m * it.Q * geo.cc * es));
+    if (it.R > fit) it.R = fit;
+    if (it.R >= 1 && n <= 2 && geo.cc % 8 == 0 && ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0 && geo.nb < 0x3fffffff &&
+        geo.nc < 0x3fffffff) {
+        it.groups = (int)((geo.nb + it.R - 1) / it.R);
+        it.spans = (int)((geo.nc + it.Q - 1) / it.Q);
+        const size_t smem = (size_t)it.R * m * it.Q * geo.cc * es + (size_t)geo.C * n + 16;  // at most 34 KB
+        const int64_t items = batch * it.groups * it.spans, cap = (int64_t)sm_count() * 6;
+        const unsigned grid = (unsigned)(items < cap ? items : cap);
+        const bool vec = (ld_dense * es) % 16 == 0 && (batch == 1 || (batch_stride * es) % 16 == 0) && (reinterpret_cast<uintptr_t>(dense) & 15) == 0;
+        NMG_DISPATCH_DTYPE(dtype, T, {
+            if (n == 1) {
+                if (vec) gather_rows_kernel<T, 1, true><<<grid, GATHER_THREADS, smem, st>>>(p, it);
+                else gather_rows_kernel<T, 1, false><<<grid, GATHER_THREADS, smem, st>>>(p, it);
+            } else {
+                if (vec) gather_rows_kernel<T, 2, true><<<grid, GATHER_THREADS, smem, st>>>(p, it);
+                else gather_rows_kernel<T, 2, false><<<grid, GATHER_THREADS, smem, st>>>(p, it);
+            }
+        });
+        NMG_CUDA(cudaGetLastError());
+        return NMG_OK;
+    }
     int64_t ctas = (p.tiles + 7) / 8;
     const int64_t max_ctas = (int64_t)sm_count() * 16;
     if (ctas > max_ctas) ctas = max_ctas;
-    cudaStream_t st = (cudaStream_t)stream;
     NMG_DISPATCH_DTYPE(dtype, T, { gather_layout_kernel<T><<<(unsigned)ctas, 256, 0, st>>>(p); });
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;

@@ -29,3 +29,18 @@ def test_sparsify_and_densify_at_tile_edges(n, m, g, dtype):
             d = torch.full((M, K + off), 7.0, dtype=dtype, device=cuda())
             ops.densify_into(val, idx, d[None, :, off:], n, m, g) if hasattr(ops, "densify_into") else None
             assert np.array_equal(np_of(ops.densify(val, idx, 1, M, K, n, m, g).float())[0], orc.densify(val_o, idx_o, (M, K), n, m, g))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,m,g,B,M,K,off", [(2, 4, 16, 1, 64, 1152, 0), (1, 8, 16, 2, 130, 1000, 3), (2, 8, 16, 1, 24, 449, 0), (1, 16, 4, 1, 17, 700, 0),
+                                              (1, 4, 4, 3, 36, 40, 0), (2, 4, 3, 1, 20, 100, 1), (1, 4, 512, 1, 9, 5000, 0)])
+def test_gather_at_tile_edges(n, m, g, B, M, K, off, dtype):
+    """Values of another tensor at a layout's positions, against the densified mask: whole and cut items, unaligned rows."""
+    from sten_b200 import ops
+    w = seeded_normal((B, M, K), 1).to(dtype).to(cuda())
+    val, idx = ops.sparsify(w, n, m, g)
+    other = seeded_normal((B, M, K + off), 2).to(dtype).to(cuda())[:, :, off:]
+    got = ops.gather_layout(other, idx, n, m, g)
+    mask = ops.densify(torch.ones_like(val), idx, B, M, K, n, m, g)
+    assert torch.equal(ops.densify(got, idx, B, M, K, n, m, g), torch.where(mask != 0, other, torch.zeros_like(other)))
+    assert torch.equal(ops.gather_layout(w, idx, n, m, g), val)

@@ -85,6 +85,12 @@ int nmg_densify(const void *val, const int16_t *idx, int64_t batch, int64_t M, i
 int nmg_gather(const void *dense, const int16_t *idx, int64_t batch, int64_t M, int64_t K, int64_t ld_dense,
                int64_t batch_stride, int n, int m, int g, int dtype, void *val, void *stream);
 
+/* Column sums of a [rows][ld] matrix, fp32 accumulation, out[cols] in x's dtype: the bias gradient of a linear.  workspace:
+ * device scratch of at least nmg_column_sum_workspace_bytes(rows, cols) bytes. */
+size_t nmg_column_sum_workspace_bytes(int64_t rows, int64_t cols);
+int nmg_column_sum(const void *x, int64_t rows, int64_t cols, int64_t ld, int dtype, void *out, void *workspace,
+                   size_t workspace_bytes, void *stream);
+
 /* Per-block top-n by magnitude without the group constraint.  Replaces PerfectNMTensor.from_dense / to_dense
  * (src/sten/grouped_nm/grouped_nm_tensor.py:1010-1066: pad, reshape, abs().argsort(descending), gather / scatter_), the
  * upper bound the reference's conversion test compares the grouped layout against (tests/test_nmg.py:73-83).

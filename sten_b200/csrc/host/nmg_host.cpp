@@ -482,11 +482,28 @@ PyObject *handle_mm(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     NMG_PY_END
 }
 
+// dx = dy W; dy's leading dims all count as rows
+at::Tensor input_gradient(Handle *h, PyObject *gnm, const at::Tensor &val, const at::Tensor &idx, const at::Tensor &dy0, const Rows &dy, int64_t sp24_min_tokens,
+                          int code, c10::Device dev) {
+    const Geo &geo = h->geo;
+    c10::DimVector sizes(dy0.sizes().begin(), dy0.sizes().end());
+    sizes.back() = geo.K;
+    const at::Tensor dx = new_empty(sizes, val.scalar_type());
+    if (dy.rows > 0) {
+        at::Tensor sp24, packed;
+        // the compressed transposed copy serves the large batches of a 16-bit weight inside the 2:4 structure
+        if (dy.rows >= sp24_min_tokens) sp24 = derived(*h->sp24, gnm, g_s_packed_sp24, val, idx);
+        if (!sp24.defined() && nmg_spmm_uses_packed(geo.M, geo.K, dy.rows, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 1))
+            packed = derived(*h->packed, gnm, g_s_packed, val, idx);
+        call_spmm_t(geo, code, dev, val, idx, packed, sp24.defined() && sp24_rows_ok(dy) ? sp24 : at::Tensor(), dy, dx, NMG_ALGO_AUTO);
+    }
+    return dx;
+}
+
 // linear_t(gnm, dy, sp24_min_tokens): dy [..., M] -> [..., K] = dy W
 PyObject *handle_linear_t(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     NMG_PY_BEGIN(3)
     Handle *h = reinterpret_cast<Handle *>(self);
-    const Geo &geo = h->geo;
     const at::Tensor val = attr_tensor(a[0], g_s_val), idx = attr_tensor(a[0], g_s_idx);
     const at::Tensor &dy0 = tensor_arg(a[1]);
     const c10::Device dev = device_of({&val, &idx, &dy0});
@@ -494,19 +511,32 @@ PyObject *handle_linear_t(PyObject *self, PyObject *const *a, Py_ssize_t nargs) 
     if (dy0.scalar_type() != val.scalar_type())
         py_raise(PyExc_TypeError, std::string("gradient dtype must match the weight dtype ") + c10::toString(val.scalar_type()));
     const c10::cuda::CUDAGuard guard(dev);
-    const Rows dy = rows_of(dy0, geo.M);
-    c10::DimVector sizes(dy0.sizes().begin(), dy0.sizes().end());
-    sizes.back() = geo.K;
-    const at::Tensor dx = new_empty(sizes, val.scalar_type());
-    if (dy.rows > 0) {
-        at::Tensor sp24, packed;
-        // the compressed transposed copy serves the large batches of a 16-bit weight inside the 2:4 structure
-        if (dy.rows >= int_arg(a[2])) sp24 = derived(*h->sp24, a[0], g_s_packed_sp24, val, idx);
-        if (!sp24.defined() && nmg_spmm_uses_packed(geo.M, geo.K, dy.rows, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 1))
-            packed = derived(*h->packed, a[0], g_s_packed, val, idx);
-        call_spmm_t(geo, code, dev, val, idx, packed, sp24.defined() && sp24_rows_ok(dy) ? sp24 : at::Tensor(), dy, dx, NMG_ALGO_AUTO);
+    return THPVariable_Wrap(input_gradient(h, a[0], val, idx, dy0, rows_of(dy0, h->geo.M), int_arg(a[2]), code, dev));
+    NMG_PY_END
+}
+
+// column_sum(dy): [..., M] -> [M], the bias gradient
+PyObject *py_column_sum(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(1)
+    const at::Tensor &x0 = tensor_arg(a[0]);
+    const c10::Device dev = device_of({&x0});
+    const int code = dtype_code(x0);
+    const c10::cuda::CUDAGuard guard(dev);
+    if (x0.dim() < 1) py_raise(PyExc_ValueError, "expected at least one dimension");
+    const Rows x = rows_of(x0, x0.size(-1));
+    const at::Tensor out = new_empty({x.cols}, x0.scalar_type());
+    if (x.rows < 1 || x.cols < 1) {
+        out.zero_();
+        return THPVariable_Wrap(out);
     }
-    return THPVariable_Wrap(dx);
+    const size_t nbytes = nmg_column_sum_workspace_bytes(x.rows, x.cols);
+    const at::Tensor ws = new_empty({(int64_t)nbytes}, at::kByte);
+    void *st = stream_of(dev);
+    PyThreadState *save = PyEval_SaveThread();
+    const int rc = nmg_column_sum(x.t.const_data_ptr(), x.rows, x.cols, x.ld, code, out.mutable_data_ptr(), ws.mutable_data_ptr(), nbytes, st);
+    PyEval_RestoreThread(save);
+    check(rc);
+    return THPVariable_Wrap(out);
     NMG_PY_END
 }
 
@@ -642,6 +672,7 @@ PyMethodDef module_methods[] = {
     NMG_METHOD("spmm_t", py_spmm_t),
     NMG_METHOD("sparsify", py_sparsify),
     NMG_METHOD("gather", py_gather),
+    NMG_METHOD("column_sum", py_column_sum),
     NMG_METHOD("densify", py_densify),
     NMG_METHOD("set_dispatch", py_set_dispatch),
     NMG_METHOD("repeat_call", py_repeat_call),

@@ -1263,3 +1263,117 @@ extern "C" int nmg_gather(const void *dense, const int16_t *idx, int64_t batch, 
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;
 }
+
+// =====================================================================================================
+// Column sums (the bias gradient): out[c] = sum over rows of x[r][c], fp32 accumulation.
+// HBM-bound.  A lane owns one 16-byte piece of columns, the warps of a CTA and the CTAs of a column group stride over the rows;
+// partial sums meet in shared memory, then in the workspace, where a second kernel adds the row ranges in order.
+// 4096 x 4096 bf16 (33.5 MB, 5.2 us at the copy rate): 12.5 + 2.8 us from HBM, torch's reduction 21.
+// =====================================================================================================
+constexpr int SUM_THREADS = 256;
+template <typename T, int V>
+__global__ void __launch_bounds__(SUM_THREADS) column_sum_kernel(const T *x, int64_t rows, int64_t cols, int64_t ld, int64_t rows_per_cta, float *partial) {
+    __shared__ float red[SUM_THREADS / 32][32 * V];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int WARPS = SUM_THREADS / 32, AHEAD = 4;
+    const int64_t c = ((int64_t)blockIdx.x * 32 + lane) * V, r0 = (int64_t)blockIdx.y * rows_per_cta;
+    const int64_t r1 = r0 + rows_per_cta < rows ? r0 + rows_per_cta : rows;
+    float acc[V];
+#pragma unroll
+    for (int u = 0; u < V; u++) acc[u] = 0.f;
+    if (c < cols) {  // V > 1: cols is a multiple of V
+        int64_t r = r0 + warp;
+        for (; r + (AHEAD - 1) * WARPS < r1; r += AHEAD * WARPS) {
+            __align__(16) T v[AHEAD][V];
+#pragma unroll
+            for (int a = 0; a < AHEAD; a++) {
+                const T *src = x + (r + a * WARPS) * ld + c;
+                if constexpr (V > 1) *reinterpret_cast<uint4 *>(v[a]) = __ldg(reinterpret_cast<const uint4 *>(src));
+                else v[a][0] = __ldg(src);
+            }
+#pragma unroll
+            for (int a = 0; a < AHEAD; a++)
+#pragma unroll
+                for (int u = 0; u < V; u++) acc[u] += DT<T>::to_f32(v[a][u]);
+        }
+        for (; r < r1; r += WARPS)
+#pragma unroll
+            for (int u = 0; u < V; u++) acc[u] += DT<T>::to_f32(__ldg(x + r * ld + c + u));
+    }
+#pragma unroll
+    for (int u = 0; u < V; u++) red[warp][lane * V + u] = acc[u];
+    __syncthreads();
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    for (int i = threadIdx.x; i < 32 * V; i += SUM_THREADS) {
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < WARPS; w++) sum += red[w][i];
+        const int64_t col = (int64_t)blockIdx.x * 32 * V + i;
+        if (col < cols) partial[(int64_t)blockIdx.y * cols + col] = sum;
+    }
+}
+template <typename T>
+__global__ void __launch_bounds__(SUM_THREADS) column_sum_finish_kernel(const float *partial, int ranges, int64_t cols, T *out) {
+    __shared__ float red[SUM_THREADS / 32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t c = (int64_t)blockIdx.x * 32 + lane;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float sum = 0.f;
+    if (c < cols) {
+#pragma unroll 4
+        for (int i = warp; i < ranges; i += SUM_THREADS / 32) sum += partial[i * cols + c];
+    }
+    red[warp][lane] = sum;
+    __syncthreads();
+    if (warp != 0 || c >= cols) return;
+    sum = red[0][lane];
+#pragma unroll
+    for (int w = 1; w < SUM_THREADS / 32; w++) sum += red[w][lane];
+    out[c] = DT<T>::from_f32(sum);
+}
+
+// Row ranges: two waves of CTAs at most, at least 32 rows each
+static int column_sum_ranges(int64_t rows, int64_t cols, int64_t per_cta) {
+    const int64_t groups = (cols + per_cta - 1) / per_cta, want = (148 * 8 + groups - 1) / groups, most = (rows + 31) / 32;
+    const int64_t r = want < most ? want : most;
+    return (int)(r < 1 ? 1 : r > 256 ? 256 : r);
+}
+
+extern "C" size_t nmg_column_sum_workspace_bytes(int64_t rows, int64_t cols) {
+    if (rows < 1 || cols < 1) return 0;
+    return (size_t)column_sum_ranges(rows, cols, 256) * (size_t)cols * 4 + 256;  // the widest column groups have the most ranges
+}
+
+extern "C" int nmg_column_sum(const void *x, int64_t rows, int64_t cols, int64_t ld, int dtype, void *out, void *workspace, size_t workspace_bytes, void *stream) {
+    int rc;
+    if ((rc = check_dtype(dtype))) return rc;
+    if (!x || !out) NMG_FAIL(NMG_ERR_INVALID, "x and out must be non-NULL");
+    if (rows < 1 || cols < 1 || ld < cols) NMG_FAIL(NMG_ERR_INVALID, "bad shape (%lld x %lld, ld %lld)", (long long)rows, (long long)cols, (long long)ld);
+    const size_t es = dtype_size(dtype);
+    const int V = 16 / (int)es;
+    const bool vec = cols % V == 0 && ld % V == 0 && (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    const int64_t per_cta = vec ? 32 * V : 32, groups = (cols + per_cta - 1) / per_cta;
+    const int ranges = column_sum_ranges(rows, cols, per_cta);
+    if (!workspace || workspace_bytes < (size_t)ranges * cols * 4 + 256)
+        NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required, got %zu", (size_t)ranges * cols * 4 + 256, workspace_bytes);
+    float *partial = reinterpret_cast<float *>(((uintptr_t)workspace + 255) & ~(uintptr_t)255);
+    const int64_t rows_per_cta = (rows + ranges - 1) / ranges;
+    cudaStream_t st = (cudaStream_t)stream;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)((cols + 31) / 32));
+    cfg.blockDim = dim3(SUM_THREADS);
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const dim3 grid((unsigned)groups, (unsigned)ranges);
+    NMG_DISPATCH_DTYPE(dtype, T, {
+        if (vec) column_sum_kernel<T, 16 / (int)sizeof(T)><<<grid, SUM_THREADS, 0, st>>>(static_cast<const T *>(x), rows, cols, ld, rows_per_cta, partial);
+        else column_sum_kernel<T, 1><<<grid, SUM_THREADS, 0, st>>>(static_cast<const T *>(x), rows, cols, ld, rows_per_cta, partial);
+        NMG_CUDA(cudaGetLastError());
+        NMG_CUDA(cudaLaunchKernelEx(&cfg, column_sum_finish_kernel<T>, static_cast<const float *>(partial), ranges, cols, static_cast<T *>(out)));
+    });
+    return NMG_OK;
+}

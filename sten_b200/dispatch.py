@@ -902,7 +902,8 @@ class SparseOperatorDispatcher(torch.autograd.Function):
                 grads.append(None)
                 continue
             g = impl(s, g)
-            if isinstance(g, SparseTensorWrapper):  # gradient wrapper must look like the input's dummy
+            # gradient wrapper must look like the input's dummy, as one that an implementation has just made for it does
+            if isinstance(g, SparseTensorWrapper) and not g.__dict__.pop("made_as_gradient", False):
                 g = SparseTensorWrapper(g._wrapped_tensor_container, torch.is_grad_enabled() and g.requires_grad, g.grad_fmt, dummy_shape=shape, shared_dummy=True)
             grads.append(g)
         return (None, *grads)

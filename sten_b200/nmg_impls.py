@@ -127,7 +127,7 @@ def _linear_bwd(ctx, grad_outputs, input_sparsifiers):
         # dense weight gradient (training of nmg weights is outside the inference hot path): plain GEMM
         dw = dy2d.t().mm(x if x.dim() == 2 else x.reshape(-1, x.shape[-1]))
     if has_bias and needs[2]:
-        db = dy2d.sum(dim=0)
+        db = nat.host().column_sum(dy2d)
     return (dx, dw, db) if has_bias else (dx, dw)
 
 
@@ -140,6 +140,7 @@ def _linear_bwd_weight_layout(ctx, grad_outputs, input_sparsifiers):
         weight = ctx.saved_tensors[1]
         masked = weight.wrapped_tensor.clone_layout(grads[1])
         grads[1] = sten.SparseTensorWrapper([masked], False, sten._DEFAULT_GRAD_FMT(), shared_dummy=True)
+        grads[1].made_as_gradient = True
     return tuple(grads)
 
 

@@ -44,3 +44,13 @@ def test_gather_at_tile_edges(n, m, g, B, M, K, off, dtype):
     mask = ops.densify(torch.ones_like(val), idx, B, M, K, n, m, g)
     assert torch.equal(ops.densify(got, idx, B, M, K, n, m, g), torch.where(mask != 0, other, torch.zeros_like(other)))
     assert torch.equal(ops.gather_layout(w, idx, n, m, g), val)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-6), (torch.bfloat16, 4e-3), (torch.float16, 5e-4)])
+@pytest.mark.parametrize("rows,cols,off", [(1, 1, 0), (31, 8, 0), (33, 257, 0), (4096, 1000, 0), (1000, 4096, 3), (5000, 40, 0), (70000, 16, 8)])
+def test_column_sums(rows, cols, off, dtype, tol):
+    from sten_b200 import _native as nat
+    x = seeded_normal((rows, cols + off), 3).to(dtype).to(cuda())[:, off:]
+    got, want = nat.host().column_sum(x), x.double().sum(0)
+    assert got.dtype == dtype and float((got.double() - want).norm() / want.norm()) <= tol
+    assert torch.equal(nat.host().column_sum(x), got)

@@ -520,19 +520,22 @@ __global__ void __launch_bounds__(256, 4) sparsify_nm_kernel(SparsifyParams prm)
 //   zeros     scores of zero are placed by the closed form of sparsify_zero_phase.
 // Entries are 64-bit keys, score above column + 1: one comparison is the format's order.  The tile is staged in shared memory
 // (16-byte asynchronous copies where the alignment allows).  A tile's slab is 32 bytes more than a multiple of 128, so that
-// the tiles of a warp use different banks.
-// 4096 x 4096, before (a warp per tile) and now: 2:4 fp32 187 -> 127 us, bf16 184 -> 111, 1:4 fp32 173 -> 98, 1:8 fp32 93 -> 80
-// (there all 32 lanes), 1:8 g = 4 fp16 195 -> 72.  Of the instructions ranking takes 40 %, the later rounds 25 %.  Tried and
-// slower: sorting a pattern per lane by a network (139), the tile left in global memory for more resident warps (129).
+// the tiles of a warp use different banks.  TWICE: the ranks of round 0 use the tile's own place and it is staged again (from
+// L2) for what follows; more warps are then resident, which pays where the grouped proposals are not small beside the tile.
+// 4096 x 4096, before (a warp per tile) and now: 2:4 fp32 187 -> 104 us, bf16 184 -> 89, 1:4 fp32 173 -> 84, 1:8 fp32 93 -> 68
+// (there all 32 lanes), 1:8 g = 4 fp16 195 -> 68.  Tried and slower: sorting a pattern per lane by a network (139 where this
+// took 121), the tile left in global memory for more resident warps (129).
 struct SparsifyLanes { int xs, x, in, list, prop, thr, sent, cnt, off, queue, qmask, zmask, words, total; };
-__host__ __device__ inline SparsifyLanes sparsify_lanes(int m, int cc, int C, int lanes, int es) {
+__host__ __device__ inline SparsifyLanes sparsify_lanes(int m, int cc, int C, int lanes, int es, bool twice) {
     SparsifyLanes l;
     const int quads = (cc + 3) / 4;
     int o = 0;
     l.words = ((quads + lanes - 1) / lanes * 4 + 31) / 32;  // one bit per column of a lane
     l.xs = quads * 4;                                       // row stride of the staged tile
-    l.x = o;      o += m * l.xs * es;                       // [m][xs] the tile
-    l.in = o = (o + 15) & ~15; o += (cc + 2 * C) * 8;       // round 0: proposals grouped by pattern, every group padded to 2
+    const int x_bytes = (m * l.xs * es + 15) & ~15, in_bytes = (cc + 2 * C) * 8;
+    l.x = o;                                                // [m][xs] the tile
+    l.in = twice ? o : o + x_bytes;                         // round 0: proposals grouped by pattern, every group padded to 2
+    o += twice ? (x_bytes > in_bytes ? x_bytes : in_bytes) : x_bytes + in_bytes;
     l.list = o = (o + 15) & ~15; o += l.xs * 8;             // [C][g] kept entries, descending (round 0: by column)
     l.prop = o;   o += lanes * 8;                           // later rounds: the proposal of every lane
     l.thr = o = (o + 15) & ~15; o += C * 4;                 // smallest score that a pattern may still keep
@@ -560,8 +563,8 @@ template <typename T> __device__ __forceinline__ void load_quad(const T *p, floa
     }
 }
 
-template <int N_, int M_, int L, typename T>
-__global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm) {
+template <int N_, int M_, int L, bool TWICE, typename T>
+__global__ void __launch_bounds__(128, 5) sparsify_lanes_kernel(SparsifyParams prm) {
     extern __shared__ __align__(16) char smem[];
     constexpr Order<N_, M_> ORD{};
     constexpr int C = Order<N_, M_>::C, TILES = 32 / L;
@@ -576,7 +579,7 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
     for (int i = threadIdx.x; i < C * N_; i += blockDim.x) ord[i] = (int8_t)ORD.v[(i / N_) * Order<N_, M_>::LD + (i % N_)];
     __syncthreads();
 
-    const SparsifyLanes lay = sparsify_lanes(M_, cc, C, L, (int)sizeof(T));
+    const SparsifyLanes lay = sparsify_lanes(M_, cc, C, L, (int)sizeof(T), TWICE);
     char *slab = smem + ORD_BYTES + (warp * TILES + sub) * lay.total;
     T *x = reinterpret_cast<T *>(slab + lay.x);
     uint64_t *in = reinterpret_cast<uint64_t *>(slab + lay.in), *list = reinterpret_cast<uint64_t *>(slab + lay.list);
@@ -606,15 +609,18 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
         const int cols_ok = (int)(prm.K - col0 < cc ? prm.K - col0 : cc);
         auto global_at = [&](int r, int c) -> T { return (r < rows_ok && c < cols_ok) ? __ldg(src + r * prm.ld + c) : DT<T>::from_f32(0.f); };
         // ---- the tile
-        if (rows_ok == M_ && cols_ok == cc && (cc % V) == 0 && (prm.ld % V) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
+        auto stage = [&]() {
+            if (rows_ok == M_ && cols_ok == cc && (cc % V) == 0 && (prm.ld % V) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
 #pragma unroll
-            for (int r = 0; r < M_; r++)
-                for (int v = sl * V; v < cc; v += L * V) cp_async_16(x + r * xs + v, src + r * prm.ld + v);
-            cp_async_commit();
-        } else {
-            for (int r = 0; r < M_; r++)
-                for (int c = sl; c < xs; c += L) x[r * xs + c] = global_at(r, c);
-        }
+                for (int r = 0; r < M_; r++)
+                    for (int v = sl * V; v < cc; v += L * V) cp_async_16(x + r * xs + v, src + r * prm.ld + v);
+                cp_async_commit();
+            } else {
+                for (int r = 0; r < M_; r++)
+                    for (int c = sl; c < xs; c += L) x[r * xs + c] = global_at(r, c);
+            }
+        };
+        stage();
         for (int p = sl; p < C; p += L) cnt[p] = 0;
         for (int w = 0; w < words; w++) my_z[w] = 0;
         if (sl == 0) *tail = 0;
@@ -690,12 +696,14 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
             if (key.y != 0) place(key.y, rank1);  // zero: padding
         }
         __syncwarp();
+        if (TWICE) stage();
         for (int p = sl; p < C; p += L) {
             const int n = min(cnt[p], g);
             cnt[p] = n;
             thr[p] = n == g ? (uint32_t)(list[p * g + g - 1] >> 32) : 1u;
             sent[p] = 0;
         }
+        if (TWICE) cp_async_wait<0>();
         __syncwarp();
 
         // ---- later rounds.  Every round with a proposal makes at least one (column, pattern) proposal that was never made
@@ -845,10 +853,10 @@ __global__ void __launch_bounds__(128) sparsify_lanes_kernel(SparsifyParams prm)
 }
 
 // Launch with L lanes per tile; *served = false when fewer than `min_warps` warps would be resident per SM.
-template <int N_, int M_, int L> static int sparsify_lanes_launch(int dtype, const SparsifyParams &p, int min_warps, bool *served, cudaStream_t st) {
+template <int N_, int M_, int L, bool TWICE> static int sparsify_lanes_launch(int dtype, const SparsifyParams &p, int min_warps, bool *served, cudaStream_t st) {
     const int es = (int)dtype_size(dtype);
     constexpr int C = Order<N_, M_>::C, ORD_BYTES = (C * N_ + 15) & ~15, TILES = 32 / L;
-    const size_t per_warp = (size_t)TILES * sparsify_lanes(M_, p.cc, C, L, es).total;
+    const size_t per_warp = (size_t)TILES * sparsify_lanes(M_, p.cc, C, L, es, TWICE).total;
     int warps = 0, resident = 0;  // whatever keeps the most warps resident; on a tie the smaller CTA
     for (int w = 1; w <= 4; w++) {
         const size_t cta = ORD_BYTES + w * per_warp;
@@ -862,8 +870,8 @@ template <int N_, int M_, int L> static int sparsify_lanes_launch(int dtype, con
     const size_t smem = ORD_BYTES + warps * per_warp;
     const int64_t ctas = (p.tiles + warps * TILES - 1) / (warps * TILES), cap = (int64_t)sm_count() * 64;
     NMG_DISPATCH_DTYPE(dtype, T, {
-        NMG_ALLOW_SMEM(smem, sparsify_lanes_kernel<N_, M_, L, T>);
-        sparsify_lanes_kernel<N_, M_, L, T><<<(unsigned)(ctas < cap ? ctas : cap), warps * 32, smem, st>>>(p);
+        NMG_ALLOW_SMEM(smem, sparsify_lanes_kernel<N_, M_, L, TWICE, T>);
+        sparsify_lanes_kernel<N_, M_, L, TWICE, T><<<(unsigned)(ctas < cap ? ctas : cap), warps * 32, smem, st>>>(p);
     });
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;
@@ -1037,14 +1045,18 @@ extern "C" int nmg_sparsify(const void *dense, int64_t batch, int64_t M, int64_t
     p.nb = geo.nb; p.nc = geo.nc; p.tiles = batch * geo.nb * geo.nc;
     p.n = n; p.m = m; p.g = g; p.C = geo.C; p.cc = geo.cc;
     cudaStream_t st = (cudaStream_t)stream;
+    // whole: tiles are staged by 16-byte copies, cheap enough to be made twice
+    const int V = 16 / (int)dtype_size(dtype);
+    const bool whole = geo.cc % V == 0 && ld_dense % V == 0 && (batch == 1 || batch_stride % V == 0) && (reinterpret_cast<uintptr_t>(dense) & 15) == 0;
     // Few patterns: several tiles per warp.  Eight lanes per tile when that leaves at least twelve resident warps to hide the
     // latency of the shared memory, else a warp per tile down to four; larger tiles, and 16 or 28 patterns (whose later rounds
     // keep 32 lanes busy: 1:16 68 us against 74 to 102, 2:8 152 against 158), go to the kernel that does not stage the tile.
 #define NMG_SPARSIFY_CASE(N_, M_)                                                                     \
     if (n == N_ && m == M_) {                                                                         \
         bool served = false;                                                                          \
-        if ((rc = sparsify_lanes_launch<N_, M_, 8>(dtype, p, 12, &served, st)) || served) return rc;  \
-        if ((rc = sparsify_lanes_launch<N_, M_, 32>(dtype, p, 4, &served, st)) || served) return rc;  \
+        if (M_ == 4 && whole && ((rc = sparsify_lanes_launch<N_, M_, 8, M_ == 4>(dtype, p, 12, &served, st)) || served)) return rc; \
+        if ((rc = sparsify_lanes_launch<N_, M_, 8, false>(dtype, p, 12, &served, st)) || served) return rc;  \
+        if ((rc = sparsify_lanes_launch<N_, M_, 32, false>(dtype, p, 4, &served, st)) || served) return rc;  \
     }
     NMG_SPARSIFY_CASE(1, 4)
     NMG_SPARSIFY_CASE(2, 4)

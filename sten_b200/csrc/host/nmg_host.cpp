@@ -12,6 +12,7 @@
 #include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <pybind11/pybind11.h>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -26,6 +27,13 @@ PyObject *g_error_class = nullptr;  // sten_b200._native.NmgError(status, messag
 PyObject *g_s_val, *g_s_idx, *g_s_packed, *g_s_packed_sp24, *g_zero;
 
 struct PyRaised {};  // a Python exception is set
+
+struct Ref {  // owned reference
+    PyObject *p;
+    explicit Ref(PyObject *o) : p(o) {}
+    Ref(const Ref &) = delete;
+    ~Ref() { Py_XDECREF(p); }
+};
 
 [[noreturn]] void py_raise(PyObject *type, const std::string &msg) {
     PyErr_SetString(type, msg.c_str());
@@ -515,20 +523,10 @@ PyObject *handle_linear_t(PyObject *self, PyObject *const *a, Py_ssize_t nargs) 
     NMG_PY_END
 }
 
-// column_sum(dy): [..., M] -> [M], the bias gradient
-PyObject *py_column_sum(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
-    NMG_PY_BEGIN(1)
-    const at::Tensor &x0 = tensor_arg(a[0]);
-    const c10::Device dev = device_of({&x0});
-    const int code = dtype_code(x0);
-    const c10::cuda::CUDAGuard guard(dev);
-    if (x0.dim() < 1) py_raise(PyExc_ValueError, "expected at least one dimension");
-    const Rows x = rows_of(x0, x0.size(-1));
-    const at::Tensor out = new_empty({x.cols}, x0.scalar_type());
-    if (x.rows < 1 || x.cols < 1) {
-        out.zero_();
-        return THPVariable_Wrap(out);
-    }
+// [rows][ld] -> [cols], the bias gradient
+at::Tensor column_sums(const Rows &x, int code, c10::Device dev) {
+    const at::Tensor out = new_empty({x.cols}, x.t.scalar_type());
+    if (x.rows < 1 || x.cols < 1) return out.zero_();
     const size_t nbytes = nmg_column_sum_workspace_bytes(x.rows, x.cols);
     const at::Tensor ws = new_empty({(int64_t)nbytes}, at::kByte);
     void *st = stream_of(dev);
@@ -536,7 +534,53 @@ PyObject *py_column_sum(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     const int rc = nmg_column_sum(x.t.const_data_ptr(), x.rows, x.cols, x.ld, code, out.mutable_data_ptr(), ws.mutable_data_ptr(), nbytes, st);
     PyEval_RestoreThread(save);
     check(rc);
-    return THPVariable_Wrap(out);
+    return out;
+}
+
+// column_sum(dy): [..., M] -> [M]
+PyObject *py_column_sum(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(1)
+    const at::Tensor &x = tensor_arg(a[0]);
+    const c10::Device dev = device_of({&x});
+    const int code = dtype_code(x);
+    const c10::cuda::CUDAGuard guard(dev);
+    if (x.dim() < 1) py_raise(PyExc_ValueError, "expected at least one dimension");
+    return THPVariable_Wrap(column_sums(rows_of(x, x.size(-1)), code, dev));
+    NMG_PY_END
+}
+
+// linear_grads(gnm, x, dy, sp24_min_tokens, needs, in_layout) -> (dx, dw, db), None where not needed (needs: bits 0, 1, 2).
+// dw is the plain product dy^T x, or with in_layout its values at the weight's kept positions.
+PyObject *handle_linear_grads(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(6)
+    Handle *h = reinterpret_cast<Handle *>(self);
+    const Geo &geo = h->geo;
+    const at::Tensor val = attr_tensor(a[0], g_s_val), idx = attr_tensor(a[0], g_s_idx);
+    const at::Tensor &x = tensor_arg(a[1]), &dy0 = tensor_arg(a[2]);
+    const int64_t needs = int_arg(a[4]);
+    const bool in_layout = int_arg(a[5]) != 0;
+    const c10::Device dev = device_of({&val, &idx, &x, &dy0});
+    const int code = dtype_code(val);
+    if (dy0.scalar_type() != val.scalar_type())
+        py_raise(PyExc_TypeError, std::string("gradient dtype must match the weight dtype ") + c10::toString(val.scalar_type()));
+    const c10::cuda::CUDAGuard guard(dev);
+    const Rows dy = rows_of(dy0, geo.M);
+    PyObject *r = PyTuple_New(3);
+    for (int i = 0; i < 3; i++) PyTuple_SET_ITEM(r, i, Py_NewRef(Py_None));
+    Ref owner(r);
+    if (needs & 1) PyTuple_SetItem(r, 0, THPVariable_Wrap(input_gradient(h, a[0], val, idx, dy0, dy, int_arg(a[3]), code, dev)));
+    if (needs & 2) {
+        // dense weight gradient (training of nmg weights is outside the inference hot path): plain GEMM
+        const at::Tensor dy2 = dy0.dim() == 2 ? dy0 : dy0.reshape({-1, geo.M}), x2 = x.dim() == 2 ? x : x.reshape({-1, geo.K});
+        at::Tensor dw;
+        {
+            pybind11::gil_scoped_release nogil;
+            dw = at::mm(dy2.t(), x2);
+        }
+        PyTuple_SetItem(r, 1, in_layout ? gather_values(Dense3{dw, 1, geo.M, geo.K, geo.K, geo.M * geo.K}, idx, geo.n, geo.m, geo.g, code, dev) : THPVariable_Wrap(dw));
+    }
+    if (needs & 4) PyTuple_SetItem(r, 2, THPVariable_Wrap(column_sums(dy, code, dev)));
+    return Py_NewRef(r);
     NMG_PY_END
 }
 
@@ -547,13 +591,6 @@ PyObject *py_column_sum(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
 PyObject *g_wrapper_type = nullptr, *g_profiling = nullptr;  // SparseTensorWrapper, [bool]
 PyObject *g_s_sparsified_ops, *g_s_sparse_op, *g_s_disp_state, *g_s_fast, *g_s_native, *g_s_repeat, *g_s_container, *g_s_native_handle, *g_s_nm_strides,
     *g_s_kernel, *g_s_expanded;
-
-struct Ref {  // owned reference
-    PyObject *p;
-    explicit Ref(PyObject *o) : p(o) {}
-    Ref(const Ref &) = delete;
-    ~Ref() { Py_XDECREF(p); }
-};
 
 // set_dispatch(wrapper_type, profiling_switch)
 PyObject *py_set_dispatch(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
@@ -663,6 +700,7 @@ PyMethodDef handle_methods[] = {
     NMG_METHOD("linear", handle_linear),
     NMG_METHOD("mm", handle_mm),
     NMG_METHOD("linear_t", handle_linear_t),
+    NMG_METHOD("linear_grads", handle_linear_grads),
     {nullptr, nullptr, 0, nullptr},
 };
 PyTypeObject handle_type = {PyVarObject_HEAD_INIT(nullptr, 0)};

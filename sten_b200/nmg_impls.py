@@ -111,37 +111,28 @@ sparse_torch_nn_functional_linear = sten.register_fwd_op_impl(
 sten.register_fwd_op_impl(operator=torch.nn.functional.linear, inp=(torch.Tensor, GroupedNMTensor), out=_LIN_OUT)(_linear_fwd)
 
 
-def _linear_bwd(ctx, grad_outputs, input_sparsifiers):
+def _linear_grads(ctx, grad_outputs, in_layout):
     saved = ctx.saved_tensors
-    x, weight = saved[0], saved[1]
-    has_bias = len(saved) == 3
-    [dy] = grad_outputs
-    needs = tuple(ctx.needs_input_grad[1:]) + (False,) * 3
-    gnm, h = _native_weight(weight)
-    dx = dw = db = None
-    if needs[0]:
-        dx = h.linear_t(gnm, dy, ops.SP24_MIN_TOKENS)
-    if needs[1] or needs[2]:
-        dy2d = dy if dy.dim() == 2 else dy.reshape(-1, dy.shape[-1])
-    if needs[1]:
-        # dense weight gradient (training of nmg weights is outside the inference hot path): plain GEMM
-        dw = dy2d.t().mm(x if x.dim() == 2 else x.reshape(-1, x.shape[-1]))
-    if has_bias and needs[2]:
-        db = nat.host().column_sum(dy2d)
-    return (dx, dw, db) if has_bias else (dx, dw)
+    needs = ctx.needs_input_grad
+    gnm, h = _native_weight(saved[1])
+    mask = (1 if needs[1] else 0) | (2 if needs[2] else 0) | (4 if len(saved) == 3 and needs[3] else 0)
+    return len(saved), gnm, h.linear_grads(gnm, saved[0], grad_outputs[0], ops.SP24_MIN_TOKENS, mask, in_layout)
+
+
+def _linear_bwd(ctx, grad_outputs, input_sparsifiers):
+    count, _, grads = _linear_grads(ctx, grad_outputs, 0)
+    return grads[:count]
 
 
 def _linear_bwd_weight_layout(ctx, grad_outputs, input_sparsifiers):
     """Same products as ``_linear_bwd``; dW leaves as a GroupedNMTensor in the weight's layout.  dY^T X runs on the tensor
     cores at the dense rate into a transient buffer (a sampled product on the FP32 pipes would be an order of magnitude
     slower on this hardware) and one gather pass keeps the layout's positions."""
-    grads = list(_linear_bwd(ctx, grad_outputs, input_sparsifiers))
-    if grads[1] is not None:
-        weight = ctx.saved_tensors[1]
-        masked = weight.wrapped_tensor.clone_layout(grads[1])
-        grads[1] = sten.SparseTensorWrapper([masked], False, sten._DEFAULT_GRAD_FMT(), shared_dummy=True)
-        grads[1].made_as_gradient = True
-    return tuple(grads)
+    count, gnm, (dx, dw, db) = _linear_grads(ctx, grad_outputs, 1)
+    if dw is not None:
+        dw = sten.SparseTensorWrapper([GroupedNMTensor(dw, gnm.idx, gnm.nm_strides)], False, sten._DEFAULT_GRAD_FMT(), shared_dummy=True)
+        dw.made_as_gradient = True
+    return (dx, dw, db)[:count]
 
 
 _DENSE_GRAD = (sten.KeepAll, torch.Tensor)

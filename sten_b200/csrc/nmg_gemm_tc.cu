@@ -956,9 +956,10 @@ int tc_expand_plain(const Geo &geo, int dtype, const void *val, const int16_t *i
 }
 
 // out = dense[rows][round_up(red, 8)] (16-bit, or three bf16 planes for fp32) x activations (16-bit, or the planes of the split).
-// CTA pairs (256 rows per tile) unless a 16-bit output has one tile of 128 features only.
+// CTA pairs (256 rows per tile) unless a 16-bit output has one tile of 128 features only.  source: expand this weight into `dense`
+// first, right before the matmul, whose prologue overlaps the expansion's end only when nothing is queued between the two.
 int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const DenseAct &act, int64_t tokens, const void *bias,
-                  void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major, cudaStream_t st, const Epilogue &epi) {
+                  void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major, cudaStream_t st, const Epilogue &epi, const DenseSource *source) {
     if (n_outs < 1 || n_outs > GEMM_MAX_OUTS) NMG_FAIL(NMG_ERR_INVALID, "between 1 and %d output buffers, got %d", GEMM_MAX_OUTS, n_outs);
     const int64_t ld = dense_ld(red);
     const int planes = dtype == NMG_F32 ? 3 : 1;
@@ -1029,6 +1030,7 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
     gp.status = status;
     gp.act = epi.act; gp.residual = epi.residual; gp.ld_res = epi.ld_res;
     gp.res_vec = (epi.residual && (epi.ld_res * osz) % 16 == 0 && (reinterpret_cast<uintptr_t>(epi.residual) & 15) == 0) ? 1 : 0;
+    if (source && (rc = tc_dense_expand(source->geo, dtype, source->transposed, source->val, source->idx, const_cast<char *>(dense), st))) return rc;
     if (dtype == NMG_F32) return gemm_launch<float, true>(gp, maps, st);
     if (dtype == NMG_F16) return pair ? gemm_launch<__half, true>(gp, maps, st) : gemm_launch<__half, false>(gp, maps, st);
     return pair ? gemm_launch<__nv_bfloat16, true>(gp, maps, st) : gemm_launch<__nv_bfloat16, false>(gp, maps, st);
@@ -1042,9 +1044,8 @@ int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val,
     const size_t need = tc_dense_workspace_bytes(geo, dtype, transposed);
     if (!ws || ws_bytes < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the expanded weight, got %zu", need, ws_bytes);
     char *dense = reinterpret_cast<char *>(((uintptr_t)ws + 255) & ~(uintptr_t)255);
-    int rc;
-    if ((rc = tc_dense_expand(geo, dtype, transposed, val, idx, dense, st))) return rc;
-    return tc_dense_gemm(rows, red, dtype, dense, act, tokens, bias, outs, n_outs, mc_out, ld_out, out_token_major, st, epi);
+    const DenseSource source{geo, transposed, val, idx};
+    return tc_dense_gemm(rows, red, dtype, dense, act, tokens, bias, outs, n_outs, mc_out, ld_out, out_token_major, st, epi, &source);
 }
 
 }  // namespace nmg

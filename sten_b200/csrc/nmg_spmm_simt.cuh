@@ -53,6 +53,7 @@ struct Epilogue {
 };
 int launch_epilogue(int dtype, void *out, int64_t rows, int64_t cols, int64_t ld_out, const Epilogue &epi, cudaStream_t st);
 // Activations of the two-pass variant: [tokens][ld], reduction contiguous, 16-byte aligned rows; three bf16 planes for fp32.
+struct DenseSource { const Geo &geo; bool transposed; const void *val; const int16_t *idx; };  // the compressed weight
 struct DenseAct { const void *base; int64_t ld, plane_elems; };
 
 bool tc_supported(const Geo &geo, int dtype);        // fused kernel
@@ -83,7 +84,8 @@ int tc_sp_matmul_t(const Geo &geo, int dtype, const void *sp_copy, const void *d
 // trades the format's memory saving for skipping the expansion pass of every call).
 int tc_dense_expand(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, char *dense, cudaStream_t st);
 int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const DenseAct &act, int64_t tokens, const void *bias,
-                  void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major, cudaStream_t st, const Epilogue &epi);
+                  void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major, cudaStream_t st, const Epilogue &epi,
+                  const DenseSource *source = nullptr);
 
 // ---- specialised forward kernel: parameters, shared-memory plan, per-(n, m) launchers
 struct FwdParams {

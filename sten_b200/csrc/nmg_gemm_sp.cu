@@ -486,10 +486,10 @@ int tc_sp_matmul_t(const Geo &geo, int dtype, const void *sp_copy, const void *d
     gp.tiles_t = (int)((tokens + TC_BN - 1) / TC_BN);
     gp.band = TC_BAND_PAIR;
     {
-        // many waves over a long reduction: keep the producers in step; the counter is zeroed in stream order
+        // many waves over a long reduction whose operands L2 does not hold: keep the producers in step; the counter is zeroed in stream order
         int sms = 148, rc_sms;
         if ((rc_sms = device_sms(&sms))) return rc_sms;
-        if ((int64_t)gp.tiles_f * gp.tiles_t >= 3 * (int64_t)(sms / 2) && geo.M >= 4096) {
+        if ((int64_t)gp.tiles_f * gp.tiles_t >= 3 * (int64_t)(sms / 2) && geo.M >= 4096 && (geo.K + 2 * tokens) * geo.M > (96ll << 20)) {
             if ((rc = get_wave_counter(&gp.wave_ctr))) return rc;
             NMG_CUDA(cudaMemsetAsync(gp.wave_ctr, 0, sizeof(unsigned), st));
         }

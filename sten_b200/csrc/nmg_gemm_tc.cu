@@ -1022,8 +1022,9 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
     gp.tiles_t = (int)((tokens + bn - 1) / bn);
     gp.bn = bn;
     gp.band = pair ? TC_BAND_PAIR : TC_BAND;
-    // many waves over a long reduction: keep the producers in step (see the kernel); the counter is zeroed in stream order
-    if ((int64_t)gp.tiles_f * gp.tiles_t >= 3 * units && red >= 4096) {
+    // many waves over a long reduction: keep the producers in step (see the kernel); the counter is zeroed in stream order.
+    // Operands that stay in L2 beside the output need no step keeping: 4096 x 4096, 4096 tokens 108.6 -> 107.4 us without.
+    if ((int64_t)gp.tiles_f * gp.tiles_t >= 3 * units && red >= 4096 && (row_ext + col_ext) * red * 2 * planes > (96ll << 20)) {
         if ((rc = get_wave_counter(&gp.wave_ctr))) return rc;
         NMG_CUDA(cudaMemsetAsync(gp.wave_ctr, 0, sizeof(unsigned), st));
     }

@@ -131,7 +131,7 @@ static int spmm_impl(const void *val, const int16_t *idx, const void *packed, in
             const size_t need = (size_t)tokens * (size_t)ld_x * 2 + 512;
             if (!ws || left < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the re-laid activation, got %zu", need, left);
             char *xt = align256(ws);
-            if ((rc = tm ? launch_pad_rows(act, tokens, K, ld_act, xt, ld_x, st) : launch_transpose(act, dtype, K, tokens, ld_act, xt, ld_x, st))) return rc;
+            if ((rc = tm ? launch_pad_rows(act, tokens, K, ld_act, xt, ld_x, st) : launch_transpose(act, K, tokens, ld_act, xt, ld_x, st))) return rc;
             act = xt;
             ld_act = ld_x;
             char *rest = xt + (size_t)tokens * ld_x * 2;

@@ -46,13 +46,12 @@ int launch_transpose_to_f32(const void *src, int dtype, int64_t rows, int64_t co
     return NMG_OK;
 }
 
-// Same-dtype transpose: src[rows][ld_src] -> dst[cols][ld_dst], 64 x 64 tiles through shared memory.  Both sides move
-// 128 bytes (fp32: 256) per warp instruction: a thread reads two neighbouring elements of a source row and writes two
+// Transpose of 16-bit elements: src[rows][ld_src] -> dst[cols][ld_dst], 64 x 64 tiles through shared memory.  Both sides move
+// 128 bytes per warp instruction: a thread reads two neighbouring elements of a source row and writes two
 // neighbouring elements of a destination row.  Columns of dst beyond `rows` (up to ld_dst) are zero.
-template <typename T>
-__global__ void __launch_bounds__(256) transpose_kernel(const T *__restrict__ src, int64_t rows, int64_t cols, int64_t ld_src,
-                                                        T *__restrict__ dst, int64_t ld_dst) {
-    __shared__ T tile[64][66];
+__global__ void __launch_bounds__(256) transpose_kernel(const uint16_t *__restrict__ src, int64_t rows, int64_t cols, int64_t ld_src,
+                                                        uint16_t *__restrict__ dst, int64_t ld_dst) {
+    __shared__ uint16_t tile[64][66];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the matmul's set-up may overlap this pass
     const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
     const int64_t c0 = (int64_t)blockIdx.x * 64, r0 = (int64_t)blockIdx.y * 64;
@@ -61,7 +60,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const T *__restrict__ sr
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             const int64_t c = c0 + 2 * tx + h;
-            tile[i][2 * tx + h] = (r < rows && c < cols) ? src[r * ld_src + c] : DT<T>::from_f32(0.f);
+            tile[i][2 * tx + h] = (r < rows && c < cols) ? src[r * ld_src + c] : (uint16_t)0;
         }
     }
     __syncthreads();
@@ -76,12 +75,12 @@ __global__ void __launch_bounds__(256) transpose_kernel(const T *__restrict__ sr
     }
 }
 
-int launch_transpose(const void *src, int dtype, int64_t rows, int64_t cols, int64_t ld_src, void *dst, int64_t ld_dst, cudaStream_t st) {
+int launch_transpose(const void *src, int64_t rows, int64_t cols, int64_t ld_src, void *dst, int64_t ld_dst, cudaStream_t st) {
     dim3 block(32, 8);
     const int64_t gy = (ld_dst + 63) / 64;
     if (gy > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "reduction axis too long for the transpose pre-pass");
     dim3 grid((unsigned)((cols + 63) / 64), (unsigned)gy);
-    NMG_DISPATCH_DTYPE(dtype, T, (transpose_kernel<T><<<grid, block, 0, st>>>(static_cast<const T *>(src), rows, cols, ld_src, static_cast<T *>(dst), ld_dst)));
+    transpose_kernel<<<grid, block, 0, st>>>(static_cast<const uint16_t *>(src), rows, cols, ld_src, static_cast<uint16_t *>(dst), ld_dst);
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;
 }

@@ -16,6 +16,7 @@
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -368,21 +369,76 @@ PyObject *py_set_error_class(PyObject *, PyObject *cls) {
     Py_RETURN_NONE;
 }
 
-// ------------------------------------------------------------------------------------------------ Handle
-// What the host keeps of one 2-D weight between calls: its geometry and, for the kernels that read them, the derived copies
-// together with the identity and version of the (val, idx) they were derived from.  The copies themselves belong to the
-// GroupedNMTensor (packed(), packed_sp24()), which is asked again as soon as either tensor has been replaced or written.
-struct Derived {
-    const void *val = nullptr, *idx = nullptr;
-    uint32_t val_version = 0, idx_version = 0;
-    bool valid = false;
-    at::Tensor copy;  // undefined: there is none for this weight
+// ------------------------------------------------------------------------------------------------ Kept
+// One of the tensors a copy was derived from.  An address says nothing by itself: a weight that was replaced twice between two
+// calls finds its third tensor where its first one was, at version 0 again.  The weak references keep both objects' addresses
+// from being given to others (they do not keep the memory of the values); the storage counts too, since `t.data = other` leaves
+// the tensor and its version as they were.
+struct Source {
+    c10::weak_intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl> tensor;
+    c10::weak_intrusive_ptr<c10::StorageImpl> storage;
+    const void *data;
+    uint32_t version;
+    at::ScalarType type;
+    explicit Source(const at::Tensor &t)
+        : tensor(t.getIntrusivePtr()), storage(t.storage().getWeakStorageImpl()), data(t.const_data_ptr()), version(t._version()), type(t.scalar_type()) {}
+    bool is(const at::Tensor &t) const {
+        return tensor._unsafe_get_target() == t.unsafeGetTensorImpl() && storage._unsafe_get_target() == t.storage().unsafeGetStorageImpl() &&
+               data == t.const_data_ptr() && version == t._version() && type == t.scalar_type();
+    }
 };
+// A copy derived from (val, idx), valid while both are the same tensors at the same version.
+struct KeptCopy {
+    Source val, idx;
+    at::Tensor copy;  // undefined: there is none for this weight
+    KeptCopy(const at::Tensor &v, const at::Tensor &i) : val(v), idx(i) {}  // before the copy is made: a write meanwhile shows
+    bool from(const at::Tensor &v, const at::Tensor &i) const { return val.is(v) && idx.is(i); }
+};
+
+// Kept(val, idx), then put(copy): the same for the caches on the Python side.
+extern PyTypeObject kept_type;
+struct Kept {
+    PyObject_HEAD
+    KeptCopy *data;
+};
+PyObject *kept_new(PyTypeObject *type, PyObject *args, PyObject *) {
+    HANDLE_TH_ERRORS
+    try {
+        if (PyTuple_GET_SIZE(args) != 2) py_raise(PyExc_TypeError, "Kept(val, idx)");
+        std::unique_ptr<KeptCopy> data(new KeptCopy(tensor_arg(PyTuple_GET_ITEM(args, 0)), tensor_arg(PyTuple_GET_ITEM(args, 1))));
+        Kept *k = reinterpret_cast<Kept *>(type->tp_alloc(type, 0));
+        if (k) k->data = data.release();
+        return reinterpret_cast<PyObject *>(k);
+    } catch (const PyRaised &) { return nullptr; }
+    END_HANDLE_TH_ERRORS
+}
+void kept_dealloc(PyObject *self) {
+    delete reinterpret_cast<Kept *>(self)->data;
+    Py_TYPE(self)->tp_free(self);
+}
+// get(val, idx) -> the copy, or None when it was made from other tensors or other contents
+PyObject *kept_get(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(2)
+    const KeptCopy *k = reinterpret_cast<Kept *>(self)->data;
+    if (!k->copy.defined() || !k->from(tensor_arg(a[0]), tensor_arg(a[1]))) Py_RETURN_NONE;
+    return THPVariable_Wrap(k->copy);
+    NMG_PY_END
+}
+PyObject *kept_put(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(1)
+    reinterpret_cast<Kept *>(self)->data->copy = tensor_arg(a[0]);
+    Py_RETURN_NONE;
+    NMG_PY_END
+}
+
+// ------------------------------------------------------------------------------------------------ Handle
+// What the host keeps of one 2-D weight between calls: its geometry and, for the kernels that read them, the derived copies.
+// They are asked for at the GroupedNMTensor (packed(), packed_sp24()) when (val, idx) are no longer what they were made from.
 extern PyTypeObject handle_type;
 struct Handle {
     PyObject_HEAD
     Geo geo;
-    Derived *packed, *sp24;
+    KeptCopy *packed, *sp24;
 };
 
 at::Tensor attr_tensor(PyObject *o, PyObject *name) {
@@ -397,19 +453,16 @@ at::Tensor attr_tensor(PyObject *o, PyObject *name) {
     return t;
 }
 
-const at::Tensor &derived(Derived &d, PyObject *gnm, PyObject *method, const at::Tensor &val, const at::Tensor &idx) {
-    const uint32_t vv = val.unsafeGetTensorImpl()->version_counter().enabled() ? val._version() : 0;
-    const uint32_t iv = idx.unsafeGetTensorImpl()->version_counter().enabled() ? idx._version() : 0;
-    const void *vp = val.const_data_ptr(), *ip = idx.const_data_ptr();
-    if (!d.valid || d.val != vp || d.idx != ip || d.val_version != vv || d.idx_version != iv) {
-        PyObject *r = PyObject_CallMethodNoArgs(gnm, method);
-        if (!r) throw PyRaised();
-        d.copy = r == Py_None || !THPVariable_Check(r) ? at::Tensor() : THPVariable_Unpack(r);
-        Py_DECREF(r);
-        d.val = vp; d.idx = ip; d.val_version = vv; d.idx_version = iv;
-        d.valid = true;
+at::Tensor derived(KeptCopy *&kept, PyObject *gnm, PyObject *method, const at::Tensor &val, const at::Tensor &idx) {
+    if (!kept || !kept->from(val, idx)) {
+        std::unique_ptr<KeptCopy> now(new KeptCopy(val, idx));
+        Ref r(PyObject_CallMethodNoArgs(gnm, method));
+        if (!r.p) throw PyRaised();
+        if (THPVariable_Check(r.p)) now->copy = THPVariable_Unpack(r.p);
+        delete kept;  // after the call: another thread may have been here while it ran
+        kept = now.release();
     }
-    return d.copy;
+    return kept->copy;
 }
 
 PyObject *handle_new(PyTypeObject *type, PyObject *args, PyObject *) {
@@ -419,8 +472,7 @@ PyObject *handle_new(PyTypeObject *type, PyObject *args, PyObject *) {
     Handle *h = reinterpret_cast<Handle *>(type->tp_alloc(type, 0));
     if (!h) return nullptr;
     h->geo = Geo{M, K, n, m, g};
-    h->packed = new Derived();
-    h->sp24 = new Derived();
+    h->packed = h->sp24 = nullptr;
     return reinterpret_cast<PyObject *>(h);
 }
 void handle_dealloc(PyObject *self) {
@@ -458,7 +510,7 @@ PyObject *handle_linear(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     }
     if (act.rows > 0) {
         const bool wants = nmg_spmm_uses_packed(geo.M, geo.K, act.rows, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 0) != 0;
-        call_spmm(geo, code, dev, val, idx, wants ? derived(*h->packed, a[0], g_s_packed, val, idx) : at::Tensor(), act, act.rows, bias, epi, out, geo.M,
+        call_spmm(geo, code, dev, val, idx, wants ? derived(h->packed, a[0], g_s_packed, val, idx) : at::Tensor(), act, act.rows, bias, epi, out, geo.M,
                   NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO);
     }
     return THPVariable_Wrap(out);
@@ -483,7 +535,7 @@ PyObject *handle_mm(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     if (act.cols > 0) {
         // a handful of columns runs on the tensor cores when the packed copy is there already: keep one for the token-major call
         const bool wants = nmg_spmm_uses_packed(geo.M, geo.K, act.cols, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 0) != 0;
-        call_spmm(geo, code, dev, val, idx, wants ? derived(*h->packed, a[0], g_s_packed, val, idx) : at::Tensor(), act, act.cols, at::Tensor(), Epi(), out,
+        call_spmm(geo, code, dev, val, idx, wants ? derived(h->packed, a[0], g_s_packed, val, idx) : at::Tensor(), act, act.cols, at::Tensor(), Epi(), out,
                   act.cols, NMG_ACT_K_MAJOR, NMG_ALGO_AUTO);
     }
     return THPVariable_Wrap(out);
@@ -500,9 +552,9 @@ at::Tensor input_gradient(Handle *h, PyObject *gnm, const at::Tensor &val, const
     if (dy.rows > 0) {
         at::Tensor sp24, packed;
         // the compressed transposed copy serves the large batches of a 16-bit weight inside the 2:4 structure
-        if (dy.rows >= sp24_min_tokens) sp24 = derived(*h->sp24, gnm, g_s_packed_sp24, val, idx);
+        if (dy.rows >= sp24_min_tokens) sp24 = derived(h->sp24, gnm, g_s_packed_sp24, val, idx);
         if (!sp24.defined() && nmg_spmm_uses_packed(geo.M, geo.K, dy.rows, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 1))
-            packed = derived(*h->packed, gnm, g_s_packed, val, idx);
+            packed = derived(h->packed, gnm, g_s_packed, val, idx);
         call_spmm_t(geo, code, dev, val, idx, packed, sp24.defined() && sp24_rows_ok(dy) ? sp24 : at::Tensor(), dy, dx, NMG_ALGO_AUTO);
     }
     return dx;
@@ -705,6 +757,13 @@ PyMethodDef handle_methods[] = {
 };
 PyTypeObject handle_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 
+PyMethodDef kept_methods[] = {
+    NMG_METHOD("get", kept_get),
+    NMG_METHOD("put", kept_put),
+    {nullptr, nullptr, 0, nullptr},
+};
+PyTypeObject kept_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
+
 PyMethodDef module_methods[] = {
     NMG_METHOD("spmm", py_spmm),
     NMG_METHOD("spmm_t", py_spmm_t),
@@ -730,6 +789,14 @@ PyMODINIT_FUNC PyInit__nmg_host(void) {
     handle_type.tp_dealloc = handle_dealloc;
     handle_type.tp_methods = handle_methods;
     if (PyType_Ready(&handle_type) < 0) return nullptr;
+    kept_type.tp_name = "sten_b200._nmg_host.Kept";
+    kept_type.tp_basicsize = sizeof(Kept);
+    kept_type.tp_flags = Py_TPFLAGS_DEFAULT;
+    kept_type.tp_doc = "Copy derived from a weight's (val, idx), valid while both are the same tensors at the same version.";
+    kept_type.tp_new = kept_new;
+    kept_type.tp_dealloc = kept_dealloc;
+    kept_type.tp_methods = kept_methods;
+    if (PyType_Ready(&kept_type) < 0) return nullptr;
     g_s_val = PyUnicode_InternFromString("val");
     g_s_idx = PyUnicode_InternFromString("idx");
     g_s_packed = PyUnicode_InternFromString("packed");
@@ -748,7 +815,8 @@ PyMODINIT_FUNC PyInit__nmg_host(void) {
     g_zero = PyLong_FromLong(0);  // NMG_EPI_NONE
     PyObject *mod = PyModule_Create(&module_def);
     if (!mod) return nullptr;
-    if (PyModule_AddObjectRef(mod, "Handle", reinterpret_cast<PyObject *>(&handle_type)) < 0) {
+    if (PyModule_AddObjectRef(mod, "Handle", reinterpret_cast<PyObject *>(&handle_type)) < 0 ||
+        PyModule_AddObjectRef(mod, "Kept", reinterpret_cast<PyObject *>(&kept_type)) < 0) {
         Py_DECREF(mod);
         return nullptr;
     }

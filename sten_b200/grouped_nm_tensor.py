@@ -135,21 +135,27 @@ class GroupedNMTensor:
             h = self.__dict__["_native"] = nat.host().Handle(int(M), int(K), s["n"], s["m"], s["group_size"])
         return h
 
-    def packed(self):
-        """Column-ordered device copy used by the tensor-core and transposed kernels (``nmg_pack``).
+    def _kept(self, name, build):
+        """The copy kept under ``name``, made by ``build`` when ``val`` / ``idx`` are not the tensors, or not at the version, that
+        the kept one was made from.  A cache, never pickled."""
+        val, idx, kept = self.val, self.idx, self.__dict__.get(name)
+        copy = kept.get(val, idx) if kept is not None else None
+        if copy is None:
+            s = self.nm_strides
+            M, K = (int(v) for v in s["dense_shape"])
+            kept = nat.host().Kept(val, idx)
+            copy = build(val, idx, M, K, s["n"], s["m"], s["group_size"])
+            kept.put(copy)
+            self.__dict__[name] = kept
+        return copy
 
-        Built on first use and kept while ``val`` / ``idx`` are the same tensors at the same version; it is a
-        cache, never pickled."""
+    def packed(self):
+        """Column-ordered device copy used by the tensor-core and transposed kernels (``nmg_pack``).  Built on first use and
+        kept while ``val`` / ``idx`` are the same tensors at the same version."""
         s = self.nm_strides
         if len(s["dense_shape"]) != 2 or s["sparse_dim"] != 0:
             raise ValueError("the packed copy exists for 2-D weights with n:m blocks along dim 0")
-        key = (self.val.data_ptr(), self.val._version, self.idx.data_ptr(), self.idx._version, self.val.dtype)
-        cache = self.__dict__.get("_packed_cache")
-        if cache is None or cache[0] != key:
-            M, K = s["dense_shape"]
-            cache = (key, ops.pack(self.val, self.idx, int(M), int(K), s["n"], s["m"], s["group_size"]))
-            self.__dict__["_packed_cache"] = cache
-        return cache[1]
+        return self._kept("_packed_cache", ops.pack)
 
     def expanded(self):
         """Kept dense 16-bit copy for ``kernel="sm100-expanded"`` (``nmg_expand``), or None when there is none (fp32,
@@ -157,13 +163,7 @@ class GroupedNMTensor:
         s = self.nm_strides
         if len(s["dense_shape"]) != 2 or s["sparse_dim"] != 0 or not self.val.is_cuda or self.val.dtype == torch.float32:
             return None
-        key = (self.val.data_ptr(), self.val._version, self.idx.data_ptr(), self.idx._version, self.val.dtype)
-        cache = self.__dict__.get("_expanded_cache")
-        if cache is None or cache[0] != key:
-            M, K = (int(v) for v in s["dense_shape"])
-            cache = (key, ops.expand(self.val, self.idx, M, K, s["n"], s["m"], s["group_size"]))
-            self.__dict__["_expanded_cache"] = cache
-        return cache[1]
+        return self._kept("_expanded_cache", ops.expand)
 
     def packed_sp24(self):
         """Compressed transposed copy for the structured-sparse backward product (``nmg_pack_sp24``), or None when the
@@ -174,12 +174,7 @@ class GroupedNMTensor:
         M, K = (int(v) for v in s["dense_shape"])
         if not self.val.is_cuda or ops.sp24_bytes(M, K, s["n"], s["m"], s["group_size"], self.val.dtype) == 0:
             return None
-        key = (self.val.data_ptr(), self.val._version, self.idx.data_ptr(), self.idx._version, self.val.dtype)
-        cache = self.__dict__.get("_sp24_cache")
-        if cache is None or cache[0] != key:
-            cache = (key, ops.pack_sp24(self.val, self.idx, M, K, s["n"], s["m"], s["group_size"]))
-            self.__dict__["_sp24_cache"] = cache
-        return cache[1]
+        return self._kept("_sp24_cache", ops.pack_sp24)
 
     def to(self, device=None, dtype=None, non_blocking=False, copy=False):
         """Same layout on another device / in another floating dtype (indices are dtype independent)."""

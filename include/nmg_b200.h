@@ -127,9 +127,9 @@ int nmg_pack(const void *val, const int16_t *idx, int64_t M, int64_t K, int n, i
  * caller for the duration of the call (may be NULL when the query returns 0).
  * algo: NMG_ALGO_AUTO uses the tensor cores for weights of at least 64 rows, at every token count (16-bit rows that are not
  * 16-byte aligned, and K-major activations, are re-laid out into the workspace first); fewer than 64 K-major columns take
- * them when `packed` is given.  The SIMT kernels serve the rest.  Two tensor-core variants exist.  Below 1536 tokens (1024
- * for fp32), for m in {4, 8, 16} and n <= 2, one fused kernel expands tiles of the packed copy inside the matmul.  From
- * there on, and for every other (n, m), the weight is first expanded into a transient dense 16-bit matrix in the workspace
+ * them when `packed` is given.  The SIMT kernels serve the rest.  Two tensor-core variants exist.  Below 1536 tokens
+ * (1025 in fp32), for m in {4, 8, 16} and n <= 2, one fused kernel expands tiles of the packed copy inside the matmul; when
+ * `packed` is NULL it serves fewer than 1280 tokens (513 in fp32).  From there on, and for every other (n, m), the weight is first expanded into a transient dense 16-bit matrix in the workspace
  * (M * round_up(K, 8) * 2 bytes; three such planes for fp32) and multiplied by a persistent TMA-fed kernel; that
  * variant reads val / idx and ignores `packed`.  fp32 operands go through the tensor cores as exact three-way bf16
  * splits with promoted fp32 accumulation (relative error ~3.5e-6, independent of K); NMG_ALGO_SIMT forces plain fp32
@@ -180,7 +180,7 @@ int nmg_pack_sp24(const void *val, const int16_t *idx, int64_t M, int64_t K, int
 int nmg_spmm_t_sp24(const void *sp24, int64_t M, int64_t K, int n, int m, int g, int dtype, const void *dy, int64_t ld_dy,
                     int64_t tokens, void *dx, int64_t ld_dx, void *stream);
 
-/* Opt-in for compute-bound serving: keep the EXPANDED 16-bit weight across calls.  From 1536 tokens on nmg_spmm expands
+/* Opt-in for compute-bound serving: keep the EXPANDED 16-bit weight across calls.  In the two-pass variant nmg_spmm expands
  * the weight into its workspace on every call (about M * K * 2.5 bytes of HBM traffic); a caller that prefers speed over
  * the format's memory saving expands once (nmg_expand: M * round_up(K, 8) * 2 bytes) and calls nmg_spmm_expanded, which
  * runs the tensor-core matmul and the fused epilogue of nmg_spmm_fused alone.  The counterpart of the kernel-choice knob
@@ -194,9 +194,11 @@ int nmg_spmm_expanded(const void *expanded, int64_t M, int64_t K, int dtype, con
                       int layout, void *stream);
 
 /* Whether nmg_spmm (transposed = 0) or nmg_spmm_t (transposed = 1) would read the packed copy for this problem under
- * `algo`, assuming aligned operands: 1 or 0.  Lets a host build and keep packed copies only for the weights and batch
- * sizes that use them (the two-pass tensor-core variant and the SIMT forward kernel do not).  `layout` is ignored for
- * transposed = 1.  No counterpart in the reference. */
+ * `algo`, assuming aligned operands: 0, NMG_PACKED_NEEDED (built in the workspace when it is not given) or
+ * NMG_PACKED_IF_KEPT (without one the call reads val / idx in the two-pass variant, which is faster than building a copy for
+ * one call).  Lets a host build and keep packed copies only for the weights and batch sizes that use them.  `layout` is
+ * ignored for transposed = 1.  No counterpart in the reference. */
+typedef enum { NMG_PACKED_NEEDED = 1, NMG_PACKED_IF_KEPT = 2 } nmg_packed_use;
 int nmg_spmm_uses_packed(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype, int layout, int algo,
                          int transposed);
 

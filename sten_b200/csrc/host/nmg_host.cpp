@@ -390,7 +390,8 @@ struct Source {
 // A copy derived from (val, idx), valid while both are the same tensors at the same version.
 struct KeptCopy {
     Source val, idx;
-    at::Tensor copy;  // undefined: there is none for this weight
+    at::Tensor copy;  // undefined: there is none for this weight, or none has been made
+    bool made = false;
     KeptCopy(const at::Tensor &v, const at::Tensor &i) : val(v), idx(i) {}  // before the copy is made: a write meanwhile shows
     bool from(const at::Tensor &v, const at::Tensor &i) const { return val.is(v) && idx.is(i); }
 };
@@ -420,13 +421,15 @@ void kept_dealloc(PyObject *self) {
 PyObject *kept_get(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     NMG_PY_BEGIN(2)
     const KeptCopy *k = reinterpret_cast<Kept *>(self)->data;
-    if (!k->copy.defined() || !k->from(tensor_arg(a[0]), tensor_arg(a[1]))) Py_RETURN_NONE;
+    if (!k->made || !k->from(tensor_arg(a[0]), tensor_arg(a[1]))) Py_RETURN_NONE;
     return THPVariable_Wrap(k->copy);
     NMG_PY_END
 }
 PyObject *kept_put(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     NMG_PY_BEGIN(1)
-    reinterpret_cast<Kept *>(self)->data->copy = tensor_arg(a[0]);
+    KeptCopy *k = reinterpret_cast<Kept *>(self)->data;
+    k->copy = tensor_arg(a[0]);
+    k->made = true;
     Py_RETURN_NONE;
     NMG_PY_END
 }
@@ -453,16 +456,28 @@ at::Tensor attr_tensor(PyObject *o, PyObject *name) {
     return t;
 }
 
-at::Tensor derived(KeptCopy *&kept, PyObject *gnm, PyObject *method, const at::Tensor &val, const at::Tensor &idx) {
-    if (!kept || !kept->from(val, idx)) {
-        std::unique_ptr<KeptCopy> now(new KeptCopy(val, idx));
+// when_reused: the first call on these contents goes without the copy.  A weight that is written before every call (a training
+// step) then never pays for copies that one call reads: 4096 x 4096 bf16, 1280 tokens 97 us with a copy made every time, 72 without.
+at::Tensor derived(KeptCopy *&kept, PyObject *gnm, PyObject *method, const at::Tensor &val, const at::Tensor &idx, bool when_reused = false) {
+    const bool known = kept && kept->from(val, idx);
+    if (known && kept->made) return kept->copy;
+    std::unique_ptr<KeptCopy> now(new KeptCopy(val, idx));
+    if (known || !when_reused) {
         Ref r(PyObject_CallMethodNoArgs(gnm, method));
         if (!r.p) throw PyRaised();
         if (THPVariable_Check(r.p)) now->copy = THPVariable_Unpack(r.p);
-        delete kept;  // after the call: another thread may have been here while it ran
-        kept = now.release();
+        now->made = true;
     }
+    delete kept;  // here, not earlier: another thread may have been here while the method ran
+    kept = now.release();
     return kept->copy;
+}
+
+// The column-ordered copy for a call of `tokens` rows, where the kernel that serves it reads one.
+at::Tensor packed_for(Handle *h, PyObject *gnm, const at::Tensor &val, const at::Tensor &idx, int64_t tokens, int code, bool transposed) {
+    const Geo &geo = h->geo;
+    const int uses = nmg_spmm_uses_packed(geo.M, geo.K, tokens, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, transposed ? 1 : 0);
+    return uses ? derived(h->packed, gnm, g_s_packed, val, idx, uses == NMG_PACKED_IF_KEPT) : at::Tensor();
 }
 
 PyObject *handle_new(PyTypeObject *type, PyObject *args, PyObject *) {
@@ -509,9 +524,8 @@ PyObject *handle_linear(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
         epi.ld = act.rows > 1 ? r.ld : geo.M;
     }
     if (act.rows > 0) {
-        const bool wants = nmg_spmm_uses_packed(geo.M, geo.K, act.rows, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 0) != 0;
-        call_spmm(geo, code, dev, val, idx, wants ? derived(h->packed, a[0], g_s_packed, val, idx) : at::Tensor(), act, act.rows, bias, epi, out, geo.M,
-                  NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO);
+        call_spmm(geo, code, dev, val, idx, packed_for(h, a[0], val, idx, act.rows, code, false), act, act.rows, bias, epi, out, geo.M, NMG_ACT_TOKEN_MAJOR,
+                  NMG_ALGO_AUTO);
     }
     return THPVariable_Wrap(out);
     NMG_PY_END
@@ -534,9 +548,8 @@ PyObject *handle_mm(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     const at::Tensor out = new_empty({geo.M, act.cols}, val.scalar_type());
     if (act.cols > 0) {
         // a handful of columns runs on the tensor cores when the packed copy is there already: keep one for the token-major call
-        const bool wants = nmg_spmm_uses_packed(geo.M, geo.K, act.cols, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 0) != 0;
-        call_spmm(geo, code, dev, val, idx, wants ? derived(h->packed, a[0], g_s_packed, val, idx) : at::Tensor(), act, act.cols, at::Tensor(), Epi(), out,
-                  act.cols, NMG_ACT_K_MAJOR, NMG_ALGO_AUTO);
+        call_spmm(geo, code, dev, val, idx, packed_for(h, a[0], val, idx, act.cols, code, false), act, act.cols, at::Tensor(), Epi(), out, act.cols,
+                  NMG_ACT_K_MAJOR, NMG_ALGO_AUTO);
     }
     return THPVariable_Wrap(out);
     NMG_PY_END
@@ -553,8 +566,7 @@ at::Tensor input_gradient(Handle *h, PyObject *gnm, const at::Tensor &val, const
         at::Tensor sp24, packed;
         // the compressed transposed copy serves the large batches of a 16-bit weight inside the 2:4 structure
         if (dy.rows >= sp24_min_tokens) sp24 = derived(h->sp24, gnm, g_s_packed_sp24, val, idx);
-        if (!sp24.defined() && nmg_spmm_uses_packed(geo.M, geo.K, dy.rows, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, 1))
-            packed = derived(h->packed, gnm, g_s_packed, val, idx);
+        if (!sp24.defined()) packed = packed_for(h, gnm, val, idx, dy.rows, code, true);
         call_spmm_t(geo, code, dev, val, idx, packed, sp24.defined() && sp24_rows_ok(dy) ? sp24 : at::Tensor(), dy, dx, NMG_ALGO_AUTO);
     }
     return dx;

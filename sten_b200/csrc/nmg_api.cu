@@ -88,7 +88,7 @@ extern "C" size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens,
     size_t tensor = 0;
     const bool tensor_runs = algo == NMG_ALGO_TENSOR ? any_tensor(geo, dtype) : algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, M);
     if (tensor_runs)
-        tensor = (tc_use_dense(geo, dtype, false, tokens) ? tc_dense_workspace_bytes(geo, dtype, false)
+        tensor = (tc_use_dense(geo, dtype, false, tokens, have_packed != 0) ? tc_dense_workspace_bytes(geo, dtype, false)
                                                    : (have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512)) +
                  tc_split_workspace_bytes(geo, dtype, false, tokens) +
                  (layout == NMG_ACT_K_MAJOR ? kmajor_transpose_bytes(geo, dtype, tokens) : algo == NMG_ALGO_AUTO ? pad_rows_bytes(dtype, tokens, K) : 0);
@@ -139,7 +139,7 @@ static int spmm_impl(const void *val, const int16_t *idx, const void *packed, in
             ws = rest;
         }
         const void *pat = nullptr, *nval = nullptr;
-        const bool dense = force_dense || tc_use_dense(geo, dtype, false, tokens);
+        const bool dense = force_dense || tc_use_dense(geo, dtype, false, tokens, packed != nullptr);
         if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st))) return rc;
         return tc_matmul(geo, dtype, false, dense, val, idx, pat, nval, act, ld_act, dtype == NMG_F32 && !tm, tokens, bias, outs, n_outs, mc_out, ld_out, out_tm ? 1 : 0,
                          ws, left, st, epi);
@@ -199,14 +199,15 @@ extern "C" int nmg_spmm_uses_packed(int64_t M, int64_t K, int64_t tokens, int n,
     const bool any_tc = any_tensor(geo, dtype);
     const bool wants = algo == NMG_ALGO_TENSOR || algo == NMG_ALGO_TENSOR_DENSE || (algo == NMG_ALGO_AUTO && (transposed ? K : M) >= 64);
     const bool tensor = any_tc && wants && (transposed || layout != NMG_ACT_K_MAJOR || tokens >= 64 || algo == NMG_ALGO_TENSOR);
-    if (tensor) return tc_use_dense(geo, dtype, transposed != 0, tokens) ? 0 : 1;
-    return transposed ? 1 : 0;  // SIMT: the transposed kernel reads the packed copy, the forward kernel val / idx
+    if (tensor && tc_use_dense(geo, dtype, transposed != 0, tokens, true)) return 0;
+    if (tensor) return tc_use_dense(geo, dtype, transposed != 0, tokens, false) ? NMG_PACKED_IF_KEPT : NMG_PACKED_NEEDED;
+    return transposed ? NMG_PACKED_NEEDED : 0;  // SIMT: the transposed kernel reads the packed copy, the forward kernel val / idx
 }
 
 // Whether nmg_spmm_t takes the structured-sparse tensor-core path: a supported 16-bit weight, enough tokens for the
 // two-pass regime, and the caller did not ask for the dense-rate kernels.
 static bool use_sp(const Geo &geo, int dtype, int64_t tokens, int algo) {
-    return algo != NMG_ALGO_SIMT && algo != NMG_ALGO_TENSOR_DENSE && tc_sp_supported(geo, dtype) && tc_use_dense(geo, dtype, true, tokens);
+    return algo != NMG_ALGO_SIMT && algo != NMG_ALGO_TENSOR_DENSE && tc_sp_supported(geo, dtype) && tc_use_dense(geo, dtype, true, tokens, false);
 }
 
 extern "C" size_t nmg_spmm_t_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype,
@@ -218,7 +219,7 @@ extern "C" size_t nmg_spmm_t_workspace_bytes(int64_t M, int64_t K, int64_t token
     const size_t simt = tensor_only ? 0 : pack + simt_bwd_workspace_bytes(geo, tokens, dtype) + 256;
     size_t tensor = 0;
     if (algo != NMG_ALGO_SIMT && any_tensor(geo, dtype))
-        tensor = (tc_use_dense(geo, dtype, true, tokens) ? tc_dense_workspace_bytes(geo, dtype, true) : pack) +
+        tensor = (tc_use_dense(geo, dtype, true, tokens, have_packed != 0) ? tc_dense_workspace_bytes(geo, dtype, true) : pack) +
                  tc_split_workspace_bytes(geo, dtype, true, tokens);
     if (use_sp(geo, dtype, tokens, algo) && tc_sp_copy_bytes(geo) + 512 > tensor) tensor = tc_sp_copy_bytes(geo) + 512;
     if (algo == NMG_ALGO_AUTO && tensor_only) tensor += pad_rows_bytes(dtype, tokens, M);
@@ -271,7 +272,7 @@ extern "C" int nmg_spmm_t(const void *val, const int16_t *idx, const void *packe
         if (rc == NMG_OK && pe.stop) NMG_CUDA(cudaEventRecord(pe.stop, st));
         return rc;
     }
-    const bool dense = tensor && tc_use_dense(geo, dtype, true, tokens);
+    const bool dense = tensor && tc_use_dense(geo, dtype, true, tokens, packed != nullptr);
     if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st))) return rc;
     void *dxs[1] = {dx};
     if (tensor) return tc_matmul(geo, dtype, true, dense, val, idx, pat, nval, dy, ld_dy, false, tokens, nullptr, dxs, 1, nullptr, ld_dx, 1, ws, left, st);

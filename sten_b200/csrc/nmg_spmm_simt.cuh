@@ -58,7 +58,7 @@ struct DenseAct { const void *base; int64_t ld, plane_elems; };
 
 bool tc_supported(const Geo &geo, int dtype);        // fused kernel
 bool tc_dense_supported(const Geo &geo, int dtype);  // two-pass variant
-bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens);
+bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens, bool have_packed);
 size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens);
 size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed);
 // outs / n_outs: the result goes to every listed buffer (same shape and pitch); more than one needs `dense`.  mc_out, when

@@ -796,15 +796,25 @@ static int tc_launch_nm(int dtype, bool transposed, const TcParams &p, const FxM
     return transposed ? tc_launch_one<N_, M_, __nv_bfloat16, true>(p, maps, st) : tc_launch_one<N_, M_, __nv_bfloat16, false>(p, maps, st);
 }
 
-// Policy of the two tensor-core variants.  Measured (us, fused / two passes; 2:4): bf16 4096 x 4096 29 / 44 at 1024 tokens,
-// 53 / 62 at 1280, 56 / 64 at 2048, 85 / 86 at 3072; 4096 x 1024 12 / 18 at 1024, 21 / 22 at 1536, 33 / 28 at 3072.  fp32
-// 4096 x 1024 27 / 50 at 512 tokens, 51 / 52 at 1024, 97 / 91 at 2048; 4096 x 4096 168 / 187 at 1024, 336 / 338 at 2048.
-// The transposed product of a 16-bit weight has the structured-sparse kernel in place of the second variant (from 1280 tokens).
-bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens) {
+// Policy of the two tensor-core variants.  The fused kernel reads the column-ordered copy; without one (have_packed) a call
+// would build it first and throw it away.  Measured, us, 2:4: fused with a kept copy / fused after building one / two passes
+//   fp32   tokens    1024 x 1024       4096 x 1024       1024 x 4096       4096 x 4096
+//             256    15 /  33 / 29     22 /  47 /  35    27 / 49 / 68      52 / 113 / 109
+//             512    18 /  37 / 29     29 /  53 /  42    33 / 56 / 70      87 / 157 / 129
+//            1000    23 /  41 / 29     51 /  77 /  60    55 / 78 / 78     189 / 250 / 180
+//            2048    29 /  48 / 36    101 / 128 /  93    95 / 125 / 111   377 / 431 / 313
+//   bf16     1024     9 /  24 / 17     12 /  30 /  21    20 / 37 / 31      27 /  65 /  42
+//            1280    10 /  24 / 17     19 /  37 /  25    21 / 37 / 32      49 /  86 /  60
+//            1500    10 /  24 / 17     20 /  39 /  25    23 / 40 / 33      50 /  88 /  61
+//            3072    11 /  26 / 17     32 /  51 /  30    26 / 44 / 33      87 / 130 /  89
+// (fp32 without a copy: up to 512 tokens the shape decides, not the count.)  The transposed product of a 16-bit weight has the
+// structured-sparse kernel in place of the second variant (from 1280 tokens).
+bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens, bool have_packed) {
     const bool fused = tc_supported(geo, dtype), dense = tc_dense_supported(geo, dtype);
     if (!dense) return false;
     if (!fused) return true;
-    return tokens >= (dtype == NMG_F32 ? 1024 : transposed ? 1280 : 1536);
+    if (!have_packed) return tokens >= (dtype == NMG_F32 ? 513 : 1280);
+    return tokens >= (dtype == NMG_F32 ? 1025 : transposed ? 1280 : 1536);
 }
 
 // act: [tokens][ld_act] with the reduction axis contiguous (X for the forward, dY for the transposed product).

@@ -149,8 +149,8 @@ def pack(val, idx, M, K, n, m, g):
 
 @functools.lru_cache(maxsize=4096)
 def uses_packed(M, K, tokens, n, m, g, dtype, layout=nat.NMG_ACT_TOKEN_MAJOR, algo=nat.NMG_ALGO_AUTO, transposed=False):
-    """Whether spmm (or spmm_t when `transposed`) would read the packed copy for this problem: the fused tensor-core
-    kernel and the SIMT transposed kernel do; the two-pass tensor-core variant and the SIMT forward kernel do not."""
+    """Whether spmm (or spmm_t when `transposed`) would read a packed copy that it is given for this problem: the fused
+    tensor-core kernel and the SIMT transposed kernel do; the two-pass tensor-core variant and the SIMT forward kernel do not."""
     code = {torch.float32: nat.NMG_F32, torch.float16: nat.NMG_F16, torch.bfloat16: nat.NMG_BF16}[dtype]
     return bool(nat.lib().nmg_spmm_uses_packed(M, K, tokens, n, m, g, code, layout, algo, 1 if transposed else 0))
 

@@ -136,6 +136,14 @@ struct Geo {
 
 void *stream_of(c10::Device dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
 
+// Whether work queued now goes into a CUDA graph.
+bool capturing(c10::Device dev) {
+    cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c10::cuda::getCurrentCUDAStream(dev.index()).stream(), &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return false;
+}
+
 struct Epi {
     int act = NMG_EPI_NONE;
     at::Tensor residual;  // rows of the output's shape, contiguous along the last dim
@@ -392,6 +400,7 @@ struct KeptCopy {
     Source val, idx;
     at::Tensor copy;  // undefined: there is none for this weight, or none has been made
     bool made = false;
+    bool captured = false;  // a CUDA graph reads the copy: it is not given back before the weight
     KeptCopy(const at::Tensor &v, const at::Tensor &i) : val(v), idx(i) {}  // before the copy is made: a write meanwhile shows
     bool from(const at::Tensor &v, const at::Tensor &i) const { return val.is(v) && idx.is(i); }
 };
@@ -420,8 +429,9 @@ void kept_dealloc(PyObject *self) {
 // get(val, idx) -> the copy, or None when it was made from other tensors or other contents
 PyObject *kept_get(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     NMG_PY_BEGIN(2)
-    const KeptCopy *k = reinterpret_cast<Kept *>(self)->data;
+    KeptCopy *k = reinterpret_cast<Kept *>(self)->data;
     if (!k->made || !k->from(tensor_arg(a[0]), tensor_arg(a[1]))) Py_RETURN_NONE;
+    if (k->copy.is_cuda() && capturing(k->copy.device())) k->captured = true;
     return THPVariable_Wrap(k->copy);
     NMG_PY_END
 }
@@ -433,6 +443,19 @@ PyObject *kept_put(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     Py_RETURN_NONE;
     NMG_PY_END
 }
+// captured() -> whether a CUDA graph reads the copy
+PyObject *kept_captured(PyObject *self, PyObject *const *, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(0)
+    return PyBool_FromLong(reinterpret_cast<Kept *>(self)->data->captured);
+    NMG_PY_END
+}
+// capturing(tensor) -> whether work queued now on the current stream of its device goes into a CUDA graph
+PyObject *py_capturing(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(1)
+    const at::Tensor &t = tensor_arg(a[0]);
+    return PyBool_FromLong(t.is_cuda() && capturing(t.device()));
+    NMG_PY_END
+}
 
 // ------------------------------------------------------------------------------------------------ Handle
 // What the host keeps of one 2-D weight between calls: its geometry and, for the kernels that read them, the derived copies.
@@ -442,6 +465,7 @@ struct Handle {
     PyObject_HEAD
     Geo geo;
     KeptCopy *packed, *sp24;
+    std::vector<at::Tensor> *held;  // copies of earlier contents that a CUDA graph still reads
 };
 
 at::Tensor attr_tensor(PyObject *o, PyObject *name) {
@@ -458,9 +482,13 @@ at::Tensor attr_tensor(PyObject *o, PyObject *name) {
 
 // when_reused: the first call on these contents goes without the copy.  A weight that is written before every call (a training
 // step) then never pays for copies that one call reads: 4096 x 4096 bf16, 1280 tokens 97 us with a copy made every time, 72 without.
-at::Tensor derived(KeptCopy *&kept, PyObject *gnm, PyObject *method, const at::Tensor &val, const at::Tensor &idx, bool when_reused = false) {
+// A copy made inside a CUDA graph holds nothing before a replay: it belongs to the graph and is not kept.
+at::Tensor derived(Handle *h, KeptCopy *&kept, PyObject *gnm, PyObject *method, const at::Tensor &val, const at::Tensor &idx, bool in_graph, bool when_reused = false) {
     const bool known = kept && kept->from(val, idx);
-    if (known && kept->made) return kept->copy;
+    if (known && kept->made) {
+        if (in_graph) kept->captured = true;
+        return kept->copy;
+    }
     std::unique_ptr<KeptCopy> now(new KeptCopy(val, idx));
     if (known || !when_reused) {
         Ref r(PyObject_CallMethodNoArgs(gnm, method));
@@ -468,16 +496,34 @@ at::Tensor derived(KeptCopy *&kept, PyObject *gnm, PyObject *method, const at::T
         if (THPVariable_Check(r.p)) now->copy = THPVariable_Unpack(r.p);
         now->made = true;
     }
+    if (in_graph) return now->copy;
+    if (kept && kept->captured) h->held->push_back(kept->copy);
     delete kept;  // here, not earlier: another thread may have been here while the method ran
     kept = now.release();
     return kept->copy;
 }
 
-// The column-ordered copy for a call of `tokens` rows, where the kernel that serves it reads one.
-at::Tensor packed_for(Handle *h, PyObject *gnm, const at::Tensor &val, const at::Tensor &idx, int64_t tokens, int code, bool transposed) {
+// A column-ordered copy for this call alone.
+at::Tensor pack_once(const Geo &geo, int code, c10::Device dev, const at::Tensor &val, const at::Tensor &idx) {
+    const at::Tensor v = packed_rows(val), i = packed_rows(idx);
+    const size_t nbytes = nmg_packed_bytes(geo.M, geo.K, geo.n, geo.m, geo.g, code);
+    at::Tensor buf = new_empty({(int64_t)nbytes}, at::kByte);
+    check(nmg_pack(v.const_data_ptr(), static_cast<const int16_t *>(i.const_data_ptr()), geo.M, geo.K, geo.n, geo.m, geo.g, code, buf.mutable_data_ptr(), nbytes,
+                   stream_of(dev)));
+    return buf;
+}
+
+// The column-ordered copy for a call of `tokens` rows (k_major: columns), where the kernel that serves it reads one.
+// In a CUDA graph only the calls of few tokens read the kept copy (a decode step: 9 us against 27 with a copy made in every
+// replay), and such a graph has to be captured again when the weight changes.  All others read val / idx in every replay.
+at::Tensor packed_for(Handle *h, PyObject *gnm, const at::Tensor &val, const at::Tensor &idx, int64_t tokens, int code, c10::Device dev, bool transposed, bool k_major = false) {
     const Geo &geo = h->geo;
     const int uses = nmg_spmm_uses_packed(geo.M, geo.K, tokens, geo.n, geo.m, geo.g, code, NMG_ACT_TOKEN_MAJOR, NMG_ALGO_AUTO, transposed ? 1 : 0);
-    return uses ? derived(h->packed, gnm, g_s_packed, val, idx, uses == NMG_PACKED_IF_KEPT) : at::Tensor();
+    if (!uses) return at::Tensor();
+    const bool in_graph = capturing(dev);
+    if (in_graph && uses == NMG_PACKED_IF_KEPT) return at::Tensor();
+    if (in_graph && ((k_major && tokens < 64) || (code == NMG_F32 && tokens >= 256))) return pack_once(geo, code, dev, val, idx);
+    return derived(h, h->packed, gnm, g_s_packed, val, idx, in_graph, uses == NMG_PACKED_IF_KEPT);
 }
 
 PyObject *handle_new(PyTypeObject *type, PyObject *args, PyObject *) {
@@ -488,12 +534,14 @@ PyObject *handle_new(PyTypeObject *type, PyObject *args, PyObject *) {
     if (!h) return nullptr;
     h->geo = Geo{M, K, n, m, g};
     h->packed = h->sp24 = nullptr;
+    h->held = new std::vector<at::Tensor>();
     return reinterpret_cast<PyObject *>(h);
 }
 void handle_dealloc(PyObject *self) {
     Handle *h = reinterpret_cast<Handle *>(self);
     delete h->packed;
     delete h->sp24;
+    delete h->held;
     Py_TYPE(self)->tp_free(self);
 }
 
@@ -524,7 +572,7 @@ PyObject *handle_linear(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
         epi.ld = act.rows > 1 ? r.ld : geo.M;
     }
     if (act.rows > 0) {
-        call_spmm(geo, code, dev, val, idx, packed_for(h, a[0], val, idx, act.rows, code, false), act, act.rows, bias, epi, out, geo.M, NMG_ACT_TOKEN_MAJOR,
+        call_spmm(geo, code, dev, val, idx, packed_for(h, a[0], val, idx, act.rows, code, dev, false), act, act.rows, bias, epi, out, geo.M, NMG_ACT_TOKEN_MAJOR,
                   NMG_ALGO_AUTO);
     }
     return THPVariable_Wrap(out);
@@ -548,7 +596,7 @@ PyObject *handle_mm(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     const at::Tensor out = new_empty({geo.M, act.cols}, val.scalar_type());
     if (act.cols > 0) {
         // a handful of columns runs on the tensor cores when the packed copy is there already: keep one for the token-major call
-        call_spmm(geo, code, dev, val, idx, packed_for(h, a[0], val, idx, act.cols, code, false), act, act.cols, at::Tensor(), Epi(), out, act.cols,
+        call_spmm(geo, code, dev, val, idx, packed_for(h, a[0], val, idx, act.cols, code, dev, false, true), act, act.cols, at::Tensor(), Epi(), out, act.cols,
                   NMG_ACT_K_MAJOR, NMG_ALGO_AUTO);
     }
     return THPVariable_Wrap(out);
@@ -565,8 +613,8 @@ at::Tensor input_gradient(Handle *h, PyObject *gnm, const at::Tensor &val, const
     if (dy.rows > 0) {
         at::Tensor sp24, packed;
         // the compressed transposed copy serves the large batches of a 16-bit weight inside the 2:4 structure
-        if (dy.rows >= sp24_min_tokens) sp24 = derived(h->sp24, gnm, g_s_packed_sp24, val, idx);
-        if (!sp24.defined()) packed = packed_for(h, gnm, val, idx, dy.rows, code, true);
+        if (dy.rows >= sp24_min_tokens) sp24 = derived(h, h->sp24, gnm, g_s_packed_sp24, val, idx, capturing(dev));
+        if (!sp24.defined()) packed = packed_for(h, gnm, val, idx, dy.rows, code, dev, true);
         call_spmm_t(geo, code, dev, val, idx, packed, sp24.defined() && sp24_rows_ok(dy) ? sp24 : at::Tensor(), dy, dx, NMG_ALGO_AUTO);
     }
     return dx;
@@ -772,6 +820,7 @@ PyTypeObject handle_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
 PyMethodDef kept_methods[] = {
     NMG_METHOD("get", kept_get),
     NMG_METHOD("put", kept_put),
+    NMG_METHOD("captured", kept_captured),
     {nullptr, nullptr, 0, nullptr},
 };
 PyTypeObject kept_type = {PyVarObject_HEAD_INIT(nullptr, 0)};
@@ -783,6 +832,7 @@ PyMethodDef module_methods[] = {
     NMG_METHOD("gather", py_gather),
     NMG_METHOD("column_sum", py_column_sum),
     NMG_METHOD("densify", py_densify),
+    NMG_METHOD("capturing", py_capturing),
     NMG_METHOD("set_dispatch", py_set_dispatch),
     NMG_METHOD("repeat_call", py_repeat_call),
     {"set_error_class", py_set_error_class, METH_O, nullptr},

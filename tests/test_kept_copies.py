@@ -62,3 +62,76 @@ def test_products_after_two_replacements_of_the_values(tokens, dtype):
         assert rel(w.native().linear_t(w, dy, ops.SP24_MIN_TOKENS), dy.double() @ dense) < 1e-2
         if dtype != torch.float32:
             assert rel(ops.spmm_expanded(w.expanded(), M, K, x), x.double() @ dense.t()) < 1e-2
+
+
+def _captured(fn, device=torch.device("cuda", 0)):
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        out = fn()
+    return graph, out
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype,tokens,op", [(torch.float32, 300, "linear"), (torch.float32, 600, "linear"), (torch.float32, 300, "mm"), (torch.float32, 600, "linear_t"),
+                                             (torch.bfloat16, 1400, "linear"), (torch.bfloat16, 8, "mm"), (torch.float32, 8, "mm")])
+def test_replays_see_what_was_written_into_the_weight(dtype, tokens, op):
+    dev, M, K = torch.device("cuda", 0), 256, 512
+    w = GroupedNMTensor.from_dense(torch.randn(M, K, device=dev).to(dtype), 2, 4, 0, 16, 1)
+    h = w.native()
+    x = torch.randn(tokens, M if op == "linear_t" else K, device=dev).to(dtype)
+    b = x.t().contiguous()
+    fn = {"linear": lambda: h.linear(w, x, None, 0, None), "mm": lambda: h.mm(w, b), "linear_t": lambda: h.linear_t(w, x, ops.SP24_MIN_TOKENS)}[op]
+    want = lambda: {"linear": lambda d: x.double() @ d.t(), "mm": lambda d: d @ b.double(), "linear_t": lambda d: x.double() @ d}[op](w.to_dense().double())  # noqa: E731
+    for _ in range(3):
+        fn()
+    graph, out = _captured(fn)
+    w.val.mul_(2)
+    graph.replay()
+    assert _rel(out, want()) < 1e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op", ["linear", "linear_t"])
+def test_a_copy_made_inside_a_graph_is_not_kept(op):
+    dev, M, K = torch.device("cuda", 0), 256, 512
+    w, warm = (GroupedNMTensor.from_dense(torch.randn(M, K, device=dev).bfloat16(), 2, 4, 0, 16, 1) for _ in range(2))
+    for tokens in (16, 1300):
+        x = torch.randn(tokens, K if op == "linear" else M, device=dev).bfloat16()
+        fn = lambda t: t.native().linear(t, x, None, 0, None) if op == "linear" else t.native().linear_t(t, x, ops.SP24_MIN_TOKENS)  # noqa: E731
+        fn(warm)
+        graph, out = _captured(lambda: fn(w))
+        assert not {"_packed_cache", "_sp24_cache"} & set(w.__dict__)
+        d = w.to_dense().double()
+        want = x.double() @ (d.t() if op == "linear" else d)
+        graph.replay()
+        assert _rel(out, want) < 1e-2
+    del graph
+    assert _rel(fn(w), want) < 1e-2
+
+
+@pytest.mark.gpu
+def test_a_graph_keeps_the_copy_that_it_reads():
+    """A captured call of few tokens reads the copy of the contents it was captured with; a later change of the weight does not
+    give that memory to somebody else."""
+    dev, M, K = torch.device("cuda", 0), 256, 512
+    w = GroupedNMTensor.from_dense(torch.randn(M, K, device=dev).bfloat16(), 2, 4, 0, 16, 1)
+    x = torch.randn(16, K, device=dev).bfloat16()
+    fn = lambda: w.native().linear(w, x, None, 0, None)  # noqa: E731
+    fn()
+    graph, out = _captured(fn)
+    graph.replay()
+    before = out.clone()
+    keep = (w.val, w.idx)  # what the graph was captured with
+    nbytes = w.packed().numel()
+    for _ in range(2):
+        w.val = w.val * 3
+        fn()
+        filler = [torch.full((nbytes,), 0x55, dtype=torch.uint8, device=dev) for _ in range(4)]
+    graph.replay()
+    assert torch.equal(out, before)
+    del filler, keep

@@ -17,6 +17,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <memory>
+#include <optional>
 #include <string>
 #include <vector>
 
@@ -395,13 +396,51 @@ struct Source {
                data == t.const_data_ptr() && version == t._version() && type == t.scalar_type();
     }
 };
-// A copy derived from (val, idx), valid while both are the same tensors at the same version.
+// A copy derived from (val, idx), valid while both are the same tensors at the same version.  It is made on the stream that first
+// asks for it; a call on another stream waits for that, and the copy's memory then counts as used there too.
 struct KeptCopy {
     Source val, idx;
     at::Tensor copy;  // undefined: there is none for this weight, or none has been made
     bool made = false;
     bool captured = false;  // a CUDA graph reads the copy: it is not given back before the weight
+    std::optional<c10::cuda::CUDAStream> stream;
+    cudaEvent_t ready = nullptr;  // behind the kernels that make it
+    bool complete = false;
     KeptCopy(const at::Tensor &v, const at::Tensor &i) : val(v), idx(i) {}  // before the copy is made: a write meanwhile shows
+    KeptCopy(const KeptCopy &) = delete;
+    ~KeptCopy() {
+        if (ready) cudaEventDestroy(ready);
+    }
+    void put(const at::Tensor &c) {
+        copy = c;
+        made = true;
+        if (!copy.defined() || !copy.is_cuda()) return;
+        const c10::cuda::CUDAGuard guard(copy.device());
+        stream = c10::cuda::getCurrentCUDAStream(copy.device().index());
+        C10_CUDA_CHECK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
+        C10_CUDA_CHECK(cudaEventRecord(ready, stream->stream()));
+    }
+    const at::Tensor &use(bool in_graph) {
+        if (!ready) return copy;
+        captured |= in_graph;
+        const c10::cuda::CUDAStream now = c10::cuda::getCurrentCUDAStream(copy.device().index());
+        if (now == *stream) return copy;
+        if (!complete) {
+            // a graph cannot wait for an event from outside it: wait here (relaxed: the event has nothing to do with the capture)
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            C10_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+            cudaError_t e = in_graph ? cudaEventSynchronize(ready) : cudaEventQuery(ready);
+            complete = e == cudaSuccess;
+            if (e == cudaErrorNotReady) {
+                cudaGetLastError();
+                e = cudaStreamWaitEvent(now.stream(), ready, 0);
+            }
+            C10_CUDA_CHECK(cudaThreadExchangeStreamCaptureMode(&mode));
+            C10_CUDA_CHECK(e);
+        }
+        if (!in_graph) c10::cuda::CUDACachingAllocator::recordStream(copy.storage().data_ptr(), now);
+        return copy;
+    }
     bool from(const at::Tensor &v, const at::Tensor &i) const { return val.is(v) && idx.is(i); }
 };
 
@@ -431,15 +470,12 @@ PyObject *kept_get(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     NMG_PY_BEGIN(2)
     KeptCopy *k = reinterpret_cast<Kept *>(self)->data;
     if (!k->made || !k->from(tensor_arg(a[0]), tensor_arg(a[1]))) Py_RETURN_NONE;
-    if (k->copy.is_cuda() && capturing(k->copy.device())) k->captured = true;
-    return THPVariable_Wrap(k->copy);
+    return THPVariable_Wrap(k->use(k->copy.is_cuda() && capturing(k->copy.device())));
     NMG_PY_END
 }
 PyObject *kept_put(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     NMG_PY_BEGIN(1)
-    KeptCopy *k = reinterpret_cast<Kept *>(self)->data;
-    k->copy = tensor_arg(a[0]);
-    k->made = true;
+    reinterpret_cast<Kept *>(self)->data->put(tensor_arg(a[0]));
     Py_RETURN_NONE;
     NMG_PY_END
 }
@@ -485,18 +521,15 @@ at::Tensor attr_tensor(PyObject *o, PyObject *name) {
 // A copy made inside a CUDA graph holds nothing before a replay: it belongs to the graph and is not kept.
 at::Tensor derived(Handle *h, KeptCopy *&kept, PyObject *gnm, PyObject *method, const at::Tensor &val, const at::Tensor &idx, bool in_graph, bool when_reused = false) {
     const bool known = kept && kept->from(val, idx);
-    if (known && kept->made) {
-        if (in_graph) kept->captured = true;
-        return kept->copy;
-    }
+    if (known && kept->made) return kept->use(in_graph);
     std::unique_ptr<KeptCopy> now(new KeptCopy(val, idx));
     if (known || !when_reused) {
         Ref r(PyObject_CallMethodNoArgs(gnm, method));
         if (!r.p) throw PyRaised();
-        if (THPVariable_Check(r.p)) now->copy = THPVariable_Unpack(r.p);
-        now->made = true;
+        const at::Tensor copy = THPVariable_Check(r.p) ? THPVariable_Unpack(r.p) : at::Tensor();
+        if (in_graph) return copy;
+        now->put(copy);
     }
-    if (in_graph) return now->copy;
     if (kept && kept->captured) h->held->push_back(kept->copy);
     delete kept;  // here, not earlier: another thread may have been here while the method ran
     kept = now.release();

@@ -135,3 +135,55 @@ def test_a_graph_keeps_the_copy_that_it_reads():
     graph.replay()
     assert torch.equal(out, before)
     del filler, keep
+
+
+_CALLS = {"linear": lambda w, x: w.native().linear(w, x, None, 0, None), "linear_t": lambda w, x: w.native().linear_t(w, x, ops.SP24_MIN_TOKENS),
+          "expanded": lambda w, x: ops.spmm_expanded(w.expanded(), x.shape[1], x.shape[1], x)}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tokens", [16, 1300])
+@pytest.mark.parametrize("op", sorted(_CALLS))
+def test_another_stream_waits_for_the_copy(op, tokens):
+    """The copy is made on one stream behind 100 ms of other work; a call on another stream uses it meanwhile."""
+    dev, M = torch.device("cuda", 0), 512
+    w = GroupedNMTensor.from_dense(torch.randn(M, M, device=dev).bfloat16(), 2, 4, 0, 16, 1)
+    x = torch.randn(tokens, M, device=dev).bfloat16()
+    dense = w.to_dense().double()
+    want = x.double() @ (dense if op == "linear_t" else dense.t())
+    one, two = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(one):
+        torch.cuda._sleep(200_000_000)
+        for _ in range(2):
+            _CALLS[op](w, x)
+    with torch.cuda.stream(two):
+        out = _CALLS[op](w, x)
+    torch.cuda.synchronize()
+    assert _rel(out, want) < 1e-2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op", sorted(_CALLS))
+def test_a_replaced_copy_stays_until_other_streams_have_read_it(op):
+    dev, M, tokens = torch.device("cuda", 0), 512, 1300
+    w = GroupedNMTensor.from_dense(torch.randn(M, M, device=dev).bfloat16(), 2, 4, 0, 16, 1)
+    x = torch.randn(tokens, M, device=dev).bfloat16()
+    dense = w.to_dense().double()
+    want = x.double() @ (dense if op == "linear_t" else dense.t())
+    for _ in range(3):
+        _CALLS[op](w, x)
+    nbytes = {n: k.get(w.val, w.idx).numel() for n, k in w.__dict__.items() if n.endswith("_cache")}
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    keep = (w.val, w.idx)
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(200_000_000)
+        out = _CALLS[op](w, x)
+    w.val = w.val * 3
+    for _ in range(3):
+        _CALLS[op](w, x)
+    filler = [torch.full((n,), 0x55, dtype=torch.uint8, device=dev) for n in nbytes.values() for _ in range(6)]
+    torch.cuda.synchronize()
+    assert _rel(out, want) < 1e-2
+    del keep, filler

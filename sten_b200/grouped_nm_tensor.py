@@ -138,16 +138,17 @@ class GroupedNMTensor:
     def _kept(self, name, build):
         """The copy kept under ``name``, made by ``build`` when ``val`` / ``idx`` are not the tensors, or not at the version, that
         the kept one was made from.  A cache, never pickled.  A copy made inside a CUDA graph holds nothing before a replay: it is
-        the graph's and not kept; a kept one that a graph reads stays until the weight goes."""
+        the graph's and not kept; a kept one that a graph reads stays until the weight goes.  Tensors made under inference mode do
+        not count their writes: nothing is kept of them."""
         val, idx, kept = self.val, self.idx, self.__dict__.get(name)
-        copy = kept.get(val, idx) if kept is not None else None
+        copy = kept.get(val, idx) if kept is not None and not val.is_inference() and not idx.is_inference() else None
         if copy is None:
             s = self.nm_strides
             M, K = (int(v) for v in s["dense_shape"])
+            if val.is_inference() or idx.is_inference() or nat.host().capturing(val):
+                return build(val, idx, M, K, s["n"], s["m"], s["group_size"])
             now = nat.host().Kept(val, idx)
             copy = build(val, idx, M, K, s["n"], s["m"], s["group_size"])
-            if nat.host().capturing(val):
-                return copy
             now.put(copy)
             if kept is not None and kept.captured():
                 self.__dict__.setdefault("_held_copies", []).append(kept)

@@ -40,6 +40,37 @@ def test_a_changed_weight_is_packed_again(change, monkeypatch):
     assert len(made) == 1
 
 
+def test_nothing_is_kept_of_inference_tensors(monkeypatch):
+    """They have no version counter: a write between two calls would go unseen."""
+    made = []
+    monkeypatch.setattr(ops, "pack", lambda val, *a: made.append(val) or torch.zeros(1))
+    with torch.inference_mode():
+        gnm = _weight(torch.zeros(12), torch.zeros(6, dtype=torch.int16))
+    for _ in range(2):
+        gnm.packed()
+    assert len(made) == 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("tokens", [16, 300, 1400])
+def test_products_of_a_weight_made_under_inference_mode(tokens, dtype):
+    dev, M, K = torch.device("cuda", 0), 256, 512
+    with torch.inference_mode():
+        w = GroupedNMTensor.from_dense(torch.randn(M, K, device=dev).to(dtype), 2, 4, 0, 16, 1)
+        x = torch.randn(tokens, K, device=dev).to(dtype)
+        for _ in range(3):
+            w.val.mul_(1.5)
+            want = x.double() @ w.to_dense().double().t()
+            assert _rel(w.native().linear(w, x, None, 0, None), want) < 1e-2
+            assert _rel(w.native().mm(w, x[:8].t()), want[:8].t()) < 1e-2
+            assert _rel(w.native().mm(w, x.t()), want.t()) < 1e-2
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("tokens", [16, 300, 1500])
@@ -70,10 +101,6 @@ def _captured(fn, device=torch.device("cuda", 0)):
     with torch.cuda.graph(graph):
         out = fn()
     return graph, out
-
-
-def _rel(a, b):
-    return float((a.double() - b).norm() / b.norm())
 
 
 @pytest.mark.gpu

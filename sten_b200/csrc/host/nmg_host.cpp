@@ -98,6 +98,12 @@ std::string shape_str(c10::IntArrayRef s) {
     return r + (s.size() == 1 ? ",)" : ")");
 }
 
+// Every kernel reads a bias of `feats` elements.
+void check_bias(const at::Tensor &bias, int64_t feats) {
+    if (bias.defined() && (bias.numel() != feats || (bias.dim() > 1 && bias.size(-1) != feats)))
+        py_raise(PyExc_ValueError, "bias must have one element per output feature (" + std::to_string(feats) + "), got shape " + shape_str(bias.sizes()));
+}
+
 // contiguous() with the call skipped where it would return the tensor itself
 at::Tensor packed_rows(const at::Tensor &t) { return t.is_contiguous() ? t : t.contiguous(); }
 
@@ -226,6 +232,7 @@ PyObject *py_spmm(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     const int code = dtype_code(val);
     if (act0.scalar_type() != val.scalar_type() || (bias.defined() && bias.scalar_type() != val.scalar_type()))
         py_raise(PyExc_TypeError, std::string("activation / bias dtype must match the weight dtype ") + c10::toString(val.scalar_type()));
+    check_bias(bias, geo.M);
     const c10::cuda::CUDAGuard guard(dev);
     const Rows act = row_major_2d(act0);
     const bool token_major = layout != NMG_ACT_K_MAJOR, out_tm = layout == NMG_ACT_TOKEN_MAJOR;
@@ -592,6 +599,7 @@ PyObject *handle_linear(PyObject *self, PyObject *const *a, Py_ssize_t nargs) {
     const int code = dtype_code(val);
     if (x.scalar_type() != val.scalar_type() || (bias.defined() && bias.scalar_type() != val.scalar_type()))
         py_raise(PyExc_TypeError, std::string("activation / bias dtype must match the weight dtype ") + c10::toString(val.scalar_type()));
+    check_bias(bias, geo.M);
     const c10::cuda::CUDAGuard guard(dev);
     const Rows act = rows_of(x, geo.K);
     c10::DimVector sizes(x.sizes().begin(), x.sizes().end());

@@ -125,6 +125,11 @@ def perfect_nm_densify(val, idx, n, m, sparse_dim, size):
     return dense
 
 
+def _check_bias(bias, feats):
+    if bias is not None and (bias.numel() != feats or (bias.dim() > 1 and bias.shape[-1] != feats)):
+        raise ValueError(f"bias must have one element per output feature ({feats}), got shape {tuple(bias.shape)}")
+
+
 def _row_major_2d(t):
     """(tensor, leading dimension) of a 2-D operand with unit stride along its rows."""
     if t.dim() != 2:
@@ -188,6 +193,7 @@ def spmm_expanded(expanded, M, K, act, bias=None, activation=None, residual=None
     """act [tokens, K] -> out [tokens, M] = activation(act @ W^T + bias) + residual from a kept expanded weight."""
     dev = _require_cuda(expanded, act, bias, residual)
     code = _dtype_code(act)
+    _check_bias(bias, M)
     act, ld_act = _row_major_2d(act)
     tokens = act.shape[0]
     if out is None:
@@ -215,6 +221,7 @@ def spmm_replicated(val, idx, M, K, n, m, g, act, out_ptrs, ld_out, bias=None, m
     code = _dtype_code(val)
     if act.dtype != val.dtype or (bias is not None and bias.dtype != val.dtype):
         raise TypeError(f"activation / bias dtype must match the weight dtype {val.dtype}")
+    _check_bias(bias, M)
     act, ld_act = _row_major_2d(act)
     tokens = act.shape[0]
     if act.shape[1] != K:

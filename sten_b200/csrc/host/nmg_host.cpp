@@ -139,7 +139,19 @@ at::Tensor new_empty(c10::IntArrayRef sizes, at::ScalarType type) {
 struct Geo {
     int64_t M, K;
     int n, m, g;
+    int64_t slots;  // entries of idx; val has n times as many
 };
+Geo make_geo(int64_t M, int64_t K, int n, int m, int g) {
+    const int64_t cc = M > 0 && K > 0 && m > 0 && g > 0 ? nmg_num_patterns(n, m) * g : 0;
+    return Geo{M, K, n, m, g, cc > 0 ? (M + m - 1) / m * ((K + cc - 1) / cc) * cc : 0};  // 0: the library says what is wrong
+}
+// The kernels read `batch` weights' worth of both.
+void check_weight(const Geo &geo, const at::Tensor &val, const at::Tensor &idx, int64_t batch = 1) {
+    if (idx.scalar_type() != at::kShort) py_raise(PyExc_TypeError, std::string("idx must be int16, got ") + c10::toString(idx.scalar_type()));
+    if (val.numel() < batch * geo.slots * geo.n || idx.numel() < batch * geo.slots)
+        py_raise(PyExc_ValueError, "val and idx are smaller than a " + std::to_string(geo.n) + ":" + std::to_string(geo.m) + " weight of shape " + shape_str({geo.M, geo.K}) +
+                                       " with groups of " + std::to_string(geo.g));
+}
 
 void *stream_of(c10::Device dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
 
@@ -160,6 +172,7 @@ struct Epi {
 // out[rows_out][ld_out] = activation(product + bias) + residual; every operand has been checked against the others.
 void call_spmm(const Geo &geo, int code, c10::Device dev, const at::Tensor &val, const at::Tensor &idx, const at::Tensor &packed, const Rows &act,
                int64_t tokens, const at::Tensor &bias, const Epi &epi, const at::Tensor &out, int64_t ld_out, int layout, int algo) {
+    check_weight(geo, val, idx);
     const at::Tensor v = packed_rows(val), i = packed_rows(idx), b = bias.defined() ? packed_rows(bias) : bias;
     const size_t nbytes = nmg_spmm_workspace_bytes(geo.M, geo.K, tokens, geo.n, geo.m, geo.g, code, layout, algo, packed.defined() ? 1 : 0);
     at::Tensor ws;
@@ -184,6 +197,7 @@ void call_spmm(const Geo &geo, int code, c10::Device dev, const at::Tensor &val,
 
 void call_spmm_t(const Geo &geo, int code, c10::Device dev, const at::Tensor &val, const at::Tensor &idx, const at::Tensor &packed, const at::Tensor &sp24,
                  const Rows &dy, const at::Tensor &dx, int algo) {
+    check_weight(geo, val, idx);
     const at::Tensor v = packed_rows(val), i = packed_rows(idx);
     void *st = stream_of(dev);
     at::Tensor ws;
@@ -219,7 +233,7 @@ bool sp24_rows_ok(const Rows &dy) { return reinterpret_cast<uintptr_t>(dy.t.cons
     } catch (const PyRaised &) { return nullptr; } \
     END_HANDLE_TH_ERRORS
 
-Geo geo_args(PyObject *const *a) { return Geo{int_arg(a[0]), int_arg(a[1]), (int)int_arg(a[2]), (int)int_arg(a[3]), (int)int_arg(a[4])}; }
+Geo geo_args(PyObject *const *a) { return make_geo(int_arg(a[0]), int_arg(a[1]), (int)int_arg(a[2]), (int)int_arg(a[3]), (int)int_arg(a[4])); }
 
 // spmm(val, idx, M, K, n, m, g, act, bias, layout, algo, out, packed, activation, residual) -> out
 PyObject *py_spmm(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
@@ -337,7 +351,7 @@ PyObject *gather_values(const Dense3 &d, const at::Tensor &idx0, int n, int m, i
     const at::Tensor &w = d.t;
     const Tiles t = tiles_of(d.B, d.M, d.K, n, m, g);
     const at::Tensor idx = packed_rows(idx0);
-    if (idx.numel() != t.count * t.cc) py_raise(PyExc_ValueError, "idx does not belong to a layout of this shape");
+    if (idx.scalar_type() != at::kShort || idx.numel() != t.count * t.cc) py_raise(PyExc_ValueError, "idx does not belong to a layout of this shape");
     const at::Tensor val = new_empty({t.count, t.C, g, n}, w.scalar_type());
     void *st = stream_of(dev);
     PyThreadState *save = PyEval_SaveThread();
@@ -367,6 +381,7 @@ PyObject *py_densify(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     const int code = dtype_code(val0);
     const int64_t B = int_arg(a[2]);
     const Geo geo = geo_args(a + 3);
+    check_weight(geo, val0, idx0, B);
     const c10::cuda::CUDAGuard guard(dev);
     const at::Tensor val = packed_rows(val0), idx = packed_rows(idx0);
     const at::Tensor out = new_empty({B, geo.M, geo.K}, val.scalar_type());
@@ -377,6 +392,14 @@ PyObject *py_densify(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     PyEval_RestoreThread(save);
     check(rc);
     return THPVariable_Wrap(out);
+    NMG_PY_END
+}
+
+// check_weight(val, idx, M, K, n, m, g): raises unless both hold a weight of this geometry
+PyObject *py_check_weight(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
+    NMG_PY_BEGIN(7)
+    check_weight(geo_args(a + 2), tensor_arg(a[0]), tensor_arg(a[1]));
+    Py_RETURN_NONE;
     NMG_PY_END
 }
 
@@ -547,6 +570,7 @@ at::Tensor derived(Handle *h, KeptCopy *&kept, PyObject *gnm, PyObject *method, 
 
 // A column-ordered copy for this call alone.
 at::Tensor pack_once(const Geo &geo, int code, c10::Device dev, const at::Tensor &val, const at::Tensor &idx) {
+    check_weight(geo, val, idx);
     const at::Tensor v = packed_rows(val), i = packed_rows(idx);
     const size_t nbytes = nmg_packed_bytes(geo.M, geo.K, geo.n, geo.m, geo.g, code);
     at::Tensor buf = new_empty({(int64_t)nbytes}, at::kByte);
@@ -574,7 +598,7 @@ PyObject *handle_new(PyTypeObject *type, PyObject *args, PyObject *) {
     if (!PyArg_ParseTuple(args, "LLiii", &M, &K, &n, &m, &g)) return nullptr;
     Handle *h = reinterpret_cast<Handle *>(type->tp_alloc(type, 0));
     if (!h) return nullptr;
-    h->geo = Geo{M, K, n, m, g};
+    h->geo = make_geo(M, K, n, m, g);
     h->packed = h->sp24 = nullptr;
     h->held = new std::vector<at::Tensor>();
     return reinterpret_cast<PyObject *>(h);
@@ -876,6 +900,7 @@ PyMethodDef module_methods[] = {
     NMG_METHOD("column_sum", py_column_sum),
     NMG_METHOD("densify", py_densify),
     NMG_METHOD("capturing", py_capturing),
+    NMG_METHOD("check_weight", py_check_weight),
     NMG_METHOD("set_dispatch", py_set_dispatch),
     NMG_METHOD("repeat_call", py_repeat_call),
     {"set_error_class", py_set_error_class, METH_O, nullptr},

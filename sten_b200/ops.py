@@ -143,6 +143,7 @@ def pack(val, idx, M, K, n, m, g):
     """Column-ordered device copy of a weight (opaque uint8 buffer) for the tensor-core and transposed kernels."""
     dev = _require_cuda(val, idx)
     code = _dtype_code(val)
+    nat.host().check_weight(val, idx, M, K, n, m, g)
     val, idx = val.contiguous(), idx.contiguous()
     L = nat.lib()
     nbytes = L.nmg_packed_bytes(M, K, n, m, g, code)
@@ -182,6 +183,7 @@ def expand(val, idx, M, K, n, m, g):
     nbytes = nat.lib().nmg_expanded_bytes(M, K, n, m, g, code)
     if nbytes == 0:
         return None
+    nat.host().check_weight(val, idx, M, K, n, m, g)
     val, idx = val.contiguous(), idx.contiguous()
     buf = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     with torch.cuda.device(dev):
@@ -226,6 +228,7 @@ def spmm_replicated(val, idx, M, K, n, m, g, act, out_ptrs, ld_out, bias=None, m
     tokens = act.shape[0]
     if act.shape[1] != K:
         raise ValueError(f"activation shape {tuple(act.shape)} does not match K={K}")
+    nat.host().check_weight(val, idx, M, K, n, m, g)
     val, idx = val.contiguous(), idx.contiguous()
     if bias is not None:
         bias = bias.contiguous()
@@ -256,6 +259,7 @@ def pack_sp24(val, idx, M, K, n, m, g):
     nbytes = sp24_bytes(M, K, n, m, g, val.dtype)
     if nbytes == 0:
         raise ValueError("this weight is outside the 2:4 structure (needs a 16-bit dtype, n <= 2 and m in {4, 8, 16, 32, 64})")
+    nat.host().check_weight(val, idx, M, K, n, m, g)
     val, idx = val.contiguous(), idx.contiguous()
     buf = torch.empty(nbytes, dtype=torch.uint8, device=dev)
     with torch.cuda.device(dev):

@@ -11,6 +11,7 @@
 #include <atomic>
 
 #include "../../include/nmg_b200.h"
+#include "nmg_limit.h"
 
 namespace nmg {
 
@@ -97,14 +98,14 @@ constexpr int kMaxDevices = 64;
 // Raise a kernel's dynamic shared-memory limit on the current device; the runtime call (about 0.5 us) is made only when a
 // launch needs more than any launch of that kernel on that device before it.
 template <auto Kernel> inline int allow_smem(size_t bytes) {
-    static std::atomic<int> have[kMaxDevices];
+    static GrowingLimit limit[kMaxDevices];
     int dev = 0;
     NMG_CUDA(cudaGetDevice(&dev));
-    if (dev >= kMaxDevices || have[dev].load(std::memory_order_relaxed) < (int)bytes) {
-        NMG_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-        if (dev < kMaxDevices) have[dev].store((int)bytes, std::memory_order_relaxed);
-    }
-    return NMG_OK;
+    auto set = [](int v) -> int {
+        NMG_CUDA(cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, v));
+        return NMG_OK;
+    };
+    return dev < kMaxDevices ? limit[dev].ensure((int)bytes, set) : set((int)bytes);
 }
 #define NMG_ALLOW_SMEM(bytes, ...)                                              \
     do {                                                                        \

@@ -758,7 +758,11 @@ PyObject *handle_linear_grads(PyObject *self, PyObject *const *a, Py_ssize_t nar
         }
         PyTuple_SetItem(r, 1, in_layout ? gather_values(Dense3{dw, 1, geo.M, geo.K, geo.K, geo.M * geo.K}, idx, geo.n, geo.m, geo.g, code, dev) : THPVariable_Wrap(dw));
     }
-    if (needs & 4) PyTuple_SetItem(r, 2, THPVariable_Wrap(column_sums(dy, code, dev)));
+    if (needs & 4) {
+        // a backward pass that is recorded itself (create_graph) needs db's dependence on dy
+        const bool recorded = c10::GradMode::is_enabled() && dy0.requires_grad();
+        PyTuple_SetItem(r, 2, THPVariable_Wrap(recorded ? dy0.reshape({-1, geo.M}).sum(0) : column_sums(dy, code, dev)));
+    }
     return Py_NewRef(r);
     NMG_PY_END
 }

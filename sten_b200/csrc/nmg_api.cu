@@ -78,7 +78,10 @@ static size_t kmajor_transpose_bytes(const Geo &geo, int dtype, int64_t tokens) 
 }
 // Fewer than 64 columns do not pay for re-ordering the weight on every call; with a packed copy in hand they take the tensor
 // cores like any other batch (192 x 3200 f16, 2 columns: 7 us against 229 us in the gather kernel).
-static bool kmajor_few(int layout, int64_t tokens, bool have_packed) { return layout == NMG_ACT_K_MAJOR && tokens < 64 && !have_packed; }
+// In fp32 only the fused kernel sums as accurately as the gather kernel does (see chunk_kb).
+static bool kmajor_few(const Geo &geo, int dtype, int layout, int64_t tokens, bool have_packed) {
+    return layout == NMG_ACT_K_MAJOR && tokens < 64 && !(have_packed && (dtype != NMG_F32 || tc_supported(geo, dtype)));
+}
 
 extern "C" size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype,
                                            int layout, int algo, int have_packed) {
@@ -93,7 +96,7 @@ extern "C" size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens,
                  tc_split_workspace_bytes(geo, dtype, false, tokens) +
                  (layout == NMG_ACT_K_MAJOR ? kmajor_transpose_bytes(geo, dtype, tokens) : algo == NMG_ALGO_AUTO ? pad_rows_bytes(dtype, tokens, K) : 0);
     // AUTO: the gather kernels serve what the tensor cores do not, and a handful of K-major columns without a packed copy
-    const bool simt_runs = algo == NMG_ALGO_SIMT || (algo == NMG_ALGO_AUTO && (!tensor_runs || kmajor_few(layout, tokens, have_packed != 0)));
+    const bool simt_runs = algo == NMG_ALGO_SIMT || (algo == NMG_ALGO_AUTO && (!tensor_runs || kmajor_few(geo, dtype, layout, tokens, have_packed != 0)));
     const size_t simt = simt_runs ? simt_fwd_workspace_bytes(geo, tokens, dtype, layout) : 0;
     return simt > tensor ? simt : tensor;
 }
@@ -118,7 +121,7 @@ static int spmm_impl(const void *val, const int16_t *idx, const void *packed, in
         NMG_FAIL(NMG_ERR_INVALID, "unknown algo %d", algo);
     if (algo == NMG_ALGO_TENSOR_DENSE) algo = NMG_ALGO_TENSOR;  // the forward product has no structured-sparse variant
     cudaStream_t st = (cudaStream_t)stream;
-    const bool tensor = algo == NMG_ALGO_TENSOR || (algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, M) && !kmajor_few(layout, tokens, packed != nullptr));
+    const bool tensor = algo == NMG_ALGO_TENSOR || (algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, M) && !kmajor_few(geo, dtype, layout, tokens, packed != nullptr));
     if (algo == NMG_ALGO_TENSOR && (!any_tensor(geo, dtype) || (tm && !rows_aligned(dtype, act, ld_act)) || (!tm && n_outs > 1)))
         NMG_FAIL(NMG_ERR_UNSUPPORTED, "tensor-core path needs activation rows that are 16-byte aligned (16-bit dtypes) and a chunk that fits shared memory");
     // AUTO: tensor cores whenever the weight has at least 64 rows, at every token count.  fp32 on tensor cores means exact bf16

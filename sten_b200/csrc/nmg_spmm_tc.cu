@@ -53,6 +53,7 @@ struct TcParams {
     int exch_off;         // exchange area of the partial tiles: offset in shared memory; 0 = on top of the rings
     int misc_off;         // selector table and barriers
     uint32_t tmem_cols;
+    int chunk_kb;         // fp32: k-blocks per accumulation chunk
     int *status;
 };
 struct FxMaps {
@@ -374,7 +375,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
     const int kb_per = (nkb_all + ks - 1) / ks;
     const int kb_base = split * kb_per;  // this CTA's first k-block
     const int nkb = (nkb_all < kb_base + kb_per ? nkb_all : kb_base + kb_per) - kb_base;  // >= 1 by the host's choice of ksplit
-    const int chunk_kb = SPLIT ? TC_CHUNK_KB : nkb;  // k-blocks per accumulation chunk
+    const int chunk_kb = SPLIT ? prm.chunk_kb : nkb;  // k-blocks per accumulation chunk
     const int nchunks = (nkb + chunk_kb - 1) / chunk_kb;
     const uint32_t tmem_cols = prm.tmem_cols;
     const int cols_live = (int)(prm.ntok - tok0 < bn ? prm.ntok - tok0 : bn);  // token columns of this tile that exist
@@ -517,8 +518,9 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
                 const uint64_t bs = bdesc0 + (uint64_t)(uint32_t)(s * (x_bytes >> 4));
 #pragma unroll
                 for (int t = 0; t < TcMode<T>::TERMS; t++) {
-                    const uint32_t at = at0 + (uint32_t)((SPLIT ? split_w(t) : 0) * FX_A_COLS);
-                    const uint64_t bt = bs + (uint64_t)(uint32_t)((SPLIT ? split_x(t) : 0) * (b_bytes >> 4));
+                    const int st = TcMode<T>::TERMS - 1 - t;  // smallest product first: its rounding is that of a small sum
+                    const uint32_t at = at0 + (uint32_t)((SPLIT ? split_w(st) : 0) * FX_A_COLS);
+                    const uint64_t bt = bs + (uint64_t)(uint32_t)((SPLIT ? split_x(st) : 0) * (b_bytes >> 4));
 #pragma unroll
                     for (int k = 0; k < TC_BK / 16; k++)  // 16 elements = 8 TMEM columns of A, 32 bytes = 2 descriptor units of B
                         tc_mma_f16_ta(d_tmem, at + 8 * k, bt + 2 * k, idesc, (first && t == 0 && k == 0) ? 0u : 1u);
@@ -889,6 +891,11 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     p.out_vec = out_token_major ? (ld_out % 2 == 0 && feats % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0)
                                 : (ld_out * es % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0);
     p.tiles_f = fx.tiles_f; p.tiles_t = fx.tiles_t; p.bn = fx.bn; p.ksplit = fx.ksplit;
+    // A handful of K-major fp32 columns is otherwise served by the gather kernels' fp32 FMAs.  With a chunk per k-block and the
+    // products added smallest first the error is below theirs at every size: K = 256 / 1024 / 16384, 2:4 0.7 / 0.9 / 1.4e-7 against
+    // 2.0 / 4.0 / 16.6e-7, 1:16 0.6 / 0.8 / 1.3e-7 against 0.8 / 1.5 / 5.8e-7 (chunks of 8, largest first: 11 / 11 / 35e-7 and
+    // 7 / 7 / 21e-7).  It costs 8 of 29 us at 4096 x 4096, nothing at K = 1024 and below.
+    p.chunk_kb = act_k_major && tokens < 64 ? 1 : TC_CHUNK_KB;
     p.masks = masks; p.mask_rows = natural_mask_rows(geo); p.nb = geo.nb;
     p.status = status;
     const ProfileEvents pe = take_profile_events();

@@ -256,14 +256,14 @@ __device__ __forceinline__ float gelu_erf(float v) {
 
 // fp32 operands run on the bf16 tensor cores as exact three-way splits x = xh + xm + xl, w = wh + wm + wl.  The
 // product keeps the six terms whose weight is >= 2^-16 of the leading one (wh xh, wm xh, wh xm, wm xm, wl xh, wh xl);
-// the dropped terms are below 2^-24 relative, the size of an fp32 rounding error.  Each term is one more pass
-// over the reduction axis with another pair of planes, accumulated in the same fp32 TMEM tile.
+// the dropped terms are below 2^-24 relative, the size of an fp32 rounding error.  Each term is one more MMA
+// per k-step with another pair of planes, accumulated in the same fp32 TMEM tile.
 //
 // The tensor core's fp32 accumulator truncates instead of rounding, which biases long sums: measured relative error
 // grows linearly with the reduction length (3.5e-6 at K = 512, 2.6e-5 at K = 4096).  fp32 mode therefore keeps a
-// second accumulator tile in TMEM: every TC_CHUNK_KB k-blocks the first expansion group adds the tensor core's
-// partial tile into it with round-to-nearest FADDs (tcgen05.ld / tcgen05.st), and the MMAs restart from zero.  The
-// error then no longer depends on K.
+// running sum outside the tensor core: every TC_CHUNK_KB k-blocks the partial tile is added to it with round-to-nearest FADDs
+// (fused kernel: a second accumulator tile in TMEM, by all twelve warps; two-pass kernel: registers of the drain warps) and the
+// MMAs restart from zero.  The error then no longer depends on K.
 template <typename T> struct TcMode { using elem = T; static constexpr int TERMS = 1; };
 template <> struct TcMode<float> { using elem = __nv_bfloat16; static constexpr int TERMS = 6; };
 __host__ __device__ constexpr int split_w(int t) { return t == 1 || t == 3 ? 1 : t == 4 ? 2 : 0; }  // planes of product t

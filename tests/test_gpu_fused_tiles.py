@@ -79,3 +79,21 @@ def test_k_major_columns(tokens, dtype, tol):
         c = torch.mm(w, b)
     want = w.wrapped_tensor.to_dense().double() @ b.double()
     assert float((c.double() - want).norm() / want.norm()) <= tol
+
+
+@pytest.mark.parametrize("n,m", [(1, 4), (2, 4), (1, 8), (2, 8), (1, 16)])
+@pytest.mark.parametrize("K,tokens", [(256, 1), (256, 63), (1000, 8), (4096, 33), (16384, 63)])
+def test_few_fp32_columns_are_summed_as_accurately_as_by_fp32_fmas(n, m, K, tokens):
+    """torch.mm of a handful of columns runs on the tensor cores when a packed copy is there, and on fp32 FMAs when it is not."""
+    from sten_b200 import _native as nat, ops
+    dev, M = cuda(), 256
+    w = (seeded_normal((M, K), 1) * K ** -0.5).to(dev)
+    val, idx = ops.sparsify(w.unsqueeze(0), n, m, 4)
+    b = seeded_normal((K, tokens), 2).to(dev)
+    want = ops.densify(val, idx, 1, M, K, n, m, 4)[0].double() @ b.double()
+    err = lambda c: float((c.double() - want).norm() / want.norm())  # noqa: E731
+    packed = ops.pack(val, idx, M, K, n, m, 4)
+    tensor = ops.spmm(val, idx, M, K, n, m, 4, b, layout=nat.NMG_ACT_K_MAJOR, packed=packed)
+    fma = ops.spmm(val, idx, M, K, n, m, 4, b, layout=nat.NMG_ACT_K_MAJOR, algo=nat.NMG_ALGO_SIMT)
+    assert not torch.equal(tensor, fma)
+    assert err(tensor) <= err(fma)

@@ -54,3 +54,17 @@ def test_column_sums(rows, cols, off, dtype, tol):
     got, want = nat.host().column_sum(x), x.double().sum(0)
     assert got.dtype == dtype and float((got.double() - want).norm() / want.norm()) <= tol
     assert torch.equal(nat.host().column_sum(x), got)
+
+
+@pytest.mark.parametrize("rows", [1, 100, 1000, 4096, 70000])
+def test_fp32_column_sums_err_no_more_than_a_torch_reduction(rows):
+    from sten_b200 import _native as nat
+    for x in (seeded_normal((rows, 512), 5) + 0.3, seeded_normal((rows, 512), 6), seeded_normal((rows, 512), 7).abs()):
+        x = x.to(cuda())
+        got, want = nat.host().column_sum(x).double(), x.double().sum(0)
+        assert float((got - want).norm()) <= float((x.sum(0).double() - want).norm())
+    for bad, expect in ((float("inf"), float("inf")), (-float("inf"), -float("inf")), (float("nan"), float("nan"))):
+        y = x.clone()
+        y[rows // 2, 7] = bad
+        s = nat.host().column_sum(y)
+        assert torch.equal(s[8:], nat.host().column_sum(x)[8:]) and np.array_equal(np_of(s[7:8]), np.float32([expect]), equal_nan=True)

@@ -246,7 +246,7 @@ template <> __device__ __forceinline__ uint16_t bits16<float>(float) { return 0;
 // carries the halved coefficients: fourteen instructions, two of them on the special-function unit (flush-to-zero forms, which
 // need no range fix-up), against the library erf's thirty.  The drain warps apply it to 128 x 256 values per tile.
 __device__ __forceinline__ float gelu_erf(float v) {
-    const float av = fabsf(v);
+    const float av = fabsf(fminf(v, 1e30f));  // +inf: the second factor below is 0 then, and the first must not be infinite
     float t, e;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.23164189f, av, 1.f)));   // p / sqrt(2)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"((v * -0.72134752f) * v));          // log2(e) / 2

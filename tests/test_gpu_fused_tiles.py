@@ -97,3 +97,22 @@ def test_few_fp32_columns_are_summed_as_accurately_as_by_fp32_fmas(n, m, K, toke
     fma = ops.spmm(val, idx, M, K, n, m, 4, b, layout=nat.NMG_ACT_K_MAJOR, algo=nat.NMG_ALGO_SIMT)
     assert not torch.equal(tensor, fma)
     assert err(tensor) <= err(fma)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("tokens", [3, 300, 2000])
+def test_gelu_of_infinities_and_nan(tokens, dtype):
+    """As torch's exact GELU has them: infinity stays, minus infinity and NaN give NaN; large finite values pass through."""
+    from sten_b200 import _native as nat, ops
+    M, K = 256, 128
+    w = (seeded_normal((M, K), 1) * K ** -0.5).to(dtype).to(cuda())
+    val, idx = ops.sparsify(w.unsqueeze(0), 2, 4, 16)
+    x = seeded_normal((tokens, K), 2).to(dtype).to(cuda())
+    bias = torch.zeros(M, dtype=dtype, device=cuda())
+    big = 6e4 if dtype == torch.float16 else 3e38
+    bias[:5] = torch.tensor([float("inf"), -float("inf"), float("nan"), big, -big], dtype=dtype)
+    for algo in (nat.NMG_ALGO_AUTO, nat.NMG_ALGO_SIMT):
+        y = ops.spmm(val, idx, M, K, 2, 4, 16, x, bias=bias, activation="gelu", algo=algo)[:, :5].float()
+        want = torch.nn.functional.gelu(bias[:5].double()).float().expand(tokens, 5)
+        assert torch.equal(y.isnan(), want.isnan())
+        assert torch.equal(y[:, 0], want[:, 0]) and float((y[:, 3] / want[:, 3] - 1).abs().max()) < 1e-2 and float(y[:, 4].abs().max()) == 0

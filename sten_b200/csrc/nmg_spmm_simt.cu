@@ -54,23 +54,26 @@ __global__ void __launch_bounds__(256) transpose_kernel(const uint16_t *__restri
     __shared__ uint16_t tile[64][66];
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the matmul's set-up may overlap this pass
     const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-    const int64_t c0 = (int64_t)blockIdx.x * 64, r0 = (int64_t)blockIdx.y * 64;
-    for (int i = ty; i < 64; i += 8) {
-        const int64_t r = r0 + i;
+    const int64_t c0 = (int64_t)blockIdx.x * 64;
+    for (int64_t r0 = (int64_t)blockIdx.y * 64; r0 < ld_dst; r0 += (int64_t)gridDim.y * 64) {
+        __syncthreads();  // the previous tile has been written out
+        for (int i = ty; i < 64; i += 8) {
+            const int64_t r = r0 + i;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int64_t c = c0 + 2 * tx + h;
-            tile[i][2 * tx + h] = (r < rows && c < cols) ? src[r * ld_src + c] : (uint16_t)0;
+            for (int h = 0; h < 2; h++) {
+                const int64_t c = c0 + 2 * tx + h;
+                tile[i][2 * tx + h] = (r < rows && c < cols) ? src[r * ld_src + c] : (uint16_t)0;
+            }
         }
-    }
-    __syncthreads();
-    for (int i = ty; i < 64; i += 8) {
-        const int64_t c = c0 + i;
-        if (c >= cols) continue;
+        __syncthreads();
+        for (int i = ty; i < 64; i += 8) {
+            const int64_t c = c0 + i;
+            if (c >= cols) continue;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
-            const int64_t r = r0 + 2 * tx + h;
-            if (r < ld_dst) dst[c * ld_dst + r] = tile[2 * tx + h][i];
+            for (int h = 0; h < 2; h++) {
+                const int64_t r = r0 + 2 * tx + h;
+                if (r < ld_dst) dst[c * ld_dst + r] = tile[2 * tx + h][i];
+            }
         }
     }
 }
@@ -78,8 +81,7 @@ __global__ void __launch_bounds__(256) transpose_kernel(const uint16_t *__restri
 int launch_transpose(const void *src, int64_t rows, int64_t cols, int64_t ld_src, void *dst, int64_t ld_dst, cudaStream_t st) {
     dim3 block(32, 8);
     const int64_t gy = (ld_dst + 63) / 64;
-    if (gy > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "reduction axis too long for the transpose pre-pass");
-    dim3 grid((unsigned)((cols + 63) / 64), (unsigned)gy);
+    dim3 grid((unsigned)((cols + 63) / 64), (unsigned)(gy < 65535 ? gy : 65535));
     transpose_kernel<<<grid, block, 0, st>>>(static_cast<const uint16_t *>(src), rows, cols, ld_src, static_cast<uint16_t *>(dst), ld_dst);
     NMG_CUDA(cudaGetLastError());
     return NMG_OK;

@@ -144,31 +144,33 @@ __global__ void __launch_bounds__(256) build_masks_kernel(const uint8_t *__restr
     __shared__ int8_t table[31 * 16];  // row -> slot of every pattern; at most 28 patterns of up to 16 rows
     for (int i = threadIdx.x; i < patterns * m; i += blockDim.x) table[i] = slot_of_row[i];
     __syncthreads();
-    const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, kb = blockIdx.y;
+    const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (row >= rows) return;
-    uint32_t mask[2][2] = {{0, 0}, {0, 0}};
-    if (row < M) {
-        const int64_t mb = row / m;
-        const int r = (int)(row - mb * m);
-        const uint4 *src = reinterpret_cast<const uint4 *>(pat + mb * Kp + kb * 64);
+    for (int64_t kb = blockIdx.y; kb < Kp / 64; kb += gridDim.y) {
+        uint32_t mask[2][2] = {{0, 0}, {0, 0}};
+        if (row < M) {
+            const int64_t mb = row / m;
+            const int r = (int)(row - mb * m);
+            const uint4 *src = reinterpret_cast<const uint4 *>(pat + mb * Kp + kb * 64);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint4 v = __ldg(src + i);
-            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+            for (int i = 0; i < 4; i++) {
+                const uint4 v = __ldg(src + i);
+                const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int c = 0; c < 16; c++) {
-                const int col = i * 16 + c, bit = 8 * (col & 3) + ((col & 31) >> 2);
-                // the byte is pattern * m: where the pattern's row table starts
-                const int s = table[((w[c >> 2] >> (8 * (c & 3))) & 0xffu) + r];
-                if (s == 0) mask[0][col >> 5] |= 1u << bit;
-                if (s == 1) mask[1][col >> 5] |= 1u << bit;
+                for (int c = 0; c < 16; c++) {
+                    const int col = i * 16 + c, bit = 8 * (col & 3) + ((col & 31) >> 2);
+                    // the byte is pattern * m: where the pattern's row table starts
+                    const int s = table[((w[c >> 2] >> (8 * (c & 3))) & 0xffu) + r];
+                    if (s == 0) mask[0][col >> 5] |= 1u << bit;
+                    if (s == 1) mask[1][col >> 5] |= 1u << bit;
+                }
             }
         }
+        uint32_t *dst = masks + (kb * rows + row) * 2 * n;
+        dst[0] = mask[0][0];
+        dst[1] = mask[0][1];
+        if (n == 2) { dst[2] = mask[1][0]; dst[3] = mask[1][1]; }
     }
-    uint32_t *dst = masks + (kb * rows + row) * 2 * n;
-    dst[0] = mask[0][0];
-    dst[1] = mask[0][1];
-    if (n == 2) { dst[2] = mask[1][0]; dst[3] = mask[1][1]; }
 }
 
 static bool bwd_specialised(int n, int m) {
@@ -243,8 +245,7 @@ int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16
         int rc = get_pattern_table(geo.n, geo.m, &tab);
         if (rc) return rc;
         const int64_t rows = natural_mask_rows(geo), kbs = natural_width(geo) / 64;
-        if (kbs > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "weight has too many columns for the column-ordered copy");
-        build_masks_kernel<<<dim3((unsigned)((rows + 255) / 256), (unsigned)kbs), 256, 0, st>>>(
+        build_masks_kernel<<<dim3((unsigned)((rows + 255) / 256), (unsigned)(kbs < 65535 ? kbs : 65535)), 256, 0, st>>>(
             static_cast<const uint8_t *>(pat), tab.slot_of_row, reinterpret_cast<uint32_t *>(static_cast<char *>(nval) + lay.val_bytes), geo.M, natural_width(geo), rows, geo.n, geo.m, geo.C);
     }
     NMG_CUDA(cudaGetLastError());

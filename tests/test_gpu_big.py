@@ -125,3 +125,21 @@ def test_sharded_benchmark_configuration_at_full_size():
     cols = _sampled_rows(K, 256, 8)
     assert _rel(dx[:, cols], x.double() @ dense[:, cols].double()) <= TOL_HALF
     assert ops.read_status() == 0
+
+
+def test_more_columns_than_a_grid_has_blocks():
+    """67200 k-blocks of 64 columns: the row masks of the packed copy and the transpose pre-pass stride over them."""
+    from sten_b200 import ops
+    from sten_b200.grouped_nm_tensor import GroupedNMTensor
+    dev, M, K = torch.device("cuda", 0), 64, 4_300_800
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    w = GroupedNMTensor.from_dense(torch.randn(M, K, device=dev, dtype=torch.bfloat16, generator=gen), 1, 4, 0, 16, 1)
+    x = torch.randn(8, K, device=dev, dtype=torch.bfloat16, generator=gen)
+    dy = torch.randn(8, M, device=dev, dtype=torch.bfloat16, generator=gen)
+    dense = w.to_dense().double()
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm())  # noqa: E731
+    want = x.double() @ dense.t()
+    assert rel(w.native().linear(w, x, None, 0, None), want) < 1e-2
+    assert rel(w.native().mm(w, x.t().contiguous()), want.t()) < 1e-2
+    assert rel(w.native().linear_t(w, dy, ops.SP24_MIN_TOKENS), dy.double() @ dense) < 1e-2
+    assert ops.read_status() == 0

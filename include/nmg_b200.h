@@ -122,7 +122,9 @@ int nmg_pack(const void *val, const int16_t *idx, int64_t M, int64_t K, int n, i
  *   layout NMG_ACT_TOKEN_MAJOR_OUT_ROWS: act as TOKEN_MAJOR, out as K_MAJOR
  * act, out, val and bias share `dtype`; accumulation is fp32.  bias may be NULL.
  * packed: result of nmg_pack for the same weight, or NULL (then it is built in the workspace when the chosen kernel
- * needs it).  have_packed in the workspace query says which of the two the caller will do.
+ * needs it).  `given` in the workspace query says what the caller will bring along: NMG_GIVEN_PACKED, the packed copy;
+ * NMG_GIVEN_ALIGNED_ROWS, an activation (gradient) whose base is 16-byte aligned and whose pitch is a multiple of 8, for which
+ * no room to lay it out again is needed.
  * workspace: device scratch of at least nmg_spmm_workspace_bytes(...) bytes, 256-byte aligned, owned by the
  * caller for the duration of the call (may be NULL when the query returns 0).
  * algo: NMG_ALGO_AUTO uses the tensor cores for weights of at least 64 rows, at every token count (16-bit rows that are not
@@ -134,8 +136,9 @@ int nmg_pack(const void *val, const int16_t *idx, int64_t M, int64_t K, int n, i
  * variant reads val / idx and ignores `packed`.  fp32 operands go through the tensor cores as exact three-way bf16
  * splits with promoted fp32 accumulation (relative error ~3.5e-6, independent of K); NMG_ALGO_SIMT forces plain fp32
  * FMA arithmetic. */
+typedef enum { NMG_GIVEN_PACKED = 1, NMG_GIVEN_ALIGNED_ROWS = 2 } nmg_given;
 size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype,
-                                int layout, int algo, int have_packed);
+                                int layout, int algo, int given);
 int nmg_spmm(const void *val, const int16_t *idx, const void *packed, int64_t M, int64_t K, int n, int m, int g,
              int dtype, const void *act, int64_t ld_act, int64_t tokens, const void *bias, void *out,
              int64_t ld_out, int layout, int algo, void *workspace, size_t workspace_bytes, void *stream);
@@ -162,7 +165,7 @@ int nmg_spmm_fused(const void *val, const int16_t *idx, const void *packed, int6
  * workspace (two values + two 2-bit positions per group of four rows) and run tcgen05.mma.sp, structured-sparse MMA at
  * twice the dense rate.  fp32 weights, other patterns and fewer tokens use the dense-rate kernels described above. */
 size_t nmg_spmm_t_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype,
-                                  int algo, int have_packed);
+                                  int algo, int given);
 int nmg_spmm_t(const void *val, const int16_t *idx, const void *packed, int64_t M, int64_t K, int n, int m, int g,
                int dtype, const void *dy, int64_t ld_dy, int64_t tokens, void *dx, int64_t ld_dx, int algo,
                void *workspace, size_t workspace_bytes, void *stream);

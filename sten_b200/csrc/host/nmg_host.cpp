@@ -169,12 +169,15 @@ struct Epi {
     int64_t ld = 0;
 };
 
+bool rows_aligned(const Rows &r) { return reinterpret_cast<uintptr_t>(r.t.const_data_ptr()) % 16 == 0 && r.ld % 8 == 0; }
+int given(const at::Tensor &packed, const Rows &rows) { return (packed.defined() ? NMG_GIVEN_PACKED : 0) | (rows_aligned(rows) ? NMG_GIVEN_ALIGNED_ROWS : 0); }
+
 // out[rows_out][ld_out] = activation(product + bias) + residual; every operand has been checked against the others.
 void call_spmm(const Geo &geo, int code, c10::Device dev, const at::Tensor &val, const at::Tensor &idx, const at::Tensor &packed, const Rows &act,
                int64_t tokens, const at::Tensor &bias, const Epi &epi, const at::Tensor &out, int64_t ld_out, int layout, int algo) {
     check_weight(geo, val, idx);
     const at::Tensor v = packed_rows(val), i = packed_rows(idx), b = bias.defined() ? packed_rows(bias) : bias;
-    const size_t nbytes = nmg_spmm_workspace_bytes(geo.M, geo.K, tokens, geo.n, geo.m, geo.g, code, layout, algo, packed.defined() ? 1 : 0);
+    const size_t nbytes = nmg_spmm_workspace_bytes(geo.M, geo.K, tokens, geo.n, geo.m, geo.g, code, layout, algo, given(packed, act));
     at::Tensor ws;
     if (nbytes) ws = new_empty({(int64_t)nbytes}, at::kByte);
     void *st = stream_of(dev);
@@ -203,7 +206,7 @@ void call_spmm_t(const Geo &geo, int code, c10::Device dev, const at::Tensor &va
     at::Tensor ws;
     size_t nbytes = 0;
     if (!sp24.defined()) {
-        nbytes = nmg_spmm_t_workspace_bytes(geo.M, geo.K, dy.rows, geo.n, geo.m, geo.g, code, algo, packed.defined() ? 1 : 0);
+        nbytes = nmg_spmm_t_workspace_bytes(geo.M, geo.K, dy.rows, geo.n, geo.m, geo.g, code, algo, given(packed, dy));
         if (nbytes) ws = new_empty({(int64_t)nbytes}, at::kByte);
     }
     int rc;
@@ -218,8 +221,6 @@ void call_spmm_t(const Geo &geo, int code, c10::Device dev, const at::Tensor &va
     PyEval_RestoreThread(save);
     check(rc);
 }
-
-bool sp24_rows_ok(const Rows &dy) { return reinterpret_cast<uintptr_t>(dy.t.const_data_ptr()) % 16 == 0 && dy.ld % 8 == 0; }
 
 // ------------------------------------------------------------------------------------------------ module functions
 #define NMG_PY_BEGIN(nargs_wanted)                                                           \
@@ -296,7 +297,7 @@ PyObject *py_spmm_t(PyObject *, PyObject *const *a, Py_ssize_t nargs) {
     const Rows dy = row_major_2d(dy0);
     if (dy.cols != geo.M) py_raise(PyExc_ValueError, "gradient shape " + shape_str(dy0.sizes()) + " does not match M=" + std::to_string(geo.M));
     const at::Tensor dx = new_empty({dy.rows, geo.K}, val.scalar_type());
-    const bool kept = sp24.defined() && dy.rows >= int_arg(a[11]) && (algo == NMG_ALGO_AUTO || algo == NMG_ALGO_TENSOR) && sp24_rows_ok(dy);
+    const bool kept = sp24.defined() && dy.rows >= int_arg(a[11]) && (algo == NMG_ALGO_AUTO || algo == NMG_ALGO_TENSOR) && rows_aligned(dy);
     if (dy.rows > 0) call_spmm_t(geo, code, dev, val, idx, packed, kept ? sp24 : at::Tensor(), dy, dx, algo);
     return THPVariable_Wrap(dx);
     NMG_PY_END
@@ -682,7 +683,7 @@ at::Tensor input_gradient(Handle *h, PyObject *gnm, const at::Tensor &val, const
         // the compressed transposed copy serves the large batches of a 16-bit weight inside the 2:4 structure
         if (dy.rows >= sp24_min_tokens) sp24 = derived(h, h->sp24, gnm, g_s_packed_sp24, val, idx, capturing(dev));
         if (!sp24.defined()) packed = packed_for(h, gnm, val, idx, dy.rows, code, dev, true);
-        call_spmm_t(geo, code, dev, val, idx, packed, sp24.defined() && sp24_rows_ok(dy) ? sp24 : at::Tensor(), dy, dx, NMG_ALGO_AUTO);
+        call_spmm_t(geo, code, dev, val, idx, packed, sp24.defined() && rows_aligned(dy) ? sp24 : at::Tensor(), dy, dx, NMG_ALGO_AUTO);
     }
     return dx;
 }

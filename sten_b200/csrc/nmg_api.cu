@@ -84,19 +84,20 @@ static bool kmajor_few(const Geo &geo, int dtype, int layout, int64_t tokens, bo
 }
 
 extern "C" size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype,
-                                           int layout, int algo, int have_packed) {
+                                           int layout, int algo, int given) {
+    const bool have_packed = (given & ~NMG_GIVEN_ALIGNED_ROWS) != 0, aligned = (given & NMG_GIVEN_ALIGNED_ROWS) != 0;
     Geo geo;
     if (make_geo(M, K, n, m, g, &geo) || tokens < 1 || n < 1) return 0;
     if (algo == NMG_ALGO_TENSOR_DENSE) algo = NMG_ALGO_TENSOR;
     size_t tensor = 0;
     const bool tensor_runs = algo == NMG_ALGO_TENSOR ? any_tensor(geo, dtype) : algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, M);
     if (tensor_runs)
-        tensor = (tc_use_dense(geo, dtype, false, tokens, have_packed != 0) ? tc_dense_workspace_bytes(geo, dtype, false)
+        tensor = (tc_use_dense(geo, dtype, false, tokens, have_packed) ? tc_dense_workspace_bytes(geo, dtype, false)
                                                    : (have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512)) +
                  tc_split_workspace_bytes(geo, dtype, false, tokens) +
-                 (layout == NMG_ACT_K_MAJOR ? kmajor_transpose_bytes(geo, dtype, tokens) : algo == NMG_ALGO_AUTO ? pad_rows_bytes(dtype, tokens, K) : 0);
+                 (layout == NMG_ACT_K_MAJOR ? kmajor_transpose_bytes(geo, dtype, tokens) : algo == NMG_ALGO_AUTO && !aligned ? pad_rows_bytes(dtype, tokens, K) : 0);
     // AUTO: the gather kernels serve what the tensor cores do not, and a handful of K-major columns without a packed copy
-    const bool simt_runs = algo == NMG_ALGO_SIMT || (algo == NMG_ALGO_AUTO && (!tensor_runs || kmajor_few(geo, dtype, layout, tokens, have_packed != 0)));
+    const bool simt_runs = algo == NMG_ALGO_SIMT || (algo == NMG_ALGO_AUTO && (!tensor_runs || kmajor_few(geo, dtype, layout, tokens, have_packed)));
     const size_t simt = simt_runs ? simt_fwd_workspace_bytes(geo, tokens, dtype, layout) : 0;
     return simt > tensor ? simt : tensor;
 }
@@ -214,7 +215,8 @@ static bool use_sp(const Geo &geo, int dtype, int64_t tokens, int algo) {
 }
 
 extern "C" size_t nmg_spmm_t_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype,
-                                             int algo, int have_packed) {
+                                             int algo, int given) {
+    const bool have_packed = (given & ~NMG_GIVEN_ALIGNED_ROWS) != 0, aligned = (given & NMG_GIVEN_ALIGNED_ROWS) != 0;
     Geo geo;
     if (make_geo(M, K, n, m, g, &geo) || tokens < 1 || n < 1) return 0;
     const size_t pack = have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512;
@@ -222,10 +224,10 @@ extern "C" size_t nmg_spmm_t_workspace_bytes(int64_t M, int64_t K, int64_t token
     const size_t simt = tensor_only ? 0 : pack + simt_bwd_workspace_bytes(geo, tokens, dtype) + 256;
     size_t tensor = 0;
     if (algo != NMG_ALGO_SIMT && any_tensor(geo, dtype))
-        tensor = (tc_use_dense(geo, dtype, true, tokens, have_packed != 0) ? tc_dense_workspace_bytes(geo, dtype, true) : pack) +
+        tensor = (tc_use_dense(geo, dtype, true, tokens, have_packed) ? tc_dense_workspace_bytes(geo, dtype, true) : pack) +
                  tc_split_workspace_bytes(geo, dtype, true, tokens);
     if (use_sp(geo, dtype, tokens, algo) && tc_sp_copy_bytes(geo) + 512 > tensor) tensor = tc_sp_copy_bytes(geo) + 512;
-    if (algo == NMG_ALGO_AUTO && tensor_only) tensor += pad_rows_bytes(dtype, tokens, M);
+    if (algo == NMG_ALGO_AUTO && tensor_only && !aligned) tensor += pad_rows_bytes(dtype, tokens, M);
     return simt > tensor ? simt : tensor;
 }
 

@@ -636,7 +636,9 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
             }
         }
     }
-    __syncthreads();
+    // A CTA whose wait for the others' partial tiles ran out must not give up shared memory that they may still write to: it stays
+    // until every CTA of the cluster has ended (exited threads count as arrived, and all waits of the others are bounded).
+    if (__syncthreads_or(ks > 1 && warp < FX_WARP_X && !ok)) cluster_sync_all();
     if (warp == FX_WARP_MMA) {
         tc_fence_after();
         tmem_dealloc(tmem_base, tmem_cols);

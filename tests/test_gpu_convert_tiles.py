@@ -1,4 +1,6 @@
 """Edges of the conversion kernels' tiles: partly filled warps, remainder tiles, unaligned rows, ties and zeros."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -16,7 +18,7 @@ def test_sparsify_and_densify_at_tile_edges(n, m, g, dtype):
     """One tile, tiles that do not fill a warp, cut tiles in both directions, rows without 16-byte alignment; few distinct
     values (ties) with many zeros, and random weights."""
     from sten_b200 import ops
-    cc = g * len(orc.nm_order(n, m)) if hasattr(orc, "nm_order") else g * {(1, 4): 4, (2, 4): 6, (1, 8): 8, (2, 8): 28, (1, 16): 16}[n, m]
+    cc = g * math.comb(m, n)
     for M, K, off in [(m, cc, 0), (3 * m + 1, cc, 1), (2 * m, 2 * cc + cc // 2 + 1, 0)]:
         for ties in (False, True):
             w = seeded_normal((M, K + off), M + K)
@@ -26,9 +28,24 @@ def test_sparsify_and_densify_at_tile_edges(n, m, g, dtype):
             val_o, idx_o = orc.sparsify(w.float().numpy(), n, m, g)
             val, idx = ops.sparsify(w.to(cuda())[None], n, m, g)
             assert np.array_equal(np_of(idx), idx_o) and np.array_equal(np_of(val.float()), val_o)
-            d = torch.full((M, K + off), 7.0, dtype=dtype, device=cuda())
-            ops.densify_into(val, idx, d[None, :, off:], n, m, g) if hasattr(ops, "densify_into") else None
             assert np.array_equal(np_of(ops.densify(val, idx, 1, M, K, n, m, g).float())[0], orc.densify(val_o, idx_o, (M, K), n, m, g))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n,m,g", [(1, 4, 16), (2, 4, 3), (2, 4, 16), (2, 8, 16), (1, 16, 16), (3, 6, 4)])
+@pytest.mark.parametrize("B,K,off,tail", [(1, 96, 8, 0), (1, 96, 1, 0), (1, 500, 0, 3), (2, 448, 8, 8), (2, 451, 1, 2), (3, 40, 0, 0)])
+def test_densify_into_rows_of_a_wider_matrix(B, K, off, tail, n, m, g, dtype):
+    """A pitch larger than the row, aligned and unaligned bases: the rows are the dense weight, what lies between them stays."""
+    from sten_b200 import _native as nat, ops
+    M = 2 * m + 1
+    val, idx = ops.sparsify(seeded_normal((B, M, K), M + K).to(dtype).to(cuda()), n, m, g)
+    pitch = off + K + tail
+    d = torch.full((B, M, pitch), 7.0, dtype=dtype, device=cuda())
+    code = nat.NMG_F32 if dtype == torch.float32 else nat.NMG_BF16
+    nat.check(nat.lib().nmg_densify(val.data_ptr(), idx.data_ptr(), B, M, K, n, m, g, code, d[:, :, off:].data_ptr(), pitch, M * pitch,
+                                    torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(d[:, :, off:off + K], ops.densify(val, idx, B, M, K, n, m, g))
+    assert bool((d[:, :, :off] == 7.0).all()) and bool((d[:, :, off + K:] == 7.0).all())
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])

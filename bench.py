@@ -563,7 +563,7 @@ def run_ours(args):
             achieved = alg / (kms * 1e-3) / 1e12
             peak = peaks["bf16_tflops"]
             roofline = {"bound": "tensor",
-                        "kernel": "gemm_tc_kernel<bf16> (persistent TMA-fed tcgen05 matmul) + expand_dense_kernel<bf16> (weight expansion pass), timed together",
+                        "kernel": "gemm_tc_kernel<bf16> (persistent TMA-fed tcgen05 matmul) + expand_rows_kernel<bf16> (weight expansion pass), timed together",
                         "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                         "peak_source": f"{peaks_src} bf16_tflops (burst: the call is timed alone), of measured",
                         "traffic": NCU_DRAM_BYTES_PER_CALL if world == 1 else None,

@@ -145,8 +145,8 @@ int nmg_spmm(const void *val, const int16_t *idx, const void *packed, int64_t M,
 
 /* nmg_spmm followed by an activation and a residual add, in one call: out = activation(product + bias) + residual.
  * The reference adds the bias in a separate pass over the output (src/sten/grouped_nm/sten_impls.py:172-173) and leaves
- * activation and residual to the model code; here the two-pass tensor-core matmul applies all three in its epilogue
- * (the output is written once), every other kernel is followed by one elementwise pass.
+ * activation and residual to the model code; here the tensor-core matmuls apply all three in their epilogues
+ * (the output is written once), the SIMT kernels are followed by one elementwise pass.
  *   activation: NMG_EPI_NONE or NMG_EPI_GELU (exact: x/2 * (1 + erf(x / sqrt 2)))
  *   residual:   NULL, or a tensor of the output's shape and orientation with row pitch ld_res.
  * Everything else as nmg_spmm (same workspace query). */

@@ -9,7 +9,8 @@
 //
 //   expand_dense_kernel   (val, idx) -> dense W [M][K] (forward) or W^T [K][M] (transposed product), 16-bit; fp32
 //                         weights become three bf16 planes (exact hi / mid / lo split).  Works for every (n, m, g).
-//   gemm_tc_kernel        persistent, one CTA per SM.  Warp 0 issues the TMA loads of both operands, warp 1 the
+//   expand_rows_kernel    the same for W with n <= 2 and chunks of whole 16-byte pieces, the usual weight: whole rows.
+//   gemm_tc_kernel        persistent, one CTA per SM, in pairs but for 16-bit outputs of one feature tile.  Warp 0 issues the TMA loads of both operands, warp 1 the
 //                         MMAs (128 x 256 x 16, fp32 accumulators in TMEM), warps 2..9 drain accumulators.  16-bit
 //                         mode double-buffers the accumulator (2 x 256 TMEM columns) so that the drain of one tile
 //                         overlaps the MMAs of the next; in fp32 mode a buffer is a chunk of TC_CHUNK_KB k-blocks, and

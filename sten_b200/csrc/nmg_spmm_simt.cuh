@@ -43,8 +43,8 @@ int simt_bwd(const Geo &geo, int dtype, const void *pat, const void *nval, const
 // inside the matmul; the two-pass variant (nmg_gemm_tc.cu, `dense` = true) first expands (val, idx) into a dense 16-bit
 // matrix in `ws` (tc_dense_workspace_bytes, after the split activation) and multiplies that.  tc_use_dense is the
 // policy: two passes for large batches, and for every (n, m) the fused kernel has no instantiation for.
-// What follows the product: out = activation(product + bias) + residual.  The two-pass tensor-core matmul applies it in its
-// epilogue; every other kernel is followed by one elementwise pass (launch_epilogue).
+// What follows the product: out = activation(product + bias) + residual.  Both tensor-core matmuls apply it in their
+// epilogues; the SIMT kernels are followed by one elementwise pass (launch_epilogue).
 struct Epilogue {
     int act = NMG_EPI_NONE;
     const void *residual = nullptr;  // same orientation as the output

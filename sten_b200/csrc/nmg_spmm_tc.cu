@@ -1,20 +1,20 @@
-// Tensor-core matmul for fp16 / bf16 grouped n:m weights: tcgen05.mma with TMEM accumulators.
+// Fused tensor-core matmul of grouped n:m weights: tcgen05.mma with the expanded weight and the accumulators in TMEM.
 //
 // In the format's orientation the n:m blocks run along the OUTPUT-feature axis of y = x W^T, so no operand of the
 // forward product is structured-sparse along the reduction axis and tcgen05.mma.sp does not apply.  What the
-// format does give is a weight that is 2/m .. n/m of its dense size in HBM and L2.  This kernel keeps it that
-// way: the weight stays compressed in global memory (column-ordered copy: one pattern id + n values per
-// (row-block, column)), is expanded tile by tile straight into the shared-memory operand layout of the
-// tensor core (128-byte swizzle, K-major) by dedicated warps, and is multiplied at dense tensor-core rate
+// format does give is a weight that is smaller than its dense form in HBM and L2.  This kernel reads the column-ordered copy
+// (bytes per dense element, 16-bit / fp32: values 2 n/m / 4 n/m; a pattern byte per column of a row-block, 1/m; row masks, n/8;
+// for fp32 three bf16 planes of the values, 6 n/m.  2:4: 1.5 against 2 dense, fp32 5.5 against 4: the fp32 copy is larger than
+// the dense weight, of which the forward product reads masks and planes, 3.25, and the transposed one values and patterns, 2.25).
+// Dedicated warps expand it tile by tile into the tensor core's A operand in TMEM, and it is multiplied at dense tensor-core rate
 // against activation tiles that arrive by TMA.  The same kernel computes the transposed product dX = dY W: only
 // the expansion routine differs (the tile is W^T, the reduction runs over weight rows).
 //
-// CTA = 14 warps: warp 0 issues TMA loads of the activation tile (up to 256 tokens x 64 reduction elements), warp 1
-// allocates TMEM and issues the MMAs (128 x tokens x 16, fp32 accumulate in TMEM), warps 2..13 form three groups
-// that expand the weight tile (128 output features x 64 reduction elements) of every third k-block each; every
-// group fetches its next tile's compressed data into registers before it scatters the current one.  fp32 weights: a
-// k-block's three bf16 planes are expanded once and multiplied six times (the split products), instead of once per product.
-// All twelve then run the epilogue (tcgen05.ld -> bias -> activation -> residual -> store).
+// CTA = 15 warps.  Warps 0..11 form three groups that expand the weight tile (128 output features x 64 reduction elements) of
+// every third k-block each, from shared memory through registers into TMEM.  Warp 12 loads activation tiles (up to 256 tokens x 64
+// reduction elements), warp 14 compressed weight tiles, both by TMA; warp 13 allocates TMEM and issues the MMAs (128 x tokens x 16,
+// fp32 accumulate in TMEM).  fp32 weights: a k-block's three bf16 planes are expanded once and multiplied six times (the split
+// products).  Warps 0..11 then run the epilogue (tcgen05.ld -> bias -> activation -> residual -> store).
 //
 // What bounds it with few tokens is latency, not bandwidth: at 4096 x 4096 and 16 tokens the 25 MB of compressed weight are
 // 4 us of HBM time.  So the reduction axis is cut over a cluster of CTAs that fills the chip, and the partial tiles meet in

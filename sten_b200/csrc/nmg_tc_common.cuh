@@ -234,16 +234,11 @@ template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float lo, f
 }
 template <> __device__ __forceinline__ uint32_t pack2<float>(float, float) { return 0; }  // never used: fp32 outputs are stored as words
 
-template <typename T> __device__ __forceinline__ uint16_t bits16(T v);
-template <> __device__ __forceinline__ uint16_t bits16<__half>(__half v) { return __half_as_ushort(v); }
-template <> __device__ __forceinline__ uint16_t bits16<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat16_as_ushort(v); }
-template <> __device__ __forceinline__ uint16_t bits16<float>(float) { return 0; }  // never used: fp32 outputs are stored as words
-
 
 // Exact (erf) GELU with a short erf: erf(x) = 1 - (a1 t + ... + a5 t^5) exp(-x^2), t = 1 / (1 + p x) for x >= 0 (Abramowitz &
 // Stegun 7.1.26, absolute error 1.5e-7, i.e. below fp32 rounding of the result for |v| of order one).  With x = |v| / sqrt(2)
 // and v * sign(v) = |v|, gelu(v) = v (1 + erf(v / sqrt 2)) / 2 collapses to max(v, 0) - |v| q(t) 2^(-v^2 log2(e) / 2) where q
-// carries the halved coefficients: fourteen instructions, two of them on the special-function unit (flush-to-zero forms, which
+// carries the halved coefficients: fifteen instructions, two of them on the special-function unit (flush-to-zero forms, which
 // need no range fix-up), against the library erf's thirty.  The drain warps apply it to 128 x 256 values per tile.
 __device__ __forceinline__ float gelu_erf(float v) {
     const float av = fabsf(fminf(v, 1e30f));  // +inf: the second factor below is 0 then, and the first must not be infinite

@@ -60,7 +60,7 @@ def dense_to_same_grouped_nm(sparsifier, tensor, grad_fmt=None):
 
 def _wants_expanded(gnm, x2d, tokens):
     """The opt-in of ``set_spmm_opt(kernel="sm100-expanded")`` applies: 16-bit weight, token-major activation whose rows TMA
-    can read, and a batch large enough for the two-pass regime (fewer tokens stay on the compressed-weight kernel)."""
+    can read, and a batch from which on the matmul of the kept weight is no slower than the compressed-weight kernel."""
     return (gnm.nm_strides.get("kernel") == "sm100-expanded" and tokens >= ops.SP24_MIN_TOKENS
             and gnm.val.dtype != torch.float32 and x2d.stride(-1) == 1 and x2d.data_ptr() % 16 == 0 and x2d.stride(0) % 8 == 0
             and gnm.expanded() is not None)

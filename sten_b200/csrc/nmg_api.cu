@@ -78,7 +78,7 @@ static size_t kmajor_transpose_bytes(const Geo &geo, int dtype, int64_t tokens) 
 }
 // Fewer than 64 columns do not pay for re-ordering the weight on every call; with a packed copy in hand they take the tensor
 // cores like any other batch (192 x 3200 f16, 2 columns: 7 us against 229 us in the gather kernel).
-// In fp32 only the fused kernel sums as accurately as the gather kernel does (see chunk_kb).
+// In fp32 only the fused kernel sums as accurately as the gather kernel does (see FINE there).
 static bool kmajor_few(const Geo &geo, int dtype, int layout, int64_t tokens, bool have_packed) {
     return layout == NMG_ACT_K_MAJOR && tokens < 64 && !(have_packed && (dtype != NMG_F32 || tc_supported(geo, dtype)));
 }

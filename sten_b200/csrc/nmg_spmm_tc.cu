@@ -53,7 +53,6 @@ struct TcParams {
     int exch_off;         // exchange area of the partial tiles: offset in shared memory; 0 = on top of the rings
     int misc_off;         // selector table and barriers
     uint32_t tmem_cols;
-    int chunk_kb;         // fp32: k-blocks per accumulation chunk
     int *status;
 };
 struct FxMaps {
@@ -333,7 +332,13 @@ __device__ __forceinline__ void finish_store(const TcParams &prm, uint32_t (&r)[
 
 // One CTA computes 128 features x bn tokens over its range of the reduction axis; the `ksplit` CTAs of a cluster share the
 // tile and add their partial tiles through distributed shared memory, in the order of the ranges.
-template <int N_, int M_, typename T, bool TRANSPOSED>
+//
+// FINE (fp32 forward): the accumulator restarts at every k-block and a k-block's products are added smallest first, so that most
+// roundings are those of a small sum.  For a handful of K-major columns, which the gather kernels otherwise serve with fp32 FMAs:
+// the error is below theirs at every size, K = 256 / 1024 / 16384, 2:4 0.7 / 0.9 / 1.4e-7 against 2.0 / 4.0 / 16.6e-7, 1:16 0.6 /
+// 0.8 / 1.3e-7 against 0.8 / 1.5 / 5.8e-7 (without FINE 11 / 11 / 35e-7 and 7 / 7 / 21e-7).  It costs 8 of 29 us at 4096 x 4096,
+// nothing at 1024 x 1024.
+template <int N_, int M_, typename T, bool TRANSPOSED, bool FINE>
 __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams prm, const __grid_constant__ FxMaps maps) {
     constexpr bool SPLIT = TcMode<T>::TERMS > 1;
     constexpr int PLANES = SPLIT ? 3 : 1;
@@ -375,7 +380,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
     const int kb_per = (nkb_all + ks - 1) / ks;
     const int kb_base = split * kb_per;  // this CTA's first k-block
     const int nkb = (nkb_all < kb_base + kb_per ? nkb_all : kb_base + kb_per) - kb_base;  // >= 1 by the host's choice of ksplit
-    const int chunk_kb = SPLIT ? prm.chunk_kb : nkb;  // k-blocks per accumulation chunk
+    const int chunk_kb = SPLIT ? (FINE ? 1 : TC_CHUNK_KB) : nkb;  // k-blocks per accumulation chunk
     const int nchunks = (nkb + chunk_kb - 1) / chunk_kb;
     const uint32_t tmem_cols = prm.tmem_cols;
     const int cols_live = (int)(prm.ntok - tok0 < bn ? prm.ntok - tok0 : bn);  // token columns of this tile that exist
@@ -518,7 +523,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
                 const uint64_t bs = bdesc0 + (uint64_t)(uint32_t)(s * (x_bytes >> 4));
 #pragma unroll
                 for (int t = 0; t < TcMode<T>::TERMS; t++) {
-                    const int st = TcMode<T>::TERMS - 1 - t;  // smallest product first: its rounding is that of a small sum
+                    const int st = FINE ? TcMode<T>::TERMS - 1 - t : t;
                     const uint32_t at = at0 + (uint32_t)((SPLIT ? split_w(st) : 0) * FX_A_COLS);
                     const uint64_t bt = bs + (uint64_t)(uint32_t)((SPLIT ? split_x(st) : 0) * (b_bytes >> 4));
 #pragma unroll
@@ -762,7 +767,7 @@ size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, int6
     return (size_t)3 * (size_t)tokens * (size_t)round_up(red, 8) * 2 + 512;
 }
 
-template <int N_, int M_, typename T, bool TR>
+template <int N_, int M_, typename T, bool TR, bool FINE = false>
 static int tc_launch_one(const TcParams &p0, const FxMaps &maps, cudaStream_t st) {
     const FxPlan plan = fx_plan(TcMode<T>::TERMS > 1 ? 3 : 1, p0.bn, p0.ksplit, fx_slot_bytes(N_, M_, (int)sizeof(T), TR));
     TcParams p = p0;
@@ -774,7 +779,7 @@ static int tc_launch_one(const TcParams &p0, const FxMaps &maps, cudaStream_t st
     p.misc_off = (int)(plan.total - 1024 - FX_MISC_BYTES);
     const int64_t ctas = (int64_t)p.tiles_f * p.tiles_t * p.ksplit;
     if (ctas > 0x7fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many output tiles for one launch");
-    NMG_ALLOW_SMEM(plan.total, spmm_tc_kernel<N_, M_, T, TR>);
+    NMG_ALLOW_SMEM(plan.total, spmm_tc_kernel<N_, M_, T, TR, FINE>);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)ctas);
     cfg.blockDim = dim3(FX_THREADS);
@@ -789,14 +794,15 @@ static int tc_launch_one(const TcParams &p0, const FxMaps &maps, cudaStream_t st
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.ksplit > 1 ? 2 : 1;
-    NMG_CUDA(cudaLaunchKernelEx(&cfg, spmm_tc_kernel<N_, M_, T, TR>, p, maps));
+    NMG_CUDA(cudaLaunchKernelEx(&cfg, spmm_tc_kernel<N_, M_, T, TR, FINE>, p, maps));
     return NMG_OK;
 }
 
 template <int N_, int M_>
-static int tc_launch_nm(int dtype, bool transposed, const TcParams &p, const FxMaps &maps, cudaStream_t st) {
+static int tc_launch_nm(int dtype, bool transposed, bool fine, const TcParams &p, const FxMaps &maps, cudaStream_t st) {
     if (dtype == NMG_F16) return transposed ? tc_launch_one<N_, M_, __half, true>(p, maps, st) : tc_launch_one<N_, M_, __half, false>(p, maps, st);
-    if (dtype == NMG_F32) return transposed ? tc_launch_one<N_, M_, float, true>(p, maps, st) : tc_launch_one<N_, M_, float, false>(p, maps, st);
+    if (dtype == NMG_F32)
+        return transposed ? tc_launch_one<N_, M_, float, true>(p, maps, st) : fine ? tc_launch_one<N_, M_, float, false, true>(p, maps, st) : tc_launch_one<N_, M_, float, false>(p, maps, st);
     return transposed ? tc_launch_one<N_, M_, __nv_bfloat16, true>(p, maps, st) : tc_launch_one<N_, M_, __nv_bfloat16, false>(p, maps, st);
 }
 
@@ -893,11 +899,6 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     p.out_vec = out_token_major ? (ld_out % 2 == 0 && feats % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0)
                                 : (ld_out * es % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0);
     p.tiles_f = fx.tiles_f; p.tiles_t = fx.tiles_t; p.bn = fx.bn; p.ksplit = fx.ksplit;
-    // A handful of K-major fp32 columns is otherwise served by the gather kernels' fp32 FMAs.  With a chunk per k-block and the
-    // products added smallest first the error is below theirs at every size: K = 256 / 1024 / 16384, 2:4 0.7 / 0.9 / 1.4e-7 against
-    // 2.0 / 4.0 / 16.6e-7, 1:16 0.6 / 0.8 / 1.3e-7 against 0.8 / 1.5 / 5.8e-7 (chunks of 8, largest first: 11 / 11 / 35e-7 and
-    // 7 / 7 / 21e-7).  It costs 8 of 29 us at 4096 x 4096, nothing at K = 1024 and below.
-    p.chunk_kb = act_k_major && tokens < 64 ? 1 : TC_CHUNK_KB;
     p.masks = masks; p.mask_rows = natural_mask_rows(geo); p.nb = geo.nb;
     p.status = status;
     const ProfileEvents pe = take_profile_events();
@@ -905,7 +906,7 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     rc = NMG_ERR_UNSUPPORTED;
 #define NMG_TC_CASE(N_, M_)                                                                         \
     if (geo.n == N_ && geo.m == M_)                                                                \
-        rc = tc_launch_nm<N_, M_>(dtype, transposed, p, maps, st);
+        rc = tc_launch_nm<N_, M_>(dtype, transposed, act_k_major && tokens < 64, p, maps, st);
     NMG_TC_CASE(1, 4)
     NMG_TC_CASE(2, 4)
     NMG_TC_CASE(1, 8)

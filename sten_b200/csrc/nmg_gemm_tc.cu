@@ -276,6 +276,16 @@ constexpr int GEMM_DRAIN_WARPS = 8;   // two per TMEM lane quarter, each takes h
 constexpr int GEMM_THREADS = 32 * (2 + GEMM_DRAIN_WARPS);  // TMA warp, MMA warp, drain warps
 constexpr int GEMM_RING_BYTES = TC_STAGES * (TC_A_BYTES + TC_B_BYTES);  // 192 KB of operand stages in either mode
 
+// The output's tiles: the first f_wide rows of tiles are bn columns wide, the f_narrow rows below them bn_tail.
+// See gemm_tiles for the choice.
+struct GemmTiles {
+    int f_wide, f_narrow;    // rows of tiles
+    int t_wide, t_narrow;    // tiles per row
+    int bn, bn_tail;         // columns of a tile
+    __host__ __device__ int wide() const { return f_wide * t_wide; }
+    __host__ __device__ int count() const { return f_wide * t_wide + f_narrow * t_narrow; }
+};
+
 constexpr int GEMM_MAX_OUTS = 8;
 struct GemmParams {
     const void *bias;  // [out_feats] or NULL
@@ -292,8 +302,7 @@ struct GemmParams {
     int out_token_major;
     int out_staged;    // feature-major output whose rows are 16-byte aligned: go through the staging tile
     int out_tm_vec;    // token-major output (and residual) whose rows are 16-byte aligned: transposed in the staging tile, 16-byte stores
-    int tiles_f, tiles_t;  // tiles_f counts tiles of 128 features (one CTA per tile) or 256 (CTA pairs)
-    int bn;                // width of a tile: TC_BN, or what gemm_split_cols chose (fp32)
+    GemmTiles tiles;       // one CTA per tile of 128 features, or a pair per 256
     int band;              // width of the tile order's bands, in feature tiles
     unsigned *wave_ctr;    // zeroed counter for the producers' soft rendezvous before every tile, or NULL
     int *status;
@@ -303,6 +312,7 @@ constexpr int GEMM_STAGING_BYTES = GEMM_DRAIN_WARPS * 4096;  // per drain warp: 
 struct GemmMaps {
     CUtensorMap a[3];  // weight planes, box 64 x 128, 128-byte swizzle
     CUtensorMap b[3];  // activation planes, box 64 x bn (64 x bn / 2 for CTA pairs)
+    CUtensorMap b_tail[3];  // the same with the box of the narrow tiles
     CUtensorMap out;   // out_tma: the output, box 128 bytes x 32 rows, 128-byte swizzle
 };
 
@@ -330,7 +340,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     constexpr int B_BYTES = PAIR ? TC_B_BYTES / 2 : TC_B_BYTES;  // room of one plane; the widest tile fills it
     constexpr int OFF_B = PLANES * TC_A_BYTES, STAGE_BYTES = OFF_B + PLANES * B_BYTES;
     constexpr int STAGES = GEMM_RING_BYTES / STAGE_BYTES;  // 4, 6 for pairs, 2 for fp32
-    const int bn = SPLIT ? prm.bn : TC_BN;
     constexpr int TILE_FEATS = PAIR ? 2 * TC_BM : TC_BM;
 
     extern __shared__ char smem_raw[];
@@ -350,7 +359,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     const int unit_id = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;      // CTA (or pair) index
     const int nunits = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
     // A "unit" is what the MMA issuer hands to the drain warps: a whole tile (16-bit) or a chunk of k-blocks (fp32).
-    const int ntiles = prm.tiles_f * prm.tiles_t;
+    const int ntiles = prm.tiles.count(), nwide = prm.tiles.wide();
     const int my_tiles = (unit_id < ntiles) ? (ntiles - unit_id + nunits - 1) / nunits : 0;
     const int nkb = (int)((prm.red + TC_BK - 1) / TC_BK);  // iterations per tile
     const int chunk_it = SPLIT ? TC_CHUNK_KB : nkb;
@@ -383,10 +392,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         if constexpr (PAIR) return mbar_wait_cluster_bounded(bar, parity, prm.status, code);
         else return mbar_wait_bounded(bar, parity, prm.status, code);
     };
-    auto tile_origin = [&](int ti, int &feat0, int &tok0) {  // feat0: first feature of THIS CTA's 128 rows
+    auto narrow = [&](int ti) -> bool { return PAIR && unit_id + ti * nunits >= nwide; };
+    auto tile_origin = [&](int ti, int &feat0, int &tok0, int &bn) {  // feat0: first feature of THIS CTA's 128 rows; bn: columns
         int tile_f, tile_t;
-        tile_of_cta(unit_id + ti * nunits, prm.tiles_f, prm.tiles_t, tile_f, tile_t, prm.band);
-        feat0 = tile_f * TILE_FEATS + (int)rank * TC_BM;
+        const bool nar = narrow(ti);
+        tile_of_cta(unit_id + ti * nunits - (nar ? nwide : 0), nar ? prm.tiles.f_narrow : prm.tiles.f_wide, nar ? prm.tiles.t_narrow : prm.tiles.t_wide, tile_f, tile_t,
+                    prm.band);
+        bn = !PAIR ? TC_BN : nar ? prm.tiles.bn_tail : prm.tiles.bn;
+        feat0 = (tile_f + (nar ? prm.tiles.f_wide : 0)) * TILE_FEATS + (int)rank * TC_BM;
         tok0 = tile_t * bn;
     };
 
@@ -400,8 +413,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         asm volatile("griddepcontrol.wait;" ::: "memory");
         unsigned arrivals = 0;
         for (int ti = 0; ti < my_tiles && ok; ti++) {
-            int feat0, tok0;
-            tile_origin(ti, feat0, tok0);
+            int feat0, tok0, bn;
+            tile_origin(ti, feat0, tok0, bn);
+            const CUtensorMap *bmap = narrow(ti) ? maps.b_tail : maps.b;
             if (prm.wave_ctr && ti > 0) {
                 // CTAs whose tiles share operand panels read them from HBM once only while they stream through the
                 // reduction in step; left alone they drift apart over the waves (measured: 2.2 MB of DRAM reads per
@@ -424,7 +438,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
 #pragma unroll
                         for (int c = 0; c < PLANES; c++) {
                             tma_load_2d_pair(stage + c * TC_A_BYTES, &maps.a[c], kb * TC_BK, feat0, full_leader + s * 8);
-                            tma_load_2d_pair(stage + OFF_B + c * B_BYTES, &maps.b[c], kb * TC_BK, tok0 + (int)rank * half, full_leader + s * 8);
+                            tma_load_2d_pair(stage + OFF_B + c * B_BYTES, &bmap[c], kb * TC_BK, tok0 + (int)rank * half, full_leader + s * 8);
                         }
                     } else {
                         mbar_expect_tx(&full[s], STAGE_BYTES);
@@ -438,14 +452,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (of the leader for pairs)
         if (leader) {
-            uint32_t idesc = make_idesc<E>(bn);
-            if constexpr (PAIR) idesc = (idesc & ~(0x1fu << 24)) | ((uint32_t)(256 >> 4) << 24);  // M = 256 across the pair
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint64_t desc0 = make_sw128_desc(smem_u32(smem));
             bool ok = true;
             int it = 0, unit = 0;
             for (int ti = 0; ti < my_tiles && ok; ti++) {
                 int kb = 0;
+                uint32_t idesc = make_idesc<E>(!PAIR ? TC_BN : narrow(ti) ? prm.tiles.bn_tail : prm.tiles.bn);
+                if constexpr (PAIR) idesc = (idesc & ~(0x1fu << 24)) | ((uint32_t)(256 >> 4) << 24);  // M = 256 across the pair
                 for (int c = 0; c < nchunks && ok; c++, unit++) {
                     const int b = unit % NBUF, use = unit / NBUF;
                     if (use > 0) ok = __all_sync(0xffffffffu, wait(&acc_free[b], (uint32_t)((use - 1) & 1), 26));
@@ -498,8 +512,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         constexpr int RQ = RES_AHEAD ? 4 : 1;                  // 16-byte pieces of one slice row of the residual
         const int q = warp & 3;  // TMEM lane quarter this warp may access
         constexpr int SLICES = (TC_BN / 32) / (GEMM_DRAIN_WARPS / 4);  // 32-column slices per warp, at most
-        const int per_warp = (bn / 32 + 1) / 2, sl0 = ((warp - 2) >> 2) * per_warp;  // this warp's first slice
-        const int nsl = min(per_warp, bn / 32 - sl0);                                // and how many it has
         const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
         char *stage_w = staging + (warp - 2) * 4096;
         const T *res = static_cast<const T *>(prm.residual);
@@ -511,8 +523,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         bool ok = true;
         float run[SPLIT ? SLICES : 1][32];  // fp32: sum of the tile's finished chunks
         for (int ti = 0; ti < my_tiles && ok; ti++) {
-            int feat0, tok0;
-            tile_origin(ti, feat0, tok0);
+            int feat0, tok0, bn;
+            tile_origin(ti, feat0, tok0, bn);
+            // this warp's first slice and how many it has: whole staged groups, the first half of the warps takes the odd one
+            const int per_warp = (bn / GROUP_TOK + 1) / 2 * GROUP_SLICES, sl0 = ((warp - 2) >> 2) * per_warp;
+            const int nsl = min(per_warp, bn / 32 - sl0);
             const int64_t feat = (int64_t)feat0 + q * 32 + lane;
             const bool feat_ok = feat < prm.out_feats;
             const float bias = (prm.bias && !prm.bias_cols && feat_ok) ? DT<T>::to_f32(static_cast<const T *>(prm.bias)[feat]) : 0.f;
@@ -866,8 +881,7 @@ template <typename T, bool PAIR, bool TMA_OUT> static int gemm_launch_as(const G
     const size_t smem = (size_t)GEMM_RING_BYTES + GEMM_STAGING_BYTES + 256 + 1024;
     int sms = 148, rc_sms;
     if ((rc_sms = device_sms(&sms))) return rc_sms;
-    const int64_t tiles = (int64_t)p.tiles_f * p.tiles_t;
-    if (tiles > 0x3fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many output tiles for one launch");
+    const int64_t tiles = p.tiles.count();
     NMG_ALLOW_SMEM(smem, gemm_tc_kernel<T, PAIR, TMA_OUT>);
     cudaLaunchConfig_t cfg = {};
     const int64_t units = PAIR ? sms / 2 : sms;  // persistent CTAs, or CTA pairs
@@ -891,16 +905,44 @@ template <typename T, bool PAIR> static int gemm_launch(const GemmParams &p, con
     return p.out_tma ? gemm_launch_as<T, PAIR, true>(p, maps, st) : gemm_launch_as<T, PAIR, false>(p, maps, st);
 }
 
-// Tile width of the fp32 product: the one whose waves cost least.  A tile of bn columns takes about as long as bn + 40 columns
-// at full rate (narrow tiles read more shared memory per product; measured 3072 <- 768, 4096 tokens: 28.6 us per wave at 256, 15.8
-// at 128, 10.8 at 64).  768 <- 3072 is 48 tiles of 256 columns on 74 pairs and 107.9 us, or 66 of 192 and 89.5; 1024 <- 4096 at
-// 1536 tokens takes 131 us at 256 and 76 at 96.
-static int gemm_split_cols(int64_t tiles_f, int64_t cols, int64_t units) {
-    int best = TC_BN;
+// Tile widths: the choice whose slowest pair costs least.  A tile of bn columns costs what bn + 40 columns at full rate do (narrow
+// tiles read more shared memory per product; fp32, 3072 <- 768, 4096 tokens: 28.6 us per wave at 256, 15.8 at 128, 10.8 at 64).
+// Tiles of one width leave most pairs without work in a last wave that is not full, so some rows of tiles at the end of the
+// order may be narrower: their tiles then fill the places that the wide ones leave.  Tile i goes to pair i % units.
+// 4096 x 4096 bf16, 4096 tokens: 256 tiles, 3.46 waves of 74 pairs, 110.0 -> 106.7 us with three of sixteen rows in tiles of 192;
+// 4096 x 1024 f16 pair, 12288 tokens: 212.0 -> 208.2.  From sixteen waves on the last one is too small a part.
+// 16-bit: wide tiles have 256 columns, narrow ones 128 or 192 (whole staged groups for both halves of the drain warps).
+static GemmTiles gemm_tiles(int64_t tiles_f, int64_t cols, int64_t units, bool fp32, bool pair) {
+    GemmTiles best{(int)tiles_f, 0, (int)((cols + TC_BN - 1) / TC_BN), 0, TC_BN, TC_BN};
+    if (!pair) return best;
+    const int step = fp32 ? 32 : 64, least = fp32 ? 64 : 128, widths = (TC_BN - least) / step + 1;
+    int per_row[7];  // tiles per row at width least + i * step
+    for (int i = 0; i < widths; i++) per_row[i] = (int)((cols + least + i * step - 1) / (least + i * step));
+    const int u = (int)units;
     int64_t best_cost = INT64_MAX;
-    for (int bn = TC_BN; bn >= 64; bn -= 32) {
-        const int64_t tiles = tiles_f * ((cols + bn - 1) / bn), cost = (tiles + units - 1) / units * (bn + 40);
-        if (cost < best_cost) { best = bn; best_cost = cost; }
+    for (int i = widths - 1; i >= (fp32 ? 0 : widths - 1); i--) {
+        const int bn = least + i * step, cost = bn + 40;
+        const int64_t all = tiles_f * per_row[i], uniform = (all + u - 1) / u * cost;
+        if (uniform < best_cost) {
+            best = GemmTiles{(int)tiles_f, 0, per_row[i], 0, bn, bn};
+            best_cost = uniform;
+        }
+        if (all > 16 * units) continue;  // a sixteenth of the last wave at most: not worth a second shape of tiles
+        for (int j = i - 1; j >= 0; j--) {
+            const int bn_tail = least + j * step, cost_tail = bn_tail + 40;
+            // more narrow tiles than two waves of them never help: a wide tile does the same columns in less time
+            for (int f = 1; f < tiles_f && f * per_row[j] <= 2 * u; f++) {
+                const int64_t wide = all - (int64_t)f * per_row[i], full = wide / u;
+                const int rest = (int)(wide - full * u), tail = f * per_row[j];
+                int64_t c = full * cost + (tail + u - 1) / u * cost_tail;                                   // a pair without a tile of the last wide wave
+                const int over = tail - (u - rest);                                                          // narrow tiles left for the pairs with one
+                if (rest > 0 && (full + 1) * cost + (over > 0 ? (over + u - 1) / u : 0) * cost_tail > c) c = (full + 1) * cost + (over > 0 ? (over + u - 1) / u : 0) * cost_tail;
+                if (c < best_cost) {
+                    best = GemmTiles{(int)tiles_f - f, f, per_row[i], per_row[j], bn, bn_tail};
+                    best_cost = c;
+                }
+            }
+        }
     }
     return best;
 }
@@ -979,13 +1021,20 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
     const int64_t units = pair ? sms / 2 : sms, row_ext = swap ? tokens : rows, col_ext = swap ? rows : tokens;
     const int tile_feats = pair ? 2 * TC_BM : TC_BM;
     const int64_t tiles_f = (row_ext + tile_feats - 1) / tile_feats;
-    const int bn = dtype == NMG_F32 ? gemm_split_cols(tiles_f, col_ext, units) : TC_BN;
+    if (tiles_f * ((col_ext + 63) / 64) > 0x3fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many output tiles for one launch");
+    const GemmTiles tiles = gemm_tiles(tiles_f, col_ext, units, dtype == NMG_F32, pair);
     for (int c = 0; c < 3; c++) {
         const int pc = c < planes ? c : 0;
         const char *w = dense + (size_t)pc * rows * ld * 2, *x = static_cast<const char *>(act.base) + (size_t)pc * act.plane_elems * 2;
-        const uint32_t col_box = (uint32_t)(pair ? bn / 2 : bn);
+        if (pc != c) {  // never used; keeps the parameter defined
+            maps.a[c] = maps.a[0]; maps.b[c] = maps.b[0]; maps.b_tail[c] = maps.b_tail[0];
+            continue;
+        }
+        const uint32_t col_box = (uint32_t)(pair ? tiles.bn / 2 : tiles.bn);
         if ((rc = encode_tmap_2d(swap ? &maps.b[c] : &maps.a[c], edt, w, (uint64_t)red, (uint64_t)rows, (uint64_t)ld, TC_BK, swap ? col_box : TC_BM, 1))) return rc;
         if ((rc = encode_tmap_2d(swap ? &maps.a[c] : &maps.b[c], edt, x, (uint64_t)red, (uint64_t)tokens, (uint64_t)act.ld, TC_BK, swap ? TC_BM : col_box, 1))) return rc;
+        if (tiles.f_narrow == 0) maps.b_tail[c] = maps.b[c];
+        else if ((rc = encode_tmap_2d(&maps.b_tail[c], edt, swap ? w : x, (uint64_t)red, (uint64_t)col_ext, (uint64_t)(swap ? ld : act.ld), TC_BK, (uint32_t)(tiles.bn_tail / 2), 1))) return rc;
     }
     if (swap) {  // from here on "rows" are the accumulator's rows (tokens) and "tokens" its columns (output features)
         const int64_t t = rows;
@@ -1019,13 +1068,11 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
         maps.out = maps.a[0];  // never used; keeps the parameter defined
     }
     gp.mc_out = (vec && mc_out && (reinterpret_cast<uintptr_t>(mc_out) & 15) == 0) ? mc_out : nullptr;
-    gp.tiles_f = (int)tiles_f;
-    gp.tiles_t = (int)((tokens + bn - 1) / bn);
-    gp.bn = bn;
+    gp.tiles = tiles;
     gp.band = pair ? TC_BAND_PAIR : TC_BAND;
     // many waves over a long reduction: keep the producers in step (see the kernel); the counter is zeroed in stream order.
     // Operands that stay in L2 beside the output need no step keeping: 4096 x 4096, 4096 tokens 108.6 -> 107.4 us without.
-    if ((int64_t)gp.tiles_f * gp.tiles_t >= 3 * units && red >= 4096 && (row_ext + col_ext) * red * 2 * planes > (96ll << 20)) {
+    if ((int64_t)tiles.count() >= 3 * units && red >= 4096 && (row_ext + col_ext) * red * 2 * planes > (96ll << 20)) {
         if ((rc = get_wave_counter(&gp.wave_ctr))) return rc;
         NMG_CUDA(cudaMemsetAsync(gp.wave_ctr, 0, sizeof(unsigned), st));
     }

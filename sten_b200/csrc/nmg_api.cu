@@ -92,9 +92,8 @@ extern "C" size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens,
     size_t tensor = 0;
     const bool tensor_runs = algo == NMG_ALGO_TENSOR ? any_tensor(geo, dtype) : algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, M);
     if (tensor_runs)
-        tensor = (tc_use_dense(geo, dtype, false, tokens, have_packed) ? tc_dense_workspace_bytes(geo, dtype, false)
-                                                   : (have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512)) +
-                 tc_split_workspace_bytes(geo, dtype, false, tokens) +
+        tensor = (tc_use_dense(geo, dtype, false, tokens, have_packed) ? tc_dense_workspace_bytes(geo, dtype, false) + tc_dense_act_bytes(geo, dtype, false, tokens)
+                                                   : (have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512) + tc_split_workspace_bytes(geo, dtype, false, tokens)) +
                  (layout == NMG_ACT_K_MAJOR ? kmajor_transpose_bytes(geo, dtype, tokens) : algo == NMG_ALGO_AUTO && !aligned ? pad_rows_bytes(dtype, tokens, K) : 0);
     // AUTO: the gather kernels serve what the tensor cores do not, and a handful of K-major columns without a packed copy
     const bool simt_runs = algo == NMG_ALGO_SIMT || (algo == NMG_ALGO_AUTO && (!tensor_runs || kmajor_few(geo, dtype, layout, tokens, have_packed)));
@@ -193,7 +192,7 @@ extern "C" int nmg_spmm_replicated(const void *val, const int16_t *idx, int64_t 
 extern "C" size_t nmg_spmm_replicated_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype) {
     Geo geo;
     if (make_geo(M, K, n, m, g, &geo) || tokens < 1 || n < 1 || !tc_dense_supported(geo, dtype)) return 0;
-    return tc_dense_workspace_bytes(geo, dtype, false) + tc_split_workspace_bytes(geo, dtype, false, tokens);
+    return tc_dense_workspace_bytes(geo, dtype, false) + tc_dense_act_bytes(geo, dtype, false, tokens);
 }
 
 extern "C" int nmg_spmm_uses_packed(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype, int layout,
@@ -224,8 +223,8 @@ extern "C" size_t nmg_spmm_t_workspace_bytes(int64_t M, int64_t K, int64_t token
     const size_t simt = tensor_only ? 0 : pack + simt_bwd_workspace_bytes(geo, tokens, dtype) + 256;
     size_t tensor = 0;
     if (algo != NMG_ALGO_SIMT && any_tensor(geo, dtype))
-        tensor = (tc_use_dense(geo, dtype, true, tokens, have_packed) ? tc_dense_workspace_bytes(geo, dtype, true) : pack) +
-                 tc_split_workspace_bytes(geo, dtype, true, tokens);
+        tensor = tc_use_dense(geo, dtype, true, tokens, have_packed) ? tc_dense_workspace_bytes(geo, dtype, true) + tc_dense_act_bytes(geo, dtype, true, tokens)
+                                                                     : pack + tc_split_workspace_bytes(geo, dtype, true, tokens);
     if (use_sp(geo, dtype, tokens, algo) && tc_sp_copy_bytes(geo) + 512 > tensor) tensor = tc_sp_copy_bytes(geo) + 512;
     if (algo == NMG_ALGO_AUTO && tensor_only && !aligned) tensor += pad_rows_bytes(dtype, tokens, M);
     return simt > tensor ? simt : tensor;
@@ -354,7 +353,7 @@ extern "C" int nmg_spmm_expanded(const void *expanded, int64_t M, int64_t K, int
     cudaStream_t st = (cudaStream_t)stream;
     const ProfileEvents pe = take_profile_events();
     if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));
-    rc = tc_dense_gemm(M, K, dtype, static_cast<const char *>(expanded), DenseAct{act, ld_act, 0}, tokens, bias, outs, 1, nullptr, ld_out, out_tm ? 1 : 0, st, epi);
+    rc = tc_dense_gemm(M, K, dtype, static_cast<const char *>(expanded), DenseAct{act, ld_act, nullptr, nullptr}, tokens, bias, outs, 1, nullptr, ld_out, out_tm ? 1 : 0, st, epi);
     if (rc == NMG_OK && pe.stop) NMG_CUDA(cudaEventRecord(pe.stop, st));
     return rc;
 }

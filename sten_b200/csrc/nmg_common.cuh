@@ -217,7 +217,8 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap *map, const void 
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 // all bulk stores of this thread have finished READING shared memory: the source may be overwritten or given up
-__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+// (all but the newest PENDING of them)
+template <int PENDING = 0> __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(PENDING) : "memory"); }
 __device__ __forceinline__ void cp_async_16(void *smem_dst, const void *gsrc) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
 }
@@ -240,7 +241,7 @@ __device__ __forceinline__ const char *stage_bytes_async(char *dst16, const void
 
 // Host: encode a 2-D tiled tensor map (row-major [rows][ld] array, box = box_rows x box_cols) without linking libcuda.
 int encode_tmap_2d(CUtensorMap *map, int dtype, const void *base, uint64_t cols, uint64_t rows, uint64_t ld_elems,
-                   uint32_t box_cols, uint32_t box_rows, int swizzle_128b);
+                   uint32_t box_cols, uint32_t box_rows, int swizzle);  // 0: none, 1: 128 bytes, 2: 64 bytes
 int encode_tmap_2d_bytes(CUtensorMap *map, const void *base, uint64_t cols, uint64_t rows, uint64_t ld, uint32_t box_cols, uint32_t box_rows);  // no swizzle
 
 }  // namespace nmg

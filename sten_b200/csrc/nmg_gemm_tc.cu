@@ -8,10 +8,12 @@
 // about 2.5 bytes per weight element) and run a plain TMA-fed tcgen05 matmul over it:
 //
 //   expand_dense_kernel   (val, idx) -> dense W [M][K] (forward) or W^T [K][M] (transposed product), 16-bit; fp32
-//                         weights become three bf16 planes (exact hi / mid / lo split).  Works for every (n, m, g).
+//                         weights become two fp16 planes of scaled rows (see line_exp).  Works for every (n, m, g).
+//   split_rows_kernel     fp32 only, first: the activation's planes, and the largest magnitudes of the weight's rows (split_columns_kernel
+//                         from a K-major activation).
 //   expand_rows_kernel    the same for W with n <= 2 and chunks of whole 16-byte pieces, the usual weight: whole rows.
 //   gemm_tc_kernel        persistent, one CTA per SM, in pairs but for 16-bit outputs of one feature tile.  Warp 0 issues the TMA loads of both operands, warp 1 the
-//                         MMAs (128 x 256 x 16, fp32 accumulators in TMEM), warps 2..9 drain accumulators.  16-bit
+//                         MMAs (128 x 256 x 16, fp32 accumulators in TMEM), warps 4..11 drain accumulators.  16-bit
 //                         mode double-buffers the accumulator (2 x 256 TMEM columns) so that the drain of one tile
 //                         overlaps the MMAs of the next; in fp32 mode a buffer is a chunk of TC_CHUNK_KB k-blocks, and
 //                         the drain warps keep the running sum of the chunks in registers.
@@ -29,17 +31,53 @@ namespace nmg {
 // =========================================================================================================
 // Expansion pass
 // =========================================================================================================
-__device__ __forceinline__ void split3(float f, __nv_bfloat16 &hi, __nv_bfloat16 &mid, __nv_bfloat16 &lo) {
-    hi = __float2bfloat16_rn(f);
-    const float r1 = f - __bfloat162float(hi);
-    mid = __float2bfloat16_rn(r1);
-    lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
+// fp32 operands run as two fp16 planes, x = (h + l) 2^e with h = fp16(x 2^-e), l = fp16(x 2^-e - h) and one exponent e per row of the
+// operand that brings the row's largest magnitude to [2^14, 2^15).  Three products (wl xh, wh xl, wh xh) then stand for the fp32 product:
+// what h + l leaves of a value and the dropped wl xl are at most 2^-22 of it, and a value below 2^-18 of its row's largest keeps an
+// absolute 2^-40 of that.  Against three bf16 planes and six products (exact to 2^-24) that halves the tensor-core work, and the
+// result is closer to the exact one, because what dominates the error is the number of truncating additions in the accumulator
+// (see TcMode): half as many.  Relative error against fp64, 1:4: 1.1e-6 -> 0.3e-6 at 128 reduction elements, 3.4e-6 -> 1.7e-6 from 3072;
+// lower in every row and column too, for normal, heavy-tailed and very large or small values, rows of different scale and outliers.
+// Time, 4096 tokens, 1:4: the matmul 3072 <- 768 86 -> 56 us, the whole call 4096 <- 4096 about 560 -> 303 us.
+//
+// Activation rows whose values are mostly far below the largest (a mask value, a saturated feature) are two rows: the values from
+// 2^-16 of the largest on, and the rest with an exponent of its own (down to about 2^-120 of the other; what lies further below loses
+// bits and then is zero) and its own planes.  A tile that holds such a row runs its reduction twice, over either pair of planes.
+__device__ __forceinline__ int line_exp(uint32_t max_bits) {  // infinities and NaN count as the largest finite value
+    const int e = (int)(max_bits >> 23) - (127 + 14);
+    return max_bits == 0 ? 0 : e < -126 ? -126 : e > 113 ? 113 : e;
 }
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 <= e <= 127
+// v 2^(er + ec) with the row's and the column's factor.  A factor below one comes first: the other order could overflow on the way.
+__device__ __forceinline__ float unscale(float v, float row_small, float row_large, float col) { return v * row_small * col * row_large; }
+// What a row's values are like: largest magnitude, sum of the exponents and number of the values that are not zero.
+struct RowStats {
+    uint32_t mx = 0, exps = 0, count = 0;
+    __device__ __forceinline__ void add(float v) {
+        const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
+        mx = max(mx, u);
+        exps += u >> 23;
+        count += u != 0;
+    }
+    // The mean exponent of the values is more than 16 below the largest one's.  (Infinities and NaN: such a row's results are not finite.)
+    __device__ __forceinline__ bool wide() const { return mx < 0x7f800000u && (uint64_t)exps + 16ull * count < (uint64_t)(mx >> 23) * count; }
+};
+__device__ __forceinline__ bool is_small(float v, uint32_t mx) { return (__float_as_uint(v) & 0x7fffffffu) < mx - min(mx, 16u << 23); }  // of a wide row
+constexpr float NOT_WIDE = -1.f;  // in place of the factor between the two parts of a row
+// two scaled values -> one word of each plane
+__device__ __forceinline__ void split2_pair(float a, float b, uint32_t &hi, uint32_t &lo) {
+    const __half2 h = __floats2half2_rn(a, b);
+    const float2 f = __half22float2(h);
+    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+    hi = *reinterpret_cast<const uint32_t *>(&h);
+    lo = *reinterpret_cast<const uint32_t *>(&l);
+}
+constexpr int SPLIT_PLANES = 2, ACT_PLANES = 4;
 
 // Move `cnt` (1..8) consecutive elements of a shared-memory line to the destination planes and clear them in shared
 // memory.  VEC: cnt == 8 and both sides are 16-byte aligned.
-// PLAIN (fp32 only): the destination is an fp32 matrix, not three bf16 planes (the densifier's use of this pass).
-template <typename T, bool VEC, bool PLAIN> __device__ __forceinline__ void expand_flush(const ExpandParams &p, T *line, int64_t off, int cnt) {
+// PLAIN (fp32 only): the destination is an fp32 matrix, not two fp16 planes of values times `scale` (the densifier's use of this pass).
+template <typename T, bool VEC, bool PLAIN> __device__ __forceinline__ void expand_flush(const ExpandParams &p, T *line, int64_t off, int cnt, float scale) {
     if constexpr (sizeof(T) == 4 && PLAIN) {
         float *d = static_cast<float *>(p.dst) + off;
         if (VEC) {
@@ -59,32 +97,34 @@ template <typename T, bool VEC, bool PLAIN> __device__ __forceinline__ void expa
             for (int i = 0; i < cnt; i++) { d[i] = line[i]; line[i] = DT<T>::from_f32(0.f); }
         }
     } else {
-        __nv_bfloat16 *d = static_cast<__nv_bfloat16 *>(p.dst) + off;
+        __half *d = static_cast<__half *>(p.dst) + off;
         if (VEC) {
             const float4 a = *reinterpret_cast<const float4 *>(line), b = *reinterpret_cast<const float4 *>(line + 4);
             *reinterpret_cast<float4 *>(line) = make_float4(0.f, 0.f, 0.f, 0.f);
             *reinterpret_cast<float4 *>(line + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-            const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-            uint32_t w[3][4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-                __nv_bfloat16 x[3], y[3];
-                split3(f[2 * i], x[0], x[1], x[2]);
-                split3(f[2 * i + 1], y[0], y[1], y[2]);
-#pragma unroll
-                for (int c = 0; c < 3; c++) w[c][i] = (uint32_t)__bfloat16_as_ushort(x[c]) | ((uint32_t)__bfloat16_as_ushort(y[c]) << 16);
-            }
-#pragma unroll
-            for (int c = 0; c < 3; c++) *reinterpret_cast<uint4 *>(d + c * p.plane_elems) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
+            uint4 h, l;
+            split2_pair(a.x * scale, a.y * scale, h.x, l.x);
+            split2_pair(a.z * scale, a.w * scale, h.y, l.y);
+            split2_pair(b.x * scale, b.y * scale, h.z, l.z);
+            split2_pair(b.z * scale, b.w * scale, h.w, l.w);
+            *reinterpret_cast<uint4 *>(d) = h;
+            *reinterpret_cast<uint4 *>(d + p.plane_elems) = l;
         } else {
             for (int i = 0; i < cnt; i++) {
-                __nv_bfloat16 x[3];
-                split3(line[i], x[0], x[1], x[2]);
+                const float x = line[i] * scale;
+                const __half h = __float2half_rn(x);
                 line[i] = 0.f;
-                for (int c = 0; c < 3; c++) d[c * p.plane_elems + i] = x[c];
+                d[i] = h;
+                d[p.plane_elems + i] = __float2half_rn(x - __half2float(h));
             }
         }
     }
+}
+// Largest magnitude of a line of the destination, from its parts
+__device__ __forceinline__ uint32_t line_max(const ExpandParams &p, int64_t line) {
+    uint32_t mx = 0;
+    for (int s = 0; s < p.spans; s++) mx = max(mx, p.maxima[s * p.lines + line]);
+    return mx;
 }
 
 // Work item = (column chunk kc, R consecutive row-blocks).  The item's dense tile lives in shared memory, in the
@@ -99,8 +139,10 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_dense_kernel(const Expa
     constexpr bool VEC_OK = N_ > 0;
     const int n = N_ > 0 ? N_ : prm.n, m = prm.m, g = prm.g, cc = prm.cc, R = prm.R, pitch = prm.pitch;
     const int lines = TR ? cc : R * m;
+    constexpr bool SCALED = sizeof(T) == 4 && !PLAIN;
     T *tile = reinterpret_cast<T *>(smem);                                  // [lines][pitch]
-    int8_t *ord = reinterpret_cast<int8_t *>(tile + (size_t)lines * pitch);  // [C][n]
+    float *scale = reinterpret_cast<float *>(tile + (size_t)lines * pitch);  // SCALED: [lines]
+    int8_t *ord = reinterpret_cast<int8_t *>(scale + (SCALED ? lines : 0));  // [C][n]
     // The matmul kernel that follows is launched with programmatic stream serialization: it may become resident and run
     // its prologue while this grid drains, and reads nothing this grid writes before its griddepcontrol.wait.
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -116,9 +158,18 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_dense_kernel(const Expa
         const int64_t kc = item / groups, mb0 = (item - kc * groups) * R;
         const int rj = (int)(prm.nb - mb0 < R ? prm.nb - mb0 : R);  // row-blocks in this item
         __syncthreads();  // the tile is all zeros again
+        const int64_t col0 = kc * cc, r0 = mb0 * m;
+        if constexpr (SCALED) {
+            const int64_t first = TR ? col0 : r0, extent = TR ? prm.K : prm.M;
+            for (int l = threadIdx.x; l < lines; l += EXPAND_THREADS) {
+                if (first + l >= extent) continue;
+                const int e = line_exp(line_max(prm, first + l));
+                scale[l] = pow2(-e);
+                if ((TR ? mb0 : kc) == 0) prm.factors[first + l] = pow2(e);
+            }
+        }
         expand_scatter_item<T, TR, N_>(prm, tile, ord, kc, mb0, rj);
         __syncthreads();
-        const int64_t col0 = kc * cc, r0 = mb0 * m;
         // line l, elements e .. e+7 -> dst[(TR ? col0 + l : r0 + l)][(TR ? r0 : col0) + e]
         const int64_t line_lim = TR ? prm.K - col0 : prm.M - r0;   // lines inside the weight
         const int64_t elem_lim = TR ? prm.M - r0 : prm.K - col0;   // elements of a line inside the weight
@@ -136,11 +187,11 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_dense_kernel(const Expa
             // A full vector may run past the item's elements only into the row's padding (last chunk / last group:
             // ld = round_up(extent, 8)), never into elements another item owns.
             if (aligned && (e + 8 <= ne || ne >= elem_lim)) {
-                expand_flush<T, true, PLAIN>(prm, line, off, 8);
+                expand_flush<T, true, PLAIN>(prm, line, off, 8, SCALED ? scale[l] : 1.f);
             } else {
                 int cnt = ne - e < 8 ? ne - e : 8;
                 if (elem_lim - e < cnt) cnt = (int)(elem_lim - e);
-                expand_flush<T, false, PLAIN>(prm, line, off, cnt);
+                expand_flush<T, false, PLAIN>(prm, line, off, cnt, SCALED ? scale[l] : 1.f);
                 // elements of the vector past cnt were never written by this item's valid slots; clear them anyway
                 for (int i = cnt; i < 8; i++) line[i] = DT<T>::from_f32(0.f);
             }
@@ -158,8 +209,10 @@ template <typename T, int N_, bool PLAIN>
 __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const ExpandParams prm) {
     extern __shared__ __align__(16) char smem[];
     const int m = prm.m, g = prm.g, cc = prm.cc, R = prm.R, Q = prm.Q, cols = Q * cc, rows = R * m;
+    constexpr bool SCALED = sizeof(T) == 4 && !PLAIN;
     T *tile = reinterpret_cast<T *>(smem);                                 // [rows][cols]
-    int8_t *ord = reinterpret_cast<int8_t *>(tile + (size_t)rows * cols);  // [C][n]
+    float *scale = reinterpret_cast<float *>(tile + (size_t)rows * cols);  // SCALED: [rows]
+    int8_t *ord = reinterpret_cast<int8_t *>(scale + (SCALED ? rows : 0));  // [C][n]
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");        // see expand_dense_kernel
 
     constexpr int VL = N_ * (int)sizeof(T) / 2;  // 16-byte loads of values per 8 slots
@@ -170,8 +223,10 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
     const int groups = (int)((prm.nb + R - 1) / R), spans = (int)((prm.nc + Q - 1) / Q);
     const int64_t items = (int64_t)groups * spans;
     uint4 iv, vv[VL];
+    uint32_t mx = 0;  // SCALED: largest magnitude of row tid
     auto load = [&](int64_t item) {
         const int span = (int)(item / groups), grp = (int)(item - (int64_t)span * groups);
+        if constexpr (SCALED) if (tid < rows && (int64_t)grp * rows + tid < prm.lines) mx = line_max(prm, (int64_t)grp * rows + tid);
         iv = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);  // column -1: no slot
         if (!has || span * Q + uq >= prm.nc || grp * R + uj >= prm.nb) return;
         const int64_t slot = ((int64_t)(span * Q + uq) * prm.nb + grp * R + uj) * cc + uslot;
@@ -195,6 +250,14 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
     for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
         const int16_t *ci = reinterpret_cast<const int16_t *>(&iv);
         const T *vals = reinterpret_cast<const T *>(vv);
+        if constexpr (SCALED) {
+            if (tid < rows) {
+                const int e = line_exp(mx);
+                const int64_t row = (item % groups) * rows + tid;
+                scale[tid] = pow2(-e);
+                if (item < groups && row < prm.M) prm.factors[row] = pow2(e);
+            }
+        }
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             const int c = ci[k];
@@ -227,7 +290,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
                 if (inside) *reinterpret_cast<uint4 *>(static_cast<T *>(prm.dst) + off) = *reinterpret_cast<const uint4 *>(line);
                 *reinterpret_cast<uint4 *>(line) = make_uint4(0, 0, 0, 0);
             } else {
-                if (inside) expand_flush<T, true, PLAIN>(prm, line, off, V);
+                if (inside) expand_flush<T, true, PLAIN>(prm, line, off, V, scale[l]);
                 else {
                     reinterpret_cast<uint4 *>(line)[0] = make_uint4(0, 0, 0, 0);
                     reinterpret_cast<uint4 *>(line)[1] = make_uint4(0, 0, 0, 0);
@@ -240,7 +303,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
     }
 }
 // R and Q of the rows kernel, false when it does not serve the weight
-static bool expand_rows_plan(const Geo &geo, size_t es, int *R, int *Q, size_t *smem) {
+static bool expand_rows_plan(const Geo &geo, size_t es, bool scaled, int *R, int *Q, size_t *smem) {
     if (geo.n < 1 || geo.n > 2 || geo.cc % 8 != 0 || geo.nb > 0x3fffffff || geo.nc > 0x3fffffff) return false;
     int q = 512 / geo.cc;
     if (q < 1) q = 1;
@@ -249,11 +312,12 @@ static bool expand_rows_plan(const Geo &geo, size_t es, int *R, int *Q, size_t *
     int r = EXPAND_THREADS * 8 / cols;                                  // one piece per thread
     const int fit = (int)(32 * 1024 / ((size_t)geo.m * cols * es));     // seven CTAs per SM
     if (r > fit) r = fit;
+    if (scaled && r * geo.m > EXPAND_THREADS) r = EXPAND_THREADS / geo.m;  // a thread per row for the scales
     if (r < 1) r = 1;
     const size_t bytes = (size_t)r * geo.m * cols * es;
-    if (bytes > 64 * 1024 || r * cols / 8 > EXPAND_THREADS) return false;
+    if (bytes > 64 * 1024 || r * cols / 8 > EXPAND_THREADS || (scaled && geo.m > EXPAND_THREADS)) return false;
     *R = r; *Q = q;
-    *smem = bytes + (size_t)geo.C * geo.n + 16;
+    *smem = bytes + (scaled ? (size_t)r * geo.m * 4 : 0) + (size_t)geo.C * geo.n + 16;
     return true;
 }
 
@@ -270,10 +334,289 @@ static int expand_rows_per_item(const Geo &geo, size_t es, bool tr) {
 }
 
 // =========================================================================================================
+// fp32 operands: row maxima and planes of the activation
+// =========================================================================================================
+// Largest magnitudes of the weight's destination lines (weight rows, or columns for the transposed product), by parts: a unit is one
+// row-block (chunk of columns) and a span of its tiles.  Magnitudes are compared as integers: NaN is largest.
+struct AbsMaxParams {
+    const float *val;
+    const int16_t *idx;
+    const int8_t *order;    // [C][n]
+    uint32_t *maxima;       // [spans][lines]
+    int64_t nb, nc, lines;
+    int n, m, g, cc, transposed;
+    int spans, per;         // parts of a line, tiles per part
+};
+constexpr int PREP_THREADS = 128;
+__device__ __forceinline__ uint32_t magnitude(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+
+__device__ __forceinline__ void weight_absmax_unit(const AbsMaxParams &p, int64_t unit, uint32_t *mx) {
+    const int64_t group = unit / p.spans;
+    if (group >= (p.transposed ? p.nc : p.nb)) return;  // all threads
+    const int span = (int)(unit - group * p.spans), cc = p.cc, lines = p.transposed ? cc : p.m;
+    const int64_t tiles = p.transposed ? p.nb : p.nc, first = (int64_t)span * p.per;
+    const int count = (int)(tiles - first < p.per ? (tiles - first > 0 ? tiles - first : 0) : p.per);
+    for (int l = threadIdx.x; l < lines; l += (int)blockDim.x) mx[l] = 0;
+    __syncthreads();
+    const bool quads = (p.g & 3) == 0;  // four consecutive slots belong to one pattern
+    for (int64_t e = (int64_t)threadIdx.x * 4; e < (int64_t)count * cc; e += (int)blockDim.x * 4) {
+        const int t = (int)(e / cc), s0 = (int)(e - (int64_t)t * cc), left = cc - s0 < 4 ? cc - s0 : 4;
+        // tiles of consecutive row-blocks of one chunk are consecutive in memory
+        const int64_t slot = (p.transposed ? group * p.nb + first + t : (first + t) * p.nb + group) * cc + s0;
+        if (left == 4 && quads && !p.transposed) {
+            for (int i = 0; i < p.n; i++) {
+                uint32_t v = 0;
+#pragma unroll
+                for (int u = 0; u < 4; u++) v = max(v, magnitude(__ldg(p.val + (slot + u) * p.n + i)));
+                atomicMax(&mx[p.order[(s0 / p.g) * p.n + i]], v);
+            }
+            continue;
+        }
+        // cc need not be a multiple of four: a piece that crosses into the next tile is finished slot by slot
+        for (int u = 0; u < 4 && e + u < (int64_t)count * cc; u++) {
+            const int tu = s0 + u < cc ? t : (int)((e + u) / cc), su = (int)(e + u - (int64_t)tu * cc);
+            const int64_t sl = (p.transposed ? group * p.nb + first + tu : (first + tu) * p.nb + group) * cc + su;
+            const int c = p.transposed ? p.idx[sl] : 0;
+            if ((unsigned)c >= (unsigned)cc) continue;  // a malformed index is ignored, never dereferenced
+            uint32_t all = 0;
+            for (int i = 0; i < p.n; i++) {
+                const uint32_t v = magnitude(__ldg(p.val + sl * p.n + i));
+                if (p.transposed) all = max(all, v);
+                else atomicMax(&mx[p.order[(su / p.g) * p.n + i]], v);
+            }
+            if (p.transposed) atomicMax(&mx[c], all);
+        }
+    }
+    __syncthreads();
+    for (int l = threadIdx.x; l < lines; l += (int)blockDim.x) p.maxima[span * p.lines + group * lines + l] = mx[l];
+}
+
+struct SplitParams {
+    const float *src;
+    __half *dst;            // [ACT_PLANES][rows][ld]: the rows' planes, then those of wide rows' small values
+    float *factors;         // [rows] 2^e
+    float *small;           // [rows] factor of the small values' planes relative to the others, or NOT_WIDE
+    int64_t rows, cols, ld_src, ld;
+    int64_t ctas;           // CTAs (clusters) of the activation; those behind them take the weight's units
+    int per;                // K-major source: reduction elements per CTA, a multiple of 64
+};
+// Scales and factors of a row of the given largest magnitudes (small: of a wide row's small values, else 0)
+__device__ __forceinline__ void write_factors(const SplitParams &p, int64_t r, bool wide, uint32_t mx, uint32_t mx_small) {
+    const int e = line_exp(mx), d = line_exp(mx_small) - e;
+    p.factors[r] = pow2(e);
+    p.small[r] = !wide ? NOT_WIDE : d >= -126 ? pow2(d) : d >= -149 ? __uint_as_float(1u << (149 + d)) : 0.f;
+}
+__device__ __forceinline__ void store_planes(const SplitParams &p, int plane, int64_t r, int64_t c, const float (&f)[8], float s) {
+    uint4 h, l;
+    split2_pair(f[0] * s, f[1] * s, h.x, l.x);
+    split2_pair(f[2] * s, f[3] * s, h.y, l.y);
+    split2_pair(f[4] * s, f[5] * s, h.z, l.z);
+    split2_pair(f[6] * s, f[7] * s, h.w, l.w);
+    __half *d = p.dst + (plane * p.rows + r) * p.ld + c;
+    *reinterpret_cast<uint4 *>(d) = h;
+    *reinterpret_cast<uint4 *>(d + p.rows * p.ld) = l;
+}
+__device__ __forceinline__ void store_split(const SplitParams &p, int64_t r, int64_t c, const float (&f)[8], bool wide, uint32_t mx, float s, float s_small) {
+    if (!wide) { store_planes(p, 0, r, c, f, s); return; }
+    float big[8], small[8];
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+        const bool sm = is_small(f[i], mx);
+        big[i] = sm ? 0.f : f[i];
+        small[i] = sm ? f[i] : 0.f;
+    }
+    store_planes(p, 0, r, c, big, s);
+    store_planes(p, 2, r, c, small, s_small);
+}
+
+// CTAs of the activation: one row per CTA, or one per warp where a warp's registers hold it (ROWS = 4).  The row is read once for what
+// its values are like and kept; what the registers do not hold is read again.  HBM-bound, 8 bytes per value.
+template <int ROWS>
+__global__ void __launch_bounds__(PREP_THREADS) split_rows_kernel(const SplitParams p, const AbsMaxParams w) {
+    extern __shared__ uint32_t mx[];
+    __shared__ RowStats warp_stats[PREP_THREADS / 32];
+    __shared__ uint32_t warp_small[PREP_THREADS / 32];
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (blockIdx.x >= p.ctas) { weight_absmax_unit(w, blockIdx.x - p.ctas, mx); return; }
+    constexpr int LANES = PREP_THREADS / ROWS, HELD = 4;
+    const int sub = threadIdx.x / LANES, tid = threadIdx.x - sub * LANES;
+    const int64_t r = (int64_t)blockIdx.x * ROWS + sub;
+    if (ROWS > 1 && r >= p.rows) return;  // whole warps
+    const float *row = p.src + r * p.ld_src;
+    const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
+    auto load = [&](int64_t c, float (&f)[8]) {
+        if (vec && c + 8 <= p.cols) {
+            const float4 a = __ldg(reinterpret_cast<const float4 *>(row + c)), b = __ldg(reinterpret_cast<const float4 *>(row + c + 4));
+            f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
+        } else {
+#pragma unroll
+            for (int i = 0; i < 8; i++) f[i] = c + i < p.cols ? row[c + i] : 0.f;
+        }
+    };
+    float held[HELD][8];
+    auto each = [&](auto &&fn) {  // fn(column, eight values), of this thread's part of the row
+#pragma unroll
+        for (int h = 0; h < HELD; h++) {
+            const int64_t c = ((int64_t)h * LANES + tid) * 8;
+            if (c < p.ld) fn(c, held[h]);
+        }
+        for (int64_t c = ((int64_t)HELD * LANES + tid) * 8; c < p.ld; c += LANES * 8) {
+            float f[8];
+            load(c, f);
+            fn(c, f);
+        }
+    };
+#pragma unroll
+    for (int h = 0; h < HELD; h++) {
+        const int64_t c = ((int64_t)h * LANES + tid) * 8;
+        if (c < p.ld) load(c, held[h]);
+    }
+    RowStats st;
+    each([&](int64_t, const float (&f)[8]) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) st.add(f[i]);
+    });
+    st.mx = __reduce_max_sync(0xffffffffu, st.mx);
+    st.exps = __reduce_add_sync(0xffffffffu, st.exps);
+    st.count = __reduce_add_sync(0xffffffffu, st.count);
+    if constexpr (ROWS == 1) {
+        if ((threadIdx.x & 31) == 0) warp_stats[threadIdx.x >> 5] = st;
+        __syncthreads();
+        st = RowStats();
+#pragma unroll
+        for (int i = 0; i < PREP_THREADS / 32; i++) {
+            st.mx = max(st.mx, warp_stats[i].mx);
+            st.exps += warp_stats[i].exps;
+            st.count += warp_stats[i].count;
+        }
+    }
+    const bool wide = st.wide();  // of the whole row: the same for all its threads
+    uint32_t mx_small = 0;
+    if (wide) {
+        each([&](int64_t, const float (&f)[8]) {
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+                if (is_small(f[i], st.mx)) mx_small = max(mx_small, magnitude(f[i]));
+        });
+        mx_small = __reduce_max_sync(0xffffffffu, mx_small);
+        if constexpr (ROWS == 1) {
+            if ((threadIdx.x & 31) == 0) warp_small[threadIdx.x >> 5] = mx_small;
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < PREP_THREADS / 32; i++) mx_small = max(mx_small, warp_small[i]);
+        }
+    }
+    if (tid == 0) write_factors(p, r, wide, st.mx, mx_small);
+    const float s = pow2(-line_exp(st.mx)), s_small = pow2(-line_exp(mx_small));
+    each([&](int64_t c, const float (&f)[8]) { store_split(p, r, c, f, wide, st.mx, s, s_small); });
+}
+
+// The same from a K-major activation src[red][ld_src >= tokens], transposed on the way.  A cluster owns 32 tokens and its CTAs a part
+// of the reduction axis each; what the tokens' values are like is put together through distributed shared memory, so that this is
+// one launch.  The first COLS_HELD reduction elements of a CTA's part stay in shared memory, the others are read again (from L2).
+constexpr int COLS_THREADS = 256, COLS_HELD = 256, COLS_CLUSTER = 8;
+__global__ void __launch_bounds__(COLS_THREADS) split_columns_kernel(const SplitParams p, const AbsMaxParams w) {
+    extern __shared__ uint32_t mx[];
+    __shared__ float tile[COLS_HELD][33];          // [reduction][token]
+    __shared__ RowStats part[COLS_THREADS / 32][32];
+    __shared__ RowStats ranks[COLS_CLUSTER][32];   // written by the cluster's CTAs
+    __shared__ uint32_t ranks_small[COLS_CLUSTER][32];
+    const int cl = (int)gridDim.x, rank = (int)blockIdx.x;  // a cluster is a row of the grid
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (blockIdx.y >= p.ctas) {  // whole clusters
+        const int64_t unit = (int64_t)(blockIdx.y - p.ctas) * cl + rank;
+        weight_absmax_unit(w, unit, mx);
+        return;
+    }
+    cluster_arrive();  // waited for before anything is written to another CTA
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t t0 = (int64_t)blockIdx.y * 32, t = t0 + lane, k0 = (int64_t)rank * p.per;
+    const int count = (int)(p.cols - k0 < p.per ? (p.cols - k0 > 0 ? p.cols - k0 : 0) : p.per);  // of this CTA's part
+    auto at = [&](int k) -> float { return k < count && t < p.rows ? __ldg(p.src + (k0 + k) * p.ld_src + t) : 0.f; };
+    RowStats st;
+#pragma unroll 8
+    for (int k = warp; k < COLS_HELD; k += COLS_THREADS / 32) {
+        const float v = at(k);
+        tile[k][lane] = v;
+        st.add(v);
+    }
+#pragma unroll 8
+    for (int k = COLS_HELD + warp; k < count; k += COLS_THREADS / 32) st.add(at(k));
+    part[warp][lane] = st;
+    __syncthreads();
+    cluster_wait();
+    if (warp == 0) {
+        for (int i = 1; i < COLS_THREADS / 32; i++) {
+            const RowStats o = part[i][lane];
+            st.mx = max(st.mx, o.mx);
+            st.exps += o.exps;
+            st.count += o.count;
+        }
+        for (int c = 0; c < cl; c++) {
+            const uint32_t dst = map_to_rank(smem_u32(&ranks[rank][lane]), (uint32_t)c);
+            st_cluster(dst, st.mx);
+            st_cluster(dst + 4, st.exps);
+            st_cluster(dst + 8, st.count);
+        }
+    }
+    cluster_sync_all();
+    auto gather = [&](int token, uint32_t &m_small) -> RowStats {
+        RowStats a;
+        m_small = 0;
+        for (int c = 0; c < cl; c++) {
+            const RowStats o = ranks[c][token];
+            a.mx = max(a.mx, o.mx);
+            a.exps += o.exps;
+            a.count += o.count;
+        }
+        return a;
+    };
+    uint32_t mx_small;
+    st = gather(lane, mx_small);
+    const bool any_wide = __any_sync(0xffffffffu, st.wide());  // the same in every warp of the cluster
+    if (any_wide) {
+        for (int k = warp; k < count; k += COLS_THREADS / 32) {
+            const float v = k < COLS_HELD ? tile[k][lane] : at(k);
+            if (is_small(v, st.mx)) mx_small = max(mx_small, magnitude(v));
+        }
+        part[warp][lane].mx = mx_small;
+        __syncthreads();
+        if (warp == 0) {
+            for (int i = 1; i < COLS_THREADS / 32; i++) mx_small = max(mx_small, part[i][lane].mx);
+            for (int c = 0; c < cl; c++) st_cluster(map_to_rank(smem_u32(&ranks_small[rank][lane]), (uint32_t)c), mx_small);
+        }
+        cluster_sync_all();
+    }
+    const int tok = threadIdx.x >> 3, c8 = (threadIdx.x & 7) * 8;  // eight reduction elements of one token
+    st = gather(tok, mx_small);
+    const bool wide = st.wide();
+    if (wide)
+        for (int c = 0; c < cl; c++) mx_small = max(mx_small, ranks_small[c][tok]);
+    if (rank == 0 && c8 == 0 && t0 + tok < p.rows) write_factors(p, t0 + tok, wide, st.mx, mx_small);
+    const float s = pow2(-line_exp(st.mx)), s_small = pow2(-line_exp(mx_small));
+    for (int kb = 0; kb < count; kb += 64) {
+        const int base = kb < COLS_HELD ? kb : 0;
+        if (kb >= COLS_HELD) {
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 8; i++) tile[warp * 8 + i][lane] = at(kb + warp * 8 + i);
+            __syncthreads();
+        }
+        const int64_t k = k0 + kb + c8;
+        if (t0 + tok < p.rows && k < p.ld) {
+            float f[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) f[i] = tile[base + c8 + i][tok];
+            store_split(p, t0 + tok, k, f, wide, st.mx, s, s_small);
+        }
+    }
+}
+
+// =========================================================================================================
 // Dense-operand matmul
 // =========================================================================================================
 constexpr int GEMM_DRAIN_WARPS = 8;   // two per TMEM lane quarter, each takes half of the accumulator's columns
-constexpr int GEMM_THREADS = 32 * (2 + GEMM_DRAIN_WARPS);  // TMA warp, MMA warp, drain warps
+constexpr int GEMM_THREADS = 32 * (4 + GEMM_DRAIN_WARPS);  // TMA warp, MMA warp, two idle ones, drain warps
 constexpr int GEMM_RING_BYTES = TC_STAGES * (TC_A_BYTES + TC_B_BYTES);  // 192 KB of operand stages in either mode
 
 // The output's tiles: the first f_wide rows of tiles are bn columns wide, the f_narrow rows below them bn_tail.
@@ -305,15 +648,20 @@ struct GemmParams {
     GemmTiles tiles;       // one CTA per tile of 128 features, or a pair per 256
     int band;              // width of the tile order's bands, in feature tiles
     unsigned *wave_ctr;    // zeroed counter for the producers' soft rendezvous before every tile, or NULL
+    const float *fac_rows, *fac_cols;  // fp32: factors of the accumulator's rows and columns (2^line_exp)
+    const float *small;                // fp32: of the activation's rows, see SplitParams
+    int a_rows, b_rows;                // rows of a plane
     int *status;
 };
+template <typename T> struct GemmElem { using type = T; };  // what the tensor cores multiply
+template <> struct GemmElem<float> { using type = __half; };
 constexpr int GEMM_STAGING_BYTES = GEMM_DRAIN_WARPS * 4096;  // per drain warp: 32 feature rows x 128 bytes
 
 struct GemmMaps {
-    CUtensorMap a[3];  // weight planes, box 64 x 128, 128-byte swizzle
-    CUtensorMap b[3];  // activation planes, box 64 x bn (64 x bn / 2 for CTA pairs)
-    CUtensorMap b_tail[3];  // the same with the box of the narrow tiles
-    CUtensorMap out;   // out_tma: the output, box 128 bytes x 32 rows, 128-byte swizzle
+    CUtensorMap a;       // row operand, its planes below one another, box 64 x 128, 128-byte swizzle
+    CUtensorMap b;       // column operand, box 64 x bn (64 x bn / 2 for CTA pairs)
+    CUtensorMap b_tail;  // the same with the box of the narrow tiles
+    CUtensorMap out;     // out_tma: the output, box 128 bytes x 32 rows, 128-byte swizzle (fp32: 64 bytes, 64-byte swizzle)
 };
 
 // PAIR = false: one CTA per 128-feature x 256-token tile.
@@ -323,23 +671,22 @@ struct GemmMaps {
 // 48 KB, which is what keeps the tensor core fed from L2.  full[s] lives in the even ("leader") CTA and receives the TMA
 // bytes of both; empty[s] and acc_full[b] exist in both CTAs and are signalled by multicast commits; acc_free[b] lives in
 // the leader and collects the drain warps of both CTAs.  No load is multicast.
-// fp32 (always pairs): a stage is one k-block of all six planes, 96 KB, and its six products run from it.  With a stage per
-// product (48 KB per 512 clocks and SM, over what L2 delivers) and the running sum in the second TMEM buffer the MMAs waited
-// for loads and for every promotion: 4096 tokens, 3072 <- 768 took 104 us, now 86, at the rate of a long cuBLAS product but for the last wave.
+// fp32 (always pairs): a stage is one k-block of all four planes, 64 KB, and its three products run from it (a stage per product
+// would take more than L2 delivers).
 // TMA_OUT = true: the one-destination staged output, leaving as tiled bulk stores; only that output path is compiled,
 // which keeps the drain warps' code and register needs small.  TMA_OUT = false: every other output form.
 template <typename T, bool PAIR, bool TMA_OUT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmParams prm, const __grid_constant__ GemmMaps maps) {
-    constexpr int TERMS = TcMode<T>::TERMS;
-    using E = typename TcMode<T>::elem;
-    constexpr bool SPLIT = TERMS > 1;
+    constexpr bool SPLIT = sizeof(T) == 4;
+    constexpr int TERMS = SPLIT ? 3 : 1;
+    using E = typename GemmElem<T>::type;
     static_assert(PAIR || !SPLIT, "fp32 runs on CTA pairs");
     constexpr int NBUF = 2;  // accumulator tiles in flight between the MMA issuer and the drain warps
     constexpr uint32_t TMEM_COLS = NBUF * TC_ACC_COLS;
-    constexpr int PLANES = SPLIT ? 3 : 1;
+    constexpr int PLANES = SPLIT ? SPLIT_PLANES : 1;
     constexpr int B_BYTES = PAIR ? TC_B_BYTES / 2 : TC_B_BYTES;  // room of one plane; the widest tile fills it
     constexpr int OFF_B = PLANES * TC_A_BYTES, STAGE_BYTES = OFF_B + PLANES * B_BYTES;
-    constexpr int STAGES = GEMM_RING_BYTES / STAGE_BYTES;  // 4, 6 for pairs, 2 for fp32
+    constexpr int STAGES = GEMM_RING_BYTES / STAGE_BYTES;  // 4, 6 for pairs, 3 for fp32
     constexpr int TILE_FEATS = PAIR ? 2 * TC_BM : TC_BM;
 
     extern __shared__ char smem_raw[];
@@ -403,6 +750,21 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         tok0 = tile_t * bn;
     };
 
+    // fp32: whether the tile holds a wide row of the activation (all lanes of a warp ask together)
+    auto tile_wide = [&](int ti) -> bool {
+        if constexpr (!SPLIT) return false;
+        int feat0, tok0, bn;
+        tile_origin(ti, feat0, tok0, bn);
+        const int64_t first = prm.bias_cols ? feat0 - (int)rank * TC_BM : tok0, limit = prm.bias_cols ? prm.out_feats : prm.ntok;
+        bool wide = false;
+        for (int i = lane; i < (prm.bias_cols ? TILE_FEATS : bn); i += 32)
+            if (first + i < limit) wide |= prm.small[first + i] != NOT_WIDE;
+        return __any_sync(0xffffffffu, wide);
+    };
+
+    // fp32: the running sums take 128 registers of a drain warp.  Shares of the launch's 384 x 168: 128 x 56 + 256 x 224.
+    if (warp < 4) {
+    if constexpr (SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         // The warp stays converged and issues under elect_one (see there).
@@ -415,7 +777,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         for (int ti = 0; ti < my_tiles && ok; ti++) {
             int feat0, tok0, bn;
             tile_origin(ti, feat0, tok0, bn);
-            const CUtensorMap *bmap = narrow(ti) ? maps.b_tail : maps.b;
+            const CUtensorMap *bmap = narrow(ti) ? &maps.b_tail : &maps.b;
+            const int total = tile_wide(ti) ? 2 * nkb : nkb;  // a wide tile: the reduction over either pair of the activation's planes
             if (prm.wave_ctr && ti > 0) {
                 // CTAs whose tiles share operand panels read them from HBM once only while they stream through the
                 // reduction in step; left alone they drift apart over the waves (measured: 2.2 MB of DRAM reads per
@@ -426,7 +789,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 if (lane == 0) soft_rendezvous(prm.wave_ctr, arrivals, (uint64_t)nkb * 40);
                 __syncwarp();
             }
-            for (int kb = 0; kb < nkb; kb++, it++) {
+            for (int i = 0; i < total; i++, it++) {
+                const int kb = i < nkb ? i : i - nkb, x_plane = i < nkb ? 0 : 2;
                 const int s = it % STAGES;
                 const uint32_t ph = (uint32_t)((it / STAGES) & 1);
                 if (!(ok = __all_sync(0xffffffffu, wait(&empty[s], ph ^ 1, 21)))) break;
@@ -437,13 +801,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                         if (leader) mbar_expect_tx(&full[s], (uint32_t)(2 * PLANES * (TC_A_BYTES + half * TC_BK * 2)));  // both CTAs report to this barrier
 #pragma unroll
                         for (int c = 0; c < PLANES; c++) {
-                            tma_load_2d_pair(stage + c * TC_A_BYTES, &maps.a[c], kb * TC_BK, feat0, full_leader + s * 8);
-                            tma_load_2d_pair(stage + OFF_B + c * B_BYTES, &bmap[c], kb * TC_BK, tok0 + (int)rank * half, full_leader + s * 8);
+                            const int ap = prm.bias_cols ? c + x_plane : c, bp = prm.bias_cols ? c : c + x_plane;
+                            tma_load_2d_pair(stage + c * TC_A_BYTES, &maps.a, kb * TC_BK, ap * prm.a_rows + feat0, full_leader + s * 8);
+                            tma_load_2d_pair(stage + OFF_B + c * B_BYTES, bmap, kb * TC_BK, bp * prm.b_rows + tok0 + (int)rank * half, full_leader + s * 8);
                         }
                     } else {
                         mbar_expect_tx(&full[s], STAGE_BYTES);
-                        tma_load_2d(stage, &maps.a[0], kb * TC_BK, feat0, &full[s]);
-                        tma_load_2d(stage + TC_A_BYTES, &maps.b[0], kb * TC_BK, tok0, &full[s]);
+                        tma_load_2d(stage, &maps.a, kb * TC_BK, feat0, &full[s]);
+                        tma_load_2d(stage + TC_A_BYTES, &maps.b, kb * TC_BK, tok0, &full[s]);
                     }
                 }
                 __syncwarp();
@@ -452,15 +817,17 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (of the leader for pairs)
         if (leader) {
+            if constexpr (SPLIT) asm volatile("griddepcontrol.wait;" ::: "memory");  // tile_wide
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint64_t desc0 = make_sw128_desc(smem_u32(smem));
             bool ok = true;
             int it = 0, unit = 0;
             for (int ti = 0; ti < my_tiles && ok; ti++) {
-                int kb = 0;
+                const int units = tile_wide(ti) ? 2 * nchunks : nchunks;
                 uint32_t idesc = make_idesc<E>(!PAIR ? TC_BN : narrow(ti) ? prm.tiles.bn_tail : prm.tiles.bn);
                 if constexpr (PAIR) idesc = (idesc & ~(0x1fu << 24)) | ((uint32_t)(256 >> 4) << 24);  // M = 256 across the pair
-                for (int c = 0; c < nchunks && ok; c++, unit++) {
+                for (int c = 0; c < units && ok; c++, unit++) {
+                    int kb = (c < nchunks ? c : c - nchunks) * chunk_it;
                     const int b = unit % NBUF, use = unit / NBUF;
                     if (use > 0) ok = __all_sync(0xffffffffu, wait(&acc_free[b], (uint32_t)((use - 1) & 1), 26));
                     if (!ok) break;
@@ -477,7 +844,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
 #pragma unroll
                             for (int t = 0; t < TERMS; t++) {
                                 // bias_cols: the operands' roles are exchanged, the order of the products is not (equal results either way)
-                                const int ap = !SPLIT ? 0 : prm.bias_cols ? split_x(t) : split_w(t), bp = !SPLIT ? 0 : prm.bias_cols ? split_w(t) : split_x(t);
+                                const int wp = t == 0, xp = t == 1;  // planes of product t: the smallest first
+                                const int ap = !SPLIT ? 0 : prm.bias_cols ? xp : wp, bp = !SPLIT ? 0 : prm.bias_cols ? wp : xp;
                                 const uint64_t adesc = stage_a + (uint32_t)(ap * (TC_A_BYTES / 16)), bdesc = stage_b + (uint32_t)(bp * (B_BYTES / 16));
 #pragma unroll
                                 for (int k = 0; k < TC_BK / 16; k++) {  // 16 elements = 32 bytes = 2 descriptor units per step
@@ -499,7 +867,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 }
             }
         }
+    }
     } else {
+        if constexpr (SPLIT) asm volatile("setmaxnreg.inc.sync.aligned.u32 224;");
         // ------------------------------------------------------------------ drain warps: promotion and epilogue
         // Feature-major output (out[feature][token]) leaves through a per-warp staging tile: the warp's 32 features x
         // 128 bytes of tokens, 16-byte chunks XOR-swizzled by row.  TMEM hands every lane one feature row; the staging
@@ -513,7 +883,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         const int q = warp & 3;  // TMEM lane quarter this warp may access
         constexpr int SLICES = (TC_BN / 32) / (GEMM_DRAIN_WARPS / 4);  // 32-column slices per warp, at most
         const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
-        char *stage_w = staging + (warp - 2) * 4096;
+        char *stage_w = staging + (warp - 4) * 4096;
         const T *res = static_cast<const T *>(prm.residual);
         const bool gelu = prm.act == NMG_EPI_GELU;
         // The bias and the residual are read with ordinary loads, possibly before the first accumulator is ready: like the
@@ -521,12 +891,12 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         asm volatile("griddepcontrol.wait;" ::: "memory");
         int unit = 0;
         bool ok = true;
-        float run[SPLIT ? SLICES : 1][32];  // fp32: sum of the tile's finished chunks
+        uint32_t run[SPLIT ? SLICES : 1][32];  // fp32: sum of the tile's finished chunks
         for (int ti = 0; ti < my_tiles && ok; ti++) {
             int feat0, tok0, bn;
             tile_origin(ti, feat0, tok0, bn);
             // this warp's first slice and how many it has: whole staged groups, the first half of the warps takes the odd one
-            const int per_warp = (bn / GROUP_TOK + 1) / 2 * GROUP_SLICES, sl0 = ((warp - 2) >> 2) * per_warp;
+            const int per_warp = (bn / GROUP_TOK + 1) / 2 * GROUP_SLICES, sl0 = ((warp - 4) >> 2) * per_warp;
             const int nsl = min(per_warp, bn / 32 - sl0);
             const int64_t feat = (int64_t)feat0 + q * 32 + lane;
             const bool feat_ok = feat < prm.out_feats;
@@ -538,6 +908,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
             for (int i = 0; i < SLICES; i++) {
                 const int64_t col = (int64_t)tok0 + (sl0 + i) * 32 + lane;
                 bcol[i] = (prm.bias && prm.bias_cols && col < prm.ntok) ? DT<T>::to_f32(static_cast<const T *>(prm.bias)[col]) : 0.f;
+            }
+            // fp32: factors of this lane's row (see unscale)
+            float row_small = 1.f, row_large = 1.f;
+            const int units = tile_wide(ti) ? 2 * nchunks : nchunks;
+            if constexpr (SPLIT) {
+                const float f = feat_ok ? prm.fac_rows[feat] : 1.f;
+                (f < 1.f ? row_small : row_large) = f;
             }
             // The residual of a slice (this lane's row, 32 elements) is fetched in 16-byte pieces one slice ahead of its
             // use, like the accumulator, when the bulk-store path runs and the residual's rows allow it.
@@ -551,11 +928,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                     }
                 }
             };
-            for (int c = 0; c < nchunks; c++, unit++) {
+            for (int c = 0; c < units; c++, unit++) {
                 const int b = unit % NBUF, use = unit / NBUF;
                 if (!(ok = wait(&acc_full[b], (uint32_t)(use & 1), 25))) break;
                 tc_fence_after();
-                const bool last = c == nchunks - 1;
+                const bool last = c == units - 1;
                 auto release = [&]() {  // this warp's TMEM reads of the unit are done: the issuer may reuse the accumulator once all warps say so
                     tc_fence_before();
                     __syncwarp();
@@ -567,8 +944,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 // handle(sl, r, qr): slice sl of the unit is in registers r (this lane's feature row, 32 tokens); qr holds the
                 // same 32 elements of the residual when res_fetch found them loadable in 16-byte pieces
                 auto handle = [&](int sl, uint32_t (&r)[32], const uint4 (&qr)[RQ]) {
-                    if (sl == sl0 + nsl - 1) release();
+                    if (!(SPLIT && TMA_OUT) && sl == sl0 + nsl - 1) release();
                     const int64_t tokc = (int64_t)tok0 + sl * 32;
+                    if constexpr (SPLIT) {  // the columns' factors are padded to whole tiles
+                        const float4 *fac = reinterpret_cast<const float4 *>(prm.fac_cols + tokc);
+#pragma unroll
+                        for (int v = 0; v < 8; v++) {
+                            const float4 f = __ldg(fac + v);
+                            r[4 * v] = __float_as_uint(unscale(__uint_as_float(r[4 * v]), row_small, row_large, f.x));
+                            r[4 * v + 1] = __float_as_uint(unscale(__uint_as_float(r[4 * v + 1]), row_small, row_large, f.y));
+                            r[4 * v + 2] = __float_as_uint(unscale(__uint_as_float(r[4 * v + 2]), row_small, row_large, f.z));
+                            r[4 * v + 3] = __float_as_uint(unscale(__uint_as_float(r[4 * v + 3]), row_small, row_large, f.w));
+                        }
+                    }
                     // activation(product + bias), kept as fp32 bits in r.  The activation sits in one warp-uniform branch
                     // around its own unrolled loop: the 32 evaluations are independent and interleave, where a test per
                     // element would run them one after the other at full dependent latency.
@@ -608,6 +996,23 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                                 for (int j = 0; j < 32; j++)
                                     if (tokc + j < prm.ntok) r[j] = __float_as_uint(__uint_as_float(r[j]) + DT<T>::to_f32(res[feat * prm.ld_res + tokc + j]));
                             }
+                        }
+                        if constexpr (sizeof(T) == 4) {
+                            // Two halves of 32 rows x 64 bytes (64-byte swizzle), used in turn: a store reads one while the other is filled.
+#pragma unroll
+                            for (int h = 0; h < 2; h++) {
+                                char *half = stage_w + h * 2048 + lane * 64;
+                                if (lane == 0) tma_store_wait_read<1>();
+                                __syncwarp();
+#pragma unroll
+                                for (int v = 0; v < 4; v++)
+                                    *reinterpret_cast<uint4 *>(half + ((v ^ ((lane >> 1) & 3)) << 4)) =
+                                        make_uint4(r[16 * h + 4 * v], r[16 * h + 4 * v + 1], r[16 * h + 4 * v + 2], r[16 * h + 4 * v + 3]);
+                                fence_proxy_async_smem();
+                                __syncwarp();
+                                if (lane == 0) tma_store_2d(&maps.out, stage_w + h * 2048, (int)tokc + 16 * h, feat0 + q * 32);
+                            }
+                            return;
                         }
                         // registers -> staging row `lane` (16-byte chunks XOR-swizzled by row: the 128-byte swizzle of the
                         // output's tensor map), once the previous group's bulk store has read the tile
@@ -781,20 +1186,34 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 uint4 qa[RQ], qb[RQ];
                 const uint32_t acc_addr = lane_base + (uint32_t)(b * TC_ACC_COLS);
                 if constexpr (SPLIT) {
-                    if (nchunks > 1) {
-                        // promotion: the chunk joins the running sum; with the last one the total goes back to TMEM for the epilogue
+                    if (TMA_OUT || units > 1) {
+                        // Promotion: the chunk joins the running sum.  With the last one the accumulator is handed back and the epilogue
+                        // works on the registers (TMA_OUT), or the total returns to TMEM for it.
 #pragma unroll
                         for (int i = 0; i < SLICES; i++) {
                             if (i >= nsl) break;
                             tmem_ld32(acc_addr + (uint32_t)((sl0 + i) * 32), ra);
+                            if (c >= nchunks) {  // small values of wide rows: only those rows take them
+                                const int64_t col = (int64_t)tok0 + (sl0 + i) * 32 + lane;
+                                const float f = prm.bias_cols ? (feat_ok ? prm.small[feat] : NOT_WIDE) : col < prm.ntok ? prm.small[col] : NOT_WIDE;
 #pragma unroll
-                            for (int j = 0; j < 32; j++) {
-                                run[i][j] = c > 0 ? __fadd_rn(run[i][j], __uint_as_float(ra[j])) : __uint_as_float(ra[j]);
-                                ra[j] = __float_as_uint(run[i][j]);
+                                for (int j = 0; j < 32; j++) {
+                                    const float fj = prm.bias_cols ? f : __shfl_sync(0xffffffffu, f, j);
+                                    ra[j] = fj == NOT_WIDE ? 0u : __float_as_uint(__uint_as_float(ra[j]) * fj);
+                                }
                             }
-                            if (last) tmem_st32(acc_addr + (uint32_t)((sl0 + i) * 32), ra);
+#pragma unroll
+                            for (int j = 0; j < 32; j++) run[i][j] = c > 0 ? __float_as_uint(__fadd_rn(__uint_as_float(run[i][j]), __uint_as_float(ra[j]))) : ra[j];
+                            if (!TMA_OUT && last) tmem_st32(acc_addr + (uint32_t)((sl0 + i) * 32), run[i]);
                         }
-                        if (!last) { release(); continue; }
+                        if (TMA_OUT || !last) release();
+                        if (!last) continue;
+                        if constexpr (TMA_OUT) {
+#pragma unroll
+                            for (int i = 0; i < SLICES; i++)
+                                if (i < nsl) handle(sl0 + i, run[i], qa);
+                            continue;
+                        }
                     }
                 }
                 const int sl_end = sl0 + nsl;
@@ -840,10 +1259,89 @@ bool tc_dense_supported(const Geo &geo, int dtype) {
     return expand_smem_bytes(geo, es, false, 1) <= 200 * 1024 && expand_smem_bytes(geo, es, true, 1) <= 200 * 1024;
 }
 
+// Parts of a weight's line in the search for its largest magnitude: enough units to fill the chip, at least a tile each.
+static void split_spans(int64_t groups, int64_t tiles, int *spans, int *per) {
+    int64_t s = (4 * 148 + groups - 1) / groups;
+    if (s > 64) s = 64;
+    if (s > tiles) s = tiles;
+    if (s < 1) s = 1;
+    *per = (int)((tiles + s - 1) / s);
+    *spans = (int)((tiles + *per - 1) / *per);
+}
+// Behind an fp32 operand's planes: its rows' factors, read in whole tiles of columns, then ([lines] of a weight) the parts of the maxima.
+struct LineScales {
+    int spans, per;
+    int64_t lines, rows;  // lines of whole tiles, rows of the operand
+    size_t bytes() const { return factor_bytes(rows) + (size_t)spans * lines * 4; }
+    static size_t factor_bytes(int64_t rows) { return ((size_t)(rows + TC_BN) * 4 + 255) & ~(size_t)255; }
+};
+static LineScales weight_scales(const Geo &geo, bool transposed) {
+    LineScales l;
+    split_spans(transposed ? geo.nc : geo.nb, transposed ? geo.nb : geo.nc, &l.spans, &l.per);
+    l.lines = transposed ? geo.nc * geo.cc : geo.nb * geo.m;
+    l.rows = transposed ? geo.K : geo.M;
+    return l;
+}
+static size_t planes_bytes(int planes, int64_t rows, int64_t red) { return ((size_t)planes * (size_t)rows * (size_t)dense_ld(red) * 2 + 255) & ~(size_t)255; }
+
 size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed) {
     const int64_t rows = transposed ? geo.K : geo.M, red = transposed ? geo.M : geo.K;
-    const size_t planes = dtype == NMG_F32 ? 3 : 1;
-    return planes * (size_t)rows * (size_t)dense_ld(red) * 2 + 512;
+    if (dtype == NMG_F32) return planes_bytes(SPLIT_PLANES, rows, red) + weight_scales(geo, transposed).bytes() + 512;
+    return (size_t)rows * (size_t)dense_ld(red) * 2 + 512;
+}
+size_t tc_dense_act_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens) {
+    if (dtype != NMG_F32) return 0;
+    return planes_bytes(ACT_PLANES, tokens, transposed ? geo.M : geo.K) + 2 * LineScales::factor_bytes(tokens) + 512;
+}
+
+// The fp32 activation as planes in `buf`, and in the same launch the weight's maxima behind its planes in `dense`.
+static int split_operands(const Geo &geo, bool transposed, const void *val, const int16_t *idx, const void *act, int64_t ld_act, bool act_k_major, int64_t tokens,
+                          char *buf, uint32_t *weight_maxima, DenseAct *out, cudaStream_t st) {
+    const int64_t red = transposed ? geo.M : geo.K;
+    int rc;
+    PatternTable tab;
+    if ((rc = get_pattern_table(geo.n, geo.m, &tab))) return rc;
+    const LineScales ws = weight_scales(geo, transposed);
+    const AbsMaxParams w{static_cast<const float *>(val), idx, tab.order, weight_maxima, geo.nb, geo.nc, ws.lines, geo.n, geo.m, geo.g, geo.cc, transposed ? 1 : 0, ws.spans, ws.per};
+    const int64_t units = (transposed ? geo.nc : geo.nb) * ws.spans;
+    const size_t smem = (size_t)(transposed ? geo.cc : geo.m) * 4;
+    SplitParams p{};
+    p.src = static_cast<const float *>(act);
+    p.dst = reinterpret_cast<__half *>(buf);
+    p.ld = dense_ld(red);
+    p.factors = reinterpret_cast<float *>(buf + planes_bytes(ACT_PLANES, tokens, red));
+    p.small = reinterpret_cast<float *>(buf + planes_bytes(ACT_PLANES, tokens, red) + LineScales::factor_bytes(tokens));
+    p.rows = tokens; p.cols = red; p.ld_src = ld_act;
+    *out = DenseAct{buf, p.ld, p.factors, p.small};
+    if (act_k_major) {
+        const int64_t blocks = (red + 63) / 64, cl = blocks < COLS_CLUSTER ? blocks : COLS_CLUSTER;
+        p.per = (int)((blocks + cl - 1) / cl * 64);
+        p.ctas = (tokens + 31) / 32;
+        const int64_t gy = p.ctas + (units + cl - 1) / cl;
+        if (tokens > 65535 * 16 || gy > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)cl, (unsigned)gy);
+        cfg.blockDim = dim3(COLS_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr;
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = (unsigned)cl;
+        attr.val.clusterDim.y = 1;
+        attr.val.clusterDim.z = 1;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        NMG_ALLOW_SMEM(smem, split_columns_kernel);
+        NMG_CUDA(cudaLaunchKernelEx(&cfg, split_columns_kernel, p, w));
+        return NMG_OK;
+    }
+    p.ctas = p.ld <= 1024 ? (tokens + 3) / 4 : tokens;
+    if (tokens > 65535 * 16 || p.ctas + units > 0x7fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
+    const unsigned grid = (unsigned)(p.ctas + units);
+    if (p.ld <= 1024) split_rows_kernel<4><<<grid, PREP_THREADS, smem, st>>>(p, w);
+    else split_rows_kernel<1><<<grid, PREP_THREADS, smem, st>>>(p, w);
+    NMG_CUDA(cudaGetLastError());
+    return NMG_OK;
 }
 
 template <typename T, bool TR, int N_, bool PLAIN> static int expand_launch_n(const ExpandParams &p, size_t smem, int64_t items, cudaStream_t st) {
@@ -947,32 +1445,42 @@ static GemmTiles gemm_tiles(int64_t tiles_f, int64_t cols, int64_t units, bool f
     return best;
 }
 // (val, idx) -> the weight with its zeros restored, rows `ld` elements apart at `dst` (16-byte aligned, ld a multiple of 8).
-// plain = false: the matmul's operand, 16-bit or three bf16 planes for fp32 (plane_rows rows each); plain = true: the
+// plain = false: the matmul's operand, 16-bit or two fp16 planes for fp32; plain = true: the
 // weight in its own dtype (the densifier), where full stores must not run past the row: K a multiple of 8, or the rows kernel.
+// An fp32 operand's factors and maxima follow its planes (LineScales).
 static int expand_to(const Geo &geo, int dtype, bool transposed, bool plain, const void *val, const int16_t *idx, void *dst, int64_t ld,
                      cudaStream_t st) {
-    const int64_t rows = transposed ? geo.K : geo.M;
+    const bool scaled = dtype == NMG_F32 && !plain;
     const size_t es = dtype == NMG_F32 ? 4 : 2;
     int rc;
     PatternTable tab;
     if ((rc = get_pattern_table(geo.n, geo.m, &tab))) return rc;
     ExpandParams ep{};
     ep.val = val; ep.idx = idx; ep.order = tab.order; ep.dst = dst;
-    ep.ld = ld; ep.plane_elems = rows * ld;
+    ep.ld = ld;
+    if (scaled) {
+        const LineScales sc = weight_scales(geo, transposed);
+        char *scales = static_cast<char *>(dst) + planes_bytes(SPLIT_PLANES, sc.rows, transposed ? geo.M : geo.K);
+        ep.plane_elems = sc.rows * ld;
+        ep.factors = reinterpret_cast<float *>(scales);
+        ep.maxima = reinterpret_cast<const uint32_t *>(scales + LineScales::factor_bytes(sc.rows));
+        ep.spans = sc.spans; ep.lines = sc.lines;
+    }
     ep.vec = geo.K % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
     ep.M = geo.M; ep.K = geo.K; ep.nb = geo.nb; ep.nc = geo.nc;
     ep.n = geo.n; ep.m = geo.m; ep.g = geo.g; ep.C = geo.C; ep.cc = geo.cc;
     size_t rsmem = 0;
     const bool aligned = ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0;
-    if (!transposed && aligned && expand_rows_plan(geo, es, &ep.R, &ep.Q, &rsmem)) {
+    if (!transposed && aligned && expand_rows_plan(geo, es, scaled, &ep.R, &ep.Q, &rsmem)) {
         if (dtype == NMG_F16) return plain ? expand_rows_launch<__half, true>(ep, rsmem, st) : expand_rows_launch<__half, false>(ep, rsmem, st);
         if (dtype == NMG_BF16) return plain ? expand_rows_launch<__nv_bfloat16, true>(ep, rsmem, st) : expand_rows_launch<__nv_bfloat16, false>(ep, rsmem, st);
         return plain ? expand_rows_launch<float, true>(ep, rsmem, st) : expand_rows_launch<float, false>(ep, rsmem, st);
     }
     ep.R = expand_rows_per_item(geo, es, transposed);
     ep.pitch = expand_pitch(geo, transposed, ep.R);
-    const size_t esmem = expand_smem_bytes(geo, es, transposed, ep.R);
+    size_t esmem = expand_smem_bytes(geo, es, transposed, ep.R);
     if (esmem > 200 * 1024) NMG_FAIL(NMG_ERR_UNSUPPORTED, "chunk of %d columns does not fit the expansion pass", geo.cc);
+    esmem += scaled ? (size_t)(transposed ? geo.cc : ep.R * geo.m) * 4 : 0;
     const int64_t items = ((geo.nb + ep.R - 1) / ep.R) * geo.nc;
     if (dtype == NMG_F16) return transposed ? expand_launch<__half, true>(ep, esmem, items, st) : expand_launch<__half, false>(ep, esmem, items, st);
     if (dtype == NMG_BF16) return transposed ? expand_launch<__nv_bfloat16, true>(ep, esmem, items, st) : expand_launch<__nv_bfloat16, false>(ep, esmem, items, st);
@@ -990,7 +1498,7 @@ bool tc_expand_plain_supported(const Geo &geo, int dtype, const void *val, const
     const size_t es = dtype == NMG_F32 ? 4 : 2;
     int R, Q;
     size_t smem;
-    if (geo.C <= 65535 && ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0 && expand_rows_plan(geo, es, &R, &Q, &smem)) return true;
+    if (geo.C <= 65535 && ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0 && expand_rows_plan(geo, es, false, &R, &Q, &smem)) return true;
     if (geo.cc > 32767 || geo.C > 65535 || geo.K % 8 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(dense) & 15) != 0) return false;
     return expand_smem_bytes(geo, es, false, expand_rows_per_item(geo, es, false)) <= 200 * 1024;
 }
@@ -998,17 +1506,18 @@ int tc_expand_plain(const Geo &geo, int dtype, const void *val, const int16_t *i
     return expand_to(geo, dtype, false, true, val, idx, dense, ld, st);
 }
 
-// out = dense[rows][round_up(red, 8)] (16-bit, or three bf16 planes for fp32) x activations (16-bit, or the planes of the split).
+// out = dense[rows][round_up(red, 8)] (16-bit, or the two fp16 planes of an fp32 weight and its factors) x activations (16-bit, or the planes of the split).
 // CTA pairs (256 rows per tile) unless a 16-bit output has one tile of 128 features only.  source: expand this weight into `dense`
 // first, right before the matmul, whose prologue overlaps the expansion's end only when nothing is queued between the two.
 int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const DenseAct &act, int64_t tokens, const void *bias,
                   void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major, cudaStream_t st, const Epilogue &epi, const DenseSource *source) {
     if (n_outs < 1 || n_outs > GEMM_MAX_OUTS) NMG_FAIL(NMG_ERR_INVALID, "between 1 and %d output buffers, got %d", GEMM_MAX_OUTS, n_outs);
     const int64_t ld = dense_ld(red);
-    const int planes = dtype == NMG_F32 ? 3 : 1;
+    const int planes = dtype == NMG_F32 ? SPLIT_PLANES : 1;
     int rc;
     GemmMaps maps;
-    const int edt = dtype == NMG_F32 ? NMG_BF16 : dtype;
+    const int edt = dtype == NMG_F32 ? NMG_F16 : dtype;
+    const float *w_factors = reinterpret_cast<const float *>(dense + planes_bytes(SPLIT_PLANES, rows, red));
     const size_t osz = dtype == NMG_F32 ? 4 : 2;
     const bool pair = dtype == NMG_F32 || rows > TC_BM;
     // Token-major output of a CTA-pair product: exchange the operands' roles.  The activations become the row operand (tokens
@@ -1023,19 +1532,12 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
     const int64_t tiles_f = (row_ext + tile_feats - 1) / tile_feats;
     if (tiles_f * ((col_ext + 63) / 64) > 0x3fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many output tiles for one launch");
     const GemmTiles tiles = gemm_tiles(tiles_f, col_ext, units, dtype == NMG_F32, pair);
-    for (int c = 0; c < 3; c++) {
-        const int pc = c < planes ? c : 0;
-        const char *w = dense + (size_t)pc * rows * ld * 2, *x = static_cast<const char *>(act.base) + (size_t)pc * act.plane_elems * 2;
-        if (pc != c) {  // never used; keeps the parameter defined
-            maps.a[c] = maps.a[0]; maps.b[c] = maps.b[0]; maps.b_tail[c] = maps.b_tail[0];
-            continue;
-        }
-        const uint32_t col_box = (uint32_t)(pair ? tiles.bn / 2 : tiles.bn);
-        if ((rc = encode_tmap_2d(swap ? &maps.b[c] : &maps.a[c], edt, w, (uint64_t)red, (uint64_t)rows, (uint64_t)ld, TC_BK, swap ? col_box : TC_BM, 1))) return rc;
-        if ((rc = encode_tmap_2d(swap ? &maps.a[c] : &maps.b[c], edt, x, (uint64_t)red, (uint64_t)tokens, (uint64_t)act.ld, TC_BK, swap ? TC_BM : col_box, 1))) return rc;
-        if (tiles.f_narrow == 0) maps.b_tail[c] = maps.b[c];
-        else if ((rc = encode_tmap_2d(&maps.b_tail[c], edt, swap ? w : x, (uint64_t)red, (uint64_t)col_ext, (uint64_t)(swap ? ld : act.ld), TC_BK, (uint32_t)(tiles.bn_tail / 2), 1))) return rc;
-    }
+    const uint64_t act_rows = (uint64_t)tokens * (dtype == NMG_F32 ? ACT_PLANES : 1), w_rows = (uint64_t)rows * planes;
+    const uint32_t col_box = (uint32_t)(pair ? tiles.bn / 2 : tiles.bn);
+    if ((rc = encode_tmap_2d(swap ? &maps.b : &maps.a, edt, dense, (uint64_t)red, w_rows, (uint64_t)ld, TC_BK, swap ? col_box : TC_BM, 1))) return rc;
+    if ((rc = encode_tmap_2d(swap ? &maps.a : &maps.b, edt, act.base, (uint64_t)red, act_rows, (uint64_t)act.ld, TC_BK, swap ? TC_BM : col_box, 1))) return rc;
+    if (tiles.f_narrow == 0) maps.b_tail = maps.b;
+    else if ((rc = encode_tmap_2d(&maps.b_tail, edt, swap ? dense : act.base, (uint64_t)red, swap ? w_rows : act_rows, (uint64_t)(swap ? ld : act.ld), TC_BK, (uint32_t)(tiles.bn_tail / 2), 1))) return rc;
     if (swap) {  // from here on "rows" are the accumulator's rows (tokens) and "tokens" its columns (output features)
         const int64_t t = rows;
         rows = tokens;
@@ -1048,6 +1550,9 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
     gp.bias = bias;
     gp.n_out = n_outs;
     gp.bias_cols = swap ? 1 : 0;
+    gp.fac_rows = swap ? act.factors : w_factors; gp.fac_cols = swap ? w_factors : act.factors;
+    gp.small = act.small;
+    gp.a_rows = (int)row_ext; gp.b_rows = (int)col_ext;
     bool vec = !out_token_major && (ld_out * osz) % 16 == 0;
     for (int d = 0; d < n_outs; d++) {
         if (!outs[d]) NMG_FAIL(NMG_ERR_INVALID, "output buffer %d is NULL", d);
@@ -1062,10 +1567,10 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
                         ? 1 : 0;
     gp.out_tma = (vec && n_outs == 1 && !mc_out) ? 1 : 0;
     if (gp.out_tma) {
-        const uint32_t box_cols = (uint32_t)(128 / osz);
-        if ((rc = encode_tmap_2d(&maps.out, dtype, outs[0], (uint64_t)tokens, (uint64_t)rows, (uint64_t)ld_out, box_cols, 32, 1))) return rc;
+        const uint32_t box_cols = dtype == NMG_F32 ? 16 : 64;
+        if ((rc = encode_tmap_2d(&maps.out, dtype, outs[0], (uint64_t)tokens, (uint64_t)rows, (uint64_t)ld_out, box_cols, 32, dtype == NMG_F32 ? 2 : 1))) return rc;
     } else {
-        maps.out = maps.a[0];  // never used; keeps the parameter defined
+        maps.out = maps.a;  // never used; keeps the parameter defined
     }
     gp.mc_out = (vec && mc_out && (reinterpret_cast<uintptr_t>(mc_out) & 15) == 0) ? mc_out : nullptr;
     gp.tiles = tiles;
@@ -1085,16 +1590,23 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
     return pair ? gemm_launch<__nv_bfloat16, true>(gp, maps, st) : gemm_launch<__nv_bfloat16, false>(gp, maps, st);
 }
 
-// Two passes: expansion into `ws`, then the matmul on the expanded weight.
-int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const DenseAct &act,
+// Two passes: expansion into `ws`, then the matmul on the expanded weight.  fp32: the activation's planes come first in `ws`.
+int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const void *act, int64_t ld_act, bool act_k_major,
                     int64_t tokens, const void *bias, void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major,
                     void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi) {
     const int64_t rows = transposed ? geo.K : geo.M, red = transposed ? geo.M : geo.K;
-    const size_t need = tc_dense_workspace_bytes(geo, dtype, transposed);
+    const size_t act_need = tc_dense_act_bytes(geo, dtype, transposed, tokens), need = act_need + tc_dense_workspace_bytes(geo, dtype, transposed);
     if (!ws || ws_bytes < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the expanded weight, got %zu", need, ws_bytes);
-    char *dense = reinterpret_cast<char *>(((uintptr_t)ws + 255) & ~(uintptr_t)255);
+    char *act_buf = reinterpret_cast<char *>(((uintptr_t)ws + 255) & ~(uintptr_t)255);
+    char *dense = reinterpret_cast<char *>(((uintptr_t)ws + act_need + 255) & ~(uintptr_t)255);
+    DenseAct planes{act, ld_act, nullptr, nullptr};
+    int rc;
+    if (dtype == NMG_F32) {
+        char *maxima = dense + planes_bytes(SPLIT_PLANES, rows, red) + LineScales::factor_bytes(rows);
+        if ((rc = split_operands(geo, transposed, val, idx, act, ld_act, act_k_major, tokens, act_buf, reinterpret_cast<uint32_t *>(maxima), &planes, st))) return rc;
+    }
     const DenseSource source{geo, transposed, val, idx};
-    return tc_dense_gemm(rows, red, dtype, dense, act, tokens, bias, outs, n_outs, mc_out, ld_out, out_token_major, st, epi, &source);
+    return tc_dense_gemm(rows, red, dtype, dense, planes, tokens, bias, outs, n_outs, mc_out, ld_out, out_token_major, st, epi, &source);
 }
 
 }  // namespace nmg

@@ -149,7 +149,7 @@ static EncodeTiledFn get_encode_fn() {
 }
 
 static int encode_tmap(CUtensorMap *map, CUtensorMapDataType dt, size_t es, const void *base, uint64_t cols, uint64_t rows, uint64_t ld_elems,
-                   uint32_t box_cols, uint32_t box_rows, int swizzle_128b) {
+                   uint32_t box_cols, uint32_t box_rows, int swizzle) {
     EncodeTiledFn fn = get_encode_fn();
     if (!fn) NMG_FAIL(NMG_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
     if (((uintptr_t)base & 15) || ((ld_elems * es) & 15))
@@ -160,7 +160,7 @@ static int encode_tmap(CUtensorMap *map, CUtensorMapDataType dt, size_t es, cons
     cuuint32_t estr[2] = {1, 1};
     auto encode = [&] {
         return fn(map, dt, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  swizzle_128b ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  swizzle == 1 ? CU_TENSOR_MAP_SWIZZLE_128B : swizzle == 2 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     };
     CUresult r = encode();
@@ -174,11 +174,11 @@ static int encode_tmap(CUtensorMap *map, CUtensorMapDataType dt, size_t es, cons
 }
 
 int encode_tmap_2d(CUtensorMap *map, int dtype, const void *base, uint64_t cols, uint64_t rows, uint64_t ld_elems,
-                   uint32_t box_cols, uint32_t box_rows, int swizzle_128b) {
+                   uint32_t box_cols, uint32_t box_rows, int swizzle) {
     const CUtensorMapDataType dt = dtype == NMG_F32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                    : dtype == NMG_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
                                                       : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
-    return encode_tmap(map, dt, dtype_size(dtype), base, cols, rows, ld_elems, box_cols, box_rows, swizzle_128b);
+    return encode_tmap(map, dt, dtype_size(dtype), base, cols, rows, ld_elems, box_cols, box_rows, swizzle);
 }
 
 int encode_tmap_2d_bytes(CUtensorMap *map, const void *base, uint64_t cols, uint64_t rows, uint64_t ld, uint32_t box_cols, uint32_t box_rows) {

@@ -38,7 +38,7 @@ int simt_bwd(const Geo &geo, int dtype, const void *pat, const void *nval, const
              int64_t tokens, void *dx, int64_t ld_dx, void *ws, size_t ws_bytes, cudaStream_t st);
 
 // Tensor-core kernels.  act: [tokens][ld_act] with the reduction axis contiguous.  fp32 operands are multiplied as
-// sums of bf16 pieces and need `ws` (tc_split_workspace_bytes) for the split activation.  Two variants share the
+// sums of 16-bit pieces and need `ws` (tc_split_workspace_bytes, tc_dense_act_bytes) for the split activation.  Two variants share the
 // entry point tc_matmul: the fused kernel (nmg_spmm_tc.cu) expands the column-ordered copy (pat / nval) tile by tile
 // inside the matmul; the two-pass variant (nmg_gemm_tc.cu, `dense` = true) first expands (val, idx) into a dense 16-bit
 // matrix in `ws` (tc_dense_workspace_bytes, after the split activation) and multiplies that.  tc_use_dense is the
@@ -52,22 +52,23 @@ struct Epilogue {
     bool any() const { return act != NMG_EPI_NONE || residual != nullptr; }
 };
 int launch_epilogue(int dtype, void *out, int64_t rows, int64_t cols, int64_t ld_out, const Epilogue &epi, cudaStream_t st);
-// Activations of the two-pass variant: [tokens][ld], reduction contiguous, 16-byte aligned rows; three bf16 planes for fp32.
+// Activations of the two-pass variant: [tokens][ld], reduction contiguous, 16-byte aligned rows; for fp32 the planes and factors of its rows (see nmg_gemm_tc.cu).
 struct DenseSource { const Geo &geo; bool transposed; const void *val; const int16_t *idx; };  // the compressed weight
-struct DenseAct { const void *base; int64_t ld, plane_elems; };
+struct DenseAct { const void *base; int64_t ld; const float *factors, *small; };
 
 bool tc_supported(const Geo &geo, int dtype);        // fused kernel
 bool tc_dense_supported(const Geo &geo, int dtype);  // two-pass variant
 bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens, bool have_packed);
 size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens);
-size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed);
+size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed);               // two-pass variant: the expanded weight,
+size_t tc_dense_act_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens);     // and before it the planes of an fp32 activation
 // outs / n_outs: the result goes to every listed buffer (same shape and pitch); more than one needs `dense`.  mc_out, when
 // not NULL, is an NVSwitch multicast address that maps onto all of them: full 16-byte chunks are then stored once.
 // act_k_major (fp32 only): act is [reduction][ld_act >= tokens]; it is transposed while it is split into planes.
 int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void *val, const int16_t *idx, const void *pat,
               const void *nval, const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, const void *bias, void *const *outs, int n_outs,
               void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi = Epilogue());
-int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const DenseAct &act,
+int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const void *act, int64_t ld_act, bool act_k_major,
                     int64_t tokens, const void *bias, void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major,
                     void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi);
 

@@ -833,11 +833,18 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
               void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi) {
     if (n_outs < 1 || (n_outs > 1 && !dense)) NMG_FAIL(NMG_ERR_UNSUPPORTED, "several output buffers need the two-pass tensor-core variant");
     void *out = outs[0];
+    int rc;
+    if (dense) {
+        const ProfileEvents pe = take_profile_events();
+        if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));
+        rc = tc_dense_matmul(geo, dtype, transposed, val, idx, act, ld_act, act_k_major, tokens, bias, outs, n_outs, mc_out, ld_out, out_token_major, ws, ws_bytes, st, epi);
+        if (rc == NMG_OK && pe.stop) NMG_CUDA(cudaEventRecord(pe.stop, st));
+        return rc;
+    }
     const int64_t red = transposed ? geo.M : geo.K;
     const int64_t feats = transposed ? geo.K : geo.M;
     const FxChoice fx = fx_choose(feats, red, tokens, dtype);
-    DenseAct planes{act, ld_act, 0};
-    int rc;
+    struct { const void *base; int64_t ld, plane_elems; } planes{act, ld_act, 0};
     if (dtype == NMG_F32) {
         const size_t need = tc_split_workspace_bytes(geo, dtype, transposed, tokens);
         if (!ws || ws_bytes < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the split activation, got %zu", need, ws_bytes);
@@ -857,16 +864,7 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
             split_f32_kernel<<<grid, 128, 0, st>>>(static_cast<const float *>(act) + r0 * ld_act, nr, red, ld_act, xs + r0 * ldp, ldp, plane_elems);
         }
         NMG_CUDA(cudaGetLastError());
-        planes = DenseAct{xs, ldp, plane_elems};
-        ws = static_cast<char *>(ws) + need;  // what follows the split activation is free for the expanded weight
-        ws_bytes -= need;
-    }
-    if (dense) {
-        const ProfileEvents pe = take_profile_events();
-        if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));
-        rc = tc_dense_matmul(geo, dtype, transposed, val, idx, planes, tokens, bias, outs, n_outs, mc_out, ld_out, out_token_major, ws, ws_bytes, st, epi);
-        if (rc == NMG_OK && pe.stop) NMG_CUDA(cudaEventRecord(pe.stop, st));
-        return rc;
+        planes = {xs, ldp, plane_elems};
     }
     int *status = nullptr;
     if ((rc = get_status_word(&status))) return rc;

@@ -159,6 +159,9 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+__device__ __forceinline__ void st_cluster(uint32_t cluster_addr, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -249,6 +252,7 @@ __device__ __forceinline__ float gelu_erf(float v) {
     return fmaf(-(av * q), e, fmaxf(v, 0.f));
 }
 
+// Fused kernel (the two-pass kernel has a split of its own, see line_exp there):
 // fp32 operands run on the bf16 tensor cores as exact three-way splits x = xh + xm + xl, w = wh + wm + wl.  The
 // product keeps the six terms whose weight is >= 2^-16 of the leading one (wh xh, wm xh, wh xm, wm xm, wl xh, wh xl);
 // the dropped terms are below 2^-24 relative, the size of an fp32 rounding error.  Each term is one more MMA

@@ -111,6 +111,23 @@ template <auto Kernel> inline int allow_smem(size_t bytes) {
     do {                                                                        \
         if (const int rc__ = ::nmg::allow_smem<__VA_ARGS__>(bytes)) return rc__; \
     } while (0)
+// Launch that may begin before the kernels queued ahead of it have ended: it runs up to its first dependents_wait() beside their
+// ends, so that neither the launch nor the set-up is waited for.  Every CTA of such a kernel has to get there before it reads or
+// writes anything another kernel does, and before it exits: what is queued behind it relies on that.
+template <class... P, class... A> int launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    NMG_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+    return NMG_OK;
+}
 int get_wave_counter(unsigned **dev_ptr);  // one of a few rotating 4-byte counters of the current device (spare bytes of the status block)
 // Status word of nmg_spmm_noalloc on device `dev` (start of the built-in scratch array), or NULL before its first call there.
 int *noalloc_status_word(int dev);
@@ -144,6 +161,12 @@ inline size_t dtype_size(int dtype) { return dtype == NMG_F32 ? 4 : 2; }
 // ------------------------------------------------------------------------------------------------ device primitives
 #ifdef __CUDACC__
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+
+// The next kernel of the stream may become resident from here on (once all CTAs are here or have ended); it only helps one that was
+// launched by launch_early or with its attribute.
+__device__ __forceinline__ void dependents_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Everything queued ahead of this kernel has ended and is visible.
+__device__ __forceinline__ void dependents_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));

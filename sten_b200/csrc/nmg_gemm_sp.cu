@@ -73,10 +73,11 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_sp_kernel(const SpExpan
     const int m = prm.m, cc = prm.cc, R = prm.R, pitch = prm.pitch;
     T *tile = reinterpret_cast<T *>(smem);                                // [cc][pitch]
     int8_t *ord = reinterpret_cast<int8_t *>(tile + (size_t)cc * pitch);  // [C][n]
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");       // the matmul kernel's prologue may overlap this grid
+    dependents_launch();  // the matmul kernel's prologue may overlap this grid
     const int n = N_ > 0 ? N_ : prm.n;
     for (int i = threadIdx.x; i < prm.C * n; i += EXPAND_THREADS) ord[i] = prm.order[i];
     for (int i = threadIdx.x; i < cc * pitch; i += EXPAND_THREADS) tile[i] = DT<T>::from_f32(0.f);
+    dependents_wait();
 
     const int64_t groups = sp.n_rt * (SP_ATOM / SP_ROWS_ITEM);  // row groups of 64 up to the padded reduction length
     const int64_t items = groups * prm.nc;
@@ -204,6 +205,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_sp_kernel(const SpGemmPara
     const int my_tiles = (pair < ntiles) ? (ntiles - pair + npairs - 1) / npairs : 0;
     const int nst = (int)((prm.red + SP_ATOM - 1) / SP_ATOM);  // stages (128 reduction elements) per output tile
 
+    dependents_launch();
     if (tid == 0) {
         for (int s = 0; s < SP_STAGES; s++) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         mbar_init(acc_full, 1);
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_sp_kernel(const SpGemmPara
         // ------------------------------------------------------------------ TMA producer (converged warp, issues under elect_one)
         int it = 0;
         bool ok = true;
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // the expansion pass's output arrives through the loads below
+        dependents_wait();  // the expansion pass's output arrives through the loads below
         unsigned arrivals = 0;
         for (int ti = 0; ti < my_tiles && ok; ti++) {
             int tile_f, tok0;
@@ -392,9 +394,7 @@ template <typename T, int N_> static int sp_expand_launch(const SpExpandParams &
     if ((rc_sms = device_sms(&sms))) return rc_sms;
     const int64_t cap = (int64_t)sms * 16;
     NMG_ALLOW_SMEM(smem, expand_sp_kernel<T, N_>);
-    expand_sp_kernel<T, N_><<<(unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st>>>(p);
-    NMG_CUDA(cudaGetLastError());
-    return NMG_OK;
+    return launch_early(expand_sp_kernel<T, N_>, (unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st, p);
 }
 
 template <typename T> static int sp_gemm_launch(const SpGemmParams &p, const SpGemmMaps &maps, cudaStream_t st) {

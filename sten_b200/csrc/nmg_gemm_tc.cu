@@ -143,11 +143,12 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_dense_kernel(const Expa
     T *tile = reinterpret_cast<T *>(smem);                                  // [lines][pitch]
     float *scale = reinterpret_cast<float *>(tile + (size_t)lines * pitch);  // SCALED: [lines]
     int8_t *ord = reinterpret_cast<int8_t *>(scale + (SCALED ? lines : 0));  // [C][n]
-    // The matmul kernel that follows is launched with programmatic stream serialization: it may become resident and run
-    // its prologue while this grid drains, and reads nothing this grid writes before its griddepcontrol.wait.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    for (int i = threadIdx.x; i < prm.C * n; i += EXPAND_THREADS) ord[i] = prm.order[i];
+    // The matmul kernel that follows may become resident and run its prologue while this grid drains, and reads nothing this grid
+    // writes before its dependents_wait; this one's prologue runs beside the kernel ahead.
+    dependents_launch();
+    for (int i = threadIdx.x; i < prm.C * n; i += EXPAND_THREADS) ord[i] = prm.order[i];  // a constant of the library
     for (int i = threadIdx.x; i < lines * pitch; i += EXPAND_THREADS) tile[i] = DT<T>::from_f32(0.f);
+    dependents_wait();
 
     const T *val = static_cast<const T *>(prm.val);
     const int64_t groups = (prm.nb + R - 1) / R;
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
     T *tile = reinterpret_cast<T *>(smem);                                 // [rows][cols]
     float *scale = reinterpret_cast<float *>(tile + (size_t)rows * cols);  // SCALED: [rows]
     int8_t *ord = reinterpret_cast<int8_t *>(scale + (SCALED ? rows : 0));  // [C][n]
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");        // see expand_dense_kernel
+    dependents_launch();  // see expand_dense_kernel
 
     constexpr int VL = N_ * (int)sizeof(T) / 2;  // 16-byte loads of values per 8 slots
     const int per_chunk = R * cc / 8, tid = (int)threadIdx.x;
@@ -234,9 +235,10 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
 #pragma unroll
         for (int i = 0; i < VL; i++) vv[i] = __ldg(reinterpret_cast<const uint4 *>(val + slot * N_) + i);
     };
-    if (blockIdx.x < items) load(blockIdx.x);
     for (int i = tid; i < prm.C * N_; i += EXPAND_THREADS) ord[i] = prm.order[i];
     for (int i = tid; i < rows * cols * (int)sizeof(T) / 16; i += EXPAND_THREADS) reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
+    dependents_wait();
+    if (blockIdx.x < items) load(blockIdx.x);
     __syncthreads();
     const bool same_pattern = (g & 7) == 0;  // 8 consecutive slots then belong to one pattern
     T *ubase = tile + uj * m * cols + uq * cc;
@@ -436,7 +438,8 @@ __global__ void __launch_bounds__(PREP_THREADS) split_rows_kernel(const SplitPar
     extern __shared__ uint32_t mx[];
     __shared__ RowStats warp_stats[PREP_THREADS / 32];
     __shared__ uint32_t warp_small[PREP_THREADS / 32];
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    dependents_launch();
+    dependents_wait();
     if (blockIdx.x >= p.ctas) { weight_absmax_unit(w, blockIdx.x - p.ctas, mx); return; }
     constexpr int LANES = PREP_THREADS / ROWS, HELD = 4;
     const int sub = threadIdx.x / LANES, tid = threadIdx.x - sub * LANES;
@@ -522,7 +525,8 @@ __global__ void __launch_bounds__(COLS_THREADS) split_columns_kernel(const Split
     __shared__ RowStats ranks[COLS_CLUSTER][32];   // written by the cluster's CTAs
     __shared__ uint32_t ranks_small[COLS_CLUSTER][32];
     const int cl = (int)gridDim.x, rank = (int)blockIdx.x;  // a cluster is a row of the grid
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    dependents_launch();
+    dependents_wait();
     if (blockIdx.y >= p.ctas) {  // whole clusters
         const int64_t unit = (int64_t)(blockIdx.y - p.ctas) * cl + rank;
         weight_absmax_unit(w, unit, mx);
@@ -712,6 +716,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     const int chunk_it = SPLIT ? TC_CHUNK_KB : nkb;
     const int nchunks = (nkb + chunk_it - 1) / chunk_it;
 
+    dependents_launch();
     if (tid == 0) {
         for (int s = 0; s < STAGES; s++) {
             mbar_init(&full[s], 1);
@@ -772,7 +777,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         bool ok = true;
         // Everything this kernel reads that an earlier kernel of the stream wrote (the expanded weight, the
         // activations) arrives through the loads below: wait here for the preceding grid to complete and flush.
-        asm volatile("griddepcontrol.wait;" ::: "memory");
+        dependents_wait();
         unsigned arrivals = 0;
         for (int ti = 0; ti < my_tiles && ok; ti++) {
             int feat0, tok0, bn;
@@ -817,7 +822,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (of the leader for pairs)
         if (leader) {
-            if constexpr (SPLIT) asm volatile("griddepcontrol.wait;" ::: "memory");  // tile_wide
+            if constexpr (SPLIT) dependents_wait();  // tile_wide
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint64_t desc0 = make_sw128_desc(smem_u32(smem));
             bool ok = true;
@@ -888,7 +893,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         const bool gelu = prm.act == NMG_EPI_GELU;
         // The bias and the residual are read with ordinary loads, possibly before the first accumulator is ready: like the
         // producer's loads they must not run ahead of the grid this one was launched behind.
-        asm volatile("griddepcontrol.wait;" ::: "memory");
+        dependents_wait();
         int unit = 0;
         bool ok = true;
         uint32_t run[SPLIT ? SLICES : 1][32];  // fp32: sum of the tile's finished chunks
@@ -1324,13 +1329,15 @@ static int split_operands(const Geo &geo, bool transposed, const void *val, cons
         cfg.blockDim = dim3(COLS_THREADS);
         cfg.dynamicSmemBytes = smem;
         cfg.stream = st;
-        cudaLaunchAttribute attr;
-        attr.id = cudaLaunchAttributeClusterDimension;
-        attr.val.clusterDim.x = (unsigned)cl;
-        attr.val.clusterDim.y = 1;
-        attr.val.clusterDim.z = 1;
-        cfg.attrs = &attr;
-        cfg.numAttrs = 1;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)cl;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
         NMG_ALLOW_SMEM(smem, split_columns_kernel);
         NMG_CUDA(cudaLaunchKernelEx(&cfg, split_columns_kernel, p, w));
         return NMG_OK;
@@ -1338,10 +1345,7 @@ static int split_operands(const Geo &geo, bool transposed, const void *val, cons
     p.ctas = p.ld <= 1024 ? (tokens + 3) / 4 : tokens;
     if (tokens > 65535 * 16 || p.ctas + units > 0x7fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
     const unsigned grid = (unsigned)(p.ctas + units);
-    if (p.ld <= 1024) split_rows_kernel<4><<<grid, PREP_THREADS, smem, st>>>(p, w);
-    else split_rows_kernel<1><<<grid, PREP_THREADS, smem, st>>>(p, w);
-    NMG_CUDA(cudaGetLastError());
-    return NMG_OK;
+    return launch_early(p.ld <= 1024 ? split_rows_kernel<4> : split_rows_kernel<1>, grid, PREP_THREADS, smem, st, p, w);
 }
 
 template <typename T, bool TR, int N_, bool PLAIN> static int expand_launch_n(const ExpandParams &p, size_t smem, int64_t items, cudaStream_t st) {
@@ -1349,9 +1353,7 @@ template <typename T, bool TR, int N_, bool PLAIN> static int expand_launch_n(co
     if ((rc_sms = device_sms(&sms))) return rc_sms;
     const int64_t cap = (int64_t)sms * 16;
     NMG_ALLOW_SMEM(smem, expand_dense_kernel<T, TR, N_, PLAIN>);
-    expand_dense_kernel<T, TR, N_, PLAIN><<<(unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st>>>(p);
-    NMG_CUDA(cudaGetLastError());
-    return NMG_OK;
+    return launch_early(expand_dense_kernel<T, TR, N_, PLAIN>, (unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st, p);
 }
 template <typename T, int N_, bool PLAIN> static int expand_rows_launch_n(const ExpandParams &p, size_t smem, cudaStream_t st) {
     int sms = 148, rc;
@@ -1360,9 +1362,7 @@ template <typename T, int N_, bool PLAIN> static int expand_rows_launch_n(const 
     int per_sm = (int)((size_t)227 * 1024 / (smem + 1024));
     if (per_sm > 8) per_sm = 8;
     const int64_t items = ((p.nb + p.R - 1) / p.R) * ((p.nc + p.Q - 1) / p.Q), cap = (int64_t)sms * per_sm;
-    expand_rows_kernel<T, N_, PLAIN><<<(unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st>>>(p);
-    NMG_CUDA(cudaGetLastError());
-    return NMG_OK;
+    return launch_early(expand_rows_kernel<T, N_, PLAIN>, (unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st, p);
 }
 template <typename T, bool PLAIN> static int expand_rows_launch(const ExpandParams &p, size_t smem, cudaStream_t st) {
     return p.n == 1 ? expand_rows_launch_n<T, 1, PLAIN>(p, smem, st) : expand_rows_launch_n<T, 2, PLAIN>(p, smem, st);

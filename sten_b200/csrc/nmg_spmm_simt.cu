@@ -52,7 +52,8 @@ int launch_transpose_to_f32(const void *src, int dtype, int64_t rows, int64_t co
 __global__ void __launch_bounds__(256) transpose_kernel(const uint16_t *__restrict__ src, int64_t rows, int64_t cols, int64_t ld_src,
                                                         uint16_t *__restrict__ dst, int64_t ld_dst) {
     __shared__ uint16_t tile[64][66];
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the matmul's set-up may overlap this pass
+    dependents_launch();  // the matmul's set-up may overlap this pass
+    dependents_wait();
     const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
     const int64_t c0 = (int64_t)blockIdx.x * 64;
     for (int64_t r0 = (int64_t)blockIdx.y * 64; r0 < ld_dst; r0 += (int64_t)gridDim.y * 64) {
@@ -82,15 +83,14 @@ int launch_transpose(const void *src, int64_t rows, int64_t cols, int64_t ld_src
     dim3 block(32, 8);
     const int64_t gy = (ld_dst + 63) / 64;
     dim3 grid((unsigned)((cols + 63) / 64), (unsigned)(gy < 65535 ? gy : 65535));
-    transpose_kernel<<<grid, block, 0, st>>>(static_cast<const uint16_t *>(src), rows, cols, ld_src, static_cast<uint16_t *>(dst), ld_dst);
-    NMG_CUDA(cudaGetLastError());
-    return NMG_OK;
+    return launch_early(transpose_kernel, grid, block, 0, st, static_cast<const uint16_t *>(src), rows, cols, ld_src, static_cast<uint16_t *>(dst), ld_dst);
 }
 
 // Eight elements per thread: 2-byte loads (the rows have no alignment; a warp's eight loads share their lines in L1), one
 // 16-byte store.
 __global__ void __launch_bounds__(256) pad_rows_kernel(const uint16_t *__restrict__ src, int64_t rows, int64_t cols, int64_t ld_src, uint16_t *__restrict__ dst, int64_t ld_dst) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the matmul's set-up may overlap this pass
+    dependents_launch();  // the matmul's set-up may overlap this pass
+    dependents_wait();
     const int64_t per_row = ld_dst / 8;
     for (int64_t r = (int64_t)blockIdx.y * blockDim.y + threadIdx.y; r < rows; r += (int64_t)gridDim.y * blockDim.y)
         for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < per_row; v += (int64_t)gridDim.x * blockDim.x) {
@@ -108,10 +108,8 @@ int launch_pad_rows(const void *src, int64_t rows, int64_t cols, int64_t ld_src,
     dim3 block(32, 8);
     while (block.x < 256 && (int64_t)block.x < per_row) { block.x *= 2; block.y /= 2; }
     const int64_t bx = (per_row + block.x - 1) / block.x, by = (rows + block.y - 1) / block.y;
-    pad_rows_kernel<<<dim3((unsigned)(bx < 1024 ? bx : 1024), (unsigned)(by < 65535 ? by : 65535)), block, 0, st>>>(
-        static_cast<const uint16_t *>(src), rows, cols, ld_src, static_cast<uint16_t *>(dst), ld_dst);
-    NMG_CUDA(cudaGetLastError());
-    return NMG_OK;
+    return launch_early(pad_rows_kernel, dim3((unsigned)(bx < 1024 ? bx : 1024), (unsigned)(by < 65535 ? by : 65535)), block, 0, st,
+                        static_cast<const uint16_t *>(src), rows, cols, ld_src, static_cast<uint16_t *>(dst), ld_dst);
 }
 
 int launch_widen_to_f32(const void *src, int dtype, int64_t rows, int64_t cols, int64_t ld_src, float *dst,

@@ -411,6 +411,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
     const int groups = prm.groups;
     const int lead_x = nkb < 2 ? nkb : 2, lead_w = nkb < groups ? nkb : groups;  // loads issued before the set-up barrier
 
+    dependents_launch();
     // ---- set-up.  The producers initialise their own barriers and issue every group's first loads before the CTA-wide barrier,
     // so that their latency runs beside the TMEM allocation.
     if (warp == FX_WARP_W) {
@@ -422,7 +423,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
             mbar_fence_init();
         }
         __syncwarp();
-        asm volatile("griddepcontrol.wait;" ::: "memory");  // from here on other kernels' results may be read
+        dependents_wait();  // from here on other kernels' results may be read
         if (elect_one())
             for (int kb = 0; kb < lead_w; kb++) load_w(kb, kb);
         __syncwarp();
@@ -444,14 +445,14 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
             }
         }
         __syncwarp();
-        asm volatile("griddepcontrol.wait;" ::: "memory");
+        dependents_wait();
         if (elect_one())
             for (int kb = 0; kb < lead_x; kb++) load_x(kb, kb);
         __syncwarp();
     } else {
         if (warp == FX_WARP_MMA) tmem_alloc(tmem_slot, tmem_cols);
         if (TRANSPOSED && warp < FX_WARP_X) build_table<N_, M_>(table, tid, FX_WARP_X * 32);
-        asm volatile("griddepcontrol.wait;" ::: "memory");
+        dependents_wait();
     }
     tc_fence_before();
     __syncthreads();
@@ -700,7 +701,8 @@ static FxChoice fx_choose(int64_t feats, int64_t red, int64_t tokens, int dtype)
 // ---- fp32 activations: three bf16 planes [3][rows][ldp], written by one elementwise pass ---------------------------
 __global__ void __launch_bounds__(128) split_f32_kernel(const float *__restrict__ src, int64_t rows, int64_t cols, int64_t ld_src,
                                                         __nv_bfloat16 *__restrict__ dst, int64_t ldp, int64_t plane_elems) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // the matmul's set-up may overlap this pass
+    dependents_launch();  // the matmul's set-up may overlap this pass
+    dependents_wait();
     const int64_t r = blockIdx.y;
     const float *row = src + r * ld_src;
     const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
@@ -738,7 +740,8 @@ __global__ void __launch_bounds__(128) split_f32_kernel(const float *__restrict_
 __global__ void __launch_bounds__(256) split_f32_t_kernel(const float *__restrict__ src, int64_t red, int64_t tokens, int64_t ld_src,
                                                           __nv_bfloat16 *__restrict__ dst, int64_t ldp, int64_t plane_elems) {
     __shared__ float tile[64][33];  // [reduction][token]
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    dependents_launch();
+    dependents_wait();
     const int64_t k0 = (int64_t)blockIdx.x * 64;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int64_t t0 = (int64_t)blockIdx.y * 32; t0 < tokens; t0 += (int64_t)gridDim.y * 32) {
@@ -854,16 +857,16 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
         if (tokens > 65535 * 16) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
         if (act_k_major) {
             const int64_t gy = (tokens + 31) / 32;
-            split_f32_t_kernel<<<dim3((unsigned)((ldp + 63) / 64), (unsigned)(gy < 65535 ? gy : 65535)), 256, 0, st>>>(static_cast<const float *>(act), red, tokens, ld_act, xs, ldp,
-                                                                                                                       plane_elems);
+            if ((rc = launch_early(split_f32_t_kernel, dim3((unsigned)((ldp + 63) / 64), (unsigned)(gy < 65535 ? gy : 65535)), 256, 0, st, static_cast<const float *>(act), red, tokens,
+                                   ld_act, xs, ldp, plane_elems)))
+                return rc;
         } else
         for (int64_t r0 = 0; r0 < tokens; r0 += 65535) {  // grid.y limit
             const int64_t nr = tokens - r0 < 65535 ? tokens - r0 : 65535;
             const int64_t bx = (ldp / 8 + 127) / 128;
             dim3 grid((unsigned)(bx > 64 ? 64 : bx), (unsigned)nr);
-            split_f32_kernel<<<grid, 128, 0, st>>>(static_cast<const float *>(act) + r0 * ld_act, nr, red, ld_act, xs + r0 * ldp, ldp, plane_elems);
+            if ((rc = launch_early(split_f32_kernel, grid, 128, 0, st, static_cast<const float *>(act) + r0 * ld_act, nr, red, ld_act, xs + r0 * ldp, ldp, plane_elems))) return rc;
         }
-        NMG_CUDA(cudaGetLastError());
         planes = {xs, ldp, plane_elems};
     }
     int *status = nullptr;

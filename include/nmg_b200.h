@@ -134,8 +134,8 @@ int nmg_pack(const void *val, const int16_t *idx, int64_t M, int64_t K, int n, i
  * `packed` is NULL it serves fewer than 1280 tokens (513 in fp32).  From there on, and for every other (n, m), the weight is first expanded into a transient dense 16-bit matrix in the workspace
  * (M * round_up(K, 8) * 2 bytes; two such planes for fp32) and multiplied by a persistent TMA-fed kernel; that
  * variant reads val / idx and ignores `packed`.  fp32 operands go through the tensor cores as 16-bit pieces with promoted
- * fp32 accumulation: exact three-way bf16 splits in the fused kernel (relative error ~3.5e-6, independent of K), two fp16
- * pieces of scaled rows in the other (~1.7e-6); NMG_ALGO_SIMT forces plain fp32 FMA arithmetic. */
+ * fp32 accumulation, two fp16 pieces of scaled rows (relative error up to 1.7e-6, independent of K from 3072 on; fewer than 64
+ * K-major columns: three bf16 pieces, 1.5e-7); NMG_ALGO_SIMT forces plain fp32 FMA arithmetic. */
 typedef enum { NMG_GIVEN_PACKED = 1, NMG_GIVEN_ALIGNED_ROWS = 2 } nmg_given;
 size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype,
                                 int layout, int algo, int given);

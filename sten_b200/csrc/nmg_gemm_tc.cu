@@ -31,48 +31,6 @@ namespace nmg {
 // =========================================================================================================
 // Expansion pass
 // =========================================================================================================
-// fp32 operands run as two fp16 planes, x = (h + l) 2^e with h = fp16(x 2^-e), l = fp16(x 2^-e - h) and one exponent e per row of the
-// operand that brings the row's largest magnitude to [2^14, 2^15).  Three products (wl xh, wh xl, wh xh) then stand for the fp32 product:
-// what h + l leaves of a value and the dropped wl xl are at most 2^-22 of it, and a value below 2^-18 of its row's largest keeps an
-// absolute 2^-40 of that.  Against three bf16 planes and six products (exact to 2^-24) that halves the tensor-core work, and the
-// result is closer to the exact one, because what dominates the error is the number of truncating additions in the accumulator
-// (see TcMode): half as many.  Relative error against fp64, 1:4: 1.1e-6 -> 0.3e-6 at 128 reduction elements, 3.4e-6 -> 1.7e-6 from 3072;
-// lower in every row and column too, for normal, heavy-tailed and very large or small values, rows of different scale and outliers.
-// Time, 4096 tokens, 1:4: the matmul 3072 <- 768 86 -> 56 us, the whole call 4096 <- 4096 about 560 -> 303 us.
-//
-// Activation rows whose values are mostly far below the largest (a mask value, a saturated feature) are two rows: the values from
-// 2^-16 of the largest on, and the rest with an exponent of its own (down to about 2^-120 of the other; what lies further below loses
-// bits and then is zero) and its own planes.  A tile that holds such a row runs its reduction twice, over either pair of planes.
-__device__ __forceinline__ int line_exp(uint32_t max_bits) {  // infinities and NaN count as the largest finite value
-    const int e = (int)(max_bits >> 23) - (127 + 14);
-    return max_bits == 0 ? 0 : e < -126 ? -126 : e > 113 ? 113 : e;
-}
-__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 <= e <= 127
-// v 2^(er + ec) with the row's and the column's factor.  A factor below one comes first: the other order could overflow on the way.
-__device__ __forceinline__ float unscale(float v, float row_small, float row_large, float col) { return v * row_small * col * row_large; }
-// What a row's values are like: largest magnitude, sum of the exponents and number of the values that are not zero.
-struct RowStats {
-    uint32_t mx = 0, exps = 0, count = 0;
-    __device__ __forceinline__ void add(float v) {
-        const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
-        mx = max(mx, u);
-        exps += u >> 23;
-        count += u != 0;
-    }
-    // The mean exponent of the values is more than 16 below the largest one's.  (Infinities and NaN: such a row's results are not finite.)
-    __device__ __forceinline__ bool wide() const { return mx < 0x7f800000u && (uint64_t)exps + 16ull * count < (uint64_t)(mx >> 23) * count; }
-};
-__device__ __forceinline__ bool is_small(float v, uint32_t mx) { return (__float_as_uint(v) & 0x7fffffffu) < mx - min(mx, 16u << 23); }  // of a wide row
-constexpr float NOT_WIDE = -1.f;  // in place of the factor between the two parts of a row
-// two scaled values -> one word of each plane
-__device__ __forceinline__ void split2_pair(float a, float b, uint32_t &hi, uint32_t &lo) {
-    const __half2 h = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
-    hi = *reinterpret_cast<const uint32_t *>(&h);
-    lo = *reinterpret_cast<const uint32_t *>(&l);
-}
-constexpr int SPLIT_PLANES = 2, ACT_PLANES = 4;
 
 // Move `cnt` (1..8) consecutive elements of a shared-memory line to the destination planes and clear them in shared
 // memory.  VEC: cnt == 8 and both sides are 16-byte aligned.
@@ -103,10 +61,10 @@ template <typename T, bool VEC, bool PLAIN> __device__ __forceinline__ void expa
             *reinterpret_cast<float4 *>(line) = make_float4(0.f, 0.f, 0.f, 0.f);
             *reinterpret_cast<float4 *>(line + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
             uint4 h, l;
-            split2_pair(a.x * scale, a.y * scale, h.x, l.x);
-            split2_pair(a.z * scale, a.w * scale, h.y, l.y);
-            split2_pair(b.x * scale, b.y * scale, h.z, l.z);
-            split2_pair(b.z * scale, b.w * scale, h.w, l.w);
+            split_pair(a.x * scale, a.y * scale, h.x, l.x);
+            split_pair(a.z * scale, a.w * scale, h.y, l.y);
+            split_pair(b.x * scale, b.y * scale, h.z, l.z);
+            split_pair(b.z * scale, b.w * scale, h.w, l.w);
             *reinterpret_cast<uint4 *>(d) = h;
             *reinterpret_cast<uint4 *>(d + p.plane_elems) = l;
         } else {
@@ -400,20 +358,22 @@ struct SplitParams {
     float *small;           // [rows] factor of the small values' planes relative to the others, or NOT_WIDE
     int64_t rows, cols, ld_src, ld;
     int64_t ctas;           // CTAs (clusters) of the activation; those behind them take the weight's units
-    int per;                // K-major source: reduction elements per CTA, a multiple of 64
+    // K-major source: the rows' values are looked at by ranges of the reduction axis, factors and small are [ranges][scale_ld]
+    int64_t range, scale_ld; // reduction elements per range, a multiple of 64
+    int cluster, per;        // CTAs of a range, and reduction elements of each
 };
 // Scales and factors of a row of the given largest magnitudes (small: of a wide row's small values, else 0)
-__device__ __forceinline__ void write_factors(const SplitParams &p, int64_t r, bool wide, uint32_t mx, uint32_t mx_small) {
+__device__ __forceinline__ void write_factors(const SplitParams &p, int64_t r, bool wide, uint32_t mx, uint32_t mx_small) {  // r: index of factors
     const int e = line_exp(mx), d = line_exp(mx_small) - e;
     p.factors[r] = pow2(e);
     p.small[r] = !wide ? NOT_WIDE : d >= -126 ? pow2(d) : d >= -149 ? __uint_as_float(1u << (149 + d)) : 0.f;
 }
 __device__ __forceinline__ void store_planes(const SplitParams &p, int plane, int64_t r, int64_t c, const float (&f)[8], float s) {
     uint4 h, l;
-    split2_pair(f[0] * s, f[1] * s, h.x, l.x);
-    split2_pair(f[2] * s, f[3] * s, h.y, l.y);
-    split2_pair(f[4] * s, f[5] * s, h.z, l.z);
-    split2_pair(f[6] * s, f[7] * s, h.w, l.w);
+    split_pair(f[0] * s, f[1] * s, h.x, l.x);
+    split_pair(f[2] * s, f[3] * s, h.y, l.y);
+    split_pair(f[4] * s, f[5] * s, h.z, l.z);
+    split_pair(f[6] * s, f[7] * s, h.w, l.w);
     __half *d = p.dst + (plane * p.rows + r) * p.ld + c;
     *reinterpret_cast<uint4 *>(d) = h;
     *reinterpret_cast<uint4 *>(d + p.rows * p.ld) = l;
@@ -433,14 +393,15 @@ __device__ __forceinline__ void store_split(const SplitParams &p, int64_t r, int
 
 // CTAs of the activation: one row per CTA, or one per warp where a warp's registers hold it (ROWS = 4).  The row is read once for what
 // its values are like and kept; what the registers do not hold is read again.  HBM-bound, 8 bytes per value.
-template <int ROWS>
+// REST: there are units of a weight, or rows that the registers do not hold.
+template <int ROWS, bool REST>
 __global__ void __launch_bounds__(PREP_THREADS) split_rows_kernel(const SplitParams p, const AbsMaxParams w) {
     extern __shared__ uint32_t mx[];
     __shared__ RowStats warp_stats[PREP_THREADS / 32];
     __shared__ uint32_t warp_small[PREP_THREADS / 32];
     dependents_launch();
     dependents_wait();
-    if (blockIdx.x >= p.ctas) { weight_absmax_unit(w, blockIdx.x - p.ctas, mx); return; }
+    if (REST && blockIdx.x >= p.ctas) { weight_absmax_unit(w, blockIdx.x - p.ctas, mx); return; }
     constexpr int LANES = PREP_THREADS / ROWS, HELD = 4;
     const int sub = threadIdx.x / LANES, tid = threadIdx.x - sub * LANES;
     const int64_t r = (int64_t)blockIdx.x * ROWS + sub;
@@ -463,7 +424,7 @@ __global__ void __launch_bounds__(PREP_THREADS) split_rows_kernel(const SplitPar
             const int64_t c = ((int64_t)h * LANES + tid) * 8;
             if (c < p.ld) fn(c, held[h]);
         }
-        for (int64_t c = ((int64_t)HELD * LANES + tid) * 8; c < p.ld; c += LANES * 8) {
+        for (int64_t c = ((int64_t)HELD * LANES + tid) * 8; REST && c < p.ld; c += LANES * 8) {
             float f[8];
             load(c, f);
             fn(c, f);
@@ -514,104 +475,115 @@ __global__ void __launch_bounds__(PREP_THREADS) split_rows_kernel(const SplitPar
     each([&](int64_t c, const float (&f)[8]) { store_split(p, r, c, f, wide, st.mx, s, s_small); });
 }
 
-// The same from a K-major activation src[red][ld_src >= tokens], transposed on the way.  A cluster owns 32 tokens and its CTAs a part
-// of the reduction axis each; what the tokens' values are like is put together through distributed shared memory, so that this is
-// one launch.  The first COLS_HELD reduction elements of a CTA's part stay in shared memory, the others are read again (from L2).
-constexpr int COLS_THREADS = 256, COLS_HELD = 256, COLS_CLUSTER = 8;
-__global__ void __launch_bounds__(COLS_THREADS) split_columns_kernel(const SplitParams p, const AbsMaxParams w) {
+// The same from a K-major activation src[red][ld_src >= tokens], transposed on the way.  A cluster owns 32 tokens of one range of the
+// reduction axis, its CTAs a part each; what the tokens' values are like is put together through distributed shared memory, so that
+// this is one launch.  The first COLS_HELD reduction elements of a CTA's part stay in shared memory, the others are read again (from
+// L2).  Ranges of a fused matmul with a split reduction are mostly one CTA's: 1024 x 256 tokens, 6 ranges.
+constexpr int COLS_THREADS = 512, COLS_WARPS = COLS_THREADS / 32, COLS_HELD = 256, COLS_CLUSTER = 8, COLS_STEP = COLS_THREADS / 4;
+struct TokenStats { uint32_t mx[32], exps[32], count[32], small[32]; };  // of 32 tokens
+// CLUSTER: a range is several CTAs'.  REST: there are units of a weight, or parts that do not fit COLS_HELD.  A few microseconds of
+// work are bound by what is executed for the first time: mm 1024 x 1024, 256 columns, took 15.5 us with all cases in one kernel, 13.1 now.
+template <bool CLUSTER, bool REST>
+__global__ void __launch_bounds__(COLS_THREADS, 2) split_columns_kernel(const SplitParams p, const AbsMaxParams w) {
     extern __shared__ uint32_t mx[];
-    __shared__ float tile[COLS_HELD][33];          // [reduction][token]
-    __shared__ RowStats part[COLS_THREADS / 32][32];
-    __shared__ RowStats ranks[COLS_CLUSTER][32];   // written by the cluster's CTAs
-    __shared__ uint32_t ranks_small[COLS_CLUSTER][32];
-    const int cl = (int)gridDim.x, rank = (int)blockIdx.x;  // a cluster is a row of the grid
+    __shared__ float tile[COLS_HELD][33];              // [reduction][token]
+    __shared__ TokenStats ours, ranks[CLUSTER ? COLS_CLUSTER : 1];   // ranks: written by the cluster's CTAs
+    const int cl = CLUSTER ? p.cluster : 1, range = (int)blockIdx.x / cl, rank = (int)blockIdx.x - range * cl;
     dependents_launch();
+    if (threadIdx.x < 4 * 32) reinterpret_cast<uint32_t *>(&ours)[threadIdx.x] = 0;
+    __syncthreads();
     dependents_wait();
-    if (blockIdx.y >= p.ctas) {  // whole clusters
-        const int64_t unit = (int64_t)(blockIdx.y - p.ctas) * cl + rank;
-        weight_absmax_unit(w, unit, mx);
+    if (REST && blockIdx.y >= p.ctas) {  // whole clusters
+        weight_absmax_unit(w, (int64_t)(blockIdx.y - p.ctas) * gridDim.x + blockIdx.x, mx);
         return;
     }
-    cluster_arrive();  // waited for before anything is written to another CTA
+    if (cl > 1) cluster_arrive();  // waited for before anything is written to another CTA
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t t0 = (int64_t)blockIdx.y * 32, t = t0 + lane, k0 = (int64_t)rank * p.per;
-    const int count = (int)(p.cols - k0 < p.per ? (p.cols - k0 > 0 ? p.cols - k0 : 0) : p.per);  // of this CTA's part
-    auto at = [&](int k) -> float { return k < count && t < p.rows ? __ldg(p.src + (k0 + k) * p.ld_src + t) : 0.f; };
+    const int64_t t0 = (int64_t)blockIdx.y * 32, t = t0 + lane, k0 = range * p.range + (int64_t)rank * p.per;
+    const int64_t range_end = (range + 1) * p.range < p.cols ? (range + 1) * p.range : p.cols, left = range_end - k0;
+    const int count = (int)(left < p.per ? (left > 0 ? left : 0) : p.per);  // of this CTA's part
+    const float *src = p.src + k0 * p.ld_src + t;
+    const int lim = t < p.rows ? count : 0;
+    auto at = [&](int k) -> float { return k < lim ? __ldg(src + k * p.ld_src) : 0.f; };
     RowStats st;
-#pragma unroll 8
-    for (int k = warp; k < COLS_HELD; k += COLS_THREADS / 32) {
-        const float v = at(k);
-        tile[k][lane] = v;
-        st.add(v);
+    {
+        constexpr int N = COLS_HELD / COLS_WARPS;
+        float v[N];
+#pragma unroll
+        for (int i = 0; i < N; i++) v[i] = at(warp + i * COLS_WARPS);
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            tile[warp + i * COLS_WARPS][lane] = v[i];
+            st.add(v[i]);
+        }
     }
+    if constexpr (REST) {
 #pragma unroll 8
-    for (int k = COLS_HELD + warp; k < count; k += COLS_THREADS / 32) st.add(at(k));
-    part[warp][lane] = st;
+        for (int k = COLS_HELD + warp; k < count; k += COLS_WARPS) st.add(at(k));
+    }
+    atomicMax(&ours.mx[lane], st.mx);
+    atomicAdd(&ours.exps[lane], st.exps);
+    atomicAdd(&ours.count[lane], st.count);
     __syncthreads();
-    cluster_wait();
-    if (warp == 0) {
-        for (int i = 1; i < COLS_THREADS / 32; i++) {
-            const RowStats o = part[i][lane];
-            st.mx = max(st.mx, o.mx);
-            st.exps += o.exps;
-            st.count += o.count;
+    const TokenStats *from = &ours;
+    int parts = 1;
+    if (cl > 1) {
+        cluster_wait();
+        if (warp < cl) {  // one warp per CTA of the cluster
+            const uint32_t dst = map_to_rank(smem_u32(&ranks[rank].mx[lane]), (uint32_t)warp);
+            st_cluster(dst, ours.mx[lane]);
+            st_cluster(dst + 128, ours.exps[lane]);
+            st_cluster(dst + 256, ours.count[lane]);
         }
-        for (int c = 0; c < cl; c++) {
-            const uint32_t dst = map_to_rank(smem_u32(&ranks[rank][lane]), (uint32_t)c);
-            st_cluster(dst, st.mx);
-            st_cluster(dst + 4, st.exps);
-            st_cluster(dst + 8, st.count);
-        }
+        cluster_sync_all();
+        from = ranks;
+        parts = cl;
     }
-    cluster_sync_all();
-    auto gather = [&](int token, uint32_t &m_small) -> RowStats {
+    auto gather = [&](int token) -> RowStats {
         RowStats a;
-        m_small = 0;
-        for (int c = 0; c < cl; c++) {
-            const RowStats o = ranks[c][token];
-            a.mx = max(a.mx, o.mx);
-            a.exps += o.exps;
-            a.count += o.count;
+        for (int c = 0; c < parts; c++) {
+            a.mx = max(a.mx, from[c].mx[token]);
+            a.exps += from[c].exps[token];
+            a.count += from[c].count[token];
         }
         return a;
     };
-    uint32_t mx_small;
-    st = gather(lane, mx_small);
-    const bool any_wide = __any_sync(0xffffffffu, st.wide());  // the same in every warp of the cluster
-    if (any_wide) {
-        for (int k = warp; k < count; k += COLS_THREADS / 32) {
-            const float v = k < COLS_HELD ? tile[k][lane] : at(k);
-            if (is_small(v, st.mx)) mx_small = max(mx_small, magnitude(v));
+    constexpr int PER_TOKEN = COLS_THREADS / 32;  // threads of a token, eight reduction elements each
+    const int tok = threadIdx.x / PER_TOKEN, c8 = (threadIdx.x % PER_TOKEN) * 8;
+    const RowStats mine = gather(lane), theirs = gather(tok);
+    const bool wide = theirs.wide();
+    uint32_t mx_small = 0;
+    if (__any_sync(0xffffffffu, mine.wide())) {  // the same in every warp of the cluster
+        uint32_t sm = 0;
+        for (int k = warp; k < count; k += COLS_WARPS) {
+            const float v = !REST || k < COLS_HELD ? tile[k][lane] : at(k);
+            if (is_small(v, mine.mx)) sm = max(sm, magnitude(v));
         }
-        part[warp][lane].mx = mx_small;
+        atomicMax(&ours.small[lane], sm);
         __syncthreads();
-        if (warp == 0) {
-            for (int i = 1; i < COLS_THREADS / 32; i++) mx_small = max(mx_small, part[i][lane].mx);
-            for (int c = 0; c < cl; c++) st_cluster(map_to_rank(smem_u32(&ranks_small[rank][lane]), (uint32_t)c), mx_small);
+        if (cl > 1) {
+            if (warp < cl) st_cluster(map_to_rank(smem_u32(&ranks[rank].small[lane]), (uint32_t)warp), ours.small[lane]);
+            cluster_sync_all();
         }
-        cluster_sync_all();
+        if (wide)
+            for (int c = 0; c < parts; c++) mx_small = max(mx_small, from[c].small[tok]);
     }
-    const int tok = threadIdx.x >> 3, c8 = (threadIdx.x & 7) * 8;  // eight reduction elements of one token
-    st = gather(tok, mx_small);
-    const bool wide = st.wide();
-    if (wide)
-        for (int c = 0; c < cl; c++) mx_small = max(mx_small, ranks_small[c][tok]);
-    if (rank == 0 && c8 == 0 && t0 + tok < p.rows) write_factors(p, t0 + tok, wide, st.mx, mx_small);
-    const float s = pow2(-line_exp(st.mx)), s_small = pow2(-line_exp(mx_small));
-    for (int kb = 0; kb < count; kb += 64) {
-        const int base = kb < COLS_HELD ? kb : 0;
-        if (kb >= COLS_HELD) {
+    if (rank == 0 && c8 == 0 && t0 + tok < p.rows) write_factors(p, range * p.scale_ld + t0 + tok, wide, theirs.mx, mx_small);
+    const float s = pow2(-line_exp(theirs.mx)), s_small = pow2(-line_exp(mx_small));
+    for (int kb = 0; kb < count; kb += COLS_STEP) {
+        const int base = !REST || kb < COLS_HELD ? kb : 0;
+        if (REST && kb >= COLS_HELD) {
             __syncthreads();
 #pragma unroll
-            for (int i = 0; i < 8; i++) tile[warp * 8 + i][lane] = at(kb + warp * 8 + i);
+            for (int i = 0; i < COLS_STEP / COLS_WARPS; i++) tile[warp + i * COLS_WARPS][lane] = at(kb + warp + i * COLS_WARPS);
             __syncthreads();
         }
         const int64_t k = k0 + kb + c8;
-        if (t0 + tok < p.rows && k < p.ld) {
+        if (t0 + tok < p.rows && kb + c8 < count) {  // ld is cols rounded up to eight
             float f[8];
 #pragma unroll
             for (int i = 0; i < 8; i++) f[i] = tile[base + c8 + i][tok];
-            store_split(p, t0 + tok, k, f, wide, st.mx, s, s_small);
+            store_split(p, t0 + tok, k, f, wide, theirs.mx, s, s_small);
         }
     }
 }
@@ -657,8 +629,6 @@ struct GemmParams {
     int a_rows, b_rows;                // rows of a plane
     int *status;
 };
-template <typename T> struct GemmElem { using type = T; };  // what the tensor cores multiply
-template <> struct GemmElem<float> { using type = __half; };
 constexpr int GEMM_STAGING_BYTES = GEMM_DRAIN_WARPS * 4096;  // per drain warp: 32 feature rows x 128 bytes
 
 struct GemmMaps {
@@ -683,7 +653,7 @@ template <typename T, bool PAIR, bool TMA_OUT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmParams prm, const __grid_constant__ GemmMaps maps) {
     constexpr bool SPLIT = sizeof(T) == 4;
     constexpr int TERMS = SPLIT ? 3 : 1;
-    using E = typename GemmElem<T>::type;
+    using E = typename TcMode<T>::elem;
     static_assert(PAIR || !SPLIT, "fp32 runs on CTA pairs");
     constexpr int NBUF = 2;  // accumulator tiles in flight between the MMA issuer and the drain warps
     constexpr uint32_t TMEM_COLS = NBUF * TC_ACC_COLS;
@@ -849,7 +819,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
 #pragma unroll
                             for (int t = 0; t < TERMS; t++) {
                                 // bias_cols: the operands' roles are exchanged, the order of the products is not (equal results either way)
-                                const int wp = t == 0, xp = t == 1;  // planes of product t: the smallest first
+                                const int wp = split_w(SPLIT_PLANES, t), xp = split_x(SPLIT_PLANES, t);
                                 const int ap = !SPLIT ? 0 : prm.bias_cols ? xp : wp, bp = !SPLIT ? 0 : prm.bias_cols ? wp : xp;
                                 const uint64_t adesc = stage_a + (uint32_t)(ap * (TC_A_BYTES / 16)), bdesc = stage_b + (uint32_t)(bp * (B_BYTES / 16));
 #pragma unroll
@@ -1291,61 +1261,79 @@ static size_t planes_bytes(int planes, int64_t rows, int64_t red) { return ((siz
 
 size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed) {
     const int64_t rows = transposed ? geo.K : geo.M, red = transposed ? geo.M : geo.K;
-    if (dtype == NMG_F32) return planes_bytes(SPLIT_PLANES, rows, red) + weight_scales(geo, transposed).bytes() + 512;
+    // fp32: two planes, in the room that three took: what callers were told to bring is still what they are told
+    if (dtype == NMG_F32) return planes_bytes(3, rows, red) + weight_scales(geo, transposed).bytes() + 512;
     return (size_t)rows * (size_t)dense_ld(red) * 2 + 512;
 }
+size_t tc_split_act_bytes(int64_t tokens, int64_t red, int ranges) {
+    return planes_bytes(ACT_PLANES, tokens, red) + (size_t)2 * ranges * LineScales::factor_bytes(tokens) + 512;
+}
 size_t tc_dense_act_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens) {
-    if (dtype != NMG_F32) return 0;
-    return planes_bytes(ACT_PLANES, tokens, transposed ? geo.M : geo.K) + 2 * LineScales::factor_bytes(tokens) + 512;
+    return dtype == NMG_F32 ? tc_split_act_bytes(tokens, transposed ? geo.M : geo.K, 1) : 0;
 }
 
-// The fp32 activation as planes in `buf`, and in the same launch the weight's maxima behind its planes in `dense`.
+// An fp32 activation as planes in `buf`; `units` of the weight's maxima in the same launch.  range: see SplitParams.
+static int split_act(const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, int64_t red, int64_t range, char *buf, const AbsMaxParams &w, int64_t units, size_t smem,
+                     DenseAct *out, cudaStream_t st) {
+    SplitParams p{};
+    p.src = static_cast<const float *>(act);
+    p.dst = reinterpret_cast<__half *>(buf);
+    p.ld = dense_ld(red);
+    char *scales = buf + planes_bytes(ACT_PLANES, tokens, red);
+    p.factors = reinterpret_cast<float *>(scales);
+    const int64_t ranges = act_k_major ? (red + range - 1) / range : 1;
+    p.small = reinterpret_cast<float *>(scales + ranges * LineScales::factor_bytes(tokens));
+    p.rows = tokens; p.cols = red; p.ld_src = ld_act;
+    p.range = range;
+    p.scale_ld = (int64_t)(LineScales::factor_bytes(tokens) / 4);
+    *out = DenseAct{buf, p.ld, p.factors, p.small, ranges > 1 ? p.scale_ld : 0};
+    if (act_k_major) {
+        const int64_t blocks = ((range < red ? range : red) + 63) / 64, parts = (blocks + COLS_HELD / 64 - 1) / (COLS_HELD / 64);
+        const int64_t cl = parts < COLS_CLUSTER ? parts : COLS_CLUSTER, gx = ranges * cl;
+        p.cluster = (int)cl;
+        p.per = (int)((blocks + cl - 1) / cl * 64);
+        p.ctas = (tokens + 31) / 32;
+        const int64_t gy = p.ctas + (units + gx - 1) / gx;
+        if (tokens > 65535 * 16 || gy > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)gx, (unsigned)gy);
+        cfg.blockDim = dim3(COLS_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[2];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        attr[1].id = cudaLaunchAttributeClusterDimension;
+        attr[1].val.clusterDim.x = (unsigned)cl;
+        attr[1].val.clusterDim.y = 1;
+        attr[1].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = cl > 1 ? 2 : 1;
+        const bool rest = units > 0 || p.per > COLS_HELD;
+        if (rest) NMG_ALLOW_SMEM(smem, split_columns_kernel<true, true>);
+        NMG_CUDA(cudaLaunchKernelEx(&cfg, rest ? split_columns_kernel<true, true> : cl > 1 ? split_columns_kernel<true, false> : split_columns_kernel<false, false>, p, w));
+        return NMG_OK;
+    }
+    p.ctas = p.ld <= 1024 ? (tokens + 3) / 4 : tokens;
+    if (tokens > 65535 * 16 || p.ctas + units > 0x7fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
+    const bool rest = units > 0 || p.ld > 4096;
+    return launch_early(p.ld <= 1024 ? (rest ? split_rows_kernel<4, true> : split_rows_kernel<4, false>) : rest ? split_rows_kernel<1, true> : split_rows_kernel<1, false>,
+                        (unsigned)(p.ctas + units), PREP_THREADS, smem, st, p, w);
+}
+int tc_split_act(const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, int64_t red, int64_t range, char *buf, DenseAct *out, cudaStream_t st) {
+    return split_act(act, ld_act, act_k_major, tokens, red, range, buf, AbsMaxParams{}, 0, 0, out, st);
+}
+// The same with the maxima of the weight's lines.
 static int split_operands(const Geo &geo, bool transposed, const void *val, const int16_t *idx, const void *act, int64_t ld_act, bool act_k_major, int64_t tokens,
                           char *buf, uint32_t *weight_maxima, DenseAct *out, cudaStream_t st) {
-    const int64_t red = transposed ? geo.M : geo.K;
     int rc;
     PatternTable tab;
     if ((rc = get_pattern_table(geo.n, geo.m, &tab))) return rc;
     const LineScales ws = weight_scales(geo, transposed);
     const AbsMaxParams w{static_cast<const float *>(val), idx, tab.order, weight_maxima, geo.nb, geo.nc, ws.lines, geo.n, geo.m, geo.g, geo.cc, transposed ? 1 : 0, ws.spans, ws.per};
-    const int64_t units = (transposed ? geo.nc : geo.nb) * ws.spans;
-    const size_t smem = (size_t)(transposed ? geo.cc : geo.m) * 4;
-    SplitParams p{};
-    p.src = static_cast<const float *>(act);
-    p.dst = reinterpret_cast<__half *>(buf);
-    p.ld = dense_ld(red);
-    p.factors = reinterpret_cast<float *>(buf + planes_bytes(ACT_PLANES, tokens, red));
-    p.small = reinterpret_cast<float *>(buf + planes_bytes(ACT_PLANES, tokens, red) + LineScales::factor_bytes(tokens));
-    p.rows = tokens; p.cols = red; p.ld_src = ld_act;
-    *out = DenseAct{buf, p.ld, p.factors, p.small};
-    if (act_k_major) {
-        const int64_t blocks = (red + 63) / 64, cl = blocks < COLS_CLUSTER ? blocks : COLS_CLUSTER;
-        p.per = (int)((blocks + cl - 1) / cl * 64);
-        p.ctas = (tokens + 31) / 32;
-        const int64_t gy = p.ctas + (units + cl - 1) / cl;
-        if (tokens > 65535 * 16 || gy > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)cl, (unsigned)gy);
-        cfg.blockDim = dim3(COLS_THREADS);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = (unsigned)cl;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 2;
-        NMG_ALLOW_SMEM(smem, split_columns_kernel);
-        NMG_CUDA(cudaLaunchKernelEx(&cfg, split_columns_kernel, p, w));
-        return NMG_OK;
-    }
-    p.ctas = p.ld <= 1024 ? (tokens + 3) / 4 : tokens;
-    if (tokens > 65535 * 16 || p.ctas + units > 0x7fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
-    const unsigned grid = (unsigned)(p.ctas + units);
-    return launch_early(p.ld <= 1024 ? split_rows_kernel<4> : split_rows_kernel<1>, grid, PREP_THREADS, smem, st, p, w);
+    const int64_t red = transposed ? geo.M : geo.K;
+    return split_act(act, ld_act, act_k_major, tokens, red, round_up(red, 64), buf, w, (transposed ? geo.nc : geo.nb) * ws.spans,
+                                   (size_t)(transposed ? geo.cc : geo.m) * 4, out, st);
 }
 
 template <typename T, bool TR, int N_, bool PLAIN> static int expand_launch_n(const ExpandParams &p, size_t smem, int64_t items, cudaStream_t st) {
@@ -1599,7 +1587,7 @@ int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val,
     if (!ws || ws_bytes < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the expanded weight, got %zu", need, ws_bytes);
     char *act_buf = reinterpret_cast<char *>(((uintptr_t)ws + 255) & ~(uintptr_t)255);
     char *dense = reinterpret_cast<char *>(((uintptr_t)ws + act_need + 255) & ~(uintptr_t)255);
-    DenseAct planes{act, ld_act, nullptr, nullptr};
+    DenseAct planes{act, ld_act, nullptr, nullptr, 0};
     int rc;
     if (dtype == NMG_F32) {
         char *maxima = dense + planes_bytes(SPLIT_PLANES, rows, red) + LineScales::factor_bytes(rows);

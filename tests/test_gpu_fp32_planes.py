@@ -1,5 +1,5 @@
-"""fp32 operands of the two-pass product as two fp16 planes with an exponent per row: the rows' scales, lengths that the pass holds in
-registers and those it reads again, both orientations, values at the ends of the range."""
+"""fp32 operands as two fp16 planes with an exponent per row, in both tensor-core kernels: the rows' scales, lengths that the pass holds
+in registers or shared memory and those it reads again, both orientations, values at the ends of the range."""
 import pytest
 import torch
 
@@ -24,14 +24,25 @@ def _weight(n, m, M, K, g, spread):
     return val, idx, ops.densify(val, idx, 1, M, K, n, m, g)[0].double()
 
 
-def _close(got, a, b):
-    """got against the fp64 product a b^T, by the sum of magnitudes of every element."""
-    err, ref = (got.double() - a @ b.t()).abs(), a.abs() @ b.abs().t()
-    assert bool((err <= BOUND * ref + 2.0 ** -148).all()), float((err / ref.clamp_min(1e-300)).max())
+def _packed(val, idx, M, K, n, m, g):
+    """The copy that the fused kernel reads (fewer tokens), where the pattern has one."""
+    from sten_b200 import ops
+    return ops.pack(val, idx, M, K, n, m, g) if (n, m) in ((1, 4), (2, 4), (1, 8), (2, 8), (1, 16)) else None
 
 
-@pytest.mark.parametrize("K,tokens", [(256, 600), (1000, 515), (1032, 513), (4096, 520), (5003, 530)])
-@pytest.mark.parametrize("n,m,g", [(1, 4, 16), (2, 4, 1), (2, 8, 4), (3, 6, 3), (1, 3, 5)])
+def _close(got, a, b, spread=False):
+    """got against the fp64 product a b^T, by the sum of magnitudes of every element.  spread: values may lie further below the largest
+    of their row than two planes reach, and are then off by up to 2^-39 of that (half of the smallest fp16 step, 2^-25, against 2^14)."""
+    err, bound = (got.double() - a @ b.t()).abs(), BOUND * (a.abs() @ b.abs().t()) + 2.0 ** -148
+    if spread:
+        top = lambda v: v.abs().amax(1, keepdim=True)  # noqa: E731
+        bound += 2.0 ** -39 * (top(a) * b.abs().sum(1) + (a.abs() @ (b != 0).double().t()) * top(b).t())
+    assert bool((err <= bound).all()), float((err / bound).max())
+
+
+@pytest.mark.parametrize("K,tokens", [(256, 1100), (1000, 1025), (1032, 1030), (4096, 1100), (5003, 1040),  # two passes
+                                      (192, 64), (256, 300), (1000, 70), (1032, 513), (4096, 1024), (5003, 200)])  # fused
+@pytest.mark.parametrize("n,m,g", [(1, 4, 16), (2, 4, 1), (2, 8, 4), (1, 16, 3), (3, 6, 3), (1, 3, 5)])
 @pytest.mark.parametrize("spread", [False, True])
 def test_products(n, m, g, K, tokens, spread):
     from sten_b200 import _native as nat, ops
@@ -43,14 +54,15 @@ def test_products(n, m, g, K, tokens, spread):
         x[5] = 0
         dy[:, 2] *= 2.0 ** 14
     x, dy = x.to(cuda())[:, 1:K + 1], dy.to(cuda())[:, :M]  # rows that take no 16-byte loads
-    _close(ops.spmm(val, idx, M, K, n, m, g, x, algo=nat.NMG_ALGO_TENSOR), x.double(), dense)
-    _close(ops.spmm(val, idx, M, K, n, m, g, x.t().contiguous(), layout=nat.NMG_ACT_K_MAJOR, algo=nat.NMG_ALGO_TENSOR).t(), x.double(), dense)
-    _close(ops.spmm_t(val, idx, M, K, n, m, g, dy, algo=nat.NMG_ALGO_TENSOR), dy.double(), dense.t())
+    copy = _packed(val, idx, M, K, n, m, g)
+    _close(ops.spmm(val, idx, M, K, n, m, g, x, packed=copy, algo=nat.NMG_ALGO_TENSOR), x.double(), dense, spread)
+    _close(ops.spmm(val, idx, M, K, n, m, g, x.t().contiguous(), layout=nat.NMG_ACT_K_MAJOR, packed=copy, algo=nat.NMG_ALGO_TENSOR).t(), x.double(), dense, spread)
+    _close(ops.spmm_t(val, idx, M, K, n, m, g, dy, packed=copy, algo=nat.NMG_ALGO_TENSOR), dy.double(), dense.t(), spread)
     assert ops.read_status() == 0
 
 
 @pytest.mark.parametrize("M", [768, 1001])
-@pytest.mark.parametrize("K,tokens", [(600, 515), (1500, 2100), (4500, 700)])
+@pytest.mark.parametrize("K,tokens", [(600, 1030), (1500, 2100), (4500, 1100), (600, 300), (300, 1000), (4500, 90)])
 def test_wide_rows(K, tokens, M):
     """Rows with a few values far above all others: what they do not reach keeps the precision of the rest."""
     from sten_b200 import _native as nat, ops
@@ -64,17 +76,19 @@ def test_wide_rows(K, tokens, M):
     x[9, 5], dy[9, 5] = -2.0 ** 100, 2.0 ** 90
     x[9, 6], dy[9, 6] = 2.0 ** -20, 2.0 ** -30
     x, dy = x.to(cuda()), dy.to(cuda())
-    _close(ops.spmm(val, idx, M, K, 2, 8, 4, x, algo=nat.NMG_ALGO_TENSOR), x.double(), dense)
-    _close(ops.spmm(val, idx, M, K, 2, 8, 4, x.t().contiguous(), layout=nat.NMG_ACT_K_MAJOR, algo=nat.NMG_ALGO_TENSOR).t(), x.double(), dense)
-    _close(ops.spmm_t(val, idx, M, K, 2, 8, 4, dy, algo=nat.NMG_ALGO_TENSOR), dy.double(), dense.t())
+    copy = _packed(val, idx, M, K, 2, 8, 4)
+    _close(ops.spmm(val, idx, M, K, 2, 8, 4, x, packed=copy, algo=nat.NMG_ALGO_TENSOR), x.double(), dense)
+    _close(ops.spmm(val, idx, M, K, 2, 8, 4, x.t().contiguous(), layout=nat.NMG_ACT_K_MAJOR, packed=copy, algo=nat.NMG_ALGO_TENSOR).t(), x.double(), dense)
+    _close(ops.spmm_t(val, idx, M, K, 2, 8, 4, dy, packed=copy, algo=nat.NMG_ALGO_TENSOR), dy.double(), dense.t())
     assert ops.read_status() == 0
 
 
+@pytest.mark.parametrize("tokens", [1100, 600, 70])
 @pytest.mark.parametrize("k_major", [False, True])
-def test_ends_of_the_range(k_major):
+def test_ends_of_the_range(k_major, tokens):
     """Rows of zeros, of denormals, of the largest values; infinities and NaN stay in their own rows."""
     from sten_b200 import _native as nat, ops
-    M, K, tokens = 256, 512, 600
+    M, K = 256, 512
     val, idx, dense = _weight(2, 4, M, K, 4, False)
     x = seeded_normal((tokens, K), 2)
     x[3] = 0
@@ -85,7 +99,8 @@ def test_ends_of_the_range(k_major):
     x[8, 10] = float("inf")
     x[9, 11] = float("nan")
     x = x.to(cuda())
-    y = ops.spmm(val, idx, M, K, 2, 4, 4, x.t().contiguous() if k_major else x, layout=nat.NMG_ACT_K_MAJOR if k_major else nat.NMG_ACT_TOKEN_MAJOR, algo=nat.NMG_ALGO_TENSOR)
+    y = ops.spmm(val, idx, M, K, 2, 4, 4, x.t().contiguous() if k_major else x, layout=nat.NMG_ACT_K_MAJOR if k_major else nat.NMG_ACT_TOKEN_MAJOR,
+                 packed=_packed(val, idx, M, K, 2, 4, 4), algo=nat.NMG_ALGO_TENSOR)
     y = y.t() if k_major else y
     assert bool((y[3] == 0).all())
     _close(y[5:8], x[5:8].double(), dense)

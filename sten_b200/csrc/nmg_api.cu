@@ -130,6 +130,7 @@ static int spmm_impl(const void *val, const int16_t *idx, const void *packed, in
         char *ws = static_cast<char *>(workspace);
         size_t left = workspace_bytes;
         const int64_t ld_x = round_up(K, 8);
+        const void *act0 = act;
         if (dtype != NMG_F32 && (!tm || !rows_aligned(dtype, act, ld_act))) {  // re-lay the activation out as [tokens][round_up(K, 8)]
             const size_t need = (size_t)tokens * (size_t)ld_x * 2 + 512;
             if (!ws || left < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the re-laid activation, got %zu", need, left);
@@ -145,7 +146,7 @@ static int spmm_impl(const void *val, const int16_t *idx, const void *packed, in
         const bool dense = force_dense || tc_use_dense(geo, dtype, false, tokens, packed != nullptr);
         if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st, tc_natural_parts(false, !tm, tokens)))) return rc;
         return tc_matmul(geo, dtype, false, dense, val, idx, pat, nval, act, ld_act, dtype == NMG_F32 && !tm, tokens, bias, outs, n_outs, mc_out, ld_out, out_tm ? 1 : 0,
-                         ws, left, st, epi);
+                         ws, left, st, epi, packed && act == act0);
     }
     if (n_outs > 1) NMG_FAIL(NMG_ERR_UNSUPPORTED, "several output buffers need the tensor-core path (aligned token-major activations, >= 64 tokens and rows)");
     if ((rc = simt_fwd(geo, dtype, val, idx, act, ld_act, tokens, bias, out, ld_out, layout, workspace, workspace_bytes, st))) return rc;
@@ -251,7 +252,9 @@ extern "C" int nmg_spmm_t(const void *val, const int16_t *idx, const void *packe
     const void *pat = nullptr;
     const void *nval = nullptr;
     const bool tensor = algo == NMG_ALGO_TENSOR || algo == NMG_ALGO_TENSOR_DENSE || (algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, K));
+    bool alone = packed != nullptr;
     if (tensor && !rows_aligned(dtype, dy, ld_dy)) {  // AUTO only: see pad_rows_bytes
+        alone = false;
         const size_t need = pad_rows_bytes(dtype, tokens, M);
         if (!ws || left < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the re-laid gradient, got %zu", need, left);
         char *yt = align256(ws);
@@ -279,7 +282,7 @@ extern "C" int nmg_spmm_t(const void *val, const int16_t *idx, const void *packe
     const bool dense = tensor && tc_use_dense(geo, dtype, true, tokens, packed != nullptr);
     if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st, tensor ? NATURAL_COLUMNS : 0))) return rc;
     void *dxs[1] = {dx};
-    if (tensor) return tc_matmul(geo, dtype, true, dense, val, idx, pat, nval, dy, ld_dy, false, tokens, nullptr, dxs, 1, nullptr, ld_dx, 1, ws, left, st);
+    if (tensor) return tc_matmul(geo, dtype, true, dense, val, idx, pat, nval, dy, ld_dy, false, tokens, nullptr, dxs, 1, nullptr, ld_dx, 1, ws, left, st, Epilogue(), alone);
     return simt_bwd(geo, dtype, pat, nval, dy, ld_dy, tokens, dx, ld_dx, ws, left, st);
 }
 

@@ -72,10 +72,11 @@ int tc_split_act(const void *act, int64_t ld_act, bool act_k_major, int64_t toke
 size_t tc_dense_act_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens);     // and before it the planes of an fp32 activation
 // outs / n_outs: the result goes to every listed buffer (same shape and pitch); more than one needs `dense`.  mc_out, when
 // not NULL, is an NVSwitch multicast address that maps onto all of them: full 16-byte chunks are then stored once.
+// alone: nothing else was launched for this call.
 // act_k_major (fp32 only): act is [reduction][ld_act >= tokens]; it is transposed while it is split into planes.
 int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void *val, const int16_t *idx, const void *pat,
               const void *nval, const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, const void *bias, void *const *outs, int n_outs,
-              void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi = Epilogue());
+              void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi = Epilogue(), bool alone = false);
 int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val, const int16_t *idx, const void *act, int64_t ld_act, bool act_k_major,
                     int64_t tokens, const void *bias, void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major,
                     void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi);

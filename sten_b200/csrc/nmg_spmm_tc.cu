@@ -53,6 +53,7 @@ struct TcParams {
     int tiles_f, tiles_t; // output tiles along features / tokens
     int bn;               // tokens per tile: a multiple of 32, at most 256 (128 for fp32)
     int stages, slots;    // ring depths, from fx_plan
+    int announce;         // tell the next kernel of the stream to start, see tc_matmul
     int groups;           // expansion groups at work: 3, or 2 with two stages
     int ksplit;           // CTAs per tile = cluster size: each takes one range of the reduction axis
     int exch_off;         // exchange area of the partial tiles: offset in shared memory; 0 = on top of the rings
@@ -403,7 +404,6 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
     const int groups = prm.groups;
     const int lead_x = nkb < 2 ? nkb : 2, lead_w = nkb < groups ? nkb : groups;  // loads issued before the set-up barrier
 
-    dependents_launch();
     // ---- set-up.  The producers initialise their own barriers and issue every group's first loads before the CTA-wide barrier,
     // so that their latency runs beside the TMEM allocation.
     if (warp == FX_WARP_W) {
@@ -594,6 +594,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
             }
         ok = mbar_wait_bounded(all_done, 0, prm.status, 17) && ok;
     }
+    if (prm.announce) dependents_launch();  // the first warps are here when the last loads have been issued
     __syncwarp();
     tc_fence_before();
     if (exch_apart) cluster_wait();          // the other CTAs have started
@@ -693,7 +694,7 @@ bool tc_supported(const Geo &geo, int dtype) {
 // A grid that does not fit the chip at once runs in waves; kFxClusters is what fits (cudaOccupancyMaxActiveClusters: the GPCs
 // are not all alike, 24 clusters of 6 do not fit although 144 < 148).
 constexpr int kFxClusters[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
-struct FxChoice { int bn, tiles_f, tiles_t, ksplit; };
+struct FxChoice { int bn, tiles_f, tiles_t, ksplit; int64_t ns; };
 static FxChoice fx_choose(int64_t feats, int64_t red, int64_t tokens, int dtype, bool fine) {
     const int max_bn = dtype == NMG_F32 ? 192 : 256;  // fp32: the accumulator, the running tile and two stages of two A planes share TMEM
     const int64_t tiles_f = (feats + TC_BM - 1) / TC_BM, nkb = (red + TC_BK - 1) / TC_BK;
@@ -715,7 +716,7 @@ static FxChoice fx_choose(int64_t feats, int64_t red, int64_t tokens, int dtype,
             ns *= waves;
             if (best_ns < 0 || ns < best_ns) {
                 best_ns = ns;
-                best = FxChoice{bn, (int)tiles_f, (int)tiles_t, ks};
+                best = FxChoice{bn, (int)tiles_f, (int)tiles_t, ks, ns};
             }
         }
     }
@@ -842,7 +843,7 @@ bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens, bo
 // act: [tokens][ld_act] with the reduction axis contiguous (X for the forward, dY for the transposed product).
 int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void *val, const int16_t *idx, const void *pat,
               const void *nval, const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, const void *bias, void *const *outs, int n_outs,
-              void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi) {
+              void *mc_out, int64_t ld_out, int out_token_major, void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi, bool alone) {
     if (n_outs < 1 || (n_outs > 1 && !dense)) NMG_FAIL(NMG_ERR_UNSUPPORTED, "several output buffers need the two-pass tensor-core variant");
     void *out = outs[0];
     int rc;
@@ -899,6 +900,10 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     p.out_vec = out_token_major ? (ld_out % 2 == 0 && feats % 2 == 0 && (reinterpret_cast<uintptr_t>(out) & 3) == 0)
                                 : (ld_out * es % 16 == 0 && (reinterpret_cast<uintptr_t>(out) & 15) == 0);
     p.tiles_f = fx.tiles_f; p.tiles_t = fx.tiles_t; p.bn = fx.bn; p.ksplit = fx.ksplit;
+    // The set-up of the next kernel beside this one's end saves 0.3 .. 0.9 us where kernels of this sort follow one another (f16 2:4, 384 x 1984,
+    // 11 tokens 6.5 -> 5.6; 4096 x 4096, 16 tokens 10.1 -> 9.7).  A pass over the activation that settles on the SMs left free then is the slower
+    // for it (mm bf16 2240 x 9216, 64 columns 14.1 -> 15.2), and so are some long ones (5440 x 10944 1:16, 128 tokens 23.8 -> 24.5).
+    p.announce = alone && dtype != NMG_F32 && fx.ns < 14000;
     p.act_factors = x.factors; p.act_small = x.small; p.scale_ld = x.scale_ld; p.act_rows = (int)tokens;
     if (dtype == NMG_F32) p.feat_max = reinterpret_cast<const uint32_t *>(masks + lay.mask_bytes + lay.plane_bytes + lay.fine_bytes) + (transposed ? natural_mask_rows(geo) : 0);
     p.masks = masks; p.mask_rows = natural_mask_rows(geo); p.nb = geo.nb;

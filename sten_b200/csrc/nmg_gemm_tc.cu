@@ -947,7 +947,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                     }
                     if (gelu) {
 #pragma unroll
-                        for (int j = 0; j < 32; j++) r[j] = __float_as_uint(gelu_erf(__uint_as_float(r[j])));
+                        for (int j = 0; j < 32; j += 2) gelu_erf_pair(r[j], r[j + 1]);
                     }
                     if constexpr (TMA_OUT) {
                         if (res && feat_ok) {

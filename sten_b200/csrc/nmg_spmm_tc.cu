@@ -821,11 +821,10 @@ static int tc_launch_nm(int dtype, bool transposed, bool fine, const TcParams &p
 
 // Policy of the two tensor-core variants.  The fused kernel reads the column-ordered copy; without one (have_packed) a call
 // would build it first and throw it away.  Measured, us, 2:4: fused with a kept copy / fused after building one / two passes
-//   fp32   tokens    1024 x 1024       4096 x 1024       1024 x 4096       4096 x 4096
-//             256    15 /  33 / 29     22 /  47 /  35    27 / 49 / 68      52 / 113 / 109
-//             512    18 /  37 / 29     29 /  53 /  42    33 / 56 / 70      87 / 157 / 129
-//            1000    23 /  41 / 29     51 /  77 /  60    55 / 78 / 78     189 / 250 / 180
-//            2048    29 /  48 / 36    101 / 128 /  93    95 / 125 / 111   377 / 431 / 313
+//   fp32   tokens    1024 x 1024       4096 x 1024       1024 x 4096       4096 x 4096       (-: not measured since the fp16 planes)
+//             256    14 /  37 /  -     19 /  53 /   -    23 / 55 /  -      40 / 124 /   -
+//             512    18 /   - /  -     24 /   - /   -    27 /  - /  -      63 /   - /   -
+//            1000    20 /   - / 25     43 /   - /  46    41 /  - / 53     119 /   - / 129
 //   bf16     1024     9 /  24 / 17     12 /  30 /  21    20 / 37 / 31      27 /  65 /  42
 //            1280    10 /  24 / 17     19 /  37 /  25    21 / 37 / 32      49 /  86 /  60
 //            1500    10 /  24 / 17     20 /  39 /  25    23 / 40 / 33      50 /  88 /  61

@@ -493,8 +493,12 @@ __global__ void __launch_bounds__(COLS_THREADS, 2) split_columns_kernel(const Sp
     if (threadIdx.x < 4 * 32) reinterpret_cast<uint32_t *>(&ours)[threadIdx.x] = 0;
     __syncthreads();
     dependents_wait();
-    if (REST && blockIdx.y >= p.ctas) {  // whole clusters
-        weight_absmax_unit(w, (int64_t)(blockIdx.y - p.ctas) * gridDim.x + blockIdx.x, mx);
+    if (REST && blockIdx.y >= p.ctas) {  // whole clusters; the units of a tall weight are more than a grid has rows
+        const int64_t units = (w.transposed ? w.nc : w.nb) * w.spans, step = (int64_t)(gridDim.y - p.ctas) * gridDim.x;
+        for (int64_t unit = (int64_t)(blockIdx.y - p.ctas) * gridDim.x + blockIdx.x; unit < units; unit += step) {
+            weight_absmax_unit(w, unit, mx);
+            __syncthreads();
+        }
         return;
     }
     if (cl > 1) cluster_arrive();  // waited for before anything is written to another CTA
@@ -1298,8 +1302,9 @@ static int split_act(const void *act, int64_t ld_act, bool act_k_major, int64_t 
         p.cluster = (int)cl;
         p.per = (int)((blocks + cl - 1) / cl * 64);
         p.ctas = (tokens + 31) / 32;
-        const int64_t gy = p.ctas + (units + gx - 1) / gx;
-        if (tokens > 65535 * 16 || gy > 65535) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
+        int64_t gy = p.ctas + (units + gx - 1) / gx;
+        if (gy > 65535) gy = 65535;
+        if (tokens > 65535 * 16) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)gx, (unsigned)gy);
         cfg.blockDim = dim3(COLS_THREADS);

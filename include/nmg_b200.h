@@ -132,10 +132,12 @@ int nmg_pack(const void *val, const int16_t *idx, int64_t M, int64_t K, int n, i
  * them when `packed` is given.  The SIMT kernels serve the rest.  Two tensor-core variants exist.  Below 1536 tokens
  * (1025 in fp32), for m in {4, 8, 16} and n <= 2, one fused kernel expands tiles of the packed copy inside the matmul; when
  * `packed` is NULL it serves fewer than 1280 tokens (513 in fp32).  From there on, and for every other (n, m), the weight is first expanded into a transient dense 16-bit matrix in the workspace
- * (M * round_up(K, 8) * 2 bytes; two such planes for fp32) and multiplied by a persistent TMA-fed kernel; that
- * variant reads val / idx and ignores `packed`.  fp32 operands go through the tensor cores as 16-bit pieces with promoted
- * fp32 accumulation, two fp16 pieces of scaled rows (relative error up to 1.7e-6, independent of K from 3072 on; fewer than 64
- * K-major columns: three bf16 pieces, 1.5e-7); NMG_ALGO_SIMT forces plain fp32 FMA arithmetic. */
+ * (M * round_up(K, 8) * 2 bytes; three such planes for fp32) and multiplied by a persistent TMA-fed kernel; that
+ * variant reads val / idx and ignores `packed`.  fp32 operands go through the tensor cores as exact three-way bf16
+ * splits with promoted fp32 accumulation: every value counts with its own 24 bits, however far below the others of its row
+ * (relative error of normally distributed operands 0.7e-7 .. 1.4e-6, independent of K from 3072 on; fewer than 64 K-major columns
+ * 1.5e-7).  Only magnitudes below 2^-110 lose their last bits: in the weight, and in rows of the activation that hold a value
+ * of 2^-80 or more as well.  NMG_ALGO_SIMT forces plain fp32 FMA arithmetic. */
 typedef enum { NMG_GIVEN_PACKED = 1, NMG_GIVEN_ALIGNED_ROWS = 2 } nmg_given;
 size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype,
                                 int layout, int algo, int given);

@@ -17,7 +17,7 @@ static char *align256(void *p) { return reinterpret_cast<char *>(((uintptr_t)p +
 static bool any_tensor(const Geo &geo, int dtype) { return tc_supported(geo, dtype) || tc_dense_supported(geo, dtype); }
 
 // The tensor-core kernels read the activation through a TMA descriptor: 16-bit dtype, reduction axis contiguous, 16-byte
-// aligned base and row pitch.  fp32 activations are re-laid out into aligned 16-bit planes first.
+// aligned base and row pitch.  fp32 activations are re-laid out into aligned bf16 planes first.
 static bool rows_aligned(int dtype, const void *act, int64_t ld_act) {
     return dtype == NMG_F32 || ((((uintptr_t)act) & 15) == 0 && (ld_act % 8) == 0);
 }
@@ -53,7 +53,7 @@ extern "C" int nmg_pack(const void *val, const int16_t *idx, int64_t M, int64_t 
 
 // Resolve the column-ordered copy: the caller's, or one built at the front of the workspace.  Advances *ws.
 static int resolve_packed(const Geo &geo, int dtype, const void *val, const int16_t *idx, const void *packed, char **ws,
-                          size_t *ws_left, const void **pat, const void **nval, cudaStream_t st, int parts) {
+                          size_t *ws_left, const void **pat, const void **nval, cudaStream_t st) {
     size_t pat_bytes = 0;
     const size_t nat = natural_bytes(geo, dtype, &pat_bytes);
     if (packed) {
@@ -68,7 +68,7 @@ static int resolve_packed(const Geo &geo, int dtype, const void *val, const int1
     *nval = base + pat_bytes;
     *ws_left -= (size_t)(base + nat - *ws);
     *ws = base + nat;
-    return launch_build_natural(geo, dtype, val, idx, base, base + pat_bytes, st, parts);
+    return launch_build_natural(geo, dtype, val, idx, base, base + pat_bytes, st);
 }
 
 // K-major activations (B[K][tokens], the torch.mm orientation) reach the tensor cores through one same-dtype transpose
@@ -92,8 +92,9 @@ extern "C" size_t nmg_spmm_workspace_bytes(int64_t M, int64_t K, int64_t tokens,
     size_t tensor = 0;
     const bool tensor_runs = algo == NMG_ALGO_TENSOR ? any_tensor(geo, dtype) : algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, M);
     if (tensor_runs)
-        tensor = (tc_use_dense(geo, dtype, false, tokens, have_packed) ? tc_dense_workspace_bytes(geo, dtype, false) + tc_dense_act_bytes(geo, dtype, false, tokens)
-                                                   : (have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512) + tc_split_workspace_bytes(geo, dtype, false, layout == NMG_ACT_K_MAJOR, tokens)) +
+        tensor = (tc_use_dense(geo, dtype, false, tokens, have_packed) ? tc_dense_workspace_bytes(geo, dtype, false)
+                                                   : (have_packed ? 0 : natural_bytes(geo, dtype, nullptr) + 512)) +
+                 tc_split_workspace_bytes(geo, dtype, false, tokens) +
                  (layout == NMG_ACT_K_MAJOR ? kmajor_transpose_bytes(geo, dtype, tokens) : algo == NMG_ALGO_AUTO && !aligned ? pad_rows_bytes(dtype, tokens, K) : 0);
     // AUTO: the gather kernels serve what the tensor cores do not, and a handful of K-major columns without a packed copy
     const bool simt_runs = algo == NMG_ALGO_SIMT || (algo == NMG_ALGO_AUTO && (!tensor_runs || kmajor_few(geo, dtype, layout, tokens, have_packed)));
@@ -124,8 +125,8 @@ static int spmm_impl(const void *val, const int16_t *idx, const void *packed, in
     const bool tensor = algo == NMG_ALGO_TENSOR || (algo == NMG_ALGO_AUTO && auto_tensor(geo, dtype, M) && !kmajor_few(geo, dtype, layout, tokens, packed != nullptr));
     if (algo == NMG_ALGO_TENSOR && (!any_tensor(geo, dtype) || (tm && !rows_aligned(dtype, act, ld_act)) || (!tm && n_outs > 1)))
         NMG_FAIL(NMG_ERR_UNSUPPORTED, "tensor-core path needs activation rows that are 16-byte aligned (16-bit dtypes) and a chunk that fits shared memory");
-    // AUTO: tensor cores whenever the weight has at least 64 rows, at every token count.  fp32 on tensor cores means 16-bit
-    // pieces with promoted accumulation (measured relative error 0.3e-6 .. 1.7e-6, independent of K from 3072 on); NMG_ALGO_SIMT keeps plain fp32 FMAs.
+    // AUTO: tensor cores whenever the weight has at least 64 rows, at every token count.  fp32 on tensor cores means exact bf16
+    // splitting with promoted accumulation (measured relative error 0.7e-7 .. 1.3e-6, independent of K from 3072 on); NMG_ALGO_SIMT keeps plain fp32 FMAs.
     if (tensor) {
         char *ws = static_cast<char *>(workspace);
         size_t left = workspace_bytes;
@@ -144,7 +145,7 @@ static int spmm_impl(const void *val, const int16_t *idx, const void *packed, in
         }
         const void *pat = nullptr, *nval = nullptr;
         const bool dense = force_dense || tc_use_dense(geo, dtype, false, tokens, packed != nullptr);
-        if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st, tc_natural_parts(false, !tm, tokens)))) return rc;
+        if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st))) return rc;
         return tc_matmul(geo, dtype, false, dense, val, idx, pat, nval, act, ld_act, dtype == NMG_F32 && !tm, tokens, bias, outs, n_outs, mc_out, ld_out, out_tm ? 1 : 0,
                          ws, left, st, epi, packed && act == act0);
     }
@@ -193,7 +194,7 @@ extern "C" int nmg_spmm_replicated(const void *val, const int16_t *idx, int64_t 
 extern "C" size_t nmg_spmm_replicated_workspace_bytes(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype) {
     Geo geo;
     if (make_geo(M, K, n, m, g, &geo) || tokens < 1 || n < 1 || !tc_dense_supported(geo, dtype)) return 0;
-    return tc_dense_workspace_bytes(geo, dtype, false) + tc_dense_act_bytes(geo, dtype, false, tokens);
+    return tc_dense_workspace_bytes(geo, dtype, false) + tc_split_workspace_bytes(geo, dtype, false, tokens);
 }
 
 extern "C" int nmg_spmm_uses_packed(int64_t M, int64_t K, int64_t tokens, int n, int m, int g, int dtype, int layout,
@@ -224,8 +225,8 @@ extern "C" size_t nmg_spmm_t_workspace_bytes(int64_t M, int64_t K, int64_t token
     const size_t simt = tensor_only ? 0 : pack + simt_bwd_workspace_bytes(geo, tokens, dtype) + 256;
     size_t tensor = 0;
     if (algo != NMG_ALGO_SIMT && any_tensor(geo, dtype))
-        tensor = tc_use_dense(geo, dtype, true, tokens, have_packed) ? tc_dense_workspace_bytes(geo, dtype, true) + tc_dense_act_bytes(geo, dtype, true, tokens)
-                                                                     : pack + tc_split_workspace_bytes(geo, dtype, true, false, tokens);
+        tensor = (tc_use_dense(geo, dtype, true, tokens, have_packed) ? tc_dense_workspace_bytes(geo, dtype, true) : pack) +
+                 tc_split_workspace_bytes(geo, dtype, true, tokens);
     if (use_sp(geo, dtype, tokens, algo) && tc_sp_copy_bytes(geo) + 512 > tensor) tensor = tc_sp_copy_bytes(geo) + 512;
     if (algo == NMG_ALGO_AUTO && tensor_only && !aligned) tensor += pad_rows_bytes(dtype, tokens, M);
     return simt > tensor ? simt : tensor;
@@ -280,7 +281,7 @@ extern "C" int nmg_spmm_t(const void *val, const int16_t *idx, const void *packe
         return rc;
     }
     const bool dense = tensor && tc_use_dense(geo, dtype, true, tokens, packed != nullptr);
-    if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st, tensor ? NATURAL_COLUMNS : 0))) return rc;
+    if (!dense && (rc = resolve_packed(geo, dtype, val, idx, packed, &ws, &left, &pat, &nval, st))) return rc;
     void *dxs[1] = {dx};
     if (tensor) return tc_matmul(geo, dtype, true, dense, val, idx, pat, nval, dy, ld_dy, false, tokens, nullptr, dxs, 1, nullptr, ld_dx, 1, ws, left, st, Epilogue(), alone);
     return simt_bwd(geo, dtype, pat, nval, dy, ld_dy, tokens, dx, ld_dx, ws, left, st);
@@ -356,7 +357,7 @@ extern "C" int nmg_spmm_expanded(const void *expanded, int64_t M, int64_t K, int
     cudaStream_t st = (cudaStream_t)stream;
     const ProfileEvents pe = take_profile_events();
     if (pe.start) NMG_CUDA(cudaEventRecord(pe.start, st));
-    rc = tc_dense_gemm(M, K, dtype, static_cast<const char *>(expanded), DenseAct{act, ld_act, nullptr, nullptr, 0}, tokens, bias, outs, 1, nullptr, ld_out, out_tm ? 1 : 0, st, epi);
+    rc = tc_dense_gemm(M, K, dtype, static_cast<const char *>(expanded), DenseAct{act, ld_act, nullptr}, tokens, bias, outs, 1, nullptr, ld_out, out_tm ? 1 : 0, st, epi);
     if (rc == NMG_OK && pe.stop) NMG_CUDA(cudaEventRecord(pe.stop, st));
     return rc;
 }

@@ -21,11 +21,6 @@ struct ExpandParams {
     int R, Q;               // row-blocks and (rows kernel) column chunks per work item
     int vec;                // the destination's rows take 16-byte stores
     int pitch;              // elements per line of the shared-memory tile
-    // fp32 as two fp16 planes: what scales the lines of the destination (LineScales)
-    const uint32_t *maxima; // [spans][lines] largest magnitude bits of every line, by parts of the line
-    float *factors;         // [rows of the operand] out: 2^exponent of the lines
-    int spans;
-    int64_t lines;
 };
 
 constexpr int EXPAND_THREADS = 256;

@@ -8,14 +8,13 @@
 // about 2.5 bytes per weight element) and run a plain TMA-fed tcgen05 matmul over it:
 //
 //   expand_dense_kernel   (val, idx) -> dense W [M][K] (forward) or W^T [K][M] (transposed product), 16-bit; fp32
-//                         weights become two fp16 planes of scaled rows (see line_exp).  Works for every (n, m, g).
-//   split_rows_kernel     fp32 only, first: the activation's planes, and the largest magnitudes of the weight's rows (split_columns_kernel
-//                         from a K-major activation).
+//                         weights become three bf16 planes (exact hi / mid / lo split).  Works for every (n, m, g).
+//   split_rows_kernel     fp32 only, first: the activation's planes (split_columns_kernel from a K-major activation).
 //   expand_rows_kernel    the same for W with n <= 2 and chunks of whole 16-byte pieces, the usual weight: whole rows.
 //   gemm_tc_kernel        persistent, one CTA per SM, in pairs but for 16-bit outputs of one feature tile.  Warp 0 issues the TMA loads of both operands, warp 1 the
 //                         MMAs (128 x 256 x 16, fp32 accumulators in TMEM), warps 4..11 drain accumulators.  16-bit
 //                         mode double-buffers the accumulator (2 x 256 TMEM columns) so that the drain of one tile
-//                         overlaps the MMAs of the next; in fp32 mode a buffer is a chunk of TC_CHUNK_KB k-blocks, and
+//                         overlaps the MMAs of the next; in fp32 mode a buffer is a chunk of k-blocks, and
 //                         the drain warps keep the running sum of the chunks in registers.
 //
 // All device-side waits are bounded: a wait that runs out sets the status word and the role leaves its loop; the
@@ -31,11 +30,10 @@ namespace nmg {
 // =========================================================================================================
 // Expansion pass
 // =========================================================================================================
-
 // Move `cnt` (1..8) consecutive elements of a shared-memory line to the destination planes and clear them in shared
 // memory.  VEC: cnt == 8 and both sides are 16-byte aligned.
-// PLAIN (fp32 only): the destination is an fp32 matrix, not two fp16 planes of values times `scale` (the densifier's use of this pass).
-template <typename T, bool VEC, bool PLAIN> __device__ __forceinline__ void expand_flush(const ExpandParams &p, T *line, int64_t off, int cnt, float scale) {
+// PLAIN (fp32 only): the destination is an fp32 matrix, not three bf16 planes (the densifier's use of this pass).
+template <typename T, bool VEC, bool PLAIN> __device__ __forceinline__ void expand_flush(const ExpandParams &p, T *line, int64_t off, int cnt) {
     if constexpr (sizeof(T) == 4 && PLAIN) {
         float *d = static_cast<float *>(p.dst) + off;
         if (VEC) {
@@ -55,34 +53,27 @@ template <typename T, bool VEC, bool PLAIN> __device__ __forceinline__ void expa
             for (int i = 0; i < cnt; i++) { d[i] = line[i]; line[i] = DT<T>::from_f32(0.f); }
         }
     } else {
-        __half *d = static_cast<__half *>(p.dst) + off;
+        __nv_bfloat16 *d = static_cast<__nv_bfloat16 *>(p.dst) + off;
         if (VEC) {
             const float4 a = *reinterpret_cast<const float4 *>(line), b = *reinterpret_cast<const float4 *>(line + 4);
             *reinterpret_cast<float4 *>(line) = make_float4(0.f, 0.f, 0.f, 0.f);
             *reinterpret_cast<float4 *>(line + 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-            uint4 h, l;
-            split_pair(a.x * scale, a.y * scale, h.x, l.x);
-            split_pair(a.z * scale, a.w * scale, h.y, l.y);
-            split_pair(b.x * scale, b.y * scale, h.z, l.z);
-            split_pair(b.z * scale, b.w * scale, h.w, l.w);
-            *reinterpret_cast<uint4 *>(d) = h;
-            *reinterpret_cast<uint4 *>(d + p.plane_elems) = l;
+            uint32_t w[3][4];
+            split3_pair(a.x, a.y, w[0][0], w[1][0], w[2][0]);
+            split3_pair(a.z, a.w, w[0][1], w[1][1], w[2][1]);
+            split3_pair(b.x, b.y, w[0][2], w[1][2], w[2][2]);
+            split3_pair(b.z, b.w, w[0][3], w[1][3], w[2][3]);
+#pragma unroll
+            for (int c = 0; c < 3; c++) *reinterpret_cast<uint4 *>(d + c * p.plane_elems) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
         } else {
             for (int i = 0; i < cnt; i++) {
-                const float x = line[i] * scale;
-                const __half h = __float2half_rn(x);
+                __nv_bfloat16 x[3];
+                split3(line[i], x);
                 line[i] = 0.f;
-                d[i] = h;
-                d[p.plane_elems + i] = __float2half_rn(x - __half2float(h));
+                for (int c = 0; c < 3; c++) d[c * p.plane_elems + i] = x[c];
             }
         }
     }
-}
-// Largest magnitude of a line of the destination, from its parts
-__device__ __forceinline__ uint32_t line_max(const ExpandParams &p, int64_t line) {
-    uint32_t mx = 0;
-    for (int s = 0; s < p.spans; s++) mx = max(mx, p.maxima[s * p.lines + line]);
-    return mx;
 }
 
 // Work item = (column chunk kc, R consecutive row-blocks).  The item's dense tile lives in shared memory, in the
@@ -97,10 +88,8 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_dense_kernel(const Expa
     constexpr bool VEC_OK = N_ > 0;
     const int n = N_ > 0 ? N_ : prm.n, m = prm.m, g = prm.g, cc = prm.cc, R = prm.R, pitch = prm.pitch;
     const int lines = TR ? cc : R * m;
-    constexpr bool SCALED = sizeof(T) == 4 && !PLAIN;
     T *tile = reinterpret_cast<T *>(smem);                                  // [lines][pitch]
-    float *scale = reinterpret_cast<float *>(tile + (size_t)lines * pitch);  // SCALED: [lines]
-    int8_t *ord = reinterpret_cast<int8_t *>(scale + (SCALED ? lines : 0));  // [C][n]
+    int8_t *ord = reinterpret_cast<int8_t *>(tile + (size_t)lines * pitch);  // [C][n]
     // The matmul kernel that follows may become resident and run its prologue while this grid drains, and reads nothing this grid
     // writes before its dependents_wait; this one's prologue runs beside the kernel ahead.
     dependents_launch();
@@ -117,18 +106,9 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_dense_kernel(const Expa
         const int64_t kc = item / groups, mb0 = (item - kc * groups) * R;
         const int rj = (int)(prm.nb - mb0 < R ? prm.nb - mb0 : R);  // row-blocks in this item
         __syncthreads();  // the tile is all zeros again
-        const int64_t col0 = kc * cc, r0 = mb0 * m;
-        if constexpr (SCALED) {
-            const int64_t first = TR ? col0 : r0, extent = TR ? prm.K : prm.M;
-            for (int l = threadIdx.x; l < lines; l += EXPAND_THREADS) {
-                if (first + l >= extent) continue;
-                const int e = line_exp(line_max(prm, first + l));
-                scale[l] = pow2(-e);
-                if ((TR ? mb0 : kc) == 0) prm.factors[first + l] = pow2(e);
-            }
-        }
         expand_scatter_item<T, TR, N_>(prm, tile, ord, kc, mb0, rj);
         __syncthreads();
+        const int64_t col0 = kc * cc, r0 = mb0 * m;
         // line l, elements e .. e+7 -> dst[(TR ? col0 + l : r0 + l)][(TR ? r0 : col0) + e]
         const int64_t line_lim = TR ? prm.K - col0 : prm.M - r0;   // lines inside the weight
         const int64_t elem_lim = TR ? prm.M - r0 : prm.K - col0;   // elements of a line inside the weight
@@ -146,11 +126,11 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_dense_kernel(const Expa
             // A full vector may run past the item's elements only into the row's padding (last chunk / last group:
             // ld = round_up(extent, 8)), never into elements another item owns.
             if (aligned && (e + 8 <= ne || ne >= elem_lim)) {
-                expand_flush<T, true, PLAIN>(prm, line, off, 8, SCALED ? scale[l] : 1.f);
+                expand_flush<T, true, PLAIN>(prm, line, off, 8);
             } else {
                 int cnt = ne - e < 8 ? ne - e : 8;
                 if (elem_lim - e < cnt) cnt = (int)(elem_lim - e);
-                expand_flush<T, false, PLAIN>(prm, line, off, cnt, SCALED ? scale[l] : 1.f);
+                expand_flush<T, false, PLAIN>(prm, line, off, cnt);
                 // elements of the vector past cnt were never written by this item's valid slots; clear them anyway
                 for (int i = cnt; i < 8; i++) line[i] = DT<T>::from_f32(0.f);
             }
@@ -168,11 +148,9 @@ template <typename T, int N_, bool PLAIN>
 __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const ExpandParams prm) {
     extern __shared__ __align__(16) char smem[];
     const int m = prm.m, g = prm.g, cc = prm.cc, R = prm.R, Q = prm.Q, cols = Q * cc, rows = R * m;
-    constexpr bool SCALED = sizeof(T) == 4 && !PLAIN;
     T *tile = reinterpret_cast<T *>(smem);                                 // [rows][cols]
-    float *scale = reinterpret_cast<float *>(tile + (size_t)rows * cols);  // SCALED: [rows]
-    int8_t *ord = reinterpret_cast<int8_t *>(scale + (SCALED ? rows : 0));  // [C][n]
-    dependents_launch();  // see expand_dense_kernel
+    int8_t *ord = reinterpret_cast<int8_t *>(tile + (size_t)rows * cols);  // [C][n]
+    dependents_launch();                                                   // see expand_dense_kernel
 
     constexpr int VL = N_ * (int)sizeof(T) / 2;  // 16-byte loads of values per 8 slots
     const int per_chunk = R * cc / 8, tid = (int)threadIdx.x;
@@ -182,10 +160,8 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
     const int groups = (int)((prm.nb + R - 1) / R), spans = (int)((prm.nc + Q - 1) / Q);
     const int64_t items = (int64_t)groups * spans;
     uint4 iv, vv[VL];
-    uint32_t mx = 0;  // SCALED: largest magnitude of row tid
     auto load = [&](int64_t item) {
         const int span = (int)(item / groups), grp = (int)(item - (int64_t)span * groups);
-        if constexpr (SCALED) if (tid < rows && (int64_t)grp * rows + tid < prm.lines) mx = line_max(prm, (int64_t)grp * rows + tid);
         iv = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);  // column -1: no slot
         if (!has || span * Q + uq >= prm.nc || grp * R + uj >= prm.nb) return;
         const int64_t slot = ((int64_t)(span * Q + uq) * prm.nb + grp * R + uj) * cc + uslot;
@@ -210,14 +186,6 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
     for (int64_t item = blockIdx.x; item < items; item += gridDim.x) {
         const int16_t *ci = reinterpret_cast<const int16_t *>(&iv);
         const T *vals = reinterpret_cast<const T *>(vv);
-        if constexpr (SCALED) {
-            if (tid < rows) {
-                const int e = line_exp(mx);
-                const int64_t row = (item % groups) * rows + tid;
-                scale[tid] = pow2(-e);
-                if (item < groups && row < prm.M) prm.factors[row] = pow2(e);
-            }
-        }
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             const int c = ci[k];
@@ -250,7 +218,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
                 if (inside) *reinterpret_cast<uint4 *>(static_cast<T *>(prm.dst) + off) = *reinterpret_cast<const uint4 *>(line);
                 *reinterpret_cast<uint4 *>(line) = make_uint4(0, 0, 0, 0);
             } else {
-                if (inside) expand_flush<T, true, PLAIN>(prm, line, off, V, scale[l]);
+                if (inside) expand_flush<T, true, PLAIN>(prm, line, off, V);
                 else {
                     reinterpret_cast<uint4 *>(line)[0] = make_uint4(0, 0, 0, 0);
                     reinterpret_cast<uint4 *>(line)[1] = make_uint4(0, 0, 0, 0);
@@ -263,7 +231,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
     }
 }
 // R and Q of the rows kernel, false when it does not serve the weight
-static bool expand_rows_plan(const Geo &geo, size_t es, bool scaled, int *R, int *Q, size_t *smem) {
+static bool expand_rows_plan(const Geo &geo, size_t es, int *R, int *Q, size_t *smem) {
     if (geo.n < 1 || geo.n > 2 || geo.cc % 8 != 0 || geo.nb > 0x3fffffff || geo.nc > 0x3fffffff) return false;
     int q = 512 / geo.cc;
     if (q < 1) q = 1;
@@ -272,12 +240,11 @@ static bool expand_rows_plan(const Geo &geo, size_t es, bool scaled, int *R, int
     int r = EXPAND_THREADS * 8 / cols;                                  // one piece per thread
     const int fit = (int)(32 * 1024 / ((size_t)geo.m * cols * es));     // seven CTAs per SM
     if (r > fit) r = fit;
-    if (scaled && r * geo.m > EXPAND_THREADS) r = EXPAND_THREADS / geo.m;  // a thread per row for the scales
     if (r < 1) r = 1;
     const size_t bytes = (size_t)r * geo.m * cols * es;
-    if (bytes > 64 * 1024 || r * cols / 8 > EXPAND_THREADS || (scaled && geo.m > EXPAND_THREADS)) return false;
+    if (bytes > 64 * 1024 || r * cols / 8 > EXPAND_THREADS) return false;
     *R = r; *Q = q;
-    *smem = bytes + (scaled ? (size_t)r * geo.m * 4 : 0) + (size_t)geo.C * geo.n + 16;
+    *smem = bytes + (size_t)geo.C * geo.n + 16;
     return true;
 }
 
@@ -294,115 +261,32 @@ static int expand_rows_per_item(const Geo &geo, size_t es, bool tr) {
 }
 
 // =========================================================================================================
-// fp32 operands: row maxima and planes of the activation
+// fp32 activations: three bf16 planes and a factor per row
 // =========================================================================================================
-// Largest magnitudes of the weight's destination lines (weight rows, or columns for the transposed product), by parts: a unit is one
-// row-block (chunk of columns) and a span of its tiles.  Magnitudes are compared as integers: NaN is largest.
-struct AbsMaxParams {
-    const float *val;
-    const int16_t *idx;
-    const int8_t *order;    // [C][n]
-    uint32_t *maxima;       // [spans][lines]
-    int64_t nb, nc, lines;
-    int n, m, g, cc, transposed;
-    int spans, per;         // parts of a line, tiles per part
-};
-constexpr int PREP_THREADS = 128;
-__device__ __forceinline__ uint32_t magnitude(float v) { return __float_as_uint(v) & 0x7fffffffu; }
-
-__device__ __forceinline__ void weight_absmax_unit(const AbsMaxParams &p, int64_t unit, uint32_t *mx) {
-    const int64_t group = unit / p.spans;
-    if (group >= (p.transposed ? p.nc : p.nb)) return;  // all threads
-    const int span = (int)(unit - group * p.spans), cc = p.cc, lines = p.transposed ? cc : p.m;
-    const int64_t tiles = p.transposed ? p.nb : p.nc, first = (int64_t)span * p.per;
-    const int count = (int)(tiles - first < p.per ? (tiles - first > 0 ? tiles - first : 0) : p.per);
-    for (int l = threadIdx.x; l < lines; l += (int)blockDim.x) mx[l] = 0;
-    __syncthreads();
-    const bool quads = (p.g & 3) == 0;  // four consecutive slots belong to one pattern
-    for (int64_t e = (int64_t)threadIdx.x * 4; e < (int64_t)count * cc; e += (int)blockDim.x * 4) {
-        const int t = (int)(e / cc), s0 = (int)(e - (int64_t)t * cc), left = cc - s0 < 4 ? cc - s0 : 4;
-        // tiles of consecutive row-blocks of one chunk are consecutive in memory
-        const int64_t slot = (p.transposed ? group * p.nb + first + t : (first + t) * p.nb + group) * cc + s0;
-        if (left == 4 && quads && !p.transposed) {
-            for (int i = 0; i < p.n; i++) {
-                uint32_t v = 0;
-#pragma unroll
-                for (int u = 0; u < 4; u++) v = max(v, magnitude(__ldg(p.val + (slot + u) * p.n + i)));
-                atomicMax(&mx[p.order[(s0 / p.g) * p.n + i]], v);
-            }
-            continue;
-        }
-        // cc need not be a multiple of four: a piece that crosses into the next tile is finished slot by slot
-        for (int u = 0; u < 4 && e + u < (int64_t)count * cc; u++) {
-            const int tu = s0 + u < cc ? t : (int)((e + u) / cc), su = (int)(e + u - (int64_t)tu * cc);
-            const int64_t sl = (p.transposed ? group * p.nb + first + tu : (first + tu) * p.nb + group) * cc + su;
-            const int c = p.transposed ? p.idx[sl] : 0;
-            if ((unsigned)c >= (unsigned)cc) continue;  // a malformed index is ignored, never dereferenced
-            uint32_t all = 0;
-            for (int i = 0; i < p.n; i++) {
-                const uint32_t v = magnitude(__ldg(p.val + sl * p.n + i));
-                if (p.transposed) all = max(all, v);
-                else atomicMax(&mx[p.order[(su / p.g) * p.n + i]], v);
-            }
-            if (p.transposed) atomicMax(&mx[c], all);
-        }
-    }
-    __syncthreads();
-    for (int l = threadIdx.x; l < lines; l += (int)blockDim.x) p.maxima[span * p.lines + group * lines + l] = mx[l];
-}
-
 struct SplitParams {
     const float *src;
-    __half *dst;            // [ACT_PLANES][rows][ld]: the rows' planes, then those of wide rows' small values
-    float *factors;         // [rows] 2^e
-    float *small;           // [rows] factor of the small values' planes relative to the others, or NOT_WIDE
+    __nv_bfloat16 *dst;     // [SPLIT_PLANES][rows][ld]
+    float *factors;         // [rows] TINY_FACTOR for rows split times TINY_SCALE; anything else counts as one (a row of zeros may have no entry)
     int64_t rows, cols, ld_src, ld;
-    int64_t ctas;           // CTAs (clusters) of the activation; those behind them take the weight's units
-    // K-major source: the rows' values are looked at by ranges of the reduction axis, factors and small are [ranges][scale_ld]
-    int64_t range, scale_ld; // reduction elements per range, a multiple of 64
-    int cluster, per;        // CTAs of a range, and reduction elements of each
 };
-// Scales and factors of a row of the given largest magnitudes (small: of a wide row's small values, else 0)
-__device__ __forceinline__ void write_factors(const SplitParams &p, int64_t r, bool wide, uint32_t mx, uint32_t mx_small) {  // r: index of factors
-    const int e = line_exp(mx), d = line_exp(mx_small) - e;
-    p.factors[r] = pow2(e);
-    p.small[r] = !wide ? NOT_WIDE : d >= -126 ? pow2(d) : d >= -149 ? __uint_as_float(1u << (149 + d)) : 0.f;
-}
-__device__ __forceinline__ void store_planes(const SplitParams &p, int plane, int64_t r, int64_t c, const float (&f)[8], float s) {
-    uint4 h, l;
-    split_pair(f[0] * s, f[1] * s, h.x, l.x);
-    split_pair(f[2] * s, f[3] * s, h.y, l.y);
-    split_pair(f[4] * s, f[5] * s, h.z, l.z);
-    split_pair(f[6] * s, f[7] * s, h.w, l.w);
-    __half *d = p.dst + (plane * p.rows + r) * p.ld + c;
-    *reinterpret_cast<uint4 *>(d) = h;
-    *reinterpret_cast<uint4 *>(d + p.rows * p.ld) = l;
-}
-__device__ __forceinline__ void store_split(const SplitParams &p, int64_t r, int64_t c, const float (&f)[8], bool wide, uint32_t mx, float s, float s_small) {
-    if (!wide) { store_planes(p, 0, r, c, f, s); return; }
-    float big[8], small[8];
+__device__ __forceinline__ void store_split(const SplitParams &p, int64_t r, int64_t c, const float (&f)[8], float scale) {
+    uint4 w[SPLIT_PLANES];
+    split3_pair(f[0] * scale, f[1] * scale, w[0].x, w[1].x, w[2].x);
+    split3_pair(f[2] * scale, f[3] * scale, w[0].y, w[1].y, w[2].y);
+    split3_pair(f[4] * scale, f[5] * scale, w[0].z, w[1].z, w[2].z);
+    split3_pair(f[6] * scale, f[7] * scale, w[0].w, w[1].w, w[2].w);
+    __nv_bfloat16 *d = p.dst + r * p.ld + c;
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        const bool sm = is_small(f[i], mx);
-        big[i] = sm ? 0.f : f[i];
-        small[i] = sm ? f[i] : 0.f;
-    }
-    store_planes(p, 0, r, c, big, s);
-    store_planes(p, 2, r, c, small, s_small);
+    for (int t = 0; t < SPLIT_PLANES; t++) *reinterpret_cast<uint4 *>(d + t * p.rows * p.ld) = w[t];
 }
 
-// CTAs of the activation: one row per CTA, or one per warp where a warp's registers hold it (ROWS = 4).  The row is read once for what
-// its values are like and kept; what the registers do not hold is read again.  HBM-bound, 8 bytes per value.
-// REST: there are units of a weight, or rows that the registers do not hold.
-template <int ROWS, bool REST>
-__global__ void __launch_bounds__(PREP_THREADS) split_rows_kernel(const SplitParams p, const AbsMaxParams w) {
-    extern __shared__ uint32_t mx[];
-    __shared__ RowStats warp_stats[PREP_THREADS / 32];
-    __shared__ uint32_t warp_small[PREP_THREADS / 32];
+// One row per CTA, or one per warp where a warp's registers hold it (ROWS = 4).  HBM-bound: 4 bytes read and 6 written per value.  The
+// part that the registers hold nearly always settles that the row is not tiny; only if it does not is the rest read twice.
+constexpr int SPLIT_THREADS = 128;
+template <int ROWS> __global__ void __launch_bounds__(SPLIT_THREADS) split_rows_kernel(const SplitParams p) {
     dependents_launch();
     dependents_wait();
-    if (REST && blockIdx.x >= p.ctas) { weight_absmax_unit(w, blockIdx.x - p.ctas, mx); return; }
-    constexpr int LANES = PREP_THREADS / ROWS, HELD = 4;
+    constexpr int LANES = SPLIT_THREADS / ROWS, HELD = 4;
     const int sub = threadIdx.x / LANES, tid = threadIdx.x - sub * LANES;
     const int64_t r = (int64_t)blockIdx.x * ROWS + sub;
     if (ROWS > 1 && r >= p.rows) return;  // whole warps
@@ -410,184 +294,109 @@ __global__ void __launch_bounds__(PREP_THREADS) split_rows_kernel(const SplitPar
     const bool vec = (reinterpret_cast<uintptr_t>(row) & 15) == 0;
     auto load = [&](int64_t c, float (&f)[8]) {
         if (vec && c + 8 <= p.cols) {
-            const float4 a = __ldg(reinterpret_cast<const float4 *>(row + c)), b = __ldg(reinterpret_cast<const float4 *>(row + c + 4));
+            const float4 a = *reinterpret_cast<const float4 *>(row + c), b = *reinterpret_cast<const float4 *>(row + c + 4);
             f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
         } else {
 #pragma unroll
             for (int i = 0; i < 8; i++) f[i] = c + i < p.cols ? row[c + i] : 0.f;
         }
     };
+    auto any = [&](bool v) -> bool { return ROWS > 1 ? __any_sync(0xffffffffu, v) : __syncthreads_or(v); };
     float held[HELD][8];
-    auto each = [&](auto &&fn) {  // fn(column, eight values), of this thread's part of the row
-#pragma unroll
-        for (int h = 0; h < HELD; h++) {
-            const int64_t c = ((int64_t)h * LANES + tid) * 8;
-            if (c < p.ld) fn(c, held[h]);
-        }
-        for (int64_t c = ((int64_t)HELD * LANES + tid) * 8; REST && c < p.ld; c += LANES * 8) {
-            float f[8];
-            load(c, f);
-            fn(c, f);
-        }
-    };
+    bool big = false;
 #pragma unroll
     for (int h = 0; h < HELD; h++) {
         const int64_t c = ((int64_t)h * LANES + tid) * 8;
-        if (c < p.ld) load(c, held[h]);
+        if (c >= p.ld) break;
+        load(c, held[h]);
     }
-    RowStats st;
-    each([&](int64_t, const float (&f)[8]) {
 #pragma unroll
-        for (int i = 0; i < 8; i++) st.add(f[i]);
-    });
-    st.mx = __reduce_max_sync(0xffffffffu, st.mx);
-    st.exps = __reduce_add_sync(0xffffffffu, st.exps);
-    st.count = __reduce_add_sync(0xffffffffu, st.count);
-    if constexpr (ROWS == 1) {
-        if ((threadIdx.x & 31) == 0) warp_stats[threadIdx.x >> 5] = st;
-        __syncthreads();
-        st = RowStats();
+    for (int h = 0; h < HELD; h++) {
+        const int64_t c = ((int64_t)h * LANES + tid) * 8;
+        if (c >= p.ld) break;
 #pragma unroll
-        for (int i = 0; i < PREP_THREADS / 32; i++) {
-            st.mx = max(st.mx, warp_stats[i].mx);
-            st.exps += warp_stats[i].exps;
-            st.count += warp_stats[i].count;
+        for (int i = 0; i < 8; i++) big |= not_tiny(held[h][i]);
+    }
+    big = any(big);
+    constexpr int64_t FIRST = (int64_t)HELD * LANES * 8;  // not held from here on
+    for (int64_t c0 = FIRST; c0 < p.ld && !big; c0 += LANES * 8) {
+        float f[8];
+        bool b = false;
+        if (c0 + tid * 8 < p.ld) {
+            load(c0 + tid * 8, f);
+#pragma unroll
+            for (int i = 0; i < 8; i++) b |= not_tiny(f[i]);
         }
+        big = any(b);
     }
-    const bool wide = st.wide();  // of the whole row: the same for all its threads
-    uint32_t mx_small = 0;
-    if (wide) {
-        each([&](int64_t, const float (&f)[8]) {
+    if (tid == 0) p.factors[r] = big ? 1.f : TINY_FACTOR;
+    const float scale = big ? 1.f : TINY_SCALE;
 #pragma unroll
-            for (int i = 0; i < 8; i++)
-                if (is_small(f[i], st.mx)) mx_small = max(mx_small, magnitude(f[i]));
-        });
-        mx_small = __reduce_max_sync(0xffffffffu, mx_small);
-        if constexpr (ROWS == 1) {
-            if ((threadIdx.x & 31) == 0) warp_small[threadIdx.x >> 5] = mx_small;
-            __syncthreads();
-#pragma unroll
-            for (int i = 0; i < PREP_THREADS / 32; i++) mx_small = max(mx_small, warp_small[i]);
-        }
+    for (int h = 0; h < HELD; h++) {
+        const int64_t c = ((int64_t)h * LANES + tid) * 8;
+        if (c >= p.ld) break;
+        store_split(p, r, c, held[h], scale);
     }
-    if (tid == 0) write_factors(p, r, wide, st.mx, mx_small);
-    const float s = pow2(-line_exp(st.mx)), s_small = pow2(-line_exp(mx_small));
-    each([&](int64_t c, const float (&f)[8]) { store_split(p, r, c, f, wide, st.mx, s, s_small); });
+    for (int64_t c = FIRST + tid * 8; c < p.ld; c += LANES * 8) {
+        float f[8];
+        load(c, f);
+        store_split(p, r, c, f, scale);
+    }
 }
 
-// The same from a K-major activation src[red][ld_src >= tokens], transposed on the way.  A cluster owns 32 tokens of one range of the
-// reduction axis, its CTAs a part each; what the tokens' values are like is put together through distributed shared memory, so that
-// this is one launch.  The first COLS_HELD reduction elements of a CTA's part stay in shared memory, the others are read again (from
-// L2).  Ranges of a fused matmul with a split reduction are mostly one CTA's: 1024 x 256 tokens, 6 ranges.
-constexpr int COLS_THREADS = 512, COLS_WARPS = COLS_THREADS / 32, COLS_HELD = 256, COLS_CLUSTER = 8, COLS_STEP = COLS_THREADS / 4;
-struct TokenStats { uint32_t mx[32], exps[32], count[32], small[32]; };  // of 32 tokens
-// CLUSTER: a range is several CTAs'.  REST: there are units of a weight, or parts that do not fit COLS_HELD.  A few microseconds of
-// work are bound by what is executed for the first time: mm 1024 x 1024, 256 columns, took 15.5 us with all cases in one kernel, 13.1 now.
-template <bool CLUSTER, bool REST>
-__global__ void __launch_bounds__(COLS_THREADS, 2) split_columns_kernel(const SplitParams p, const AbsMaxParams w) {
-    extern __shared__ uint32_t mx[];
-    __shared__ float tile[COLS_HELD][33];              // [reduction][token]
-    __shared__ TokenStats ours, ranks[CLUSTER ? COLS_CLUSTER : 1];   // ranks: written by the cluster's CTAs
-    const int cl = CLUSTER ? p.cluster : 1, range = (int)blockIdx.x / cl, rank = (int)blockIdx.x - range * cl;
+// The same from a K-major activation src[red][ld_src >= tokens], transposed through a 64 x 32 tile on the way.  A CTA looks at the rest of
+// a token's row only if its own part holds values of it and none that settles the matter.
+constexpr int COLS_THREADS = 256, COLS_RED = 64;
+__global__ void __launch_bounds__(COLS_THREADS) split_columns_kernel(const SplitParams p) {
+    __shared__ float tile[COLS_RED][33];   // [reduction][token]
+    __shared__ unsigned big, nonzero;      // by token
     dependents_launch();
-    if (threadIdx.x < 4 * 32) reinterpret_cast<uint32_t *>(&ours)[threadIdx.x] = 0;
-    __syncthreads();
     dependents_wait();
-    if (REST && blockIdx.y >= p.ctas) {  // whole clusters; the units of a tall weight are more than a grid has rows
-        const int64_t units = (w.transposed ? w.nc : w.nb) * w.spans, step = (int64_t)(gridDim.y - p.ctas) * gridDim.x;
-        for (int64_t unit = (int64_t)(blockIdx.y - p.ctas) * gridDim.x + blockIdx.x; unit < units; unit += step) {
-            weight_absmax_unit(w, unit, mx);
-            __syncthreads();
-        }
-        return;
-    }
-    if (cl > 1) cluster_arrive();  // waited for before anything is written to another CTA
+    const int64_t k0 = (int64_t)blockIdx.x * COLS_RED;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t t0 = (int64_t)blockIdx.y * 32, t = t0 + lane, k0 = range * p.range + (int64_t)rank * p.per;
-    const int64_t range_end = (range + 1) * p.range < p.cols ? (range + 1) * p.range : p.cols, left = range_end - k0;
-    const int count = (int)(left < p.per ? (left > 0 ? left : 0) : p.per);  // of this CTA's part
-    const float *src = p.src + k0 * p.ld_src + t;
-    const int lim = t < p.rows ? count : 0;
-    auto at = [&](int k) -> float { return k < lim ? __ldg(src + k * p.ld_src) : 0.f; };
-    RowStats st;
-    {
-        constexpr int N = COLS_HELD / COLS_WARPS;
-        float v[N];
-#pragma unroll
-        for (int i = 0; i < N; i++) v[i] = at(warp + i * COLS_WARPS);
-#pragma unroll
-        for (int i = 0; i < N; i++) {
-            tile[warp + i * COLS_WARPS][lane] = v[i];
-            st.add(v[i]);
-        }
-    }
-    if constexpr (REST) {
-#pragma unroll 8
-        for (int k = COLS_HELD + warp; k < count; k += COLS_WARPS) st.add(at(k));
-    }
-    atomicMax(&ours.mx[lane], st.mx);
-    atomicAdd(&ours.exps[lane], st.exps);
-    atomicAdd(&ours.count[lane], st.count);
-    __syncthreads();
-    const TokenStats *from = &ours;
-    int parts = 1;
-    if (cl > 1) {
-        cluster_wait();
-        if (warp < cl) {  // one warp per CTA of the cluster
-            const uint32_t dst = map_to_rank(smem_u32(&ranks[rank].mx[lane]), (uint32_t)warp);
-            st_cluster(dst, ours.mx[lane]);
-            st_cluster(dst + 128, ours.exps[lane]);
-            st_cluster(dst + 256, ours.count[lane]);
-        }
-        cluster_sync_all();
-        from = ranks;
-        parts = cl;
-    }
-    auto gather = [&](int token) -> RowStats {
-        RowStats a;
-        for (int c = 0; c < parts; c++) {
-            a.mx = max(a.mx, from[c].mx[token]);
-            a.exps += from[c].exps[token];
-            a.count += from[c].count[token];
-        }
-        return a;
-    };
-    constexpr int PER_TOKEN = COLS_THREADS / 32;  // threads of a token, eight reduction elements each
-    const int tok = threadIdx.x / PER_TOKEN, c8 = (threadIdx.x % PER_TOKEN) * 8;
-    const RowStats mine = gather(lane), theirs = gather(tok);
-    const bool wide = theirs.wide();
-    uint32_t mx_small = 0;
-    if (__any_sync(0xffffffffu, mine.wide())) {  // the same in every warp of the cluster
-        uint32_t sm = 0;
-        for (int k = warp; k < count; k += COLS_WARPS) {
-            const float v = !REST || k < COLS_HELD ? tile[k][lane] : at(k);
-            if (is_small(v, mine.mx)) sm = max(sm, magnitude(v));
-        }
-        atomicMax(&ours.small[lane], sm);
+    for (int64_t t0 = (int64_t)blockIdx.y * 32; t0 < p.rows; t0 += (int64_t)gridDim.y * 32) {
+        __syncthreads();  // the tile and the masks of the tokens before have been read
+        if (threadIdx.x == 0) big = nonzero = 0;
         __syncthreads();
-        if (cl > 1) {
-            if (warp < cl) st_cluster(map_to_rank(smem_u32(&ranks[rank].small[lane]), (uint32_t)warp), ours.small[lane]);
-            cluster_sync_all();
-        }
-        if (wide)
-            for (int c = 0; c < parts; c++) mx_small = max(mx_small, from[c].small[tok]);
-    }
-    if (rank == 0 && c8 == 0 && t0 + tok < p.rows) write_factors(p, range * p.scale_ld + t0 + tok, wide, theirs.mx, mx_small);
-    const float s = pow2(-line_exp(theirs.mx)), s_small = pow2(-line_exp(mx_small));
-    for (int kb = 0; kb < count; kb += COLS_STEP) {
-        const int base = !REST || kb < COLS_HELD ? kb : 0;
-        if (REST && kb >= COLS_HELD) {
-            __syncthreads();
+        const int64_t t = t0 + lane;
+        auto at = [&](int64_t k) -> float { return k < p.cols && t < p.rows ? p.src[k * p.ld_src + t] : 0.f; };
+        bool b = false, nz = false;
 #pragma unroll
-            for (int i = 0; i < COLS_STEP / COLS_WARPS; i++) tile[warp + i * COLS_WARPS][lane] = at(kb + warp + i * COLS_WARPS);
-            __syncthreads();
+        for (int i = 0; i < COLS_RED / 8; i++) {
+            const float v = at(k0 + warp + i * 8);
+            tile[warp + i * 8][lane] = v;
+            b |= not_tiny(v);
+            nz |= v != 0.f;
         }
-        const int64_t k = k0 + kb + c8;
-        if (t0 + tok < p.rows && kb + c8 < count) {  // ld is cols rounded up to eight
+        const unsigned bm = __ballot_sync(0xffffffffu, b), nm = __ballot_sync(0xffffffffu, nz);
+        if (lane == 0) {
+            atomicOr(&big, bm);
+            atomicOr(&nonzero, nm);
+        }
+        __syncthreads();
+        const unsigned here = big, own = nonzero;  // `big` may grow below
+        if (own & ~here) {  // the same for all threads
+            __syncthreads();
+            for (int64_t k = 0; k < p.cols; k += 64) {
+                b = false;
+#pragma unroll
+                for (int i = 0; i < 8; i++) b |= not_tiny(at(k + warp + i * 8));
+                const unsigned m = __ballot_sync(0xffffffffu, b);
+                if (lane == 0) atomicOr(&big, m);
+                __syncthreads();
+                const unsigned now = big;
+                __syncthreads();
+                if (!(own & ~now)) break;
+            }
+        }
+        const unsigned mask = big;
+        if (threadIdx.x < 32 && t < p.rows && ((own >> lane) & 1)) p.factors[t] = ((mask >> lane) & 1) ? 1.f : TINY_FACTOR;  // CTAs that write agree
+        const int r = threadIdx.x >> 3, c8 = (threadIdx.x & 7) * 8;  // token within the tile, reduction offset
+        if (t0 + r < p.rows && k0 + c8 < p.ld) {
             float f[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) f[i] = tile[base + c8 + i][tok];
-            store_split(p, t0 + tok, k, f, wide, theirs.mx, s, s_small);
+            for (int i = 0; i < 8; i++) f[i] = tile[c8 + i][r];
+            store_split(p, t0 + r, k0 + c8, f, ((own & ~mask) >> r) & 1 ? TINY_SCALE : 1.f);
         }
     }
 }
@@ -628,8 +437,8 @@ struct GemmParams {
     GemmTiles tiles;       // one CTA per tile of 128 features, or a pair per 256
     int band;              // width of the tile order's bands, in feature tiles
     unsigned *wave_ctr;    // zeroed counter for the producers' soft rendezvous before every tile, or NULL
-    const float *fac_rows, *fac_cols;  // fp32: factors of the accumulator's rows and columns (2^line_exp)
-    const float *small;                // fp32: of the activation's rows, see SplitParams
+    const float *factors;  // fp32: of the activation's rows, see SplitParams
+    int chunk_kb;          // fp32: k-blocks per chunk of the accumulator, see tc_dense_gemm
     int a_rows, b_rows;                // rows of a plane
     int *status;
 };
@@ -649,14 +458,14 @@ struct GemmMaps {
 // 48 KB, which is what keeps the tensor core fed from L2.  full[s] lives in the even ("leader") CTA and receives the TMA
 // bytes of both; empty[s] and acc_full[b] exist in both CTAs and are signalled by multicast commits; acc_free[b] lives in
 // the leader and collects the drain warps of both CTAs.  No load is multicast.
-// fp32 (always pairs): a stage is one k-block of all four planes, 64 KB, and its three products run from it (a stage per product
-// would take more than L2 delivers).
+// fp32 (always pairs): a stage is one k-block of all six planes, 96 KB, and its six products run from it (a stage per product, 48 KB per
+// 512 clocks and SM, is over what L2 delivers).
 // TMA_OUT = true: the one-destination staged output, leaving as tiled bulk stores; only that output path is compiled,
 // which keeps the drain warps' code and register needs small.  TMA_OUT = false: every other output form.
 template <typename T, bool PAIR, bool TMA_OUT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmParams prm, const __grid_constant__ GemmMaps maps) {
     constexpr bool SPLIT = sizeof(T) == 4;
-    constexpr int TERMS = SPLIT ? 3 : 1;
+    constexpr int TERMS = SPLIT ? SPLIT_TERMS : 1;
     using E = typename TcMode<T>::elem;
     static_assert(PAIR || !SPLIT, "fp32 runs on CTA pairs");
     constexpr int NBUF = 2;  // accumulator tiles in flight between the MMA issuer and the drain warps
@@ -664,7 +473,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     constexpr int PLANES = SPLIT ? SPLIT_PLANES : 1;
     constexpr int B_BYTES = PAIR ? TC_B_BYTES / 2 : TC_B_BYTES;  // room of one plane; the widest tile fills it
     constexpr int OFF_B = PLANES * TC_A_BYTES, STAGE_BYTES = OFF_B + PLANES * B_BYTES;
-    constexpr int STAGES = GEMM_RING_BYTES / STAGE_BYTES;  // 4, 6 for pairs, 3 for fp32
+    constexpr int STAGES = GEMM_RING_BYTES / STAGE_BYTES;  // 4, 6 for pairs, 2 for fp32
     constexpr int TILE_FEATS = PAIR ? 2 * TC_BM : TC_BM;
 
     extern __shared__ char smem_raw[];
@@ -687,7 +496,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     const int ntiles = prm.tiles.count(), nwide = prm.tiles.wide();
     const int my_tiles = (unit_id < ntiles) ? (ntiles - unit_id + nunits - 1) / nunits : 0;
     const int nkb = (int)((prm.red + TC_BK - 1) / TC_BK);  // iterations per tile
-    const int chunk_it = SPLIT ? TC_CHUNK_KB : nkb;
+    const int chunk_it = SPLIT ? prm.chunk_kb : nkb;
     const int nchunks = (nkb + chunk_it - 1) / chunk_it;
 
     dependents_launch();
@@ -729,18 +538,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
         tok0 = tile_t * bn;
     };
 
-    // fp32: whether the tile holds a wide row of the activation (all lanes of a warp ask together)
-    auto tile_wide = [&](int ti) -> bool {
-        if constexpr (!SPLIT) return false;
-        int feat0, tok0, bn;
-        tile_origin(ti, feat0, tok0, bn);
-        const int64_t first = prm.bias_cols ? feat0 - (int)rank * TC_BM : tok0, limit = prm.bias_cols ? prm.out_feats : prm.ntok;
-        bool wide = false;
-        for (int i = lane; i < (prm.bias_cols ? TILE_FEATS : bn); i += 32)
-            if (first + i < limit) wide |= prm.small[first + i] != NOT_WIDE;
-        return __any_sync(0xffffffffu, wide);
-    };
-
     // fp32: the running sums take 128 registers of a drain warp.  Shares of the launch's 384 x 168: 128 x 56 + 256 x 224.
     if (warp < 4) {
     if constexpr (SPLIT) asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
@@ -757,7 +554,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
             int feat0, tok0, bn;
             tile_origin(ti, feat0, tok0, bn);
             const CUtensorMap *bmap = narrow(ti) ? &maps.b_tail : &maps.b;
-            const int total = tile_wide(ti) ? 2 * nkb : nkb;  // a wide tile: the reduction over either pair of the activation's planes
             if (prm.wave_ctr && ti > 0) {
                 // CTAs whose tiles share operand panels read them from HBM once only while they stream through the
                 // reduction in step; left alone they drift apart over the waves (measured: 2.2 MB of DRAM reads per
@@ -768,8 +564,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 if (lane == 0) soft_rendezvous(prm.wave_ctr, arrivals, (uint64_t)nkb * 40);
                 __syncwarp();
             }
-            for (int i = 0; i < total; i++, it++) {
-                const int kb = i < nkb ? i : i - nkb, x_plane = i < nkb ? 0 : 2;
+            for (int kb = 0; kb < nkb; kb++, it++) {
                 const int s = it % STAGES;
                 const uint32_t ph = (uint32_t)((it / STAGES) & 1);
                 if (!(ok = __all_sync(0xffffffffu, wait(&empty[s], ph ^ 1, 21)))) break;
@@ -780,9 +575,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                         if (leader) mbar_expect_tx(&full[s], (uint32_t)(2 * PLANES * (TC_A_BYTES + half * TC_BK * 2)));  // both CTAs report to this barrier
 #pragma unroll
                         for (int c = 0; c < PLANES; c++) {
-                            const int ap = prm.bias_cols ? c + x_plane : c, bp = prm.bias_cols ? c : c + x_plane;
-                            tma_load_2d_pair(stage + c * TC_A_BYTES, &maps.a, kb * TC_BK, ap * prm.a_rows + feat0, full_leader + s * 8);
-                            tma_load_2d_pair(stage + OFF_B + c * B_BYTES, bmap, kb * TC_BK, bp * prm.b_rows + tok0 + (int)rank * half, full_leader + s * 8);
+                            tma_load_2d_pair(stage + c * TC_A_BYTES, &maps.a, kb * TC_BK, c * prm.a_rows + feat0, full_leader + s * 8);
+                            tma_load_2d_pair(stage + OFF_B + c * B_BYTES, bmap, kb * TC_BK, c * prm.b_rows + tok0 + (int)rank * half, full_leader + s * 8);
                         }
                     } else {
                         mbar_expect_tx(&full[s], STAGE_BYTES);
@@ -796,17 +590,15 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (of the leader for pairs)
         if (leader) {
-            if constexpr (SPLIT) dependents_wait();  // tile_wide
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint64_t desc0 = make_sw128_desc(smem_u32(smem));
             bool ok = true;
             int it = 0, unit = 0;
             for (int ti = 0; ti < my_tiles && ok; ti++) {
-                const int units = tile_wide(ti) ? 2 * nchunks : nchunks;
                 uint32_t idesc = make_idesc<E>(!PAIR ? TC_BN : narrow(ti) ? prm.tiles.bn_tail : prm.tiles.bn);
                 if constexpr (PAIR) idesc = (idesc & ~(0x1fu << 24)) | ((uint32_t)(256 >> 4) << 24);  // M = 256 across the pair
-                for (int c = 0; c < units && ok; c++, unit++) {
-                    int kb = (c < nchunks ? c : c - nchunks) * chunk_it;
+                int kb = 0;
+                for (int c = 0; c < nchunks && ok; c++, unit++) {
                     const int b = unit % NBUF, use = unit / NBUF;
                     if (use > 0) ok = __all_sync(0xffffffffu, wait(&acc_free[b], (uint32_t)((use - 1) & 1), 26));
                     if (!ok) break;
@@ -823,8 +615,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
 #pragma unroll
                             for (int t = 0; t < TERMS; t++) {
                                 // bias_cols: the operands' roles are exchanged, the order of the products is not (equal results either way)
-                                const int wp = split_w(SPLIT_PLANES, t), xp = split_x(SPLIT_PLANES, t);
-                                const int ap = !SPLIT ? 0 : prm.bias_cols ? xp : wp, bp = !SPLIT ? 0 : prm.bias_cols ? wp : xp;
+                                const int ap = !SPLIT ? 0 : prm.bias_cols ? split_x(t) : split_w(t), bp = !SPLIT ? 0 : prm.bias_cols ? split_w(t) : split_x(t);
                                 const uint64_t adesc = stage_a + (uint32_t)(ap * (TC_A_BYTES / 16)), bdesc = stage_b + (uint32_t)(bp * (B_BYTES / 16));
 #pragma unroll
                                 for (int k = 0; k < TC_BK / 16; k++) {  // 16 elements = 32 bytes = 2 descriptor units per step
@@ -888,13 +679,6 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 const int64_t col = (int64_t)tok0 + (sl0 + i) * 32 + lane;
                 bcol[i] = (prm.bias && prm.bias_cols && col < prm.ntok) ? DT<T>::to_f32(static_cast<const T *>(prm.bias)[col]) : 0.f;
             }
-            // fp32: factors of this lane's row (see unscale)
-            float row_small = 1.f, row_large = 1.f;
-            const int units = tile_wide(ti) ? 2 * nchunks : nchunks;
-            if constexpr (SPLIT) {
-                const float f = feat_ok ? prm.fac_rows[feat] : 1.f;
-                (f < 1.f ? row_small : row_large) = f;
-            }
             // The residual of a slice (this lane's row, 32 elements) is fetched in 16-byte pieces one slice ahead of its
             // use, like the accumulator, when the bulk-store path runs and the residual's rows allow it.
             auto res_vec_ok = [&](int64_t tokc) -> bool { return TMA_OUT && prm.res_vec && tokc + 32 <= prm.ntok; };
@@ -907,11 +691,11 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                     }
                 }
             };
-            for (int c = 0; c < units; c++, unit++) {
+            for (int c = 0; c < nchunks; c++, unit++) {
                 const int b = unit % NBUF, use = unit / NBUF;
                 if (!(ok = wait(&acc_full[b], (uint32_t)(use & 1), 25))) break;
                 tc_fence_after();
-                const bool last = c == units - 1;
+                const bool last = c == nchunks - 1;
                 auto release = [&]() {  // this warp's TMEM reads of the unit are done: the issuer may reuse the accumulator once all warps say so
                     tc_fence_before();
                     __syncwarp();
@@ -925,15 +709,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 auto handle = [&](int sl, uint32_t (&r)[32], const uint4 (&qr)[RQ]) {
                     if (!(SPLIT && TMA_OUT) && sl == sl0 + nsl - 1) release();
                     const int64_t tokc = (int64_t)tok0 + sl * 32;
-                    if constexpr (SPLIT) {  // the columns' factors are padded to whole tiles
-                        const float4 *fac = reinterpret_cast<const float4 *>(prm.fac_cols + tokc);
+                    if constexpr (SPLIT) {  // tiny rows of the activation: this lane's row, or columns of the slice
+                        const bool rows = prm.bias_cols != 0;
+                        const int64_t at = rows ? feat : tokc + lane;
+                        const float f = at < (rows ? prm.out_feats : prm.ntok) && prm.factors[at] == TINY_FACTOR ? TINY_FACTOR : 1.f;
+                        if (__any_sync(0xffffffffu, f != 1.f)) {
 #pragma unroll
-                        for (int v = 0; v < 8; v++) {
-                            const float4 f = __ldg(fac + v);
-                            r[4 * v] = __float_as_uint(unscale(__uint_as_float(r[4 * v]), row_small, row_large, f.x));
-                            r[4 * v + 1] = __float_as_uint(unscale(__uint_as_float(r[4 * v + 1]), row_small, row_large, f.y));
-                            r[4 * v + 2] = __float_as_uint(unscale(__uint_as_float(r[4 * v + 2]), row_small, row_large, f.z));
-                            r[4 * v + 3] = __float_as_uint(unscale(__uint_as_float(r[4 * v + 3]), row_small, row_large, f.w));
+                            for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * (rows ? f : __shfl_sync(0xffffffffu, f, j)));
                         }
                     }
                     // activation(product + bias), kept as fp32 bits in r.  The activation sits in one warp-uniform branch
@@ -1165,22 +947,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                 uint4 qa[RQ], qb[RQ];
                 const uint32_t acc_addr = lane_base + (uint32_t)(b * TC_ACC_COLS);
                 if constexpr (SPLIT) {
-                    if (TMA_OUT || units > 1) {
+                    if (TMA_OUT || nchunks > 1) {
                         // Promotion: the chunk joins the running sum.  With the last one the accumulator is handed back and the epilogue
                         // works on the registers (TMA_OUT), or the total returns to TMEM for it.
 #pragma unroll
                         for (int i = 0; i < SLICES; i++) {
                             if (i >= nsl) break;
                             tmem_ld32(acc_addr + (uint32_t)((sl0 + i) * 32), ra);
-                            if (c >= nchunks) {  // small values of wide rows: only those rows take them
-                                const int64_t col = (int64_t)tok0 + (sl0 + i) * 32 + lane;
-                                const float f = prm.bias_cols ? (feat_ok ? prm.small[feat] : NOT_WIDE) : col < prm.ntok ? prm.small[col] : NOT_WIDE;
-#pragma unroll
-                                for (int j = 0; j < 32; j++) {
-                                    const float fj = prm.bias_cols ? f : __shfl_sync(0xffffffffu, f, j);
-                                    ra[j] = fj == NOT_WIDE ? 0u : __float_as_uint(__uint_as_float(ra[j]) * fj);
-                                }
-                            }
 #pragma unroll
                             for (int j = 0; j < 32; j++) run[i][j] = c > 0 ? __float_as_uint(__fadd_rn(__uint_as_float(run[i][j]), __uint_as_float(ra[j]))) : ra[j];
                             if (!TMA_OUT && last) tmem_st32(acc_addr + (uint32_t)((sl0 + i) * 32), run[i]);
@@ -1238,112 +1011,26 @@ bool tc_dense_supported(const Geo &geo, int dtype) {
     return expand_smem_bytes(geo, es, false, 1) <= 200 * 1024 && expand_smem_bytes(geo, es, true, 1) <= 200 * 1024;
 }
 
-// Parts of a weight's line in the search for its largest magnitude: enough units to fill the chip, at least a tile each.
-static void split_spans(int64_t groups, int64_t tiles, int *spans, int *per) {
-    int64_t s = (4 * 148 + groups - 1) / groups;
-    if (s > 64) s = 64;
-    if (s > tiles) s = tiles;
-    if (s < 1) s = 1;
-    *per = (int)((tiles + s - 1) / s);
-    *spans = (int)((tiles + *per - 1) / *per);
-}
-// Behind an fp32 operand's planes: its rows' factors, read in whole tiles of columns, then ([lines] of a weight) the parts of the maxima.
-struct LineScales {
-    int spans, per;
-    int64_t lines, rows;  // lines of whole tiles, rows of the operand
-    size_t bytes() const { return factor_bytes(rows) + (size_t)spans * lines * 4; }
-    static size_t factor_bytes(int64_t rows) { return ((size_t)(rows + TC_BN) * 4 + 255) & ~(size_t)255; }
-};
-static LineScales weight_scales(const Geo &geo, bool transposed) {
-    LineScales l;
-    split_spans(transposed ? geo.nc : geo.nb, transposed ? geo.nb : geo.nc, &l.spans, &l.per);
-    l.lines = transposed ? geo.nc * geo.cc : geo.nb * geo.m;
-    l.rows = transposed ? geo.K : geo.M;
-    return l;
-}
-static size_t planes_bytes(int planes, int64_t rows, int64_t red) { return ((size_t)planes * (size_t)rows * (size_t)dense_ld(red) * 2 + 255) & ~(size_t)255; }
+static size_t planes_bytes(int64_t rows, int64_t red) { return ((size_t)SPLIT_PLANES * (size_t)rows * (size_t)dense_ld(red) * 2 + 255) & ~(size_t)255; }
 
 size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed) {
     const int64_t rows = transposed ? geo.K : geo.M, red = transposed ? geo.M : geo.K;
-    // fp32: two planes, in the room that three took: what callers were told to bring is still what they are told
-    if (dtype == NMG_F32) return planes_bytes(3, rows, red) + weight_scales(geo, transposed).bytes() + 512;
-    return (size_t)rows * (size_t)dense_ld(red) * 2 + 512;
+    return (dtype == NMG_F32 ? SPLIT_PLANES : 1) * (size_t)rows * (size_t)dense_ld(red) * 2 + 512;
 }
-size_t tc_split_act_bytes(int64_t tokens, int64_t red, int ranges) {
-    return planes_bytes(ACT_PLANES, tokens, red) + (size_t)2 * ranges * LineScales::factor_bytes(tokens) + 512;
-}
-size_t tc_dense_act_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens) {
-    return dtype == NMG_F32 ? tc_split_act_bytes(tokens, transposed ? geo.M : geo.K, 1) : 0;
-}
+size_t tc_split_act_bytes(int64_t tokens, int64_t red) { return planes_bytes(tokens, red) + (size_t)tokens * 4 + 512; }
 
-// An fp32 activation as planes in `buf`; `units` of the weight's maxima in the same launch.  range: see SplitParams.
-static int split_act(const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, int64_t red, int64_t range, char *buf, const AbsMaxParams &w, int64_t units, size_t smem,
-                     DenseAct *out, cudaStream_t st) {
+int tc_split_act(const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, int64_t red, char *buf, DenseAct *out, cudaStream_t st) {
+    if (tokens > 65535 * 16) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
     SplitParams p{};
     p.src = static_cast<const float *>(act);
-    p.dst = reinterpret_cast<__half *>(buf);
-    p.ld = dense_ld(red);
-    char *scales = buf + planes_bytes(ACT_PLANES, tokens, red);
-    p.factors = reinterpret_cast<float *>(scales);
-    const int64_t ranges = act_k_major ? (red + range - 1) / range : 1;
-    p.small = reinterpret_cast<float *>(scales + ranges * LineScales::factor_bytes(tokens));
-    p.rows = tokens; p.cols = red; p.ld_src = ld_act;
-    p.range = range;
-    p.scale_ld = (int64_t)(LineScales::factor_bytes(tokens) / 4);
-    *out = DenseAct{buf, p.ld, p.factors, p.small, ranges > 1 ? p.scale_ld : 0};
-    if (act_k_major) {
-        const int64_t blocks = ((range < red ? range : red) + 63) / 64, parts = (blocks + COLS_HELD / 64 - 1) / (COLS_HELD / 64);
-        // as many CTAs as fill the chip: with more a cluster's rendezvous costs more than a longer part does (mm 320 x 320 fp32, 7811 columns
-        // 48.5 -> 45.4 us, 2048 x 4096, 1500 columns 111.6 -> 108.4)
-        const int64_t fill = (148 + ranges * ((tokens + 31) / 32) - 1) / (ranges * ((tokens + 31) / 32));
-        int64_t cl = parts < COLS_CLUSTER ? parts : COLS_CLUSTER;
-        if (cl > fill) cl = fill;
-        const int64_t gx = ranges * cl;
-        p.cluster = (int)cl;
-        p.per = (int)((blocks + cl - 1) / cl * 64);
-        p.ctas = (tokens + 31) / 32;
-        int64_t gy = p.ctas + (units + gx - 1) / gx;
-        if (gy > 65535) gy = 65535;
-        if (tokens > 65535 * 16) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)gx, (unsigned)gy);
-        cfg.blockDim = dim3(COLS_THREADS);
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = st;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        attr[1].id = cudaLaunchAttributeClusterDimension;
-        attr[1].val.clusterDim.x = (unsigned)cl;
-        attr[1].val.clusterDim.y = 1;
-        attr[1].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = cl > 1 ? 2 : 1;
-        const bool rest = units > 0 || p.per > COLS_HELD;
-        if (rest) NMG_ALLOW_SMEM(smem, split_columns_kernel<true, true>);
-        NMG_CUDA(cudaLaunchKernelEx(&cfg, rest ? split_columns_kernel<true, true> : cl > 1 ? split_columns_kernel<true, false> : split_columns_kernel<false, false>, p, w));
-        return NMG_OK;
-    }
-    p.ctas = p.ld <= 1024 ? (tokens + 3) / 4 : tokens;
-    if (tokens > 65535 * 16 || p.ctas + units > 0x7fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many tokens for the split pre-pass");
-    const bool rest = units > 0 || p.ld > 4096;
-    return launch_early(p.ld <= 1024 ? (rest ? split_rows_kernel<4, true> : split_rows_kernel<4, false>) : rest ? split_rows_kernel<1, true> : split_rows_kernel<1, false>,
-                        (unsigned)(p.ctas + units), PREP_THREADS, smem, st, p, w);
-}
-int tc_split_act(const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, int64_t red, int64_t range, char *buf, DenseAct *out, cudaStream_t st) {
-    return split_act(act, ld_act, act_k_major, tokens, red, range, buf, AbsMaxParams{}, 0, 0, out, st);
-}
-// The same with the maxima of the weight's lines.
-static int split_operands(const Geo &geo, bool transposed, const void *val, const int16_t *idx, const void *act, int64_t ld_act, bool act_k_major, int64_t tokens,
-                          char *buf, uint32_t *weight_maxima, DenseAct *out, cudaStream_t st) {
-    int rc;
-    PatternTable tab;
-    if ((rc = get_pattern_table(geo.n, geo.m, &tab))) return rc;
-    const LineScales ws = weight_scales(geo, transposed);
-    const AbsMaxParams w{static_cast<const float *>(val), idx, tab.order, weight_maxima, geo.nb, geo.nc, ws.lines, geo.n, geo.m, geo.g, geo.cc, transposed ? 1 : 0, ws.spans, ws.per};
-    const int64_t red = transposed ? geo.M : geo.K;
-    return split_act(act, ld_act, act_k_major, tokens, red, round_up(red, 64), buf, w, (transposed ? geo.nc : geo.nb) * ws.spans,
-                                   (size_t)(transposed ? geo.cc : geo.m) * 4, out, st);
+    p.dst = reinterpret_cast<__nv_bfloat16 *>(buf);
+    p.factors = reinterpret_cast<float *>(buf + planes_bytes(tokens, red));
+    p.rows = tokens; p.cols = red; p.ld_src = ld_act; p.ld = dense_ld(red);
+    *out = DenseAct{buf, p.ld, p.factors};
+    if (act_k_major)
+        return launch_early(split_columns_kernel, dim3((unsigned)((p.ld + COLS_RED - 1) / COLS_RED), (unsigned)((tokens + 31) / 32)), COLS_THREADS, 0, st, p);
+    if (p.ld <= 1024) return launch_early(split_rows_kernel<4>, (unsigned)((tokens + 3) / 4), SPLIT_THREADS, 0, st, p);
+    return launch_early(split_rows_kernel<1>, (unsigned)tokens, SPLIT_THREADS, 0, st, p);
 }
 
 template <typename T, bool TR, int N_, bool PLAIN> static int expand_launch_n(const ExpandParams &p, size_t smem, int64_t items, cudaStream_t st) {
@@ -1443,42 +1130,32 @@ static GemmTiles gemm_tiles(int64_t tiles_f, int64_t cols, int64_t units, bool f
     return best;
 }
 // (val, idx) -> the weight with its zeros restored, rows `ld` elements apart at `dst` (16-byte aligned, ld a multiple of 8).
-// plain = false: the matmul's operand, 16-bit or two fp16 planes for fp32; plain = true: the
+// plain = false: the matmul's operand, 16-bit or three bf16 planes for fp32; plain = true: the
 // weight in its own dtype (the densifier), where full stores must not run past the row: K a multiple of 8, or the rows kernel.
-// An fp32 operand's factors and maxima follow its planes (LineScales).
 static int expand_to(const Geo &geo, int dtype, bool transposed, bool plain, const void *val, const int16_t *idx, void *dst, int64_t ld,
                      cudaStream_t st) {
-    const bool scaled = dtype == NMG_F32 && !plain;
+    const int64_t rows = transposed ? geo.K : geo.M;
     const size_t es = dtype == NMG_F32 ? 4 : 2;
     int rc;
     PatternTable tab;
     if ((rc = get_pattern_table(geo.n, geo.m, &tab))) return rc;
     ExpandParams ep{};
     ep.val = val; ep.idx = idx; ep.order = tab.order; ep.dst = dst;
-    ep.ld = ld;
-    if (scaled) {
-        const LineScales sc = weight_scales(geo, transposed);
-        char *scales = static_cast<char *>(dst) + planes_bytes(SPLIT_PLANES, sc.rows, transposed ? geo.M : geo.K);
-        ep.plane_elems = sc.rows * ld;
-        ep.factors = reinterpret_cast<float *>(scales);
-        ep.maxima = reinterpret_cast<const uint32_t *>(scales + LineScales::factor_bytes(sc.rows));
-        ep.spans = sc.spans; ep.lines = sc.lines;
-    }
+    ep.ld = ld; ep.plane_elems = rows * ld;
     ep.vec = geo.K % 8 == 0 && ld % 8 == 0 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
     ep.M = geo.M; ep.K = geo.K; ep.nb = geo.nb; ep.nc = geo.nc;
     ep.n = geo.n; ep.m = geo.m; ep.g = geo.g; ep.C = geo.C; ep.cc = geo.cc;
     size_t rsmem = 0;
     const bool aligned = ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0;
-    if (!transposed && aligned && expand_rows_plan(geo, es, scaled, &ep.R, &ep.Q, &rsmem)) {
+    if (!transposed && aligned && expand_rows_plan(geo, es, &ep.R, &ep.Q, &rsmem)) {
         if (dtype == NMG_F16) return plain ? expand_rows_launch<__half, true>(ep, rsmem, st) : expand_rows_launch<__half, false>(ep, rsmem, st);
         if (dtype == NMG_BF16) return plain ? expand_rows_launch<__nv_bfloat16, true>(ep, rsmem, st) : expand_rows_launch<__nv_bfloat16, false>(ep, rsmem, st);
         return plain ? expand_rows_launch<float, true>(ep, rsmem, st) : expand_rows_launch<float, false>(ep, rsmem, st);
     }
     ep.R = expand_rows_per_item(geo, es, transposed);
     ep.pitch = expand_pitch(geo, transposed, ep.R);
-    size_t esmem = expand_smem_bytes(geo, es, transposed, ep.R);
+    const size_t esmem = expand_smem_bytes(geo, es, transposed, ep.R);
     if (esmem > 200 * 1024) NMG_FAIL(NMG_ERR_UNSUPPORTED, "chunk of %d columns does not fit the expansion pass", geo.cc);
-    esmem += scaled ? (size_t)(transposed ? geo.cc : ep.R * geo.m) * 4 : 0;
     const int64_t items = ((geo.nb + ep.R - 1) / ep.R) * geo.nc;
     if (dtype == NMG_F16) return transposed ? expand_launch<__half, true>(ep, esmem, items, st) : expand_launch<__half, false>(ep, esmem, items, st);
     if (dtype == NMG_BF16) return transposed ? expand_launch<__nv_bfloat16, true>(ep, esmem, items, st) : expand_launch<__nv_bfloat16, false>(ep, esmem, items, st);
@@ -1496,7 +1173,7 @@ bool tc_expand_plain_supported(const Geo &geo, int dtype, const void *val, const
     const size_t es = dtype == NMG_F32 ? 4 : 2;
     int R, Q;
     size_t smem;
-    if (geo.C <= 65535 && ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0 && expand_rows_plan(geo, es, false, &R, &Q, &smem)) return true;
+    if (geo.C <= 65535 && ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0 && expand_rows_plan(geo, es, &R, &Q, &smem)) return true;
     if (geo.cc > 32767 || geo.C > 65535 || geo.K % 8 != 0 || ld % 8 != 0 || (reinterpret_cast<uintptr_t>(dense) & 15) != 0) return false;
     return expand_smem_bytes(geo, es, false, expand_rows_per_item(geo, es, false)) <= 200 * 1024;
 }
@@ -1504,7 +1181,7 @@ int tc_expand_plain(const Geo &geo, int dtype, const void *val, const int16_t *i
     return expand_to(geo, dtype, false, true, val, idx, dense, ld, st);
 }
 
-// out = dense[rows][round_up(red, 8)] (16-bit, or the two fp16 planes of an fp32 weight and its factors) x activations (16-bit, or the planes of the split).
+// out = dense[rows][round_up(red, 8)] (16-bit, or the three bf16 planes of an fp32 weight) x activations (16-bit, or the planes of the split).
 // CTA pairs (256 rows per tile) unless a 16-bit output has one tile of 128 features only.  source: expand this weight into `dense`
 // first, right before the matmul, whose prologue overlaps the expansion's end only when nothing is queued between the two.
 int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const DenseAct &act, int64_t tokens, const void *bias,
@@ -1514,8 +1191,7 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
     const int planes = dtype == NMG_F32 ? SPLIT_PLANES : 1;
     int rc;
     GemmMaps maps;
-    const int edt = dtype == NMG_F32 ? NMG_F16 : dtype;
-    const float *w_factors = reinterpret_cast<const float *>(dense + planes_bytes(SPLIT_PLANES, rows, red));
+    const int edt = dtype == NMG_F32 ? NMG_BF16 : dtype;
     const size_t osz = dtype == NMG_F32 ? 4 : 2;
     const bool pair = dtype == NMG_F32 || rows > TC_BM;
     // Token-major output of a CTA-pair product: exchange the operands' roles.  The activations become the row operand (tokens
@@ -1530,7 +1206,7 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
     const int64_t tiles_f = (row_ext + tile_feats - 1) / tile_feats;
     if (tiles_f * ((col_ext + 63) / 64) > 0x3fffffff) NMG_FAIL(NMG_ERR_UNSUPPORTED, "too many output tiles for one launch");
     const GemmTiles tiles = gemm_tiles(tiles_f, col_ext, units, dtype == NMG_F32, pair);
-    const uint64_t act_rows = (uint64_t)tokens * (dtype == NMG_F32 ? ACT_PLANES : 1), w_rows = (uint64_t)rows * planes;
+    const uint64_t act_rows = (uint64_t)tokens * planes, w_rows = (uint64_t)rows * planes;
     const uint32_t col_box = (uint32_t)(pair ? tiles.bn / 2 : tiles.bn);
     if ((rc = encode_tmap_2d(swap ? &maps.b : &maps.a, edt, dense, (uint64_t)red, w_rows, (uint64_t)ld, TC_BK, swap ? col_box : TC_BM, 1))) return rc;
     if ((rc = encode_tmap_2d(swap ? &maps.a : &maps.b, edt, act.base, (uint64_t)red, act_rows, (uint64_t)act.ld, TC_BK, swap ? TC_BM : col_box, 1))) return rc;
@@ -1548,8 +1224,10 @@ int tc_dense_gemm(int64_t rows, int64_t red, int dtype, const char *dense, const
     gp.bias = bias;
     gp.n_out = n_outs;
     gp.bias_cols = swap ? 1 : 0;
-    gp.fac_rows = swap ? act.factors : w_factors; gp.fac_cols = swap ? w_factors : act.factors;
-    gp.small = act.small;
+    gp.factors = act.factors;
+    // fp32: the drain warps keep up with short chunks, which leave fewer truncating additions in a row (tc_common).  3072 <- 768, 4096 tokens,
+    // chunks of 4 / 2 / 1 k-blocks: 81.8 / 84.1 / 88.8 us and a relative error of 1.33e-6 / 5.4e-7 / 0.9e-7; up to 512 elements: within 1 %.
+    gp.chunk_kb = red <= 8 * TC_BK ? 1 : 2;
     gp.a_rows = (int)row_ext; gp.b_rows = (int)col_ext;
     bool vec = !out_token_major && (ld_out * osz) % 16 == 0;
     for (int d = 0; d < n_outs; d++) {
@@ -1593,16 +1271,13 @@ int tc_dense_matmul(const Geo &geo, int dtype, bool transposed, const void *val,
                     int64_t tokens, const void *bias, void *const *outs, int n_outs, void *mc_out, int64_t ld_out, int out_token_major,
                     void *ws, size_t ws_bytes, cudaStream_t st, const Epilogue &epi) {
     const int64_t rows = transposed ? geo.K : geo.M, red = transposed ? geo.M : geo.K;
-    const size_t act_need = tc_dense_act_bytes(geo, dtype, transposed, tokens), need = act_need + tc_dense_workspace_bytes(geo, dtype, transposed);
+    const size_t act_need = dtype == NMG_F32 ? tc_split_act_bytes(tokens, red) : 0, need = act_need + tc_dense_workspace_bytes(geo, dtype, transposed);
     if (!ws || ws_bytes < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the expanded weight, got %zu", need, ws_bytes);
     char *act_buf = reinterpret_cast<char *>(((uintptr_t)ws + 255) & ~(uintptr_t)255);
     char *dense = reinterpret_cast<char *>(((uintptr_t)ws + act_need + 255) & ~(uintptr_t)255);
-    DenseAct planes{act, ld_act, nullptr, nullptr, 0};
+    DenseAct planes{act, ld_act, nullptr};
     int rc;
-    if (dtype == NMG_F32) {
-        char *maxima = dense + planes_bytes(SPLIT_PLANES, rows, red) + LineScales::factor_bytes(rows);
-        if ((rc = split_operands(geo, transposed, val, idx, act, ld_act, act_k_major, tokens, act_buf, reinterpret_cast<uint32_t *>(maxima), &planes, st))) return rc;
-    }
+    if (dtype == NMG_F32 && (rc = tc_split_act(act, ld_act, act_k_major, tokens, red, act_buf, &planes, st))) return rc;
     const DenseSource source{geo, transposed, val, idx};
     return tc_dense_gemm(rows, red, dtype, dense, planes, tokens, bias, outs, n_outs, mc_out, ld_out, out_token_major, st, epi, &source);
 }

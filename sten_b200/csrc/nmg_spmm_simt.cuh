@@ -20,15 +20,12 @@ int launch_widen_to_f32(const void *src, int dtype, int64_t rows, int64_t cols, 
 
 // Column-order ("natural") copy of a weight: for every row-block mb and column k of the padded width Kp,
 // pat[mb][k] = pattern of that column (id * m in one byte for the specialised patterns, else a 16-bit id), nval[mb][k][s] = its n kept values.
-struct NaturalLayout { size_t pat_bytes, val_bytes, mask_bytes, plane_bytes, fine_bytes, max_bytes, total; };
+struct NaturalLayout { size_t pat_bytes, val_bytes, mask_bytes, plane_bytes, total; };
 NaturalLayout natural_layout(const Geo &geo, int dtype);
 int64_t natural_width(const Geo &geo);
 int64_t natural_mask_rows(const Geo &geo);  // rows of the row masks: M rounded up to the tensor-core tile
 size_t natural_bytes(const Geo &geo, int dtype, size_t *pat_bytes_out);
-// Which parts of the copy behind patterns and values to build: all of them (a copy that is kept), or those that one call reads.
-// PLANES and FINE (either brings the row masks): the forward product; COLUMNS: the transposed one.
-enum { NATURAL_PLANES = 1, NATURAL_FINE = 2, NATURAL_COLUMNS = 4, NATURAL_ALL = 7 };
-int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16_t *idx, void *pat, void *nval, cudaStream_t st, int parts = NATURAL_ALL);
+int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16_t *idx, void *pat, void *nval, cudaStream_t st);
 
 // SIMT kernels (fp32 accumulate).  xt is the activation as [K][ld_xt] fp32 (tokens contiguous).
 size_t simt_fwd_workspace_bytes(const Geo &geo, int64_t tokens, int dtype, int layout);
@@ -41,7 +38,7 @@ int simt_bwd(const Geo &geo, int dtype, const void *pat, const void *nval, const
              int64_t tokens, void *dx, int64_t ld_dx, void *ws, size_t ws_bytes, cudaStream_t st);
 
 // Tensor-core kernels.  act: [tokens][ld_act] with the reduction axis contiguous.  fp32 operands are multiplied as
-// sums of 16-bit pieces and need `ws` (tc_split_workspace_bytes, tc_dense_act_bytes) for the split activation.  Two variants share the
+// sums of 16-bit pieces and need `ws` (tc_split_act_bytes) for the split activation.  Two variants share the
 // entry point tc_matmul: the fused kernel (nmg_spmm_tc.cu) expands the column-ordered copy (pat / nval) tile by tile
 // inside the matmul; the two-pass variant (nmg_gemm_tc.cu, `dense` = true) first expands (val, idx) into a dense 16-bit
 // matrix in `ws` (tc_dense_workspace_bytes, after the split activation) and multiplies that.  tc_use_dense is the
@@ -55,21 +52,18 @@ struct Epilogue {
     bool any() const { return act != NMG_EPI_NONE || residual != nullptr; }
 };
 int launch_epilogue(int dtype, void *out, int64_t rows, int64_t cols, int64_t ld_out, const Epilogue &epi, cudaStream_t st);
-// Activations of the two-pass variant: [tokens][ld], reduction contiguous, 16-byte aligned rows; for fp32 the planes and factors of its rows (see nmg_tc_common.cuh).
+// Activations of the two-pass variant: [tokens][ld], reduction contiguous, 16-byte aligned rows; for fp32 the planes and the factors of its rows (see nmg_tc_common.cuh).
 struct DenseSource { const Geo &geo; bool transposed; const void *val; const int16_t *idx; };  // the compressed weight
-struct DenseAct { const void *base; int64_t ld; const float *factors, *small; int64_t scale_ld; };  // scale_ld: between ranges of the reduction axis, 0 for one
+struct DenseAct { const void *base; int64_t ld; const float *factors; };
 
 bool tc_supported(const Geo &geo, int dtype);        // fused kernel
 bool tc_dense_supported(const Geo &geo, int dtype);  // two-pass variant
-int tc_natural_parts(bool transposed, bool act_k_major, int64_t tokens);  // of the copy, that the fused kernel reads
 bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens, bool have_packed);
-size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, bool act_k_major, int64_t tokens);
-size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed);               // two-pass variant: the expanded weight,
-// An fp32 activation [tokens][red] (k_major: [red][ld]) as fp16 planes of its rows (see nmg_tc_common.cuh) in `buf`, 256-byte aligned.
-// K-major rows have their factors by ranges of `range` reduction elements (a multiple of 64; `ranges` of them).
-size_t tc_split_act_bytes(int64_t tokens, int64_t red, int ranges);
-int tc_split_act(const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, int64_t red, int64_t range, char *buf, DenseAct *out, cudaStream_t st);
-size_t tc_dense_act_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens);     // and before it the planes of an fp32 activation
+size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens);
+size_t tc_dense_workspace_bytes(const Geo &geo, int dtype, bool transposed);
+// An fp32 activation [tokens][red] (k_major: [red][ld]) as planes and factors of its rows (see nmg_tc_common.cuh) in `buf`, 256-byte aligned.
+size_t tc_split_act_bytes(int64_t tokens, int64_t red);
+int tc_split_act(const void *act, int64_t ld_act, bool act_k_major, int64_t tokens, int64_t red, char *buf, DenseAct *out, cudaStream_t st);
 // outs / n_outs: the result goes to every listed buffer (same shape and pitch); more than one needs `dense`.  mc_out, when
 // not NULL, is an NVSwitch multicast address that maps onto all of them: full 16-byte chunks are then stored once.
 // alone: nothing else was launched for this call.

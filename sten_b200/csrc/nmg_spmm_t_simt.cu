@@ -18,86 +18,12 @@ namespace nmg {
 // ------------------------------------------------------------------------------------------ column-ordered copy
 struct NaturalParams {
     const void *val; const int16_t *idx; void *pat; void *nval;
-    __half *planes;         // fp32 weights the tensor-core kernel serves: two fp16 planes of scaled values, else NULL,
-    __nv_bfloat16 *fine;    // and three bf16 planes of the values
-    uint32_t *row_max, *col_max;  // and the largest magnitudes of the weight's rows and columns, as bits
-    const int8_t *order;          // [C][n]
-    int patterns;                 // C
-    int parts;                    // of an fp32 copy: NATURAL_...
+    __nv_bfloat16 *planes;  // fp32 weights the tensor-core kernel serves: three bf16 planes, else NULL
     int64_t nb, nc, Kp;
     int n, m, g, cc;
     int wide;    // 16-bit pattern ids
     int planar;  // n = 2: neighbouring columns' first values, then their second values
 };
-// Scale of the value in slot s of a column with the given pattern
-__device__ __forceinline__ float natural_scale(const NaturalParams &prm, int64_t mb, int pattern, int s) {
-    return pow2(-line_exp(prm.row_max[mb * prm.m + prm.order[pattern * prm.n + s]]));
-}
-__device__ __forceinline__ void natural_split(float x, __half &h, __half &l) {  // a scaled value
-    h = __float2half_rn(x);
-    l = __float2half_rn(x - __half2float(h));
-}
-__device__ __forceinline__ void natural_split3(float x, __nv_bfloat16 &hi, __nv_bfloat16 &mid, __nv_bfloat16 &lo) {
-    hi = __float2bfloat16_rn(x);
-    const float r = x - __bfloat162float(hi);
-    mid = __float2bfloat16_rn(r);
-    lo = __float2bfloat16_rn(r - __bfloat162float(mid));
-}
-// Largest magnitudes of rows and columns: an item is NATURAL_MAX_ROWS row-blocks of one chunk, whose maxima meet in shared memory (DIRECT:
-// chunks too wide for that).  EIGHT: eight slots of one pattern per thread, in 16-byte loads.
-constexpr int NATURAL_MAX_ROWS = 32;
-template <bool DIRECT, bool EIGHT, int N_> __global__ void __launch_bounds__(256) natural_max_kernel(const NaturalParams prm) {
-    extern __shared__ uint32_t mx[];  // [rows of the item], [cc]
-    constexpr int P = EIGHT ? 8 : 1;
-    const int cc = prm.cc, rows = NATURAL_MAX_ROWS * prm.m;
-    const int64_t groups = (prm.nb + NATURAL_MAX_ROWS - 1) / NATURAL_MAX_ROWS;
-    const float *val = static_cast<const float *>(prm.val);
-    for (int64_t item = blockIdx.x; item < groups * prm.nc; item += gridDim.x) {
-        const int64_t kc = item / groups, mb0 = (item - kc * groups) * NATURAL_MAX_ROWS;
-        const int count = (int)(prm.nb - mb0 < NATURAL_MAX_ROWS ? prm.nb - mb0 : NATURAL_MAX_ROWS);
-        uint32_t *rmax = DIRECT ? prm.row_max + mb0 * prm.m : mx, *cmax = DIRECT ? prm.col_max + kc * cc : mx + rows;
-        if (!DIRECT) {
-            __syncthreads();
-            for (int i = threadIdx.x; i < rows + cc; i += blockDim.x) mx[i] = 0;
-            __syncthreads();
-        }
-        for (int64_t e = (int64_t)threadIdx.x * P; e < (int64_t)count * cc; e += (int64_t)blockDim.x * P) {
-            const int j = (int)(e / cc), slot = (int)(e - (int64_t)j * cc);
-            const int64_t o = (kc * prm.nb + mb0) * cc + e;
-            __align__(16) int16_t c[8];
-            if (EIGHT) *reinterpret_cast<uint4 *>(c) = __ldg(reinterpret_cast<const uint4 *>(prm.idx + o));
-            else c[0] = prm.idx[o];
-            __align__(16) float v[P * N_];
-            if (EIGHT) {
-#pragma unroll
-                for (int i = 0; i < 2 * N_; i++) reinterpret_cast<float4 *>(v)[i] = __ldg(reinterpret_cast<const float4 *>(val + o * N_) + i);
-            } else {
-                for (int s = 0; s < N_; s++) v[s] = __ldg(val + o * N_ + s);
-            }
-            uint32_t of_row[N_] = {};
-#pragma unroll
-            for (int u = 0; u < P; u++) {
-                if ((unsigned)c[u] >= (unsigned)cc) continue;
-                uint32_t all = 0;
-#pragma unroll
-                for (int s = 0; s < N_; s++) {
-                    const uint32_t bits = __float_as_uint(v[u * N_ + s]) & 0x7fffffffu;
-                    of_row[s] = max(of_row[s], bits);
-                    all = max(all, bits);
-                }
-                if (prm.parts & NATURAL_COLUMNS) atomicMax(cmax + c[u], all);
-            }
-#pragma unroll
-            for (int s = 0; s < N_; s++) atomicMax(rmax + j * prm.m + prm.order[slot / prm.g * N_ + s], of_row[s]);
-        }
-        if (!DIRECT) {
-            __syncthreads();
-            for (int i = threadIdx.x; i < count * prm.m; i += blockDim.x) atomicMax(prm.row_max + mb0 * prm.m + i, rmax[i]);
-            for (int i = threadIdx.x; i < cc; i += blockDim.x) atomicMax(prm.col_max + kc * cc + i, cmax[i]);
-        }
-    }
-}
-
 // One thread per stored column slot.  SMALL: fewer than 2^31 slots, 32-bit index arithmetic.
 template <typename T, bool SMALL>
 __global__ void build_natural_kernel(const NaturalParams prm) {
@@ -118,10 +44,11 @@ __global__ void build_natural_kernel(const NaturalParams prm) {
             const int64_t d = prm.planar ? (o & ~(int64_t)1) * 2 + s * 2 + (o & 1) : o * prm.n + s;
             const T v = val[(int64_t)e * prm.n + s];
             nval[d] = v;
-            if (sizeof(T) == 4 && prm.planes) {
+            if (sizeof(T) == 4 && prm.planes) {  // exact three-way split
                 const int64_t plane = prm.nb * prm.Kp * prm.n;
-                if (prm.parts & NATURAL_PLANES) natural_split(DT<T>::to_f32(v) * natural_scale(prm, mb, slot / prm.g, s), prm.planes[d], prm.planes[plane + d]);
-                if (prm.parts & NATURAL_FINE) natural_split3(DT<T>::to_f32(v), prm.fine[d], prm.fine[plane + d], prm.fine[2 * plane + d]);
+                __nv_bfloat16 w[3];
+                split3(DT<T>::to_f32(v), w);
+                for (int t = 0; t < 3; t++) prm.planes[t * plane + d] = w[t];
             }
         }
     }
@@ -139,7 +66,6 @@ __global__ void __launch_bounds__(NATURAL_THREADS) build_natural_rows_kernel(con
     const int R = it.R, Q = it.Q, cc = prm.cc, cols = Q * cc, tid = (int)threadIdx.x;
     T *vals = reinterpret_cast<T *>(smem);                               // [R][cols * N_]
     uint8_t *pats = reinterpret_cast<uint8_t *>(vals + R * cols * N_);  // [R][cols]
-    float *scales = reinterpret_cast<float *>(pats + R * cols);          // [R][C][n] with planes: by row-block, pattern and slot
     for (int i = tid; i < R * cols * N_ / V; i += NATURAL_THREADS) reinterpret_cast<uint4 *>(vals)[i] = make_uint4(0, 0, 0, 0);
     for (int i = tid; i < R * cols / 8; i += NATURAL_THREADS) reinterpret_cast<uint2 *>(pats)[i] = make_uint2(0, 0);
     const int per_chunk = R * cc / 8, q = tid / per_chunk, e8 = (tid - q * per_chunk) * 8, j = e8 / cc, slot0 = e8 - j * cc;
@@ -151,11 +77,6 @@ __global__ void __launch_bounds__(NATURAL_THREADS) build_natural_rows_kernel(con
         const int span = (int)(item / it.groups), grp = (int)(item - (int64_t)span * it.groups);
         __syncthreads();  // the buffers are zeros
         const int64_t mb0 = (int64_t)grp * R;
-        if (sizeof(T) == 4 && prm.planes && (prm.parts & NATURAL_PLANES))
-            for (int i = tid; i < R * prm.patterns * N_; i += NATURAL_THREADS) {
-                const int l = i / (prm.patterns * N_), ps = i - l * prm.patterns * N_;
-                scales[i] = mb0 + l < prm.nb ? pow2(-line_exp(prm.row_max[(mb0 + l) * prm.m + prm.order[ps]])) : 1.f;
-            }
         if (has && span * Q + q < prm.nc && mb0 + j < prm.nb) {
             const int64_t e = ((int64_t)(span * Q + q) * prm.nb + mb0 + j) * cc + slot0;
             const uint4 iv = __ldg(reinterpret_cast<const uint4 *>(prm.idx + e));
@@ -189,27 +110,15 @@ __global__ void __launch_bounds__(NATURAL_THREADS) build_natural_rows_kernel(con
                 *reinterpret_cast<uint2 *>(static_cast<uint8_t *>(prm.pat) + o) = *reinterpret_cast<const uint2 *>(pats + i * 8);
 #pragma unroll
                 for (int u = 0; u < VL; u++) reinterpret_cast<uint4 *>(nval + o * N_)[u] = reinterpret_cast<const uint4 *>(vals + i * 8 * N_)[u];
-                if (sizeof(T) == 4 && prm.planes) {
+                if (sizeof(T) == 4 && prm.planes) {  // exact three-way split
 #pragma unroll
                     for (int u = 0; u < N_; u++) {
-                        if (prm.parts & NATURAL_PLANES) {
-                            __align__(16) __half w[2][8];
+                        __align__(16) uint32_t w[3][4];
 #pragma unroll
-                            for (int k = 0; k < 8; k++) {
-                                const int at = u * 8 + k;  // n = 2: two columns' first values, then their second values
-                                const int col = N_ == 1 ? at : (at >> 2) * 2 + (at & 1), s = N_ == 1 ? 0 : (at >> 1) & 1;
-                                natural_split(DT<T>::to_f32(vals[i * N_ * 8 + at]) * scales[(l * prm.patterns + pats[i * 8 + col] / prm.m) * N_ + s], w[0][k], w[1][k]);
-                            }
+                        for (int k = 0; k < 4; k++)
+                            split3_pair(DT<T>::to_f32(vals[(i * N_ + u) * 8 + 2 * k]), DT<T>::to_f32(vals[(i * N_ + u) * 8 + 2 * k + 1]), w[0][k], w[1][k], w[2][k]);
 #pragma unroll
-                            for (int t = 0; t < 2; t++) *reinterpret_cast<uint4 *>(prm.planes + t * plane + o * N_ + u * 8) = *reinterpret_cast<const uint4 *>(w[t]);
-                        }
-                        if (prm.parts & NATURAL_FINE) {
-                            __align__(16) __nv_bfloat16 f[3][8];
-#pragma unroll
-                            for (int k = 0; k < 8; k++) natural_split3(DT<T>::to_f32(vals[i * N_ * 8 + u * 8 + k]), f[0][k], f[1][k], f[2][k]);
-#pragma unroll
-                            for (int t = 0; t < 3; t++) *reinterpret_cast<uint4 *>(prm.fine + t * plane + o * N_ + u * 8) = *reinterpret_cast<const uint4 *>(f[t]);
-                        }
+                        for (int t = 0; t < 3; t++) *reinterpret_cast<uint4 *>(prm.planes + t * plane + o * N_ + u * 8) = *reinterpret_cast<const uint4 *>(w[t]);
                     }
                 }
             }
@@ -266,9 +175,8 @@ static bool bwd_specialised(int n, int m) {
 int64_t natural_width(const Geo &geo) { return round_up(geo.nc * geo.cc, 128); }
 
 // Sections of the copy: one pattern entry per column, the values in the weight's dtype and, where the tensor-core kernel
-// serves the pattern, the row masks and an fp32 weight's values as two fp16 planes of scaled rows and as three bf16 planes (the product
-// of a few K-major columns; split in the kernel, every one of a block's m rows would repeat the conversions), and the largest
-// magnitudes of rows and columns.  The patterns with specialised
+// serves the pattern, the row masks and an fp32 weight's values split into three bf16 planes (split in the kernel, every one
+// of a block's m rows would repeat the conversions: 4096 x 4096 2:4, 256 tokens 132 us).  The patterns with specialised
 // kernels (at most 28) store one byte, pattern id times m: the offset of the pattern's row selectors in the expansion table of
 // the tensor-core kernel; with n = 2 their values are stored pair-wise planar.  All others store 16-bit ids.
 NaturalLayout natural_layout(const Geo &geo, int dtype) {
@@ -277,10 +185,8 @@ NaturalLayout natural_layout(const Geo &geo, int dtype) {
     l.pat_bytes = (entries * (bwd_specialised(geo.n, geo.m) ? 1 : 2) + 255) & ~(size_t)255;
     l.val_bytes = (entries * geo.n * dtype_size(dtype) + 255) & ~(size_t)255;
     l.mask_bytes = tc_supported(geo, dtype) ? (size_t)(natural_width(geo) / 64) * (size_t)natural_mask_rows(geo) * 8 * geo.n : 0;
-    l.plane_bytes = (dtype == NMG_F32 && tc_supported(geo, dtype)) ? (2 * entries * geo.n * 2 + 255) & ~(size_t)255 : 0;
-    l.fine_bytes = l.plane_bytes ? (3 * entries * geo.n * 2 + 255) & ~(size_t)255 : 0;
-    l.max_bytes = l.plane_bytes ? ((size_t)(natural_mask_rows(geo) + natural_width(geo)) * 4 + 255) & ~(size_t)255 : 0;
-    l.total = l.pat_bytes + l.val_bytes + l.mask_bytes + l.plane_bytes + l.fine_bytes + l.max_bytes;
+    l.plane_bytes = (dtype == NMG_F32 && tc_supported(geo, dtype)) ? (3 * entries * geo.n * 2 + 255) & ~(size_t)255 : 0;
+    l.total = l.pat_bytes + l.val_bytes + l.mask_bytes + l.plane_bytes;
     return l;
 }
 int64_t natural_mask_rows(const Geo &geo) { return round_up(geo.M, 128); }
@@ -291,37 +197,16 @@ size_t natural_bytes(const Geo &geo, int dtype, size_t *pat_bytes_out) {
     return l.total;
 }
 
-int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16_t *idx, void *pat, void *nval, cudaStream_t st, int parts) {
+int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16_t *idx, void *pat, void *nval, cudaStream_t st) {
     const NaturalLayout lay = natural_layout(geo, dtype);
-    NaturalParams p{val, idx, pat, nval, nullptr, nullptr, nullptr, nullptr, nullptr, geo.C, parts, geo.nb, geo.nc, natural_width(geo), geo.n, geo.m, geo.g, geo.cc, bwd_specialised(geo.n, geo.m) ? 0 : 1,
+    NaturalParams p{val, idx, pat, nval, nullptr, geo.nb, geo.nc, natural_width(geo), geo.n, geo.m, geo.g, geo.cc, bwd_specialised(geo.n, geo.m) ? 0 : 1,
                     bwd_specialised(geo.n, geo.m) && geo.n == 2 ? 1 : 0};
     const int64_t total = geo.nb * geo.nc * geo.cc;
     int64_t blocks = (total + 255) / 256;
     if (blocks > 148 * 64) blocks = 148 * 64;
     const bool rows_kernel = bwd_specialised(geo.n, geo.m) && geo.n <= 2 && geo.cc % 8 == 0 && geo.cc <= 8 * NATURAL_THREADS &&
                              ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0;
-    if (lay.plane_bytes) {
-        PatternTable tab;
-        if (const int rc = get_pattern_table(geo.n, geo.m, &tab)) return rc;
-        char *planes = static_cast<char *>(nval) + lay.val_bytes + lay.mask_bytes;
-        p.planes = reinterpret_cast<__half *>(planes);
-        p.fine = reinterpret_cast<__nv_bfloat16 *>(planes + lay.plane_bytes);
-        p.row_max = reinterpret_cast<uint32_t *>(planes + lay.plane_bytes + lay.fine_bytes);
-        p.col_max = p.row_max + natural_mask_rows(geo);
-        p.order = tab.order;
-    }
-    if (lay.plane_bytes && (parts & (NATURAL_PLANES | NATURAL_COLUMNS))) {
-        NMG_CUDA(cudaMemsetAsync(p.row_max, 0, lay.max_bytes, st));
-        const int64_t items = (geo.nb + NATURAL_MAX_ROWS - 1) / NATURAL_MAX_ROWS * geo.nc;
-        const unsigned grid = (unsigned)(items < 148 * 16 ? items : 148 * 16);
-        const size_t smem = (size_t)(NATURAL_MAX_ROWS * geo.m + geo.cc) * 4;
-        const bool eight = geo.g % 8 == 0 && ((reinterpret_cast<uintptr_t>(val) | reinterpret_cast<uintptr_t>(idx)) & 15) == 0;
-        auto kernel = smem > 48 * 1024 ? (geo.n == 1 ? natural_max_kernel<true, false, 1> : natural_max_kernel<true, false, 2>)
-                      : eight          ? (geo.n == 1 ? natural_max_kernel<false, true, 1> : natural_max_kernel<false, true, 2>)
-                                       : (geo.n == 1 ? natural_max_kernel<false, false, 1> : natural_max_kernel<false, false, 2>);
-        kernel<<<grid, 256, smem > 48 * 1024 ? 0 : smem, st>>>(p);
-        NMG_CUDA(cudaGetLastError());
-    }
+    if (lay.plane_bytes) p.planes = reinterpret_cast<__nv_bfloat16 *>(static_cast<char *>(nval) + lay.val_bytes + lay.mask_bytes);
     if (rows_kernel) {
         NaturalRows it;
         it.Q = 512 / geo.cc < 1 ? 1 : 512 / geo.cc;
@@ -331,7 +216,7 @@ int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16
         int sms = 148, rc;
         if ((rc = device_sms(&sms))) return rc;
         const int64_t items = (int64_t)it.groups * it.spans, cap = (int64_t)sms * 8;
-        const size_t smem = (size_t)it.R * it.Q * geo.cc * (geo.n * dtype_size(dtype) + 1) + (lay.plane_bytes ? (size_t)it.R * geo.C * geo.n * 4 : 0);
+        const size_t smem = (size_t)it.R * it.Q * geo.cc * (geo.n * dtype_size(dtype) + 1);
         NMG_DISPATCH_DTYPE(dtype, T, {
             if (geo.n == 1) build_natural_rows_kernel<T, 1><<<(unsigned)(items < cap ? items : cap), NATURAL_THREADS, smem, st>>>(p, it);
             else build_natural_rows_kernel<T, 2><<<(unsigned)(items < cap ? items : cap), NATURAL_THREADS, smem, st>>>(p, it);
@@ -340,14 +225,14 @@ int launch_build_natural(const Geo &geo, int dtype, const void *val, const int16
     // every (mb, k) of the chunks is written exactly once because idx is a permutation per tile; clear first so that the
     // columns between the last chunk and the padded width, and what a malformed idx leaves out, are zeros
     NMG_CUDA(cudaMemsetAsync(pat, 0, lay.pat_bytes + lay.val_bytes, st));  // the values follow the patterns
-    if (lay.plane_bytes) NMG_CUDA(cudaMemsetAsync(p.planes, 0, lay.plane_bytes + lay.fine_bytes, st));
+    if (lay.plane_bytes) NMG_CUDA(cudaMemsetAsync(p.planes, 0, lay.plane_bytes, st));
     if (total < 0x40000000ll) {
         NMG_DISPATCH_DTYPE(dtype, T, (build_natural_kernel<T, true><<<(unsigned)blocks, 256, 0, st>>>(p)));
     } else {
         NMG_DISPATCH_DTYPE(dtype, T, (build_natural_kernel<T, false><<<(unsigned)blocks, 256, 0, st>>>(p)));
     }
     }
-    if (lay.mask_bytes && (parts & (NATURAL_PLANES | NATURAL_FINE))) {  // the transposed product reads none
+    if (lay.mask_bytes) {
         PatternTable tab;
         int rc = get_pattern_table(geo.n, geo.m, &tab);
         if (rc) return rc;

@@ -4,9 +4,8 @@
 // forward product is structured-sparse along the reduction axis and tcgen05.mma.sp does not apply.  What the
 // format does give is a weight that is smaller than its dense form in HBM and L2.  This kernel reads the column-ordered copy
 // (bytes per dense element, 16-bit / fp32: values 2 n/m / 4 n/m; a pattern byte per column of a row-block, 1/m; row masks, n/8;
-// for fp32 two fp16 planes of the values, 4 n/m, and three bf16 planes, 6 n/m.  2:4: 1.5 against 2 dense, fp32 7.5 against 4: the
-// fp32 copy is larger than the dense weight, of which the forward product reads masks and fp16 planes, 2.25, the transposed one
-// values and patterns, 2.25, and the product of a few K-major columns masks and bf16 planes, 3.25).
+// for fp32 three bf16 planes of the values, 6 n/m.  2:4: 1.5 against 2 dense, fp32 5.5 against 4: the fp32 copy is larger than
+// the dense weight, of which the forward product reads masks and planes, 3.25, and the transposed one values and patterns, 2.25).
 // Dedicated warps expand it tile by tile into the tensor core's A operand in TMEM, and it is multiplied at dense tensor-core rate
 // against activation tiles that arrive by TMA.  The same kernel computes the transposed product dX = dY W: only
 // the expansion routine differs (the tile is W^T, the reduction runs over weight rows).
@@ -14,8 +13,8 @@
 // CTA = 15 warps.  Warps 0..11 form three groups that expand the weight tile (128 output features x 64 reduction elements) of
 // every third k-block each, from shared memory through registers into TMEM.  Warp 12 loads activation tiles (up to 256 tokens x 64
 // reduction elements), warp 14 compressed weight tiles, both by TMA; warp 13 allocates TMEM and issues the MMAs (128 x tokens x 16,
-// fp32 accumulate in TMEM).  fp32 weights: a k-block's two fp16 planes are expanded once and multiplied three times (the
-// split products, see nmg_tc_common.cuh; three bf16 planes and six products took 55 us where two take 40: 4096 x 4096 2:4, 256 tokens).  Warps 0..11 then run the epilogue (tcgen05.ld -> bias -> activation -> residual -> store).
+// fp32 accumulate in TMEM).  fp32 weights: a k-block's three bf16 planes are expanded once and multiplied six times (the split
+// products).  Warps 0..11 then run the epilogue (tcgen05.ld -> bias -> activation -> residual -> store).
 //
 // What bounds it with few tokens is latency, not bandwidth: at 4096 x 4096 and 16 tokens the 25 MB of compressed weight are
 // 4 us of HBM time.  So the reduction axis is cut over a cluster of CTAs that fills the chip, and the partial tiles meet in
@@ -46,9 +45,7 @@ struct TcParams {
     int64_t ntok, ld_out;
     int out_token_major;  // 1: out[token][feature], 0: out[feature][token]
     int out_vec;          // token-major 16-bit: rows are 4-byte aligned and hold an even count; feature-major: rows are 16-byte aligned
-    const float *act_factors, *act_small;  // fp32: factors of the activation's rows (DenseAct),
-    int64_t scale_ld;                      // by CTA of a cluster, or 0
-    const uint32_t *feat_max;              // fp32: largest magnitudes of the output features' weight rows (columns if transposed), as bits
+    const float *act_factors;  // fp32: of the activation's rows (DenseAct)
     int act_rows;         // fp32: rows of an activation plane
     int tiles_f, tiles_t; // output tiles along features / tokens
     int bn;               // tokens per tile: a multiple of 32, at most 256 (128 for fp32)
@@ -173,7 +170,7 @@ template <int N_, int M_> __device__ __forceinline__ void build_table(char *tabl
 }
 
 template <int N_, int M_, typename T, int PLANES>
-__device__ __forceinline__ void expand_transposed(const char *vals, const char *pats, const char *table, uint32_t a_tmem, int row, float scale) {
+__device__ __forceinline__ void expand_transposed(const char *vals, const char *pats, const char *table, uint32_t a_tmem, int row) {
     constexpr int W = M_ / 4, J = 32 / M_;  // row-blocks per 32 reduction elements
 #pragma unroll
     for (int h = 0; h < 2; h++) {
@@ -186,7 +183,7 @@ __device__ __forceinline__ void expand_transposed(const char *vals, const char *
             if constexpr (N_ == 1) {
                 const char *src = vals + (j * TC_BM + row) * (int)sizeof(T);
                 if constexpr (PLANES == 1) v[0] = *reinterpret_cast<const uint16_t *>(src);
-                else split_pair(*reinterpret_cast<const float *>(src) * scale, 0.f, v[0], v[PLANES - 1]);
+                else split3_pair(*reinterpret_cast<const float *>(src), 0.f, v[0], v[1], v[2]);
             } else {  // two columns' first values, then their second values
                 const char *src = vals + (j * TC_BM + (row & ~1)) * 2 * (int)sizeof(T);
                 if constexpr (PLANES == 1) {
@@ -194,7 +191,7 @@ __device__ __forceinline__ void expand_transposed(const char *vals, const char *
                     v[0] = __byte_perm(a.x, a.y, (row & 1) ? 0x7632 : 0x5410);
                 } else {
                     const float *f = reinterpret_cast<const float *>(src) + (row & 1);
-                    split_pair(f[0] * scale, f[2] * scale, v[0], v[PLANES - 1]);
+                    split3_pair(f[0], f[2], v[0], v[1], v[2]);
                 }
             }
 #pragma unroll
@@ -217,11 +214,11 @@ constexpr int FX_MAX_STAGES = 8, FX_MAX_SLOTS = 12;
 constexpr int FX_SMEM_LIMIT = 224 * 1024;
 constexpr int FX_MISC_BYTES = 512 + FX_TABLE_BYTES;
 struct FxPlan { int stages, slots, groups, exch_off; uint32_t tmem_cols; size_t total; };
-__host__ __device__ constexpr int fx_val_bytes(int n, int m, int es, bool transposed, int planes) {  // forward: 16-bit planes
-    return 128 * TC_BK / m * n * (transposed ? es : 2 * planes);
+__host__ __device__ constexpr int fx_val_bytes(int n, int m, int es, bool transposed) {  // forward fp32: three 16-bit planes
+    return 128 * TC_BK / m * n * (es == 4 && !transposed ? 6 : es);
 }
-__host__ __device__ constexpr int fx_slot_bytes(int n, int m, int es, bool transposed, int planes) {  // values, then masks (forward) or pattern bytes
-    return fx_val_bytes(n, m, es, transposed, planes) + (transposed ? 128 * TC_BK / m : 128 * 8 * n);
+__host__ __device__ constexpr int fx_slot_bytes(int n, int m, int es, bool transposed) {  // values, then masks (forward) or pattern bytes
+    return fx_val_bytes(n, m, es, transposed) + (transposed ? 128 * TC_BK / m : 128 * 8 * n);
 }
 // columns per CTA of a cluster in the exchange, a multiple of four.  The area is [source][4 columns][128 features][4]: a warp's
 // push is 512 consecutive bytes (16-byte pieces scattered over feature rows moved 16 bytes per clock), and so is its read.
@@ -331,12 +328,11 @@ __device__ __forceinline__ void finish_store(const TcParams &prm, uint32_t (&r)[
 template <int N_, int M_, typename T, bool TRANSPOSED, bool FINE>
 __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams prm, const __grid_constant__ FxMaps maps) {
     constexpr bool SPLIT = sizeof(T) == 4;
-    constexpr int PLANES = SPLIT ? (FINE ? 3 : SPLIT_PLANES) : 1, TERMS = PLANES * (PLANES + 1) / 2;
-    constexpr bool SCALED = SPLIT && !FINE;  // fp16 planes of scaled rows
-    using E = typename std::conditional<FINE, __nv_bfloat16, typename TcMode<T>::elem>::type;  // element type the tensor cores see
+    constexpr int PLANES = SPLIT ? SPLIT_PLANES : 1, TERMS = SPLIT ? SPLIT_TERMS : 1;
+    using E = typename TcMode<T>::elem;  // element type the tensor cores see
     static_assert(TC_BM % M_ == 0 && 32 % M_ == 0 && M_ % 4 == 0 && N_ <= 2, "tile must hold whole row-blocks; a column's values fit one word");
     static_assert(Order<N_, M_>::C * M_ <= FX_TABLE_BYTES, "a pattern byte is an offset into the selector table");
-    constexpr int SLOT_BYTES = fx_slot_bytes(N_, M_, (int)sizeof(T), TRANSPOSED, PLANES), VAL_BYTES = fx_val_bytes(N_, M_, (int)sizeof(T), TRANSPOSED, PLANES);
+    constexpr int SLOT_BYTES = fx_slot_bytes(N_, M_, (int)sizeof(T), TRANSPOSED), VAL_BYTES = fx_val_bytes(N_, M_, (int)sizeof(T), TRANSPOSED);
     static_assert(TRANSPOSED || (SLOT_BYTES % 1024 == 0 && VAL_BYTES % 1024 == 0), "swizzled boxes start on 1024-byte boundaries");
 
     extern __shared__ char smem_raw[];
@@ -371,8 +367,14 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
     const int kb_per = (nkb_all + ks - 1) / ks;
     const int kb_base = split * kb_per;  // this CTA's first k-block
     const int nkb = (nkb_all < kb_base + kb_per ? nkb_all : kb_base + kb_per) - kb_base;  // >= 1 by the host's choice of ksplit
-    const int chunk_kb = SPLIT ? (FINE ? 1 : TC_CHUNK_KB) : nkb;  // k-blocks per accumulation chunk
-    const int nchunks = (nkb + chunk_kb - 1) / chunk_kb;  // per pass over the reduction axis: a tile with a wide row of the activation takes two
+    // k-blocks per accumulation chunk.  fp32: 4, and two chunks at least, so that at most 76 of the additions to an accumulator find a sum of
+    // full size there.  A promotion costs 0.5 us at 64 tokens and 1.2 at 256, so up to four k-blocks make one chunk where their stages are
+    // there together: the largest product of the first `hold` waits for the small ones of all of them, which leaves four such additions per
+    // k-block (three k-blocks in two stages: 32).  Relative error 0.8 .. 1.4e-7 then, else at most 1.3e-6.
+    const bool at_once = nkb <= 3 || (nkb == 4 && prm.stages >= 4);
+    const int chunk_kb = SPLIT ? (FINE ? 1 : at_once ? nkb : nkb < 8 ? (nkb + 1) / 2 : 4) : nkb;
+    const int hold = SPLIT && !FINE && at_once ? min(nkb, prm.stages) : 1;
+    const int nchunks = (nkb + chunk_kb - 1) / chunk_kb;
     const uint32_t tmem_cols = prm.tmem_cols;
     const int cols_live = (int)(prm.ntok - tok0 < bn ? prm.ntok - tok0 : bn);  // token columns of this tile that exist
     const int cpo = fx_cols_per_owner(bn, ks);                                    // columns each CTA of the cluster finishes
@@ -383,11 +385,9 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
         mbar_expect_tx(&full[s], (uint32_t)x_bytes);
 #pragma unroll
         for (int pl = 0; pl < PLANES; pl++)
-            tma_load_2d(smem + s * x_bytes + pl * b_bytes, &maps.x, (kb_base + (kb < nkb ? kb : kb - nkb)) * TC_BK,
-                        (SPLIT ? (pl + (kb < nkb ? 0 : SPLIT_PLANES)) * prm.act_rows : 0) + (int)tok0, &full[s]);
+            tma_load_2d(smem + s * x_bytes + pl * b_bytes, &maps.x, (kb_base + kb) * TC_BK, (SPLIT ? pl * prm.act_rows : 0) + (int)tok0, &full[s]);
     };
     auto load_w = [&](int kb, int s) {
-        if (kb >= nkb) kb -= nkb;
         mbar_expect_tx(&full_w[s], (uint32_t)SLOT_BYTES);
         char *w = slot0 + s * SLOT_BYTES;
         if constexpr (TRANSPOSED) {
@@ -446,14 +446,9 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
         if (TRANSPOSED && warp < FX_WARP_X) build_table<N_, M_>(table, tid, FX_WARP_X * 32);
         dependents_wait();
     }
-    const float *act_small = prm.act_small + split * prm.scale_ld + tok0, *act_factors = prm.act_factors + split * prm.scale_ld + tok0;  // of this tile and range
-    bool wide = false;
-    if constexpr (SCALED)
-        for (int i = lane; i < cols_live; i += 32) wide |= act_small[i] != NOT_WIDE;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const int passes = SCALED && __any_sync(0xffffffffu, wide) ? 2 : 1, total = passes * nkb, all_chunks = passes * nchunks;
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t a_base = tmem_base + (uint32_t)(SPLIT ? 2 * bn : bn);  // A stages follow the accumulator (and the running tile)
     // A partial tile is pushed into the other CTAs' shared memory: they must have started (waited for before the push).
@@ -462,15 +457,6 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
 
     // fp32 mode: a finished chunk of the accumulator is added to the running tile (columns bn .. 2 bn) with round-to-nearest
     // adds.  The MMAs wait for it, so all twelve warps take part: each its quarter of the lanes of every third slice.
-    // small values of wide rows, relative to the others' scale; the other tokens have none
-    auto scale_small = [&](int sl, uint32_t (&r)[32]) {
-        const float f = sl * 32 + lane < cols_live ? act_small[sl * 32 + lane] : NOT_WIDE;
-#pragma unroll
-        for (int j = 0; j < 32; j++) {
-            const float fj = __shfl_sync(0xffffffffu, f, j);
-            r[j] = fj == NOT_WIDE ? 0u : __float_as_uint(__uint_as_float(r[j]) * fj);
-        }
-    };
     auto promote_chunk = [&](int c) -> bool {
         const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
         if (!__all_sync(0xffffffffu, mbar_wait_bounded(chunk_done, (uint32_t)(c & 1), prm.status, 15))) return false;
@@ -478,7 +464,6 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
         for (int sl = warp >> 2; sl < bn / 32; sl += FX_GROUPS) {
             uint32_t r[32];
             tmem_ld32(lane_base + (uint32_t)(sl * 32), r);
-            if (SCALED && c >= nchunks) scale_small(sl, r);
             if (c > 0) {
                 uint32_t run[32];
                 tmem_ld32(lane_base + (uint32_t)(bn + sl * 32), run);
@@ -502,7 +487,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
         int s = is_x ? lead_x : lead_w;
         uint32_t ph = 1;
         if (s >= ring) { s -= ring; ph ^= 1; }
-        for (int kb = is_x ? lead_x : lead_w; kb < total; kb++) {
+        for (int kb = is_x ? lead_x : lead_w; kb < nkb; kb++) {
             ok = mbar_wait_bounded(&freed[s], ph, prm.status, is_x ? 11 : 18);
             if (!__all_sync(0xffffffffu, ok)) break;
             if (elect_one()) {
@@ -519,25 +504,31 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
         const uint64_t bdesc0 = make_sw128_desc(smem_u32(smem));
         int s = 0, chunk = 0, in_chunk = 0;
         uint32_t ph = 0;
-        for (int kb = 0; kb < total; kb++) {
+        for (int kb = 0; kb < nkb; kb++) {
             const bool first = in_chunk == 0;
             if (first && chunk > 0) ok = mbar_wait_bounded(promoted, (uint32_t)((chunk - 1) & 1), prm.status, 16);
             ok = ok && mbar_wait_bounded(&full[s], ph, prm.status, 12);
             if (!__all_sync(0xffffffffu, ok)) break;
             tc_fence_after();
-            const bool chunk_end = (in_chunk + 1 == chunk_kb || kb + 1 == nkb) && kb + 1 < total;
+            const bool chunk_end = in_chunk + 1 == chunk_kb && kb + 1 < nkb;
             if (elect_one()) {
-                const uint32_t at0 = at_base + (uint32_t)(s * PLANES * FX_A_COLS);
-                const uint64_t bs = bdesc0 + (uint64_t)(uint32_t)(s * (x_bytes >> 4));
-#pragma unroll
-                for (int t = 0; t < TERMS; t++) {
-                    const uint32_t at = at0 + (uint32_t)((SPLIT ? split_w(PLANES, t) : 0) * FX_A_COLS);
-                    const uint64_t bt = bs + (uint64_t)(uint32_t)((SPLIT ? split_x(PLANES, t) : 0) * (b_bytes >> 4));
+                auto product = [&](int stage, int t, bool restart) {
+                    const uint32_t at = at_base + (uint32_t)((stage * PLANES + (SPLIT ? split_w(t) : 0)) * FX_A_COLS);
+                    const uint64_t bt = bdesc0 + (uint64_t)(uint32_t)(stage * (x_bytes >> 4) + (SPLIT ? split_x(t) : 0) * (b_bytes >> 4));
 #pragma unroll
                     for (int k = 0; k < TC_BK / 16; k++)  // 16 elements = 8 TMEM columns of A, 32 bytes = 2 descriptor units of B
-                        tc_mma_f16_ta(d_tmem, at + 8 * k, bt + 2 * k, idesc, (first && t == 0 && k == 0) ? 0u : 1u);
+                        tc_mma_f16_ta(d_tmem, at + 8 * k, bt + 2 * k, idesc, (restart && k == 0) ? 0u : 1u);
+                };
+#pragma unroll
+                for (int t = 0; t < TERMS - 1; t++) product(s, t, first && t == 0);
+                if (kb >= hold - 1) {
+                    for (int held = 0; SPLIT && kb == hold - 1 && held < kb; held++) {  // k-block = stage
+                        product(held, TERMS - 1, false);
+                        tc_commit(&empty[held]);
+                    }
+                    product(s, TERMS - 1, first && TERMS == 1);
+                    tc_commit(&empty[s]);  // arrives when the MMAs above have read the stage
                 }
-                tc_commit(&empty[s]);  // arrives when the MMAs above have read the stage
                 if (chunk_end) tc_commit(chunk_done);
             }
             __syncwarp();
@@ -559,13 +550,12 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
         const uint32_t a_lane = a_base + ((uint32_t)((warp & 3) * 32) << 16);
         uint32_t off[8];
         if constexpr (!TRANSPOSED) piece_offsets<M_>(gtid, off);
-        const float scale = SPLIT && TRANSPOSED && feat0 + gtid < prm.out_feats ? pow2(-line_exp(prm.feat_max[feat0 + gtid])) : 1.f;  // of this thread's row
-        for (int kb = group; group < groups && kb < total; kb += groups) {
+        for (int kb = group; group < groups && kb < nkb; kb += groups) {
             if constexpr (SPLIT) {
                 // Before feeding a later chunk, promote the finished ones: the MMAs of a chunk depend only on tiles that are
                 // already published, so this wait cannot deadlock, and the MMA issuer needs the promotion before it may
                 // restart the accumulator.
-                while (ok && drained < (kb < nkb ? kb / chunk_kb : nchunks + (kb - nkb) / chunk_kb)) {
+                while (ok && drained < kb / chunk_kb) {
                     ok = promote_chunk(drained);
                     drained++;
                 }
@@ -576,7 +566,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
             tc_fence_after();  // the MMAs that read this stage are done
             const char *vals = slot0 + w * SLOT_BYTES;
             const uint32_t a_tmem = a_lane + (uint32_t)(s * PLANES * FX_A_COLS);
-            if constexpr (TRANSPOSED) expand_transposed<N_, M_, T, PLANES>(vals, vals + VAL_BYTES, table, a_tmem, gtid, scale);
+            if constexpr (TRANSPOSED) expand_transposed<N_, M_, T, PLANES>(vals, vals + VAL_BYTES, table, a_tmem, gtid);
             else expand_forward<N_, M_, PLANES>(vals, vals + VAL_BYTES, a_tmem, gtid, off);
             __syncwarp();
             if (lane == 0) mbar_arrive(&empty_w[w]);  // the slot has been read
@@ -588,7 +578,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
             if ((w += groups) >= slots) { w -= slots; phw ^= 1; }
         }
         if constexpr (SPLIT)
-            while (ok && drained < all_chunks - 1) {  // the chunks behind the last tile this group published (all of them for an idle group)
+            while (ok && drained < nchunks - 1) {  // the chunks behind the last tile this group published (all of them for an idle group)
                 ok = promote_chunk(drained);
                 drained++;
             }
@@ -599,7 +589,7 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
     tc_fence_before();
     if (exch_apart) cluster_wait();          // the other CTAs have started
     else if (ks > 1) cluster_sync_all();     // every CTA's MMAs are done: shared memory of all of them is free for the exchange
-    if (SPLIT && all_chunks > 1) __syncthreads();  // group 0's promotions, before everybody's reads of the running tile
+    if (SPLIT && nchunks > 1) __syncthreads();  // group 0's promotions, before everybody's reads of the running tile
     tc_fence_after();
 
     // ---- epilogue: warps 0 .. 11, each a quarter of the TMEM lanes and every third slice of 32 token columns
@@ -607,11 +597,6 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
     const int64_t feat = feat0 + fl;
     const bool feat_ok = warp < FX_WARP_X && feat < prm.out_feats;
     const float bias = (prm.bias && feat_ok) ? DT<T>::to_f32(static_cast<const T *>(prm.bias)[feat]) : 0.f;
-    float row_small = 1.f, row_large = 1.f;  // fp32: the feature's factor, see unscale
-    if constexpr (SCALED) {
-        const float f = feat_ok ? pow2(line_exp(prm.feat_max[feat])) : 1.f;
-        (f < 1.f ? row_small : row_large) = f;
-    }
     if (warp < FX_WARP_X) {
         const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16);
         const uint32_t exch = smem_u32(smem + prm.exch_off) + (uint32_t)(split * cpo * 128 * 4 + fl * 16), bar = smem_u32(exchanged);
@@ -620,22 +605,17 @@ __global__ void __launch_bounds__(FX_THREADS, 1) spmm_tc_kernel(const TcParams p
             uint32_t r[32];
             __syncwarp();
             tmem_ld32(lane_base + (uint32_t)(sl * 32), r);
-            if (SPLIT && all_chunks > 1) {
-                if (SCALED && passes == 2) scale_small(sl, r);
+            if (SPLIT && nchunks > 1) {
                 uint32_t run[32];
                 tmem_ld32(lane_base + (uint32_t)(bn + sl * 32), run);
 #pragma unroll
                 for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__fadd_rn(__uint_as_float(run[j]), __uint_as_float(r[j])));
             }
-            if constexpr (SCALED) {  // the tokens' factors are padded to whole tiles
-                const float4 *fac = reinterpret_cast<const float4 *>(act_factors + sl * 32);
+            if constexpr (SPLIT) {  // tokens with a tiny row
+                const float f = sl * 32 + lane < cols_live && prm.act_factors[tok0 + sl * 32 + lane] == TINY_FACTOR ? TINY_FACTOR : 1.f;
+                if (__any_sync(0xffffffffu, f != 1.f)) {
 #pragma unroll
-                for (int v = 0; v < 8; v++) {
-                    const float4 f = __ldg(fac + v);
-                    r[4 * v] = __float_as_uint(unscale(__uint_as_float(r[4 * v]), row_small, row_large, f.x));
-                    r[4 * v + 1] = __float_as_uint(unscale(__uint_as_float(r[4 * v + 1]), row_small, row_large, f.y));
-                    r[4 * v + 2] = __float_as_uint(unscale(__uint_as_float(r[4 * v + 2]), row_small, row_large, f.z));
-                    r[4 * v + 3] = __float_as_uint(unscale(__uint_as_float(r[4 * v + 3]), row_small, row_large, f.w));
+                    for (int j = 0; j < 32; j++) r[j] = __float_as_uint(__uint_as_float(r[j]) * __shfl_sync(0xffffffffu, f, j));
                 }
             }
             if (ks > 1) {
@@ -685,8 +665,8 @@ bool tc_supported(const Geo &geo, int dtype) {
 
 // Tile width and cluster size: the pair with the smallest estimate of a CTA's time, from what the parts of the kernel measure
 // on a B200 (timestamps inside the kernel, 2:4 weights, ns):
-//   per k-block of 64: 300, the expansion and the issue of its MMAs (two planes in fp32: 650, three: 900); above 192 tokens the MMAs
-//     themselves (2 clocks per token), in fp32 above 96 (4096 x 4096: 800 at 128 tokens, 1090 at 192)
+//   per k-block of 64: 300, the expansion and the issue of its MMAs (three planes in fp32: 900); above 192 tokens the MMAs
+//     themselves (2 clocks per token)
 //   per 32-column slice a warp finishes: 450
 //   exchange between ks CTAs: 900 for its barriers, 17 per column for the distributed-shared-memory traffic, 27 per column
 //     finished (bn / ks of them)
@@ -695,8 +675,8 @@ bool tc_supported(const Geo &geo, int dtype) {
 // are not all alike, 24 clusters of 6 do not fit although 144 < 148).
 constexpr int kFxClusters[9] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
 struct FxChoice { int bn, tiles_f, tiles_t, ksplit; int64_t ns; };
-static FxChoice fx_choose(int64_t feats, int64_t red, int64_t tokens, int dtype, bool fine) {
-    const int max_bn = dtype == NMG_F32 ? 192 : 256;  // fp32: the accumulator, the running tile and two stages of two A planes share TMEM
+static FxChoice fx_choose(int64_t feats, int64_t red, int64_t tokens, int dtype) {
+    const int max_bn = dtype == NMG_F32 ? 128 : 256;  // fp32: the accumulator, the running tile and two stages of three A planes share TMEM
     const int64_t tiles_f = (feats + TC_BM - 1) / TC_BM, nkb = (red + TC_BK - 1) / TC_BK;
     FxChoice best{};
     int64_t best_ns = -1;
@@ -710,7 +690,7 @@ static FxChoice fx_choose(int64_t feats, int64_t red, int64_t tokens, int dtype,
             const int64_t per = (nkb + want - 1) / want;
             const int ks = (int)((nkb + per - 1) / per);  // every range non-empty
             const int64_t waves = (tiles + kFxClusters[ks] - 1) / kFxClusters[ks];
-            int64_t ns = 3000 + per * (dtype == NMG_F32 ? (fine ? 900 : bn > 96 ? 220 + bn * 9 / 2 : 650) : bn > 192 ? 300 + (bn - 192) : 300);
+            int64_t ns = 3000 + per * (dtype == NMG_F32 ? 900 : bn > 192 ? 300 + (bn - 192) : 300);
             if (ks > 1) ns += 900 + bn * 17 + bn * 27 / ks;
             else ns += (bn / 32 + 2) / 3 * 450;
             ns *= waves;
@@ -723,66 +703,13 @@ static FxChoice fx_choose(int64_t feats, int64_t red, int64_t tokens, int dtype,
     return best;
 }
 
-// ---- FINE: a K-major fp32 activation src[red][ld_src >= tokens] as three bf16 planes [3][rows][ldp], transposed through a 64 x 32 tile on
-// the way.
-__device__ __forceinline__ void split3_bits(float f, uint32_t (&x)[3]) {  // exact three-way bf16 split, as 16-bit patterns
-    const __nv_bfloat16 hi = __float2bfloat16_rn(f);
-    const float r1 = f - __bfloat162float(hi);
-    const __nv_bfloat16 mid = __float2bfloat16_rn(r1);
-    x[0] = __bfloat16_as_ushort(hi);
-    x[1] = __bfloat16_as_ushort(mid);
-    x[2] = __bfloat16_as_ushort(__float2bfloat16_rn(r1 - __bfloat162float(mid)));
-}
-// two fp32 values -> one word of each bf16 plane
-__device__ __forceinline__ void split3_pair(float lo, float hi, uint32_t &w0, uint32_t &w1, uint32_t &w2) {
-    uint32_t a[3], b[3];
-    split3_bits(lo, a);
-    split3_bits(hi, b);
-    w0 = a[0] | (b[0] << 16); w1 = a[1] | (b[1] << 16); w2 = a[2] | (b[2] << 16);
-}
-__global__ void __launch_bounds__(256) split_f32_t_kernel(const float *__restrict__ src, int64_t red, int64_t tokens, int64_t ld_src,
-                                                          __nv_bfloat16 *__restrict__ dst, int64_t ldp, int64_t plane_elems) {
-    __shared__ float tile[64][33];  // [reduction][token]
-    dependents_launch();
-    dependents_wait();
-    const int64_t k0 = (int64_t)blockIdx.x * 64;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int64_t t0 = (int64_t)blockIdx.y * 32; t0 < tokens; t0 += (int64_t)gridDim.y * 32) {
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int64_t k = k0 + warp * 8 + i, t = t0 + lane;
-            tile[warp * 8 + i][lane] = (k < red && t < tokens) ? __ldg(src + k * ld_src + t) : 0.f;
-        }
-        __syncthreads();
-        const int tok = threadIdx.x >> 3, c = (threadIdx.x & 7) * 8;  // eight reduction elements of one token
-        if (t0 + tok < tokens && k0 + c < ldp) {
-            uint32_t w[3][4];
-#pragma unroll
-            for (int i = 0; i < 4; i++) split3_pair(tile[c + 2 * i][tok], tile[c + 2 * i + 1][tok], w[0][i], w[1][i], w[2][i]);
-#pragma unroll
-            for (int p = 0; p < 3; p++)
-                *reinterpret_cast<uint4 *>(dst + p * plane_elems + (t0 + tok) * ldp + k0 + c) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
-        }
-    }
-}
-
-static bool fine_product(int dtype, int64_t tokens, bool act_k_major) { return dtype == NMG_F32 && act_k_major && tokens < 64; }
-int tc_natural_parts(bool transposed, bool act_k_major, int64_t tokens) {
-    return transposed ? NATURAL_COLUMNS : fine_product(NMG_F32, tokens, act_k_major) ? NATURAL_FINE : NATURAL_PLANES;
-}
-static size_t fine_act_bytes(int64_t tokens, int64_t red) { return (size_t)3 * (size_t)tokens * (size_t)round_up(red, 8) * 2 + 512; }
-size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, bool act_k_major, int64_t tokens) {
-    if (dtype != NMG_F32) return 0;
-    const int64_t red = transposed ? geo.M : geo.K;
-    if (fine_product(dtype, tokens, act_k_major)) return fine_act_bytes(tokens, red);
-    return tc_split_act_bytes(tokens, red, act_k_major ? 8 : 1);  // a range per CTA of a cluster, 8 at most
+size_t tc_split_workspace_bytes(const Geo &geo, int dtype, bool transposed, int64_t tokens) {
+    return dtype == NMG_F32 ? tc_split_act_bytes(tokens, transposed ? geo.M : geo.K) : 0;
 }
 
 template <int N_, int M_, typename T, bool TR, bool FINE = false>
 static int tc_launch_one(const TcParams &p0, const FxMaps &maps, cudaStream_t st) {
-    constexpr int planes = sizeof(T) == 4 ? (FINE ? 3 : SPLIT_PLANES) : 1;
-    const FxPlan plan = fx_plan(planes, p0.bn, p0.ksplit, fx_slot_bytes(N_, M_, (int)sizeof(T), TR, planes));
+    const FxPlan plan = fx_plan(sizeof(T) == 4 ? SPLIT_PLANES : 1, p0.bn, p0.ksplit, fx_slot_bytes(N_, M_, (int)sizeof(T), TR));
     TcParams p = p0;
     p.stages = plan.stages;
     p.slots = plan.slots;
@@ -821,10 +748,11 @@ static int tc_launch_nm(int dtype, bool transposed, bool fine, const TcParams &p
 
 // Policy of the two tensor-core variants.  The fused kernel reads the column-ordered copy; without one (have_packed) a call
 // would build it first and throw it away.  Measured, us, 2:4: fused with a kept copy / fused after building one / two passes
-//   fp32   tokens    1024 x 1024       4096 x 1024       1024 x 4096       4096 x 4096       (-: not measured since the fp16 planes)
-//             256    14 /  37 /  -     19 /  53 /   -    23 / 55 /  -      40 / 124 /   -
-//             512    18 /   - /  -     24 /   - /   -    27 /  - /  -      63 /   - /   -
-//            1000    20 /   - / 25     43 /   - /  46    41 /  - / 53     119 /   - / 129
+//   fp32   tokens    1024 x 1024       4096 x 1024       1024 x 4096       4096 x 4096
+//             256    15 /  33 / 29     22 /  47 /  35    27 / 49 / 68      52 / 113 / 109
+//             512    18 /  37 / 29     29 /  53 /  42    33 / 56 / 70      87 / 157 / 129
+//            1000    23 /  41 / 29     51 /  77 /  60    55 / 78 / 78     189 / 250 / 180
+//            2048    29 /  48 / 36    101 / 128 /  93    95 / 125 / 111   377 / 431 / 313
 //   bf16     1024     9 /  24 / 17     12 /  30 /  21    20 / 37 / 31      27 /  65 /  42
 //            1280    10 /  24 / 17     19 /  37 /  25    21 / 37 / 32      49 /  86 /  60
 //            1500    10 /  24 / 17     20 /  39 /  25    23 / 40 / 33      50 /  88 /  61
@@ -855,30 +783,20 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     }
     const int64_t red = transposed ? geo.M : geo.K;
     const int64_t feats = transposed ? geo.K : geo.M;
-    const bool fine = fine_product(dtype, tokens, act_k_major);
-    const FxChoice fx = fx_choose(feats, red, tokens, dtype, fine);
-    DenseAct x{act, ld_act, nullptr, nullptr, 0};
+    const bool fine = dtype == NMG_F32 && act_k_major && tokens < 64;
+    const FxChoice fx = fx_choose(feats, red, tokens, dtype);
+    DenseAct x{act, ld_act, nullptr};
     if (dtype == NMG_F32) {
-        // the ranges of the reduction axis that the CTAs of a cluster take
-        const int64_t nkb = (red + TC_BK - 1) / TC_BK, range = (nkb + fx.ksplit - 1) / fx.ksplit * TC_BK;
-        const size_t need = fine ? fine_act_bytes(tokens, red) : tc_split_act_bytes(tokens, red, act_k_major ? fx.ksplit : 1);
+        const size_t need = tc_split_act_bytes(tokens, red);
         if (!ws || ws_bytes < need) NMG_FAIL(NMG_ERR_WORKSPACE, "workspace of %zu bytes required for the split activation, got %zu", need, ws_bytes);
-        char *buf = reinterpret_cast<char *>(((uintptr_t)ws + 255) & ~(uintptr_t)255);
-        if (fine) {
-            x = DenseAct{buf, round_up(red, 8), nullptr, nullptr, 0};
-            if ((rc = launch_early(split_f32_t_kernel, dim3((unsigned)((x.ld + 63) / 64), (unsigned)((tokens + 31) / 32)), 256, 0, st, static_cast<const float *>(act), red, tokens, ld_act,
-                                   reinterpret_cast<__nv_bfloat16 *>(buf), x.ld, tokens * x.ld)))
-                return rc;
-        } else if ((rc = tc_split_act(act, ld_act, act_k_major, tokens, red, range, buf, &x, st))) {
-            return rc;
-        }
+        if ((rc = tc_split_act(act, ld_act, act_k_major, tokens, red, reinterpret_cast<char *>(((uintptr_t)ws + 255) & ~(uintptr_t)255), &x, st))) return rc;
     }
     int *status = nullptr;
     if ((rc = get_status_word(&status))) return rc;
     const size_t es = dtype_size(dtype);
     FxMaps maps;
-    const int edt = fine ? NMG_BF16 : dtype == NMG_F32 ? NMG_F16 : dtype;
-    if ((rc = encode_tmap_2d(&maps.x, edt, x.base, (uint64_t)red, (uint64_t)tokens * (fine ? 3 : dtype == NMG_F32 ? ACT_PLANES : 1), (uint64_t)x.ld, TC_BK, (uint32_t)fx.bn, 1))) return rc;
+    const int edt = dtype == NMG_F32 ? NMG_BF16 : dtype, planes = dtype == NMG_F32 ? SPLIT_PLANES : 1;
+    if ((rc = encode_tmap_2d(&maps.x, edt, x.base, (uint64_t)red, (uint64_t)tokens * planes, (uint64_t)x.ld, TC_BK, (uint32_t)fx.bn, 1))) return rc;
     const int64_t Kpn = natural_width(geo);
     const NaturalLayout lay = natural_layout(geo, dtype);
     const char *masks = static_cast<const char *>(nval) + lay.val_bytes;
@@ -887,8 +805,7 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
         if ((rc = encode_tmap_2d_bytes(&maps.pat, pat, (uint64_t)Kpn, (uint64_t)geo.nb, (uint64_t)Kpn, TC_BM, (uint32_t)(TC_BK / geo.m)))) return rc;
         if ((rc = encode_tmap_2d(&maps.val, dtype, nval, row_elems, (uint64_t)geo.nb, row_elems, (uint32_t)(TC_BM * geo.n), (uint32_t)(TC_BK / geo.m), 0))) return rc;
     } else {
-        const int planes = fine ? 3 : dtype == NMG_F32 ? SPLIT_PLANES : 1;
-        const char *vals = dtype != NMG_F32 ? static_cast<const char *>(nval) : masks + lay.mask_bytes + (fine ? lay.plane_bytes : 0);
+        const char *vals = dtype != NMG_F32 ? static_cast<const char *>(nval) : masks + lay.mask_bytes;
         if ((rc = encode_tmap_2d(&maps.val, edt, vals, row_elems, (uint64_t)(geo.nb * planes), row_elems, TC_BK, (uint32_t)(TC_BM / geo.m), 1))) return rc;
         maps.pat = maps.val;  // never used; keeps the parameter defined
     }
@@ -903,8 +820,7 @@ int tc_matmul(const Geo &geo, int dtype, bool transposed, bool dense, const void
     // 11 tokens 6.5 -> 5.6; 4096 x 4096, 16 tokens 10.1 -> 9.7).  A pass over the activation that settles on the SMs left free then is the slower
     // for it (mm bf16 2240 x 9216, 64 columns 14.1 -> 15.2), and so are some long ones (5440 x 10944 1:16, 128 tokens 23.8 -> 24.5).
     p.announce = alone && dtype != NMG_F32 && fx.ns < 14000;
-    p.act_factors = x.factors; p.act_small = x.small; p.scale_ld = x.scale_ld; p.act_rows = (int)tokens;
-    if (dtype == NMG_F32) p.feat_max = reinterpret_cast<const uint32_t *>(masks + lay.mask_bytes + lay.plane_bytes + lay.fine_bytes) + (transposed ? natural_mask_rows(geo) : 0);
+    p.act_factors = x.factors; p.act_rows = (int)tokens;
     p.masks = masks; p.mask_rows = natural_mask_rows(geo); p.nb = geo.nb;
     p.status = status;
     const ProfileEvents pe = take_profile_events();

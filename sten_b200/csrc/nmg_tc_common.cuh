@@ -9,7 +9,6 @@ constexpr int TC_BM = 128;    // output features per CTA (MMA M)
 constexpr int TC_BN = 256;    // tokens per CTA (MMA N)
 constexpr int TC_BK = 64;     // reduction elements per stage: one 128-byte swizzle span of 16-bit data
 constexpr int TC_STAGES = 4;
-constexpr int TC_CHUNK_KB = 8;       // fp32 mode: k-blocks (of 64) accumulated in the tensor core before promotion
 constexpr int TC_A_BYTES = TC_BM * TC_BK * 2;  // 16 KB
 constexpr int TC_B_BYTES = TC_BN * TC_BK * 2;  // 32 KB
 constexpr int TC_ACC_COLS = 256;    // one fp32 accumulator tile: 128 lanes x 256 columns
@@ -159,9 +158,6 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t local, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
-__device__ __forceinline__ void st_cluster(uint32_t cluster_addr, uint32_t v) {
-    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
-}
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
@@ -294,57 +290,44 @@ __device__ __forceinline__ void gelu_erf_pair(uint32_t &ra, uint32_t &rb) {
 
 // ---- fp32 operands ---------------------------------------------------------------------------------------------------------
 // The tensor core's fp32 accumulator truncates instead of rounding, which biases long sums: the relative error grows linearly with the
-// reduction length.  fp32 products therefore keep a running sum outside the tensor core: every TC_CHUNK_KB k-blocks the partial tile
-// is added to it with round-to-nearest FADDs (fused kernel: a second accumulator tile in TMEM, by all twelve warps; two-pass
-// kernel: registers of the drain warps) and the MMAs restart from zero.  The error then does not depend on the length.
+// number of additions to a sum that has its size already, by 2e-8 each.  fp32 products therefore keep a running sum outside the tensor
+// core: after every chunk of k-blocks the partial tile is added to it with round-to-nearest FADDs (fused kernel: a second accumulator
+// tile in TMEM, by all twelve warps; two-pass kernel: registers of the drain warps) and the MMAs restart from zero.  The error
+// then does not depend on the length.
 //
-// fp32 operands run as fp16 planes, x = (h + l) 2^e with h = fp16(x 2^-e), l = fp16(x 2^-e - h) and one exponent e per row of the
-// operand that brings the row's largest magnitude to [2^14, 2^15).  Three products (wl xh, wh xl, wh xh) then stand for the fp32 product:
-// what h + l leaves of a value and the dropped wl xl are at most 2^-22 of it, and a value below 2^-18 of its row's largest keeps an
-// absolute 2^-39 of that.  Against three bf16 planes and six products (exact to 2^-24) that halves the tensor-core work, and the
-// result is closer to the exact one, because what dominates the error is the number of truncating additions in the accumulator
-// (above): half as many.  Relative error against fp64, 1:4: 1.1e-6 -> 0.3e-6 at 128 reduction elements, 3.4e-6 -> 1.7e-6 from 3072;
-// lower in every row and column too, for normal, heavy-tailed and very large or small values, rows of different scale and outliers.
-// Time, 4096 tokens, 1:4: the matmul 3072 <- 768 86 -> 56 us, the whole call 4096 <- 4096 about 560 -> 303 us.
+// fp32 operands run as exact sums of three bf16 pieces, x = xh + xm + xl, which have fp32's range: every value keeps its own precision,
+// however far it lies below the others of its row.  Of the nine products of pieces six are computed, smallest first; the three left
+// out are at most 2^-24 of the product each, the size of an fp32 rounding.
+// Two fp16 pieces under one exponent per row take three products (3072 <- 768, 4096 tokens: 62.6 us against 84.1), but they lose
+// what lies more than 2^-18 below the largest of its row, and outputs that meet only such values are wrong without a sign of it.
 //
-// Activation rows whose values are mostly far below the largest (a mask value, a saturated feature) are two rows: the values from
-// 2^-16 of the largest on, and the rest with an exponent of its own (down to about 2^-120 of the other; what lies further below loses
-// bits and then is zero) and its own planes.  A tile that holds such a row runs its reduction twice, over either pair of planes.
-__device__ __forceinline__ int line_exp(uint32_t max_bits) {  // infinities and NaN count as the largest finite value
-    const int e = (int)(max_bits >> 23) - (127 + 14);
-    return max_bits == 0 ? 0 : e < -126 ? -126 : e > 113 ? 113 : e;
-}
-__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 <= e <= 127
-// v 2^(er + ec) with the row's and the column's factor.  A factor below one comes first: the other order could overflow on the way.
-__device__ __forceinline__ float unscale(float v, float row_small, float row_large, float col) { return v * row_small * col * row_large; }
-// What a row's values are like: largest magnitude, sum of the exponents and number of the values that are not zero.
-struct RowStats {
-    uint32_t mx = 0, exps = 0, count = 0;
-    __device__ __forceinline__ void add(float v) {
-        const uint32_t u = __float_as_uint(v) & 0x7fffffffu;
-        mx = max(mx, u);
-        exps += u >> 23;
-        count += u != 0;
-    }
-    // The mean exponent of the values is more than 16 below the largest one's.  (Infinities and NaN: such a row's results are not finite.)
-    __device__ __forceinline__ bool wide() const { return mx < 0x7f800000u && (uint64_t)exps + 16ull * count < (uint64_t)(mx >> 23) * count; }
-};
-__device__ __forceinline__ bool is_small(float v, uint32_t mx) { return (__float_as_uint(v) & 0x7fffffffu) < mx - min(mx, 16u << 23); }  // of a wide row
-constexpr float NOT_WIDE = -1.f;  // in place of the factor between the two parts of a row
-// two scaled values -> one word of each plane
-__device__ __forceinline__ void split_pair(float a, float b, uint32_t &hi, uint32_t &lo) {
-    const __half2 h = __floats2half2_rn(a, b);
-    const float2 f = __half22float2(h);
-    const __half2 l = __floats2half2_rn(a - f.x, b - f.y);
+// Pieces below bf16's range: a value below 2^-110 loses its last bits.  An activation row that has no value of 2^-80 or more is
+// split times 2^40, and its results are multiplied by 2^-40.
+constexpr int SPLIT_PLANES = 3, SPLIT_TERMS = 6;
+constexpr uint32_t TINY_ROW = (uint32_t)(127 - 80) << 23;  // magnitude bits: rows below are tiny
+constexpr float TINY_SCALE = 0x1p40f, TINY_FACTOR = 0x1p-40f;
+__device__ __forceinline__ bool not_tiny(float v) { return (__float_as_uint(v) & 0x7fffffffu) >= TINY_ROW; }  // infinities and NaN too
+// Two values -> one word of each plane.  The largest magnitudes would round up to infinity: their first piece is the largest finite one.
+__device__ __forceinline__ void split3_pair(float a, float b, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
+    constexpr float TOP = 0x1.fep127f;
+    const __nv_bfloat162 h = __floats2bfloat162_rn(fminf(fmaxf(a, -TOP), TOP), fminf(fmaxf(b, -TOP), TOP));
+    const float ra = a - __low2float(h), rb = b - __high2float(h);
+    const __nv_bfloat162 m = __floats2bfloat162_rn(ra, rb);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(ra - __low2float(m), rb - __high2float(m));
     hi = *reinterpret_cast<const uint32_t *>(&h);
+    mid = *reinterpret_cast<const uint32_t *>(&m);
     lo = *reinterpret_cast<const uint32_t *>(&l);
 }
-constexpr int SPLIT_PLANES = 2, ACT_PLANES = 4;
-// Planes of product t, the smallest products first.  Three planes: bf16, x = xh + xm + xl exactly (fused kernel, FINE), the six products
-// whose weight is >= 2^-16 of the leading one.
-constexpr int split_w(int planes, int t) { return planes == 2 ? t == 0 : t == 1 ? 2 : t == 2 || t == 4 ? 1 : 0; }
-constexpr int split_x(int planes, int t) { return planes == 2 ? t == 1 : t == 0 ? 2 : t == 2 || t == 3 ? 1 : 0; }
+__device__ __forceinline__ void split3(float f, __nv_bfloat16 (&piece)[3]) {
+    uint32_t w[3];
+    split3_pair(f, 0.f, w[0], w[1], w[2]);
+#pragma unroll
+    for (int c = 0; c < 3; c++) piece[c] = __ushort_as_bfloat16((unsigned short)(w[c] & 0xffffu));
+}
+// Planes of product t, the smallest products first
+constexpr int split_w(int t) { return t == 1 ? 2 : t == 2 || t == 4 ? 1 : 0; }
+constexpr int split_x(int t) { return t == 0 ? 2 : t == 2 || t == 3 ? 1 : 0; }
 template <typename T> struct TcMode { using elem = T; };  // what the tensor cores multiply
-template <> struct TcMode<float> { using elem = __half; };
+template <> struct TcMode<float> { using elem = __nv_bfloat16; };
 
 }  // namespace nmg

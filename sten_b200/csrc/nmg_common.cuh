@@ -113,7 +113,9 @@ template <auto Kernel> inline int allow_smem(size_t bytes) {
     } while (0)
 // Launch that may begin before the kernels queued ahead of it have ended: it runs up to its first dependents_wait() beside their
 // ends, so that neither the launch nor the set-up is waited for.  Every CTA of such a kernel has to get there before it reads or
-// writes anything another kernel does, and before it exits: what is queued behind it relies on that.
+// writes anything another kernel does, and before it exits: what is queued behind it relies on that.  What an earlier kernel may write is
+// read with ordinary loads: __ldg, and const __restrict__ parameters, assert that it stays as it is for the kernel's whole life, and
+// such a load need not stay behind the wait.
 template <class... P, class... A> int launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;

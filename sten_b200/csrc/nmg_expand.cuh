@@ -52,10 +52,10 @@ __device__ __forceinline__ void expand_scatter_item(const ExpandParams &prm, T *
         constexpr int VL = N_ * (int)sizeof(T) / 2;  // 16-byte loads of values per 8 slots
         const bool same_pattern = (g & 7) == 0;  // 8 consecutive slots then belong to one pattern
         for (int e8 = threadIdx.x * 8; e8 < total; e8 += EXPAND_THREADS * 8) {
-            const uint4 iv = __ldg(reinterpret_cast<const uint4 *>(isrc + e8));
+            const uint4 iv = *reinterpret_cast<const uint4 *>(isrc + e8);
             uint4 vv[VL];
 #pragma unroll
-            for (int u = 0; u < VL; u++) vv[u] = __ldg(reinterpret_cast<const uint4 *>(vsrc + (int64_t)e8 * N_) + u);
+            for (int u = 0; u < VL; u++) vv[u] = reinterpret_cast<const uint4 *>(vsrc + (int64_t)e8 * N_)[u];
             const int16_t *ci = reinterpret_cast<const int16_t *>(&iv);
             const T *vals = reinterpret_cast<const T *>(vv);
             const int j = e8 / cc, s0 = e8 - j * cc;  // cc is a multiple of 8: the 8 slots share the row-block

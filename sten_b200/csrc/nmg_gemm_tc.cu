@@ -165,9 +165,9 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
         iv = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);  // column -1: no slot
         if (!has || span * Q + uq >= prm.nc || grp * R + uj >= prm.nb) return;
         const int64_t slot = ((int64_t)(span * Q + uq) * prm.nb + grp * R + uj) * cc + uslot;
-        iv = __ldg(reinterpret_cast<const uint4 *>(prm.idx + slot));
+        iv = *reinterpret_cast<const uint4 *>(prm.idx + slot);
 #pragma unroll
-        for (int i = 0; i < VL; i++) vv[i] = __ldg(reinterpret_cast<const uint4 *>(val + slot * N_) + i);
+        for (int i = 0; i < VL; i++) vv[i] = reinterpret_cast<const uint4 *>(val + slot * N_)[i];
     };
     for (int i = tid; i < prm.C * N_; i += EXPAND_THREADS) ord[i] = prm.order[i];
     for (int i = tid; i < rows * cols * (int)sizeof(T) / 16; i += EXPAND_THREADS) reinterpret_cast<uint4 *>(smem)[i] = make_uint4(0, 0, 0, 0);
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                     const int64_t tokc = (int64_t)tok0 + sl * 32;
                     if (res && feat_ok && res_vec_ok(tokc)) {
 #pragma unroll
-                        for (int v = 0; v < RQ; v++) qr[v] = __ldg(reinterpret_cast<const uint4 *>(res + feat * prm.ld_res + tokc) + v);
+                        for (int v = 0; v < RQ; v++) qr[v] = reinterpret_cast<const uint4 *>(res + feat * prm.ld_res + tokc)[v];
                     }
                 }
             };
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                                     const uint4 *src = reinterpret_cast<const uint4 *>(res + feat * prm.ld_res + tokc);
 #pragma unroll
                                     for (int v = 0; v < 8; v++) {
-                                        const uint4 w = __ldg(src + v);
+                                        const uint4 w = src[v];
                                         r[4 * v] = __float_as_uint(__uint_as_float(r[4 * v]) + __uint_as_float(w.x));
                                         r[4 * v + 1] = __float_as_uint(__uint_as_float(r[4 * v + 1]) + __uint_as_float(w.y));
                                         r[4 * v + 2] = __float_as_uint(__uint_as_float(r[4 * v + 2]) + __uint_as_float(w.z));
@@ -819,7 +819,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                             for (int i = 0; i < CPR; i++) {
                                 const int64_t tok = tokc + i * (32 / CPR) + lane / CPR;
                                 rv[i] = make_uint4(0u, 0u, 0u, 0u);
-                                if (tok < prm.ntok && whole) rv[i] = __ldg(reinterpret_cast<const uint4 *>(res + tok * prm.ld_res + fbase));
+                                if (tok < prm.ntok && whole) rv[i] = *reinterpret_cast<const uint4 *>(res + tok * prm.ld_res + fbase);
                             }
                         }
                         T *st = reinterpret_cast<T *>(stage_w);
@@ -917,7 +917,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
                         if (res && res_late) {  // the loads of the eight rows are independent of one another and of the staging tile
                             __align__(16) T a[CHUNK_TOK], b[CHUNK_TOK];
                             *reinterpret_cast<uint4 *>(a) = w;
-                            if (tokg + CHUNK_TOK <= prm.ntok) *reinterpret_cast<uint4 *>(b) = __ldg(reinterpret_cast<const uint4 *>(res + f * prm.ld_res + tokg));
+                            if (tokg + CHUNK_TOK <= prm.ntok) *reinterpret_cast<uint4 *>(b) = *reinterpret_cast<const uint4 *>(res + f * prm.ld_res + tokg);
                             else
                                 for (int k = 0; k < CHUNK_TOK; k++) b[k] = tokg + k < prm.ntok ? res[f * prm.ld_res + tokg + k] : DT<T>::from_f32(0.f);
 #pragma unroll

@@ -49,8 +49,7 @@ int launch_transpose_to_f32(const void *src, int dtype, int64_t rows, int64_t co
 // Transpose of 16-bit elements: src[rows][ld_src] -> dst[cols][ld_dst], 64 x 64 tiles through shared memory.  Both sides move
 // 128 bytes per warp instruction: a thread reads two neighbouring elements of a source row and writes two
 // neighbouring elements of a destination row.  Columns of dst beyond `rows` (up to ld_dst) are zero.
-__global__ void __launch_bounds__(256) transpose_kernel(const uint16_t *__restrict__ src, int64_t rows, int64_t cols, int64_t ld_src,
-                                                        uint16_t *__restrict__ dst, int64_t ld_dst) {
+__global__ void __launch_bounds__(256) transpose_kernel(const uint16_t *src, int64_t rows, int64_t cols, int64_t ld_src, uint16_t *dst, int64_t ld_dst) {
     __shared__ uint16_t tile[64][66];
     dependents_launch();  // the matmul's set-up may overlap this pass
     dependents_wait();
@@ -88,7 +87,7 @@ int launch_transpose(const void *src, int64_t rows, int64_t cols, int64_t ld_src
 
 // Eight elements per thread: 2-byte loads (the rows have no alignment; a warp's eight loads share their lines in L1), one
 // 16-byte store.
-__global__ void __launch_bounds__(256) pad_rows_kernel(const uint16_t *__restrict__ src, int64_t rows, int64_t cols, int64_t ld_src, uint16_t *__restrict__ dst, int64_t ld_dst) {
+__global__ void __launch_bounds__(256) pad_rows_kernel(const uint16_t *src, int64_t rows, int64_t cols, int64_t ld_src, uint16_t *dst, int64_t ld_dst) {
     dependents_launch();  // the matmul's set-up may overlap this pass
     dependents_wait();
     const int64_t per_row = ld_dst / 8;
@@ -98,7 +97,7 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(const uint16_t *__restric
             const int left = (int)(cols - v * 8 < 8 ? cols - v * 8 : 8);
             uint32_t e[8];
 #pragma unroll
-            for (int i = 0; i < 8; i++) e[i] = i < left ? (uint32_t)__ldg(s + i) : 0u;
+            for (int i = 0; i < 8; i++) e[i] = i < left ? (uint32_t)s[i] : 0u;
             *reinterpret_cast<uint4 *>(dst + r * ld_dst + v * 8) = make_uint4(e[0] | (e[1] << 16), e[2] | (e[3] << 16), e[4] | (e[5] << 16), e[6] | (e[7] << 16));
         }
 }

@@ -144,7 +144,9 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_dense_kernel(const Expa
 // its stores.  Here an item is R row-blocks x Q chunks, about 512 columns of as many rows as give every thread one piece of
 // eight slots, so that rows leave in whole lines; what a thread does with its piece -- row-block, pattern rows, place in the
 // tile -- is the same for every item and computed once; the next item's loads are in flight while a tile is moved out.
-template <typename T, int N_, bool PLAIN>
+// STRIPS (PLAIN only): rows of the destination are not 16-byte aligned.  A kernel of its own: together the two took 64 to 78 registers for
+// 16-bit n = 2, as the compiler pleased, and with 78 three CTAs fit an SM where four do: densify 8192 x 8192 bf16 38.0 .. 39.9 -> 34.5 us.
+template <typename T, int N_, bool PLAIN, bool STRIPS>
 __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const ExpandParams prm) {
     extern __shared__ __align__(16) char smem[];
     const int m = prm.m, g = prm.g, cc = prm.cc, R = prm.R, Q = prm.Q, cols = Q * cc, rows = R * m;
@@ -198,7 +200,7 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
         const int span = (int)(item / groups), grp = (int)(item - (int64_t)span * groups);
         const int64_t r0 = (int64_t)grp * rows, c0 = (int64_t)span * cols;
         const int row_lim = (int)(prm.M - r0 < rows ? prm.M - r0 : rows), col_lim = (int)(prm.K - c0 < cols ? prm.K - c0 : cols);
-        if (PLAIN && !prm.vec) {  // rows of the destination are not 16-byte aligned: neighbouring threads store neighbouring elements
+        if constexpr (STRIPS) {  // rows of the destination are not 16-byte aligned: neighbouring threads store neighbouring elements
             const int dle = EXPAND_THREADS / cols, dee = EXPAND_THREADS - dle * cols;
             for (int v = tid, l = tid / cols, e = tid - l * cols; v < rows * cols; v += EXPAND_THREADS) {
                 if (l < row_lim && e < col_lim) static_cast<T *>(prm.dst)[(r0 + l) * prm.ld + c0 + e] = tile[v];
@@ -207,27 +209,31 @@ __global__ void __launch_bounds__(EXPAND_THREADS) expand_rows_kernel(const Expan
                 if ((e += dee) >= cols) { e -= cols; l++; }
             }
             __syncthreads();
-            continue;
-        }
-        // A vector that starts inside the weight may run past K only into the row's padding (ld = round_up(K, 8)).
-        for (int v = tid, l = l0, e = e0; v < total; v += EXPAND_THREADS) {
-            T *line = tile + v * V;
-            const int64_t off = (r0 + l) * prm.ld + c0 + e * V;
-            const bool inside = l < row_lim && e * V < col_lim;
-            if constexpr (V * sizeof(T) == 16) {
-                if (inside) *reinterpret_cast<uint4 *>(static_cast<T *>(prm.dst) + off) = *reinterpret_cast<const uint4 *>(line);
-                *reinterpret_cast<uint4 *>(line) = make_uint4(0, 0, 0, 0);
-            } else {
-                if (inside) expand_flush<T, true, PLAIN>(prm, line, off, V);
-                else {
-                    reinterpret_cast<uint4 *>(line)[0] = make_uint4(0, 0, 0, 0);
-                    reinterpret_cast<uint4 *>(line)[1] = make_uint4(0, 0, 0, 0);
+        } else {
+            // A vector that starts inside the weight may run past K only into the row's padding (ld = round_up(K, 8)).
+            // Pieces in flight per thread against registers, us with 1 / 2: densify bf16 2:8 8192 x 8192 34.4 / 35.0, f16 1:4 4096 x 4096 9.7 / 9.2;
+            // the pass and the matmul behind it, bf16 1:8 4096 x 4096, 4096 tokens 104.1 / 105.1.
+            constexpr int FLUSH = PLAIN && sizeof(T) == 2 && N_ == 1 ? 2 : 1;
+#pragma unroll FLUSH
+            for (int v = tid, l = l0, e = e0; v < total; v += EXPAND_THREADS) {
+                T *line = tile + v * V;
+                const int64_t off = (r0 + l) * prm.ld + c0 + e * V;
+                const bool inside = l < row_lim && e * V < col_lim;
+                if constexpr (V * sizeof(T) == 16) {
+                    if (inside) *reinterpret_cast<uint4 *>(static_cast<T *>(prm.dst) + off) = *reinterpret_cast<const uint4 *>(line);
+                    *reinterpret_cast<uint4 *>(line) = make_uint4(0, 0, 0, 0);
+                } else {
+                    if (inside) expand_flush<T, true, PLAIN>(prm, line, off, V);
+                    else {
+                        reinterpret_cast<uint4 *>(line)[0] = make_uint4(0, 0, 0, 0);
+                        reinterpret_cast<uint4 *>(line)[1] = make_uint4(0, 0, 0, 0);
+                    }
                 }
+                l += dl;
+                if ((e += de) >= vpl) { e -= vpl; l++; }
             }
-            l += dl;
-            if ((e += de) >= vpl) { e -= vpl; l++; }
+            __syncthreads();
         }
-        __syncthreads();
     }
 }
 // R and Q of the rows kernel, false when it does not serve the weight
@@ -1040,14 +1046,15 @@ template <typename T, bool TR, int N_, bool PLAIN> static int expand_launch_n(co
     NMG_ALLOW_SMEM(smem, expand_dense_kernel<T, TR, N_, PLAIN>);
     return launch_early(expand_dense_kernel<T, TR, N_, PLAIN>, (unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st, p);
 }
-template <typename T, int N_, bool PLAIN> static int expand_rows_launch_n(const ExpandParams &p, size_t smem, cudaStream_t st) {
+template <typename T, int N_, bool PLAIN, bool STRIPS = false> static int expand_rows_launch_n(const ExpandParams &p, size_t smem, cudaStream_t st) {
     int sms = 148, rc;
     if ((rc = device_sms(&sms))) return rc;
-    NMG_ALLOW_SMEM(smem, expand_rows_kernel<T, N_, PLAIN>);
+    if (PLAIN && !STRIPS && !p.vec) return expand_rows_launch_n<T, N_, PLAIN, PLAIN>(p, smem, st);
+    NMG_ALLOW_SMEM(smem, expand_rows_kernel<T, N_, PLAIN, STRIPS>);
     int per_sm = (int)((size_t)227 * 1024 / (smem + 1024));
     if (per_sm > 8) per_sm = 8;
     const int64_t items = ((p.nb + p.R - 1) / p.R) * ((p.nc + p.Q - 1) / p.Q), cap = (int64_t)sms * per_sm;
-    return launch_early(expand_rows_kernel<T, N_, PLAIN>, (unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st, p);
+    return launch_early(expand_rows_kernel<T, N_, PLAIN, STRIPS>, (unsigned)(items < cap ? items : cap), EXPAND_THREADS, smem, st, p);
 }
 template <typename T, bool PLAIN> static int expand_rows_launch(const ExpandParams &p, size_t smem, cudaStream_t st) {
     return p.n == 1 ? expand_rows_launch_n<T, 1, PLAIN>(p, smem, st) : expand_rows_launch_n<T, 2, PLAIN>(p, smem, st);

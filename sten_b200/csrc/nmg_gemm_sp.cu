@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_sp_kernel(const SpGemmPara
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (of the leader; converged warp)
         if (leader) {
+            dependents_wait();  // the limits of the waits below count from here, not while kernels ahead run
             const uint32_t idesc = make_idesc_sp_pair<T>();
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0), stage0 = smem_u32(smem);
             const uint64_t desc0 = make_sw128_desc(stage0);
@@ -299,6 +300,7 @@ __global__ void __launch_bounds__(SP_THREADS, 1) gemm_sp_kernel(const SpGemmPara
         const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
         T *out = static_cast<T *>(prm.out);
         bool ok = true;
+        dependents_wait();
         for (int ti = 0; ti < my_tiles && ok; ti++) {
             int tile_f, tok0;
             tile_origin(ti, tile_f, tok0);

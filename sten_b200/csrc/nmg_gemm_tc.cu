@@ -596,6 +596,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) gemm_tc_kernel(const GemmPara
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (of the leader for pairs)
         if (leader) {
+            dependents_wait();  // the limits of the waits below count from here, not while kernels ahead run
             const uint32_t tmem_u = __shfl_sync(0xffffffffu, tmem_base, 0);
             const uint64_t desc0 = make_sw128_desc(smem_u32(smem));
             bool ok = true;

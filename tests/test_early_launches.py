@@ -14,7 +14,7 @@ def _sources():
 
 def _kernels(text):
     """(name, signature and body) of every __global__ function."""
-    for m in re.finditer(r"__global__[^;{]*?(\w+)\s*\([^;{]*\)\s*\{", text):
+    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\([^)]*\)\s*)?(\w+)\s*\([^;{]*\)\s*\{", text):
         depth, i = 1, m.end()
         while depth:
             depth += {"{": 1, "}": -1}.get(text[i], 0)
@@ -39,4 +39,21 @@ def test_early_kernels_wait_and_read_with_ordinary_loads():
             assert "__ldg" not in code and "__restrict__" not in code, f"{name}: {kernel}"
         if name in ("nmg_expand.cuh", "nmg_tc_common.cuh"):  # device functions that they call
             assert "__ldg" not in text and "__restrict__" not in text, name
+    assert seen >= 9
+
+
+def test_bounded_waits_begin_behind_the_kernels_ahead():
+    """A wait that gives up after a time must not count the time that earlier kernels of the stream take."""
+    seen = 0
+    for name, text in _sources():
+        for kernel, code in _kernels(text):
+            if kernel not in ("gemm_tc_kernel", "gemm_sp_kernel", "spmm_tc_kernel"):
+                continue
+            parts = re.split(r"// -{20,}", code)  # what comes before the roles of the warps, then a part for each
+            ahead = parts[0].count("dependents_wait();") == 3  # spmm_tc_kernel: all three branches of its set-up
+            for part in parts[1:]:
+                first = re.search(r"[^_]wait\(&|mbar_wait\w*\(", part)
+                if first:
+                    seen += 1
+                    assert ahead or "dependents_wait();" in part[:first.start()], f"{name}: {kernel}: {part.strip().splitlines()[0]}"
     assert seen >= 9

@@ -24,6 +24,7 @@
 #include "nmg_expand.cuh"
 #include "nmg_spmm_simt.cuh"
 #include "nmg_tc_common.cuh"
+#include "nmg_tiles.h"
 
 namespace nmg {
 
@@ -410,19 +411,10 @@ __global__ void __launch_bounds__(COLS_THREADS) split_columns_kernel(const Split
 // =========================================================================================================
 // Dense-operand matmul
 // =========================================================================================================
+static_assert(TILE_COLS == TC_BN, "one accumulator");
 constexpr int GEMM_DRAIN_WARPS = 8;   // two per TMEM lane quarter, each takes half of the accumulator's columns
 constexpr int GEMM_THREADS = 32 * (4 + GEMM_DRAIN_WARPS);  // TMA warp, MMA warp, two idle ones, drain warps
 constexpr int GEMM_RING_BYTES = TC_STAGES * (TC_A_BYTES + TC_B_BYTES);  // 192 KB of operand stages in either mode
-
-// The output's tiles: the first f_wide rows of tiles are bn columns wide, the f_narrow rows below them bn_tail.
-// See gemm_tiles for the choice.
-struct GemmTiles {
-    int f_wide, f_narrow;    // rows of tiles
-    int t_wide, t_narrow;    // tiles per row
-    int bn, bn_tail;         // columns of a tile
-    __host__ __device__ int wide() const { return f_wide * t_wide; }
-    __host__ __device__ int count() const { return f_wide * t_wide + f_narrow * t_narrow; }
-};
 
 constexpr int GEMM_MAX_OUTS = 8;
 struct GemmParams {
@@ -1096,47 +1088,6 @@ template <typename T, bool PAIR> static int gemm_launch(const GemmParams &p, con
     return p.out_tma ? gemm_launch_as<T, PAIR, true>(p, maps, st) : gemm_launch_as<T, PAIR, false>(p, maps, st);
 }
 
-// Tile widths: the choice whose slowest pair costs least.  A tile of bn columns costs what bn + 40 columns at full rate do (narrow
-// tiles read more shared memory per product; fp32, 3072 <- 768, 4096 tokens: 28.6 us per wave at 256, 15.8 at 128, 10.8 at 64).
-// Tiles of one width leave most pairs without work in a last wave that is not full, so some rows of tiles at the end of the
-// order may be narrower: their tiles then fill the places that the wide ones leave.  Tile i goes to pair i % units.
-// 4096 x 4096 bf16, 4096 tokens: 256 tiles, 3.46 waves of 74 pairs, 110.0 -> 106.7 us with three of sixteen rows in tiles of 192;
-// 4096 x 1024 f16 pair, 12288 tokens: 212.0 -> 208.2.  From sixteen waves on the last one is too small a part.
-// 16-bit: wide tiles have 256 columns, narrow ones 128 or 192 (whole staged groups for both halves of the drain warps).
-static GemmTiles gemm_tiles(int64_t tiles_f, int64_t cols, int64_t units, bool fp32, bool pair) {
-    GemmTiles best{(int)tiles_f, 0, (int)((cols + TC_BN - 1) / TC_BN), 0, TC_BN, TC_BN};
-    if (!pair) return best;
-    const int step = fp32 ? 32 : 64, least = fp32 ? 64 : 128, widths = (TC_BN - least) / step + 1;
-    int per_row[7];  // tiles per row at width least + i * step
-    for (int i = 0; i < widths; i++) per_row[i] = (int)((cols + least + i * step - 1) / (least + i * step));
-    const int u = (int)units;
-    int64_t best_cost = INT64_MAX;
-    for (int i = widths - 1; i >= (fp32 ? 0 : widths - 1); i--) {
-        const int bn = least + i * step, cost = bn + 40;
-        const int64_t all = tiles_f * per_row[i], uniform = (all + u - 1) / u * cost;
-        if (uniform < best_cost) {
-            best = GemmTiles{(int)tiles_f, 0, per_row[i], 0, bn, bn};
-            best_cost = uniform;
-        }
-        if (all > 16 * units) continue;  // a sixteenth of the last wave at most: not worth a second shape of tiles
-        for (int j = i - 1; j >= 0; j--) {
-            const int bn_tail = least + j * step, cost_tail = bn_tail + 40;
-            // more narrow tiles than two waves of them never help: a wide tile does the same columns in less time
-            for (int f = 1; f < tiles_f && f * per_row[j] <= 2 * u; f++) {
-                const int64_t wide = all - (int64_t)f * per_row[i], full = wide / u;
-                const int rest = (int)(wide - full * u), tail = f * per_row[j];
-                int64_t c = full * cost + (tail + u - 1) / u * cost_tail;                                   // a pair without a tile of the last wide wave
-                const int over = tail - (u - rest);                                                          // narrow tiles left for the pairs with one
-                if (rest > 0 && (full + 1) * cost + (over > 0 ? (over + u - 1) / u : 0) * cost_tail > c) c = (full + 1) * cost + (over > 0 ? (over + u - 1) / u : 0) * cost_tail;
-                if (c < best_cost) {
-                    best = GemmTiles{(int)tiles_f - f, f, per_row[i], per_row[j], bn, bn_tail};
-                    best_cost = c;
-                }
-            }
-        }
-    }
-    return best;
-}
 // (val, idx) -> the weight with its zeros restored, rows `ld` elements apart at `dst` (16-byte aligned, ld a multiple of 8).
 // plain = false: the matmul's operand, 16-bit or three bf16 planes for fp32; plain = true: the
 // weight in its own dtype (the densifier), where full stores must not run past the row: K a multiple of 8, or the rows kernel.

@@ -764,7 +764,8 @@ bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens, bo
     if (!dense) return false;
     if (!fused) return true;
     if (!have_packed) return tokens >= (dtype == NMG_F32 ? 513 : 1280);
-    return tokens >= (dtype == NMG_F32 ? 1025 : transposed ? 1280 : 1536);
+    if (dtype == NMG_F32) return tokens > 1024 || (tokens > 512 && ((transposed ? geo.K : geo.M) + TC_BM - 1) / TC_BM * ((tokens + 127) / 128) > kFxClusters[1]);
+    return tokens >= (transposed ? 1280 : 1536);
 }
 
 // act: [tokens][ld_act] with the reduction axis contiguous (X for the forward, dY for the transposed product).

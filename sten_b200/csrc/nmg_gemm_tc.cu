@@ -353,58 +353,54 @@ template <int ROWS> __global__ void __launch_bounds__(SPLIT_THREADS) split_rows_
 
 // The same from a K-major activation src[red][ld_src >= tokens], transposed through a 64 x 32 tile on the way.  A CTA looks at the rest of
 // a token's row only if its own part holds values of it and none that settles the matter.
-constexpr int COLS_THREADS = 256, COLS_RED = 64;
+constexpr int COLS_THREADS = 256, COLS_RED = 64, COLS_WARPS = COLS_THREADS / 32;
 __global__ void __launch_bounds__(COLS_THREADS) split_columns_kernel(const SplitParams p) {
-    __shared__ float tile[COLS_RED][33];   // [reduction][token]
-    __shared__ unsigned big, nonzero;      // by token
+    __shared__ float tile[COLS_RED][33];                                        // [reduction][token]
+    __shared__ __align__(16) unsigned found_big[COLS_WARPS], found_any[COLS_WARPS];  // bits by token
     dependents_launch();
     dependents_wait();
-    const int64_t k0 = (int64_t)blockIdx.x * COLS_RED;
+    const int64_t k0 = (int64_t)blockIdx.x * COLS_RED, t0 = (int64_t)blockIdx.y * 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int64_t t0 = (int64_t)blockIdx.y * 32; t0 < p.rows; t0 += (int64_t)gridDim.y * 32) {
-        __syncthreads();  // the tile and the masks of the tokens before have been read
-        if (threadIdx.x == 0) big = nonzero = 0;
+    const int64_t t = t0 + lane;
+    auto at = [&](int64_t k) -> float { return k < p.cols && t < p.rows ? p.src[k * p.ld_src + t] : 0.f; };
+    auto all = [](const unsigned *found) -> unsigned {
+        const uint4 a = reinterpret_cast<const uint4 *>(found)[0], b = reinterpret_cast<const uint4 *>(found)[1];
+        return a.x | a.y | a.z | a.w | b.x | b.y | b.z | b.w;
+    };
+    static_assert(COLS_WARPS == 8, "two 16-byte reads");
+    bool b = false, any = false;
+#pragma unroll
+    for (int i = 0; i < COLS_RED / COLS_WARPS; i++) {
+        const float v = at(k0 + warp + i * COLS_WARPS);
+        tile[warp + i * COLS_WARPS][lane] = v;
+        b |= not_tiny(v);
+        any |= v != 0.f;
+    }
+    const unsigned bm = __ballot_sync(0xffffffffu, b), am = __ballot_sync(0xffffffffu, any);
+    if (lane == 0) {
+        found_big[warp] = bm;
+        found_any[warp] = am;
+    }
+    __syncthreads();
+    unsigned big = all(found_big);
+    const unsigned own = all(found_any);
+    for (int64_t k = 0; k < p.cols && (own & ~big); k += COLS_RED) {  // the same for all threads
+        b = false;
+#pragma unroll
+        for (int i = 0; i < COLS_RED / COLS_WARPS; i++) b |= not_tiny(at(k + warp + i * COLS_WARPS));
+        const unsigned m = __ballot_sync(0xffffffffu, b);
+        __syncthreads();  // what was found before has been read
+        if (lane == 0) found_big[warp] = m;
         __syncthreads();
-        const int64_t t = t0 + lane;
-        auto at = [&](int64_t k) -> float { return k < p.cols && t < p.rows ? p.src[k * p.ld_src + t] : 0.f; };
-        bool b = false, nz = false;
+        big |= all(found_big);
+    }
+    if (threadIdx.x < 32 && t < p.rows && ((own >> lane) & 1)) p.factors[t] = ((big >> lane) & 1) ? 1.f : TINY_FACTOR;  // CTAs that write agree
+    const int r = threadIdx.x >> 3, c8 = (threadIdx.x & 7) * 8;  // token within the tile, reduction offset
+    if (t0 + r < p.rows && k0 + c8 < p.ld) {
+        float f[8];
 #pragma unroll
-        for (int i = 0; i < COLS_RED / 8; i++) {
-            const float v = at(k0 + warp + i * 8);
-            tile[warp + i * 8][lane] = v;
-            b |= not_tiny(v);
-            nz |= v != 0.f;
-        }
-        const unsigned bm = __ballot_sync(0xffffffffu, b), nm = __ballot_sync(0xffffffffu, nz);
-        if (lane == 0) {
-            atomicOr(&big, bm);
-            atomicOr(&nonzero, nm);
-        }
-        __syncthreads();
-        const unsigned here = big, own = nonzero;  // `big` may grow below
-        if (own & ~here) {  // the same for all threads
-            __syncthreads();
-            for (int64_t k = 0; k < p.cols; k += 64) {
-                b = false;
-#pragma unroll
-                for (int i = 0; i < 8; i++) b |= not_tiny(at(k + warp + i * 8));
-                const unsigned m = __ballot_sync(0xffffffffu, b);
-                if (lane == 0) atomicOr(&big, m);
-                __syncthreads();
-                const unsigned now = big;
-                __syncthreads();
-                if (!(own & ~now)) break;
-            }
-        }
-        const unsigned mask = big;
-        if (threadIdx.x < 32 && t < p.rows && ((own >> lane) & 1)) p.factors[t] = ((mask >> lane) & 1) ? 1.f : TINY_FACTOR;  // CTAs that write agree
-        const int r = threadIdx.x >> 3, c8 = (threadIdx.x & 7) * 8;  // token within the tile, reduction offset
-        if (t0 + r < p.rows && k0 + c8 < p.ld) {
-            float f[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) f[i] = tile[c8 + i][r];
-            store_split(p, t0 + r, k0 + c8, f, ((own & ~mask) >> r) & 1 ? TINY_SCALE : 1.f);
-        }
+        for (int i = 0; i < 8; i++) f[i] = tile[c8 + i][r];
+        store_split(p, t0 + r, k0 + c8, f, ((own & ~big) >> r) & 1 ? TINY_SCALE : 1.f);
     }
 }
 

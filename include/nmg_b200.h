@@ -130,7 +130,7 @@ int nmg_pack(const void *val, const int16_t *idx, int64_t M, int64_t K, int n, i
  * algo: NMG_ALGO_AUTO uses the tensor cores for weights of at least 64 rows, at every token count (16-bit rows that are not
  * 16-byte aligned, and K-major activations, are re-laid out into the workspace first); fewer than 64 K-major columns take
  * them when `packed` is given.  The SIMT kernels serve the rest.  Two tensor-core variants exist.  Below 1536 tokens
- * (1025 in fp32), for m in {4, 8, 16} and n <= 2, one fused kernel expands tiles of the packed copy inside the matmul; when
+ * (1025 in fp32, 513 where its 128 x 128 tiles are more than the 148 SMs), for m in {4, 8, 16} and n <= 2, one fused kernel expands tiles of the packed copy inside the matmul; when
  * `packed` is NULL it serves fewer than 1280 tokens (513 in fp32).  From there on, and for every other (n, m), the weight is first expanded into a transient dense 16-bit matrix in the workspace
  * (M * round_up(K, 8) * 2 bytes; three such planes for fp32) and multiplied by a persistent TMA-fed kernel; that
  * variant reads val / idx and ignores `packed`.  fp32 operands go through the tensor cores as exact three-way bf16

@@ -749,16 +749,18 @@ static int tc_launch_nm(int dtype, bool transposed, bool fine, const TcParams &p
 // Policy of the two tensor-core variants.  The fused kernel reads the column-ordered copy; without one (have_packed) a call
 // would build it first and throw it away.  Measured, us, 2:4: fused with a kept copy / fused after building one / two passes
 //   fp32   tokens    1024 x 1024       4096 x 1024       1024 x 4096       4096 x 4096
-//             256    15 /  33 / 29     22 /  47 /  35    27 / 49 / 68      52 / 113 / 109
-//             512    18 /  37 / 29     29 /  53 /  42    33 / 56 / 70      87 / 157 / 129
-//            1000    23 /  41 / 29     51 /  77 /  60    55 / 78 / 78     189 / 250 / 180
-//            2048    29 /  48 / 36    101 / 128 /  93    95 / 125 / 111   377 / 431 / 313
+//              64    10 /  23 / 21     13 /  33 / 27    17 / 35 / 61      26 /  81 /  98
+//             256    13 /  26 / 23     22 /  43 / 30    27 / 46 / 62      58 / 114 / 104
+//             512    18 /  31 / 25     31 /  51 / 35    36 / 55 / 65     100 / 156 / 119
+//             768    20 /   - / 27     54 /   - / 44    55 /  - / 67     171 /   - / 139
+//            1024    24 /   - / 28     58 /   - / 53    61 /  - / 71     197 /   - / 166
 //   bf16     1024     9 /  24 / 17     12 /  30 /  21    20 / 37 / 31      27 /  65 /  42
 //            1280    10 /  24 / 17     19 /  37 /  25    21 / 37 / 32      49 /  86 /  60
 //            1500    10 /  24 / 17     20 /  39 /  25    23 / 40 / 33      50 /  88 /  61
 //            3072    11 /  26 / 17     32 /  51 /  30    26 / 44 / 33      87 / 130 /  89
-// (fp32 without a copy: up to 512 tokens the shape decides, not the count.)  The transposed product of a 16-bit weight has the
-// structured-sparse kernel in place of the second variant (from 1280 tokens).
+// fp32 with a copy: above 512 tokens the fused kernel wins while all its tiles are resident, and loses in its second wave.  Without one,
+// up to 512 tokens the shape decides, not the count; the fused kernel takes them, with the same results as with a copy.  The transposed
+// product of a 16-bit weight has the structured-sparse kernel in place of the second variant (from 1280 tokens).
 bool tc_use_dense(const Geo &geo, int dtype, bool transposed, int64_t tokens, bool have_packed) {
     const bool fused = tc_supported(geo, dtype), dense = tc_dense_supported(geo, dtype);
     if (!dense) return false;

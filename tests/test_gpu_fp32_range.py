@@ -147,3 +147,50 @@ def test_tiny_rows_longer_than_the_registers():
     wide[:, 1:] = x
     for a in (x, wide[:, 1:]):  # the second: rows that take no 16-byte loads
         _close(ops.spmm(val, idx, rows, cols, 2, 4, 4, a, algo=nat.NMG_ALGO_TENSOR), a.double(), dense)
+
+
+@pytest.mark.parametrize("m_rows,k_cols,tokens", [(512, 1000, 1025), (517, 1032, 1030), (203, 5003, 1040), (512, 1000, 70), (517, 1032, 513), (203, 5003, 200)])
+@pytest.mark.parametrize("n,m,g", [(1, 4, 16), (2, 4, 1), (2, 8, 4), (3, 6, 3)])
+def test_rows_of_different_magnitude(n, m, g, m_rows, k_cols, tokens):
+    """Rows of both operands over many binades, some columns apart from the others, rows that take no 16-byte loads: the plain bound holds."""
+    from sten_b200 import _native as nat, ops
+    gen = lambda seed: torch.Generator().manual_seed(seed)  # noqa: E731
+    w = seeded_normal((m_rows, k_cols), 1) * k_cols ** -0.5 * torch.exp2(torch.randint(-40, 40, (m_rows, 1), generator=gen(7)).float())
+    w[:, 1::7] *= 2.0 ** -9
+    w = w.to(cuda())
+    val, idx = ops.sparsify(w.unsqueeze(0), n, m, g)
+    dense = ops.densify(val, idx, 1, m_rows, k_cols, n, m, g)[0].double()
+    x, dy = seeded_normal((tokens, k_cols + 3), 2), seeded_normal((tokens, m_rows + 1), 3)
+    x = x * torch.exp2(torch.randint(-60, 60, (tokens, 1), generator=gen(8)).float())
+    x[5] = 0
+    dy[:, 2] *= 2.0 ** 14
+    x, dy = x.to(cuda())[:, 1:k_cols + 1], dy.to(cuda())[:, :m_rows]
+    copy = ops.pack(val, idx, m_rows, k_cols, n, m, g) if (n, m) != (3, 6) else None
+    _close(ops.spmm(val, idx, m_rows, k_cols, n, m, g, x, packed=copy, algo=nat.NMG_ALGO_TENSOR), x.double(), dense)
+    y = ops.spmm(val, idx, m_rows, k_cols, n, m, g, x.t().contiguous(), layout=nat.NMG_ACT_K_MAJOR, packed=copy, algo=nat.NMG_ALGO_TENSOR)
+    _close(y.t(), x.double(), dense)
+    _close(ops.spmm_t(val, idx, m_rows, k_cols, n, m, g, dy, packed=copy, algo=nat.NMG_ALGO_TENSOR), dy.double(), dense.t())
+    assert ops.read_status() == 0
+
+
+@pytest.mark.parametrize("features,tokens,fused", [(4736, 512, True), (4737, 512, True), (3712, 513, True), (3713, 513, False), (3712, 640, True), (3200, 641, False),
+                                                   (3072, 768, True), (3073, 768, False), (2304, 1024, True), (2305, 1024, False), (64, 1024, True), (64, 1025, False)])
+@pytest.mark.parametrize("transposed", [False, True])
+def test_both_sides_of_the_line(transposed, features, tokens, fused):
+    """With a kept copy: the fused kernel while its tiles of 128 x 128 fit the chip at once, two passes from there on; with aligned rows, rows that
+    take no 16-byte loads and K-major ones."""
+    from sten_b200 import _native as nat, ops
+    n, m, g, red = 2, 4, 4, 200
+    rows, cols = (red, features) if transposed else (features, red)
+    val, idx = ops.sparsify(seeded_normal((rows, cols), 1).to(cuda()).unsqueeze(0), n, m, g)
+    dense = ops.densify(val, idx, 1, rows, cols, n, m, g)[0].double()
+    copy = ops.pack(val, idx, rows, cols, n, m, g)
+    assert ops.uses_packed(rows, cols, tokens, n, m, g, torch.float32, transposed=transposed) == fused
+    wide = seeded_normal((tokens, red + 1), 2).to(cuda())
+    for a in (wide[:, :red].contiguous(), wide[:, 1:]):
+        if transposed:
+            _close(ops.spmm_t(val, idx, rows, cols, n, m, g, a, packed=copy), a.double(), dense.t())
+            continue
+        _close(ops.spmm(val, idx, rows, cols, n, m, g, a, packed=copy), a.double(), dense)
+        _close(ops.spmm(val, idx, rows, cols, n, m, g, a.t().contiguous(), layout=nat.NMG_ACT_K_MAJOR, packed=copy).t(), a.double(), dense)
+    assert ops.read_status() == 0
